@@ -170,7 +170,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(hempty + MAX_HALOS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::MAX_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -199,7 +199,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -256,7 +256,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, P::A_MN ? 1 : 0, P::B_MN ? 1 : 0);
       // The issuing thread is one lane with nothing to hide its instruction latency behind: every instruction
       // between two tcgen05.mma widens the gap between them.  (Timestamps taken in this loop: a 128 x 64 x 16
