@@ -53,9 +53,9 @@ __device__ inline void control_step(DevChannel* ch, int flush) {
   ch->t_phase[2] = DevEnv::now_ns();
 }
 
-__global__ void __launch_bounds__(256, 3) pack_ctl_kernel(DevChannel* ch, int flush) {
+__global__ void __launch_bounds__(256, 3) pack_ctl_kernel(DevChannel* ch, int flush, int grad_src) {
   __shared__ int s_flag;
-  if (!flush) pack_phase(ch, blockIdx.x, gridDim.x, &s_flag);
+  if (!flush) pack_phase(ch, grad_src, blockIdx.x, gridDim.x, &s_flag);
   // Device-scope fence per thread, system-scope fence once: the control step fences at system scope before
   // it publishes the epoch, and that fence carries the other blocks' slot writes with it (they are ordered
   // before it through this counter).
@@ -75,6 +75,19 @@ __global__ void __launch_bounds__(256, 3) data_kernel(DevChannel* ch) {
   data_phase(ch, blockIdx.x, gridDim.x, &s_flag);
 }
 
+// One step of a one-rank channel in one launch (see local_apply).
+__global__ void __launch_bounds__(256, 4) local_step_kernel(DevChannel* ch, int grad_src) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) ch->t_phase[0] = DevEnv::now_ns();
+  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
+  if (ch->slot_bf16) local_apply<__nv_bfloat16>(ch, grad_src, tid, nth);
+  else local_apply<float>(ch, grad_src, tid, nth);
+  __syncthreads();
+  if (threadIdx.x == 0 && (gridDim.x == 1 || atomicAdd(&ch->bar_end, 1u) == gridDim.x - 1)) {
+    ch->bar_end = 0;
+    local_records(ch);
+  }
+}
+
 // All ranks of a (small) world inside ONE launch, one block per rank: used to
 // exercise the multi-rank protocol on a single GPU, where separate launches
 // that wait on one another are not guaranteed to run concurrently.
@@ -86,7 +99,7 @@ __global__ void __launch_bounds__(256) emulated_step_kernel(DevChannel** chans, 
     while (DevEnv::now_ns() - t0 < delay_ns[blockIdx.x]) __nanosleep(200);
   }
   __syncthreads();
-  if (!flush) pack_phase(ch, 0, 1, &s_flag);
+  if (!flush) pack_phase(ch, SRC_FLAT, 0, 1, &s_flag);
   __threadfence_system();
   __syncthreads();
   if (threadIdx.x == 0) { ch->pack_ticket = 0; control_step(ch, flush); }
@@ -153,6 +166,9 @@ struct esgd_channel_desc {
   void* mc_slot1;                 // (all null: the arenas have no multicast mapping)
   void* mc_red;
   uint64_t mc_min;                // element count from which full rounds go over the switch
+  uint64_t valid;                 // elements of grad_in / out that exist (0: count)
+  int32_t keep_out, pad4;         // leave out alone in a step that applies nothing
+  void* outcome;                  // pinned host memory for the step's outcome (may be null)
 };
 
 uint64_t esgd_dev_channel_bytes(void) { return sizeof(DevChannel); }
@@ -179,6 +195,7 @@ int esgd_channel_configure(void* dch, const esgd_channel_desc* d, void* stream) 
   h.pol.seed = d->seed; h.pol.accumulate = d->accumulate; h.pol.adaptive_grace = d->adaptive_grace;
   h.count = d->count; h.slot_bf16 = d->slot_bf16; h.grad_in_bf16 = d->grad_in_bf16;
   h.grad_in = d->grad_in; h.w32 = (float*)d->w32; h.mom = (float*)d->mom; h.w16 = (__nv_bfloat16*)d->w16;
+  h.valid = d->valid ? d->valid : d->count; h.keep_out = d->keep_out; h.outcome = (StepOutcome*)d->outcome;
   h.out = d->out; h.out_bf16 = d->out_bf16; h.hyper = (const float*)d->hyper;
   cudaError_t e = cudaMemcpyAsync(dch, &h, sizeof(h), cudaMemcpyHostToDevice, (cudaStream_t)stream);
   if (e != cudaSuccess) return (int)e;
@@ -209,20 +226,93 @@ static inline int grid_for(uint64_t count, int max_blocks) {
   return (int)(need < (uint64_t)max_blocks ? need : (uint64_t)max_blocks);
 }
 
-// One full step of one channel on `stream`: two launches.
-int esgd_channel_step(void* dch, uint64_t count, int max_blocks, void* stream) {
+// One full step of one channel on `stream`: two launches.  grad_src: bit 0 the flat gradient, bit 1 the accumulators.
+int esgd_channel_step(void* dch, uint64_t count, int max_blocks, int grad_src, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   int g = grid_for(count, max_blocks);
-  pack_ctl_kernel<<<g, 256, 0, s>>>((DevChannel*)dch, 0);
+  pack_ctl_kernel<<<g, 256, 0, s>>>((DevChannel*)dch, 0, grad_src);
   data_kernel<<<g, 256, 0, s>>>((DevChannel*)dch);
   count_launch(2);
   return (int)cudaGetLastError();
 }
 
+// The same for a channel of one rank whose gradient is in a flat buffer of its own: one launch.
+int esgd_channel_step_local(void* dch, uint64_t count, int max_blocks, int grad_src, void* stream) {
+  uint64_t need = (count / 8 + 255) / 256;
+  if (need < 1) need = 1;
+  local_step_kernel<<<(int)(need < (uint64_t)max_blocks ? need : (uint64_t)max_blocks), 256, 0, (cudaStream_t)stream>>>(
+      (DevChannel*)dch, grad_src);
+  count_launch();
+  return (int)cudaGetLastError();
+}
+
+// Give a channel fp32 gradient accumulators of `count` elements beside its flat gradient.
+int esgd_channel_set_grad_acc(void* dch, float* acc, void* stream) {
+  cudaError_t e = cudaMemcpyAsync((char*)dch + offsetof(DevChannel, grad_acc), &acc, sizeof(acc), cudaMemcpyHostToDevice,
+                                  (cudaStream_t)stream);
+  if (e != cudaSuccess) return (int)e;
+  return (int)cudaStreamSynchronize((cudaStream_t)stream);
+}
+
+// ---- post / wait of a stand-alone collective: each one native call --------------------------------------------
+struct esgd_collective {
+  cudaEvent_t ready, done;        // the caller's stream has written the tensor; the step has completed
+  cudaStream_t side;
+  void* dch;
+  uint64_t count;
+  int max_blocks, local;
+};
+
+int esgd_collective_create(void* dch, uint64_t count, int max_blocks, int local, void* side, void** out) {
+  esgd_collective* c = new esgd_collective{nullptr, nullptr, (cudaStream_t)side, dch, count, max_blocks, local};
+  cudaError_t e = cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming);
+  *out = c;
+  return (int)e;
+}
+void esgd_collective_destroy(void* h) {
+  esgd_collective* c = (esgd_collective*)h;
+  if (c == nullptr) return;
+  if (c->ready) cudaEventDestroy(c->ready);
+  if (c->done) cudaEventDestroy(c->done);
+  delete c;
+}
+// Launch a step on the side stream behind what `stream` holds so far.
+int esgd_collective_post(void* h, void* stream) {
+  esgd_collective* c = (esgd_collective*)h;
+  cudaError_t e = cudaEventRecord(c->ready, (cudaStream_t)stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ready, 0);
+  if (e != cudaSuccess) return (int)e;
+  int rc = c->local ? esgd_channel_step_local(c->dch, c->count, c->max_blocks, SRC_FLAT, c->side)
+                    : esgd_channel_step(c->dch, c->count, c->max_blocks, SRC_FLAT, c->side);
+  if (rc != 0) return rc;
+  return (int)cudaEventRecord(c->done, c->side);
+}
+// Has the posted step completed?  1 yes, 0 no, negative CUDA error code.
+int esgd_collective_test(void* h) {
+  cudaError_t e = cudaEventQuery(((esgd_collective*)h)->done);
+  return e == cudaSuccess ? 1 : (e == cudaErrorNotReady ? 0 : -(int)e);
+}
+// Order `stream` behind the posted step and wait for it on the host.
+int esgd_collective_wait(void* h, void* stream) {
+  esgd_collective* c = (esgd_collective*)h;
+  cudaError_t e = cudaStreamWaitEvent((cudaStream_t)stream, c->done, 0);
+  if (e == cudaSuccess) e = cudaEventSynchronize(c->done);
+  return (int)e;
+}
+
+// Pinned, device-visible host memory for a channel's outcome.
+int esgd_host_alloc(uint64_t bytes, void** ptr) {
+  cudaError_t e = cudaHostAlloc(ptr, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
+  if (e == cudaSuccess) memset(*ptr, 0, bytes);
+  return (int)e;
+}
+int esgd_host_free(void* ptr) { return (int)cudaFreeHost(ptr); }
+
 int esgd_channel_flush(void* dch, uint64_t count, int max_blocks, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   int g = grid_for(count, max_blocks);
-  pack_ctl_kernel<<<1, 32, 0, s>>>((DevChannel*)dch, 1);
+  pack_ctl_kernel<<<1, 32, 0, s>>>((DevChannel*)dch, 1, SRC_FLAT);
   data_kernel<<<g, 256, 0, s>>>((DevChannel*)dch);
   count_launch(2);
   return (int)cudaGetLastError();

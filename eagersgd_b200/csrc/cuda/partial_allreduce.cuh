@@ -47,6 +47,13 @@ namespace esgd {
 
 enum HyperIdx { HP_LR = 0, HP_MOMENTUM = 1, HP_WD = 2, HP_NESTEROV = 3, HP_GRAD_SCALE = 4, HP_COUNT = 8 };
 
+// What a step did, written by its last thread into pinned host memory: the host reads it after the step's event
+// without a copy of its own.
+struct StepOutcome {
+  uint64_t round;
+  uint32_t role, contributors, is_sync, applied, status, pad;
+};
+
 struct DevChannel {
   ChannelView view;
   void* slot[kMaxRanks][kSlotDepth];
@@ -79,6 +86,11 @@ struct DevChannel {
   uint64_t mc_min;           // smallest element count that goes over the switch when it can
   uint64_t t_phase[8];       // clock at: first block packing, control start, control end, first data block,
                              // share reduced (two-shot), data end; for the latency break-down of the benchmarks
+  uint64_t valid;            // elements of grad_in and out that exist (count is this rounded up to eight)
+  int32_t keep_out;          // a step that applies nothing leaves out alone instead of zeroing it
+  int32_t pad2;
+  float* grad_acc;           // fp32 gradient accumulators beside a bf16 grad_in (or null)
+  StepOutcome* outcome;      // pinned host memory (or null): what the newest step did, readable once it has completed
 };
 
 __device__ __forceinline__ void load8(const __nv_bfloat16* p, uint64_t i, float v[8]) {
@@ -116,6 +128,22 @@ __device__ __forceinline__ void round8(const __nv_bfloat16*, float v[8]) {
 }
 __device__ __forceinline__ void round8(const float*, float[8]) {}
 
+// Eight elements of the caller's tensors (gradient in, averaged gradient out), whose length need not be a multiple of
+// eight: the last vector is moved element by element, elements past the end read as zeros.
+template <typename T>
+__device__ __forceinline__ void load8_tail(const T* p, uint64_t i, uint64_t valid, float v[8]) {
+  if (i + 8 <= valid) { load8(p, i, v); return; }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = i + q < valid ? (float)p[i + q] : 0.0f;
+}
+template <typename T>
+__device__ __forceinline__ void store8_tail(T* p, uint64_t i, uint64_t valid, const float v[8]) {
+  if (i + 8 <= valid) { store8(p, i, v); return; }
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (i + q < valid) p[i + q] = (T)v[q];
+}
+
 // Apply one 8-vector of the averaged gradient.
 __device__ __forceinline__ void apply8(const DevChannel* ch, uint64_t i, float g[8], float lr, float mu, float wd,
                                        float nesterov, float gscale) {
@@ -134,9 +162,34 @@ __device__ __forceinline__ void apply8(const DevChannel* ch, uint64_t i, float g
     store8(ch->mom, i, m);
     if (ch->w16 != nullptr) store8(ch->w16, i, w);
   } else if (ch->out != nullptr) {
-    if (ch->out_bf16) store8(reinterpret_cast<__nv_bfloat16*>(ch->out), i, g);
-    else store8(reinterpret_cast<float*>(ch->out), i, g);
+    if (ch->out_bf16) store8_tail(reinterpret_cast<__nv_bfloat16*>(ch->out), i, ch->valid, g);
+    else store8_tail(reinterpret_cast<float*>(ch->out), i, ch->valid, g);
   }
+}
+
+// Where a step finds the gradient: the flat gradient, the fp32 accumulators that operators add to directly, or (their
+// sum) both.
+enum GradSource { SRC_FLAT = 1, SRC_ACC = 2 };
+
+__device__ __forceinline__ void load_grad8(const DevChannel* ch, uint64_t i, int src, float v[8]) {
+  if (src & SRC_FLAT) {
+    if (ch->grad_in_bf16) load8_tail(reinterpret_cast<const __nv_bfloat16*>(ch->grad_in), i, ch->valid, v);
+    else load8_tail(reinterpret_cast<const float*>(ch->grad_in), i, ch->valid, v);
+  }
+  if (src & SRC_ACC) {
+    float a[8];
+    load8(ch->grad_acc, i, a);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = (src & SRC_FLAT) ? v[q] + a[q] : a[q];
+  }
+}
+__device__ __forceinline__ void clear_grad8(const DevChannel* ch, uint64_t i, int src) {
+  const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (src & SRC_FLAT) {
+    if (ch->grad_in_bf16) store8_tail(reinterpret_cast<__nv_bfloat16*>(ch->grad_in), i, ch->valid, z);
+    else store8_tail(reinterpret_cast<float*>(ch->grad_in), i, ch->valid, z);
+  }
+  if (src & SRC_ACC) store8(ch->grad_acc, i, z);
 }
 
 struct Hyper {
@@ -290,12 +343,84 @@ __device__ inline void data_drain(const DevChannel* ch, uint64_t tid, uint64_t n
 }
 
 __device__ inline void data_zero_out(const DevChannel* ch, uint64_t tid, uint64_t nthreads) {
-  if (ch->w32 != nullptr || ch->out == nullptr) return;  // fused mode: nothing to apply
+  if (ch->w32 != nullptr || ch->out == nullptr || ch->keep_out) return;  // fused mode: nothing to apply
   float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (uint64_t i = tid * 8; i < ch->count; i += nthreads * 8) {
-    if (ch->out_bf16) store8(reinterpret_cast<__nv_bfloat16*>(ch->out), i, z);
-    else store8(reinterpret_cast<float*>(ch->out), i, z);
+    if (ch->out_bf16) store8_tail(reinterpret_cast<__nv_bfloat16*>(ch->out), i, ch->valid, z);
+    else store8_tail(reinterpret_cast<float*>(ch->out), i, ch->valid, z);
   }
+}
+
+__device__ inline void report_outcome(const DevChannel* ch) {
+  if (ch->outcome == nullptr) return;
+  const ChannelCtl* me = ch->view.ctl[ch->cfg.rank];
+  StepOutcome o;
+  o.round = me->stat_last_round;
+  o.role = (uint32_t)ch->plan.role;
+  o.contributors = ch->plan.role == ROLE_PARTICIPANT ? (uint32_t)me->stat_last_contrib : 0u;
+  o.is_sync = (uint32_t)ch->plan.is_sync;
+  o.applied = (uint32_t)ch->applied;
+  o.status = me->status;
+  o.pad = 0;
+  *ch->outcome = o;
+}
+
+// A step of a channel whose world is one rank, in one pass: nobody reads the publish slot and no wait has anything to
+// wait for, so the gradient goes straight to where it is applied and the round's records are written once at the end.
+// The gradient takes the same rounding to the slot's element type as in a round with peers.
+template <typename ST>
+__device__ __forceinline__ void local_apply(DevChannel* ch, int grad_src, uint64_t tid, uint64_t nth) {
+  const Hyper hp(ch->hyper);
+  for (uint64_t i = tid * 8; i < ch->count; i += nth * 8) {
+    float g[8];
+    load_grad8(ch, i, grad_src, g);
+    if (ch->clear_grad) clear_grad8(ch, i, grad_src);
+    round8(static_cast<const ST*>(nullptr), g);
+    apply8(ch, i, g, hp.lr, hp.mu, hp.wd, hp.nesterov, hp.gscale);
+  }
+}
+
+// What ctl_step, activate_round and finish_step leave behind after a round of one rank (one thread).
+__device__ inline void local_records(DevChannel* ch) {
+  ChannelCtl* me = ch->view.ctl[0];
+  const uint64_t k = me->local_step + 1, t = DevEnv::now_ns();
+  const bool sync_round = round_is_sync(ch->pol, k);
+  me->local_step = k;
+  me->pub_epoch[0] = k;
+  me->owner = me->snap_round = me->latest_round = me->round_done = k;
+  me->taken[k % kSlotDepth] = k;
+  me->done_count[k % kDescRing] = 1;
+  RoundDesc* d = &me->desc[k % kDescRing];
+  d->round = k;
+  d->activator = 0;
+  d->n_fresh = d->n_contrib = d->fresh_mask = d->contrib_mask = 1;
+  d->push_mask = d->accum_mask = 0;
+  d->is_sync = sync_round ? 1u : 0u;
+  d->read_epoch[0] = d->consumed[0] = k;
+  me->stat_rounds_participated++;
+  me->stat_rounds_activated++;
+  me->stat_contrib_sum++;
+  if (sync_round) me->stat_sync_rounds++;
+  me->stat_last_round = k;
+  me->stat_last_contrib = 1;
+  for (int q = 0; q < 6; ++q) me->ctl_t[q] = t;
+  TraceEntry* te = &me->trace[k % kTraceRing];
+  te->step = te->round = k;
+  te->t_ns = t;
+  te->wait_ns = 0;
+  te->role = ROLE_PARTICIPANT;
+  te->activator = 0;
+  te->fresh_mask = te->contrib_mask = 1;
+  te->is_sync = sync_round ? 1u : 0u;
+  te->drain_rounds = 0;
+  ch->plan.role = ROLE_PARTICIPANT;
+  ch->plan.is_sync = sync_round ? 1 : 0;
+  ch->plan.round = k;
+  ch->applied = 1;
+  ch->t_phase[1] = ch->t_phase[2] = ch->t_phase[3] = ch->t_phase[0];
+  ch->t_phase[4] = 0;
+  ch->t_phase[5] = DevEnv::now_ns();
+  report_outcome(ch);
 }
 
 // The whole data phase of one rank, run by `nblk` blocks of which this is block `blk`.  `s_flag` is a
@@ -371,6 +496,7 @@ __device__ inline void data_phase(DevChannel* ch, uint32_t blk, uint32_t nblk, i
         atomicOr(&ch->view.ctl[ch->cfg.rank]->status, (uint32_t)ST_DESC_LAPPED);
       finish_step<DevEnv>(ch->view, ch->cfg, &ch->plan);
       ch->t_phase[5] = DevEnv::now_ns();
+      report_outcome(ch);
     }
   }
 }
@@ -378,7 +504,7 @@ __device__ inline void data_phase(DevChannel* ch, uint32_t blk, uint32_t nblk, i
 // Copy (and convert) the flat gradient into publish slot (next epoch % 2), or add it to what the slot
 // still holds when the gradient published two epochs ago was never picked up by a round; clear the flat
 // gradient for the next backward pass if asked to.  `s_flag` is a word of shared memory.
-__device__ inline void pack_phase(DevChannel* ch, uint32_t blk, uint32_t nblk, int* s_flag) {
+__device__ inline void pack_phase(DevChannel* ch, int grad_src, uint32_t blk, uint32_t nblk, int* s_flag) {
   const uint64_t tid = (uint64_t)blk * blockDim.x + threadIdx.x, nthreads = (uint64_t)nblk * blockDim.x;
   ChannelCtl* me = ch->view.ctl[ch->cfg.rank];
   const uint64_t k = me->local_step + 1;
@@ -410,7 +536,6 @@ __device__ inline void pack_phase(DevChannel* ch, uint32_t blk, uint32_t nblk, i
   if (ch->grad_in == nullptr) return;      // the caller has written this epoch's gradient into the slot itself
   const bool fold = fate == SLOT_FOLD;
   void* dst = ch->slot[ch->cfg.rank][k % kSlotDepth];
-  const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   constexpr int kUnroll = 4;     // independent 16-byte loads in flight per thread
   const uint64_t stride = nthreads * 8;
   for (uint64_t base = tid * 8; base < ch->count; base += stride * kUnroll) {
@@ -419,8 +544,7 @@ __device__ inline void pack_phase(DevChannel* ch, uint32_t blk, uint32_t nblk, i
     for (int u = 0; u < kUnroll; ++u) {
       const uint64_t i = base + u * stride;
       if (i >= ch->count) break;
-      if (ch->grad_in_bf16) load8(reinterpret_cast<const __nv_bfloat16*>(ch->grad_in), i, v[u]);
-      else load8(reinterpret_cast<const float*>(ch->grad_in), i, v[u]);
+      load_grad8(ch, i, grad_src, v[u]);
     }
     if (fold) {
 #pragma unroll
@@ -440,10 +564,7 @@ __device__ inline void pack_phase(DevChannel* ch, uint32_t blk, uint32_t nblk, i
       if (i >= ch->count) break;
       if (ch->slot_bf16) store8(reinterpret_cast<__nv_bfloat16*>(dst), i, v[u]);
       else store8(reinterpret_cast<float*>(dst), i, v[u]);
-      if (ch->clear_grad) {
-        if (ch->grad_in_bf16) store8(reinterpret_cast<__nv_bfloat16*>(ch->grad_in), i, z);
-        else store8(reinterpret_cast<float*>(ch->grad_in), i, z);
-      }
+      if (ch->clear_grad) clear_grad8(ch, i, grad_src);
     }
   }
 }

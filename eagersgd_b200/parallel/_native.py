@@ -10,6 +10,7 @@ MODE_SOLO, MODE_MAJORITY, MODE_SYNC = 0, 1, 2
 ROLE_ABORT, ROLE_PARTICIPANT, ROLE_DRAIN, ROLE_IDLE = 0, 1, 2, 3
 ROLE_NAMES = {0: "abort", 1: "participant", 2: "drain", 3: "idle"}
 AVG_CONTRIBUTORS, AVG_WORLD, AVG_SUM = 0, 1, 2
+SRC_FLAT, SRC_ACC = 1, 2            # where a step finds its gradient: the flat gradient, fp32 accumulators
 DT_F32, DT_F64, DT_I32, DT_I64 = 0, 1, 2, 3
 
 STATUS_BITS = {
@@ -62,7 +63,14 @@ class ChannelDesc(C.Structure):
                [("out_bf16", C.c_int32), ("pad", C.c_int32), ("hyper", C.c_void_p), ("two_shot_min", C.c_uint64),
                 ("accumulate", C.c_int32), ("adaptive_grace", C.c_int32), ("clear_grad", C.c_int32),
                 ("pad3", C.c_int32), ("mc_slot0", C.c_void_p), ("mc_slot1", C.c_void_p), ("mc_red", C.c_void_p),
-                ("mc_min", C.c_uint64)]
+                ("mc_min", C.c_uint64), ("valid", C.c_uint64), ("keep_out", C.c_int32), ("pad4", C.c_int32),
+                ("outcome", C.c_void_p)]
+
+
+class StepOutcome(C.Structure):
+    """What a channel's newest step did (``esgd::StepOutcome``), in pinned host memory."""
+    _fields_ = [("round", C.c_uint64)] + [(n, C.c_uint32) for n in
+                                          "role contributors is_sync applied status pad".split()]
 
 
 STAT_NAMES = ("local_step", "participated", "absent", "activated", "sync_rounds", "dropped_grads",
@@ -104,7 +112,17 @@ def cuda():
         lib.esgd_dev_channel_bytes.restype = C.c_uint64
         lib.esgd_dev_ctl_bytes.restype = C.c_uint64
         lib.esgd_channel_configure.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
-        lib.esgd_channel_step.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_void_p]
+        lib.esgd_channel_step.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p]
+        lib.esgd_channel_set_grad_acc.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+        lib.esgd_channel_step_local.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p]
+        lib.esgd_collective_create.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p, C.POINTER(C.c_void_p)]
+        lib.esgd_collective_destroy.argtypes = [C.c_void_p]
+        lib.esgd_collective_destroy.restype = None
+        lib.esgd_collective_post.argtypes = [C.c_void_p, C.c_void_p]
+        lib.esgd_collective_test.argtypes = [C.c_void_p]
+        lib.esgd_collective_wait.argtypes = [C.c_void_p, C.c_void_p]
+        lib.esgd_host_alloc.argtypes = [C.c_uint64, C.POINTER(C.c_void_p)]
+        lib.esgd_host_free.argtypes = [C.c_void_p]
         lib.esgd_channel_applied.argtypes = [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]
         lib.esgd_channel_times.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
         lib.esgd_set_hyper.argtypes = [C.c_void_p, C.c_float, C.c_float, C.c_float, C.c_int, C.c_float, C.c_void_p]

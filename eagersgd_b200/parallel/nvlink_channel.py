@@ -162,6 +162,9 @@ class NvlinkChannel:
     then pulls the others' shares); ``two_shot_min=None`` keeps the one-shot form.
     With ``mc_base`` (the multicast address of arenas from ``create_arenas``) rounds in which every rank is
     on time are reduced inside the NVSwitch from ``mc_min`` elements up.
+    ``valid``: elements of ``grad_in`` and ``out`` when they are not ``count`` (which is a multiple of eight);
+    ``keep_out`` leaves ``out`` alone in a step that applies nothing; ``outcome``: address of a ``StepOutcome`` in pinned
+    host memory that every step fills in.
     ``accumulate`` folds a gradient that no round picked up into the rank's next publish of
     the same slot instead of dropping it; ``clear_grad`` zeroes ``grad_in`` behind the copy
     into the publish slot, so the caller needs no separate fill before the next backward.
@@ -176,7 +179,8 @@ class NvlinkChannel:
                  hyper: Optional[torch.Tensor] = None, max_blocks: int = 592,
                  two_shot_min: Optional[int] = TWO_SHOT_MIN, accumulate: bool = False,
                  adaptive_grace: bool = True, clear_grad: bool = False, mc_base: int = 0,
-                 mc_min: int = MULTICAST_MIN):
+                 mc_min: int = MULTICAST_MIN, valid: Optional[int] = None, keep_out: bool = False,
+                 outcome: Optional[int] = None):
         if slot_dtype not in _FLOAT_DTYPES:
             raise ValueError("slot_dtype must be torch.float32 or torch.bfloat16, not %s" % slot_dtype)
         _check_dtype(grad_in, "grad_in")
@@ -187,8 +191,10 @@ class NvlinkChannel:
         _check_dtype(w16, "w16", (torch.bfloat16,))
         _check_dtype(out, "out")
         for name, t in (("w32", w32), ("mom", mom), ("w16", w16), ("out", out)):
-            if t is not None and (t.numel() != count or not t.is_contiguous()):
+            if t is not None and (t.numel() != (valid or count if name == "out" else count) or not t.is_contiguous()):
                 raise ValueError("%s must be a contiguous tensor of %d elements" % (name, count))
+        if valid is not None and (not count - 8 < valid <= count or grad_in is None):
+            raise ValueError("valid must be within eight of count, and needs a gradient tensor of its own")
         self.lib = N.cuda()
         self.count, self.rank, self.world, self.device = count, rank, world, device
         self.max_blocks = max_blocks
@@ -199,7 +205,10 @@ class NvlinkChannel:
             hyper = torch.zeros(HYPER_LEN, dtype=torch.float32, device=device)
             hyper[4] = 1.0
         self.hyper = hyper
-        assert grad_in is None or (grad_in.numel() == count and grad_in.is_contiguous())
+        assert grad_in is None or (grad_in.numel() == (valid or count) and grad_in.is_contiguous())
+        # One rank that publishes to nobody: a step is a single pass over the gradient, straight into the fused update or a
+        # stand-alone collective's result.  (Wrapped optimizers keep the two launches: their own kernels dominate.)
+        self.local = world == 1 and grad_in is not None and (w32 is not None or keep_out)
         self.slot_dtype = slot_dtype
         self._steps = 0
         self._dch = torch.zeros(int(self.lib.esgd_dev_channel_bytes()), dtype=torch.uint8, device=device)
@@ -233,6 +242,7 @@ class NvlinkChannel:
         d.out = out.data_ptr() if out is not None else None
         d.out_bf16 = int(out is not None and out.dtype == torch.bfloat16)
         d.hyper = self.hyper.data_ptr()
+        d.valid, d.keep_out, d.outcome = int(valid or 0), int(keep_out), outcome
         self._desc = d
         stream = torch.cuda.current_stream(device)
         N.check_cuda(self.lib.esgd_channel_configure(self._dch.data_ptr(), C.byref(d), stream.cuda_stream),
@@ -245,10 +255,20 @@ class NvlinkChannel:
     def dev_ptr(self) -> int:
         return self._dch.data_ptr()
 
-    def step(self, stream: Optional[torch.cuda.Stream] = None) -> None:
-        """Enqueue one step on ``stream``: pack + control, then reduce + update."""
+    def set_grad_acc(self, acc: torch.Tensor) -> None:
+        """Give the channel fp32 gradient accumulators beside its bf16 ``grad_in``; a step is told which of the two (or
+        both: their sum) holds this step's gradient, and clears what it read when ``clear_grad`` is set."""
+        _check_dtype(acc, "acc", (torch.float32,))
+        assert acc.numel() == self.count and acc.is_contiguous() and self.grad_in is not None
+        self.grad_acc = acc
+        N.check_cuda(self.lib.esgd_channel_set_grad_acc(self._dch.data_ptr(), acc.data_ptr(),
+                                                        torch.cuda.current_stream(self.device).cuda_stream), "channel set-up")
+
+    def step(self, stream: Optional[torch.cuda.Stream] = None, grad_src: int = N.SRC_FLAT) -> None:
+        """Enqueue one step on ``stream``: pack + control, then reduce + update (one launch when the world is one rank)."""
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
-        N.check_cuda(self.lib.esgd_channel_step(self._dch.data_ptr(), self.count, self.max_blocks, s.cuda_stream),
+        launch = self.lib.esgd_channel_step_local if self.local else self.lib.esgd_channel_step
+        N.check_cuda(launch(self._dch.data_ptr(), self.count, self.max_blocks, grad_src, s.cuda_stream),
                      "partial allreduce launch")
         self._steps += 1
 

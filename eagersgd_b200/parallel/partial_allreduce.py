@@ -20,6 +20,7 @@ programs that want the collective by itself.
 """
 from __future__ import annotations
 
+import ctypes as C
 import threading
 from typing import Callable, Optional
 
@@ -30,6 +31,49 @@ from . import _native as N
 from .group import Group
 
 _ROLES = {N.ROLE_PARTICIPANT: "participant", N.ROLE_DRAIN: "drain"}      # anything else: the rank missed the round
+
+
+class _PinnedOutcome:
+    """A ``StepOutcome`` in pinned host memory: the kernels fill it in, the host reads it once the step's event has passed."""
+
+    def __init__(self):
+        self._ptr = C.c_void_p()
+        N.check_cuda(N.cuda().esgd_host_alloc(C.sizeof(N.StepOutcome), C.byref(self._ptr)), "pinned allocation")
+        self.address = int(self._ptr.value)
+        self.value = N.StepOutcome.from_address(self.address)
+
+    def free(self):
+        if self._ptr:
+            self.value = None
+            N.cuda().esgd_host_free(self._ptr)
+            self._ptr = C.c_void_p()
+
+
+class _Collective:
+    """Post / test / wait of one channel on a side stream, each a single native call."""
+
+    def __init__(self, ch, stream: torch.cuda.Stream):
+        self._lib, self._h, self._ch = N.cuda(), C.c_void_p(), ch
+        N.check_cuda(self._lib.esgd_collective_create(ch.dev_ptr, ch.count, ch.max_blocks, int(ch.local), stream.cuda_stream,
+                                                      C.byref(self._h)), "collective")
+
+    def post(self, stream: int) -> None:
+        N.check_cuda(self._lib.esgd_collective_post(self._h, stream), "partial allreduce launch")
+        self._ch._steps += 1
+
+    def test(self) -> bool:
+        rc = self._lib.esgd_collective_test(self._h)
+        if rc < 0:
+            N.check_cuda(-rc, "partial allreduce")
+        return rc == 1
+
+    def wait(self, stream: int) -> None:
+        N.check_cuda(self._lib.esgd_collective_wait(self._h, stream), "partial allreduce")
+
+    def close(self) -> None:
+        if self._h:
+            self._lib.esgd_collective_destroy(self._h)
+            self._h = C.c_void_p()
 
 
 class PartialAllreduce:
@@ -64,15 +108,20 @@ class PartialAllreduce:
             if tensor.dtype not in (torch.float32, torch.bfloat16):
                 raise ValueError("GPU tensors must be float32 or bfloat16")
             dev = tensor.device
-            self._grad = tensor.view(-1) if n == self.count else torch.zeros(self.count, dtype=tensor.dtype, device=dev)
-            self._res = (self.out.view(-1) if n == self.count else torch.zeros(self.count, dtype=torch.float32, device=dev))
-            if self._res.dtype != torch.float32:           # the kernels write fp32 averages (or bf16 working copies)
-                self._res = torch.zeros(self.count, dtype=torch.float32, device=dev)
+            # The kernels read and write the caller's tensors directly, ragged lengths included; a tensor that does not
+            # start on 16 bytes, or a result in another type than theirs, goes through a staging buffer.
+            direct_in = tensor.data_ptr() % 16 == 0
+            direct_out = self.out.data_ptr() % 16 == 0 and self.out.dtype in (torch.float32, torch.bfloat16)
+            self._grad = tensor.detach().view(-1) if direct_in else torch.zeros(n, dtype=tensor.dtype, device=dev)
+            self._res = self.out.detach().view(-1) if direct_out else torch.zeros(n, dtype=torch.float32, device=dev)
+            self._direct_out = direct_out
             self._arena, bases = create_arenas(self.count, tensor.dtype, g.rank, g.world, g.exchange)
             self._stream = torch.cuda.Stream(device=dev)
-            self._done = torch.cuda.Event()
+            self._outcome = _PinnedOutcome()
             self._ch = NvlinkChannel(self.count, g.rank, g.world, bases, dev, self._grad, slot_dtype=tensor.dtype,
-                                     out=self._res, grace_us=self.grace_us, mc_base=self._arena.mc_base, **self._kw)
+                                     out=self._res, grace_us=self.grace_us, mc_base=self._arena.mc_base, valid=n,
+                                     keep_out=True, outcome=self._outcome.address, **self._kw)
+            self._col = _Collective(self._ch, self._stream)
         else:
             from .cpu_channel import CpuChannel, LocalSegments, SharedSegments
             npdt = {torch.float32: np.float32, torch.float64: np.float64, torch.int32: np.int32,
@@ -101,12 +150,9 @@ class PartialAllreduce:
         if self._posted:
             raise RuntimeError("the previous post has not been waited for")
         if self.on_gpu:
-            cur = torch.cuda.current_stream(self.tensor.device)
             if self._grad.data_ptr() != self.tensor.data_ptr():
-                self._grad[:self.tensor.numel()].copy_(self.tensor.view(-1))
-            self._stream.wait_stream(cur)
-            self._ch.step(self._stream)
-            self._done.record(self._stream)
+                self._grad.copy_(self.tensor.view(-1))
+            self._col.post(torch.cuda.current_stream(self.tensor.device).cuda_stream)
         else:
             src = self.tensor.detach().view(-1).numpy().copy()
 
@@ -124,7 +170,7 @@ class PartialAllreduce:
         """Has the posted round completed?  Completes it (like ``wait``) when it has."""
         if not self._posted:
             return True
-        done = self._done.query() if self.on_gpu else not self._thread.is_alive()
+        done = self._col.test() if self.on_gpu else not self._thread.is_alive()
         if done:
             self.wait()
         return done
@@ -135,19 +181,15 @@ class PartialAllreduce:
         if not self._posted:
             return self._last
         if self.on_gpu:
-            torch.cuda.current_stream(self.tensor.device).wait_stream(self._stream)
-            self._done.synchronize()
-            self._ch.check("partial allreduce")
-            n = self.tensor.numel()
-            if self._ch.applied():
-                if self._res.data_ptr() != self.out.data_ptr():
-                    self.out.view(-1).copy_(self._res[:n])
-            tr = self._ch.trace()
-            last = tr[-1] if tr else {}
-            role = last.get("role")
-            info = {"role": role if role in ("participant", "drain") else "absent", "round": last.get("round"),
-                    "contributors": bin(int(last.get("contrib_mask", 0))).count("1"), "sync": bool(last.get("is_sync", 0)),
-                    "applied": self._ch.applied()}
+            self._col.wait(torch.cuda.current_stream(self.tensor.device).cuda_stream)
+            o = self._outcome.value
+            if o.status:
+                raise N.ChannelError(o.status, "partial allreduce")
+            applied = bool(o.applied)
+            if applied and not self._direct_out:
+                self.out.view(-1).copy_(self._res)
+            info = {"role": _ROLES.get(o.role, "absent"), "round": int(o.round), "contributors": int(o.contributors),
+                    "sync": bool(o.is_sync), "applied": applied}
         else:
             self._thread.join()
             self._thread = None
@@ -174,8 +216,8 @@ class PartialAllreduce:
         if self.on_gpu:
             self._ch.flush(self._stream)
             self._stream.synchronize()
-            if self._ch.applied() and self._res.data_ptr() != self.out.data_ptr():
-                self.out.view(-1).copy_(self._res[:self.tensor.numel()])
+            if self._ch.applied() and not self._direct_out:
+                self.out.view(-1).copy_(self._res)
         else:
             out, i = self._ch.flush(self._np_out)
             if i.role in (N.ROLE_PARTICIPANT, N.ROLE_DRAIN):
@@ -213,6 +255,8 @@ class PartialAllreduce:
         self.group.barrier()                                 # nobody frees memory a peer may still read
         if self.on_gpu:
             torch.cuda.synchronize(self.tensor.device)
+            self._col.close()
+            self._outcome.free()
             self._arena.free()
         else:
             self._seg.close()
