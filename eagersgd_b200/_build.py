@@ -1,11 +1,13 @@
 """In-tree native builds.
 
-Two shared libraries are produced under ``eagersgd_b200/_lib``:
+Three shared libraries are produced under ``eagersgd_b200/_lib``:
 
 * ``libesgd_host.so``  — C++ control plane and CPU backend (g++), no CUDA needed;
 * ``libesgd_cuda.so``  — every CUDA kernel, compiled for sm_100a only (nvcc).
 
-Both export plain ``extern "C"`` launchers taking raw pointers and a stream, so
+* ``_esgd_torch.so``   — the autograd operators over those kernels (g++ against PyTorch's headers), a Python module.
+
+The first two export plain ``extern "C"`` launchers taking raw pointers and a stream, so
 they are loaded with ``ctypes`` and rebuilt in seconds.  The arch is pinned
 (the reference probes the local GPU instead:
 deep500/lv0/operators/tools/get_cuda_arch.cpp:8-33).
@@ -24,6 +26,7 @@ CSRC = os.path.join(_ROOT, "csrc")
 LIBDIR = os.path.join(_ROOT, "_lib")
 HOST_LIB = os.path.join(LIBDIR, "libesgd_host.so")
 CUDA_LIB = os.path.join(LIBDIR, "libesgd_cuda.so")
+TORCH_LIB = os.path.join(LIBDIR, "_esgd_torch.so")
 
 CUDA_ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 _lock = threading.Lock()
@@ -165,9 +168,49 @@ def _build_cuda_locked(srcs, force, verbose, jobs):
     return CUDA_LIB
 
 
+def _torch_stamp(srcs):
+    import torch
+    return _digest(srcs) + " torch " + torch.__version__
+
+
+def build_torch(force: bool = False, verbose: bool = False) -> str:
+    """The autograd operators: C++ against PyTorch's headers, linked to the kernel library beside it."""
+    srcs = _sources("torch", [".cpp"])
+
+    def stale():
+        return not os.path.exists(TORCH_LIB) or not os.path.exists(TORCH_LIB + ".sha") or \
+            open(TORCH_LIB + ".sha").read().strip() != _torch_stamp(srcs)
+
+    if not force and not stale():
+        return TORCH_LIB
+    build_cuda(verbose=verbose)
+    with _FileLock(os.path.join(LIBDIR, ".build.lock")):
+        if not force and not stale():
+            return TORCH_LIB
+        import sysconfig
+
+        from torch.utils import cpp_extension as ext
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-pthread", "-DTORCH_EXTENSION_NAME=_esgd_torch", "-I", CSRC,
+               "-I", sysconfig.get_paths()["include"]]
+        for d in ext.include_paths("cuda"):
+            cmd += ["-isystem", d]
+        for d in ext.library_paths("cuda"):
+            cmd += ["-L", d]
+        cmd += srcs + ["-o", TORCH_LIB + ".tmp", "-L", LIBDIR, "-lesgd_cuda", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
+                       "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+        if verbose:
+            print(" ".join(cmd))
+        subprocess.run(cmd, check=True)
+        os.replace(TORCH_LIB + ".tmp", TORCH_LIB)
+        with open(TORCH_LIB + ".sha", "w") as f:
+            f.write(_torch_stamp(srcs))
+    return TORCH_LIB
+
+
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_host(force, verbose)
     build_cuda(force, verbose)
+    build_torch(force, verbose)
 
 
 def load_host() -> ctypes.CDLL:
@@ -187,6 +230,23 @@ def load_cuda() -> ctypes.CDLL:
                 path = build_cuda()
             _cache["cuda"] = ctypes.CDLL(path, mode=ctypes.RTLD_GLOBAL)
         return _cache["cuda"]
+
+
+def load_torch():
+    """The module of autograd operators.  Fails loudly, like the kernel library it sits on."""
+    load_cuda()
+    with _lock:
+        if "torch" not in _cache:
+            import importlib.machinery
+            import importlib.util
+
+            import torch  # noqa: F401  (its libraries must be in the process first)
+            spec = importlib.util.spec_from_file_location(
+                "_esgd_torch", build_torch(), loader=importlib.machinery.ExtensionFileLoader("_esgd_torch", TORCH_LIB))
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            _cache["torch"] = mod
+        return _cache["torch"]
 
 
 def write_pkgconfig() -> str:

@@ -1,8 +1,8 @@
 // Fused batch-norm kernels for NHWC bf16 activations viewed as [M = N*H*W, C].
 //
 //   bn_stats        : per-channel sum / sum of squares (fp32) of a conv output
-//   bn_finalize     : mean / inv-std, scale / shift, running-statistics update
-//   bn_apply        : z = act(scale*y + shift [+ residual])           (one read, one write)
+//   bn_fwd          : mean / inv-std, scale / shift, running-statistics update and
+//                     z = act(scale*y + shift [+ residual])           (one read, one write)
 //   bn_bwd_reduce   : g = dz * [z > 0];  dbeta = sum g, dgamma = sum g*xhat
 //   bn_bwd_apply    : dy = gamma*invstd*(g - dbeta/M - xhat*dgamma/M), optional dres = g
 //
@@ -89,56 +89,56 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const __nv_bfloat16* __re
   }
 }
 
-// One thread per channel.  Writes mean, invstd, scale = gamma*invstd, shift = beta - mean*scale.
-__global__ void bn_finalize_kernel(const float* sum, const float* sqsum, const float* gamma, const float* beta,
-                                   float* running_mean, float* running_var, float* mean_out, float* invstd_out,
-                                   float* scale, float* shift, int C, float inv_count, float unbias, float momentum,
-                                   float eps) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float mean = sum[c] * inv_count;
-  float var = fmaxf(sqsum[c] * inv_count - mean * mean, 0.0f);
-  float invstd = rsqrtf(var + eps);
-  mean_out[c] = mean;
-  invstd_out[c] = invstd;
-  float sc = gamma[c] * invstd;
-  scale[c] = sc;
-  shift[c] = beta[c] - mean * sc;
-  if (running_mean != nullptr) {
-    running_mean[c] = (1.0f - momentum) * running_mean[c] + momentum * mean;
-    running_var[c] = (1.0f - momentum) * running_var[c] + momentum * var * unbias;
-  }
-}
-
-// Threads keep a fixed group of 8 channels and walk over rows, so the per-channel
-// coefficients live in registers for the whole kernel.
+// z = act(scale * y + shift [+ residual]) with scale / shift from the batch sums.  Every thread derives the coefficients
+// of its own 8 channels (32 loads and 8 reciprocal roots against thousands of elements: a launch of its own for
+// them cost 4 us a layer); the first block also leaves them, and the running statistics, for later.  Threads keep a
+// fixed group of 8 channels and walk over rows, last row first: the producer of y wrote its end last, so that part
+// is still in L2, and what is left there afterwards is z's beginning, where the next layer starts.
 template <int kMinBlocks>
-__global__ void __launch_bounds__(256, kMinBlocks) bn_apply_kernel(const __nv_bfloat16* __restrict__ y,
-                                                       const __nv_bfloat16* __restrict__ res,
-                                                       __nv_bfloat16* __restrict__ z, const float* __restrict__ scale,
-                                                       const float* __restrict__ shift, int64_t M, int C, int relu) {
+__global__ void __launch_bounds__(256, kMinBlocks)
+bn_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ z,
+              const float* __restrict__ sum, const float* __restrict__ sqsum, const float* __restrict__ gamma,
+              const float* __restrict__ beta, float* running_mean, float* running_var, float* __restrict__ aux, int64_t M,
+              int C, int relu, float inv_count, float unbias, float momentum, float eps) {
   const Map mp = make_map(C);
   const int gl = threadIdx.x % mp.g_per_blk, rl = threadIdx.x / mp.g_per_blk;
   if (rl >= mp.rows_par) return;
   for (int g = gl; g < mp.groups; g += mp.g_per_blk) {
     float sc[8], sh[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) { sc[q] = scale[g * 8 + q]; sh[q] = shift[g * 8 + q]; }
+    for (int q = 0; q < 8; ++q) {
+      const int c = g * 8 + q;
+      const float mean = sum[c] * inv_count;
+      const float var = fmaxf(sqsum[c] * inv_count - mean * mean, 0.0f);
+      const float invstd = rsqrtf(var + eps);
+      sc[q] = gamma[c] * invstd;
+      sh[q] = beta[c] - mean * sc[q];
+      if (blockIdx.x == 0 && rl == 0) {
+        aux[c] = mean;
+        aux[C + c] = invstd;
+        aux[2 * C + c] = sc[q];
+        aux[3 * C + c] = sh[q];
+        if (running_mean != nullptr) {
+          running_mean[c] = (1.0f - momentum) * running_mean[c] + momentum * mean;
+          running_var[c] = (1.0f - momentum) * running_var[c] + momentum * var * unbias;
+        }
+      }
+    }
     const int64_t step = (int64_t)gridDim.x * mp.rows_par;
-    for (int64_t r = (int64_t)blockIdx.x * mp.rows_par + rl; r < M; r += 4 * step) {
+    for (int64_t r = M - 1 - ((int64_t)blockIdx.x * mp.rows_par + rl); r >= 0; r -= 4 * step) {
       uint4 ry[4], rr_[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int64_t rr = r + u * step;
-        if (rr < M) {
+        const int64_t rr = r - u * step;
+        if (rr >= 0) {
           ry[u] = *reinterpret_cast<const uint4*>(y + rr * C + g * 8);
           if (res != nullptr) rr_[u] = *reinterpret_cast<const uint4*>(res + rr * C + g * 8);
         }
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int64_t rr = r + u * step;
-        if (rr < M) {
+        const int64_t rr = r - u * step;
+        if (rr >= 0) {
           const __nv_bfloat162* hy = reinterpret_cast<const __nv_bfloat162*>(&ry[u]);
           const __nv_bfloat162* hr = reinterpret_cast<const __nv_bfloat162*>(&rr_[u]);
           float v[8];
@@ -182,13 +182,14 @@ bn_bwd_reduce_kernel(const __nv_bfloat16* __restrict__ dz, const __nv_bfloat16* 
         fsh[q] = relu == 2 ? fshift[g * 8 + q] : 0.0f;
       }
       const int64_t step = (int64_t)gridDim.x * mp.rows_par;
-      // sum g and g*(y - mean); the 1/std factor is applied once at the end.  Four rows in flight.
-      for (int64_t r = (int64_t)blockIdx.x * mp.rows_par + rl; r < M; r += 4 * step) {
+      // sum g and g*(y - mean); the 1/std factor is applied once at the end.  Four rows in flight, last rows first
+      // (dz was produced front to back); the apply pass then goes front to back over what this one read last.
+      for (int64_t r = M - 1 - ((int64_t)blockIdx.x * mp.rows_par + rl); r >= 0; r -= 4 * step) {
         uint4 rd[4], ry[4], rz[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int64_t rr = r + u * step;
-          if (rr < M) {
+          const int64_t rr = r - u * step;
+          if (rr >= 0) {
             const int64_t off = rr * C + g * 8;
             rd[u] = *reinterpret_cast<const uint4*>(dz + off);
             ry[u] = *reinterpret_cast<const uint4*>(y + off);
@@ -197,7 +198,7 @@ bn_bwd_reduce_kernel(const __nv_bfloat16* __restrict__ dz, const __nv_bfloat16* 
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          if (r + u * step < M) {
+          if (r - u * step >= 0) {
             const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&rd[u]);
             const __nv_bfloat162* hy = reinterpret_cast<const __nv_bfloat162*>(&ry[u]);
             const __nv_bfloat162* hz = reinterpret_cast<const __nv_bfloat162*>(&rz[u]);
@@ -249,9 +250,15 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dz, const __nv_bfloat16* _
                     const float* __restrict__ dbeta, const float* __restrict__ dgamma,
                     const float* __restrict__ fscale, const float* __restrict__ fshift,
                     __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dres, int64_t M, int C, int relu,
-                    float inv_count) {
+                    float inv_count, float* acc_dgamma, float* acc_dbeta) {
   const Map mp = make_map(C);
   const int gl = threadIdx.x % mp.g_per_blk, rl = threadIdx.x / mp.g_per_blk;
+  if (blockIdx.x == 0) {       // the parameters' own gradient accumulators, when the caller gives them
+    for (int c = threadIdx.x; c < C; c += blockDim.x) {
+      if (acc_dgamma != nullptr) acc_dgamma[c] += dgamma[c];
+      if (acc_dbeta != nullptr) acc_dbeta[c] += dbeta[c];
+    }
+  }
   if (rl >= mp.rows_par) return;
   for (int g = gl; g < mp.groups; g += mp.g_per_blk) {
     float ca[8], cb[8], cc[8], fsc[8], fsh[8];
@@ -344,29 +351,22 @@ int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, voi
   return (int)cudaGetLastError();
 }
 
-int esgd_bn_finalize(const float* sum, const float* sqsum, const float* gamma, const float* beta,
-                     float* running_mean, float* running_var, float* mean, float* invstd, float* scale,
-                     float* shift, int C, int64_t count, float momentum, float eps, void* stream) {
-  float unbias = count > 1 ? (float)count / (float)(count - 1) : 1.0f;
-  bn_finalize_kernel<<<(C + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-      sum, sqsum, gamma, beta, running_mean, running_var, mean, invstd, scale, shift, C, 1.0f / (float)count,
-      unbias, momentum, eps);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
-}
-
-int esgd_bn_apply(const void* y, const void* residual, void* z, const float* scale, const float* shift, int64_t M,
-                  int C, int relu, void* stream) {
+// sum / sqsum: the batch sums of y.  aux [4][C] receives mean, inverse standard deviation, scale and shift.
+int esgd_bn_fwd(const void* y, const void* residual, void* z, const float* sum, const float* sqsum, const float* gamma,
+                const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu,
+                float momentum, float eps, void* stream) {
   if (C % 8) return -1;
+  const float unbias = M > 1 ? (float)M / (float)(M - 1) : 1.0f;
   int g = C / 8 < 256 ? C / 8 : 256;
   int rows_par = 256 / g;
-#define ESGD_BN_APPLY(MB)                                                                          \
-  bn_apply_kernel<MB><<<blocks_for(M, rows_par * 8), 256, 0, (cudaStream_t)stream>>>(             \
-      (const __nv_bfloat16*)y, (const __nv_bfloat16*)residual, (__nv_bfloat16*)z, scale, shift, M, C, relu)
+#define ESGD_BN_FWD(MB)                                                                                            \
+  bn_fwd_kernel<MB><<<blocks_for(M, rows_par * 8), 256, 0, (cudaStream_t)stream>>>(                               \
+      (const __nv_bfloat16*)y, (const __nv_bfloat16*)residual, (__nv_bfloat16*)z, sum, sqsum, gamma, beta,        \
+      running_mean, running_var, aux, M, C, relu, 1.0f / (float)M, unbias, momentum, eps)
   switch (occupancy_choice(0)) {
-    case 3: ESGD_BN_APPLY(3); break;
-    case 4: ESGD_BN_APPLY(4); break;
-    default: ESGD_BN_APPLY(2); break;
+    case 3: ESGD_BN_FWD(3); break;
+    case 4: ESGD_BN_FWD(4); break;
+    default: ESGD_BN_FWD(2); break;
   }
   esgd::count_launch();
   return (int)cudaGetLastError();
@@ -393,16 +393,19 @@ int esgd_bn_bwd_reduce(const void* dz, const void* z, const void* y, const float
   return (int)cudaGetLastError();
 }
 
+// acc_dgamma / acc_dbeta (optional): fp32 accumulators the two parameter gradients are added to.
 int esgd_bn_bwd_apply(const void* dz, const void* z, const void* y, const float* mean, const float* invstd,
                       const float* gamma, const float* dbeta, const float* dgamma, const float* fscale,
-                      const float* fshift, void* dy, void* dres, int64_t M, int C, int relu, void* stream) {
+                      const float* fshift, void* dy, void* dres, int64_t M, int C, int relu, float* acc_dgamma,
+                      float* acc_dbeta, void* stream) {
   if (C % 8) return -1;
   int g = C / 8 < 256 ? C / 8 : 256;
   int rows_par = 256 / g;
 #define ESGD_BN_BWD_APPLY(MB)                                                                              \
   bn_bwd_apply_kernel<MB><<<blocks_for(M, rows_par * 8), 256, 0, (cudaStream_t)stream>>>(                   \
       (const __nv_bfloat16*)dz, (const __nv_bfloat16*)z, (const __nv_bfloat16*)y, mean, invstd, gamma, dbeta, \
-      dgamma, fscale, fshift, (__nv_bfloat16*)dy, (__nv_bfloat16*)dres, M, C, relu, 1.0f / (float)M)
+      dgamma, fscale, fshift, (__nv_bfloat16*)dy, (__nv_bfloat16*)dres, M, C, relu, 1.0f / (float)M, \
+      acc_dgamma, acc_dbeta)
   switch (occupancy_choice(2)) {
     case 3: ESGD_BN_BWD_APPLY(3); break;
     case 4: ESGD_BN_BWD_APPLY(4); break;

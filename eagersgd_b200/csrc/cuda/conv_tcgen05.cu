@@ -28,14 +28,36 @@ using namespace umma;
 
 namespace {
 
-template <int BN_>
+// The filter bank of a problem, read by TMA as stored ([K][R][S][C], channels_last).  Forward: the rows of a k-block's
+// B tile are output channels and its 64 columns the input channels of one tap (K-major).  Data gradient
+// (kTransposed): rows are the 64 reduced output channels, columns the input channels (MN-major), and the taps of
+// the problem are taps (r0 + r * dr, s0 + s * ds) of the stored filter -- rotated by 180 degrees, or the subset that
+// meets one output parity of a strided convolution -- so that no rotated copy of the weights is ever made.
+// Channel counts that are no multiple of 64 are zero-filled by TMA on both operands.
+struct FilterTaps { int r0, dr, s0, ds; };
+
+template <int BN, bool kTransposed>
+__device__ __forceinline__ void load_filter_tap(const CUtensorMap* tm, const FilterTaps& f, int r, int s, int cb, int n0,
+                                                uint8_t* b, uint64_t* bar) {
+  const int rw = f.r0 + r * f.dr, sw = f.s0 + s * f.ds;
+  if (kTransposed) {
+#pragma unroll
+    for (int i = 0; i < BN / 64; ++i) tma_load_4d(b + i * 8192, tm, bar, n0 + 64 * i, sw, rw, cb * 64);
+  } else {
+    tma_load_4d(b, tm, bar, cb * 64, sw, rw, n0);
+  }
+}
+
+template <int BN_, bool kT>
 struct ConvProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = false, kZeroStages = false, kHalo = false;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false;
   CUtensorMap tmX, tmW, tmY;
   int N, Ho, Wo, Cout;
   int R, S, stride, pad;
-  int cblks;                 // Cin / 64
+  FilterTaps taps;
+  int cblks;                 // 64-channel blocks of the reduction
+  int ksteps, n_mma;         // 16-channel steps of a block that hold anything; columns the MMA computes
   int BW, BH, BI;            // output-pixel box of a tile (BW*BH*BI <= 128)
   int w_tiles, h_tiles, i_tiles, n_tiles;
   int fixed_n;
@@ -70,7 +92,9 @@ struct ConvProblem {
     tma_load_4d(a, &tmX, bar, cb * 64, t.w0 * stride + s - pad, t.h0 * stride + r - pad, t.i0);
   }
   __device__ __forceinline__ void load_b(const Tile& t, int kb, uint8_t* b, uint64_t* bar) const {
-    tma_load_2d(b, &tmW, bar, kb * 64, t.n0);
+    const int tap = kb / cblks, cb = kb - tap * cblks;
+    const int r = tap / S, s = tap - r * S;
+    load_filter_tap<BN, kT>(&tmW, taps, r, s, cb, t.n0, b, bar);
   }
   __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint64_t* bar) const {
     load_a(t, kb, a, bar);
@@ -95,14 +119,16 @@ struct ConvProblem {
 // pipeline).  A tile is BH full output rows of one image; GEMM row m stands for the pixel (m / PW, m % PW) of
 // the box pitch PW = Wo + S - 1, so the S - 1 margin columns of every row (and the rows past BH * PW) compute
 // values that are dropped: out_row() gives a GEMM row its place in the dense [BH][Wo] tile that is stored.
-template <int BN_>
+template <int BN_, bool kT>
 struct ConvHaloProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = false, kZeroStages = false, kHalo = true;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true;
   CUtensorMap tmX, tmW, tmY;
   int N, Ho, Wo, Cout;
   int R, S, pad;
-  int cblks;                 // Cin / 64
+  FilterTaps taps;
+  int cblks;                 // 64-channel blocks of the reduction
+  int ksteps, n_mma;
   int BH, PW;                // output rows per tile, pixel pitch of the input box
   int h_tiles, n_tiles;
   int res_kb;                // > 0: the filter bank of the CTA's channel range is resident
@@ -124,7 +150,9 @@ struct ConvHaloProblem {
     tma_load_4d(smem, &tmX, bar, cb * 64, -pad, t.h0 - pad, t.i0);
   }
   __device__ __forceinline__ void load_b(const Tile& t, int kb, uint8_t* b, uint64_t* bar) const {
-    tma_load_2d(b, &tmW, bar, kb * 64, t.n0);
+    const int tap = kb / cblks, cb = kb - tap * cblks;
+    const int r = tap / S, s = tap - r * S;
+    load_filter_tap<BN, kT>(&tmW, taps, r, s, cb, t.n0, b, bar);
   }
   __device__ __forceinline__ void load_a(const Tile&, int, uint8_t*, uint64_t*) const {}
   __device__ __forceinline__ void load(const Tile&, int, uint8_t*, uint8_t*, uint64_t*) const {}
@@ -159,6 +187,8 @@ struct ConvWgradProblem {
   int m_tiles, n_tiles, splits, boxes_total, boxes_per_split;
   float* dw;   // [Cout][R*S][Cin]
   static constexpr int res_kb = 0;   // both operands change with every k-block
+  static constexpr int ksteps = BK / 16;
+  int n_mma;
 
   struct Tile { int kb0, kb1, n0, m0, tap; };
 
@@ -234,11 +264,26 @@ struct ConvArgs {
   int N, H, W, Cin, Cout, R, S, stride, pad;
   int out_h = 0, out_w = 0;                 // output extent override (0: from the usual formula)
   int64_t ys_w = 0, ys_h = 0, ys_n = 0;     // output strides in elements (0: dense NHWC)
+  FilterTaps taps = {0, 1, 0, 1};           // taps of the stored filter that the problem uses
+  int fR = 0, fS = 0;                       // extent of the stored filter
 };
 
-template <int BN>
+// Tensor map over the stored filter bank [K][fR][fS][C]; forward: K = a.Cout, C = a.Cin, data gradient the other way.
+template <int BN, bool kT>
+int filter_map(CUtensorMap* tm, const ConvArgs& a) {
+  const int C = kT ? a.Cout : a.Cin, K = kT ? a.Cin : a.Cout;
+  uint64_t dims[4] = {(uint64_t)C, (uint64_t)a.fS, (uint64_t)a.fR, (uint64_t)K};
+  uint64_t strides[3] = {(uint64_t)C * 2, (uint64_t)a.fS * C * 2, (uint64_t)a.fR * a.fS * C * 2};
+  uint32_t box[4] = {64, 1, 1, kT ? 64u : (uint32_t)BN};
+  return esgd::make_tensormap_bf16(tm, a.w, 4, dims, strides, box, nullptr);
+}
+inline int ksteps_of(int c) { return c >= 64 ? BK / 16 : (c + 15) / 16; }
+// narrow layers: the MMA computes no more columns than there are (the epilogue drops the rest either way)
+inline int mma_columns(int n, int bn) { return n >= bn ? bn : (n + 15) / 16 * 16; }
+
+template <int BN, bool kT>
 int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
-  using P = ConvProblem<BN>;
+  using P = ConvProblem<BN, kT>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(conv_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -250,7 +295,10 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
   p.N = a.N; p.Cout = a.Cout; p.R = a.R; p.S = a.S; p.stride = a.stride; p.pad = a.pad;
   p.Ho = a.out_h ? a.out_h : (a.H + 2 * a.pad - a.R) / a.stride + 1;
   p.Wo = a.out_w ? a.out_w : (a.W + 2 * a.pad - a.S) / a.stride + 1;
-  p.cblks = a.Cin / 64;
+  p.cblks = (a.Cin + 63) / 64;
+  p.ksteps = ksteps_of(a.Cin);
+  p.n_mma = mma_columns(a.Cout, BN);
+  p.taps = a.taps;
   // output-pixel box: whole rows when they fit, as many rows / images as 128 GEMM rows allow
   if (p.Wo >= 128) { p.BW = 128; p.BH = 1; p.BI = 1; }
   else {
@@ -276,10 +324,7 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
     if (r != 0) return 1000 + r;
   }
   {
-    uint64_t dims[2] = {(uint64_t)a.R * a.S * a.Cin, (uint64_t)a.Cout};
-    uint64_t strides[1] = {(uint64_t)a.R * a.S * a.Cin * 2};
-    uint32_t box[2] = {64, (uint32_t)BN};
-    int r = esgd::make_tensormap_bf16(&p.tmW, a.w, 2, dims, strides, box, nullptr);
+    int r = filter_map<BN, kT>(&p.tmW, a);
     if (r != 0) return 2000 + r;
   }
   {
@@ -332,9 +377,9 @@ bool halo_applicable(const ConvArgs& a, int Ho, int Wo, int* bh_out) {
   return true;
 }
 
-template <int BN>
+template <int BN, bool kT>
 int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
-  using P = ConvHaloProblem<BN>;
+  using P = ConvHaloProblem<BN, kT>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(conv_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -346,7 +391,10 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
   p.N = a.N; p.Cout = a.Cout; p.R = a.R; p.S = a.S; p.pad = a.pad;
   p.Ho = a.H + 2 * a.pad - a.R + 1;
   p.Wo = a.W + 2 * a.pad - a.S + 1;
-  p.cblks = a.Cin / 64;
+  p.cblks = (a.Cin + 63) / 64;
+  p.ksteps = ksteps_of(a.Cin);
+  p.n_mma = mma_columns(a.Cout, BN);
+  p.taps = a.taps;
   p.BH = bh;
   p.PW = p.Wo + a.S - 1;
   p.h_tiles = p.Ho / bh;
@@ -359,10 +407,7 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
     if (r != 0) return 1000 + r;
   }
   {
-    uint64_t dims[2] = {(uint64_t)a.R * a.S * a.Cin, (uint64_t)a.Cout};
-    uint64_t strides[1] = {(uint64_t)a.R * a.S * a.Cin * 2};
-    uint32_t box[2] = {64, (uint32_t)BN};
-    int r = esgd::make_tensormap_bf16(&p.tmW, a.w, 2, dims, strides, box, nullptr);
+    int r = filter_map<BN, kT>(&p.tmW, a);
     if (r != 0) return 2000 + r;
   }
   {
@@ -414,6 +459,7 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
   p.h_tiles = (p.Ho + p.BH - 1) / p.BH;
   p.i_tiles = a.N;
   p.boxes_total = p.w_tiles * p.h_tiles * p.i_tiles;
+  p.n_mma = mma_columns(a.Cin, BN);
   p.m_tiles = (a.Cout + BM - 1) / BM;
   p.n_tiles = (a.Cin + BN - 1) / BN;
   const int sms = sm_count();
@@ -443,7 +489,7 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
     if (r != 0) return 2000 + r;
   }
   Epilogue ep;
-  ep.out_mode = OUT_F32_ATOMIC; ep.relu = 0; ep.n_total = a.Cin; ep.bias = nullptr;
+  ep.out_mode = OUT_F32_ATOMIC; ep.relu = 0; ep.n_total = a.Cin; ep.bias = nullptr; ep.bias_bf16 = 0;
   ep.col_sum = nullptr; ep.col_sqsum = nullptr; ep.error_flag = error_flag;
   ep.tx_bytes = (uint32_t)(p.BW * p.BH * 128 * (BM / 64 + BN / 64));
   ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
@@ -452,6 +498,25 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
   conv_wgrad_kernel<P><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(p, ep);
   esgd::count_launch();
   return (int)cudaGetLastError();
+}
+
+Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* error_flag) {
+  Epilogue ep;
+  ep.out_mode = OUT_BF16; ep.relu = relu; ep.n_total = n; ep.bias = nullptr; ep.bias_bf16 = 0;
+  ep.col_sum = col_sum; ep.col_sqsum = col_sqsum; ep.error_flag = error_flag;
+  ep.tx_bytes = 0; ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
+  return ep;
+}
+
+template <bool kT>
+int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
+  const int BN = a.Cout <= 64 ? 64 : (a.Cout <= 128 ? 128 : 256);
+  int bh = 0;
+  if (BN <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
+    return BN == 64 ? launch_halo<64, kT>(a, ep, bh, s) : launch_halo<128, kT>(a, ep, bh, s);
+  if (BN == 64) return launch<64, kT>(a, ep, s);
+  if (BN == 128) return launch<128, kT>(a, ep, s);
+  return launch<256, kT>(a, ep, s);
 }
 
 }  // namespace
@@ -471,39 +536,44 @@ int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, in
   return launch_wgrad<256>(a, dy, dw, error_flag, s);
 }
 
-// x: [N,H,W,Cin] bf16, w: [Cout,R,S,Cin] bf16, y: [N,Ho,Wo,Cout] bf16.  Cin % 64 == 0, Cout % 8 == 0.
+// x: [N,H,W,Cin] bf16, w: [Cout,R,S,Cin] bf16, y: [N,Ho,Wo,Cout] bf16.  Cin % 8 == 0, Cout % 8 == 0.
 // col_sum / col_sqsum (optional, caller-zeroed fp32[Cout]) receive the statistics of the stored y.
-// out_h / out_w override the output extent (taps that fall outside the input read zeros); ys_w / ys_h / ys_n
-// (elements, 0 = dense) let y be a strided view, e.g. every second pixel of a larger tensor.
-int esgd_conv2d_fwd_ex(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S,
-                       int stride, int pad, int out_h, int out_w, int64_t ys_w, int64_t ys_h, int64_t ys_n, int relu,
-                       float* col_sum, float* col_sqsum, int* error_flag, void* stream);
-
 int esgd_conv2d_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S,
                     int stride, int pad, int relu, float* col_sum, float* col_sqsum, int* error_flag, void* stream) {
-  return esgd_conv2d_fwd_ex(x, w, y, N, H, W, Cin, Cout, R, S, stride, pad, 0, 0, 0, 0, 0, relu, col_sum, col_sqsum,
-                            error_flag, stream);
+  if (Cin % 8 || Cout % 8 || stride < 1 || stride > 2) return -1;
+  ConvArgs a{x, w, y, N, H, W, Cin, Cout, R, S, stride, pad};
+  a.fR = R; a.fS = S;
+  return dispatch<false>(a, epilogue_for(Cout, relu, col_sum, col_sqsum, error_flag), (cudaStream_t)stream);
 }
 
-int esgd_conv2d_fwd_ex(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S,
-                       int stride, int pad, int out_h, int out_w, int64_t ys_w, int64_t ys_h, int64_t ys_n, int relu,
-                       float* col_sum, float* col_sqsum, int* error_flag, void* stream) {
-  if (Cin % 64 || Cout % 8 || stride < 1 || stride > 2) return -1;
-  if (ys_w && ((ys_w % 8) || (ys_h % 8) || (ys_n % 8))) return -6;
-  ConvArgs a{x, w, y, N, H, W, Cin, Cout, R, S, stride, pad};
-  a.out_h = out_h; a.out_w = out_w; a.ys_w = ys_w; a.ys_h = ys_h; a.ys_n = ys_n;
-  Epilogue ep;
-  ep.out_mode = OUT_BF16; ep.relu = relu; ep.n_total = Cout; ep.bias = nullptr;
-  ep.col_sum = col_sum; ep.col_sqsum = col_sqsum; ep.error_flag = error_flag;
-  ep.tx_bytes = 0; ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
+// Data gradient on the weights as stored: dy [N,Ho,Wo,Cout], w [Cout,R,S,Cin], dx [N,H,W,Cin] (dense NHWC).
+// Stride 1: one launch, any R x S with padding up to min(R, S) - 1.  Stride 2: 3x3 filters with padding 1 on even H and W;
+// each output parity (h % 2, w % 2) meets 1, 2, 2 or 4 of the nine taps and is a dense stride-1 problem written
+// into its interleaved pixels of dx (dx[2i + p] uses the filter rows r with (p + 1 - r) even).
+int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, int R, int S,
+                      int stride, int pad, int* error_flag, void* stream) {
+  if (Cin % 8 || Cout % 8) return -1;
+  const Epilogue ep = epilogue_for(Cin, 0, nullptr, nullptr, error_flag);
   cudaStream_t s = (cudaStream_t)stream;
-  const int BN = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
-  int bh = 0;
-  if (BN <= 128 && halo_applicable(a, (H + 2 * pad - R) / stride + 1, (W + 2 * pad - S) / stride + 1, &bh))
-    return BN == 64 ? launch_halo<64>(a, ep, bh, s) : launch_halo<128>(a, ep, bh, s);
-  if (BN == 64) return launch<64>(a, ep, s);
-  if (BN == 128) return launch<128>(a, ep, s);
-  return launch<256>(a, ep, s);
+  if (stride == 1) {
+    if (pad > R - 1 || pad > S - 1 || R != S) return -1;
+    ConvArgs a{dy, w, dx, N, H + 2 * pad - R + 1, W + 2 * pad - S + 1, Cout, Cin, R, S, 1, R - 1 - pad};
+    a.fR = R; a.fS = S;
+    a.taps = FilterTaps{R - 1, -1, S - 1, -1};
+    return dispatch<true>(a, ep, s);
+  }
+  if (stride != 2 || R != 3 || S != 3 || pad != 1 || H % 2 || W % 2) return -1;
+  for (int ph = 0; ph < 2; ++ph)
+    for (int pw = 0; pw < 2; ++pw) {
+      ConvArgs a{dy, w, (char*)dx + ((int64_t)ph * W + pw) * Cin * 2, N, H / 2, W / 2, Cout, Cin, 1 + ph, 1 + pw, 1, 0};
+      a.out_h = H / 2; a.out_w = W / 2;
+      a.ys_w = 2 * (int64_t)Cin; a.ys_h = 2 * (int64_t)W * Cin; a.ys_n = (int64_t)H * W * Cin;
+      a.fR = a.fS = 3;
+      a.taps = FilterTaps{ph ? 2 : 1, -2, pw ? 2 : 1, -2};
+      int rc = dispatch<true>(a, ep, s);
+      if (rc != 0) return rc;
+    }
+  return 0;
 }
 
 // Host arithmetic of the halo-mode forward / data-gradient launch, without launching (no device needed).
@@ -511,14 +581,14 @@ int esgd_conv2d_fwd_ex(const void* x, const void* w, void* y, int N, int H, int 
 // bytes of one input box, bytes the most shifted view reaches, stage area used.
 void esgd_conv2d_halo_plan(int N, int H, int W, int Cin, int Cout, int R, int S, int stride, int pad, int* out) {
   for (int i = 0; i < 10; ++i) out[i] = 0;
-  if (Cin % 64 || Cout % 8) return;
+  if (Cin % 8 || Cout % 8) return;
   ConvArgs a{nullptr, nullptr, nullptr, N, H, W, Cin, Cout, R, S, stride, pad};
   const int BN = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
   int bh = 0;
   if (BN > 128 || stride != 1 || !halo_applicable(a, H + 2 * pad - R + 1, W + 2 * pad - S + 1, &bh)) return;
   const int PW = W + 2 * pad;
   const int b_stage = BN * 128, stage_area = BN == 64 ? Cfg<64>::STAGE_AREA : Cfg<128>::STAGE_AREA;
-  const int kb_total = R * S * (Cin / 64);
+  const int kb_total = R * S * ((Cin + 63) / 64);
   const int res_kb = (kb_total * b_stage + 2 * HALO_BYTES <= stage_area) ? kb_total : 0;
   const int nhalo = res_kb > 0 ? 2 : MAX_HALOS;
   int nstages = 1;

@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      const uint32_t tx = (uint32_t)(NA * p.BH * p.PW * 128 + NB * (p.BH + p.R - 1) * p.PW * 128);
+      const int na = min(NA, (p.Cout - m0 + 63) / 64);     // atoms of dy that hold channels; the other stays zero
+      const uint32_t tx = (uint32_t)(na * p.BH * p.PW * 128 + NB * (p.BH + p.R - 1) * p.PW * 128);
       for (int b = box0; b < box1; ++b) {
         if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) break;
         const int h0 = (b % p.h_tiles) * p.BH, n = b / p.h_tiles;
@@ -99,7 +100,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
         uint8_t* sb = sa + NA * p.abox;
         mbar_expect_tx(&full[stage], tx);
 #pragma unroll
-        for (int i = 0; i < NA; ++i) tma_load_4d(sa + i * p.abox, &p.tmDY, &full[stage], m0 + 64 * i, 0, h0, n);
+        for (int i = 0; i < NA; ++i)
+          if (i < na) tma_load_4d(sa + i * p.abox, &p.tmDY, &full[stage], m0 + 64 * i, 0, h0, n);
 #pragma unroll
         for (int i = 0; i < NB; ++i)
           tma_load_4d(sb + i * p.xbox, &p.tmX, &full[stage], n0 + 64 * i, -p.pad, h0 - p.pad, n);
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(128, BN, 1, 1);
+      const uint32_t idesc = umma_idesc_bf16(128, min(BN, (p.Cin - n0 + 15) / 16 * 16), 1, 1);
       int stage = 0;
       uint32_t phase = 0;
       uint32_t accumulate = 0;
@@ -232,7 +234,7 @@ int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int
 
 // Largest number of full output rows whose pitched pixels fit one 128-row K range; 0: outside this kernel's range.
 int wg_pick_bh(int H, int W, int Cin, int Cout, int R, int S, int pad) {
-  if (Cin % 64 || Cout % 8 || R * S < 2) return 0;
+  if (Cin % 8 || Cout % 8 || R * S < 2) return 0;
   const int Ho = H + 2 * pad - R + 1, Wo = W + 2 * pad - S + 1;
   const int PW = Wo + S - 1;
   if (Ho < 1 || Wo < 1 || PW > 128) return 0;
@@ -282,7 +284,7 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
 extern "C" {
 
 // Returns -100 when the shape is outside this kernel's range (the caller then uses the per-tap kernel).
-// dw: fp32 [Cout][R][S][Cin], zeroed by the caller.  Stride 1 only; Cin % 64 == 0, Cout % 8 == 0.
+// dw: fp32 [Cout][R][S][Cin], zeroed by the caller.  Stride 1 only; Cin % 8 == 0, Cout % 8 == 0.
 int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R,
                            int S, int pad, int* error_flag, void* stream) {
   {

@@ -29,6 +29,7 @@ struct GemmProblem {
   int res_kb;         // > 0: all k-blocks of B for the CTA's column range stay in shared memory
   float* c_f32;       // fp32 output (direct modes)
   int ldc;
+  static constexpr int ksteps = BK / 16, n_mma = BN_;
   int chained;        // launched with programmatic stream serialization: wait for the previous kernel in the kernel
 
   struct Tile { int kb0, kb1, n0, m0; };
@@ -224,19 +225,22 @@ extern "C" {
 // C[M,N] = A * B^T (+bias, ReLU, column statistics).  A is [M][K] (a_mn=0, row stride lda)
 // or stored [K][M] (a_mn=1); B is [N][K] (b_mn=0, row stride ldb) or stored [K][N] (b_mn=1).
 // out_mode: 0 bf16, 1 fp32, 2 fp32 atomic accumulate (split-K; C must be zeroed by the caller).
-// Requirements: 16-byte aligned bases, lda/ldb/ldc multiples of 8, N multiple of 8.
+// Requirements: 16-byte aligned bases, lda/ldb/ldc multiples of 8.  N need not be a multiple of 8: an fp32 output is
+// then written up to the next multiple of 4 columns, inside its row stride.
+// relu: bit 0 ReLU, bit 1 the bias is bf16.
 // col_sum / col_sqsum (bf16 output only) accumulate into caller-zeroed fp32 arrays of N.
 // residual (bf16 output only): a bf16 [M][N] tensor with row stride ldr (multiple of 8), added before rounding.
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
                    int b_mn, int out_mode, const float* bias, int relu, int splits, float* col_sum,
                    float* col_sqsum, const void* residual, int ldr, int* error_flag, void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || (N % 8) || (lda % 8) || (ldb % 8) || (ldc % 8)) return -1;
+  if (M <= 0 || N <= 0 || K <= 0 || (lda % 8) || (ldb % 8) || (ldc % 8)) return -1;
+  if (out_mode == OUT_F32_ATOMIC ? N % 4 : ldc < (N + 7) / 8 * 8) return -1;
   if (col_sum != nullptr && out_mode != OUT_BF16) return -4;
   if (residual != nullptr && (out_mode != OUT_BF16 || (ldr % 8) || ((uintptr_t)residual & 15))) return -5;
-  if (out_mode != OUT_BF16 && (((uintptr_t)C & 15) || ((uintptr_t)bias & 15))) return -6;   // 16-byte fp32 accesses
+  if (out_mode != OUT_BF16 && (((uintptr_t)C & 15) || ((uintptr_t)bias & (relu & 2 ? 7 : 15)))) return -6;   // 16-byte fp32 accesses
   GemmArgs g{A, B, C, M, N, K, lda, ldb, ldc, out_mode, splits};
   Epilogue ep;
-  ep.out_mode = out_mode; ep.relu = relu; ep.n_total = N; ep.bias = bias;
+  ep.out_mode = out_mode; ep.relu = relu & 1; ep.n_total = N; ep.bias = bias; ep.bias_bf16 = (relu >> 1) & 1;
   ep.col_sum = col_sum; ep.col_sqsum = col_sqsum; ep.error_flag = error_flag;
   ep.tx_bytes = 0; ep.tx_bytes_a = 0;
   ep.residual = residual; ep.ldr = ldr;

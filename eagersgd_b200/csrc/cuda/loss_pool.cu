@@ -321,6 +321,56 @@ __global__ void __launch_bounds__(256) im2col_rows_kernel(const __nv_bfloat16* _
   }
 }
 
+// Stem filters [Cout][R][S][C] -> the column layout above ([Cout][Kpad], segments of `seg`, zeros elsewhere).
+__global__ void __launch_bounds__(256) stem_pack_kernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
+                                                        int Cout, int R, int sc, int seg, int Kpad) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= Cout * Kpad) return;
+  const int co = i / Kpad, k = i - co * Kpad, r = k / seg, j = k - r * seg;
+  out[i] = r < R && j < sc ? w[(co * R + r) * sc + j] : __float2bfloat16(0.0f);
+}
+// The way back for the filter gradient: fp32 columns -> bf16 filters (dw) or added to an fp32 accumulator (acc).
+__global__ void __launch_bounds__(256) stem_unpack_kernel(const float* __restrict__ col, __nv_bfloat16* dw, float* acc, int Cout,
+                                                          int R, int sc, int seg, int Kpad) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= Cout * R * sc) return;
+  const int co = i / (R * sc), k = i - co * R * sc, r = k / sc, j = k - r * sc;
+  const float v = col[(int64_t)co * Kpad + r * seg + j];
+  if (acc != nullptr) acc[i] += v;
+  else dw[i] = __float2bfloat16(v);
+}
+
+// Gradient of a dense layer's fp32 output: bf16 copy with the row padded to np columns (zeros), and its column sums in the
+// same pass (dy is read once).  A thread keeps four columns and walks down the rows of its block.
+constexpr int kCastRows = 64;
+__global__ void __launch_bounds__(256) cast_colsum_kernel(const float* __restrict__ dy, int64_t ld, int M, int N, int np,
+                                                          __nv_bfloat16* __restrict__ out, float* __restrict__ colsum, int vec) {
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+  if (c >= np) return;
+  const int r0 = blockIdx.y * kCastRows, r1 = min(M, r0 + kCastRows);
+  float s[4] = {0, 0, 0, 0};
+#pragma unroll 4
+  for (int r = r0; r < r1; ++r) {
+    float v[4];
+    if (vec && c + 4 <= N) {
+      const float4 f = __ldcs(reinterpret_cast<const float4*>(dy + r * ld + c));
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = c + q < N ? dy[r * ld + c + q] : 0.0f;
+    }
+    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+    *reinterpret_cast<uint2*>(out + (int64_t)r * np + c) = *reinterpret_cast<const uint2*>(h);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[q] += v[q];
+  }
+  if (colsum != nullptr) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (c + q < N) atomicAdd(colsum + c + q, s[q]);
+  }
+}
+
 int grid_for(int64_t items) {
   int64_t b = (items + 255) / 256;
   const int64_t cap = 148 * 16;
@@ -402,6 +452,31 @@ int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, in
   }
   im2col_small_c_kernel<32><<<grid_for((int64_t)N * Ho * Wo * (Kpad / seg)), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)x, (__nv_bfloat16*)col, N, H, W, C, R, S, stride, pad, Ho, Wo, seg, Kpad);
+  esgd::count_launch();
+  return (int)cudaGetLastError();
+}
+
+// seg / Kpad as in esgd_im2col_small_c; w [Cout][R][S*C], sc = S*C.
+int esgd_stem_pack(const void* w, void* out, int Cout, int R, int sc, int seg, int Kpad, void* stream) {
+  stem_pack_kernel<<<(Cout * Kpad + 255) / 256, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)w, (__nv_bfloat16*)out,
+                                                                               Cout, R, sc, seg, Kpad);
+  esgd::count_launch();
+  return (int)cudaGetLastError();
+}
+int esgd_stem_unpack(const float* col, void* dw, float* acc, int Cout, int R, int sc, int seg, int Kpad, void* stream) {
+  stem_unpack_kernel<<<(Cout * R * sc + 255) / 256, 256, 0, (cudaStream_t)stream>>>(col, (__nv_bfloat16*)dw, acc, Cout, R, sc,
+                                                                                   seg, Kpad);
+  esgd::count_launch();
+  return (int)cudaGetLastError();
+}
+
+// out [M][np] bf16 (np a multiple of 8, zeros from column N on) = dy [M][N] fp32 with row stride ld; colsum (optional, zeroed
+// by the caller) += column sums of dy.
+int esgd_cast_colsum(const float* dy, int64_t ld, int M, int N, int np, void* out, float* colsum, void* stream) {
+  if (np % 8 || np < N) return -1;
+  const int vec = ld % 4 == 0 && ((uintptr_t)dy & 15) == 0;
+  dim3 grid((np / 4 + 255) / 256, (M + kCastRows - 1) / kCastRows);
+  cast_colsum_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(dy, ld, M, N, np, (__nv_bfloat16*)out, colsum, vec);
   esgd::count_launch();
   return (int)cudaGetLastError();
 }

@@ -45,6 +45,7 @@ struct Epilogue {
   int relu;
   int n_total;             // number of valid output columns (channels)
   const float* bias;       // per column, may be null
+  int bias_bf16;           // ... and bf16 instead of fp32
   float* col_sum;          // optional per-column statistics of the stored bf16 values
   float* col_sqsum;
   int* error_flag;
@@ -89,6 +90,11 @@ inline bool resident_enabled() {
   return v == 1;
 }
 
+__device__ __forceinline__ float bias_at(const Epilogue& ep, int col) {
+  if (col >= ep.n_total) return 0.0f;
+  return ep.bias_bf16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(ep.bias) + col)) : __ldg(ep.bias + col);
+}
+
 // 32 accumulator columns of one row -> bf16 -> four 16-byte chunks of the swizzled staging panel.
 // kPlain leaves out the bias / ReLU code altogether: as run-time options they would be predicated
 // instructions that still take issue slots in the common case that uses neither.
@@ -115,7 +121,7 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
       if (ep.bias != nullptr) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-          if (col0 + g * 8 + j < ep.n_total) v[j] += __ldg(ep.bias + col0 + g * 8 + j);
+          v[j] += bias_at(ep, col0 + g * 8 + j);
       }
       if (ep.relu) {
 #pragma unroll
@@ -133,6 +139,7 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
 // Problem policy requirements (all __device__ const):
 //   static constexpr int BN; static constexpr bool A_MN, B_MN, kZeroStages;
 //   struct Tile { int kb0, kb1, n0; ... };
+//   int ksteps, n_mma                              16-wide K steps of a k-block that hold anything; MMA columns
 //   bool tile(int it, Tile&)                       enumerate this CTA's tiles
 //   void load(const Tile&, int kb, uint8_t* a, uint8_t* b, uint64_t* bar)
 //   void load_a(...a, bar) / load_b(...b, bar)     the two halves of load(); int res_kb (0: B not resident)
@@ -257,7 +264,8 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, P::A_MN ? 1 : 0, P::B_MN ? 1 : 0);
+      const uint32_t idesc = umma_idesc_bf16(BM, prob.n_mma, P::A_MN ? 1 : 0, P::B_MN ? 1 : 0);
+      const int ksteps = prob.ksteps;            // < 4: the reduction has fewer than 64 channels, the rest is zero fill
       // The issuing thread is one lane with nothing to hide its instruction latency behind: every instruction
       // between two tcgen05.mma widens the gap between them.  (Timestamps taken in this loop: a 128 x 64 x 16
       // MMA goes out every ~115 cycles, a 128 x 256 x 16 one every ~185 -- 32 and 128 cycles of tensor-pipe work
@@ -299,7 +307,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
                 }
 #pragma unroll
                 for (int j = 0; j < BK / 16; ++j) {
-                  umma_bf16(d_tmem, a_tap + j * kStepA, b_cur + j * kStepB, idesc, accumulate);
+                  if (j < ksteps) umma_bf16(d_tmem, a_tap + j * kStepA, b_cur + j * kStepB, idesc, accumulate);
                   accumulate = 1;
                 }
                 if (res_kb == 0) {
@@ -320,7 +328,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           const uint64_t b_cur = b_desc0 + (uint64_t)((res_kb > 0 ? kb : stage) * (C::B_STAGE_BYTES >> 4));
 #pragma unroll
           for (int j = 0; j < BK / 16; ++j) {
-            umma_bf16(d_tmem, a_cur + j * kStepA, b_cur + j * kStepB, idesc, accumulate);
+            if (j < ksteps) umma_bf16(d_tmem, a_cur + j * kStepA, b_cur + j * kStepB, idesc, accumulate);
             accumulate = 1;
           }
           umma_commit(&empty[stage]);
@@ -462,8 +470,13 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
                 float4 v = make_float4(__uint_as_float(r[j4 * 4]), __uint_as_float(r[j4 * 4 + 1]),
                                        __uint_as_float(r[j4 * 4 + 2]), __uint_as_float(r[j4 * 4 + 3]));
                 if (ep.bias != nullptr) {
-                  const float4 b4 = __ldg(reinterpret_cast<const float4*>(ep.bias + col0 + j4 * 4));
-                  v.x += b4.x; v.y += b4.y; v.z += b4.z; v.w += b4.w;
+                  const int c0 = col0 + j4 * 4;
+                  if (!ep.bias_bf16 && c0 + 4 <= ep.n_total) {
+                    const float4 b4 = __ldg(reinterpret_cast<const float4*>(ep.bias + c0));
+                    v.x += b4.x; v.y += b4.y; v.z += b4.z; v.w += b4.w;
+                  } else {
+                    v.x += bias_at(ep, c0); v.y += bias_at(ep, c0 + 1); v.z += bias_at(ep, c0 + 2); v.w += bias_at(ep, c0 + 3);
+                  }
                 }
                 if (ep.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
                 float4* dst = reinterpret_cast<float4*>(out_row + col0 + j4 * 4);

@@ -1,0 +1,657 @@
+// Autograd operators over the sm_100a kernels, in C++.
+//
+// The kernels themselves are plain launchers in libesgd_cuda.so.  What surrounds a launch -- shape checks, output
+// allocation, autograd bookkeeping, the choice of a kernel -- used to run in Python and cost 60 to 150 us per operator and
+// direction, several times what the GPU needs for a CIFAR layer or a single image; here it costs a few microseconds, and
+// the backward half runs on the autograd thread without the interpreter lock.
+//
+// GradSinks: while a training step of this package is active, the backward of an operator adds its parameter gradients
+// straight to fp32 accumulators of the optimizer's flat buckets and tells the bucket so, instead of handing autograd a
+// bf16 tensor that is cast, added to a zeroed .grad and cast again: three small kernels and a Python hook fewer per tensor.
+#include <torch/extension.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <atomic>
+#include <mutex>
+#include <shared_mutex>
+#include <unordered_map>
+
+extern "C" {
+int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn, int b_mn,
+                   int out_mode, const void* bias, int relu, int splits, float* col_sum, float* col_sqsum,
+                   const void* residual, int ldr, int* error_flag, void* stream);
+int esgd_conv2d_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S, int stride,
+                    int pad, int relu, float* col_sum, float* col_sqsum, int* error_flag, void* stream);
+int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, int R, int S, int stride,
+                      int pad, int* error_flag, void* stream);
+int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
+                      int stride, int pad, int* error_flag, void* stream);
+int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
+                           int pad, int* error_flag, void* stream);
+int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, int R, int S, int stride, int pad, int seg,
+                        int Kpad, void* stream);
+int esgd_stem_pack(const void* w, void* out, int Cout, int R, int sc, int seg, int Kpad, void* stream);
+int esgd_stem_unpack(const float* col, void* dw, float* acc, int Cout, int R, int sc, int seg, int Kpad, void* stream);
+int esgd_subsample2_fwd(const void* x, void* y, int N, int H, int W, int C, void* stream);
+int esgd_subsample2_bwd(const void* dy, void* dx, int N, int H, int W, int C, void* stream);
+int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, void* stream);
+int esgd_bn_fwd(const void* y, const void* residual, void* z, const float* sum, const float* sqsum, const float* gamma,
+                const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu,
+                float momentum, float eps, void* stream);
+int esgd_bn_bwd_reduce(const void* dz, const void* z, const void* y, const float* mean, const float* invstd,
+                       const float* fscale, const float* fshift, int64_t M, int C, int relu, float* dbeta, float* dgamma,
+                       void* stream);
+int esgd_bn_bwd_apply(const void* dz, const void* z, const void* y, const float* mean, const float* invstd, const float* gamma,
+                      const float* dbeta, const float* dgamma, const float* fscale, const float* fshift, void* dy, void* dres,
+                      int64_t M, int C, int relu, float* acc_dgamma, float* acc_dbeta, void* stream);
+int esgd_softmax_ce(const void* logits, int is_bf16, const int64_t* labels, int batch, int classes, int ld, float grad_scale,
+                    float* loss_sum, float* per_sample, void* dlogits, void* stream);
+int esgd_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream);
+int esgd_maxpool3x3s2_bwd(const void* idx, const void* dy, void* dx, int N, int H, int W, int C, void* stream);
+int esgd_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream);
+int esgd_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, void* stream);
+int esgd_cast_colsum(const float* dy, int64_t ld, int M, int N, int np, void* out, float* colsum, void* stream);
+}
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+constexpr auto kCL = at::MemoryFormat::ChannelsLast;
+constexpr float kBnEps = 1e-5f;
+
+void ck(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed with code ", rc); }
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+float* fptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+Tensor nhwc(const Tensor& t) { return t.contiguous(kCL); }
+Tensor empty_nhwc(int64_t n, int64_t c, int64_t h, int64_t w, const Tensor& like) {
+  return at::empty({n, c, h, w}, like.options(), kCL);
+}
+
+// ---------------------------------------------------------------- per-device error word of the tensor-core kernels
+Tensor error_flag(int64_t device) {
+  static std::mutex m;
+  static Tensor flags[64];
+  TORCH_CHECK(device >= 0 && device < 64);
+  std::lock_guard<std::mutex> g(m);
+  if (!flags[device].defined())
+    flags[device] = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, (c10::DeviceIndex)device));
+  return flags[device];
+}
+int* flag_ptr(const Tensor& t) {
+  static std::atomic<int*> cached[64];
+  const int d = t.get_device();
+  int* p = cached[d].load(std::memory_order_acquire);
+  if (p == nullptr) {
+    p = error_flag(d).data_ptr<int>();
+    cached[d].store(p, std::memory_order_release);
+  }
+  return p;
+}
+
+// ---------------------------------------------------------------- zeroed scratch of a training step
+// One fp32 buffer cleared by a single memset at the start of a step, from which the operators take their zero-initialised
+// scratch (statistics and reduction accumulators).  A slice must not outlive the step.
+class ZeroArena {
+ public:
+  void begin(at::Device device, int64_t numel);
+  void end();
+  Tensor take(at::IntArrayRef shape) {
+    std::lock_guard<std::mutex> g(m_);
+    const int64_t n = c10::multiply_integers(shape), n_al = (n + 63) / 64 * 64;    // 256-byte aligned slices
+    if (off_ + n_al > cap_) return Tensor();
+    if (!buf_.defined()) buf_ = at::zeros({cap_}, at::TensorOptions().dtype(at::kFloat).device(device_));
+    std::vector<int64_t> strides(shape.size());
+    int64_t s = 1;
+    for (int i = (int)shape.size() - 1; i >= 0; --i) { strides[i] = s; s *= shape[i]; }
+    Tensor out = buf_.as_strided(shape, strides, off_);
+    off_ += n_al;
+    dirty_ = std::max(dirty_, off_);
+    return out;
+  }
+
+ private:
+  std::mutex m_;
+  Tensor buf_;
+  int64_t off_ = 0, dirty_ = 0, cap_ = 0;
+  at::Device device_ = at::Device(at::kCPU);
+};
+std::atomic<ZeroArena*> g_arena[65];        // the active arena of the CPU (0) and of every GPU (1 + index)
+std::atomic<ZeroArena*>& arena_slot(at::Device d) { return g_arena[d.is_cuda() ? 1 + d.index() : 0]; }
+
+void ZeroArena::begin(at::Device device, int64_t numel) {
+  if (device.is_cuda() && !device.has_index()) device = at::Device(at::kCUDA, c10::cuda::current_device());
+  std::lock_guard<std::mutex> g(m_);
+  if (buf_.defined() && (buf_.device() != device || buf_.numel() < numel)) { buf_ = Tensor(); dirty_ = 0; }
+  device_ = device;
+  if (buf_.defined() && dirty_ > 0) buf_.narrow(0, 0, dirty_).zero_();             // what earlier steps used
+  off_ = 0;
+  cap_ = numel;
+  arena_slot(device).store(this, std::memory_order_release);
+}
+void ZeroArena::end() {
+  ZeroArena* me = this;
+  arena_slot(device_).compare_exchange_strong(me, nullptr);
+}
+
+Tensor zeros_f32(at::IntArrayRef shape, at::Device device) {
+  if (ZeroArena* a = arena_slot(device).load(std::memory_order_acquire)) {
+    Tensor t = a->take(shape);
+    if (t.defined()) return t;
+  }
+  return at::zeros(shape, at::TensorOptions().dtype(at::kFloat).device(device));
+}
+
+// ---------------------------------------------------------------- gradient sinks
+class GradSinks;
+struct SinkEntry : torch::CustomClassHolder {
+  float* acc = nullptr;          // fp32 accumulator, in the parameter's own memory order (OHWI for channels_last filters)
+  int bucket = 0;
+  int uses = 0;                  // forward uses of this step whose backward has not run yet
+  bool used = false;             // took part in this step
+  std::atomic<GradSinks*> owner{nullptr};
+};
+using Sink = c10::intrusive_ptr<SinkEntry>;
+
+std::shared_mutex g_sink_mutex;
+std::unordered_map<at::TensorImpl*, Sink> g_sinks;
+
+class GradSinks {
+ public:
+  GradSinks(std::vector<int> params_per_bucket, py::function on_bucket)
+      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), on_bucket_(std::move(on_bucket)) {}
+  ~GradSinks() { close(); }
+  void close() {
+    std::unique_lock<std::shared_mutex> g(g_sink_mutex);
+    for (auto& kv : mine_) { kv.second->owner.store(nullptr); g_sinks.erase(kv.first); }
+    mine_.clear();
+  }
+  void add(const Tensor& param, const Tensor& acc, int bucket) {
+    TORCH_CHECK(acc.scalar_type() == at::kFloat && acc.numel() == param.numel());
+    auto e = c10::make_intrusive<SinkEntry>();
+    e->acc = acc.data_ptr<float>();
+    e->bucket = bucket;
+    e->owner.store(this);
+    std::unique_lock<std::shared_mutex> g(g_sink_mutex);
+    g_sinks[param.unsafeGetTensorImpl()] = e;
+    mine_[param.unsafeGetTensorImpl()] = e;
+  }
+  void begin_step() {
+    pending_ = total_;
+    for (auto& kv : mine_) { kv.second->uses = 0; kv.second->used = false; }
+  }
+  void set_active(bool on) { active_.store(on); }
+  bool active() const { return active_.load(); }
+  bool used(const Tensor& param) const {
+    auto it = mine_.find(param.unsafeGetTensorImpl());
+    return it != mine_.end() && it->second->used;
+  }
+  bool written(int bucket) const { return written_[bucket] != 0; }
+  void clear_written() { std::fill(written_.begin(), written_.end(), 0); }
+  void mark_written(int bucket) { written_[bucket] = 1; }
+  void param_done(int bucket) {
+    if (--pending_[bucket] == 0) {
+      py::gil_scoped_acquire gil;
+      on_bucket_(bucket);
+    }
+  }
+
+ private:
+  std::vector<int> total_, pending_, written_;
+  std::atomic<bool> active_{false};
+  py::function on_bucket_;
+  std::unordered_map<at::TensorImpl*, Sink> mine_;
+};
+
+// The sink of a parameter in a step that is under way, or null.
+Sink find_sink(const Tensor& p) {
+  if (!p.defined() || !p.requires_grad() || !p.is_leaf() || !at::GradMode::is_enabled()) return Sink();
+  std::shared_lock<std::shared_mutex> g(g_sink_mutex);
+  if (g_sinks.empty()) return Sink();
+  auto it = g_sinks.find(p.unsafeGetTensorImpl());
+  if (it == g_sinks.end()) return Sink();
+  GradSinks* o = it->second->owner.load();
+  return o != nullptr && o->active() ? it->second : Sink();
+}
+// Called in an operator's forward for a parameter that its backward will write.
+void sink_use(const Sink& s) {
+  if (s) { ++s->uses; s->used = true; }
+}
+// Called in its backward once the kernel that writes the accumulator has been launched.
+void sink_done(const Sink& s) {
+  GradSinks* o = s->owner.load();
+  if (o == nullptr || s->uses <= 0) return;
+  o->mark_written(s->bucket);
+  if (--s->uses == 0) o->param_done(s->bucket);
+}
+void save_sink(AutogradContext* ctx, const char* key, const Sink& s) {
+  if (s) ctx->saved_data[key] = c10::IValue::make_capsule(s);
+}
+Sink load_sink(AutogradContext* ctx, const char* key) {
+  auto it = ctx->saved_data.find(key);
+  if (it == ctx->saved_data.end()) return Sink();
+  Sink s = c10::static_intrusive_pointer_cast<SinkEntry>(it->second.toCapsule());
+  return s->owner.load() != nullptr ? s : Sink();
+}
+
+// ---------------------------------------------------------------- GEMM
+int gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, int64_t ldc,
+         bool a_mn, bool b_mn, int mode, int splits, float* cs, float* cq, const void* res, int64_t ldr, const Tensor& like,
+         const void* bias = nullptr, int flags = 0) {
+  return esgd_gemm_bf16(a, b, c, (int)m, (int)n, (int)k, (int)lda, (int)ldb, (int)ldc, a_mn, b_mn, mode, bias, flags, splits, cs,
+                        cq, res, (int)ldr, flag_ptr(like), stream_of(like));
+}
+
+// Split-K factor of a weight-gradient GEMM (K = pixels): about one wave of tiles.  Each split adds a full [Cout, Cin]
+// partial result with atomics, so large filter banks take few splits.
+int wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int64_t sms = 148) {
+  const int64_t bn = cin <= 64 ? 64 : (cin <= 128 ? 128 : 256);
+  const int64_t tiles = ((cout + 127) / 128) * ((cin + bn - 1) / bn);
+  return (int)std::max<int64_t>(2, std::min((sms + tiles - 1) / tiles, std::max<int64_t>(1, (pixels / 64) / 8)));
+}
+
+// ---------------------------------------------------------------- convolutions
+enum ConvKind : int64_t { kOneByOne = 0, kGeneral = 1, kStem = 2 };
+
+struct StemGeometry {
+  int64_t seg, kpad;
+  StemGeometry(int64_t c, int64_t r, int64_t s) {
+    seg = (s * c + 7) / 8 * 8;                        // one filter row, padded to 16 bytes
+    kpad = (r * seg + 63) / 64 * 64;
+    while (kpad % seg) kpad += 64;
+  }
+};
+
+// y = x (*) w, and on request the per-channel sum / sum of squares of y and the input itself.
+//
+// With `tap` the input is returned as a last output.  A residual block takes its shortcut from that output instead of
+// from x itself: backward then receives the shortcut's gradient together with dy and adds it in the epilogue of the
+// data-gradient GEMM, instead of autograd summing the two branches of x with a separate pass over the tensor.
+struct ConvFn : public Function<ConvFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w, int64_t kind, int64_t stride, int64_t pad,
+                               bool want_stats, bool tap, const Sink& sink) {
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = nhwc(x_in);
+    const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3);
+    const int64_t cout = w.size(0), r = w.size(2), s = w.size(3);
+    const int64_t ho = (h + 2 * pad - r) / stride + 1, wo = (wd + 2 * pad - s) / stride + 1;
+    void* st = stream_of(x);
+    Tensor stats;
+    if (want_stats) stats = zeros_f32({2, cout}, x.device());
+    float *cs = fptr(stats), *cq = want_stats ? cs + cout : nullptr;
+    Tensor y = empty_nhwc(n, cout, ho, wo, x);
+    Tensor saved_x, wk;
+    if (kind == kOneByOne) {
+      wk = w.contiguous();                            // [Cout, Cin]: a 1x1 filter has one memory order
+      saved_x = x;
+      if (stride == 2) {
+        saved_x = empty_nhwc(n, cin, ho, wo, x);
+        ck(esgd_subsample2_fwd(x.data_ptr(), saved_x.data_ptr(), n, h, wd, cin, st), "subsample");
+      }
+      ck(gemm(saved_x.data_ptr(), wk.data_ptr(), y.data_ptr(), n * ho * wo, cout, cin, cin, cin, cout, false, false, 0, 1, cs, cq,
+              nullptr, 0, x), "1x1 convolution");
+    } else if (kind == kGeneral) {
+      wk = nhwc(w);                                   // [Cout][R][S][Cin] in memory
+      saved_x = x;
+      ck(esgd_conv2d_fwd(x.data_ptr(), wk.data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, 0, cs, cq, flag_ptr(x),
+                         st), "conv2d");
+    } else {
+      wk = nhwc(w);
+      const StemGeometry g(cin, r, s);
+      saved_x = at::empty({n * ho * wo, g.kpad}, x.options());
+      ck(esgd_im2col_small_c(x.data_ptr(), saved_x.data_ptr(), n, h, wd, cin, r, s, stride, pad, g.seg, g.kpad, st), "im2col");
+      Tensor w2d = at::empty({cout, g.kpad}, x.options());
+      ck(esgd_stem_pack(wk.data_ptr(), w2d.data_ptr(), cout, r, s * cin, g.seg, g.kpad, st), "stem filters");
+      ck(gemm(saved_x.data_ptr(), w2d.data_ptr(), y.data_ptr(), n * ho * wo, cout, g.kpad, g.kpad, g.kpad, cout, false, false, 0, 1,
+              cs, cq, nullptr, 0, x), "stem convolution");
+    }
+    ctx->save_for_backward({saved_x, wk});
+    ctx->saved_data["cfg"] = std::vector<int64_t>{kind, stride, pad, n, cin, h, wd, want_stats, tap};
+    save_sink(ctx, "w", sink);
+    ctx->set_materialize_grads(false);                // an unused tap must not cost a tensor of zeros
+    variable_list out{y};
+    if (want_stats) {
+      ctx->mark_non_differentiable({stats});
+      out.push_back(stats);
+    }
+    if (tap) out.push_back(x_in.view_as(x_in));
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto cfg = ctx->saved_data["cfg"].toIntVector();
+    const int64_t kind = cfg[0], stride = cfg[1], pad = cfg[2], n = cfg[3], cin = cfg[4], h = cfg[5], wd = cfg[6];
+    const bool want_stats = cfg[7], tap = cfg[8];
+    variable_list none(8);
+    Tensor d_tap = tap ? grads[want_stats ? 2 : 1] : Tensor();   // gradient that reached the input through the shortcut
+    Sink sink = load_sink(ctx, "w");
+    if (!grads[0].defined()) {
+      none[0] = d_tap;
+      return none;
+    }
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    const int64_t cout = w.size(0), r = w.size(2), s = w.size(3);
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor dy = nhwc(grads[0]);
+    const int64_t ho = dy.size(2), wo = dy.size(3), m = n * ho * wo;
+    void* st = stream_of(x);
+    Tensor dx, dw;
+    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
+    if (need_dx && kind == kOneByOne) {
+      Tensor res;
+      if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
+      dx = empty_nhwc(n, cin, ho, wo, x);
+      ck(gemm(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), m, cin, cout, cout, cin, cin, false, true, 0, 1, nullptr, nullptr,
+              res.defined() ? res.data_ptr() : nullptr, cin, x), "1x1 convolution data gradient");
+      if (stride == 2) {
+        Tensor full = empty_nhwc(n, cin, h, wd, x);
+        ck(esgd_subsample2_bwd(dx.data_ptr(), full.data_ptr(), n, h, wd, cin, st), "subsample backward");
+        dx = full;
+      }
+    } else if (need_dx && kind == kGeneral) {
+      const bool square = r == s && pad <= r - 1;
+      dx = empty_nhwc(n, cin, h, wd, x);
+      if (square && stride == 1) {
+        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, flag_ptr(x), st),
+           "conv2d data gradient");
+      } else if (stride == 2 && r == 3 && s == 3 && pad == 1 && h % 2 == 0 && wd % 2 == 0) {
+        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, 3, 3, 2, 1, flag_ptr(x), st),
+           "strided conv2d data gradient");
+      } else if (square) {
+        // Any other stride / size: the gradient is spread out with (stride - 1) zeros between its pixels (plus the rows and
+        // columns at the far edge that no window reached) and then goes through the stride-1 form above.
+        const int64_t eh = (h + 2 * pad - r) % stride, ew = (wd + 2 * pad - s) % stride;
+        Tensor spread = at::zeros({n, cout, (ho - 1) * stride + 1 + eh, (wo - 1) * stride + 1 + ew}, dy.options()).contiguous(kCL);
+        spread.slice(2, 0, (ho - 1) * stride + 1, stride).slice(3, 0, (wo - 1) * stride + 1, stride).copy_(dy);
+        ck(esgd_conv2d_dgrad(spread.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, flag_ptr(x), st),
+           "conv2d data gradient");
+      } else {
+        dx = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {stride, stride}, {pad, pad}, {1, 1}, false, {0, 0}, 1,
+                                                  {true, false, false}));
+      }
+      if (d_tap.defined()) dx = dx + d_tap;
+    } else if (need_dx) {
+      dx = d_tap;
+    }
+    if (need_dw) {
+      if (kind == kOneByOne) {
+        Tensor dw32;
+        if (!sink) dw32 = zeros_f32({cout, cin}, x.device());
+        ck(gemm(dy.data_ptr(), x.data_ptr(), sink ? sink->acc : fptr(dw32), cout, cin, m, cout, cin, cin, true, true, 2,
+                wgrad_splits(m, cout, cin), nullptr, nullptr, nullptr, 0, x), "1x1 convolution weight gradient");
+        if (!sink) dw = dw32.to(w.scalar_type()).view(w.sizes());
+      } else if (kind == kGeneral) {
+        Tensor dw32;
+        if (!sink) dw32 = zeros_f32({cout, r, s, cin}, x.device());
+        float* acc = sink ? sink->acc : fptr(dw32);
+        int rc = -100;
+        if (stride == 1)         // shared input boxes, taps as shifted views (returns -100 outside its range)
+          rc = esgd_conv2d_wgrad_halo(x.data_ptr(), dy.data_ptr(), acc, n, h, wd, cin, cout, r, s, pad, flag_ptr(x), st);
+        if (rc == -100)
+          rc = esgd_conv2d_wgrad(x.data_ptr(), dy.data_ptr(), acc, n, h, wd, cin, cout, r, s, stride, pad, flag_ptr(x), st);
+        ck(rc, "conv2d weight gradient");
+        if (!sink) dw = dw32.to(w.scalar_type()).permute({0, 3, 1, 2});
+      } else {
+        const StemGeometry g(cin, r, s);
+        Tensor col = zeros_f32({cout, g.kpad}, x.device());
+        ck(gemm(dy.data_ptr(), x.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, 148, nullptr, nullptr,
+                nullptr, 0, x), "stem weight gradient");
+        if (!sink) dw = at::empty(w.sizes(), w.options(), kCL);
+        ck(esgd_stem_unpack(fptr(col), sink ? nullptr : dw.data_ptr(), sink ? sink->acc : nullptr, cout, r, s * cin, g.seg, g.kpad,
+                            st), "stem filter gradient");
+      }
+      if (sink) sink_done(sink);
+    }
+    none[0] = dx;
+    none[1] = dw;
+    return none;
+  }
+};
+
+// Returns (y, stats | None, tapped input | None), or None when the shape is not this package's.
+py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap, bool narrow) {
+  const int64_t c = x.size(1), k0 = w.size(0), r = w.size(2), s = w.size(3);
+  int64_t kind;
+  if (r == 1 && s == 1 && pad == 0 && stride <= 2 && c % 8 == 0 && k0 % 8 == 0) kind = kOneByOne;
+  else if (r > 1 && c <= 4 && k0 % 8 == 0 && !x.requires_grad()) kind = kStem;
+  else if (r > 1 && c % 8 == 0 && k0 % 8 == 0 && stride <= 2 && (narrow || c % 64 == 0)) kind = kGeneral;
+  else return py::none();
+  // only the 1x1 data gradient adds the shortcut's gradient in its epilogue: elsewhere the tap is the input itself
+  const bool fuse_tap = tap && kind == kOneByOne && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
+  Sink sink = find_sink(w);
+  sink_use(sink);
+  variable_list out = ConvFn::apply(x, w, kind, stride, pad, want_stats, fuse_tap, sink);
+  py::object st = want_stats ? py::cast(out[1]) : py::none();
+  py::object tp = !tap ? py::none() : py::cast(fuse_tap ? out.back() : x);
+  return py::make_tuple(out[0], st, tp);
+}
+
+// ---------------------------------------------------------------- dense layer: fp32 logits out of bf16 operands
+struct LinearFn : public Function<LinearFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w_in, const c10::optional<Tensor>& b_in,
+                        const Sink& ws, const Sink& bs) {
+    const Tensor b = b_in.has_value() ? *b_in : Tensor();
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = x_in.contiguous(), w = w_in.contiguous();
+    const int64_t m = x.size(0), k = x.size(1), n = w.size(0), np = (n + 7) / 8 * 8;
+    Tensor y = at::empty({m, np}, x.options().dtype(at::kFloat));
+    Tensor bias = b.defined() ? b.contiguous() : Tensor();
+    if (bias.defined() && (bias.scalar_type() != at::kBFloat16 || ((uintptr_t)bias.data_ptr() & 7))) bias = bias.to(at::kFloat).clone();
+    ck(gemm(x.data_ptr(), w.data_ptr(), y.data_ptr(), m, n, k, k, k, np, false, false, 1, 1, nullptr, nullptr, nullptr, 0, x,
+            bias.defined() ? bias.data_ptr() : nullptr, bias.defined() && bias.scalar_type() == at::kBFloat16 ? 2 : 0), "dense layer");
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["bias"] = b.defined() ? (int64_t)b.scalar_type() : (int64_t)-1;
+    save_sink(ctx, "w", ws);
+    save_sink(ctx, "b", bs);
+    return n == np ? y : y.narrow(1, 0, n);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t m = x.size(0), k = x.size(1), n = w.size(0), np = (n + 7) / 8 * 8;
+    Sink ws = load_sink(ctx, "w"), bs = load_sink(ctx, "b");
+    Tensor dy = grads[0];
+    if (dy.scalar_type() != at::kFloat) dy = dy.to(at::kFloat);
+    if (dy.stride(1) != 1 || (dy.stride(0) < n && m > 1)) dy = dy.contiguous();
+    const int64_t bias_type = ctx->saved_data["bias"].toInt();
+    const bool need_b = bias_type >= 0 && ctx->needs_input_grad(2);
+    Tensor db32;
+    if (need_b && !bs) db32 = zeros_f32({n}, x.device());
+    Tensor dy16 = at::empty({m, np}, x.options());
+    ck(esgd_cast_colsum(dy.data_ptr<float>(), dy.stride(0), m, n, np, dy16.data_ptr(), !need_b ? nullptr : (bs ? bs->acc : fptr(db32)),
+                        stream_of(x)), "dense layer gradient");
+    Tensor dx, dw, db;
+    if (ctx->needs_input_grad(0)) {
+      dx = at::empty({m, k}, x.options());
+      ck(gemm(dy16.data_ptr(), w.data_ptr(), dx.data_ptr(), m, k, n, np, k, k, false, true, 0, 1, nullptr, nullptr, nullptr, 0, x),
+         "dense layer data gradient");
+    }
+    if (ctx->needs_input_grad(1)) {
+      if (!ws) dw = at::empty({n, k}, w.options());
+      ck(gemm(dy16.data_ptr(), x.data_ptr(), ws ? (void*)ws->acc : dw.data_ptr(), n, k, m, np, k, k, true, true, ws ? 2 : 0, 1, nullptr,
+              nullptr, nullptr, 0, x), "dense layer weight gradient");
+      if (ws) sink_done(ws);
+    }
+    if (need_b) {
+      if (bs) sink_done(bs);
+      else db = db32.to((at::ScalarType)bias_type, false, true);
+    }
+    return {dx, dw, db, Tensor(), Tensor()};
+  }
+};
+
+// None when the shape is not this package's.
+py::object linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& b) {
+  if (x.size(1) % 8 || w.scalar_type() != at::kBFloat16) return py::none();
+  Tensor bias = b.has_value() ? *b : Tensor();
+  Sink ws = find_sink(w), bs = find_sink(bias);
+  sink_use(ws);
+  sink_use(bs);
+  return py::cast(LinearFn::apply(x, w, b, ws, bs));
+}
+
+// ---------------------------------------------------------------- batch norm (+ residual) (+ ReLU)
+struct BnActFn : public Function<BnActFn> {
+  using Opt = c10::optional<Tensor>;
+  static Tensor forward(AutogradContext* ctx, const Tensor& y_in, const Tensor& gamma, const Tensor& beta, const Opt& res_in,
+                        const Opt& rm_in, const Opt& rv_in, double momentum, bool relu, const Opt& stats_in, const Sink& gs,
+                        const Sink& bs) {
+    c10::cuda::CUDAGuard guard(y_in.device());
+    auto get = [](const Opt& o) { return o.has_value() ? *o : Tensor(); };
+    Tensor y = nhwc(y_in), res = res_in.has_value() ? nhwc(*res_in) : Tensor(), stats = get(stats_in), rm = get(rm_in), rv = get(rv_in);
+    const int64_t n = y.size(0), c = y.size(1), m = n * y.size(2) * y.size(3);
+    void* st = stream_of(y);
+    if (!stats.defined()) {
+      stats = zeros_f32({2, c}, y.device());
+      ck(esgd_bn_stats(y.data_ptr(), m, c, fptr(stats), fptr(stats) + c, st), "bn_stats");
+    }
+    Tensor aux = at::empty({4, c}, gamma.options());       // mean, invstd, scale, shift
+    Tensor z = empty_nhwc(n, c, y.size(2), y.size(3), y);
+    ck(esgd_bn_fwd(y.data_ptr(), res.defined() ? res.data_ptr() : nullptr, z.data_ptr(), fptr(stats), fptr(stats) + c, fptr(gamma),
+                   fptr(beta), fptr(rm), fptr(rv), fptr(aux), m, c, relu, (float)momentum, kBnEps, st), "bn_fwd");
+    // ReLU mask of the backward pass: from the saved output when a residual was added, else recomputed from y
+    const int64_t mode = !relu ? 0 : (res.defined() ? 1 : 2);
+    ctx->save_for_backward({y, mode == 1 ? z : Tensor(), gamma, aux});
+    ctx->saved_data["mode"] = mode;
+    ctx->saved_data["res"] = res.defined();
+    save_sink(ctx, "g", gs);
+    save_sink(ctx, "b", bs);
+    return z;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &y = saved[0], &z = saved[1], &gamma = saved[2], &aux = saved[3];
+    c10::cuda::CUDAGuard guard(y.device());
+    const int64_t mode = ctx->saved_data["mode"].toInt(), c = y.size(1), m = y.numel() / c;
+    const bool has_res = ctx->saved_data["res"].toBool();
+    Sink gs = load_sink(ctx, "g"), bs = load_sink(ctx, "b");
+    Tensor dz = nhwc(grads[0]);
+    void* st = stream_of(y);
+    // dbeta, dgamma; handed to autograd unless both go to sinks, so then not from the step's scratch
+    Tensor red = gs && bs ? zeros_f32({2, c}, y.device()) : at::zeros({2, c}, aux.options());
+    float *a = fptr(aux), *rd = fptr(red);
+    const void* zp = z.defined() ? z.data_ptr() : nullptr;
+    ck(esgd_bn_bwd_reduce(dz.data_ptr(), zp, y.data_ptr(), a, a + c, a + 2 * c, a + 3 * c, m, c, (int)mode, rd, rd + c, st),
+       "bn_bwd_reduce");
+    Tensor dy = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y), dres;
+    if (has_res) dres = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y);
+    ck(esgd_bn_bwd_apply(dz.data_ptr(), zp, y.data_ptr(), a, a + c, fptr(gamma), rd, rd + c, a + 2 * c, a + 3 * c, dy.data_ptr(),
+                         has_res ? dres.data_ptr() : nullptr, m, c, (int)mode, gs ? gs->acc : nullptr, bs ? bs->acc : nullptr, st),
+       "bn_bwd_apply");
+    Tensor dgamma, dbeta;
+    if (gs) sink_done(gs);
+    else dgamma = red.select(0, 1);
+    if (bs) sink_done(bs);
+    else dbeta = red.select(0, 0);
+    variable_list out(11);
+    out[0] = dy; out[1] = dgamma; out[2] = dbeta; out[3] = dres;
+    return out;
+  }
+};
+
+Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& res,
+              const c10::optional<Tensor>& rm, const c10::optional<Tensor>& rv, double momentum, bool relu,
+              const c10::optional<Tensor>& stats) {
+  Sink gs = find_sink(gamma), bs = find_sink(beta);
+  sink_use(gs);
+  sink_use(bs);
+  return BnActFn::apply(y, gamma, beta, res, rm, rv, momentum, relu, stats, gs, bs);
+}
+
+// ---------------------------------------------------------------- softmax cross-entropy
+struct SoftmaxCEFn : public Function<SoftmaxCEFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& logits_in, const Tensor& labels) {
+    c10::cuda::CUDAGuard guard(logits_in.device());
+    Tensor logits = logits_in.stride(1) == 1 && logits_in.stride(0) >= logits_in.size(1) ? logits_in : logits_in.contiguous();
+    const int64_t b = logits.size(0), c = logits.size(1);
+    Tensor loss = at::zeros({}, logits.options().dtype(at::kFloat));
+    Tensor d = at::empty_strided({b, c}, {logits.stride(0), 1}, logits.options());
+    ck(esgd_softmax_ce(logits.data_ptr(), logits.scalar_type() == at::kBFloat16, labels.contiguous().data_ptr<int64_t>(), b, c,
+                       logits.stride(0), 1.0f / (float)b, fptr(loss), nullptr, d.data_ptr(), stream_of(logits)), "softmax_ce");
+    ctx->save_for_backward({d});
+    return loss;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) { return {ctx->get_saved_variables()[0] * grads[0], Tensor()}; }
+};
+Tensor softmax_ce(const Tensor& logits, const Tensor& labels) { return SoftmaxCEFn::apply(logits, labels); }
+
+// ---------------------------------------------------------------- pooling
+struct MaxPoolFn : public Function<MaxPoolFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_in) {
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = nhwc(x_in);
+    const int64_t n = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3), oh = (h + 1) / 2, ow = (w + 1) / 2;
+    Tensor y = empty_nhwc(n, c, oh, ow, x);
+    Tensor idx;
+    if (x_in.requires_grad()) idx = at::empty({n * oh * ow, c}, x.options().dtype(at::kByte));
+    ck(esgd_maxpool3x3s2_fwd(x.data_ptr(), y.data_ptr(), idx.defined() ? idx.data_ptr() : nullptr, n, h, w, c, stream_of(x)), "maxpool");
+    if (idx.defined()) ctx->save_for_backward({idx});
+    ctx->saved_data["dims"] = std::vector<int64_t>{n, c, h, w};
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto d = ctx->saved_data["dims"].toIntVector();
+    const Tensor idx = ctx->get_saved_variables()[0];
+    Tensor dy = nhwc(grads[0]);
+    c10::cuda::CUDAGuard guard(dy.device());
+    Tensor dx = empty_nhwc(d[0], d[1], d[2], d[3], dy);
+    ck(esgd_maxpool3x3s2_bwd(idx.data_ptr(), dy.data_ptr(), dx.data_ptr(), d[0], d[2], d[3], d[1], stream_of(dy)), "maxpool backward");
+    return {dx};
+  }
+};
+Tensor max_pool(const Tensor& x) { return MaxPoolFn::apply(x); }
+
+struct AvgPoolFn : public Function<AvgPoolFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_in) {
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = nhwc(x_in);
+    const int64_t n = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3);
+    Tensor y = at::empty({n, c}, x.options());
+    ck(esgd_avgpool_fwd(x.data_ptr(), y.data_ptr(), n, h * w, c, stream_of(x)), "avgpool");
+    ctx->saved_data["dims"] = std::vector<int64_t>{n, c, h, w};
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto d = ctx->saved_data["dims"].toIntVector();
+    Tensor dy = grads[0].contiguous();
+    c10::cuda::CUDAGuard guard(dy.device());
+    Tensor dx = empty_nhwc(d[0], d[1], d[2], d[3], dy);
+    ck(esgd_avgpool_bwd(dy.data_ptr(), dx.data_ptr(), d[0], d[2] * d[3], d[1], stream_of(dy)), "avgpool backward");
+    return {dx};
+  }
+};
+Tensor avg_pool(const Tensor& x) { return AvgPoolFn::apply(x); }
+
+}  // namespace
+
+PYBIND11_MODULE(_esgd_torch, m) {
+  m.doc() = "autograd operators over the sm_100a kernels of eagersgd_b200";
+  m.def("error_flag", &error_flag);
+  m.def("zeros_f32", [](std::vector<int64_t> shape, at::Device d) { return zeros_f32(shape, d); });
+  m.def("wgrad_splits", &wgrad_splits, py::arg("pixels"), py::arg("cout"), py::arg("cin"), py::arg("sms") = 148);
+  m.def("conv2d", &conv2d);
+  m.def("linear", &linear);
+  m.def("bn_act", &bn_act);
+  m.def("softmax_ce", &softmax_ce);
+  m.def("max_pool", &max_pool);
+  m.def("avg_pool", &avg_pool);
+  py::class_<ZeroArena, std::shared_ptr<ZeroArena>>(m, "ZeroArena")
+      .def(py::init<>())
+      .def("begin", &ZeroArena::begin)
+      .def("end", &ZeroArena::end);
+  py::class_<GradSinks, std::shared_ptr<GradSinks>>(m, "GradSinks")
+      .def(py::init<std::vector<int>, py::function>())
+      .def("add", &GradSinks::add)
+      .def("begin_step", &GradSinks::begin_step)
+      .def("clear_written", &GradSinks::clear_written)
+      .def("set_active", &GradSinks::set_active)
+      .def("active", &GradSinks::active)
+      .def("used", &GradSinks::used)
+      .def("written", &GradSinks::written)
+      .def("param_done", &GradSinks::param_done)
+      .def("close", &GradSinks::close);
+}

@@ -16,9 +16,8 @@ from typing import Optional
 
 import torch
 
+from .. import _build
 from ..parallel import _native as N
-
-_err_flags = {}
 
 
 def _lib():
@@ -32,10 +31,7 @@ def _lib():
 
 def error_flag(device: torch.device) -> torch.Tensor:
     """Per-device int32 word the tensor-core kernels raise when a bounded wait runs out."""
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    if key not in _err_flags:
-        _err_flags[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _err_flags[key]
+    return _build.load_torch().error_flag(device.index if device.index is not None else torch.cuda.current_device())
 
 
 def check_error(device: torch.device) -> None:

@@ -12,6 +12,8 @@ when the wrapped optimizer is ``torch.optim.SGD``.
 """
 from __future__ import annotations
 
+import contextlib
+import weakref
 from typing import Dict, List, Optional
 
 import numpy as np
@@ -42,6 +44,8 @@ class _Bucket:
         self.hyper_vals = None
         self.self_clearing = False
         self.dirty = True
+        self.acc32 = None           # fp32 accumulators that operators add parameter gradients to (see grad_sinks)
+        self.touched: List = []     # (parameter, offset) pairs whose .grad autograd has written since the last launch
 
     def add(self, p):
         self.params.append(p)
@@ -104,6 +108,7 @@ class EagerOptimizer:
         self.slot_dtype = slot_dtype
         self._build_buckets(bucket_mb)
         self._hooks = []
+        self._sinks, self._sinks_proven, self._sinks_conflict = None, False, False
         if self.on_gpu:
             self._setup_gpu()
             self._install_hooks()
@@ -297,30 +302,88 @@ class EagerOptimizer:
     def _install_hooks(self):
         for b in self.buckets:
             b.pending = len(b.params)
-            for p in b.params:
-                self._hooks.append(p.register_post_accumulate_grad_hook(self._make_hook(b)))
+            for p, off in zip(b.params, b.offsets):
+                self._hooks.append(p.register_post_accumulate_grad_hook(self._make_hook(b, off)))
 
-    def _make_hook(self, b: _Bucket):
+    def _make_hook(self, b: _Bucket, off: int):
         def hook(p):
             b.dirty = True
+            b.touched.append((p, off))
+            if self._sinks is not None and self._sinks.active():
+                if self._sinks.used(p):          # one parameter, two routes: see grad_sinks
+                    self._sinks_conflict = True
+                self._sinks.param_done(b.index)
+                return
             b.pending -= 1
             if b.pending == 0 and self.overlap:
-                self._launch(b)
+                self._launch(b, b.touched)
         return hook
 
-    def _launch(self, b: _Bucket):
-        """Start the bucket's partial allreduce on the side stream, behind backward."""
+    def _launch(self, b: _Bucket, written=None):
+        """Start the bucket's partial allreduce on the side stream, behind backward.  ``written``: the (parameter, offset)
+        pairs whose ``.grad`` may not be the bucket's own storage (default: all)."""
         if b.launched:
             return
-        for p, off in zip(b.params, b.offsets):  # a foreign .grad (zero_grad(set_to_none)) is copied back in
+        for p, off in (zip(b.params, b.offsets) if written is None else written):
+            # a foreign .grad (zero_grad(set_to_none)) is copied back in
             if p.grad is not None and p.grad.data_ptr() != b.grad_flat.data_ptr() + off * b.grad_flat.element_size():
                 _view_like(b.grad_flat, off, p).copy_(p.grad)
                 p.grad = _view_like(b.grad_flat, off, p)
+        src = N.SRC_FLAT
+        if b.acc32 is not None and b.acc32 is not b.grad_flat and self._sinks.written(b.index):
+            src = N.SRC_FLAT | N.SRC_ACC if b.dirty else N.SRC_ACC
         self._refresh_hyper(b)
         self.comm_stream.wait_stream(torch.cuda.current_stream(self.device))
         with nvtx_range("partial_allreduce"):
-            b.channel.step(self.comm_stream)
+            b.channel.step(self.comm_stream, src)
         b.launched = True
+
+    @contextlib.contextmanager
+    def grad_sinks(self):
+        """Around the forward and backward pass of a training step: operators of this package add the gradients of their
+        parameters straight to fp32 accumulators of the buckets (``csrc/torch/ops.cpp``) instead of returning them to
+        autograd, so those parameters' ``.grad`` stays zero and is not to be looked at before ``step()``.  Parameters that
+        carry hooks of the user's own are left to autograd."""
+        if not self.prepare_grad_sinks():
+            yield
+            return
+        s = self._sinks
+        s.begin_step()
+        s.set_active(True)
+        try:
+            yield
+        finally:
+            s.set_active(False)
+
+    def prepare_grad_sinks(self) -> bool:
+        """Set the accumulators of ``grad_sinks`` up if they are not yet; False where they cannot be used."""
+        if not self.on_gpu or self._sinks_conflict:
+            return False
+        for b in self.buckets:
+            for p in b.params:
+                if p._backward_hooks or len(p._post_accumulate_grad_hooks or ()) != 1 or not p.requires_grad:
+                    return False
+        if self._sinks is None:
+            from .. import _build
+            weak = weakref.ref(self)
+
+            def on_bucket(i):
+                me = weak()
+                # A parameter that is also used outside this package's operators would get the rest of its gradient from
+                # autograd after its bucket has gone: the first step launches nothing early and finds such parameters out.
+                if me is not None and me.overlap and me._sinks_proven:
+                    me._launch(me.buckets[i], me.buckets[i].touched)
+
+            self._sinks = _build.load_torch().GradSinks([len(b.params) for b in self.buckets], on_bucket)
+            for b in self.buckets:
+                if b.grad_flat.dtype == torch.float32:
+                    b.acc32 = b.grad_flat
+                else:
+                    b.acc32 = torch.zeros(b.count, dtype=torch.float32, device=self.device)
+                    b.channel.set_grad_acc(b.acc32)
+                for p, off in zip(b.params, b.offsets):
+                    self._sinks.add(p, b.acc32[off:off + p.numel()], b.index)
+        return True
 
     # ------------------------------------------------------------------ API
     @property
@@ -332,12 +395,17 @@ class EagerOptimizer:
         the reduce kernel clears a bucket behind its copy into the publish slot, so after ``step()`` there
         is nothing left to do here; a fill is launched only for a bucket that backward has written since."""
         for b in self.buckets:
-            if not (self.on_gpu and getattr(b, "self_clearing", False) and not b.dirty):
+            written = self._sinks is not None and self._sinks.written(b.index)   # a backward pass that no step followed
+            if written and b.acc32 is not b.grad_flat:
+                b.acc32.zero_()
+            if written or not (self.on_gpu and getattr(b, "self_clearing", False) and not b.dirty):
                 b.grad_flat.zero_()
                 if self.on_gpu:
                     b.dirty = False
             if any(p.grad is None for p in b.params):
                 self._point_grads(b)
+        if self._sinks is not None:
+            self._sinks.clear_written()
 
     def step(self, closure=None):
         loss = closure() if closure is not None else None
@@ -349,7 +417,12 @@ class EagerOptimizer:
             for b in self.buckets:
                 b.launched = False
                 b.pending = len(b.params)
+                # what the step read it has cleared; an fp32 bucket may also have been written without a hook
                 b.dirty = not b.self_clearing
+                b.touched = []
+            if self._sinks is not None:
+                self._sinks.clear_written()
+                self._sinks_proven = not self._sinks_conflict
             if not self.fused:
                 self._inner_step()
         else:
@@ -369,10 +442,11 @@ class EagerOptimizer:
         """Step the wrapped optimizer with the averaged gradients the kernels wrote — unless no bucket had
         anything to apply (the rank missed the round and its mailbox was empty, or a bounded wait ran out):
         then momentum and weight decay must not move the weights either, as on the CPU path and in the
-        fused kernel.  Reading the flags synchronises with the device; inside stream capture the step is
+        fused kernel.  Reading the flags synchronises with the device (a single rank misses no round and
+        is not asked); inside stream capture the step is
         recorded unconditionally."""
         if not torch.cuda.is_current_stream_capturing():
-            if not any(b.channel.applied() for b in self.buckets):
+            if not any(b.channel.world == 1 or b.channel.applied() for b in self.buckets):
                 return
         if self.lars:
             return self._lars_step()
@@ -501,6 +575,8 @@ class EagerOptimizer:
         for h in self._hooks:
             h.remove()
         self._hooks = []
+        if self._sinks is not None:
+            self._sinks.close()
         if self.on_gpu:
             torch.cuda.synchronize(self.device)
             self.group.barrier()

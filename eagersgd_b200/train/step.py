@@ -82,8 +82,9 @@ class TrainStep:
             self.opt = cls(inner, group, **kw)
             self.opt.grad_scale = 1.0 / self.loss_scale   # static loss scaling is undone inside the update
             self.autocast = False
-        n_params = sum(p.numel() for p in self.net.parameters())
-        self._arena_numel = n_params + 64 * (len(list(self.net.parameters())) + 8) + (1 << 20)
+        # the operators' zeroed scratch of a step; parameter gradients go to the buckets' own accumulators where they can
+        self._arena = None
+        self._arena_numel = 1 << 20
         self._xbuf = self._ybuf = None
         self._graph = None
         self.graph_kernel_launches = 0
@@ -111,6 +112,7 @@ class TrainStep:
             raise NotImplementedError("only the fused momentum-SGD path can be captured in a CUDA graph; "
                                       "run a wrapped optimizer without capture")
         self._gx, self._gy = x.clone(), y.clone()
+        self.opt.prepare_grad_sinks()        # allocates and synchronises: not inside the capture
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(side):
@@ -147,10 +149,15 @@ class TrainStep:
             loss.backward()
             self.opt.step()
             return loss.detach()
-        from ..ops.functional import zero_arena
-        # every operator's zeroed fp32 scratch (statistics, weight-gradient accumulators) comes out of one
-        # buffer cleared by a single memset per step
-        with zero_arena(self.device, self._arena_numel) if self.device.type == "cuda" else contextlib.nullcontext():
+        # every operator's zeroed fp32 scratch (statistics, reductions) comes out of one buffer of this object's, cleared
+        # by a single memset per step; parameter gradients are added straight to the optimizer's buckets
+        with contextlib.ExitStack() as scope:
+            if self.device.type == "cuda":
+                from ..ops.functional import new_zero_arena, zero_arena
+                if self._arena is None:
+                    self._arena = new_zero_arena()
+                scope.enter_context(zero_arena(self.device, self._arena_numel, self._arena))
+                scope.enter_context(self.opt.grad_sinks())
             with nvtx_range("forward"):
                 logits = self.net(x if x.dtype == self.compute_dtype or not x.is_floating_point()
                                   else x.to(self.compute_dtype))
