@@ -260,16 +260,6 @@ int splits_for(int m, int k) {
 
 extern "C" {
 
-int esgd_lstm_cell_fwd(const void* xproj, const float* hprojT, const float* bias, const float* c_prev, float* c_out,
-                       void* h_out, void* gates, int B, int H, int ldh, void* stream) {
-  return cell_fwd(xproj, const_cast<float*>(hprojT), bias, c_prev, c_out, h_out, gates, B, H, ldh, 0, stream);
-}
-
-int esgd_lstm_cell_bwd(const void* gates, const float* c_prev, const float* c_cur, const void* dh_ext,
-                       const float* dh_recT, float* dc, void* dgates, int B, int H, int ldr, void* stream) {
-  return cell_bwd(gates, c_prev, c_cur, dh_ext, const_cast<float*>(dh_recT), dc, dgates, B, H, ldr, 0, stream);
-}
-
 // ---- whole sequences: the time loop runs here, not in Python ----------------------------------------------------
 // One call per layer and direction issues every launch of the recurrence (per step: the swapped recurrent GEMM
 // on the tensor cores and the fused cell kernel), so the GPU never waits for an interpreter between steps.

@@ -50,6 +50,16 @@ int esgd_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W
 int esgd_maxpool3x3s2_bwd(const void* idx, const void* dy, void* dx, int N, int H, int W, int C, void* stream);
 int esgd_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream);
 int esgd_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, void* stream);
+int esgd_lstm_persistent_ok(int B, int H, int backward);
+int esgd_lstm_persistent_scratch(void);
+int esgd_lstm_persistent_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates, void* scratch,
+                             int T, int B, int H, int* error_flag, void* stream);
+int esgd_lstm_persistent_bwd(const void* gates, const float* c, const void* dy, const void* w_hh, void* dG, float* db, void* scratch,
+                             int T, int B, int H, int* error_flag, void* stream);
+int esgd_lstm_seq_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates, float* hprojT, int T,
+                      int B, int H, int* error_flag, void* stream);
+int esgd_lstm_seq_bwd(const void* gates, const float* c, const void* dy, const void* w_hh, void* dG, float* dc, float* dh_recT, int T,
+                      int B, int H, int* error_flag, void* stream);
 int esgd_cast_colsum(const float* dy, int64_t ld, int M, int N, int np, void* out, float* colsum, void* stream);
 }
 
@@ -626,6 +636,120 @@ struct AvgPoolFn : public Function<AvgPoolFn> {
 };
 Tensor avg_pool(const Tensor& x) { return AvgPoolFn::apply(x); }
 
+// ---------------------------------------------------------------- LSTM layer
+// x . W_ih^T of all steps is one GEMM; the recurrence is one persistent kernel per direction where the shape allows it
+// (weights resident on the chip), else a native loop of split-K GEMMs and cell kernels; the weight and input gradients are
+// single GEMMs over all steps.
+struct LstmFn : public Function<LstmFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w_ih_in, const Tensor& w_hh_in, const Tensor& bias,
+                        const Sink& s_ih, const Sink& s_hh, const Sink& s_b) {
+    c10::cuda::CUDAGuard guard(x_in.device());
+    Tensor x = x_in.contiguous(), w_ih = w_ih_in.contiguous(), w_hh = w_hh_in.contiguous();
+    const int64_t t = x.size(0), b = x.size(1), in = x.size(2), h = w_hh.size(1);
+    void* st = stream_of(x);
+    const auto f32 = x.options().dtype(at::kFloat);
+    Tensor xproj = at::empty({t * b, 4 * h}, x.options());
+    ck(gemm(x.data_ptr(), w_ih.data_ptr(), xproj.data_ptr(), t * b, 4 * h, in, in, in, 4 * h, false, false, 0, 1, nullptr, nullptr,
+            nullptr, 0, x), "lstm input projection");
+    Tensor y = at::empty({t, b, h}, x.options()), c = at::empty({t, b, h}, f32), gates = at::empty({t, b, 4 * h}, x.options());
+    if (esgd_lstm_persistent_ok((int)b, (int)h, 0)) {
+      Tensor scratch = at::empty({esgd_lstm_persistent_scratch()}, f32);
+      ck(esgd_lstm_persistent_fwd(xproj.data_ptr(), w_hh.data_ptr(), fptr(bias), fptr(c), y.data_ptr(), gates.data_ptr(),
+                                  scratch.data_ptr(), t, b, h, flag_ptr(x), st), "lstm forward recurrence");
+    } else {
+      Tensor hproj = at::empty({4 * h, b}, f32);
+      ck(esgd_lstm_seq_fwd(xproj.data_ptr(), w_hh.data_ptr(), fptr(bias), fptr(c), y.data_ptr(), gates.data_ptr(), fptr(hproj), t, b, h,
+                           flag_ptr(x), st), "lstm forward recurrence");
+    }
+    ctx->save_for_backward({x, w_ih, w_hh, y, c, gates});
+    save_sink(ctx, "ih", s_ih);
+    save_sink(ctx, "hh", s_hh);
+    save_sink(ctx, "b", s_b);
+    return y;
+  }
+
+  // dw [m][n] = a^T b over `rows`, added to the sink's accumulator or returned in the weights' type.  The tiles of these
+  // gradients fill the GPU by themselves unless the layer is small: only then is the reduction split.
+  static Tensor weight_grad(const Sink& sink, const Tensor& a, const void* ap, const Tensor& w, const void* bp, int64_t rows, int64_t m,
+                            int64_t n) {
+    const int64_t bn = n <= 64 ? 64 : (n <= 128 ? 128 : 256), tiles = ((m + 127) / 128) * ((n + bn - 1) / bn);
+    const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(148 / tiles, rows / 512));
+    Tensor dw;
+    if (sink || splits > 1) {
+      if (!sink) dw = at::zeros({m, n}, w.options().dtype(at::kFloat));
+      ck(gemm(ap, bp, sink ? sink->acc : fptr(dw), m, n, rows, m, n, n, true, true, 2, (int)splits, nullptr, nullptr, nullptr, 0, a),
+         "lstm weight gradient");
+      return sink ? Tensor() : dw.to(w.scalar_type());
+    }
+    dw = at::empty({m, n}, w.options());
+    ck(gemm(ap, bp, dw.data_ptr(), m, n, rows, m, n, n, true, true, 0, 1, nullptr, nullptr, nullptr, 0, a), "lstm weight gradient");
+    return dw;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w_ih = saved[1], &w_hh = saved[2], &y = saved[3], &c = saved[4], &gates = saved[5];
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t t = x.size(0), b = x.size(1), in = x.size(2), h = w_hh.size(1);
+    Sink s_ih = load_sink(ctx, "ih"), s_hh = load_sink(ctx, "hh"), s_b = load_sink(ctx, "b");
+    const auto f32 = x.options().dtype(at::kFloat);
+    void* st = stream_of(x);
+    Tensor dy = grads[0].contiguous();
+    Tensor dG = at::empty({t * b, 4 * h}, x.options());
+    Tensor dx, dw_ih, dw_hh, db;
+    const bool need_b = ctx->needs_input_grad(3);
+    if (esgd_lstm_persistent_ok((int)b, (int)h, 1)) {
+      Tensor scratch = at::empty({esgd_lstm_persistent_scratch()}, f32);
+      if (need_b && !s_b) db = at::zeros({4 * h}, f32);
+      ck(esgd_lstm_persistent_bwd(gates.data_ptr(), fptr(c), dy.data_ptr(), w_hh.data_ptr(), dG.data_ptr(),
+                                  !need_b ? nullptr : (s_b ? s_b->acc : fptr(db)), scratch.data_ptr(), t, b, h, flag_ptr(x), st),
+         "lstm backward recurrence");
+    } else {
+      Tensor dc = at::empty({b, h}, f32), dh = at::empty({h, b}, f32);
+      ck(esgd_lstm_seq_bwd(gates.data_ptr(), fptr(c), dy.data_ptr(), w_hh.data_ptr(), dG.data_ptr(), fptr(dc), fptr(dh), t, b, h,
+                           flag_ptr(x), st), "lstm backward recurrence");
+      if (need_b) {
+        db = dG.sum(0, false, at::kFloat);
+        if (s_b) {
+          at::from_blob(s_b->acc, {4 * h}, f32).add_(db);
+          db = Tensor();
+        }
+      }
+    }
+    if (need_b && s_b) sink_done(s_b);
+    if (ctx->needs_input_grad(0)) {
+      dx = at::empty({t, b, in}, x.options());
+      ck(gemm(dG.data_ptr(), w_ih.data_ptr(), dx.data_ptr(), t * b, in, 4 * h, 4 * h, in, in, false, true, 0, 1, nullptr, nullptr,
+              nullptr, 0, x), "lstm input gradient");
+    }
+    if (ctx->needs_input_grad(1)) {
+      dw_ih = weight_grad(s_ih, x, dG.data_ptr(), w_ih, x.data_ptr(), t * b, 4 * h, in);
+      if (s_ih) sink_done(s_ih);
+    }
+    if (ctx->needs_input_grad(2)) {
+      if (t > 1)
+        dw_hh = weight_grad(s_hh, x, (const char*)dG.data_ptr() + b * 4 * h * 2, w_hh, y.data_ptr(), (t - 1) * b, 4 * h, h);
+      else if (!s_hh)
+        dw_hh = at::zeros_like(w_hh);
+      if (s_hh) sink_done(s_hh);
+    }
+    variable_list out(7);
+    out[0] = dx; out[1] = dw_ih; out[2] = dw_hh; out[3] = db;
+    return out;
+  }
+};
+
+// x [T, B, I] bf16, weights [4H, I] / [4H, H] bf16, bias [4H] fp32 -> h [T, B, H]; T, B, I, H multiples of 8 except T.
+Tensor lstm_layer(const Tensor& x, const Tensor& w_ih, const Tensor& w_hh, const Tensor& bias) {
+  TORCH_CHECK(w_ih.scalar_type() == at::kBFloat16 && w_hh.scalar_type() == at::kBFloat16 && bias.scalar_type() == at::kFloat &&
+              bias.is_contiguous(), "lstm_layer takes bf16 weights and an fp32 bias");
+  Sink s_ih = find_sink(w_ih), s_hh = find_sink(w_hh), s_b = find_sink(bias);
+  sink_use(s_ih);
+  sink_use(s_hh);
+  sink_use(s_b);
+  return LstmFn::apply(x, w_ih, w_hh, bias, s_ih, s_hh, s_b);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_esgd_torch, m) {
@@ -637,6 +761,7 @@ PYBIND11_MODULE(_esgd_torch, m) {
   m.def("linear", &linear);
   m.def("bn_act", &bn_act);
   m.def("softmax_ce", &softmax_ce);
+  m.def("lstm_layer", &lstm_layer);
   m.def("max_pool", &max_pool);
   m.def("avg_pool", &avg_pool);
   py::class_<ZeroArena, std::shared_ptr<ZeroArena>>(m, "ZeroArena")

@@ -1,17 +1,11 @@
-"""LSTM layer on the hand-written kernels: tensor-core projections + fused cell kernels.
+"""LSTM layer on the hand-written kernels: tensor-core projections + a persistent recurrence.
 
 * ``x . W_ih^T`` for every time step is ONE tcgen05 GEMM ([T*B, I] x [4H, I]^T).
-* Per time step the recurrent product runs in swapped form ``W_hh . h_{t-1}^T -> [4H, B]`` so the
-  4H dimension fills the 128-row MMA tile and the small batch is the N dimension; the fused cell
-  kernel adds it to the input projection, applies the gates and updates c and h.
-* Backward keeps only the ``dh`` recurrence sequential (one swapped GEMM + one fused kernel per
-  step); the three weight/input gradients are single large GEMMs over all time steps (split-K).
-* The time loop is native: ``esgd_lstm_seq_fwd`` / ``esgd_lstm_seq_bwd`` issue every launch of a layer's
-  recurrence from C++.  The recurrent GEMMs are split over K so that about every SM has a tile (their fp32
-  partial sums meet by atomics; the cell kernel zeroes each element as it reads it), and all launches of the
-  loop form a chain of programmatic dependent launches, so a kernel is already resident when the one before
-  it ends.  Layer forward + backward at (T, B, H) = (16, 16, 2048): 0.72 ms against 1.26 ms for cuDNN;
-  (600, 16, 2048): 19.8 against 20.8 ms.
+* The recurrence is one kernel per direction that keeps the recurrent weights on chip for the whole sequence
+  (csrc/cuda/lstm_persistent.cu), for H a multiple of 128 up to 2048 and batches up to 32; other shapes take a native
+  loop of split-K GEMMs and cell kernels (csrc/cuda/lstm_cell.cu).
+* The three weight / input gradients are single large GEMMs over all time steps.
+* The autograd function around them is C++ (csrc/torch/ops.cpp).
 
 Stands where the reference calls ``torch.nn.LSTM`` (cuDNN) in its video classifier
 (deep500 samples/ucf101_resnetlstm.py:41-59).  Gate order i, f, g, o; weights are
@@ -19,82 +13,9 @@ Stands where the reference calls ``torch.nn.LSTM`` (cuDNN) in its video classifi
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
-from ..parallel import _native as N
-from .gemm import error_flag, gemm
-
-
-def _lib():
-    lib = N.cuda()
-    if not getattr(lib, "_lstm_bound", False):
-        vp, i32 = C.c_void_p, C.c_int
-        lib.esgd_lstm_cell_fwd.argtypes = [vp] * 7 + [i32, i32, i32, vp]
-        lib.esgd_lstm_cell_bwd.argtypes = [vp] * 7 + [i32, i32, i32, vp]
-        lib.esgd_lstm_seq_fwd.argtypes = [vp] * 7 + [i32, i32, i32, vp, vp]
-        lib.esgd_lstm_seq_bwd.argtypes = [vp] * 7 + [i32, i32, i32, vp, vp]
-        lib._lstm_bound = True
-    return lib
-
-
-def _ck(rc, what):
-    if rc != 0:
-        raise RuntimeError("%s failed with code %d" % (what, rc))
-
-
-class _LstmLayer(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w_ih, w_hh, bias):
-        T, B, I = x.shape
-        H = w_hh.shape[1]
-        lib = _lib()
-        s = torch.cuda.current_stream(x.device).cuda_stream
-        x2d = x.reshape(T * B, I)
-        xproj = gemm(x2d, w_ih)                                          # [T*B, 4H] bf16
-        y = torch.empty(T, B, H, dtype=torch.bfloat16, device=x.device)
-        c = torch.empty(T, B, H, dtype=torch.float32, device=x.device)
-        gates = torch.empty(T, B, 4 * H, dtype=torch.bfloat16, device=x.device)
-        hprojT = torch.empty(4 * H, B, dtype=torch.float32, device=x.device)
-        # every step's recurrent GEMM (W_hh . h^T : [4H, B] fp32) and cell kernel, issued by one native call
-        _ck(lib.esgd_lstm_seq_fwd(xproj.data_ptr(), w_hh.data_ptr(), bias.data_ptr(), c.data_ptr(), y.data_ptr(),
-                                  gates.data_ptr(), hprojT.data_ptr(), T, B, H, error_flag(x.device).data_ptr(), s),
-            "lstm forward recurrence")
-        ctx.save_for_backward(x2d, w_ih, w_hh, y, c, gates)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2d, w_ih, w_hh, y, c, gates = ctx.saved_tensors
-        T, B, H = y.shape
-        I = w_ih.shape[1]
-        lib = _lib()
-        s = torch.cuda.current_stream(dy.device).cuda_stream
-        dy = dy.contiguous()
-        dG = torch.empty(T, B, 4 * H, dtype=torch.bfloat16, device=dy.device)
-        dc = torch.empty(B, H, dtype=torch.float32, device=dy.device)
-        dh_recT = torch.empty(H, B, dtype=torch.float32, device=dy.device)
-        # per step one cell kernel and W_hh^T . dG_t^T : [H, B] fp32, issued by one native call
-        _ck(lib.esgd_lstm_seq_bwd(gates.data_ptr(), c.data_ptr(), dy.data_ptr(), w_hh.data_ptr(), dG.data_ptr(),
-                                  dc.data_ptr(), dh_recT.data_ptr(), T, B, H, error_flag(dy.device).data_ptr(), s),
-            "lstm backward recurrence")
-        dG2d = dG.view(T * B, 4 * H)
-        splits = max(2, min(64, (T * B) // 256))
-        dx = dw_ih = dw_hh = db = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dG2d, w_ih, b_kmajor=False).view(T, B, I)          # [T*B, 4H] x W_ih[4H(K), I]
-        if ctx.needs_input_grad[1]:
-            dw_ih = gemm(dG2d, x2d, a_kmajor=False, b_kmajor=False, splits=splits).to(w_ih.dtype)
-        if ctx.needs_input_grad[2]:
-            if T > 1:
-                dw_hh = gemm(dG2d[B:], y.view(T * B, H)[:-B], a_kmajor=False, b_kmajor=False,
-                             splits=splits).to(w_hh.dtype)
-            else:
-                dw_hh = torch.zeros_like(w_hh)
-        if ctx.needs_input_grad[3]:
-            db = dG2d.float().sum(0)
-        return dx, dw_ih, dw_hh, db
+from .. import _build
 
 
 def lstm_layer(x: torch.Tensor, w_ih: torch.Tensor, w_hh: torch.Tensor, bias: torch.Tensor) -> torch.Tensor:
@@ -102,7 +23,7 @@ def lstm_layer(x: torch.Tensor, w_ih: torch.Tensor, w_hh: torch.Tensor, bias: to
     T, B, I = x.shape
     H = w_hh.shape[1]
     if x.is_cuda and x.dtype == torch.bfloat16 and B % 8 == 0 and I % 8 == 0 and H % 8 == 0:
-        return _LstmLayer.apply(x.contiguous(), w_ih, w_hh, bias.float())
+        return _build.load_torch().lstm_layer(x.contiguous(), w_ih, w_hh, bias.float())
     return lstm_layer_reference(x, w_ih, w_hh, bias)
 
 
