@@ -18,6 +18,9 @@
 #include <stddef.h>
 #include <stdio.h>
 #include <string.h>
+#include <mutex>
+#include <utility>
+#include <vector>
 #include "partial_allreduce.cuh"
 #include "launch_count.cuh"
 
@@ -301,13 +304,43 @@ int esgd_collective_wait(void* h, void* stream) {
   return (int)e;
 }
 
-// Pinned, device-visible host memory for a channel's outcome.
-int esgd_host_alloc(uint64_t bytes, void** ptr) {
-  cudaError_t e = cudaHostAlloc(ptr, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
-  if (e == cudaSuccess) memset(*ptr, 0, bytes);
-  return (int)e;
+// Pinned, device-visible host memory for channels' outcomes, 64 bytes each.  Pinning a page takes the driver a millisecond
+// or two, so 64 slots share one; a page whose slots are all free again is given back unless it is the last one.
+static std::mutex g_outcome_mutex;
+static std::vector<std::pair<char*, uint64_t>> g_outcome_pages;    // base, bit mask of the slots in use
+
+int esgd_outcome_alloc(void** ptr) {
+  std::lock_guard<std::mutex> g(g_outcome_mutex);
+  for (auto& pg : g_outcome_pages)
+    if (~pg.second) {
+      const int slot = __builtin_ctzll(~pg.second);
+      pg.second |= 1ull << slot;
+      memset(*ptr = pg.first + 64 * slot, 0, 64);
+      return 0;
+    }
+  void* base = nullptr;
+  cudaError_t e = cudaHostAlloc(&base, 64 * 64, cudaHostAllocPortable | cudaHostAllocMapped);
+  if (e != cudaSuccess) return (int)e;
+  g_outcome_pages.emplace_back((char*)base, 1ull);
+  memset(*ptr = base, 0, 64);
+  return 0;
 }
-int esgd_host_free(void* ptr) { return (int)cudaFreeHost(ptr); }
+int esgd_outcome_free(void* ptr) {
+  std::lock_guard<std::mutex> g(g_outcome_mutex);
+  for (size_t i = 0; i < g_outcome_pages.size(); ++i) {
+    auto& pg = g_outcome_pages[i];
+    const ptrdiff_t off = (char*)ptr - pg.first;
+    if (off < 0 || off >= 64 * 64) continue;
+    pg.second &= ~(1ull << (off / 64));
+    if (pg.second == 0 && g_outcome_pages.size() > 1) {
+      char* base = pg.first;
+      g_outcome_pages.erase(g_outcome_pages.begin() + i);
+      return (int)cudaFreeHost(base);
+    }
+    return 0;
+  }
+  return -1;
+}
 
 int esgd_channel_flush(void* dch, uint64_t count, int max_blocks, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;

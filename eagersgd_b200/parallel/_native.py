@@ -121,8 +121,8 @@ def cuda():
         lib.esgd_collective_post.argtypes = [C.c_void_p, C.c_void_p]
         lib.esgd_collective_test.argtypes = [C.c_void_p]
         lib.esgd_collective_wait.argtypes = [C.c_void_p, C.c_void_p]
-        lib.esgd_host_alloc.argtypes = [C.c_uint64, C.POINTER(C.c_void_p)]
-        lib.esgd_host_free.argtypes = [C.c_void_p]
+        lib.esgd_outcome_alloc.argtypes = [C.POINTER(C.c_void_p)]
+        lib.esgd_outcome_free.argtypes = [C.c_void_p]
         lib.esgd_channel_applied.argtypes = [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]
         lib.esgd_channel_times.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
         lib.esgd_set_hyper.argtypes = [C.c_void_p, C.c_float, C.c_float, C.c_float, C.c_int, C.c_float, C.c_void_p]

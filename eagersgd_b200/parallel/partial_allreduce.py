@@ -38,14 +38,14 @@ class _PinnedOutcome:
 
     def __init__(self):
         self._ptr = C.c_void_p()
-        N.check_cuda(N.cuda().esgd_host_alloc(C.sizeof(N.StepOutcome), C.byref(self._ptr)), "pinned allocation")
+        N.check_cuda(N.cuda().esgd_outcome_alloc(C.byref(self._ptr)), "pinned allocation")
         self.address = int(self._ptr.value)
         self.value = N.StepOutcome.from_address(self.address)
 
     def free(self):
         if self._ptr:
             self.value = None
-            N.cuda().esgd_host_free(self._ptr)
+            N.cuda().esgd_outcome_free(self._ptr)
             self._ptr = C.c_void_p()
 
 

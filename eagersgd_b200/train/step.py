@@ -80,6 +80,7 @@ class TrainStep:
             if mode != "sync":
                 kw["limiter"] = limiter
             self.opt = cls(inner, group, **kw)
+            self.opt.prepare_grad_sinks()
             self.opt.grad_scale = 1.0 / self.loss_scale   # static loss scaling is undone inside the update
             self.autocast = False
         # the operators' zeroed scratch of a step; parameter gradients go to the buckets' own accumulators where they can
@@ -112,7 +113,6 @@ class TrainStep:
             raise NotImplementedError("only the fused momentum-SGD path can be captured in a CUDA graph; "
                                       "run a wrapped optimizer without capture")
         self._gx, self._gy = x.clone(), y.clone()
-        self.opt.prepare_grad_sinks()        # allocates and synchronises: not inside the capture
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(side):
