@@ -229,6 +229,19 @@ Sink find_sink(const Tensor& p) {
 void sink_use(const Sink& s) {
   if (s) { ++s->uses; s->used = true; }
 }
+// The parameter as the operator's autograd input: detached when a sink takes its gradient, so that autograd neither
+// expects one nor calls the parameter's hooks.
+Tensor graph_input(const Tensor& p, const Sink& s) { return s ? p.detach() : p; }
+// What then keeps the operator in the graph when nothing else requires a gradient (the first layer of a network).
+c10::optional<Tensor> anchor_for(const Tensor& x, bool any_sink) {
+  if (!any_sink || x.requires_grad()) return c10::nullopt;
+  static std::mutex m;
+  static Tensor anchors[64];
+  const int d = x.get_device();
+  std::lock_guard<std::mutex> g(m);
+  if (!anchors[d].defined()) anchors[d] = at::empty({0}, x.options().dtype(at::kFloat)).set_requires_grad(true);
+  return anchors[d];
+}
 // Called in its backward once the kernel that writes the accumulator has been launched.
 void sink_done(const Sink& s) {
   GradSinks* o = s->owner.load();
@@ -281,7 +294,7 @@ struct StemGeometry {
 // data-gradient GEMM, instead of autograd summing the two branches of x with a separate pass over the tensor.
 struct ConvFn : public Function<ConvFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w, int64_t kind, int64_t stride, int64_t pad,
-                               bool want_stats, bool tap, const Sink& sink) {
+                               bool want_stats, bool tap, const Sink& sink, const c10::optional<Tensor>& anchor) {
     c10::cuda::CUDAGuard guard(x_in.device());
     Tensor x = nhwc(x_in);
     const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3);
@@ -334,7 +347,7 @@ struct ConvFn : public Function<ConvFn> {
     const auto cfg = ctx->saved_data["cfg"].toIntVector();
     const int64_t kind = cfg[0], stride = cfg[1], pad = cfg[2], n = cfg[3], cin = cfg[4], h = cfg[5], wd = cfg[6];
     const bool want_stats = cfg[7], tap = cfg[8];
-    variable_list none(8);
+    variable_list none(9);
     Tensor d_tap = tap ? grads[want_stats ? 2 : 1] : Tensor();   // gradient that reached the input through the shortcut
     Sink sink = load_sink(ctx, "w");
     if (!grads[0].defined()) {
@@ -349,7 +362,7 @@ struct ConvFn : public Function<ConvFn> {
     const int64_t ho = dy.size(2), wo = dy.size(3), m = n * ho * wo;
     void* st = stream_of(x);
     Tensor dx, dw;
-    const bool need_dx = ctx->needs_input_grad(0), need_dw = ctx->needs_input_grad(1);
+    const bool need_dx = ctx->needs_input_grad(0), need_dw = sink || ctx->needs_input_grad(1);
     if (need_dx && kind == kOneByOne) {
       Tensor res;
       if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
@@ -433,7 +446,7 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
   const bool fuse_tap = tap && kind == kOneByOne && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
   Sink sink = find_sink(w);
   sink_use(sink);
-  variable_list out = ConvFn::apply(x, w, kind, stride, pad, want_stats, fuse_tap, sink);
+  variable_list out = ConvFn::apply(x, graph_input(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink));
   py::object st = want_stats ? py::cast(out[1]) : py::none();
   py::object tp = !tap ? py::none() : py::cast(fuse_tap ? out.back() : x);
   return py::make_tuple(out[0], st, tp);
@@ -442,7 +455,7 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
 // ---------------------------------------------------------------- dense layer: fp32 logits out of bf16 operands
 struct LinearFn : public Function<LinearFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w_in, const c10::optional<Tensor>& b_in,
-                        const Sink& ws, const Sink& bs) {
+                        const Sink& ws, const Sink& bs, const c10::optional<Tensor>& anchor) {
     const Tensor b = b_in.has_value() ? *b_in : Tensor();
     c10::cuda::CUDAGuard guard(x_in.device());
     Tensor x = x_in.contiguous(), w = w_in.contiguous();
@@ -468,7 +481,7 @@ struct LinearFn : public Function<LinearFn> {
     if (dy.scalar_type() != at::kFloat) dy = dy.to(at::kFloat);
     if (dy.stride(1) != 1 || (dy.stride(0) < n && m > 1)) dy = dy.contiguous();
     const int64_t bias_type = ctx->saved_data["bias"].toInt();
-    const bool need_b = bias_type >= 0 && ctx->needs_input_grad(2);
+    const bool need_b = bs || (bias_type >= 0 && ctx->needs_input_grad(2));
     Tensor db32;
     if (need_b && !bs) db32 = zeros_f32({n}, x.device());
     Tensor dy16 = at::empty({m, np}, x.options());
@@ -480,7 +493,7 @@ struct LinearFn : public Function<LinearFn> {
       ck(gemm(dy16.data_ptr(), w.data_ptr(), dx.data_ptr(), m, k, n, np, k, k, false, true, 0, 1, nullptr, nullptr, nullptr, 0, x),
          "dense layer data gradient");
     }
-    if (ctx->needs_input_grad(1)) {
+    if (ws || ctx->needs_input_grad(1)) {
       if (!ws) dw = at::empty({n, k}, w.options());
       ck(gemm(dy16.data_ptr(), x.data_ptr(), ws ? (void*)ws->acc : dw.data_ptr(), n, k, m, np, k, k, true, true, ws ? 2 : 0, 1, nullptr,
               nullptr, nullptr, 0, x), "dense layer weight gradient");
@@ -490,7 +503,7 @@ struct LinearFn : public Function<LinearFn> {
       if (bs) sink_done(bs);
       else db = db32.to((at::ScalarType)bias_type, false, true);
     }
-    return {dx, dw, db, Tensor(), Tensor()};
+    return {dx, dw, db, Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -501,7 +514,9 @@ py::object linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>&
   Sink ws = find_sink(w), bs = find_sink(bias);
   sink_use(ws);
   sink_use(bs);
-  return py::cast(LinearFn::apply(x, w, b, ws, bs));
+  c10::optional<Tensor> bias_in;
+  if (bias.defined()) bias_in = graph_input(bias, bs);
+  return py::cast(LinearFn::apply(x, graph_input(w, ws), bias_in, ws, bs, anchor_for(x, ws || bs)));
 }
 
 // ---------------------------------------------------------------- batch norm (+ residual) (+ ReLU)
@@ -509,7 +524,7 @@ struct BnActFn : public Function<BnActFn> {
   using Opt = c10::optional<Tensor>;
   static Tensor forward(AutogradContext* ctx, const Tensor& y_in, const Tensor& gamma, const Tensor& beta, const Opt& res_in,
                         const Opt& rm_in, const Opt& rv_in, double momentum, bool relu, const Opt& stats_in, const Sink& gs,
-                        const Sink& bs) {
+                        const Sink& bs, const Opt& anchor) {
     c10::cuda::CUDAGuard guard(y_in.device());
     auto get = [](const Opt& o) { return o.has_value() ? *o : Tensor(); };
     Tensor y = nhwc(y_in), res = res_in.has_value() ? nhwc(*res_in) : Tensor(), stats = get(stats_in), rm = get(rm_in), rv = get(rv_in);
@@ -557,7 +572,7 @@ struct BnActFn : public Function<BnActFn> {
     else dgamma = red.select(0, 1);
     if (bs) sink_done(bs);
     else dbeta = red.select(0, 0);
-    variable_list out(11);
+    variable_list out(12);
     out[0] = dy; out[1] = dgamma; out[2] = dbeta; out[3] = dres;
     return out;
   }
@@ -569,7 +584,8 @@ Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c1
   Sink gs = find_sink(gamma), bs = find_sink(beta);
   sink_use(gs);
   sink_use(bs);
-  return BnActFn::apply(y, gamma, beta, res, rm, rv, momentum, relu, stats, gs, bs);
+  return BnActFn::apply(y, graph_input(gamma, gs), graph_input(beta, bs), res, rm, rv, momentum, relu, stats, gs, bs,
+                        anchor_for(y, gs || bs));
 }
 
 // ---------------------------------------------------------------- softmax cross-entropy
@@ -642,7 +658,7 @@ Tensor avg_pool(const Tensor& x) { return AvgPoolFn::apply(x); }
 // single GEMMs over all steps.
 struct LstmFn : public Function<LstmFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w_ih_in, const Tensor& w_hh_in, const Tensor& bias,
-                        const Sink& s_ih, const Sink& s_hh, const Sink& s_b) {
+                        const Sink& s_ih, const Sink& s_hh, const Sink& s_b, const c10::optional<Tensor>& anchor) {
     c10::cuda::CUDAGuard guard(x_in.device());
     Tensor x = x_in.contiguous(), w_ih = w_ih_in.contiguous(), w_hh = w_hh_in.contiguous();
     const int64_t t = x.size(0), b = x.size(1), in = x.size(2), h = w_hh.size(1);
@@ -697,7 +713,7 @@ struct LstmFn : public Function<LstmFn> {
     Tensor dy = grads[0].contiguous();
     Tensor dG = at::empty({t * b, 4 * h}, x.options());
     Tensor dx, dw_ih, dw_hh, db;
-    const bool need_b = ctx->needs_input_grad(3);
+    const bool need_b = s_b || ctx->needs_input_grad(3);
     if (esgd_lstm_persistent_ok((int)b, (int)h, 1)) {
       Tensor scratch = at::empty({esgd_lstm_persistent_scratch()}, f32);
       if (need_b && !s_b) db = at::zeros({4 * h}, f32);
@@ -722,18 +738,18 @@ struct LstmFn : public Function<LstmFn> {
       ck(gemm(dG.data_ptr(), w_ih.data_ptr(), dx.data_ptr(), t * b, in, 4 * h, 4 * h, in, in, false, true, 0, 1, nullptr, nullptr,
               nullptr, 0, x), "lstm input gradient");
     }
-    if (ctx->needs_input_grad(1)) {
+    if (s_ih || ctx->needs_input_grad(1)) {
       dw_ih = weight_grad(s_ih, x, dG.data_ptr(), w_ih, x.data_ptr(), t * b, 4 * h, in);
       if (s_ih) sink_done(s_ih);
     }
-    if (ctx->needs_input_grad(2)) {
+    if (s_hh || ctx->needs_input_grad(2)) {
       if (t > 1)
         dw_hh = weight_grad(s_hh, x, (const char*)dG.data_ptr() + b * 4 * h * 2, w_hh, y.data_ptr(), (t - 1) * b, 4 * h, h);
       else if (!s_hh)
         dw_hh = at::zeros_like(w_hh);
       if (s_hh) sink_done(s_hh);
     }
-    variable_list out(7);
+    variable_list out(8);
     out[0] = dx; out[1] = dw_ih; out[2] = dw_hh; out[3] = db;
     return out;
   }
@@ -747,7 +763,8 @@ Tensor lstm_layer(const Tensor& x, const Tensor& w_ih, const Tensor& w_hh, const
   sink_use(s_ih);
   sink_use(s_hh);
   sink_use(s_b);
-  return LstmFn::apply(x, w_ih, w_hh, bias, s_ih, s_hh, s_b);
+  return LstmFn::apply(x, graph_input(w_ih, s_ih), graph_input(w_hh, s_hh), graph_input(bias, s_b), s_ih, s_hh, s_b,
+                       anchor_for(x, s_ih || s_hh || s_b));
 }
 
 }  // namespace
