@@ -52,7 +52,7 @@ template <int BN_, bool kT>
 struct ConvProblem {
   static constexpr int BN = BN_;
   static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false;
-  CUtensorMap tmX, tmW, tmY;
+  CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, stride, pad;
   FilterTaps taps;
@@ -110,8 +110,10 @@ struct ConvProblem {
   __device__ __forceinline__ int valid_prefix(const Tile& t) const {   // box inside the tensor: its pixels, in order
     return (t.w0 + BW <= Wo && t.h0 + BH <= Ho && t.i0 + BI <= N) ? BW * BH * BI : -1;
   }
-  __device__ __forceinline__ void* row_ptr(const Tile&, int) const { return nullptr; }
-  __device__ __forceinline__ void load_res_panel(const Tile&, int, void*, uint64_t*) const {}
+  __device__ __forceinline__ void store_f32(const Tile&, int, const void*, bool) const {}
+  __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
+    tma_load_4d(smem, &tmR, bar, t.n0 + panel * 64, t.w0, t.h0, t.i0);
+  }
   __device__ __forceinline__ int out_row(int row) const { return row; }
 };
 
@@ -123,7 +125,7 @@ template <int BN_, bool kT>
 struct ConvHaloProblem {
   static constexpr int BN = BN_;
   static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true;
-  CUtensorMap tmX, tmW, tmY;
+  CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, pad;
   FilterTaps taps;
@@ -165,8 +167,10 @@ struct ConvHaloProblem {
   }
   __device__ __forceinline__ bool row_valid(const Tile&, int row) const { return row < BH * Wo; }
   __device__ __forceinline__ int valid_prefix(const Tile&) const { return BH * Wo; }
-  __device__ __forceinline__ void* row_ptr(const Tile&, int) const { return nullptr; }
-  __device__ __forceinline__ void load_res_panel(const Tile&, int, void*, uint64_t*) const {}
+  __device__ __forceinline__ void store_f32(const Tile&, int, const void*, bool) const {}
+  __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
+    tma_load_4d(smem, &tmR, bar, t.n0 + panel * 64, 0, t.h0, t.i0);
+  }
 };
 
 
@@ -180,12 +184,11 @@ template <int BN_>
 struct ConvWgradProblem {
   static constexpr int BN = BN_;
   static constexpr bool A_MN = true, B_MN = true, kZeroStages = true;
-  CUtensorMap tmDY, tmX;
+  CUtensorMap tmDY, tmX, tmDW;
   int N, Ho, Wo, Cout, Cin;
   int R, S, stride, pad;
   int BW, BH, BI, w_tiles, h_tiles, i_tiles;
   int m_tiles, n_tiles, splits, boxes_total, boxes_per_split;
-  float* dw;   // [Cout][R*S][Cin]
   static constexpr int res_kb = 0;   // both operands change with every k-block
   static constexpr int ksteps = BK / 16;
   int n_mma;
@@ -223,9 +226,8 @@ struct ConvWgradProblem {
   __device__ __forceinline__ void load_res_panel(const Tile&, int, void*, uint64_t*) const {}
   __device__ __forceinline__ int out_row(int row) const { return row; }
   static constexpr bool kHalo = false;
-  __device__ __forceinline__ void* row_ptr(const Tile& t, int row) const {
-    const int k = t.m0 + row;
-    return k < Cout ? (void*)(dw + ((size_t)k * (R * S) + t.tap) * Cin) : nullptr;
+  __device__ __forceinline__ void store_f32(const Tile& t, int col, const void* smem, bool) const {
+    tma_reduce_3d(&tmDW, smem, col, t.tap, t.m0);
   }
 };
 
@@ -333,7 +335,9 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
     if (a.ys_w) { strides[0] = (uint64_t)a.ys_w * 2; strides[1] = (uint64_t)a.ys_h * 2; strides[2] = (uint64_t)a.ys_n * 2; }
     uint32_t box[4] = {64, (uint32_t)p.BW, (uint32_t)p.BH, (uint32_t)p.BI};
     int r = esgd::make_tensormap_bf16(&p.tmY, a.y, 4, dims, strides, box, nullptr);
+    if (r == 0 && ep.residual != nullptr) r = esgd::make_tensormap_bf16(&p.tmR, ep.residual, 4, dims, strides, box, nullptr);
     if (r != 0) return 3000 + r;
+    ep.res_bytes = (uint32_t)(p.BW * p.BH * p.BI * 128);
   }
   const int sms = sm_count();
   const int total = p.w_tiles * p.h_tiles * p.i_tiles * p.n_tiles;
@@ -352,7 +356,6 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
     grid = total < sms ? total : sms;
   }
   ep.tx_bytes_a = (uint32_t)(p.BW * p.BH * p.BI * 128);
-  ep.residual = nullptr; ep.ldr = 0;
   ep.tx_bytes = ep.tx_bytes_a + (uint32_t)Cfg<BN>::B_STAGE_BYTES;
   conv_kernel<P><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(p, ep);
   esgd::count_launch();
@@ -415,7 +418,9 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
     uint64_t strides[3] = {(uint64_t)a.Cout * 2, (uint64_t)p.Wo * a.Cout * 2, (uint64_t)p.Ho * p.Wo * a.Cout * 2};
     uint32_t box[4] = {64, (uint32_t)p.Wo, (uint32_t)bh, 1};
     int r = esgd::make_tensormap_bf16(&p.tmY, a.y, 4, dims, strides, box, nullptr);
+    if (r == 0 && ep.residual != nullptr) r = esgd::make_tensormap_bf16(&p.tmR, ep.residual, 4, dims, strides, box, nullptr);
     if (r != 0) return 3000 + r;
+    ep.res_bytes = (uint32_t)(p.Wo * bh * 128);
   }
   const int sms = sm_count();
   if (p.n_tiles > sms) return -3;
@@ -427,7 +432,6 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
   if (grid > total) grid = total;
   ep.tx_bytes_a = (uint32_t)(p.PW * (bh + a.R - 1) * 128);
   ep.tx_bytes = 0;
-  ep.residual = nullptr; ep.ldr = 0;
   conv_kernel<P><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(p, ep);
   esgd::count_launch();
   return (int)cudaGetLastError();
@@ -472,7 +476,13 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
   if (splits > p.boxes_total) splits = p.boxes_total;
   p.boxes_per_split = (p.boxes_total + splits - 1) / splits;
   p.splits = (p.boxes_total + p.boxes_per_split - 1) / p.boxes_per_split;
-  p.dw = dw;
+  {
+    uint64_t dims[3] = {(uint64_t)a.Cin, (uint64_t)a.R * a.S, (uint64_t)a.Cout};
+    uint64_t strides[2] = {(uint64_t)a.Cin * 4, (uint64_t)a.R * a.S * a.Cin * 4};
+    uint32_t box[3] = {32, 1, 128};
+    int r = esgd::make_tensormap_f32(&p.tmDW, dw, 3, dims, strides, box, nullptr);
+    if (r != 0) return 3000 + r;
+  }
   {
     uint64_t dims[4] = {(uint64_t)a.Cout, (uint64_t)p.Wo, (uint64_t)p.Ho, (uint64_t)a.N};
     uint64_t strides[3] = {(uint64_t)a.Cout * 2, (uint64_t)p.Wo * a.Cout * 2, (uint64_t)p.Ho * p.Wo * a.Cout * 2};
@@ -489,7 +499,7 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
     if (r != 0) return 2000 + r;
   }
   Epilogue ep;
-  ep.out_mode = OUT_F32_ATOMIC; ep.relu = 0; ep.n_total = a.Cin; ep.bias = nullptr; ep.bias_bf16 = 0;
+  ep.out_mode = OUT_F32_ATOMIC; ep.relu = 0; ep.n_total = a.Cin; ep.scale = nullptr; ep.bias = nullptr; ep.bias_kind = BIAS_F32; ep.res_bytes = 0;
   ep.col_sum = nullptr; ep.col_sqsum = nullptr; ep.error_flag = error_flag;
   ep.tx_bytes = (uint32_t)(p.BW * p.BH * 128 * (BM / 64 + BN / 64));
   ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
@@ -502,7 +512,7 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
 
 Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* error_flag) {
   Epilogue ep;
-  ep.out_mode = OUT_BF16; ep.relu = relu; ep.n_total = n; ep.bias = nullptr; ep.bias_bf16 = 0;
+  ep.out_mode = OUT_BF16; ep.relu = relu; ep.n_total = n; ep.scale = nullptr; ep.bias = nullptr; ep.bias_kind = BIAS_F32; ep.res_bytes = 0;
   ep.col_sum = col_sum; ep.col_sqsum = col_sqsum; ep.error_flag = error_flag;
   ep.tx_bytes = 0; ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
   return ep;
@@ -537,23 +547,31 @@ int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, in
 }
 
 // x: [N,H,W,Cin] bf16, w: [Cout,R,S,Cin] bf16, y: [N,Ho,Wo,Cout] bf16.  Cin % 8 == 0, Cout % 8 == 0.
+// y = act(scale * conv + bias + residual), each part optional (scale needs a bias; all 16-byte aligned; residual like y).
 // col_sum / col_sqsum (optional, caller-zeroed fp32[Cout]) receive the statistics of the stored y.
 int esgd_conv2d_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S,
-                    int stride, int pad, int relu, float* col_sum, float* col_sqsum, int* error_flag, void* stream) {
+                    int stride, int pad, const float* scale, const float* bias, const void* residual, int relu, float* col_sum,
+                    float* col_sqsum, int* error_flag, void* stream) {
   if (Cin % 8 || Cout % 8 || stride < 1 || stride > 2) return -1;
+  if ((scale != nullptr && bias == nullptr) || (((uintptr_t)scale | (uintptr_t)bias | (uintptr_t)residual) & 15)) return -7;
   ConvArgs a{x, w, y, N, H, W, Cin, Cout, R, S, stride, pad};
   a.fR = R; a.fS = S;
-  return dispatch<false>(a, epilogue_for(Cout, relu, col_sum, col_sqsum, error_flag), (cudaStream_t)stream);
+  Epilogue ep = epilogue_for(Cout, relu, col_sum, col_sqsum, error_flag);
+  ep.scale = scale; ep.bias = bias; ep.residual = residual;
+  return dispatch<false>(a, ep, (cudaStream_t)stream);
 }
 
-// Data gradient on the weights as stored: dy [N,Ho,Wo,Cout], w [Cout,R,S,Cin], dx [N,H,W,Cin] (dense NHWC).
+// Data gradient on the weights as stored: dy [N,Ho,Wo,Cout], w [Cout,R,S,Cin], dx [N,H,W,Cin] (dense NHWC); residual
+// (optional, stride 1, like dx) is added before the rounding.
 // Stride 1: one launch, any R x S with padding up to min(R, S) - 1.  Stride 2: 3x3 filters with padding 1 on even H and W;
 // each output parity (h % 2, w % 2) meets 1, 2, 2 or 4 of the nine taps and is a dense stride-1 problem written
 // into its interleaved pixels of dx (dx[2i + p] uses the filter rows r with (p + 1 - r) even).
 int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, int R, int S,
-                      int stride, int pad, int* error_flag, void* stream) {
-  if (Cin % 8 || Cout % 8) return -1;
-  const Epilogue ep = epilogue_for(Cin, 0, nullptr, nullptr, error_flag);
+                      int stride, int pad, const void* residual, int* error_flag, void* stream) {
+  if (Cin % 8 || Cout % 8 || ((uintptr_t)residual & 15)) return -1;
+  if (residual != nullptr && stride != 1) return -2;
+  Epilogue ep = epilogue_for(Cin, 0, nullptr, nullptr, error_flag);
+  ep.residual = residual;
   cudaStream_t s = (cudaStream_t)stream;
   if (stride == 1) {
     if (pad > R - 1 || pad > S - 1 || R != S) return -1;

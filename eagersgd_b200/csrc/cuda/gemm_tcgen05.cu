@@ -22,13 +22,11 @@ template <int BN_, bool A_MN_, bool B_MN_>
 struct GemmProblem {
   static constexpr int BN = BN_;
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false;
-  CUtensorMap tmA, tmB, tmC, tmR;   // tmR: optional residual, same geometry as the output
+  CUtensorMap tmA, tmB, tmC, tmR;   // tmC: bf16 panels of 64 columns or fp32 ones of 32; tmR: optional residual
   int M, N, K;
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
   int fixed_n;        // every CTA keeps one column range (needed for the per-CTA statistics flush)
   int res_kb;         // > 0: all k-blocks of B for the CTA's column range stay in shared memory
-  float* c_f32;       // fp32 output (direct modes)
-  int ldc;
   static constexpr int ksteps = BK / 16, n_mma = BN_;
   int chained;        // launched with programmatic stream serialization: wait for the previous kernel in the kernel
 
@@ -85,8 +83,9 @@ struct GemmProblem {
   __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
     tma_load_2d(smem, &tmR, bar, t.n0 + panel * 64, t.m0);
   }
-  __device__ __forceinline__ void* row_ptr(const Tile& t, int row) const {
-    return (t.m0 + row < M) ? (void*)(c_f32 + (size_t)(t.m0 + row) * ldc) : nullptr;
+  __device__ __forceinline__ void store_f32(const Tile& t, int col, const void* smem, bool add) const {
+    if (add) tma_reduce_2d(&tmC, smem, col, t.m0);
+    else tma_store_2d(&tmC, smem, col, t.m0);
   }
 };
 
@@ -154,7 +153,10 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
     r = esgd::make_tensormap_bf16(&p.tmC, g.C, 2, dims, strides, box, nullptr);
     if (r != 0) return 3000 + r;
   } else {
-    p.tmC = p.tmA;  // unused
+    dims[0] = (uint64_t)g.N; dims[1] = (uint64_t)g.M; box[0] = 32; box[1] = 128;
+    strides[0] = (uint64_t)g.ldc * 4;
+    r = esgd::make_tensormap_f32(&p.tmC, g.C, 2, dims, strides, box, nullptr);
+    if (r != 0) return 3000 + r;
   }
   p.tmR = p.tmC;
   if (ep.residual != nullptr) {
@@ -172,8 +174,7 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   p.kb_per_split = (p.kb_total + splits - 1) / splits;
   p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
   if (p.splits > 1 && g.out_mode != OUT_F32_ATOMIC) return -2;
-  p.c_f32 = (float*)g.C;
-  p.ldc = g.ldc;
+  ep.res_bytes = PANEL_BYTES;
   const int sms = sm_count();
   int grid;
   // B stays in shared memory when its whole K extent fits beside four A stages and every CTA has several
@@ -225,22 +226,24 @@ extern "C" {
 // C[M,N] = A * B^T (+bias, ReLU, column statistics).  A is [M][K] (a_mn=0, row stride lda)
 // or stored [K][M] (a_mn=1); B is [N][K] (b_mn=0, row stride ldb) or stored [K][N] (b_mn=1).
 // out_mode: 0 bf16, 1 fp32, 2 fp32 atomic accumulate (split-K; C must be zeroed by the caller).
-// Requirements: 16-byte aligned bases, lda/ldb/ldc multiples of 8.  N need not be a multiple of 8: an fp32 output is
-// then written up to the next multiple of 4 columns, inside its row stride.
-// relu: bit 0 ReLU, bit 1 the bias is bf16.
+// Requirements: 16-byte aligned bases, lda/ldb/ldc multiples of 8; N need not be.
+// relu: bit 0 ReLU, bit 1 the bias is bf16.  scale (optional, with an fp32 bias, both 16-byte aligned): the product's
+// columns are multiplied by it before the bias is added.
 // col_sum / col_sqsum (bf16 output only) accumulate into caller-zeroed fp32 arrays of N.
 // residual (bf16 output only): a bf16 [M][N] tensor with row stride ldr (multiple of 8), added before rounding.
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
-                   int b_mn, int out_mode, const float* bias, int relu, int splits, float* col_sum,
+                   int b_mn, int out_mode, const float* scale, const float* bias, int relu, int splits, float* col_sum,
                    float* col_sqsum, const void* residual, int ldr, int* error_flag, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || (lda % 8) || (ldb % 8) || (ldc % 8)) return -1;
-  if (out_mode == OUT_F32_ATOMIC ? N % 4 : ldc < (N + 7) / 8 * 8) return -1;
+  if (ldc < N) return -1;
   if (col_sum != nullptr && out_mode != OUT_BF16) return -4;
   if (residual != nullptr && (out_mode != OUT_BF16 || (ldr % 8) || ((uintptr_t)residual & 15))) return -5;
-  if (out_mode != OUT_BF16 && (((uintptr_t)C & 15) || ((uintptr_t)bias & (relu & 2 ? 7 : 15)))) return -6;   // 16-byte fp32 accesses
+  if ((uintptr_t)C & 15) return -6;
+  if (scale != nullptr && (bias == nullptr || (relu & 2) || (((uintptr_t)scale | (uintptr_t)bias) & 15))) return -7;
   GemmArgs g{A, B, C, M, N, K, lda, ldb, ldc, out_mode, splits};
   Epilogue ep;
-  ep.out_mode = out_mode; ep.relu = relu & 1; ep.n_total = N; ep.bias = bias; ep.bias_bf16 = (relu >> 1) & 1;
+  ep.out_mode = out_mode; ep.relu = relu & 1; ep.n_total = N; ep.scale = scale; ep.bias = bias;
+  ep.bias_kind = relu & 2 ? BIAS_BF16 : (((uintptr_t)bias & 15) ? BIAS_F32_UNALIGNED : BIAS_F32);
   ep.col_sum = col_sum; ep.col_sqsum = col_sqsum; ep.error_flag = error_flag;
   ep.tx_bytes = 0; ep.tx_bytes_a = 0;
   ep.residual = residual; ep.ldr = ldr;

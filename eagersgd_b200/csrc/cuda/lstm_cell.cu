@@ -265,8 +265,8 @@ extern "C" {
 // on the tensor cores and the fused cell kernel), so the GPU never waits for an interpreter between steps.
 
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
-                   int b_mn, int out_mode, const float* bias, int relu, int splits, float* col_sum, float* col_sqsum,
-                   const void* residual, int ldr, int* error_flag, void* stream);
+                   int b_mn, int out_mode, const float* scale, const float* bias, int relu, int splits, float* col_sum,
+                   float* col_sqsum, const void* residual, int ldr, int* error_flag, void* stream);
 void esgd_gemm_set_chained(int on);
 
 // xproj [T*B, 4H] bf16 (input projection of every step), w_hh [4H, H] bf16, bias [4H] fp32;
@@ -286,7 +286,7 @@ int esgd_lstm_seq_fwd(const void* xproj, const void* w_hh, const float* bias, fl
   ChainScope chain;
   for (int t = 0; t < T; ++t) {
     if (t > 0) {   // hprojT[4H, B] += W_hh[4H, H] . h_{t-1}[B, H]^T
-      int rc = esgd_gemm_bf16(w_hh, yp + (t - 1) * bh, hprojT, 4 * H, B, H, H, H, B, 0, 0, 2, nullptr, 0, splits,
+      int rc = esgd_gemm_bf16(w_hh, yp + (t - 1) * bh, hprojT, 4 * H, B, H, H, H, B, 0, 0, 2, nullptr, nullptr, 0, splits,
                               nullptr, nullptr, nullptr, 0, error_flag, stream);
       if (rc != 0) return rc;
     }
@@ -316,7 +316,7 @@ int esgd_lstm_seq_bwd(const void* gates, const float* c, const void* dy, const v
                       t < T - 1 ? dh_recT : nullptr, dc, dgp + (size_t)t * 4 * bh, B, H, B, 1, stream);
     if (rc != 0) return rc;
     if (t > 0) {   // dh_recT[H, B] += W_hh^T . dG_t^T: A stored [K = 4H][M = H]
-      rc = esgd_gemm_bf16(w_hh, dgp + (size_t)t * 4 * bh, dh_recT, H, B, 4 * H, H, 4 * H, B, 1, 0, 2, nullptr, 0, splits,
+      rc = esgd_gemm_bf16(w_hh, dgp + (size_t)t * 4 * bh, dh_recT, H, B, 4 * H, H, 4 * H, B, 1, 0, 2, nullptr, nullptr, 0, splits,
                           nullptr, nullptr, nullptr, 0, error_flag, stream);
       if (rc != 0) return rc;
     }

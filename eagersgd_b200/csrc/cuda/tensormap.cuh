@@ -34,10 +34,10 @@ inline void bind_primary_context() {
   }
 }
 
-// bf16 tensor of rank `rank` (dims innermost first), 128-byte swizzle, zero fill
+// Tensor of rank `rank` (dims innermost first), 128-byte swizzle, zero fill
 // outside the tensor.  strides_bytes has rank-1 entries (dims 1..rank-1).
-inline int make_tensormap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
-                               const uint64_t* strides_bytes, const uint32_t* box, const uint32_t* elem_strides) {
+inline int make_tensormap(CUtensorMapDataType type, CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                          const uint64_t* strides_bytes, const uint32_t* box, const uint32_t* elem_strides) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (fn == nullptr) return -100;
   bind_primary_context();
@@ -49,10 +49,18 @@ inline int make_tensormap_bf16(CUtensorMap* out, const void* base, int rank, con
     e[i] = elem_strides ? elem_strides[i] : 1;
     if (i < rank - 1) s[i] = strides_bytes[i];
   }
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e,
+  CUresult r = fn(out, type, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, e,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return (int)r;
+}
+inline int make_tensormap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                               const uint64_t* strides_bytes, const uint32_t* box, const uint32_t* elem_strides) {
+  return make_tensormap(CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, out, base, rank, dims, strides_bytes, box, elem_strides);
+}
+inline int make_tensormap_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                              const uint64_t* strides_bytes, const uint32_t* box, const uint32_t* elem_strides) {
+  return make_tensormap(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, out, base, rank, dims, strides_bytes, box, elem_strides);
 }
 
 }  // namespace esgd

@@ -4,11 +4,14 @@
 //   warp 0     : TMA producer — the Problem policy issues the loads of one k-block
 //   warp 1     : tcgen05.mma issuer (one thread); two TMEM accumulators so the
 //                epilogue of tile i overlaps the main loop of tile i+1
-//   warps 2..9 : epilogue — tcgen05.ld, bias / ReLU, bf16 tile staged in shared
-//                memory in the 128-byte-swizzled layout and written with a TMA
-//                store (coalesced, clipped at the tensor edge); per-channel sum and
-//                sum of squares of the stored tile are taken from shared memory and
-//                flushed with one atomic per column per CTA (batch-norm statistics)
+//   warps 2..17: epilogue, four groups of four warps.  A unit of work is one 64-column panel of a tile: tcgen05.ld, affine
+//                map / residual / ReLU, the panel staged in shared memory in the 128-byte-swizzled layout and written
+//                with a TMA store (coalesced, clipped at the tensor edge); per-channel sum and sum of squares of the
+//                stored panel are taken from shared memory and flushed with one atomic per column per CTA (batch-norm
+//                statistics).  The groups work on different panels with barriers of their own: one group of eight warps
+//                in lock step left the SM idle in every barrier and load it waited for (64-deep products with
+//                statistics ran at half the speed of those without).  fp32 outputs leave the same way, 32 columns at a
+//                time; split-K sums are TMA reductions (whole rows into L2 instead of one atomic per 16 bytes).
 //
 // B-resident mode: when a CTA keeps one column range for all of its tiles and the whole K
 // extent of B for that range fits beside four A stages, B is loaded ONCE and stays in shared
@@ -18,7 +21,8 @@
 //
 // A tile is 128 rows x BN columns; a k-block is 64 bf16 (one 128-byte swizzle row).
 // Every mbarrier wait is bounded; on expiry the CTA raises an error flag, lets the
-// copies in flight land, frees its tensor memory and returns.
+// copies in flight land, frees its tensor memory and returns.  A role that has given up still meets its group at the
+// barriers, so nobody waits for it.
 #pragma once
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -34,35 +38,39 @@ constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int A_STAGE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int PANEL_BYTES = BM * 64 * 2;     // one 128 x 64 bf16 output panel
-constexpr int NUM_EPI_THREADS = 256;         // eight epilogue warps
-constexpr int NUM_THREADS = 64 + NUM_EPI_THREADS;
-constexpr int NUM_PANEL_BUFS = 4;            // output staging ring (the one-barrier hand-over below needs four)
+constexpr int NUM_GROUPS = 4;                // epilogue groups, each with a staging buffer of one panel
+constexpr int GROUP_THREADS = 128;
+constexpr int NUM_THREADS = 64 + NUM_GROUPS * GROUP_THREADS;
 
+enum BiasKind { BIAS_F32 = 0, BIAS_BF16 = 1, BIAS_F32_UNALIGNED = 2 };
 enum OutMode { OUT_BF16 = 0, OUT_F32 = 1, OUT_F32_ATOMIC = 2 };
 
 struct Epilogue {
   int out_mode;
   int relu;
   int n_total;             // number of valid output columns (channels)
+  const float* scale;      // per column factor applied before the bias, may be null (needs a bias)
   const float* bias;       // per column, may be null
-  int bias_bf16;           // ... and bf16 instead of fp32
+  int bias_kind;           // BIAS_F32 (16-byte aligned, like scale), BIAS_BF16 or BIAS_F32_UNALIGNED
   float* col_sum;          // optional per-column statistics of the stored bf16 values
   float* col_sqsum;
   int* error_flag;
   uint32_t tx_bytes;       // bytes the loads of one k-block deliver (0: full A and B stage tiles)
   uint32_t tx_bytes_a;     // bytes of the A loads alone (B-resident mode; 0: a full A stage tile)
   const void* residual;    // optional bf16 tensor added to the product before rounding (same shape as the output)
-  int ldr;                 // its row stride in elements
+  int ldr;                 // its row stride in elements (GEMM)
+  uint32_t res_bytes;      // bytes one panel of it delivers
 };
 
 template <int BN>
 struct Cfg {
   static constexpr int B_STAGE_BYTES = BN * BK * 2;
   static constexpr int STAGES = BN == 256 ? 3 : (BN == 128 ? 5 : 6);
-  static constexpr int TMEM_COLS = 2 * BN;
+  static constexpr int ACCS = BN == 256 ? 2 : 4;       // accumulators in tensor memory: tiles in flight
+  static constexpr int TMEM_COLS = ACCS * BN;
   static constexpr int MAX_STAGES = 8;                 // A-only ring of the B-resident mode
   static constexpr int STAGE_AREA = 161 * 1024;        // operand stages (ring, or A ring + resident B)
-  static constexpr int SMEM_BYTES = 1024 + STAGE_AREA + NUM_PANEL_BUFS * PANEL_BYTES + 512;
+  static constexpr int SMEM_BYTES = 1024 + STAGE_AREA + NUM_GROUPS * PANEL_BYTES + 512;
   static_assert(STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) <= STAGE_AREA, "ring does not fit");
   static_assert(SMEM_BYTES <= 227 * 1024, "over the shared-memory limit of a CTA");
   // k-blocks of B that may stay resident: four A stages must still fit
@@ -92,12 +100,31 @@ inline bool resident_enabled() {
 
 __device__ __forceinline__ float bias_at(const Epilogue& ep, int col) {
   if (col >= ep.n_total) return 0.0f;
-  return ep.bias_bf16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(ep.bias) + col)) : __ldg(ep.bias + col);
+  return ep.bias_kind == BIAS_BF16 ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(ep.bias) + col)) : __ldg(ep.bias + col);
+}
+
+// Column `col` .. +3 of the affine map (and the bias alone without a scale).
+__device__ __forceinline__ void affine4(const Epilogue& ep, int col, float v[4]) {
+  if (ep.bias_kind == BIAS_F32 && col + 4 <= ep.n_total) {
+    const float4 b = __ldg(reinterpret_cast<const float4*>(ep.bias + col));
+    if (ep.scale != nullptr) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(ep.scale + col));
+      v[0] = fmaf(v[0], a.x, b.x); v[1] = fmaf(v[1], a.y, b.y); v[2] = fmaf(v[2], a.z, b.z); v[3] = fmaf(v[3], a.w, b.w);
+    } else {
+      v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (ep.scale != nullptr && col + q < ep.n_total) v[q] *= __ldg(ep.scale + col + q);
+      v[q] += bias_at(ep, col + q);
+    }
+  }
 }
 
 // 32 accumulator columns of one row -> bf16 -> four 16-byte chunks of the swizzled staging panel.
-// kPlain leaves out the bias / ReLU code altogether: as run-time options they would be predicated
-// instructions that still take issue slots in the common case that uses neither.
+// kPlain leaves out the affine / residual / ReLU code altogether: as run-time options they would be predicated
+// instructions that still take issue slots in the common case that uses none.
 template <bool kPlain>
 __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* panel, int row, int half, int col0,
                                                   const Epilogue& ep, bool has_residual) {
@@ -109,6 +136,10 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
     const int chunk = half * 4 + g;          // 16-byte chunk within the 128-byte row
     uint4* slot = reinterpret_cast<uint4*>(panel + row * 128 + ((chunk ^ (row & 7)) << 4));
     if (!kPlain) {
+      if (ep.bias != nullptr) {
+        affine4(ep, col0 + g * 8, v);
+        affine4(ep, col0 + g * 8 + 4, v + 4);
+      }
       if (has_residual) {     // the residual panel was brought into this very buffer by TMA; add in place
         const uint4 rv = *slot;
         const uint32_t* rw = reinterpret_cast<const uint32_t*>(&rv);
@@ -117,11 +148,6 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
           v[2 * j] += __uint_as_float(rw[j] << 16);
           v[2 * j + 1] += __uint_as_float(rw[j] & 0xffff0000u);
         }
-      }
-      if (ep.bias != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          v[j] += bias_at(ep, col0 + g * 8 + j);
       }
       if (ep.relu) {
 #pragma unroll
@@ -134,6 +160,36 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
     for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
     *slot = pk;
   }
+}
+
+// 32 fp32 accumulator columns of one row -> eight 16-byte chunks of a staging panel of 32 columns.
+__device__ __forceinline__ void stage_row_f32(const uint32_t* r, uint8_t* panel, int row, int col0, const Epilogue& ep) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r[c * 4 + j]);
+    if (ep.bias != nullptr) affine4(ep, col0 + c * 4, v);
+    if (ep.relu) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = fmaxf(v[j], 0.0f);
+    }
+    *reinterpret_cast<float4*>(panel + row * 128 + ((c ^ (row & 7)) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
+// Two fp32 additions / multiply-adds in one instruction.
+__device__ __forceinline__ uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
+  return r;
+}
+__device__ __forceinline__ void add_f32x2(uint64_t& a, uint64_t b) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b)); }
+__device__ __forceinline__ void fma_f32x2(uint64_t& acc, uint64_t a) { asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc) : "l"(a)); }
+__device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
+  uint32_t lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
+  return make_float2(__uint_as_float(lo), __uint_as_float(hi));
 }
 
 // Problem policy requirements (all __device__ const):
@@ -149,7 +205,7 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
 //   static constexpr bool kHalo; int out_row(int row)   row of the stored tile for a GEMM row (identity unless kHalo)
 //   kHalo only: int cblks, R, S, PW; void load_halo(const Tile&, int cb, void* smem, uint64_t* bar)
 //   int valid_prefix(const Tile&)                  n if exactly rows [0, n) are real outputs, -1 if irregular
-//   void* row_ptr(const Tile&, int row)            fp32 output row pointer (direct modes), or nullptr
+//   void store_f32(const Tile&, int col, const void* smem, bool add)   TMA store / reduction of 128 x 32 fp32 columns
 template <class P>
 __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   constexpr int BN = P::BN;
@@ -166,13 +222,13 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   uint8_t* sA = smem;                        // halo mode: the input boxes
   uint8_t* sB = kHalo ? sA + nhalo * HALO_BYTES : sA + nstages * A_STAGE_BYTES;
   uint8_t* sC = smem + C::STAGE_AREA;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sC + NUM_PANEL_BUFS * PANEL_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sC + NUM_GROUPS * PANEL_BYTES);
   uint64_t* empty = full + C::MAX_STAGES;
   uint64_t* tfull = empty + C::MAX_STAGES;
-  uint64_t* tempty = tfull + 2;
-  uint64_t* bres = tempty + 2;               // the resident B tiles have landed
-  uint64_t* rfull = bres + 1;                // residual panel has landed in staging buffer [NUM_PANEL_BUFS]
-  uint64_t* hfull = rfull + NUM_PANEL_BUFS;  // halo mode: input box has landed / has been consumed [MAX_HALOS]
+  uint64_t* tempty = tfull + C::ACCS;
+  uint64_t* bres = tempty + C::ACCS;         // the resident B tiles have landed
+  uint64_t* rfull = bres + 1;                // residual panel has landed in the staging buffer of a group
+  uint64_t* hfull = rfull + NUM_GROUPS;      // halo mode: input box has landed / has been consumed [MAX_HALOS]
   uint64_t* hempty = hfull + MAX_HALOS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(hempty + MAX_HALOS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -181,9 +237,9 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::MAX_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], NUM_EPI_THREADS / 32); }
+    for (int a = 0; a < C::ACCS; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], BN / 64 * GROUP_THREADS / 32); }
     mbar_init(bres, 1);
-    for (int b = 0; b < NUM_PANEL_BUFS; ++b) mbar_init(&rfull[b], 1);
+    for (int b = 0; b < NUM_GROUPS; ++b) mbar_init(&rfull[b], 1);
     for (int b = 0; b < MAX_HALOS; ++b) { mbar_init(&hfull[b], 1); mbar_init(&hempty[b], 1); }
     *abort_flag = 0;
     mbar_fence_init();
@@ -265,15 +321,27 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     // ------------------------------------------------------------ MMA issuer
     if (elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(BM, prob.n_mma, P::A_MN ? 1 : 0, P::B_MN ? 1 : 0);
-      const int ksteps = prob.ksteps;            // < 4: the reduction has fewer than 64 channels, the rest is zero fill
+      // Products of one k-block.  Below 64 reduced channels (narrow convolutions) the last steps would multiply zero fill;
+      // the full block is a path of its own because a predicate per instruction slows the issue loop of narrow tiles.
+      const int ksteps = prob.ksteps;
+      auto issue_block = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t& accumulate) {
+        constexpr uint64_t sa = P::A_MN ? (2048 >> 4) : (32 >> 4), sb = P::B_MN ? (2048 >> 4) : (32 >> 4);   // 16 K elements
+        if (ksteps == BK / 16) {
+          umma_bf16(d, a, b, idesc, accumulate);
+#pragma unroll
+          for (int j = 1; j < BK / 16; ++j) umma_bf16(d, a + j * sa, b + j * sb, idesc, 1u);
+        } else {
+          umma_bf16(d, a, b, idesc, accumulate);
+          for (int j = 1; j < ksteps; ++j) umma_bf16(d, a + j * sa, b + j * sb, idesc, 1u);
+        }
+        accumulate = 1;
+      };
       // The issuing thread is one lane with nothing to hide its instruction latency behind: every instruction
       // between two tcgen05.mma widens the gap between them.  (Timestamps taken in this loop: a 128 x 64 x 16
       // MMA goes out every ~115 cycles, a 128 x 256 x 16 one every ~185 -- 32 and 128 cycles of tensor-pipe work
       // plus a fixed cost per instruction; narrow tiles are bound by that cost, not by their operands' traffic.
       // Dealing the K steps to several accumulators did not shorten it.)  Descriptors are therefore built once and advanced
       // by adding to their address field (bits 0-13, in 16-byte units; shared memory is < 256 KB, so no carry).
-      constexpr uint64_t kStepA = P::A_MN ? (2048 >> 4) : (32 >> 4);      // K advance of 16 elements
-      constexpr uint64_t kStepB = P::B_MN ? (2048 >> 4) : (32 >> 4);
       const uint64_t a_desc0 = P::A_MN ? umma_smem_desc(smem_u32(sA), 8192, 1024) : umma_smem_desc(smem_u32(sA), 16, 1024);
       const uint64_t b_desc0 = P::B_MN ? umma_smem_desc(smem_u32(sB), 8192, 1024) : umma_smem_desc(smem_u32(sB), 16, 1024);
       int stage = 0, acc = 0, hs = 0;
@@ -305,11 +373,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
                   tc_fence_after();
                   b_cur = b_desc0 + (uint64_t)(stage * (C::B_STAGE_BYTES >> 4));
                 }
-#pragma unroll
-                for (int j = 0; j < BK / 16; ++j) {
-                  if (j < ksteps) umma_bf16(d_tmem, a_tap + j * kStepA, b_cur + j * kStepB, idesc, accumulate);
-                  accumulate = 1;
-                }
+                issue_block(d_tmem, a_tap, b_cur, accumulate);
                 if (res_kb == 0) {
                   umma_commit(&empty[stage]);
                   if (++stage == nstages) { stage = 0; phase ^= 1u; }
@@ -326,188 +390,176 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           tc_fence_after();
           const uint64_t a_cur = a_desc0 + (uint64_t)(stage * (A_STAGE_BYTES >> 4));
           const uint64_t b_cur = b_desc0 + (uint64_t)((res_kb > 0 ? kb : stage) * (C::B_STAGE_BYTES >> 4));
-#pragma unroll
-          for (int j = 0; j < BK / 16; ++j) {
-            if (j < ksteps) umma_bf16(d_tmem, a_cur + j * kStepA, b_cur + j * kStepB, idesc, accumulate);
-            accumulate = 1;
-          }
+          issue_block(d_tmem, a_cur, b_cur, accumulate);
           umma_commit(&empty[stage]);
           if (++stage == nstages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         umma_commit(&tfull[acc]);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1u;
+        if (++acc == C::ACCS) { acc = 0; acc_phase ^= 1u; }
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (8 warps)
-    // A warp may only touch TMEM lanes [32*(warp%4), +32): two warps share each lane quarter and
-    // split every 64-column panel into halves.
-    const int q = warp & 3;
-    const int half = (warp - 2) >> 2;       // which 32 columns of a 64-column panel
-    const int et = threadIdx.x - 64;        // 0..255 among the epilogue threads
+    // ------------------------------------------------------------ epilogue
+    // A warp may only touch TMEM lanes [32*(warp%4), +32); four consecutive warps cover all rows.  Group g works on
+    // panel g % PANELS of the tiles it is dealt, so its columns within a tile never change.
+    constexpr int PANELS = BN / 64, TURNS = NUM_GROUPS / PANELS;     // groups per panel: they take turns over the tiles
+    const int q = warp & 3, grp = (warp - 2) >> 2;
+    const int gt = (int)threadIdx.x - 64 - grp * GROUP_THREADS;      // 0..127 among the group's threads
+    const int pnl = grp % PANELS, turn = grp / PANELS;
     const int row = q * 32 + lane;          // tile row owned by this thread
     const int drow = prob.out_row(row);     // its row in the stored tile (halo mode: margin rows have none)
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    int buf = 0;                            // staging panel buffer in use (ring)
-    // statistics: thread (cp = et % 32, rg = et / 32) covers columns 2cp, 2cp+1 of each panel, rows 16rg..+16
-    float st_sum[BN / 64][2], st_sq[BN / 64][2];
-#pragma unroll
-    for (int pnl = 0; pnl < BN / 64; ++pnl) { st_sum[pnl][0] = st_sum[pnl][1] = st_sq[pnl][0] = st_sq[pnl][1] = 0.f; }
-    int stats_n0 = -1;
+    uint8_t* panel = sC + grp * PANEL_BYTES;
+    const bool leader = gt == 0;            // issues the group's copies
     const bool has_res = ep.residual != nullptr;
     const bool plain = ep.bias == nullptr && !ep.relu && !has_res;
-    uint32_t gpanel = 0;                    // panels processed so far (all threads count alike)
-    // Residual prefetch (thread 0): the residual's panels are brought into the staging ring by TMA two panels
-    // ahead of the epilogue, which then adds them in place.
-    typename P::Tile pf_t;
-    int pf_it = 0, pf_pnl = 0;
-    uint32_t pf_g = 0;
-    bool pf_valid = false;
-    auto prefetch_residual = [&]() {
-      if (!pf_valid) return;
-      const int b = (int)(pf_g % NUM_PANEL_BUFS);
-      mbar_expect_tx(&rfull[b], (uint32_t)PANEL_BYTES);
-      prob.load_res_panel(pf_t, pf_pnl, sC + b * PANEL_BYTES, &rfull[b]);
-      ++pf_g;
-      if (++pf_pnl >= min(BN / 64, (ep.n_total - pf_t.n0 + 63) / 64)) {
-        pf_pnl = 0;
-        pf_valid = prob.tile(++pf_it, pf_t);
-      }
-    };
-    if (has_res && et == 0) {
-      pf_valid = prob.tile(0, pf_t);
-      prefetch_residual();
-      prefetch_residual();
-    }
+    // statistics: thread (cp, rg) covers columns 2cp, 2cp+1 of the panel, rows 32rg .. 32rg+31
+    const int cp = gt & 31, rg = gt >> 5;
+    uint64_t st_sum = 0, st_sq = 0;
+    uint32_t res_phase = 0;
     bool ok = true;
     typename P::Tile t;
-    for (int it = 0; ok && prob.tile(it, t); ++it) {
-      if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
+    // The residual panel of a unit travels while the group finishes the one before it.
+    auto fetch_residual = [&](int it) {
+      typename P::Tile n;
+      if (!leader || !prob.tile(it, n) || n.n0 + pnl * 64 >= ep.n_total) return;
+      mbar_expect_tx(&rfull[grp], ep.res_bytes);
+      prob.load_res_panel(n, pnl, panel, &rfull[grp]);
+    };
+    if (has_res) fetch_residual(turn);
+    for (int it = turn; prob.tile(it, t); it += TURNS) {
+      const int acc = it % C::ACCS;
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&tfull[acc], (uint32_t)(it / C::ACCS) & 1u, abort_flag));
       tc_fence_after();
-      stats_n0 = t.n0;
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + half * 32);
-      if (ep.out_mode == OUT_BF16) {
-        const int npan = min(BN / 64, (ep.n_total - t.n0 + 63) / 64);   // uniform across the CTA
-        uint32_t row_mask = 0xffffu;          // validity of this thread's 16 statistics rows, once per tile
-        if (ep.col_sum != nullptr) {
-          const int prefix = prob.valid_prefix(t);      // rows [0, prefix) are the real outputs, or -1
-          if (prefix >= 0) {
-            const int mine = min(16, max(0, prefix - (et >> 5) * 16));
-            row_mask = (1u << mine) - 1u;
-          } else {
-            row_mask = 0u;
-            for (int rr = 0; rr < 16; ++rr)
-              if (prob.row_valid(t, (et >> 5) * 16 + rr)) row_mask |= 1u << rr;
-          }
+      const int col0 = t.n0 + pnl * 64;
+      if (col0 < ep.n_total) {              // uniform across the group
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + pnl * 64);
+        uint32_t r[32];                       // 32 columns at a time: two halves would not fit 96 registers beside the rest
+        tmem_ld_32x32b_x32(t_row, r);
+        if (has_res) {
+          ok = __all_sync(0xffffffffu, ok && mbar_wait(&rfull[grp], res_phase, abort_flag));
+          res_phase ^= 1u;
+        } else {
+          if (leader) tma_store_wait_read<0>();               // the group's previous panel has left the buffer
+          named_barrier_sync(1 + grp, GROUP_THREADS);
         }
-        uint32_t rbuf[2][32];
-        tmem_ld_32x32b_x32(t_row, rbuf[0]);
-#pragma unroll
-        for (int pnl = 0; pnl < BN / 64; ++pnl) {
-          if (pnl < npan) {
-            tmem_ld_wait();
-            if (pnl + 1 < npan)   // the next panel's accumulators travel while this one is converted
-              tmem_ld_32x32b_x32(t_row + (uint32_t)((pnl + 1) * 64), rbuf[(pnl + 1) & 1]);
-            uint8_t* panel = sC + buf * PANEL_BYTES;
-            // This buffer was last read by the store issued NUM_PANEL_BUFS panels ago; thread 0 waited for
-            // that read before it arrived at the previous panel's barrier (see below), so it is free.
-            const int col0 = t.n0 + pnl * 64 + half * 32;
-            if (has_res && !mbar_wait(&rfull[buf], (gpanel / NUM_PANEL_BUFS) & 1u, abort_flag)) { ok = false; break; }
-            if (drow >= 0) {
-              if (plain) pack_row_to_panel<true>(rbuf[pnl & 1], panel, drow, half, col0, ep, false);
-              else pack_row_to_panel<false>(rbuf[pnl & 1], panel, drow, half, col0, ep, has_res);
-            }
-            fence_proxy_async();
-            named_barrier_sync(1, NUM_EPI_THREADS);    // the panel is complete and visible to the TMA engine
-            if (et == 0) {
-              prob.store_panel(t, pnl, panel);
-              tma_store_commit();
-              // One barrier per panel: before thread 0 reaches the NEXT panel's barrier it makes sure that all
-              // but the two newest stores have read their buffers, so after that barrier everyone may overwrite
-              // the buffer used three panels ago -- the one the panel after next needs.
-              tma_store_wait_read<2>();
-              if (has_res) prefetch_residual();       // into the buffer the panel after next will use
-            }
-            if (ep.col_sum != nullptr) {
-              // thread (cp, rg): columns 2cp, 2cp+1 of the panel, rows 16rg .. 16rg+15, read back as stored
-              const int cp = et & 31, rg = et >> 5;
-              const uint8_t* colp = panel + (cp & 3) * 4;
-              const int chunk = cp >> 2;
-              float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-#pragma unroll
-              for (int rr = 0; rr < 16; ++rr) {
-                const int r_ = rg * 16 + rr;
-                uint32_t w = *reinterpret_cast<const uint32_t*>(colp + r_ * 128 + ((chunk ^ (r_ & 7)) << 4));
-                if (!((row_mask >> rr) & 1u)) w = 0u;        // rows outside the tensor count as zeros
-                const float f0 = __uint_as_float(w << 16), f1 = __uint_as_float(w & 0xffff0000u);
-                s0 += f0; s1 += f1; q0 = fmaf(f0, f0, q0); q1 = fmaf(f1, f1, q1);
-              }
-              st_sum[pnl][0] += s0; st_sum[pnl][1] += s1; st_sq[pnl][0] += q0; st_sq[pnl][1] += q1;
-            }
-            buf = (buf + 1) % NUM_PANEL_BUFS;
-            ++gpanel;
-          }
-        }
-        if (!ok) break;
-      } else {
-        // fp32 outputs (logits, split-K weight gradients): direct stores / atomics from registers
-        float* out_row = reinterpret_cast<float*>(prob.row_ptr(t, row));
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(t_row + (uint32_t)(c * 64), r);
+        tmem_ld_wait();
+        auto next_half = [&]() {                              // the accumulator is free once every panel has been read
+          tmem_ld_32x32b_x32(t_row + 32, r);
           tmem_ld_wait();
-          const int col0 = t.n0 + c * 64 + half * 32;
-          if (out_row != nullptr) {
-            // four columns at a time (rows are 32-byte aligned and N is a multiple of 8): 16-byte stores, and
-            // 16-byte reductions for the split-K case, a quarter of the atomic instructions
-#pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4) {
-              if (col0 + j4 * 4 < ep.n_total) {
-                float4 v = make_float4(__uint_as_float(r[j4 * 4]), __uint_as_float(r[j4 * 4 + 1]),
-                                       __uint_as_float(r[j4 * 4 + 2]), __uint_as_float(r[j4 * 4 + 3]));
-                if (ep.bias != nullptr) {
-                  const int c0 = col0 + j4 * 4;
-                  if (!ep.bias_bf16 && c0 + 4 <= ep.n_total) {
-                    const float4 b4 = __ldg(reinterpret_cast<const float4*>(ep.bias + c0));
-                    v.x += b4.x; v.y += b4.y; v.z += b4.z; v.w += b4.w;
-                  } else {
-                    v.x += bias_at(ep, c0); v.y += bias_at(ep, c0 + 1); v.z += bias_at(ep, c0 + 2); v.w += bias_at(ep, c0 + 3);
-                  }
-                }
-                if (ep.relu) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
-                float4* dst = reinterpret_cast<float4*>(out_row + col0 + j4 * 4);
-                if (ep.out_mode == OUT_F32) *dst = v;
-                else atomicAdd(dst, v);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[acc]);
+        };
+        if (ep.out_mode == OUT_BF16) {
+          if (plain) {
+            if (drow >= 0) pack_row_to_panel<true>(r, panel, drow, 0, col0, ep, false);
+            next_half();
+            if (drow >= 0) pack_row_to_panel<true>(r, panel, drow, 1, col0 + 32, ep, false);
+          } else {
+            if (drow >= 0) pack_row_to_panel<false>(r, panel, drow, 0, col0, ep, has_res);
+            next_half();
+            if (drow >= 0) pack_row_to_panel<false>(r, panel, drow, 1, col0 + 32, ep, has_res);
+          }
+          fence_proxy_async();
+          named_barrier_sync(1 + grp, GROUP_THREADS);         // the panel is complete and visible to the TMA engine
+          if (leader) {
+            prob.store_panel(t, pnl, panel);
+            tma_store_commit();
+          }
+          if (ep.col_sum != nullptr) {
+            const int prefix = prob.valid_prefix(t);          // rows [0, prefix) are the real outputs, or -1
+            uint32_t mask = 0xffffffffu;                      // this thread's 32 rows
+            if (prefix >= 0) {
+              const int mine = min(32, max(0, prefix - rg * 32));
+              mask = mine >= 32 ? 0xffffffffu : (1u << mine) - 1u;
+            } else {
+              mask = 0u;
+              for (int rr = 0; rr < 32; ++rr)
+                if (prob.row_valid(t, rg * 32 + rr)) mask |= 1u << rr;
+            }
+            const uint8_t* colp = panel + rg * 32 * 128 + (cp & 3) * 4;
+            const int chunk = cp >> 2;
+            uint64_t s = 0, sq = 0;
+            if (__all_sync(0xffffffffu, mask == 0xffffffffu)) {
+#pragma unroll 16
+              for (int rr = 0; rr < 32; ++rr) {
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(colp + rr * 128 + ((chunk ^ (rr & 7)) << 4));
+                const uint64_t f = pack_f32x2(w << 16, w & 0xffff0000u);
+                add_f32x2(s, f);
+                fma_f32x2(sq, f);
               }
+            } else {
+#pragma unroll 8
+              for (int rr = 0; rr < 32; ++rr) {
+                uint32_t w = *reinterpret_cast<const uint32_t*>(colp + rr * 128 + ((chunk ^ (rr & 7)) << 4));
+                if (!((mask >> rr) & 1u)) w = 0u;             // rows outside the tensor count as zeros
+                const uint64_t f = pack_f32x2(w << 16, w & 0xffff0000u);
+                add_f32x2(s, f);
+                fma_f32x2(sq, f);
+              }
+            }
+            add_f32x2(st_sum, s);
+            add_f32x2(st_sq, sq);
+          }
+        } else {
+          // fp32 outputs (logits, split-K weight gradients): 32 columns at a time through the same buffer
+          const bool add = ep.out_mode == OUT_F32_ATOMIC;
+          stage_row_f32(r, panel, row, col0, ep);
+          next_half();
+          fence_proxy_async();
+          named_barrier_sync(1 + grp, GROUP_THREADS);
+          if (leader) {
+            prob.store_f32(t, col0, panel, add);
+            tma_store_commit();
+            tma_store_wait_read<0>();
+          }
+          named_barrier_sync(1 + grp, GROUP_THREADS);
+          if (col0 + 32 < ep.n_total) {
+            stage_row_f32(r, panel, row, col0 + 32, ep);
+            fence_proxy_async();
+            named_barrier_sync(1 + grp, GROUP_THREADS);
+            if (leader) {
+              prob.store_f32(t, col0 + 32, panel, add);
+              tma_store_commit();
             }
           }
         }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[acc]);
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1u;
-    }
-    if (ep.col_sum != nullptr && stats_n0 >= 0) {   // one flush per CTA: its tiles share the column range
-      const int cp = et & 31;
-#pragma unroll
-      for (int pnl = 0; pnl < BN / 64; ++pnl) {
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const int col = stats_n0 + pnl * 64 + cp * 2 + k;
-          if (col < ep.n_total) {
-            atomicAdd(ep.col_sum + col, st_sum[pnl][k]);
-            atomicAdd(ep.col_sqsum + col, st_sq[pnl][k]);
+        if (has_res) {
+          named_barrier_sync(1 + grp, GROUP_THREADS);         // the statistics are done with the panel, too
+          if (leader) {
+            tma_store_wait_read<0>();
+            fetch_residual(it + TURNS);
           }
+        }
+      } else {
+        if (lane == 0) mbar_arrive(&tempty[acc]);
+        if (has_res && leader) {
+          tma_store_wait_read<0>();
+          fetch_residual(it + TURNS);
         }
       }
     }
-    if (et == 0) tma_store_wait_all();               // shared memory must outlive the bulk stores
+    if (ep.col_sum != nullptr && prob.tile(0, t)) {
+      // One atomic per column and CTA (its tiles share the column range): the threads' sums meet in shared memory first.
+      // Flushed thread by thread, a 64-channel layer sent 2400 atomics to every address and waited 17 us for them.
+      float* sums = reinterpret_cast<float*>(sC);             // [2][BN]
+      const int tid = (int)threadIdx.x - 64;
+      if (leader) tma_store_wait_read<0>();
+      named_barrier_sync(1 + NUM_GROUPS, NUM_GROUPS * GROUP_THREADS);
+      if (tid < 2 * BN) sums[tid] = 0.0f;
+      named_barrier_sync(1 + NUM_GROUPS, NUM_GROUPS * GROUP_THREADS);
+      const float2 s = unpack_f32x2(st_sum), sq = unpack_f32x2(st_sq);
+      float* mine = sums + pnl * 64 + cp * 2;
+      atomicAdd(mine, s.x);
+      atomicAdd(mine + 1, s.y);
+      atomicAdd(mine + BN, sq.x);
+      atomicAdd(mine + BN + 1, sq.y);
+      named_barrier_sync(1 + NUM_GROUPS, NUM_GROUPS * GROUP_THREADS);
+      const int c = tid % BN, col = t.n0 + c;
+      if (tid < 2 * BN && col < ep.n_total) atomicAdd((tid < BN ? ep.col_sum : ep.col_sqsum) + col, sums[tid]);
+    }
+    if (leader) tma_store_wait_all();                // shared memory must outlive the bulk stores
   }
 
   // ---------------------------------------------------------------- teardown

@@ -18,12 +18,13 @@
 
 extern "C" {
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn, int b_mn,
-                   int out_mode, const void* bias, int relu, int splits, float* col_sum, float* col_sqsum,
+                   int out_mode, const float* scale, const void* bias, int relu, int splits, float* col_sum, float* col_sqsum,
                    const void* residual, int ldr, int* error_flag, void* stream);
 int esgd_conv2d_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S, int stride,
-                    int pad, int relu, float* col_sum, float* col_sqsum, int* error_flag, void* stream);
+                    int pad, const float* scale, const float* bias, const void* residual, int relu, float* col_sum,
+                    float* col_sqsum, int* error_flag, void* stream);
 int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, int R, int S, int stride,
-                      int pad, int* error_flag, void* stream);
+                      int pad, const void* residual, int* error_flag, void* stream);
 int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
                       int stride, int pad, int* error_flag, void* stream);
 int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
@@ -262,8 +263,8 @@ Sink load_sink(AutogradContext* ctx, const char* key) {
 // ---------------------------------------------------------------- GEMM
 int gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, int64_t ldc,
          bool a_mn, bool b_mn, int mode, int splits, float* cs, float* cq, const void* res, int64_t ldr, const Tensor& like,
-         const void* bias = nullptr, int flags = 0) {
-  return esgd_gemm_bf16(a, b, c, (int)m, (int)n, (int)k, (int)lda, (int)ldb, (int)ldc, a_mn, b_mn, mode, bias, flags, splits, cs,
+         const void* bias = nullptr, int flags = 0, const float* scale = nullptr) {
+  return esgd_gemm_bf16(a, b, c, (int)m, (int)n, (int)k, (int)lda, (int)ldb, (int)ldc, a_mn, b_mn, mode, scale, bias, flags, splits, cs,
                         cq, res, (int)ldr, flag_ptr(like), stream_of(like));
 }
 
@@ -318,8 +319,8 @@ struct ConvFn : public Function<ConvFn> {
     } else if (kind == kGeneral) {
       wk = nhwc(w);                                   // [Cout][R][S][Cin] in memory
       saved_x = x;
-      ck(esgd_conv2d_fwd(x.data_ptr(), wk.data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, 0, cs, cq, flag_ptr(x),
-                         st), "conv2d");
+      ck(esgd_conv2d_fwd(x.data_ptr(), wk.data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, nullptr, nullptr, nullptr, 0,
+                         cs, cq, flag_ptr(x), st), "conv2d");
     } else {
       wk = nhwc(w);
       const StemGeometry g(cin, r, s);
@@ -378,10 +379,11 @@ struct ConvFn : public Function<ConvFn> {
       const bool square = r == s && pad <= r - 1;
       dx = empty_nhwc(n, cin, h, wd, x);
       if (square && stride == 1) {
-        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, flag_ptr(x), st),
-           "conv2d data gradient");
+        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad,
+                             d_tap.defined() ? nhwc(d_tap).data_ptr() : nullptr, flag_ptr(x), st), "conv2d data gradient");
+        d_tap = Tensor();
       } else if (stride == 2 && r == 3 && s == 3 && pad == 1 && h % 2 == 0 && wd % 2 == 0) {
-        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, 3, 3, 2, 1, flag_ptr(x), st),
+        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, 3, 3, 2, 1, nullptr, flag_ptr(x), st),
            "strided conv2d data gradient");
       } else if (square) {
         // Any other stride / size: the gradient is spread out with (stride - 1) zeros between its pixels (plus the rows and
@@ -389,7 +391,7 @@ struct ConvFn : public Function<ConvFn> {
         const int64_t eh = (h + 2 * pad - r) % stride, ew = (wd + 2 * pad - s) % stride;
         Tensor spread = at::zeros({n, cout, (ho - 1) * stride + 1 + eh, (wo - 1) * stride + 1 + ew}, dy.options()).contiguous(kCL);
         spread.slice(2, 0, (ho - 1) * stride + 1, stride).slice(3, 0, (wo - 1) * stride + 1, stride).copy_(dy);
-        ck(esgd_conv2d_dgrad(spread.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, flag_ptr(x), st),
+        ck(esgd_conv2d_dgrad(spread.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, nullptr, flag_ptr(x), st),
            "conv2d data gradient");
       } else {
         dx = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {stride, stride}, {pad, pad}, {1, 1}, false, {0, 0}, 1,
@@ -442,8 +444,8 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
   else if (r > 1 && c <= 4 && k0 % 8 == 0 && !x.requires_grad()) kind = kStem;
   else if (r > 1 && c % 8 == 0 && k0 % 8 == 0 && stride <= 2 && (narrow || c % 64 == 0)) kind = kGeneral;
   else return py::none();
-  // only the 1x1 data gradient adds the shortcut's gradient in its epilogue: elsewhere the tap is the input itself
-  const bool fuse_tap = tap && kind == kOneByOne && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
+  // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
+  const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
   Sink sink = find_sink(w);
   sink_use(sink);
   variable_list out = ConvFn::apply(x, graph_input(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink));

@@ -24,7 +24,7 @@ def _lib():
     lib = N.cuda()
     if not getattr(lib, "_gemm_bound", False):
         lib.esgd_gemm_bf16.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p] + [C.c_int] * 9 + \
-            [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+            [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
         lib._gemm_bound = True
     return lib
 
@@ -69,7 +69,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_kmajor: bool = True, b_kmajor: b
         assert residual.dtype == torch.bfloat16 and residual.shape == (M, Nn) and residual.stride(1) == 1 and mode == 0
     stream = torch.cuda.current_stream(a.device).cuda_stream
     rc = _lib().esgd_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, a.stride(0), b.stride(0),
-                               out.stride(0), int(not a_kmajor), int(not b_kmajor), mode,
+                               out.stride(0), int(not a_kmajor), int(not b_kmajor), mode, None,
                                bias.data_ptr() if bias is not None else None, int(relu), splits,
                                col_sum.data_ptr() if col_sum is not None else None,
                                col_sqsum.data_ptr() if col_sqsum is not None else None,
