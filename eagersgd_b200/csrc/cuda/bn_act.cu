@@ -3,6 +3,7 @@
 //   bn_stats        : per-channel sum / sum of squares (fp32) of a conv output
 //   bn_fwd          : mean / inv-std, scale / shift, running-statistics update and
 //                     z = act(scale*y + shift [+ residual])           (one read, one write)
+//   bn_coefficients : inference scale / shift of every layer of a network
 //   bn_bwd_reduce   : g = dz * [z > 0];  dbeta = sum g, dgamma = sum g*xhat
 //   bn_bwd_apply    : dy = gamma*invstd*(g - dbeta/M - xhat*dgamma/M), optional dres = g
 //
@@ -317,6 +318,21 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dz, const __nv_bfloat16* _
   }
 }
 
+// Inference: the affine maps of all batch norms of a network in one launch, one block per layer.
+struct CoefLayer {
+  const float *gamma, *beta, *mean, *var;
+  float* out;            // [2][C]: scale, shift
+  int64_t C;
+};
+__global__ void __launch_bounds__(256) bn_coefficients_kernel(const CoefLayer* __restrict__ layers, float eps) {
+  const CoefLayer l = layers[blockIdx.x];
+  for (int c = threadIdx.x; c < l.C; c += 256) {
+    const float sc = l.gamma[c] * rsqrtf(l.var[c] + eps);
+    l.out[c] = sc;
+    l.out[l.C + c] = l.beta[c] - l.mean[c] * sc;
+  }
+}
+
 int blocks_for(int64_t work_items, int per_block, int64_t cap = 148 * 16) {
   int64_t b = (work_items + per_block - 1) / per_block;
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
@@ -368,6 +384,12 @@ int esgd_bn_fwd(const void* y, const void* residual, void* z, const float* sum, 
     case 4: ESGD_BN_FWD(4); break;
     default: ESGD_BN_FWD(2); break;
   }
+  esgd::count_launch();
+  return (int)cudaGetLastError();
+}
+
+int esgd_bn_coefficients(const void* layers, int n, float eps, void* stream) {
+  bn_coefficients_kernel<<<n, 256, 0, (cudaStream_t)stream>>>((const CoefLayer*)layers, eps);
   esgd::count_launch();
   return (int)cudaGetLastError();
 }

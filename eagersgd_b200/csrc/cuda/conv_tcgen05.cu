@@ -520,9 +520,10 @@ Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* er
 
 template <bool kT>
 int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
-  const int BN = a.Cout <= 64 ? 64 : (a.Cout <= 128 ? 128 : 256);
+  const int Ho = a.out_h ? a.out_h : (a.H + 2 * a.pad - a.R) / a.stride + 1, Wo = a.out_w ? a.out_w : (a.W + 2 * a.pad - a.S) / a.stride + 1;
+  const int BN = tile_columns(a.Cout, (int)(((int64_t)a.N * Ho * Wo + BM - 1) / BM), sm_count());
   int bh = 0;
-  if (BN <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
+  if (a.Cout <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
     return BN == 64 ? launch_halo<64, kT>(a, ep, bh, s) : launch_halo<128, kT>(a, ep, bh, s);
   if (BN == 64) return launch<64, kT>(a, ep, s);
   if (BN == 128) return launch<128, kT>(a, ep, s);

@@ -248,7 +248,7 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
   ep.tx_bytes = 0; ep.tx_bytes_a = 0;
   ep.residual = residual; ep.ldr = ldr;
   cudaStream_t s = (cudaStream_t)stream;
-  const int BN = N <= 64 ? 64 : (N <= 128 ? 128 : 256);
+  const int BN = tile_columns(N, (M + BM - 1) / BM * (splits > 1 ? splits : 1), sm_count());
   if (BN == 64) return launch_major<64>(a_mn, b_mn, g, ep, s);
   if (BN == 128) return launch_major<128>(a_mn, b_mn, g, ep, s);
   return launch_major<256>(a_mn, b_mn, g, ep, s);

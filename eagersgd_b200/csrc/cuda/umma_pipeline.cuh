@@ -88,6 +88,15 @@ struct Cfg {
 constexpr int HALO_BYTES = 32 * 1024;        // one input box (incl. the rows a shifted view may touch past it)
 constexpr int MAX_HALOS = 3;
 
+// Columns of a tile for `n` output columns and `m_tiles` row tiles.  Wide tiles re-read the rows least, but a problem with
+// few of them leaves SMs idle while each CTA walks the whole reduction: as long as twice the tiles still fit one wave,
+// half the width is faster (one image, 7x7 pixels, 3x3 over 512 channels: 2 CTAs of 72 blocks become 8).
+inline int tile_columns(int n, int m_tiles, int sms) {
+  int bn = n <= 64 ? 64 : (n <= 128 ? 128 : 256);
+  while (bn > 64 && 2 * m_tiles * ((n + bn - 1) / bn) <= sms) bn /= 2;
+  return bn;
+}
+
 // ESGD_GEMM_B_RESIDENT=0 in the environment turns the B-resident mode off (for A/B timing).
 inline bool resident_enabled() {
   static int v = -1;

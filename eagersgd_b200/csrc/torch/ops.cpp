@@ -39,6 +39,7 @@ int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, voi
 int esgd_bn_fwd(const void* y, const void* residual, void* z, const float* sum, const float* sqsum, const float* gamma,
                 const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu,
                 float momentum, float eps, void* stream);
+int esgd_bn_coefficients(const void* layers, int n, float eps, void* stream);
 int esgd_bn_bwd_reduce(const void* dz, const void* z, const void* y, const float* mean, const float* invstd,
                        const float* fscale, const float* fshift, int64_t M, int C, int relu, float* dbeta, float* dgamma,
                        void* stream);
@@ -288,6 +289,47 @@ struct StemGeometry {
   }
 };
 
+// What a convolution's epilogue does to the product: statistics of it (training), or the affine map of an inference batch
+// norm, a residual and a ReLU.
+struct ConvEpilogue {
+  float *sum = nullptr, *sqsum = nullptr;
+  const float *scale = nullptr, *shift = nullptr;
+  const void* residual = nullptr;
+  bool relu = false;
+};
+
+// Launches the convolution of NHWC x with w into y; `kept` and `filters` are what a backward pass needs of the two.
+void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y, int64_t stride, int64_t pad, const ConvEpilogue& e,
+                 Tensor* kept, Tensor* filters) {
+  const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3), cout = w.size(0), r = w.size(2), s = w.size(3);
+  const int64_t ho = y.size(2), wo = y.size(3);
+  void* st = stream_of(x);
+  if (kind == kOneByOne) {
+    *filters = w.contiguous();                      // [Cout, Cin]: a 1x1 filter has one memory order
+    *kept = x;
+    if (stride == 2) {
+      *kept = empty_nhwc(n, cin, ho, wo, x);
+      ck(esgd_subsample2_fwd(x.data_ptr(), kept->data_ptr(), n, h, wd, cin, st), "subsample");
+    }
+    ck(gemm(kept->data_ptr(), filters->data_ptr(), y.data_ptr(), n * ho * wo, cout, cin, cin, cin, cout, false, false, 0, 1, e.sum,
+            e.sqsum, e.residual, cout, x, e.shift, e.relu, e.scale), "1x1 convolution");
+  } else if (kind == kGeneral) {
+    *filters = nhwc(w);                             // [Cout][R][S][Cin] in memory
+    *kept = x;
+    ck(esgd_conv2d_fwd(x.data_ptr(), filters->data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, e.scale, e.shift,
+                       e.residual, e.relu, e.sum, e.sqsum, flag_ptr(x), st), "conv2d");
+  } else {
+    *filters = nhwc(w);
+    const StemGeometry g(cin, r, s);
+    *kept = at::empty({n * ho * wo, g.kpad}, x.options());
+    ck(esgd_im2col_small_c(x.data_ptr(), kept->data_ptr(), n, h, wd, cin, r, s, stride, pad, g.seg, g.kpad, st), "im2col");
+    Tensor w2d = at::empty({cout, g.kpad}, x.options());
+    ck(esgd_stem_pack(filters->data_ptr(), w2d.data_ptr(), cout, r, s * cin, g.seg, g.kpad, st), "stem filters");
+    ck(gemm(kept->data_ptr(), w2d.data_ptr(), y.data_ptr(), n * ho * wo, cout, g.kpad, g.kpad, g.kpad, cout, false, false, 0, 1, e.sum,
+            e.sqsum, e.residual, cout, x, e.shift, e.relu, e.scale), "stem convolution");
+  }
+}
+
 // y = x (*) w, and on request the per-channel sum / sum of squares of y and the input itself.
 //
 // With `tap` the input is returned as a last output.  A residual block takes its shortcut from that output instead of
@@ -301,36 +343,16 @@ struct ConvFn : public Function<ConvFn> {
     const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3);
     const int64_t cout = w.size(0), r = w.size(2), s = w.size(3);
     const int64_t ho = (h + 2 * pad - r) / stride + 1, wo = (wd + 2 * pad - s) / stride + 1;
-    void* st = stream_of(x);
     Tensor stats;
-    if (want_stats) stats = zeros_f32({2, cout}, x.device());
-    float *cs = fptr(stats), *cq = want_stats ? cs + cout : nullptr;
+    ConvEpilogue e;
+    if (want_stats) {
+      stats = zeros_f32({2, cout}, x.device());
+      e.sum = fptr(stats);
+      e.sqsum = e.sum + cout;
+    }
     Tensor y = empty_nhwc(n, cout, ho, wo, x);
     Tensor saved_x, wk;
-    if (kind == kOneByOne) {
-      wk = w.contiguous();                            // [Cout, Cin]: a 1x1 filter has one memory order
-      saved_x = x;
-      if (stride == 2) {
-        saved_x = empty_nhwc(n, cin, ho, wo, x);
-        ck(esgd_subsample2_fwd(x.data_ptr(), saved_x.data_ptr(), n, h, wd, cin, st), "subsample");
-      }
-      ck(gemm(saved_x.data_ptr(), wk.data_ptr(), y.data_ptr(), n * ho * wo, cout, cin, cin, cin, cout, false, false, 0, 1, cs, cq,
-              nullptr, 0, x), "1x1 convolution");
-    } else if (kind == kGeneral) {
-      wk = nhwc(w);                                   // [Cout][R][S][Cin] in memory
-      saved_x = x;
-      ck(esgd_conv2d_fwd(x.data_ptr(), wk.data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, nullptr, nullptr, nullptr, 0,
-                         cs, cq, flag_ptr(x), st), "conv2d");
-    } else {
-      wk = nhwc(w);
-      const StemGeometry g(cin, r, s);
-      saved_x = at::empty({n * ho * wo, g.kpad}, x.options());
-      ck(esgd_im2col_small_c(x.data_ptr(), saved_x.data_ptr(), n, h, wd, cin, r, s, stride, pad, g.seg, g.kpad, st), "im2col");
-      Tensor w2d = at::empty({cout, g.kpad}, x.options());
-      ck(esgd_stem_pack(wk.data_ptr(), w2d.data_ptr(), cout, r, s * cin, g.seg, g.kpad, st), "stem filters");
-      ck(gemm(saved_x.data_ptr(), w2d.data_ptr(), y.data_ptr(), n * ho * wo, cout, g.kpad, g.kpad, g.kpad, cout, false, false, 0, 1,
-              cs, cq, nullptr, 0, x), "stem convolution");
-    }
+    launch_conv(kind, x, w, y, stride, pad, e, &saved_x, &wk);
     ctx->save_for_backward({saved_x, wk});
     ctx->saved_data["cfg"] = std::vector<int64_t>{kind, stride, pad, n, cin, h, wd, want_stats, tap};
     save_sink(ctx, "w", sink);
@@ -436,14 +458,19 @@ struct ConvFn : public Function<ConvFn> {
   }
 };
 
+// Which kernel takes a convolution; -1: none, the shape is not this package's.
+int64_t conv_kind(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool narrow) {
+  const int64_t c = x.size(1), k0 = w.size(0), r = w.size(2), s = w.size(3);
+  if (r == 1 && s == 1 && pad == 0 && stride <= 2 && c % 8 == 0 && k0 % 8 == 0) return kOneByOne;
+  if (r > 1 && c <= 4 && k0 % 8 == 0 && !x.requires_grad()) return kStem;
+  if (r > 1 && c % 8 == 0 && k0 % 8 == 0 && stride <= 2 && (narrow || c % 64 == 0)) return kGeneral;
+  return -1;
+}
+
 // Returns (y, stats | None, tapped input | None), or None when the shape is not this package's.
 py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap, bool narrow) {
-  const int64_t c = x.size(1), k0 = w.size(0), r = w.size(2), s = w.size(3);
-  int64_t kind;
-  if (r == 1 && s == 1 && pad == 0 && stride <= 2 && c % 8 == 0 && k0 % 8 == 0) kind = kOneByOne;
-  else if (r > 1 && c <= 4 && k0 % 8 == 0 && !x.requires_grad()) kind = kStem;
-  else if (r > 1 && c % 8 == 0 && k0 % 8 == 0 && stride <= 2 && (narrow || c % 64 == 0)) kind = kGeneral;
-  else return py::none();
+  const int64_t r = w.size(2), s = w.size(3), kind = conv_kind(x, w, stride, pad, narrow);
+  if (kind < 0) return py::none();
   // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
   const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
   Sink sink = find_sink(w);
@@ -453,6 +480,68 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
   py::object tp = !tap ? py::none() : py::cast(fuse_tap ? out.back() : x);
   return py::make_tuple(out[0], st, tp);
 }
+
+// Inference: act(batch_norm(conv(x)) + residual) in one kernel.  coef [2][Cout] fp32: scale and shift (BnCoefficients), or
+// None for a bare convolution.  No autograd; None when the shape is not this package's.
+py::object conv_bn_eval(const Tensor& x_in, const Tensor& w, int64_t stride, int64_t pad, const c10::optional<Tensor>& coef,
+                        const c10::optional<Tensor>& residual, bool relu, bool narrow) {
+  const int64_t kind = conv_kind(x_in, w, stride, pad, narrow);
+  if (kind < 0 || w.scalar_type() != at::kBFloat16) return py::none();
+  c10::cuda::CUDAGuard guard(x_in.device());
+  Tensor x = nhwc(x_in), res = residual.has_value() ? nhwc(*residual) : Tensor(), kept, filters;
+  const int64_t cout = w.size(0);
+  Tensor y = empty_nhwc(x.size(0), cout, (x.size(2) + 2 * pad - w.size(2)) / stride + 1, (x.size(3) + 2 * pad - w.size(3)) / stride + 1, x);
+  ConvEpilogue e;
+  if (coef.has_value()) {
+    e.scale = fptr(*coef);
+    e.shift = e.scale + cout;
+  }
+  if (res.defined()) e.residual = res.data_ptr();
+  e.relu = relu;
+  launch_conv(kind, x, w, y, stride, pad, e, &kept, &filters);
+  return py::cast(y);
+}
+
+// The affine maps of a network's batch norms, computed from their parameters and running statistics by one launch per
+// forward pass.  The table of pointers lives on the device and is rebuilt when a tensor has moved.
+class BnCoefficients {
+ public:
+  std::vector<Tensor> compute(const std::vector<std::array<Tensor, 4>>& layers) {      // gamma, beta, mean, var
+    std::lock_guard<std::mutex> g(m_);
+    c10::cuda::CUDAGuard guard(layers.at(0)[0].device());
+    std::vector<int64_t> key;
+    key.reserve(layers.size() * 6);
+    for (const auto& l : layers) {
+      for (const auto& t : l) key.push_back((int64_t)t.data_ptr<float>());
+      key.push_back(0);
+      key.push_back(l[0].numel());
+    }
+    if (key != key_) {
+      key_ = key;
+      int64_t total = 0;
+      for (const auto& l : layers) total += 2 * l[0].numel();
+      const auto opt = layers[0][0].options().requires_grad(false);
+      Tensor buf = at::empty({total}, opt);
+      out_.clear();
+      int64_t off = 0;
+      for (size_t i = 0; i < layers.size(); ++i) {
+        const int64_t c = layers[i][0].numel();
+        out_.push_back(buf.narrow(0, off, 2 * c));
+        key[6 * i + 4] = (int64_t)out_.back().data_ptr<float>();
+        off += 2 * c;
+      }
+      table_ = at::tensor(key, at::kLong).to(buf.device());
+    }
+    ck(esgd_bn_coefficients(table_.data_ptr(), (int)layers.size(), kBnEps, stream_of(table_)), "batch-norm coefficients");
+    return out_;
+  }
+
+ private:
+  std::mutex m_;
+  std::vector<int64_t> key_;
+  std::vector<Tensor> out_;
+  Tensor table_;
+};
 
 // ---------------------------------------------------------------- dense layer: fp32 logits out of bf16 operands
 struct LinearFn : public Function<LinearFn> {
@@ -777,6 +866,8 @@ PYBIND11_MODULE(_esgd_torch, m) {
   m.def("zeros_f32", [](std::vector<int64_t> shape, at::Device d) { return zeros_f32(shape, d); });
   m.def("wgrad_splits", &wgrad_splits, py::arg("pixels"), py::arg("cout"), py::arg("cin"), py::arg("sms") = 148);
   m.def("conv2d", &conv2d);
+  m.def("conv_bn_eval", &conv_bn_eval);
+  py::class_<BnCoefficients, std::shared_ptr<BnCoefficients>>(m, "BnCoefficients").def(py::init<>()).def("compute", &BnCoefficients::compute);
   m.def("linear", &linear);
   m.def("bn_act", &bn_act);
   m.def("softmax_ce", &softmax_ce);

@@ -12,14 +12,20 @@ Activations are NHWC (channels_last) bf16 on GPUs.
 """
 from __future__ import annotations
 
+import weakref
 from typing import List, Tuple
 
+import torch
 import torch.nn as nn
 
 from ..ops import functional as ops
 
 BN_MOMENTUM_TF = 0.997  # tf decay; torch momentum = 1 - decay
 BN_EPS = 1e-5
+
+# what the fused inference path keeps per network (module lists, device tables); not an attribute of the module, which has
+# to stay copyable and picklable
+_eval_state = weakref.WeakKeyDictionary()
 
 IMAGENET_BLOCKS = {
     18: ("building", [2, 2, 2, 2]), 34: ("building", [3, 4, 6, 3]), 50: ("bottleneck", [3, 4, 6, 3]),
@@ -37,7 +43,6 @@ class BatchNormAct(nn.BatchNorm2d):
     def forward(self, y, relu: bool = True, residual=None, stats=None):  # noqa: D102
         v = self.virtual_batch_size
         if v and self.training and y.shape[0] > v:
-            import torch
             outs = [ops.bn_act(y[i:i + v], self.weight, self.bias, self.running_mean, self.running_var, self.momentum,
                                relu, None if residual is None else residual[i:i + v], None, True)
                     for i in range(0, y.shape[0], v)]
@@ -159,7 +164,62 @@ class ResNet(nn.Module):
         self.registry.append(("dense", self.fc))
         self.feature_dim = cin
 
+    # ---- inference: every convolution with its batch norm, shortcut and ReLU as one kernel
+    def _fused_eval(self, x):
+        """The coefficients of the network's batch norms by module, when the fused inference path applies: no gradients,
+        every layer in evaluation mode and nobody listening to a layer's output; else None."""
+        if self.training or torch.is_grad_enabled() or not ops.native(x):
+            return None
+        st = _eval_state.get(self)
+        if st is None:
+            norms = [m for m in self.modules() if isinstance(m, BatchNormAct)]
+            st = _eval_state[self] = {"norms": norms, "modules": [m for m in self.modules() if m is not self]}
+        for m in st["modules"]:
+            if m.training or m._forward_hooks or m._forward_pre_hooks:
+                return None
+        layers = [(m.weight, m.bias, m.running_mean, m.running_var) for m in st["norms"]]
+        if not all(t is not None and t.is_cuda and t.dtype == torch.float32 for layer in layers for t in layer):
+            return None
+        return dict(zip(st["norms"], ops.bn_coefficients(layers, st)))
+
+    @staticmethod
+    def _conv_eval(conv, bn, x, coef, relu, residual=None):
+        y = ops.conv_bn_eval(x, conv.weight, conv.stride[0], conv.padding[0], coef[bn] if bn is not None else None, relu, residual)
+        if y is None:
+            y = conv(x)[0]
+            if bn is not None:
+                return bn(y, relu=relu, residual=residual)
+            y = y + residual if residual is not None else y
+        return y
+
+    def _features_eval(self, x, coef):
+        conv = self._conv_eval
+        x = conv(self.stem, self.stem_bn, x, coef, self.stem_bn is not None)
+        if self.first_pool:
+            x = ops.max_pool_3x3_s2(x)
+        for blk in self.blocks:
+            n, y, shortcut = len(blk.convs), x, x
+            if self.version == 1:
+                if blk.proj is not None:
+                    shortcut = conv(blk.proj, blk.proj_bn, x, coef, False)
+                for i in range(n):
+                    y = conv(blk.convs[i], blk.bns[i], y, coef, True, shortcut if i == n - 1 else None)
+            else:
+                y = blk.pre_bn(x, relu=True)
+                if blk.proj is not None:
+                    shortcut = conv(blk.proj, None, y, coef, False)
+                for i in range(n):
+                    last = i == n - 1
+                    y = conv(blk.convs[i], None if last else blk.bns[i], y, coef, not last, shortcut if last else None)
+            x = y
+        if self.final_bn is not None:
+            x = self.final_bn(x, relu=True)
+        return ops.global_avg_pool(x)
+
     def features(self, x):
+        coef = self._fused_eval(x)
+        if coef is not None:
+            return self._features_eval(x, coef)
         x, st = self.stem(x)
         if self.stem_bn is not None:
             x = self.stem_bn(x, relu=True, stats=st)

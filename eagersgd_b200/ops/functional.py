@@ -151,6 +151,21 @@ def bn_act(y: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, running_mea
     return F.relu(z) if relu else z
 
 
+# --------------------------------------------------------------------------- inference: convolution + batch norm in one kernel
+def bn_coefficients(layers, store):
+    """Scale and shift (``[2 * C]`` fp32, one after the other) of each inference batch norm in ``layers`` -- tuples of gamma,
+    beta, running mean, running variance -- from one launch.  ``store``: a dict of the caller's that keeps the device table."""
+    if "bn" not in store:
+        store["bn"] = _ext().BnCoefficients()
+    return store["bn"].compute(layers)
+
+
+def conv_bn_eval(x: torch.Tensor, w: torch.Tensor, stride: int, padding: int, coef: Optional[torch.Tensor], relu: bool,
+                 residual: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """act(scale * conv(x) + shift [+ residual]) rounded once, without autograd; None for shapes the kernels do not take."""
+    return _ext().conv_bn_eval(x, w, stride, padding, coef, residual, relu, _SMALL_CHANNELS_NATIVE)
+
+
 # --------------------------------------------------------------------------- softmax cross-entropy
 def softmax_cross_entropy(logits: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
     """Mean sparse softmax cross-entropy; forward and gradient come out of one kernel."""
