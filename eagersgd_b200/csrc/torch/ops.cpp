@@ -29,6 +29,11 @@ int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, in
                       int stride, int pad, int* error_flag, void* stream);
 int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
                            int pad, int* error_flag, void* stream);
+int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int stride, const float* scale,
+                         const float* shift, const void* residual, int relu, float* sum, float* sqsum, void* stream);
+int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, const void* residual,
+                           void* stream);
+int esgd_conv_narrow_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int stride, void* stream);
 int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, int R, int S, int stride, int pad, int seg,
                         int Kpad, void* stream);
 int esgd_stem_pack(const void* w, void* out, int Cout, int R, int sc, int seg, int Kpad, void* stream);
@@ -280,6 +285,8 @@ int wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int64_t sms = 148) {
 // ---------------------------------------------------------------- convolutions
 enum ConvKind : int64_t { kOneByOne = 0, kGeneral = 1, kStem = 2 };
 
+constexpr int kNotTaken = -100;      // a kernel's answer to a shape outside its range: the next one takes it
+
 struct StemGeometry {
   int64_t seg, kpad;
   StemGeometry(int64_t c, int64_t r, int64_t s) {
@@ -316,8 +323,14 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
   } else if (kind == kGeneral) {
     *filters = nhwc(w);                             // [Cout][R][S][Cin] in memory
     *kept = x;
-    ck(esgd_conv2d_fwd(x.data_ptr(), filters->data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, e.scale, e.shift,
-                       e.residual, e.relu, e.sum, e.sqsum, flag_ptr(x), st), "conv2d");
+    int rc = kNotTaken;
+    if (r == 3 && s == 3 && pad == 1)
+      rc = esgd_conv_narrow_fwd(x.data_ptr(), filters->data_ptr(), y.data_ptr(), n, h, wd, cin, cout, stride, e.scale, e.shift,
+                                e.residual, e.relu, e.sum, e.sqsum, st);
+    if (rc == kNotTaken)
+      rc = esgd_conv2d_fwd(x.data_ptr(), filters->data_ptr(), y.data_ptr(), n, h, wd, cin, cout, r, s, stride, pad, e.scale, e.shift,
+                           e.residual, e.relu, e.sum, e.sqsum, flag_ptr(x), st);
+    ck(rc, "conv2d");
   } else {
     *filters = nhwc(w);
     const StemGeometry g(cin, r, s);
@@ -401,8 +414,15 @@ struct ConvFn : public Function<ConvFn> {
       const bool square = r == s && pad <= r - 1;
       dx = empty_nhwc(n, cin, h, wd, x);
       if (square && stride == 1) {
-        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad,
-                             d_tap.defined() ? nhwc(d_tap).data_ptr() : nullptr, flag_ptr(x), st), "conv2d data gradient");
+        Tensor res;
+        if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
+        const void* rp = res.defined() ? res.data_ptr() : nullptr;
+        int rc = kNotTaken;
+        if (r == 3 && pad == 1)
+          rc = esgd_conv_narrow_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, rp, st);
+        if (rc == kNotTaken)
+          rc = esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, rp, flag_ptr(x), st);
+        ck(rc, "conv2d data gradient");
         d_tap = Tensor();
       } else if (stride == 2 && r == 3 && s == 3 && pad == 1 && h % 2 == 0 && wd % 2 == 0) {
         ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, 3, 3, 2, 1, nullptr, flag_ptr(x), st),
@@ -434,10 +454,12 @@ struct ConvFn : public Function<ConvFn> {
         Tensor dw32;
         if (!sink) dw32 = zeros_f32({cout, r, s, cin}, x.device());
         float* acc = sink ? sink->acc : fptr(dw32);
-        int rc = -100;
-        if (stride == 1)         // shared input boxes, taps as shifted views (returns -100 outside its range)
+        int rc = kNotTaken;
+        if (r == 3 && s == 3 && pad == 1)
+          rc = esgd_conv_narrow_wgrad(x.data_ptr(), dy.data_ptr(), acc, n, h, wd, cin, cout, stride, st);
+        if (rc == kNotTaken && stride == 1)      // shared input boxes, taps as shifted views
           rc = esgd_conv2d_wgrad_halo(x.data_ptr(), dy.data_ptr(), acc, n, h, wd, cin, cout, r, s, pad, flag_ptr(x), st);
-        if (rc == -100)
+        if (rc == kNotTaken)
           rc = esgd_conv2d_wgrad(x.data_ptr(), dy.data_ptr(), acc, n, h, wd, cin, cout, r, s, stride, pad, flag_ptr(x), st);
         ck(rc, "conv2d weight gradient");
         if (!sink) dw = dw32.to(w.scalar_type()).permute({0, 3, 1, 2});
