@@ -11,7 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <atomic>
-#include "launch_count.cuh"
+#include "launch.cuh"
 
 namespace {
 
@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(kThreads) conv_narrow_kernel(const Shape s, co
   __shared__ float s_stat[2 * CN];
   uint8_t* sW = smem;                                          // [9][COUT] rows
   uint8_t* sX = smem + 9 * COUT * WR;
+  esgd::pdl_enter();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = warp / WN, wn = warp % WN;
   for (int i = threadIdx.x; i < 9 * COUT * (CIN / 8); i += kThreads) {      // filters: [COUT][9][CIN] -> [9][COUT][CIN]
     const int ch = i % (CIN / 8), rest = i / (CIN / 8), tap = rest % 9, co = rest / 9;
@@ -190,6 +191,7 @@ __global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS) wgrad_narrow_kerne
   extern __shared__ __align__(16) uint8_t smem[];
   uint8_t* sX = smem;
   uint8_t* sD = smem + s.ti * s.rows * s.pw * PX;
+  esgd::pdl_enter();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp % P::SETS, slice = warp / P::SETS;
   float acc[P::TAPS][MT][NT][4];
 #pragma unroll
@@ -328,9 +330,7 @@ int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t str
   const int smem = 9 * cout * (cin * 2 + 16) + s.ti * s.rows * s.pw * (CR * 2 + 16);
   if (smem > kSmemMax) return -100;
   const int resident = blocks_per_sm(conv_narrow_kernel<CR, CN, kT>, kThreads, smem, occ) * 148;
-  conv_narrow_kernel<CR, CN, kT><<<s.tiles < resident ? s.tiles : resident, kThreads, smem, stream>>>(s, a);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(conv_narrow_kernel<CR, CN, kT>, dim3(s.tiles < resident ? s.tiles : resident), kThreads, smem, stream, s, a);
 }
 
 template <int CI, int CO>
@@ -345,9 +345,8 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
   blocks_per_sm(wgrad_narrow_kernel<CI, CO>, WgradPlan<CI, CO>::THREADS, smem, occ);
   // one block per SM at most: every block ends with a reduction of the whole filter bank
   const int grid = s.tiles < 148 ? s.tiles : 148;
-  wgrad_narrow_kernel<CI, CO><<<grid, WgradPlan<CI, CO>::THREADS, smem, stream>>>(s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, dw);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), WgradPlan<CI, CO>::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
+                      (const __nv_bfloat16*)dy, dw);
 }
 
 }  // namespace

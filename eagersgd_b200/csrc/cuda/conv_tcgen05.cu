@@ -20,7 +20,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
-#include "launch_count.cuh"
+#include "launch.cuh"
 #include "tensormap.cuh"
 #include "umma_pipeline.cuh"
 
@@ -357,9 +357,7 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
   }
   ep.tx_bytes_a = (uint32_t)(p.BW * p.BH * p.BI * 128);
   ep.tx_bytes = ep.tx_bytes_a + (uint32_t)Cfg<BN>::B_STAGE_BYTES;
-  conv_kernel<P><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(p, ep);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(conv_kernel<P>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 // Halo mode applies to stride-1 convolutions with full-width tiles: the box (output rows + filter margin, full
@@ -432,9 +430,7 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
   if (grid > total) grid = total;
   ep.tx_bytes_a = (uint32_t)(p.PW * (bh + a.R - 1) * 128);
   ep.tx_bytes = 0;
-  conv_kernel<P><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(p, ep);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(conv_kernel<P>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 template <int BN>
@@ -505,9 +501,7 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
   ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
   const int total = base_tiles * p.splits;
   const int grid = total < sms ? total : sms;
-  conv_wgrad_kernel<P><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(p, ep);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(conv_wgrad_kernel<P>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* error_flag) {

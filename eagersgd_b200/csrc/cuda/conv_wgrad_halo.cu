@@ -13,7 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
-#include "launch_count.cuh"
+#include "launch.cuh"
 #include "sm100_primitives.cuh"
 #include "tensormap.cuh"
 
@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  esgd::pdl_enter();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -274,9 +275,7 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
     if (r != 0) return 2000 + r;
   }
   const int grid = p.sets * p.m_tiles * p.n_tiles * p.splits;
-  conv_wgrad_halo_kernel<BN><<<grid, WG_THREADS, WG_SMEM, stream>>>(p);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(conv_wgrad_halo_kernel<BN>, dim3(grid), WG_THREADS, WG_SMEM, stream, p);
 }
 
 }  // namespace

@@ -10,9 +10,11 @@
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
-#include "launch_count.cuh"
+#include "launch.cuh"
 
 namespace {
+
+using esgd::pdl_enter;
 
 template <typename T> __device__ __forceinline__ float to_f(T v);
 template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
@@ -43,6 +45,7 @@ __global__ void __launch_bounds__(256) softmax_ce_kernel(const T* __restrict__ l
                                                          int classes, int ld, float inv_batch, float grad_scale,
                                                          float* __restrict__ loss_sum, float* __restrict__ per_sample,
                                                          T* __restrict__ dlogits) {
+  pdl_enter();
   __shared__ float sh[8];
   const int row = blockIdx.x;
   const T* x = logits + (size_t)row * ld;
@@ -90,80 +93,109 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float v[8]) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
+// One output row of an image per block (the only divisions left are by the row's own extent).
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                           __nv_bfloat16* __restrict__ y, uint8_t* __restrict__ idx,
                                                           int N, int H, int W, int C, int OH, int OW) {
+  pdl_enter();
   const int G = C / 8;
-  const int64_t total = (int64_t)N * OH * OW * G;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    int64_t t = i / G;
-    const int ow = (int)(t % OW); t /= OW;
-    const int oh = (int)(t % OH);
-    const int n = (int)(t / OH);
-    float m[8];
-    uint32_t first[8];
+  for (int row = blockIdx.x; row < N * OH; row += gridDim.x) {
+    const int n = row / OH, oh = row - n * OH;
+    const int64_t out0 = (int64_t)row * OW * G;
+    for (int i = threadIdx.x; i < OW * G; i += blockDim.x) {
+      const int ow = i / G, g = i - ow * G;
+      float m[8];
+      uint32_t first[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) { m[q] = -FLT_MAX; first[q] = 0; }
-    for (int r = 0; r < 3; ++r) {
-      const int h = oh * 2 - 1 + r;
-      if (h < 0 || h >= H) continue;
-      for (int s = 0; s < 3; ++s) {
-        const int w = ow * 2 - 1 + s;
-        if (w < 0 || w >= W) continue;
-        float v[8];
-        ld8(x + (((int64_t)n * H + h) * W + w) * C + g * 8, v);
+      for (int q = 0; q < 8; ++q) { m[q] = -FLT_MAX; first[q] = 0; }
+      uint4 raw[9];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (v[q] > m[q]) { m[q] = v[q]; first[q] = (uint32_t)(r * 3 + s); }   // first maximum in scan order
+      for (int t = 0; t < 9; ++t) {                 // every load before the first use
+        const int h = oh * 2 - 1 + t / 3, w = ow * 2 - 1 + t % 3;
+        if (h >= 0 && h < H && w >= 0 && w < W)
+          raw[t] = __ldg(reinterpret_cast<const uint4*>(x + (((int64_t)n * H + h) * W + w) * C + g * 8));
       }
-    }
-    st8(y + i * 8, m);
-    if (idx != nullptr) {
-      uint2 pk;
-      pk.x = first[0] | (first[1] << 8) | (first[2] << 16) | (first[3] << 24);
-      pk.y = first[4] | (first[5] << 8) | (first[6] << 16) | (first[7] << 24);
-      *reinterpret_cast<uint2*>(idx + i * 8) = pk;
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        const int h = oh * 2 - 1 + t / 3, w = ow * 2 - 1 + t % 3;
+        if (h < 0 || h >= H || w < 0 || w >= W) continue;
+        const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&raw[t]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = __bfloat1622float2(hv[q]);
+          if (f.x > m[2 * q]) { m[2 * q] = f.x; first[2 * q] = (uint32_t)t; }      // first maximum in scan order
+          if (f.y > m[2 * q + 1]) { m[2 * q + 1] = f.y; first[2 * q + 1] = (uint32_t)t; }
+        }
+      }
+      st8(y + (out0 + i) * 8, m);
+      if (idx != nullptr) {
+        uint2 pk;
+        pk.x = first[0] | (first[1] << 8) | (first[2] << 16) | (first[3] << 24);
+        pk.y = first[4] | (first[5] << 8) | (first[6] << 16) | (first[7] << 24);
+        *reinterpret_cast<uint2*>(idx + (out0 + i) * 8) = pk;
+      }
     }
   }
 }
 
-// Gather form: an input pixel receives dy of every window whose recorded arg-max it is.
+// Gather form: an input pixel receives dy of every window whose recorded arg-max it is.  A thread makes the 2 x 2 pixels
+// (2k, 2j) .. (2k+1, 2j+1), which meet the windows (k, j) .. (k+1, j+1) and no others: four windows are read for four
+// pixels, where a thread per pixel read nine.
 __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const uint8_t* __restrict__ idx,
                                                           const __nv_bfloat16* __restrict__ dy,
                                                           __nv_bfloat16* __restrict__ dx, int N, int H, int W, int C,
                                                           int OH, int OW) {
-  const int G = C / 8;
-  const int64_t total = (int64_t)N * H * W * G;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    int64_t t = i / G;
-    const int w = (int)(t % W); t /= W;
-    const int h = (int)(t % H);
-    const int n = (int)(t / H);
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // windows that contain row h: oh in {h/2, (h+1)/2} (one window when h is even); same for columns
-    const int ohs[2] = {h / 2, (h + 1) / 2}, ows[2] = {w / 2, (w + 1) / 2};
-    const int noh = ohs[0] == ohs[1] ? 1 : 2, now = ows[0] == ows[1] ? 1 : 2;
-    for (int a = 0; a < noh; ++a) {
-      const int oh = ohs[a];
-      if (oh >= OH) continue;
-      for (int b = 0; b < now; ++b) {
-        const int ow = ows[b];
-        if (ow >= OW) continue;
-        const uint32_t my_pos = (uint32_t)((h - (oh * 2 - 1)) * 3 + (w - (ow * 2 - 1)));
-        const int64_t o = (((int64_t)n * OH + oh) * OW + ow) * C + g * 8;
-        const uint2 pk = *reinterpret_cast<const uint2*>(idx + o);
-        float d[8];
-        ld8(dy + o, d);
+  pdl_enter();
+  const int G = C / 8, HP = (H + 1) / 2, WP = (W + 1) / 2;
+  for (int row = blockIdx.x; row < N * HP; row += gridDim.x) {
+    const int n = row / HP, k = row - n * HP;
+    for (int i = threadIdx.x; i < WP * G; i += blockDim.x) {
+      const int j = i / G, g = i - j * G;
+      uint2 pk[4];
+      uint4 dv[4];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const uint32_t word = q < 4 ? pk.x : pk.y;
-          if (((word >> ((q & 3) * 8)) & 0xffu) == my_pos) acc[q] += d[q];
+      for (int a = 0; a < 4; ++a) {
+        const int oh = k + (a >> 1), ow = j + (a & 1);
+        pk[a] = make_uint2(0xffffffffu, 0xffffffffu);          // no position: a window outside the output
+        dv[a] = make_uint4(0, 0, 0, 0);
+        if (oh < OH && ow < OW) {
+          const int64_t o = (((int64_t)n * OH + oh) * OW + ow) * C + g * 8;
+          pk[a] = __ldg(reinterpret_cast<const uint2*>(idx + o));
+          dv[a] = __ldg(reinterpret_cast<const uint4*>(dy + o));
         }
       }
+      float acc[4][8];
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[p][q] = 0.0f;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&dv[a]);
+        float d[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = __bfloat1622float2(hv[q]);
+          d[2 * q] = f.x; d[2 * q + 1] = f.y;
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {                          // pixel (2k + p/2, 2j + p%2) inside window (k + a/2, j + a%2)
+          const int r = 1 + (p >> 1) - 2 * (a >> 1), c = 1 + (p & 1) - 2 * (a & 1);
+          if (r < 0 || c < 0) continue;                        // (compile time)
+          const uint32_t pos = (uint32_t)(r * 3 + c);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t word = q < 4 ? pk[a].x : pk[a].y;
+            if (((word >> ((q & 3) * 8)) & 0xffu) == pos) acc[p][q] += d[q];
+          }
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const int h = 2 * k + (p >> 1), w = 2 * j + (p & 1);
+        if (h < H && w < W) st8(dx + (((int64_t)n * H + h) * W + w) * C + g * 8, acc[p]);
+      }
     }
-    st8(dx + i * 8, acc);
   }
 }
 
@@ -171,6 +203,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const uint8_t* __restr
 __global__ void __launch_bounds__(256) subsample2_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                              __nv_bfloat16* __restrict__ y, int N, int H, int W,
                                                              int C, int OH, int OW) {
+  pdl_enter();
   const int G = C / 8;
   const int64_t total = (int64_t)N * OH * OW * G;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -186,6 +219,7 @@ __global__ void __launch_bounds__(256) subsample2_fwd_kernel(const __nv_bfloat16
 __global__ void __launch_bounds__(256) subsample2_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                              __nv_bfloat16* __restrict__ dx, int N, int H, int W,
                                                              int C, int OH, int OW) {
+  pdl_enter();
   const int G = C / 8;
   const int64_t total = (int64_t)N * H * W * G;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -202,29 +236,39 @@ __global__ void __launch_bounds__(256) subsample2_bwd_kernel(const __nv_bfloat16
 }
 
 // ---- global average pool: [N, HW, C] -> [N, C] -----------------------------------
+// A block covers up to 16 channel groups of one image with 16 or more pixels at a time.
 __global__ void __launch_bounds__(256) avgpool_fwd_kernel(const __nv_bfloat16* __restrict__ x,
-                                                          __nv_bfloat16* __restrict__ y, int N, int HW, int C) {
-  const int G = C / 8;
-  const int64_t total = (int64_t)N * G;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int g = (int)(i % G);
-    const int n = (int)(i / G);
-    float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int p = 0; p < HW; ++p) {
+                                                          __nv_bfloat16* __restrict__ y, int N, int HW, int C, int cg) {
+  pdl_enter();
+  __shared__ float part[256 * 9];
+  const int G = C / 8, n = blockIdx.x, gl = threadIdx.x % cg, rl = threadIdx.x / cg, rows = 256 / cg;
+  const int g = blockIdx.y * cg + gl;
+  float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (g < G) {
+    for (int p = rl; p < HW; p += rows) {
       float v[8];
       ld8(x + ((int64_t)n * HW + p) * C + g * 8, v);
 #pragma unroll
       for (int q = 0; q < 8; ++q) a[q] += v[q];
     }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) part[threadIdx.x * 9 + q] = a[q];
+  __syncthreads();
+  if (rl == 0 && g < G) {
     const float inv = 1.0f / (float)HW;
+    for (int r = 1; r < rows; ++r)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] += part[(r * cg + gl) * 9 + q];
 #pragma unroll
     for (int q = 0; q < 8; ++q) a[q] *= inv;
-    st8(y + i * 8, a);
+    st8(y + ((int64_t)n * G + g) * 8, a);
   }
 }
 
 __global__ void __launch_bounds__(256) avgpool_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                           __nv_bfloat16* __restrict__ dx, int N, int HW, int C) {
+  pdl_enter();
   const int G = C / 8;
   const int64_t total = (int64_t)N * HW * G;
   const float inv = 1.0f / (float)HW;
@@ -249,6 +293,7 @@ __global__ void __launch_bounds__(256) im2col_small_c_kernel(const __nv_bfloat16
                                                              __nv_bfloat16* __restrict__ col, int N, int H, int W,
                                                              int C, int R, int S, int stride, int pad, int Ho, int Wo,
                                                              int seg, int Kpad) {
+  pdl_enter();
   const int segs = Kpad / seg;              // R real segments + zero segments
   const int64_t total = (int64_t)N * Ho * Wo * segs;
   const int sc = S * C;
@@ -286,6 +331,7 @@ __global__ void __launch_bounds__(256) im2col_rows_kernel(const __nv_bfloat16* _
                                                           __nv_bfloat16* __restrict__ col, int N, int H, int W, int C,
                                                           int R, int S, int stride, int pad, int Ho, int Wo, int seg,
                                                           int Kpad) {
+  pdl_enter();
   extern __shared__ __align__(16) uint8_t im_rows[];
   const int rowbytes = W * C * 2;
   const int pitch = kImLeftGuard + rowbytes + kImRightGuard;
@@ -324,6 +370,7 @@ __global__ void __launch_bounds__(256) im2col_rows_kernel(const __nv_bfloat16* _
 // Stem filters [Cout][R][S][C] -> the column layout above ([Cout][Kpad], segments of `seg`, zeros elsewhere).
 __global__ void __launch_bounds__(256) stem_pack_kernel(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                         int Cout, int R, int sc, int seg, int Kpad) {
+  pdl_enter();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= Cout * Kpad) return;
   const int co = i / Kpad, k = i - co * Kpad, r = k / seg, j = k - r * seg;
@@ -332,6 +379,7 @@ __global__ void __launch_bounds__(256) stem_pack_kernel(const __nv_bfloat16* __r
 // The way back for the filter gradient: fp32 columns -> bf16 filters (dw) or added to an fp32 accumulator (acc).
 __global__ void __launch_bounds__(256) stem_unpack_kernel(const float* __restrict__ col, __nv_bfloat16* dw, float* acc, int Cout,
                                                           int R, int sc, int seg, int Kpad) {
+  pdl_enter();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i >= Cout * R * sc) return;
   const int co = i / (R * sc), k = i - co * R * sc, r = k / sc, j = k - r * sc;
@@ -342,14 +390,15 @@ __global__ void __launch_bounds__(256) stem_unpack_kernel(const float* __restric
 
 // Gradient of a dense layer's fp32 output: bf16 copy with the row padded to np columns (zeros), and its column sums in the
 // same pass (dy is read once).  A thread keeps four columns and walks down the rows of its block.
-constexpr int kCastRows = 64;
+constexpr int kCastRows = 16;      // rows of a block: short enough that a small batch is not one serial chain of loads
 __global__ void __launch_bounds__(256) cast_colsum_kernel(const float* __restrict__ dy, int64_t ld, int M, int N, int np,
                                                           __nv_bfloat16* __restrict__ out, float* __restrict__ colsum, int vec) {
+  pdl_enter();
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= np) return;
   const int r0 = blockIdx.y * kCastRows, r1 = min(M, r0 + kCastRows);
   float s[4] = {0, 0, 0, 0};
-#pragma unroll 4
+#pragma unroll 8
   for (int r = r0; r < r1; ++r) {
     float v[4];
     if (vec && c + 4 <= N) {
@@ -384,53 +433,40 @@ extern "C" {
 // loss_sum (one float) must be zeroed by the caller.
 int esgd_softmax_ce(const void* logits, int is_bf16, const int64_t* labels, int batch, int classes, int ld,
                     float grad_scale, float* loss_sum, float* per_sample, void* dlogits, void* stream) {
-  cudaStream_t s = (cudaStream_t)stream;
   if (is_bf16)
-    softmax_ce_kernel<__nv_bfloat16><<<batch, 256, 0, s>>>((const __nv_bfloat16*)logits, labels, classes, ld,
-                                                           1.0f / batch, grad_scale, loss_sum, per_sample,
-                                                           (__nv_bfloat16*)dlogits);
-  else
-    softmax_ce_kernel<float><<<batch, 256, 0, s>>>((const float*)logits, labels, classes, ld, 1.0f / batch,
-                                                   grad_scale, loss_sum, per_sample, (float*)dlogits);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+    return esgd::launch(softmax_ce_kernel<__nv_bfloat16>, dim3(batch), 256, 0, stream, (const __nv_bfloat16*)logits, labels, classes, ld,
+                        1.0f / batch, grad_scale, loss_sum, per_sample, (__nv_bfloat16*)dlogits);
+  return esgd::launch(softmax_ce_kernel<float>, dim3(batch), 256, 0, stream, (const float*)logits, labels, classes, ld, 1.0f / batch,
+                      grad_scale, loss_sum, per_sample, (float*)dlogits);
 }
 
 // idx (optional, one byte per output element) records the arg-max for the backward pass.
 int esgd_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream) {
   if (C % 8) return -1;
   const int OH = (H + 1) / 2, OW = (W + 1) / 2;
-  maxpool_fwd_kernel<<<grid_for((int64_t)N * OH * OW * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (__nv_bfloat16*)y, (uint8_t*)idx, N, H, W, C, OH, OW);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(maxpool_fwd_kernel, dim3(N * OH), 256, 0, stream,
+                      (const __nv_bfloat16*)x, (__nv_bfloat16*)y, (uint8_t*)idx, N, H, W, C, OH, OW);
 }
 
 int esgd_maxpool3x3s2_bwd(const void* idx, const void* dy, void* dx, int N, int H, int W, int C, void* stream) {
   if (C % 8) return -1;
   const int OH = (H + 1) / 2, OW = (W + 1) / 2;
-  maxpool_bwd_kernel<<<grid_for((int64_t)N * H * W * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const uint8_t*)idx, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, N, H, W, C, OH, OW);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(maxpool_bwd_kernel, dim3(N * ((H + 1) / 2)), 256, 0, stream, (const uint8_t*)idx,
+                      (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, N, H, W, C, OH, OW);
 }
 
 // y[n, oh, ow, :] = x[n, 2*oh, 2*ow, :]   (OH = ceil(H/2), OW = ceil(W/2))
 int esgd_subsample2_fwd(const void* x, void* y, int N, int H, int W, int C, void* stream) {
   if (C % 8) return -1;
   const int OH = (H + 1) / 2, OW = (W + 1) / 2;
-  subsample2_fwd_kernel<<<grid_for((int64_t)N * OH * OW * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (__nv_bfloat16*)y, N, H, W, C, OH, OW);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(subsample2_fwd_kernel, dim3(grid_for((int64_t)N * OH * OW * (C / 8))), 256, 0, stream,
+                      (const __nv_bfloat16*)x, (__nv_bfloat16*)y, N, H, W, C, OH, OW);
 }
 int esgd_subsample2_bwd(const void* dy, void* dx, int N, int H, int W, int C, void* stream) {
   if (C % 8) return -1;
   const int OH = (H + 1) / 2, OW = (W + 1) / 2;
-  subsample2_bwd_kernel<<<grid_for((int64_t)N * H * W * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, N, H, W, C, OH, OW);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(subsample2_bwd_kernel, dim3(grid_for((int64_t)N * H * W * (C / 8))), 256, 0, stream,
+                      (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, N, H, W, C, OH, OW);
 }
 
 // col: [N*Ho*Wo, Kpad] bf16; seg = roundup8(S*C) <= 32; Kpad a multiple of seg with Kpad >= R*seg.
@@ -445,29 +481,21 @@ int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, in
   // the over-read of the last window, and the rows must fit in the default shared-memory budget
   if (rowbytes % 16 == 0 && ((uintptr_t)x & 15) == 0 && pad * C * 2 <= kImLeftGuard &&
       ((Wo - 1) * stride - pad) * C * 2 + seg * 2 + 8 <= rowbytes + kImRightGuard && smem <= 48 * 1024) {
-    im2col_rows_kernel<<<N * Ho, 256, smem, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)x, (__nv_bfloat16*)col, N, H, W, C, R, S, stride, pad, Ho, Wo, seg, Kpad);
-    esgd::count_launch();
-    return (int)cudaGetLastError();
+    return esgd::launch(im2col_rows_kernel, dim3(N * Ho), 256, smem, stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)col, N,
+                        H, W, C, R, S, stride, pad, Ho, Wo, seg, Kpad);
   }
-  im2col_small_c_kernel<32><<<grid_for((int64_t)N * Ho * Wo * (Kpad / seg)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (__nv_bfloat16*)col, N, H, W, C, R, S, stride, pad, Ho, Wo, seg, Kpad);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(im2col_small_c_kernel<32>, dim3(grid_for((int64_t)N * Ho * Wo * (Kpad / seg))), 256, 0, stream,
+                      (const __nv_bfloat16*)x, (__nv_bfloat16*)col, N, H, W, C, R, S, stride, pad, Ho, Wo, seg, Kpad);
 }
 
 // seg / Kpad as in esgd_im2col_small_c; w [Cout][R][S*C], sc = S*C.
 int esgd_stem_pack(const void* w, void* out, int Cout, int R, int sc, int seg, int Kpad, void* stream) {
-  stem_pack_kernel<<<(Cout * Kpad + 255) / 256, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)w, (__nv_bfloat16*)out,
-                                                                               Cout, R, sc, seg, Kpad);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(stem_pack_kernel, dim3((Cout * Kpad + 255) / 256), 256, 0, stream, (const __nv_bfloat16*)w,
+                      (__nv_bfloat16*)out, Cout, R, sc, seg, Kpad);
 }
 int esgd_stem_unpack(const float* col, void* dw, float* acc, int Cout, int R, int sc, int seg, int Kpad, void* stream) {
-  stem_unpack_kernel<<<(Cout * R * sc + 255) / 256, 256, 0, (cudaStream_t)stream>>>(col, (__nv_bfloat16*)dw, acc, Cout, R, sc,
-                                                                                   seg, Kpad);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(stem_unpack_kernel, dim3((Cout * R * sc + 255) / 256), 256, 0, stream, col, (__nv_bfloat16*)dw, acc,
+                      Cout, R, sc, seg, Kpad);
 }
 
 // out [M][np] bf16 (np a multiple of 8, zeros from column N on) = dy [M][N] fp32 with row stride ld; colsum (optional, zeroed
@@ -476,25 +504,21 @@ int esgd_cast_colsum(const float* dy, int64_t ld, int M, int N, int np, void* ou
   if (np % 8 || np < N) return -1;
   const int vec = ld % 4 == 0 && ((uintptr_t)dy & 15) == 0;
   dim3 grid((np / 4 + 255) / 256, (M + kCastRows - 1) / kCastRows);
-  cast_colsum_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(dy, ld, M, N, np, (__nv_bfloat16*)out, colsum, vec);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(cast_colsum_kernel, grid, 256, 0, stream, dy, ld, M, N, np, (__nv_bfloat16*)out, colsum, vec);
 }
 
 int esgd_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream) {
   if (C % 8) return -1;
-  avgpool_fwd_kernel<<<grid_for((int64_t)N * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)x, (__nv_bfloat16*)y, N, HW, C);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  int cg = 1;
+  while (cg < 16 && cg < C / 8) cg *= 2;
+  return esgd::launch(avgpool_fwd_kernel, dim3(N, (C / 8 + cg - 1) / cg), 256, 0, stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, N,
+                      HW, C, cg);
 }
 
 int esgd_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, void* stream) {
   if (C % 8) return -1;
-  avgpool_bwd_kernel<<<grid_for((int64_t)N * HW * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, N, HW, C);
-  esgd::count_launch();
-  return (int)cudaGetLastError();
+  return esgd::launch(avgpool_bwd_kernel, dim3(grid_for((int64_t)N * HW * (C / 8))), 256, 0, stream, (const __nv_bfloat16*)dy,
+                      (__nv_bfloat16*)dx, N, HW, C);
 }
 
 }  // extern "C"

@@ -15,9 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include "launch_count.cuh"
-
-extern "C" void esgd_gemm_set_chained(int on);
+#include "launch.cuh"
 
 namespace {
 
@@ -242,11 +240,6 @@ int cell_bwd(const void* gates, const float* c_prev, const float* c_cur, const v
   return (int)cudaGetLastError();
 }
 
-struct ChainScope {   // the GEMM launches of this thread are chain links while one of these is alive
-  ChainScope() { esgd_gemm_set_chained(1); }
-  ~ChainScope() { esgd_gemm_set_chained(0); }
-};
-
 // Split-K factor that brings a recurrent GEMM of `m` output rows to about one CTA per SM.
 int splits_for(int m, int k) {
   const int tiles = (m + 127) / 128;
@@ -267,7 +260,6 @@ extern "C" {
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn,
                    int b_mn, int out_mode, const float* scale, const float* bias, int relu, int splits, float* col_sum,
                    float* col_sqsum, const void* residual, int ldr, int* error_flag, void* stream);
-void esgd_gemm_set_chained(int on);
 
 // xproj [T*B, 4H] bf16 (input projection of every step), w_hh [4H, H] bf16, bias [4H] fp32;
 // out: c [T, B, H] fp32, y [T, B, H] bf16, gates [T, B, 4H] bf16; scratch hprojT [4H, B] fp32.
@@ -283,7 +275,6 @@ int esgd_lstm_seq_fwd(const void* xproj, const void* w_hh, const float* bias, fl
   const int splits = splits_for(4 * H, H);
   cudaError_t e = cudaMemsetAsync(hprojT, 0, (size_t)4 * bh * sizeof(float), (cudaStream_t)stream);
   if (e != cudaSuccess) return (int)e;
-  ChainScope chain;
   for (int t = 0; t < T; ++t) {
     if (t > 0) {   // hprojT[4H, B] += W_hh[4H, H] . h_{t-1}[B, H]^T
       int rc = esgd_gemm_bf16(w_hh, yp + (t - 1) * bh, hprojT, 4 * H, B, H, H, H, B, 0, 0, 2, nullptr, nullptr, 0, splits,
@@ -310,7 +301,6 @@ int esgd_lstm_seq_bwd(const void* gates, const float* c, const void* dy, const v
   if (e == cudaSuccess) e = cudaMemsetAsync(dh_recT, 0, bh * sizeof(float), (cudaStream_t)stream);
   if (e != cudaSuccess) return (int)e;
   const int splits = splits_for(H, 4 * H);   // H / 128 row tiles only: the split over K = 4H is what fills the GPU
-  ChainScope chain;
   for (int t = T - 1; t >= 0; --t) {
     int rc = cell_bwd(gp + (size_t)t * 4 * bh, t > 0 ? c + (t - 1) * bh : nullptr, c + t * bh, dyp + t * bh,
                       t < T - 1 ? dh_recT : nullptr, dc, dgp + (size_t)t * 4 * bh, B, H, B, 1, stream);

@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include "launch.cuh"
 #include "sm100_primitives.cuh"
 
 namespace umma {
@@ -268,6 +269,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  esgd::pdl_enter();       // the setup above overlaps the end of the kernel before; from here on its results are there
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer

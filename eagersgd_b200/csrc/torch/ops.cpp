@@ -41,16 +41,15 @@ int esgd_stem_unpack(const float* col, void* dw, float* acc, int Cout, int R, in
 int esgd_subsample2_fwd(const void* x, void* y, int N, int H, int W, int C, void* stream);
 int esgd_subsample2_bwd(const void* dy, void* dx, int N, int H, int W, int C, void* stream);
 int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, void* stream);
-int esgd_bn_fwd(const void* y, const void* residual, void* z, const float* sum, const float* sqsum, const float* gamma,
-                const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu,
-                float momentum, float eps, void* stream);
+int esgd_bn_fwd(const void* y, const void* residual, void* z, void* mask, const float* sum, const float* sqsum, const float* gamma,
+                const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu, float momentum,
+                float eps, void* stream);
 int esgd_bn_coefficients(const void* layers, int n, float eps, void* stream);
-int esgd_bn_bwd_reduce(const void* dz, const void* z, const void* y, const float* mean, const float* invstd,
-                       const float* fscale, const float* fshift, int64_t M, int C, int relu, float* dbeta, float* dgamma,
-                       void* stream);
-int esgd_bn_bwd_apply(const void* dz, const void* z, const void* y, const float* mean, const float* invstd, const float* gamma,
-                      const float* dbeta, const float* dgamma, const float* fscale, const float* fshift, void* dy, void* dres,
-                      int64_t M, int C, int relu, float* acc_dgamma, float* acc_dbeta, void* stream);
+int esgd_bn_bwd_reduce(const void* dz, const void* mask, const void* y, const float* aux, int64_t M, int C, int mode, float* dbeta,
+                       float* dgamma, void* stream);
+int esgd_bn_bwd_apply(const void* dz, const void* mask, const void* y, const float* aux, const float* gamma, const float* dbeta,
+                      const float* dgamma, void* dy, void* dres, int64_t M, int C, int mode, float* acc_dgamma, float* acc_dbeta,
+                      void* stream);
 int esgd_softmax_ce(const void* logits, int is_bf16, const int64_t* labels, int batch, int classes, int ld, float grad_scale,
                     float* loss_sum, float* per_sample, void* dlogits, void* stream);
 int esgd_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream);
@@ -649,11 +648,14 @@ struct BnActFn : public Function<BnActFn> {
     }
     Tensor aux = at::empty({4, c}, gamma.options());       // mean, invstd, scale, shift
     Tensor z = empty_nhwc(n, c, y.size(2), y.size(3), y);
-    ck(esgd_bn_fwd(y.data_ptr(), res.defined() ? res.data_ptr() : nullptr, z.data_ptr(), fptr(stats), fptr(stats) + c, fptr(gamma),
-                   fptr(beta), fptr(rm), fptr(rv), fptr(aux), m, c, relu, (float)momentum, kBnEps, st), "bn_fwd");
-    // ReLU mask of the backward pass: from the saved output when a residual was added, else recomputed from y
+    // ReLU mask of the backward pass: a bit per element where a residual was added, else recomputed from y
     const int64_t mode = !relu ? 0 : (res.defined() ? 1 : 2);
-    ctx->save_for_backward({y, mode == 1 ? z : Tensor(), gamma, aux});
+    Tensor mask;
+    if (mode == 1) mask = at::empty({m, c / 8}, y.options().dtype(at::kByte));
+    ck(esgd_bn_fwd(y.data_ptr(), res.defined() ? res.data_ptr() : nullptr, z.data_ptr(), mode == 1 ? mask.data_ptr() : nullptr,
+                   fptr(stats), fptr(stats) + c, fptr(gamma), fptr(beta), fptr(rm), fptr(rv), fptr(aux), m, c, relu, (float)momentum,
+                   kBnEps, st), "bn_fwd");
+    ctx->save_for_backward({y, mask, gamma, aux});
     ctx->saved_data["mode"] = mode;
     ctx->saved_data["res"] = res.defined();
     save_sink(ctx, "g", gs);
@@ -662,7 +664,7 @@ struct BnActFn : public Function<BnActFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &y = saved[0], &z = saved[1], &gamma = saved[2], &aux = saved[3];
+    const Tensor &y = saved[0], &mask = saved[1], &gamma = saved[2], &aux = saved[3];
     c10::cuda::CUDAGuard guard(y.device());
     const int64_t mode = ctx->saved_data["mode"].toInt(), c = y.size(1), m = y.numel() / c;
     const bool has_res = ctx->saved_data["res"].toBool();
@@ -671,13 +673,12 @@ struct BnActFn : public Function<BnActFn> {
     void* st = stream_of(y);
     // dbeta, dgamma; handed to autograd unless both go to sinks, so then not from the step's scratch
     Tensor red = gs && bs ? zeros_f32({2, c}, y.device()) : at::zeros({2, c}, aux.options());
-    float *a = fptr(aux), *rd = fptr(red);
-    const void* zp = z.defined() ? z.data_ptr() : nullptr;
-    ck(esgd_bn_bwd_reduce(dz.data_ptr(), zp, y.data_ptr(), a, a + c, a + 2 * c, a + 3 * c, m, c, (int)mode, rd, rd + c, st),
-       "bn_bwd_reduce");
+    float* rd = fptr(red);
+    const void* mp = mask.defined() ? mask.data_ptr() : nullptr;
+    ck(esgd_bn_bwd_reduce(dz.data_ptr(), mp, y.data_ptr(), fptr(aux), m, c, (int)mode, rd, rd + c, st), "bn_bwd_reduce");
     Tensor dy = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y), dres;
     if (has_res) dres = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y);
-    ck(esgd_bn_bwd_apply(dz.data_ptr(), zp, y.data_ptr(), a, a + c, fptr(gamma), rd, rd + c, a + 2 * c, a + 3 * c, dy.data_ptr(),
+    ck(esgd_bn_bwd_apply(dz.data_ptr(), mp, y.data_ptr(), fptr(aux), fptr(gamma), rd, rd + c, dy.data_ptr(),
                          has_res ? dres.data_ptr() : nullptr, m, c, (int)mode, gs ? gs->acc : nullptr, bs ? bs->acc : nullptr, st),
        "bn_bwd_apply");
     Tensor dgamma, dbeta;
