@@ -3,8 +3,8 @@
 // A time step is a product with the recurrent weights (32 MB of bf16 at 2048 units) and a few hundred bytes of state per
 // SM; as two launches per step (split-K GEMM + cell kernel) it cost 13.8 us forward and 15.3 us backward at batch 16, bound
 // by the two kernel boundaries and by re-reading the weights from L2.  Here every CTA keeps its share of the weights on
-// chip for the whole sequence and a step is: wait until the previous step's state is complete, fetch it (32 KB), 64 MMAs,
-// exchange partial sums inside the cluster, apply the cell to 16 units, publish.
+// chip for the whole sequence and a step is: fetch the previous step's state as it appears (32 KB), 64 MMAs, exchange
+// partial sums inside the cluster, apply the cell to 16 units, publish.
 //
 //   weights   the A operand of tcgen05.mma, 64 columns of K at a time: up to 15 such blocks (240 KB) in tensor memory, the
 //             rest in shared memory, as the room left by the state and the partial sums allows
@@ -12,12 +12,14 @@
 //   backward  128 rows = 128 units of dh (weights transposed), K = 4H split over clusters of up to 8 CTAs: the largest
 //             cluster size whose whole grid is resident (of 16 clusters, a B200's GPCs hold 15 of size 8 or 7 but all of size 6)
 //   cluster   each finalising CTA owns 16 (forward) or 32 (backward) units x batch: partial sums go to its shared memory
-//             (DSMEM), double buffered by step parity; a CTA can be at most one step ahead of a cluster mate (it needs a
+//             (st.async: the bytes carry their own arrival), double buffered by step parity; a CTA can be at most one step ahead of a cluster mate (it needs a
 //             state that transitively needs the mate's previous one), so two buffers are enough
-//   grid      counters of finished CTAs, on lines of their own; a CTA waits for those that its K range needs (forward: the
-//             half of the units it multiplies with).  Four counters share the arrivals: 64 on one word queue up, and a
-//             flag per CTA has 128 SMs polling the lines 64 CTAs write to (5.9 and 6.3 us a step).  Launched cooperatively
-//             (all CTAs resident); every wait is bounded and ends in the error flag.
+//   grid      the state is published by writing it to y (forward) or dG (backward), which are filled with a bit pattern that
+//             no result has (0xffff per bf16; conversions round every NaN to 0x7fff) before the launch: eight warps read the
+//             words they need until none of them is the pattern, and put them where the tensor core reads them.  The data is
+//             its own flag, so no fence, counter or second trip to L2 stands between a store and its use.  With counters, a
+//             release and a TMA load the way from a stored state to the first MMA took 3 of the step's 5.2 us.
+//             Launched cooperatively (all CTAs resident); every wait is bounded and ends in the error flag.
 //
 // Cell state (forward) and cell gradient (backward) of an element stay in the register of the thread that owns it.
 // Gate order i, f, g, o as in torch.nn.LSTM.
@@ -34,18 +36,19 @@ namespace {
 
 constexpr int kRows = 128;          // weight rows of a CTA (MMA M)
 constexpr int kEpiThreads = 256;
-constexpr int kThreads = kEpiThreads + 32;
+constexpr int kFetchWarps = 8;
+constexpr int kThreads = kEpiThreads + 32 + kFetchWarps * 32;
 constexpr int kATile = kRows * 128; // one 64-column block of A
-constexpr int kGroups = 4;          // the state arrives in up to four pieces, so that the MMAs start before all of it is there
+constexpr int kPiece = 4;           // K blocks of a piece of the state: the MMAs of one run while the next is fetched
+constexpr int kMaxPieces = 8;
 constexpr int kTBlocks = 15;        // blocks of the weights that tensor memory holds, 32 columns each
 constexpr int kDCol = 480;          // first TMEM column of the accumulator (at most 32 columns)
 constexpr int kSmemLimit = 227 * 1024;
-constexpr int kCounters = 4;
-constexpr int kCounterWords = 2 * kCounters * 32;
+constexpr uint32_t kUnset = 0xffffffffu;      // two bf16 that have not been written yet
 constexpr uint64_t kWaitNs = 4000000000ull;   // bound on every wait
 
 struct SeqParams {
-  CUtensorMap tmW, tmS;             // recurrent weights; the state a step multiplies with (forward y, backward dG)
+  CUtensorMap tmW;                  // recurrent weights
   const __nv_bfloat16* w;           // [4H][H]
   int T, B, H, S;                   // S: cluster size, the split of K
   const __nv_bfloat16* xproj;       // forward: [T][B][4H]
@@ -56,7 +59,6 @@ struct SeqParams {
   const __nv_bfloat16* dy;          // backward: [T][B][H]
   __nv_bfloat16* dG;                // backward: [T][B][4H]
   float* db;                        // backward: [4H] bias gradient, added to (may be null)
-  uint32_t* counters;               // [2][kCounters] at a distance of 32 words, zeroed before the launch
   int* error_flag;
 };
 
@@ -71,11 +73,10 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void arrive_cluster(uint32_t bar_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");
+// 16 bytes into a mate's shared memory, counted by its barrier.
+__device__ __forceinline__ void st_async_x4(uint32_t addr, const uint32_t* v, uint32_t bar_addr) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(v[0]),
+               "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar_addr) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -108,22 +109,22 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
     if (p.over(it, abort_flag)) return false;
   return true;
 }
-// One warp waits until kCounters counters have reached `target`.
-__device__ __forceinline__ bool wait_counters(const uint32_t* c, uint32_t target, int lane, volatile int* abort_flag) {
-  Patience p;
-  for (uint32_t it = 0;; ++it) {
-    uint32_t v = target;
-    if (lane < kCounters) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c + 32 * lane) : "memory");
-    if (__all_sync(0xffffffffu, v >= target)) break;
-    if (__any_sync(0xffffffffu, p.over(it, abort_flag))) return false;
-  }
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
-  return true;
+__device__ __forceinline__ uint4 ld_state(const void* p) {
+  uint4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
 }
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(m), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2) : "memory");
+__device__ __forceinline__ bool unset(const uint4& v) { return v.x == kUnset || v.y == kUnset || v.z == kUnset || v.w == kUnset; }
+__device__ __forceinline__ uint32_t bf16_bits(float v) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(v)); }
+// Four lanes' values, in lane order, in each of the four.
+__device__ __forceinline__ uint2 gather_quad(uint32_t v, int lane) {
+  const uint32_t other = __shfl_xor_sync(0xffffffffu, v, 1);
+  const uint32_t pair = lane & 1 ? other | (v << 16) : v | (other << 16);
+  const uint32_t far = __shfl_xor_sync(0xffffffffu, pair, 2);
+  return lane & 2 ? make_uint2(far, pair) : make_uint2(pair, far);
+}
+__device__ __forceinline__ void publish(void* p, uint2 v) {
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]: A holds two consecutive K elements of a row per 32-bit cell, K-major.
 __device__ __forceinline__ void umma_bf16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -147,13 +148,15 @@ struct Layout {
   static constexpr int kUnits = kBwd ? 32 : 16;                       // units a finalising CTA owns
   static constexpr int kFinal = kBwd ? 4 : 2;                         // finalising CTAs of a cluster
   static constexpr int kPer = kUnits * N / kEpiThreads;               // elements of a finalising thread
-  int kblocks, per, tblocks, sblocks, part;                           // per: K blocks of a CTA (the last may have fewer)
+  static constexpr int kPitch = N + 4;                                // floats of a unit's batch in the partial sums
+  int kblocks, per, tblocks, sblocks, part;                           // per: K blocks of a CTA (the last may have fewer);
+                                                                      // part: floats for one step's partial sums
   __host__ __device__ Layout(int H, int S) {
     kblocks = (kBwd ? 4 * H : H) / 64;
     per = (kblocks + S - 1) / S;
     tblocks = per < kTBlocks ? per : kTBlocks;
     sblocks = per - tblocks;
-    part = S * (kBwd ? 1 : 4) * N * kUnits;                           // floats a finalising CTA receives per step
+    part = S * (kBwd ? 1 : 4) * kUnits * kPitch;
   }
   int smem() const { return 1024 + sblocks * kATile + per * (N * 128) + 2 * part * 4 + 256; }
 };
@@ -173,8 +176,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
   uint8_t* sA = smem;
   uint8_t* sB = sA + lay.sblocks * kATile;
   float* sP = reinterpret_cast<float*>(sB + lay.per * (N * 128));
-  uint64_t* full = reinterpret_cast<uint64_t*>(sP + 2 * lay.part);    // [kGroups] pieces of the state have landed
-  uint64_t* wfull = full + kGroups;                                   // the weights have landed
+  uint64_t* full = reinterpret_cast<uint64_t*>(sP + 2 * lay.part);    // [kMaxPieces] pieces of the state are in place
+  uint64_t* wfull = full + kMaxPieces;                                 // the weights have landed
   uint64_t* dfull = wfull + 1;                                        // the step's product is in tensor memory
   uint64_t* dfree = dfull + 1;                                        // ... and has been read out of it
   uint64_t* pfull = dfree + 1;                                        // [2] partial sums of all cluster mates are here
@@ -184,26 +187,27 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const bool final_cta = rank < L::kFinal;
   const int u0 = (kBwd ? group * 128 : group * 32) + rank * UNITS;    // first unit this CTA finalises
-  const uint32_t* wait_on = p.counters + (kBwd ? 0 : rank * kCounters * 32);
-  uint32_t* signal_to = p.counters + (kBwd || u0 < H / 2 ? 0 : kCounters * 32) + (u0 / UNITS) % kCounters * 32;
-  const uint32_t per_step = (uint32_t)(H / 32 / kCounters);           // arrivals on a counter per step
+  const int npieces = (kblocks + kPiece - 1) / kPiece;
+  const int p0 = group % npieces;        // CTAs start at different pieces: 128 SMs asking for one line queue up at its L2 slice
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kGroups; ++i) mbar_init(&full[i], 1);
+    for (int i = 0; i < kMaxPieces; ++i) mbar_init(&full[i], kFetchWarps);
     mbar_init(wfull, 1);
     mbar_init(dfull, 1);
     mbar_init(dfree, kEpiThreads / 32);
-    mbar_init(&pfull[0], kBwd ? 2 * S : 16);
-    mbar_init(&pfull[1], kBwd ? 2 * S : 16);
+    mbar_init(&pfull[0], 1);
+    mbar_init(&pfull[1], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&p.tmW);
-    tma_prefetch_desc(&p.tmS);
   }
   if (warp == 8) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  for (int i = threadIdx.x; i < lay.per * N * 8; i += kThreads)       // batch rows that do not exist stay zero
+    reinterpret_cast<uint4*>(sB)[i] = make_uint4(0, 0, 0, 0);
+  fence_proxy_async();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -222,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
         }
       }
     }
-  } else {
+  } else if (warp < 8) {
     const int q = warp & 3, row = q * 32 + lane;
     for (int k0 = (warp >> 2) * 16; k0 < tblocks * 64; k0 += 32) {            // 16 K elements = 8 columns at a time
       uint32_t r[8];
@@ -247,60 +251,114 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
   tc_fence_after();
 
   if (warp == 8) {
-    // ------------------------------------------------------------ control: fetch the state, issue the products
+    // ------------------------------------------------------------ issue the products
     const uint32_t idesc_s = umma_idesc_bf16(kRows, N, kBwd ? 1 : 0, 0), idesc_t = umma_idesc_bf16(kRows, N, 0, 0);
     const uint64_t a_desc0 = kBwd ? umma_smem_desc(smem_u32(sA), 8192, 1024) : umma_smem_desc(smem_u32(sA), 16, 1024);
     const uint64_t b_desc0 = umma_smem_desc(smem_u32(sB), 16, 1024);
     constexpr uint64_t kStepA = kBwd ? (2048 >> 4) : (32 >> 4), kStepB = 32 >> 4;
-    const int per_group = (kblocks + kGroups - 1) / kGroups;
-    const bool leader = elect_one();
-    bool ok = __all_sync(0xffffffffu, wait_bar(wfull, 0u, abort_flag));
-    for (int s = 1; ok && s < T; ++s) {                      // step 0 has no recurrent product
-      const int t_state = kBwd ? T - s : s - 1;
-      const uint32_t ph = (uint32_t)(s - 1) & 1u;
-      ok = wait_counters(wait_on, per_step * (uint32_t)s, lane, abort_flag);
-      if (ok && s > 1)       // the previous product has read its state, and has been read itself
-        ok = __all_sync(0xffffffffu, wait_bar(dfull, ph ^ 1u, abort_flag) && wait_bar(dfree, ph ^ 1u, abort_flag));
-      if (!ok) break;
-      if (leader) {
-        asm volatile("fence.proxy.async;" ::: "memory");     // other SMs' ordinary stores, about to be read by TMA
-        for (int g = 0; g < kGroups; ++g) {
-          const int k0 = g * per_group, k1 = min(kblocks, k0 + per_group);
-          if (k0 >= k1) break;
-          mbar_expect_tx(&full[g], (uint32_t)((k1 - k0) * N * 128));
-          for (int kb = k0; kb < k1; ++kb) tma_load_3d(sB + kb * (N * 128), &p.tmS, &full[g], kbase + kb * 64, 0, t_state);
-        }
-        tc_fence_after();
+    if (elect_one()) {
+      bool ok = wait_bar(wfull, 0u, abort_flag);
+      for (int s = 1; ok && s < T; ++s) {                    // step 0 has no recurrent product
+        const uint32_t ph = (uint32_t)(s - 1) & 1u;
+        if (s > 1) ok = wait_bar(dfree, ph ^ 1u, abort_flag);               // the previous product has been read
         uint32_t acc = 0;
-        for (int g = 0; ok && g < kGroups; ++g) {
-          const int k0 = g * per_group, k1 = min(kblocks, k0 + per_group);
-          if (k0 >= k1) break;
-          ok = wait_bar(&full[g], ph, abort_flag);
+        for (int j = 0; ok && j < npieces; ++j) {
+          const int piece = p0 + j < npieces ? p0 + j : p0 + j - npieces;
+          ok = wait_bar(&full[piece], ph, abort_flag);
           tc_fence_after();
-          for (int kb = k0; ok && kb < k1; ++kb) {
+          const int k1 = min(kblocks, (piece + 1) * kPiece);
+          for (int kb = piece * kPiece; ok && kb < k1; ++kb) {
             const uint64_t b_desc = b_desc0 + (uint64_t)(kb * (N * 128 >> 4));
             if (kb >= tblocks) {
               const uint64_t a_desc = a_desc0 + (uint64_t)((kb - tblocks) * (kATile >> 4));
 #pragma unroll
-              for (int j = 0; j < 4; ++j) { umma_bf16(tmem + kDCol, a_desc + j * kStepA, b_desc + j * kStepB, idesc_s, acc); acc = 1; }
+              for (int i = 0; i < 4; ++i) { umma_bf16(tmem + kDCol, a_desc + i * kStepA, b_desc + i * kStepB, idesc_s, acc); acc = 1; }
             } else {
               const uint32_t a_t = tmem + (uint32_t)(kb * 32);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) { umma_bf16_ta(tmem + kDCol, a_t + j * 8, b_desc + j * kStepB, idesc_t, acc); acc = 1; }
+              for (int i = 0; i < 4; ++i) { umma_bf16_ta(tmem + kDCol, a_t + i * 8, b_desc + i * kStepB, idesc_t, acc); acc = 1; }
             }
           }
         }
         if (ok) umma_commit(dfull);
       }
-      ok = __all_sync(0xffffffffu, ok);
     }
     __syncwarp();
+  } else if (warp > 8) {
+    // ------------------------------------------------------------ fetch the state
+    // A load of a warp is four batch rows of one K block (64 values).  Up to eight are in flight; the first piece is polled
+    // alone, so that waiting SMs leave the L2 to those that still work.
+    constexpr int kLoads = N / 8;                            // loads of a warp per piece, at most
+    constexpr int kWindow = 8 / kLoads;                      // pieces in flight
+    const int fw = warp - 9, width = kBwd ? 4 * H : H, quads = B / 4;
+    const __nv_bfloat16* state = (kBwd ? p.dG : p.y) + kbase + (size_t)(lane >> 3) * width + (lane & 7) * 8;
+    bool ok = true;
+    for (int s = 1; ok && s < T; ++s) {
+      const uint32_t ph = (uint32_t)(s - 1) & 1u;
+      const __nv_bfloat16* from = state + (size_t)(kBwd ? T - s : s - 1) * B * width;
+      for (int j0 = 0; ok && j0 < npieces; j0 += kWindow) {
+        uint4 v[kWindow][kLoads];
+        auto chunk = [&](int w, int l, int& kb, int& b) {    // the l-th load of this warp in piece j0 + w; false: none
+          const int j = j0 + w, piece = p0 + j < npieces ? p0 + j : p0 + j - npieces, c = fw + l * kFetchWarps;
+          kb = piece * kPiece + c / quads;
+          b = c % quads * 4;
+          return j < npieces && c < kPiece * quads && kb < kblocks;
+        };
+        auto load_unset = [&](int w, bool all) {
+#pragma unroll
+          for (int l = 0; l < kLoads; ++l) {
+            int kb, b;
+            if (chunk(w, l, kb, b) && (all || unset(v[w][l]))) v[w][l] = ld_state(from + (size_t)b * width + kb * 64);
+          }
+        };
+        auto complete = [&](int w) {
+          bool missing = false;
+#pragma unroll
+          for (int l = 0; l < kLoads; ++l) {
+            int kb, b;
+            missing |= chunk(w, l, kb, b) && unset(v[w][l]);
+          }
+          return !__any_sync(0xffffffffu, missing);
+        };
+        Patience patience;
+        load_unset(0, true);
+        if (j0 == 0)
+          for (uint32_t it = 0; ok && !complete(0); ++it) {
+            load_unset(0, false);
+            ok = !__any_sync(0xffffffffu, patience.over(it, abort_flag));
+          }
+#pragma unroll
+        for (int w = 1; w < kWindow; ++w) load_unset(w, true);
+        if (s > 1 && j0 == 0 && ok) ok = __all_sync(0xffffffffu, wait_bar(dfull, ph ^ 1u, abort_flag));   // the last product has been taken
+#pragma unroll
+        for (int w = 0; w < kWindow; ++w) {
+          const int j = j0 + w;
+          if (!ok || j >= npieces) break;
+          for (uint32_t it = 0; ok && !complete(w); ++it) {
+#pragma unroll
+            for (int x = w; x < kWindow; ++x) load_unset(x, false);
+            ok = !__any_sync(0xffffffffu, patience.over(it, abort_flag));
+          }
+#pragma unroll
+          for (int l = 0; l < kLoads; ++l) {
+            int kb, b;
+            if (!chunk(w, l, kb, b)) continue;
+            b += lane >> 3;
+            *reinterpret_cast<uint4*>(sB + kb * (N * 128) + b * 128 + (((lane & 7) ^ (b & 7)) << 4)) = v[w][l];
+          }
+          fence_proxy_async();                               // the tensor core reads what was written here
+          __syncwarp();
+          if (ok && lane == 0) mbar_arrive(&full[p0 + j < npieces ? p0 + j : p0 + j - npieces]);
+        }
+      }
+    }
   } else {
     // ------------------------------------------------------------ cells
     const int q = warp & 3, half = warp >> 2;                // TMEM lane quarter, half of the batch columns
     const int dest = kBwd ? q : lane >> 4;                   // the mate that finalises this lane's unit
     const uint32_t p_remote = map_to_rank(smem_u32(sP), (uint32_t)dest);
     const uint32_t bar_remote = map_to_rank(smem_u32(&pfull[0]), (uint32_t)dest);
+    const uint32_t part_bytes = (uint32_t)(S * (kBwd ? 1 : 4) * UNITS * N * 4);
     float state[PER];                                        // c (forward) / dc (backward) of this thread's elements
 #pragma unroll
     for (int e = 0; e < PER; ++e) state[e] = 0.0f;
@@ -309,7 +367,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
     for (int s = 0; s < T; ++s) {
       const int t = kBwd ? T - 1 - s : s;
       // what does not depend on the recurrence is on its way before the wait
-      float in[PER][4], cc[PER], cp[PER], dyv[PER];
+      if (s > 0 && final_cta && threadIdx.x == 0) mbar_expect_tx(&pfull[(s - 1) & 1], part_bytes);
+      float in[PER][4], cc[PER], dyv[PER], fgate[PER];
 #pragma unroll
       for (int e = 0; e < PER; ++e) {
         const int i = threadIdx.x + e * kEpiThreads, b = i / UNITS, u = u0 + i % UNITS;
@@ -319,9 +378,16 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
 #pragma unroll
           for (int k = 0; k < 4; ++k) in[e][k] = __bfloat162float(g4[(size_t)k * H]);
           if (kBwd) {
-            cc[e] = p.c[row * H + u];
-            cp[e] = t > 0 ? p.c[(row - B) * H + u] : 0.0f;
+            // d(gate) = dc * in[gate] (output gate: dh * in), dc = state + dh * cc
+            const float ig = in[e][0], fg = in[e][1], gg = in[e][2], og = in[e][3];
+            const float tc = tanhf(p.c[row * H + u]), before = t > 0 ? p.c[(row - B) * H + u] : 0.0f;
             dyv[e] = __bfloat162float(p.dy[row * H + u]);
+            cc[e] = og * (1.0f - tc * tc);
+            in[e][0] = gg * ig * (1.0f - ig);
+            in[e][1] = before * fg * (1.0f - fg);
+            in[e][2] = ig * (1.0f - gg * gg);
+            in[e][3] = tc * og * (1.0f - og);
+            fgate[e] = fg;
           } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) in[e][k] += __ldg(p.bias + k * H + u);
@@ -340,13 +406,11 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(dfree);
-        // partial sums to the finaliser: [parity][source rank][gate][batch][unit]
-        const uint32_t dst = p_remote + 4u * (uint32_t)((int)ph * lay.part + (kBwd ? rank : rank * 4 + q) * (N * UNITS) +
-                                                        half * (N / 2) * UNITS + lane % UNITS);
+        // partial sums to the finaliser: [parity][source rank][gate][unit][batch]
+        const uint32_t dst = p_remote + 4u * (uint32_t)((int)ph * lay.part + ((kBwd ? rank : rank * 4 + q) * UNITS + lane % UNITS) * L::kPitch +
+                                                        half * (N / 2));
 #pragma unroll
-        for (int j = 0; j < N / 2; ++j) st_cluster_f32(dst + 4u * (uint32_t)(j * UNITS), __uint_as_float(r[j]));
-        __syncwarp();
-        if (lane % UNITS == 0) arrive_cluster(bar_remote + 8u * ph);
+        for (int j = 0; j < N / 2; j += 4) st_async_x4(dst + 4u * j, r + j, bar_remote + 8u * ph);
         if (final_cta) ok = __all_sync(0xffffffffu, wait_bar(&pfull[ph], (uint32_t)((s - 1) >> 1) & 1u, abort_flag));
       }
       const float* part = sP + ((s - 1) & 1) * lay.part;
@@ -355,43 +419,38 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
         const int i = threadIdx.x + e * kEpiThreads, b = i / UNITS, u = u0 + i % UNITS;
         if (b < B && final_cta) {
           const size_t row = (size_t)t * B + b;
+          const float* mine = part + i % UNITS * L::kPitch + b;
           if (!kBwd) {
             float pre[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               pre[k] = in[e][k];
-              if (s > 0) pre[k] += part[k * (N * UNITS) + i] + part[(4 + k) * (N * UNITS) + i];
+              if (s > 0) pre[k] += mine[k * UNITS * L::kPitch] + mine[(4 + k) * UNITS * L::kPitch];
             }
             const float ig = sigmoidf_(pre[0]), fg = sigmoidf_(pre[1]), gg = tanhf(pre[2]), og = sigmoidf_(pre[3]);
             const float c = fg * state[e] + ig * gg;
             state[e] = c;
-            p.y[row * H + u] = __float2bfloat16(og * tanhf(c));
+            const uint2 h4 = gather_quad(bf16_bits(og * tanhf(c)), lane);
+            if ((lane & 3) == 0) publish(p.y + row * H + u, h4);
             in[e][0] = ig; in[e][1] = fg; in[e][2] = gg; in[e][3] = og;
           } else {
-            const float ig = in[e][0], fg = in[e][1], gg = in[e][2], og = in[e][3];
             float dh = dyv[e];
             if (s > 0) {
-              for (int k = 0; k < S; ++k) dh += part[k * (N * UNITS) + i];
+              for (int k = 0; k < S; ++k) dh += mine[k * UNITS * L::kPitch];
             }
-            const float tc = tanhf(cc[e]);
-            const float dct = state[e] + dh * og * (1.0f - tc * tc);
-            state[e] = dct * fg;
-            __nv_bfloat16* dp = p.dG + row * 4 * H + u;
-            const float d[4] = {dct * gg * ig * (1.0f - ig), dct * cp[e] * fg * (1.0f - fg), dct * ig * (1.0f - gg * gg),
-                                dh * tc * og * (1.0f - og)};
+            const float dct = state[e] + dh * cc[e];
+            state[e] = dct * fgate[e];
+            const float d[4] = {dct * in[e][0], dct * in[e][1], dct * in[e][2], dh * in[e][3]};
+            uint2 d4 = make_uint2(0, 0);                     // lane k of four publishes gate k
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              dp[(size_t)k * H] = __float2bfloat16(d[k]);
+              const uint2 g = gather_quad(bf16_bits(d[k]), lane);
+              if ((lane & 3) == k) d4 = g;
               db[k] += d[k];
             }
+            publish(p.dG + row * 4 * H + (lane & 3) * H + (u & ~3), d4);
           }
         }
-      }
-      if (s + 1 < T && final_cta) {       // publish: every thread's stores, then one arrival of the CTA
-        asm volatile("fence.proxy.async.global;" ::: "memory");
-        named_barrier_sync(1, kEpiThreads);
-        if (threadIdx.x == 0)
-          asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(signal_to), "r"(1u) : "memory");
       }
       if (!kBwd) {                        // what only the backward pass reads leaves after the hand-over
 #pragma unroll
@@ -442,7 +501,8 @@ int cluster_size(int H) {
     cudaError_t e = cudaFuncSetAttribute(lstm_sequence_kernel<kBwd, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     for (int S = kBwd ? 8 : 2; e == cudaSuccess && found == 0 && S >= Layout<kBwd, N>::kFinal; --S) {
       const Layout<kBwd, N> lay(H, S);
-      if (lay.smem() > kSmemLimit || lay.per * (S - 1) >= lay.kblocks) continue;     // too much per CTA; an empty CTA
+      if (lay.smem() > kSmemLimit || lay.per * (S - 1) >= lay.kblocks ||      // too much per CTA; an empty CTA
+          lay.per > kPiece * kMaxPieces) continue;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(grid_of(kBwd, H, S));
       cfg.blockDim = dim3(kThreads);
@@ -475,14 +535,7 @@ int launch(SeqParams& p, cudaStream_t stream) {
     int r = esgd::make_tensormap_bf16(&p.tmW, p.w, 2, dims, strides, box, nullptr);
     if (r != 0) return 1000 + r;
   }
-  {
-    const uint64_t width = kBwd ? 4 * (uint64_t)H : (uint64_t)H;
-    uint64_t dims[3] = {width, (uint64_t)p.B, (uint64_t)p.T}, strides[2] = {width * 2, width * 2 * p.B};
-    uint32_t box[3] = {64, (uint32_t)N, 1};
-    int r = esgd::make_tensormap_bf16(&p.tmS, kBwd ? (const void*)p.dG : (const void*)p.y, 3, dims, strides, box, nullptr);
-    if (r != 0) return 2000 + r;
-  }
-  cudaError_t e = cudaMemsetAsync(p.counters, 0, kCounterWords * sizeof(uint32_t), stream);
+  cudaError_t e = cudaMemsetAsync(kBwd ? (void*)p.dG : (void*)p.y, 0xff, (size_t)p.T * p.B * H * (kBwd ? 8 : 2), stream);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid_of(kBwd, H, p.S));
@@ -505,9 +558,6 @@ int launch(SeqParams& p, cudaStream_t stream) {
 
 extern "C" {
 
-// Words of zeroable scratch (device, fp32-sized) a call needs.
-int esgd_lstm_persistent_scratch(void) { return kCounterWords; }
-
 // Whether the persistent kernels take this shape on the current device: units a multiple of 128 up to 2048 (the weights
 // must fit on the chip), a batch of up to 32 that is a multiple of 8, and every CTA resident.  1 yes, 0 no.
 int esgd_lstm_persistent_ok(int B, int H, int backward) {
@@ -517,25 +567,25 @@ int esgd_lstm_persistent_ok(int B, int H, int backward) {
 }
 
 // xproj [T*B, 4H] bf16, w_hh [4H, H] bf16, bias [4H] fp32; out: c [T, B, H] fp32, y [T, B, H] bf16, gates [T, B, 4H] bf16.
-int esgd_lstm_persistent_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates, void* scratch,
+int esgd_lstm_persistent_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates,
                              int T, int B, int H, int* error_flag, void* stream) {
   if (T <= 0 || !esgd_lstm_persistent_ok(B, H, 0)) return -1;
   SeqParams p = {};
   p.w = (const __nv_bfloat16*)w_hh; p.T = T; p.B = B; p.H = H;
   p.xproj = (const __nv_bfloat16*)xproj; p.bias = bias; p.c = c; p.y = (__nv_bfloat16*)y; p.gates = (__nv_bfloat16*)gates;
-  p.counters = (uint32_t*)scratch; p.error_flag = error_flag;
+  p.error_flag = error_flag;
   return B <= 16 ? launch<false, 16>(p, (cudaStream_t)stream) : launch<false, 32>(p, (cudaStream_t)stream);
 }
 
 // dG [T, B, 4H] bf16 (pre-activation gradients of every step) from dy [T, B, H] bf16 and the saved gates and cell states;
 // db [4H] fp32 (or null) += their sum over steps and batch.
-int esgd_lstm_persistent_bwd(const void* gates, const float* c, const void* dy, const void* w_hh, void* dG, float* db, void* scratch,
+int esgd_lstm_persistent_bwd(const void* gates, const float* c, const void* dy, const void* w_hh, void* dG, float* db,
                              int T, int B, int H, int* error_flag, void* stream) {
   if (T <= 0 || !esgd_lstm_persistent_ok(B, H, 1)) return -1;
   SeqParams p = {};
   p.w = (const __nv_bfloat16*)w_hh; p.T = T; p.B = B; p.H = H;
   p.gates = (__nv_bfloat16*)gates; p.c = const_cast<float*>(c); p.dy = (const __nv_bfloat16*)dy; p.dG = (__nv_bfloat16*)dG; p.db = db;
-  p.counters = (uint32_t*)scratch; p.error_flag = error_flag;
+  p.error_flag = error_flag;
   return B <= 16 ? launch<true, 16>(p, (cudaStream_t)stream) : launch<true, 32>(p, (cudaStream_t)stream);
 }
 

@@ -57,10 +57,9 @@ int esgd_maxpool3x3s2_bwd(const void* idx, const void* dy, void* dx, int N, int 
 int esgd_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream);
 int esgd_avgpool_bwd(const void* dy, void* dx, int N, int HW, int C, void* stream);
 int esgd_lstm_persistent_ok(int B, int H, int backward);
-int esgd_lstm_persistent_scratch(void);
-int esgd_lstm_persistent_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates, void* scratch,
+int esgd_lstm_persistent_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates,
                              int T, int B, int H, int* error_flag, void* stream);
-int esgd_lstm_persistent_bwd(const void* gates, const float* c, const void* dy, const void* w_hh, void* dG, float* db, void* scratch,
+int esgd_lstm_persistent_bwd(const void* gates, const float* c, const void* dy, const void* w_hh, void* dG, float* db,
                              int T, int B, int H, int* error_flag, void* stream);
 int esgd_lstm_seq_fwd(const void* xproj, const void* w_hh, const float* bias, float* c, void* y, void* gates, float* hprojT, int T,
                       int B, int H, int* error_flag, void* stream);
@@ -783,9 +782,8 @@ struct LstmFn : public Function<LstmFn> {
             nullptr, 0, x), "lstm input projection");
     Tensor y = at::empty({t, b, h}, x.options()), c = at::empty({t, b, h}, f32), gates = at::empty({t, b, 4 * h}, x.options());
     if (esgd_lstm_persistent_ok((int)b, (int)h, 0)) {
-      Tensor scratch = at::empty({esgd_lstm_persistent_scratch()}, f32);
       ck(esgd_lstm_persistent_fwd(xproj.data_ptr(), w_hh.data_ptr(), fptr(bias), fptr(c), y.data_ptr(), gates.data_ptr(),
-                                  scratch.data_ptr(), t, b, h, flag_ptr(x), st), "lstm forward recurrence");
+                                  t, b, h, flag_ptr(x), st), "lstm forward recurrence");
     } else {
       Tensor hproj = at::empty({4 * h, b}, f32);
       ck(esgd_lstm_seq_fwd(xproj.data_ptr(), w_hh.data_ptr(), fptr(bias), fptr(c), y.data_ptr(), gates.data_ptr(), fptr(hproj), t, b, h,
@@ -829,10 +827,9 @@ struct LstmFn : public Function<LstmFn> {
     Tensor dx, dw_ih, dw_hh, db;
     const bool need_b = s_b || ctx->needs_input_grad(3);
     if (esgd_lstm_persistent_ok((int)b, (int)h, 1)) {
-      Tensor scratch = at::empty({esgd_lstm_persistent_scratch()}, f32);
       if (need_b && !s_b) db = at::zeros({4 * h}, f32);
       ck(esgd_lstm_persistent_bwd(gates.data_ptr(), fptr(c), dy.data_ptr(), w_hh.data_ptr(), dG.data_ptr(),
-                                  !need_b ? nullptr : (s_b ? s_b->acc : fptr(db)), scratch.data_ptr(), t, b, h, flag_ptr(x), st),
+                                  !need_b ? nullptr : (s_b ? s_b->acc : fptr(db)), t, b, h, flag_ptr(x), st),
          "lstm backward recurrence");
     } else {
       Tensor dc = at::empty({b, h}, f32), dh = at::empty({h, b}, f32);
