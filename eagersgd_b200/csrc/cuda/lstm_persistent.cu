@@ -6,7 +6,7 @@
 // chip for the whole sequence and a step is: fetch the previous step's state as it appears (32 KB), 64 MMAs, exchange
 // partial sums inside the cluster, apply the cell to 16 units, publish.
 //
-//   weights   the A operand of tcgen05.mma, 64 columns of K at a time: up to 15 such blocks (240 KB) in tensor memory, the
+//   weights   the A operand of tcgen05.mma, 64 columns of K at a time: up to 14 such blocks (224 KB) in tensor memory, the
 //             rest in shared memory, as the room left by the state and the partial sums allows
 //   forward   128 rows = 4 gates x 32 units, K = half of the hidden state: clusters of 2, H/16 CTAs
 //   backward  128 rows = 128 units of dh (weights transposed), K = 4H split over clusters of up to 8 CTAs: the largest
@@ -37,12 +37,12 @@ namespace {
 constexpr int kRows = 128;          // weight rows of a CTA (MMA M)
 constexpr int kEpiThreads = 256;
 constexpr int kFetchWarps = 8;
-constexpr int kThreads = kEpiThreads + 32 + kFetchWarps * 32;
+constexpr int kIssuers = 4;         // warps that issue MMAs, one on each scheduler of the SM
+constexpr int kIssue0 = kEpiThreads / 32, kFetch0 = kIssue0 + kIssuers;
+constexpr int kThreads = (kFetch0 + kFetchWarps) * 32;
 constexpr int kATile = kRows * 128; // one 64-column block of A
-constexpr int kPiece = 4;           // K blocks of a piece of the state: the MMAs of one run while the next is fetched
+constexpr int kPiece = kIssuers;    // K blocks of a piece of the state, one per issuer: the MMAs of one run while the next is fetched
 constexpr int kMaxPieces = 8;
-constexpr int kTBlocks = 15;        // blocks of the weights that tensor memory holds, 32 columns each
-constexpr int kDCol = 480;          // first TMEM column of the accumulator (at most 32 columns)
 constexpr int kSmemLimit = 227 * 1024;
 constexpr uint32_t kUnset = 0xffffffffu;      // two bf16 that have not been written yet
 constexpr uint64_t kWaitNs = 4000000000ull;   // bound on every wait
@@ -123,6 +123,12 @@ __device__ __forceinline__ uint2 gather_quad(uint32_t v, int lane) {
   const uint32_t far = __shfl_xor_sync(0xffffffffu, pair, 2);
   return lane & 2 ? make_uint2(far, pair) : make_uint2(pair, far);
 }
+template <int N>
+__device__ __forceinline__ void ld_shared_vec(float (&v)[N], const float* p) {
+  if constexpr (N == 1) v[0] = *p;
+  else if constexpr (N == 2) { const float2 x = *reinterpret_cast<const float2*>(p); v[0] = x.x; v[1] = x.y; }
+  else { const float4 x = *reinterpret_cast<const float4*>(p); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+}
 __device__ __forceinline__ void publish(void* p, uint2 v) {
   asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
 }
@@ -148,6 +154,8 @@ struct Layout {
   static constexpr int kUnits = kBwd ? 32 : 16;                       // units a finalising CTA owns
   static constexpr int kFinal = kBwd ? 4 : 2;                         // finalising CTAs of a cluster
   static constexpr int kPer = kUnits * N / kEpiThreads;               // elements of a finalising thread
+  static constexpr int kTBlocks = 16 - kIssuers * N / 32;             // K blocks of the weights in tensor memory, 32 columns each
+  static constexpr int kDCol = kTBlocks * 32;                         // the issuers' accumulators, N columns each
   static constexpr int kPitch = N + 4;                                // floats of a unit's batch in the partial sums
   int kblocks, per, tblocks, sblocks, part;                           // per: K blocks of a CTA (the last may have fewer);
                                                                       // part: floats for one step's partial sums
@@ -193,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxPieces; ++i) mbar_init(&full[i], kFetchWarps);
     mbar_init(wfull, 1);
-    mbar_init(dfull, 1);
+    mbar_init(dfull, kIssuers);
     mbar_init(dfree, kEpiThreads / 32);
     mbar_init(&pfull[0], 1);
     mbar_init(&pfull[1], 1);
@@ -201,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
     mbar_fence_init();
     tma_prefetch_desc(&p.tmW);
   }
-  if (warp == 8) {
+  if (warp == kIssue0) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -214,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
   const uint32_t tmem = *tmem_slot;
 
   // ---- the weights: shared-memory part by TMA, tensor-memory part through registers
-  if (warp == 8) {
+  if (warp == kIssue0) {
     if (elect_one()) {
       mbar_expect_tx(wfull, (uint32_t)((kblocks - tblocks) * kATile));
       for (int kb = tblocks; kb < kblocks; ++kb) {
@@ -226,7 +234,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
         }
       }
     }
-  } else if (warp < 8) {
+  } else if (warp < kIssue0) {
     const int q = warp & 3, row = q * 32 + lane;
     for (int k0 = (warp >> 2) * 16; k0 < tblocks * 64; k0 += 32) {            // 16 K elements = 8 columns at a time
       uint32_t r[8];
@@ -250,12 +258,16 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
   cluster_sync();          // barriers of all mates are initialised, every thread's part of the weights is in place
   tc_fence_after();
 
-  if (warp == 8) {
+  if (warp >= kIssue0 && warp < kFetch0) {
     // ------------------------------------------------------------ issue the products
     const uint32_t idesc_s = umma_idesc_bf16(kRows, N, kBwd ? 1 : 0, 0), idesc_t = umma_idesc_bf16(kRows, N, 0, 0);
     const uint64_t a_desc0 = kBwd ? umma_smem_desc(smem_u32(sA), 8192, 1024) : umma_smem_desc(smem_u32(sA), 16, 1024);
     const uint64_t b_desc0 = umma_smem_desc(smem_u32(sB), 16, 1024);
     constexpr uint64_t kStepA = kBwd ? (2048 >> 4) : (32 >> 4), kStepB = 32 >> 4;
+    // The thread's own instructions between two MMAs bound it (one issuer: 40 to 57 cycles apart, 128 x 16 x 16 is a
+    // fraction of that), so four of them share the K blocks of a piece, each with an accumulator of its own.
+    const int issuer = warp - kIssue0;
+    const uint32_t d_tmem = tmem + (uint32_t)(L::kDCol + issuer * N);
     if (elect_one()) {
       bool ok = wait_bar(wfull, 0u, abort_flag);
       for (int s = 1; ok && s < T; ++s) {                    // step 0 has no recurrent product
@@ -266,31 +278,30 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
           const int piece = p0 + j < npieces ? p0 + j : p0 + j - npieces;
           ok = wait_bar(&full[piece], ph, abort_flag);
           tc_fence_after();
-          const int k1 = min(kblocks, (piece + 1) * kPiece);
-          for (int kb = piece * kPiece; ok && kb < k1; ++kb) {
-            const uint64_t b_desc = b_desc0 + (uint64_t)(kb * (N * 128 >> 4));
-            if (kb >= tblocks) {
-              const uint64_t a_desc = a_desc0 + (uint64_t)((kb - tblocks) * (kATile >> 4));
+          const int kb = piece * kPiece + issuer;
+          if (!ok || kb >= kblocks) continue;
+          const uint64_t b_desc = b_desc0 + (uint64_t)(kb * (N * 128 >> 4));
+          if (kb >= tblocks) {
+            const uint64_t a_desc = a_desc0 + (uint64_t)((kb - tblocks) * (kATile >> 4));
 #pragma unroll
-              for (int i = 0; i < 4; ++i) { umma_bf16(tmem + kDCol, a_desc + i * kStepA, b_desc + i * kStepB, idesc_s, acc); acc = 1; }
-            } else {
-              const uint32_t a_t = tmem + (uint32_t)(kb * 32);
+            for (int i = 0; i < 4; ++i) { umma_bf16(d_tmem, a_desc + i * kStepA, b_desc + i * kStepB, idesc_s, acc); acc = 1; }
+          } else {
+            const uint32_t a_t = tmem + (uint32_t)(kb * 32);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) { umma_bf16_ta(tmem + kDCol, a_t + i * 8, b_desc + i * kStepB, idesc_t, acc); acc = 1; }
-            }
+            for (int i = 0; i < 4; ++i) { umma_bf16_ta(d_tmem, a_t + i * 8, b_desc + i * kStepB, idesc_t, acc); acc = 1; }
           }
         }
         if (ok) umma_commit(dfull);
       }
     }
     __syncwarp();
-  } else if (warp > 8) {
+  } else if (warp >= kFetch0) {
     // ------------------------------------------------------------ fetch the state
-    // A load of a warp is four batch rows of one K block (64 values).  Up to eight are in flight; the first piece is polled
-    // alone, so that waiting SMs leave the L2 to those that still work.
+    // A load of a warp is four batch rows of one K block (64 values), up to eight are in flight.  All of them poll (asking for
+    // the first piece alone until it is there costs a second trip to L2: 2.4 instead of 2.2 us a step at 256 units).
     constexpr int kLoads = N / 8;                            // loads of a warp per piece, at most
     constexpr int kWindow = 8 / kLoads;                      // pieces in flight
-    const int fw = warp - 9, width = kBwd ? 4 * H : H, quads = B / 4;
+    const int fw = warp - kFetch0, width = kBwd ? 4 * H : H, quads = B / 4;
     const __nv_bfloat16* state = (kBwd ? p.dG : p.y) + kbase + (size_t)(lane >> 3) * width + (lane & 7) * 8;
     bool ok = true;
     for (int s = 1; ok && s < T; ++s) {
@@ -321,14 +332,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
           return !__any_sync(0xffffffffu, missing);
         };
         Patience patience;
-        load_unset(0, true);
-        if (j0 == 0)
-          for (uint32_t it = 0; ok && !complete(0); ++it) {
-            load_unset(0, false);
-            ok = !__any_sync(0xffffffffu, patience.over(it, abort_flag));
-          }
 #pragma unroll
-        for (int w = 1; w < kWindow; ++w) load_unset(w, true);
+        for (int w = 0; w < kWindow; ++w) load_unset(w, true);
         if (s > 1 && j0 == 0 && ok) ok = __all_sync(0xffffffffu, wait_bar(dfull, ph ^ 1u, abort_flag));   // the last product has been taken
 #pragma unroll
         for (int w = 0; w < kWindow; ++w) {
@@ -359,6 +364,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
     const uint32_t p_remote = map_to_rank(smem_u32(sP), (uint32_t)dest);
     const uint32_t bar_remote = map_to_rank(smem_u32(&pfull[0]), (uint32_t)dest);
     const uint32_t part_bytes = (uint32_t)(S * (kBwd ? 1 : 4) * UNITS * N * 4);
+    const int u = u0 + threadIdx.x % UNITS, b0 = threadIdx.x / UNITS * PER;        // this thread's unit and its PER batch rows
     float state[PER];                                        // c (forward) / dc (backward) of this thread's elements
 #pragma unroll
     for (int e = 0; e < PER; ++e) state[e] = 0.0f;
@@ -371,7 +377,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
       float in[PER][4], cc[PER], dyv[PER], fgate[PER];
 #pragma unroll
       for (int e = 0; e < PER; ++e) {
-        const int i = threadIdx.x + e * kEpiThreads, b = i / UNITS, u = u0 + i % UNITS;
+        const int b = b0 + e;
         if (b < B && final_cta) {
           const size_t row = (size_t)t * B + b;
           const __nv_bfloat16* g4 = (kBwd ? p.gates : p.xproj) + row * 4 * H + u;
@@ -399,10 +405,30 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
       if (s > 0 && ok) {
         tc_fence_after();
         uint32_t r[N / 2];
+        const uint32_t t_row = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(L::kDCol + half * (N / 2));
 #pragma unroll
-        for (int i = 0; i < N / 16; ++i)
-          tmem_ld_x8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(kDCol + half * (N / 2) + i * 8), r + i * 8);
-        tmem_ld_wait();
+        for (int i = 0; i < N / 16; ++i) tmem_ld_x8(t_row + i * 8, r + i * 8);
+        constexpr int kAtOnce = N == 16 ? 3 : 1;
+#pragma unroll
+        for (int a0 = 1; a0 < kIssuers; a0 += kAtOnce) {
+          uint32_t x[kAtOnce][N / 2];
+#pragma unroll
+          for (int a = 0; a < kAtOnce; ++a)
+            if (a0 + a < kblocks) {
+#pragma unroll
+              for (int i = 0; i < N / 16; ++i) tmem_ld_x8(t_row + (a0 + a) * N + i * 8, x[a] + i * 8);
+            }
+          tmem_ld_wait();
+#pragma unroll
+          for (int a = 0; a < kAtOnce; ++a)
+            if (a0 + a < kblocks) {
+#pragma unroll
+              for (int j = 0; j < N / 2; ++j) {
+                asm volatile("" : "+r"(r[j]), "+r"(x[a][j]));        // no addition moves above the wait
+                r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[a][j]));
+              }
+            }
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(dfree);
@@ -413,49 +439,67 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
         for (int j = 0; j < N / 2; j += 4) st_async_x4(dst + 4u * j, r + j, bar_remote + 8u * ph);
         if (final_cta) ok = __all_sync(0xffffffffu, wait_bar(&pfull[ph], (uint32_t)((s - 1) >> 1) & 1u, abort_flag));
       }
-      const float* part = sP + ((s - 1) & 1) * lay.part;
+      if (final_cta && b0 < B) {          // a batch that is not there is a whole warp's, or none of its lanes'
+        constexpr int SRC = 8, PITCH = UNITS * L::kPitch;  // blocks of [unit][batch]: up to 8 ranks; 2 ranks x 4 gates
+        const float* part = sP + ((s - 1) & 1) * lay.part + threadIdx.x % UNITS * L::kPitch + b0;
+        float sum[kBwd ? 1 : 4][PER];
 #pragma unroll
-      for (int e = 0; e < PER; ++e) {
-        const int i = threadIdx.x + e * kEpiThreads, b = i / UNITS, u = u0 + i % UNITS;
-        if (b < B && final_cta) {
-          const size_t row = (size_t)t * B + b;
-          const float* mine = part + i % UNITS * L::kPitch + b;
-          if (!kBwd) {
-            float pre[4];
+        for (int e = 0; e < PER; ++e) {
+          if (kBwd) sum[0][e] = dyv[e];
+          else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              pre[k] = in[e][k];
-              if (s > 0) pre[k] += mine[k * UNITS * L::kPitch] + mine[(4 + k) * UNITS * L::kPitch];
+            for (int k = 0; k < 4; ++k) sum[kBwd ? 0 : k][e] = in[e][k];
+          }
+        }
+        if (s > 0) {
+          float v[SRC][PER];
+#pragma unroll
+          for (int k = 0; k < SRC; ++k)
+            if (!kBwd || k < S) ld_shared_vec<PER>(v[k], part + k * PITCH);
+#pragma unroll
+          for (int k = 0; k < SRC; ++k)
+            if (!kBwd || k < S) {
+#pragma unroll
+              for (int e = 0; e < PER; ++e) sum[kBwd ? 0 : k & 3][e] += v[k][e];
             }
-            const float ig = sigmoidf_(pre[0]), fg = sigmoidf_(pre[1]), gg = tanhf(pre[2]), og = sigmoidf_(pre[3]);
+        }
+        if (!kBwd) {
+          uint2 h4[PER];
+#pragma unroll
+          for (int e = 0; e < PER; ++e) {
+            const float ig = sigmoidf_(sum[0][e]), fg = sigmoidf_(sum[kBwd ? 0 : 1][e]), gg = tanhf(sum[kBwd ? 0 : 2][e]),
+                        og = sigmoidf_(sum[kBwd ? 0 : 3][e]);
             const float c = fg * state[e] + ig * gg;
             state[e] = c;
-            const uint2 h4 = gather_quad(bf16_bits(og * tanhf(c)), lane);
-            if ((lane & 3) == 0) publish(p.y + row * H + u, h4);
+            h4[e] = gather_quad(bf16_bits(og * tanhf(c)), lane);
             in[e][0] = ig; in[e][1] = fg; in[e][2] = gg; in[e][3] = og;
-          } else {
-            float dh = dyv[e];
-            if (s > 0) {
-              for (int k = 0; k < S; ++k) dh += mine[k * UNITS * L::kPitch];
-            }
-            const float dct = state[e] + dh * cc[e];
+          }
+#pragma unroll
+          for (int e = 0; e < PER; ++e)
+            if ((lane & 3) == 0) publish(p.y + ((size_t)t * B + b0 + e) * H + u, h4[e]);
+        } else {
+          uint2 d4[PER];                                     // lane k of four publishes gate k
+#pragma unroll
+          for (int e = 0; e < PER; ++e) {
+            const float dh = sum[0][e], dct = state[e] + dh * cc[e];
             state[e] = dct * fgate[e];
             const float d[4] = {dct * in[e][0], dct * in[e][1], dct * in[e][2], dh * in[e][3]};
-            uint2 d4 = make_uint2(0, 0);                     // lane k of four publishes gate k
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const uint2 g = gather_quad(bf16_bits(d[k]), lane);
-              if ((lane & 3) == k) d4 = g;
+              if (k == 0 || (lane & 3) == k) d4[e] = g;
               db[k] += d[k];
             }
-            publish(p.dG + row * 4 * H + (lane & 3) * H + (u & ~3), d4);
           }
+#pragma unroll
+          for (int e = 0; e < PER; ++e)
+            publish(p.dG + (((size_t)t * B + b0 + e) * 4 + (lane & 3)) * H + (u & ~3), d4[e]);
         }
       }
       if (!kBwd) {                        // what only the backward pass reads leaves after the hand-over
 #pragma unroll
         for (int e = 0; e < PER; ++e) {
-          const int i = threadIdx.x + e * kEpiThreads, b = i / UNITS, u = u0 + i % UNITS;
+          const int b = b0 + e;
           if (b < B) {
             const size_t row = (size_t)t * B + b;
             p.c[row * H + u] = state[e];
@@ -479,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_sequence_kernel(const __grid
     __nanosleep(1000000);
     if (threadIdx.x == 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 1);
   }
-  if (warp == 8) {
+  if (warp == kIssue0) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
