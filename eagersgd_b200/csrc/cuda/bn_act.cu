@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const __nv_bfloat16* __re
 // them cost 4 us a layer); the first block also leaves them, and the running statistics, for later.  Threads keep a
 // fixed group of 8 channels and walk over rows, last row first: the producer of y wrote its end last, so that part
 // is still in L2, and what is left there afterwards is z's beginning, where the next layer starts.
-// With a residual the sign of z cannot be told from y alone: the backward passes then read one bit per element (mask) instead
-// of z, a sixteenth of the bytes.
+// With a residual the sign of z cannot be told from y alone, and a convolution's data gradient has no y to tell it from: the
+// backward passes then read one bit per element (mask) instead of z, a sixteenth of the bytes.
 template <bool kRes>
 __global__ void __launch_bounds__(256, 2)
 bn_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ z,
@@ -164,7 +164,7 @@ bn_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restri
           if (relu) { v[2 * q] = fmaxf(v[2 * q], 0.0f); v[2 * q + 1] = fmaxf(v[2 * q + 1], 0.0f); }
         }
         const uint4 out = st8(z + rr * C + g * 8, v);
-        if (kRes && mask != nullptr) mask[rr * mp.groups + g] = sign_bits(out);
+        if (mask != nullptr) mask[rr * mp.groups + g] = sign_bits(out);
       }
     }
   }
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256, 2)
 bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dz, const uint8_t* __restrict__ mask, const __nv_bfloat16* __restrict__ y,
                     const float* __restrict__ aux, const float* __restrict__ gamma, const float* __restrict__ dbeta,
                     const float* __restrict__ dgamma, __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dres, int64_t M,
-                    int C, Map mp, float inv_count, float* acc_dgamma, float* acc_dbeta) {
+                    int C, Map mp, float inv_count, float* acc_dgamma, float* acc_dbeta, int last_first) {
   pdl_enter();
   const int gl = threadIdx.x % mp.cg, rl = threadIdx.x / mp.cg, g = blockIdx.y * mp.cg + gl;
   if (g >= mp.groups) return;
@@ -268,14 +268,15 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dz, const uint8_t* __restr
     }
   }
   const int64_t step = (int64_t)gridDim.x * mp.rows_par;
+  // last_first: straight after a data gradient, which wrote dz (and read y) front to back
+  const int64_t flip = last_first ? M - 1 : 0, sign = last_first ? -1 : 1;
   for (int64_t r = (int64_t)blockIdx.x * mp.rows_par + rl; r < M; r += 4 * step) {
     uint4 rd[4], ry[4];
     uint32_t bits[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int64_t rr = r + u * step;
-      if (rr < M) {
-        const int64_t off = rr * C + g * 8;
+      if (r + u * step < M) {
+        const int64_t rr = flip + sign * (r + u * step), off = rr * C + g * 8;
         rd[u] = *reinterpret_cast<const uint4*>(dz + off);
         ry[u] = *reinterpret_cast<const uint4*>(y + off);
         if (kMode == 1) bits[u] = mask[rr * mp.groups + g];
@@ -283,8 +284,8 @@ bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dz, const uint8_t* __restr
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int64_t rr = r + u * step;
-      if (rr < M) {
+      if (r + u * step < M) {
+        const int64_t rr = flip + sign * (r + u * step);
         const int64_t off = rr * C + g * 8;
         float d[8], yy[8], o[8];
         masked<kMode>(rd[u], ry[u], bits[u], fsc, fsh, d, yy);
@@ -346,7 +347,7 @@ int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, voi
 }
 
 // sum / sqsum: the batch sums of y.  aux [4][C] receives mean, inverse standard deviation, scale and shift; mask (optional,
-// with a residual: [M][C / 8] bytes) which elements of z are above zero.
+// [M][C / 8] bytes) which elements of z are above zero.
 int esgd_bn_fwd(const void* y, const void* residual, void* z, void* mask, const float* sum, const float* sqsum, const float* gamma,
                 const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu,
                 float momentum, float eps, void* stream) {
@@ -375,18 +376,18 @@ int esgd_bn_bwd_reduce(const void* dz, const void* mask, const void* y, const fl
                       (const __nv_bfloat16*)y, aux, M, C, mp, dbeta, dgamma);
 }
 
-// dres (optional): the gradient behind the ReLU, for the shortcut.
+// dres (optional): the gradient behind the ReLU, for the shortcut.  last_first: rows in descending order.
 // acc_dgamma / acc_dbeta (optional): fp32 accumulators the two parameter gradients are added to.
 int esgd_bn_bwd_apply(const void* dz, const void* mask, const void* y, const float* aux, const float* gamma, const float* dbeta,
-                      const float* dgamma, void* dy, void* dres, int64_t M, int C, int mode, float* acc_dgamma, float* acc_dbeta,
-                      void* stream) {
+                      const float* dgamma, void* dy, void* dres, int64_t M, int C, int mode, int last_first, float* acc_dgamma,
+                      float* acc_dbeta, void* stream) {
   if (C % 8 || mode < 0 || mode > 2 || (mode == 1 && mask == nullptr)) return -1;
   const Map mp = make_map(C);
   auto kernel = dres != nullptr ? (mode == 0 ? bn_bwd_apply_kernel<0, true> : mode == 1 ? bn_bwd_apply_kernel<1, true> : bn_bwd_apply_kernel<2, true>)
                                 : (mode == 0 ? bn_bwd_apply_kernel<0, false> : mode == 1 ? bn_bwd_apply_kernel<1, false> : bn_bwd_apply_kernel<2, false>);
   return esgd::launch(kernel, grid_for(mp, M, kApplyBlocks), 256, 0, stream, (const __nv_bfloat16*)dz, (const uint8_t*)mask,
                       (const __nv_bfloat16*)y, aux, gamma, dbeta, dgamma, (__nv_bfloat16*)dy, (__nv_bfloat16*)dres, M, C, mp,
-                      1.0f / (float)M, acc_dgamma, acc_dbeta);
+                      1.0f / (float)M, acc_dgamma, acc_dbeta, last_first);
 }
 
 }  // extern "C"

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <atomic>
+#include "bn_grad.h"
 #include "launch.cuh"
 
 namespace {
@@ -46,7 +47,10 @@ struct Args {
   const float *scale, *shift;
   const __nv_bfloat16* residual;
   int relu;
-  float *sum, *sqsum;
+  float *sum, *sqsum;                                          // statistics of y; with bn_y dbeta and dgamma (bn_grad.h)
+  const __nv_bfloat16* bn_y;
+  const uint8_t* bn_mask;
+  const float* bn_aux;
 };
 
 // The input rows of a tile with a margin of one pixel (zeros outside the image): [ti][rows][pw] pixels of C channels.
@@ -105,6 +109,24 @@ __global__ void __launch_bounds__(kThreads) conv_narrow_kernel(const Shape s, co
       float acc[NT][4];
 #pragma unroll
       for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f;
+      // batch-norm input and mask of this thread's outputs: on their way while the products run
+      __nv_bfloat162 by[kT ? NT : 1][2];
+      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};           // bits 8t + (c % 8) of the thread's columns
+      if (kT && a.bn_y != nullptr) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int pp = m * 16 + (lane >> 2) + h * 8, im2 = pp / (s.tr * s.Wo);
+          if (pp >= pixels || n0 + im2 >= s.N) continue;
+          const int64_t pix = ((int64_t)(n0 + im2) * s.Ho + oh0) * s.Wo + (pp - im2 * s.tr * s.Wo);
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+            by[t][h] = *reinterpret_cast<const __nv_bfloat162*>(a.bn_y + pix * CN + wn * NT * 8 + t * 8 + (lane & 3) * 2);
+          if (a.bn_mask != nullptr) {
+            const uint8_t* mp = a.bn_mask + pix * (CN / 8) + wn * NT;
+            keep[h] = NT == 2 ? *reinterpret_cast<const uint16_t*>(mp) : *reinterpret_cast<const uint32_t*>(mp);
+          }
+        }
+      }
 #pragma unroll
       for (int tap = 0; tap < 9; ++tap) {
         const uint32_t xt = x0 + (uint32_t)((tap / 3 * s.pw + tap % 3) * PX);
@@ -144,12 +166,23 @@ __global__ void __launch_bounds__(kThreads) conv_narrow_kernel(const Shape s, co
             v1 += r.y;
           }
           if (a.relu) { v0 = fmaxf(v0, 0.0f); v1 = fmaxf(v1, 0.0f); }
+          if (kT) {
+            const uint32_t bits = keep[h] >> (t * 8 + (lane & 3) * 2);
+            v0 = bits & 1u ? v0 : 0.0f;
+            v1 = bits & 2u ? v1 : 0.0f;
+          }
           const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
           *reinterpret_cast<__nv_bfloat162*>(a.y + pix * CN + c) = o;
           if (a.sum != nullptr) {
             const float2 f = __bfloat1622float2(o);
+            float2 g = f;
+            if (kT) {
+              g = __bfloat1622float2(by[kT ? t : 0][h]);
+              g.x -= __ldg(a.bn_aux + c);
+              g.y -= __ldg(a.bn_aux + c + 1);
+            }
             st[t][0] += f.x; st[t][1] += f.y;
-            st[t][2] = fmaf(f.x, f.x, st[t][2]); st[t][3] = fmaf(f.y, f.y, st[t][3]);
+            st[t][2] = fmaf(f.x, g.x, st[t][2]); st[t][3] = fmaf(f.y, g.y, st[t][3]);
           }
         }
       }
@@ -167,7 +200,10 @@ __global__ void __launch_bounds__(kThreads) conv_narrow_kernel(const Shape s, co
         if (lane < 4) atomicAdd(&s_stat[(q >> 1) * CN + wn * NT * 8 + t * 8 + lane * 2 + (q & 1)], v);
       }
     __syncthreads();
-    if (threadIdx.x < 2 * CN) atomicAdd((threadIdx.x < CN ? a.sum : a.sqsum) + threadIdx.x % CN, s_stat[threadIdx.x]);
+    if (threadIdx.x < 2 * CN) {
+      const float scale = kT && threadIdx.x >= CN ? __ldg(a.bn_aux + threadIdx.x) : 1.0f;      // 1 / std
+      atomicAdd((threadIdx.x < CN ? a.sum : a.sqsum) + threadIdx.x % CN, s_stat[threadIdx.x] * scale);
+    }
   }
 }
 
@@ -357,7 +393,8 @@ extern "C" {
 // y = act(scale * conv + shift + residual), each part optional; sum / sqsum (caller-zeroed) receive y's statistics.
 int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int stride, const float* scale,
                          const float* shift, const void* residual, int relu, float* sum, float* sqsum, void* stream) {
-  Args a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, scale, shift, (const __nv_bfloat16*)residual, relu, sum, sqsum};
+  Args a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, scale, shift, (const __nv_bfloat16*)residual, relu, sum, sqsum,
+         nullptr, nullptr, nullptr};
   cudaStream_t s = (cudaStream_t)stream;
   if (Cin == 16 && Cout == 16) return launch_conv<16, 16, false>(a, N, H, W, stride, s);
   if (Cin == 16 && Cout == 32) return launch_conv<16, 32, false>(a, N, H, W, stride, s);
@@ -367,10 +404,15 @@ int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, in
   return -100;
 }
 
-// dx [N,H,W,Cin] from dy [N,H,W,Cout], stride 1; residual (optional) is added before the rounding.
+// dx [N,H,W,Cin] from dy [N,H,W,Cout], stride 1; residual (optional) is added before the rounding; bn (optional): bn_grad.h.
 int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, const void* residual,
-                           void* stream) {
-  Args a{(const __nv_bfloat16*)dy, (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, nullptr, nullptr, (const __nv_bfloat16*)residual, 0, nullptr, nullptr};
+                           const esgd_bn_grad* bn, void* stream) {
+  Args a{(const __nv_bfloat16*)dy, (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, nullptr, nullptr, (const __nv_bfloat16*)residual, 0,
+         nullptr, nullptr, nullptr, nullptr, nullptr};
+  if (bn != nullptr) {
+    a.sum = bn->sums; a.sqsum = bn->sums + Cin;
+    a.bn_y = (const __nv_bfloat16*)bn->y; a.bn_mask = (const uint8_t*)bn->mask; a.bn_aux = bn->aux;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   if (Cin == 16 && Cout == 16) return launch_conv<16, 16, true>(a, N, H, W, 1, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, true>(a, N, H, W, 1, s);

@@ -51,7 +51,7 @@ __device__ __forceinline__ void load_filter_tap(const CUtensorMap* tm, const Fil
 template <int BN_, bool kT>
 struct ConvProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kTwoPanels = false;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, stride, pad;
@@ -103,13 +103,11 @@ struct ConvProblem {
   __device__ __forceinline__ void store_panel(const Tile& t, int panel, const void* smem) const {
     tma_store_4d(&tmY, smem, t.n0 + panel * 64, t.w0, t.h0, t.i0);
   }
-  __device__ __forceinline__ bool row_valid(const Tile& t, int row) const {
-    const int wi = row % BW, hi = (row / BW) % BH, ni = row / (BW * BH);
-    return ni < BI && t.w0 + wi < Wo && t.h0 + hi < Ho && t.i0 + ni < N;
+  // A box is part of one row (BH = BI = 1), whole rows of one image (BH divides Ho) or whole images: consecutive pixels.
+  __device__ __forceinline__ int valid_prefix(const Tile& t) const {
+    return BI > 1 ? min(BI, N - t.i0) * BW * BH : min(BW, Wo - t.w0) * BH;
   }
-  __device__ __forceinline__ int valid_prefix(const Tile& t) const {   // box inside the tensor: its pixels, in order
-    return (t.w0 + BW <= Wo && t.h0 + BH <= Ho && t.i0 + BI <= N) ? BW * BH * BI : -1;
-  }
+  __device__ __forceinline__ int64_t first_row(const Tile& t) const { return ((int64_t)t.i0 * Ho + t.h0) * Wo + t.w0; }
   __device__ __forceinline__ void store_f32(const Tile&, int, const void*, bool) const {}
   __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
     tma_load_4d(smem, &tmR, bar, t.n0 + panel * 64, t.w0, t.h0, t.i0);
@@ -124,7 +122,7 @@ struct ConvProblem {
 template <int BN_, bool kT>
 struct ConvHaloProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kTwoPanels = false;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, pad;
@@ -165,8 +163,8 @@ struct ConvHaloProblem {
     const int hl = row / PW, wl = row - hl * PW;
     return (hl < BH && wl < Wo) ? hl * Wo + wl : -1;
   }
-  __device__ __forceinline__ bool row_valid(const Tile&, int row) const { return row < BH * Wo; }
   __device__ __forceinline__ int valid_prefix(const Tile&) const { return BH * Wo; }
+  __device__ __forceinline__ int64_t first_row(const Tile& t) const { return ((int64_t)t.i0 * Ho + t.h0) * Wo; }
   __device__ __forceinline__ void store_f32(const Tile&, int, const void*, bool) const {}
   __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
     tma_load_4d(smem, &tmR, bar, t.n0 + panel * 64, 0, t.h0, t.i0);
@@ -183,7 +181,7 @@ struct ConvHaloProblem {
 template <int BN_>
 struct ConvWgradProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = true, B_MN = true, kZeroStages = true;
+  static constexpr bool A_MN = true, B_MN = true, kZeroStages = true, kTwoPanels = false;
   CUtensorMap tmDY, tmX, tmDW;
   int N, Ho, Wo, Cout, Cin;
   int R, S, stride, pad;
@@ -221,8 +219,8 @@ struct ConvWgradProblem {
   __device__ __forceinline__ void load_a(const Tile&, int, uint8_t*, uint64_t*) const {}
   __device__ __forceinline__ void load_b(const Tile&, int, uint8_t*, uint64_t*) const {}
   __device__ __forceinline__ void store_panel(const Tile&, int, const void*) const {}
-  __device__ __forceinline__ bool row_valid(const Tile& t, int row) const { return t.m0 + row < Cout; }
   __device__ __forceinline__ int valid_prefix(const Tile& t) const { return min(BM, Cout - t.m0); }
+  __device__ __forceinline__ int64_t first_row(const Tile& t) const { return t.m0; }
   __device__ __forceinline__ void load_res_panel(const Tile&, int, void*, uint64_t*) const {}
   __device__ __forceinline__ int out_row(int row) const { return row; }
   static constexpr bool kHalo = false;
@@ -231,14 +229,14 @@ struct ConvWgradProblem {
   }
 };
 
-template <class P>
+template <class P, bool kBn>
 __global__ void __launch_bounds__(NUM_THREADS, 1) conv_kernel(const __grid_constant__ P prob, const Epilogue ep) {
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&prob.tmX);
     tma_prefetch_desc(&prob.tmW);
     tma_prefetch_desc(&prob.tmY);
   }
-  run(prob, ep);
+  run<P, kBn>(prob, ep);
 }
 
 template <class P>
@@ -283,12 +281,12 @@ inline int ksteps_of(int c) { return c >= 64 ? BK / 16 : (c + 15) / 16; }
 // narrow layers: the MMA computes no more columns than there are (the epilogue drops the rest either way)
 inline int mma_columns(int n, int bn) { return n >= bn ? bn : (n + 15) / 16 * 16; }
 
-template <int BN, bool kT>
+template <int BN, bool kT, bool kBn>
 int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
   using P = ConvProblem<BN, kT>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(conv_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg<BN>::SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
@@ -357,7 +355,7 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
   }
   ep.tx_bytes_a = (uint32_t)(p.BW * p.BH * p.BI * 128);
   ep.tx_bytes = ep.tx_bytes_a + (uint32_t)Cfg<BN>::B_STAGE_BYTES;
-  return esgd::launch(conv_kernel<P>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+  return esgd::launch(conv_kernel<P, kBn>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 // Halo mode applies to stride-1 convolutions with full-width tiles: the box (output rows + filter margin, full
@@ -378,12 +376,12 @@ bool halo_applicable(const ConvArgs& a, int Ho, int Wo, int* bh_out) {
   return true;
 }
 
-template <int BN, bool kT>
+template <int BN, bool kT, bool kBn>
 int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
   using P = ConvHaloProblem<BN, kT>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(conv_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg<BN>::SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
@@ -430,7 +428,7 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
   if (grid > total) grid = total;
   ep.tx_bytes_a = (uint32_t)(p.PW * (bh + a.R - 1) * 128);
   ep.tx_bytes = 0;
-  return esgd::launch(conv_kernel<P>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+  return esgd::launch(conv_kernel<P, kBn>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 template <int BN>
@@ -512,16 +510,16 @@ Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* er
   return ep;
 }
 
-template <bool kT>
+template <bool kT, bool kBn = false>
 int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
   const int Ho = a.out_h ? a.out_h : (a.H + 2 * a.pad - a.R) / a.stride + 1, Wo = a.out_w ? a.out_w : (a.W + 2 * a.pad - a.S) / a.stride + 1;
   const int BN = tile_columns(a.Cout, (int)(((int64_t)a.N * Ho * Wo + BM - 1) / BM), sm_count());
   int bh = 0;
   if (a.Cout <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
-    return BN == 64 ? launch_halo<64, kT>(a, ep, bh, s) : launch_halo<128, kT>(a, ep, bh, s);
-  if (BN == 64) return launch<64, kT>(a, ep, s);
-  if (BN == 128) return launch<128, kT>(a, ep, s);
-  return launch<256, kT>(a, ep, s);
+    return BN == 64 ? launch_halo<64, kT, kBn>(a, ep, bh, s) : launch_halo<128, kT, kBn>(a, ep, bh, s);
+  if (BN == 64) return launch<64, kT, kBn>(a, ep, s);
+  if (BN == 128) return launch<128, kT, kBn>(a, ep, s);
+  return launch<256, kT, kBn>(a, ep, s);
 }
 
 }  // namespace
@@ -557,23 +555,25 @@ int esgd_conv2d_fwd(const void* x, const void* w, void* y, int N, int H, int W, 
 }
 
 // Data gradient on the weights as stored: dy [N,Ho,Wo,Cout], w [Cout,R,S,Cin], dx [N,H,W,Cin] (dense NHWC); residual
-// (optional, stride 1, like dx) is added before the rounding.
+// (optional, stride 1, like dx) is added before the rounding.  bn (optional, stride 1): see bn_grad.h; -100 for channels it
+// does not take.
 // Stride 1: one launch, any R x S with padding up to min(R, S) - 1.  Stride 2: 3x3 filters with padding 1 on even H and W;
 // each output parity (h % 2, w % 2) meets 1, 2, 2 or 4 of the nine taps and is a dense stride-1 problem written
 // into its interleaved pixels of dx (dx[2i + p] uses the filter rows r with (p + 1 - r) even).
 int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, int R, int S,
-                      int stride, int pad, const void* residual, int* error_flag, void* stream) {
+                      int stride, int pad, const void* residual, const esgd_bn_grad* bn, int* error_flag, void* stream) {
   if (Cin % 8 || Cout % 8 || ((uintptr_t)residual & 15)) return -1;
-  if (residual != nullptr && stride != 1) return -2;
+  if ((residual != nullptr || bn != nullptr) && stride != 1) return -2;
   Epilogue ep = epilogue_for(Cin, 0, nullptr, nullptr, error_flag);
   ep.residual = residual;
+  if (!set_bn_grad(ep, bn)) return -100;
   cudaStream_t s = (cudaStream_t)stream;
   if (stride == 1) {
     if (pad > R - 1 || pad > S - 1 || R != S) return -1;
     ConvArgs a{dy, w, dx, N, H + 2 * pad - R + 1, W + 2 * pad - S + 1, Cout, Cin, R, S, 1, R - 1 - pad};
     a.fR = R; a.fS = S;
     a.taps = FilterTaps{R - 1, -1, S - 1, -1};
-    return dispatch<true>(a, ep, s);
+    return bn != nullptr ? dispatch<true, true>(a, ep, s) : dispatch<true>(a, ep, s);
   }
   if (stride != 2 || R != 3 || S != 3 || pad != 1 || H % 2 || W % 2) return -1;
   for (int ph = 0; ph < 2; ++ph)

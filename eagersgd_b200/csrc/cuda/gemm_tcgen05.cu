@@ -21,7 +21,7 @@ namespace {
 template <int BN_, bool A_MN_, bool B_MN_>
 struct GemmProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false;
+  static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false, kTwoPanels = true;
   CUtensorMap tmA, tmB, tmC, tmR;   // tmC: bf16 panels of 64 columns or fp32 ones of 32; tmR: optional residual
   int M, N, K;
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
@@ -76,9 +76,9 @@ struct GemmProblem {
   __device__ __forceinline__ void store_panel(const Tile& t, int panel, const void* smem) const {
     tma_store_2d(&tmC, smem, t.n0 + panel * 64, t.m0);
   }
-  __device__ __forceinline__ bool row_valid(const Tile& t, int row) const { return t.m0 + row < M; }
   __device__ __forceinline__ int out_row(int row) const { return row; }
   __device__ __forceinline__ int valid_prefix(const Tile& t) const { return min(BM, M - t.m0); }
+  __device__ __forceinline__ int64_t first_row(const Tile& t) const { return t.m0; }
   __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
     tma_load_2d(smem, &tmR, bar, t.n0 + panel * 64, t.m0);
   }
@@ -88,13 +88,13 @@ struct GemmProblem {
   }
 };
 
-template <class P>
+template <class P, bool kBn>
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_kernel(const __grid_constant__ P prob, const Epilogue ep) {
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&prob.tmA);
     tma_prefetch_desc(&prob.tmB);
   }
-  run(prob, ep);
+  run<P, kBn>(prob, ep);
 }
 
 int sm_count() {
@@ -113,12 +113,12 @@ struct GemmArgs {
   int M, N, K, lda, ldb, ldc, out_mode, splits;
 };
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool kBn = false>
 int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   using P = GemmProblem<BN, A_MN, B_MN>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg<BN>::SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
@@ -164,11 +164,13 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
   if (p.splits > 1 && g.out_mode != OUT_F32_ATOMIC) return -2;
   ep.res_bytes = PANEL_BYTES;
+  const bool two_panels = kBn && ep.residual != nullptr;
   const int sms = sm_count();
   int grid;
   // B stays in shared memory when its whole K extent fits beside four A stages and every CTA has several
   // tiles of one column range to amortise the load over
-  const bool resident = resident_enabled() && p.splits == 1 && p.kb_total <= Cfg<BN>::MAX_RES_KB &&
+  const bool resident = resident_enabled() && p.splits == 1 &&
+                        p.kb_total <= (two_panels ? Cfg<BN>::MAX_RES_KB2 : Cfg<BN>::MAX_RES_KB) &&
                         p.n_tiles <= sms / 2 && p.m_tiles >= 2 * (sms / p.n_tiles);
   p.res_kb = resident ? p.kb_total : 0;
   p.fixed_n = (ep.col_sum != nullptr || resident) ? 1 : 0;
@@ -181,7 +183,7 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
     const int total = p.m_tiles * p.n_tiles * p.splits;
     grid = total < sms ? total : sms;
   }
-  return esgd::launch(gemm_kernel<P>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+  return esgd::launch(gemm_kernel<P, kBn>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 template <int BN>
@@ -225,6 +227,25 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
   if (BN == 64) return launch_major<64>(a_mn, b_mn, g, ep, s);
   if (BN == 128) return launch_major<128>(a_mn, b_mn, g, ep, s);
   return launch_major<256>(a_mn, b_mn, g, ep, s);
+}
+
+// Data gradient of a 1x1 convolution behind a batch norm: dx [M][N] = dy [M][K] * w [K][N] (+ residual), see bn_grad.h.
+// -100: not a shape for it.
+int esgd_gemm_bn_dgrad(const void* dy, const void* w, void* dx, int M, int N, int K, const void* residual, const esgd_bn_grad* bn,
+                       int* error_flag, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || N % 8 || K % 8 || ((uintptr_t)dx & 15) || ((uintptr_t)residual & 15)) return -1;
+  GemmArgs g{dy, w, dx, M, N, K, K, N, N, OUT_BF16, 1};
+  Epilogue ep;
+  ep.out_mode = OUT_BF16; ep.relu = 0; ep.n_total = N; ep.scale = nullptr; ep.bias = nullptr; ep.bias_kind = BIAS_F32;
+  ep.col_sum = nullptr; ep.col_sqsum = nullptr; ep.error_flag = error_flag;
+  ep.tx_bytes = 0; ep.tx_bytes_a = 0;
+  ep.residual = residual; ep.ldr = N;
+  if (!set_bn_grad(ep, bn)) return -100;
+  cudaStream_t s = (cudaStream_t)stream;
+  const int BN = tile_columns(N, (M + BM - 1) / BM, sm_count());
+  if (BN == 64) return launch<64, false, true, true>(g, ep, s);
+  if (BN == 128) return launch<128, false, true, true>(g, ep, s);
+  return launch<256, false, true, true>(g, ep, s);
 }
 
 }  // extern "C"

@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include "bn_grad.h"
 #include "launch.cuh"
 #include "sm100_primitives.cuh"
 
@@ -61,21 +62,40 @@ struct Epilogue {
   const void* residual;    // optional bf16 tensor added to the product before rounding (same shape as the output)
   int ldr;                 // its row stride in elements (GEMM)
   uint32_t res_bytes;      // bytes one panel of it delivers
+  // Data gradients: the product is the gradient of z = act(batch_norm(bn_y)).  Elements whose bit in bn_mask is clear are
+  // stored as zeros, and col_sum / col_sqsum receive dbeta and dgamma: sum g and sum g * (bn_y - mean) / std.
+  const __nv_bfloat16* bn_y = nullptr;       // [rows][n_total], n_total a multiple of 64
+  const uint8_t* bn_mask = nullptr;          // [rows][n_total / 8], null: no ReLU
+  const float* bn_aux = nullptr;             // mean [n_total], 1 / std [n_total]
 };
+
+// False: the kernels do not take this many channels.
+inline bool set_bn_grad(Epilogue& ep, const esgd_bn_grad* bn) {
+  if (bn == nullptr) return true;
+  if (ep.n_total % 64 || ((uintptr_t)bn->mask & 7) || ((uintptr_t)bn->aux & 7)) return false;
+  ep.bn_y = (const __nv_bfloat16*)bn->y;
+  ep.bn_mask = (const uint8_t*)bn->mask;
+  ep.bn_aux = bn->aux;
+  ep.col_sum = bn->sums;
+  ep.col_sqsum = bn->sums + ep.n_total;
+  return true;
+}
 
 template <int BN>
 struct Cfg {
   static constexpr int B_STAGE_BYTES = BN * BK * 2;
-  static constexpr int STAGES = BN == 256 ? 3 : (BN == 128 ? 5 : 6);
+  static constexpr int STAGES = BN == 256 ? 3 : (BN == 128 ? 5 : 6);             // with one panel per group
   static constexpr int ACCS = BN == 256 ? 2 : 4;       // accumulators in tensor memory: tiles in flight
   static constexpr int TMEM_COLS = ACCS * BN;
   static constexpr int MAX_STAGES = 8;                 // A-only ring of the B-resident mode
   static constexpr int STAGE_AREA = 161 * 1024;        // operand stages (ring, or A ring + resident B)
+  static constexpr int STAGE_AREA2 = STAGE_AREA - NUM_GROUPS * PANEL_BYTES;      // ... beside two panels per group
   static constexpr int SMEM_BYTES = 1024 + STAGE_AREA + NUM_GROUPS * PANEL_BYTES + 512;
   static_assert(STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) <= STAGE_AREA, "ring does not fit");
   static_assert(SMEM_BYTES <= 227 * 1024, "over the shared-memory limit of a CTA");
   // k-blocks of B that may stay resident: four A stages must still fit
   static constexpr int MAX_RES_KB = (STAGE_AREA - 4 * A_STAGE_BYTES) / B_STAGE_BYTES;
+  static constexpr int MAX_RES_KB2 = (STAGE_AREA2 - 4 * A_STAGE_BYTES) / B_STAGE_BYTES;
 };
 
 // Halo mode (policies with kHalo): a convolution tile loads, per 64-channel block, ONE box of input pixels
@@ -133,25 +153,26 @@ __device__ __forceinline__ void affine4(const Epilogue& ep, int col, float v[4])
 }
 
 // 32 accumulator columns of one row -> bf16 -> four 16-byte chunks of the swizzled staging panel.
-// kPlain leaves out the affine / residual / ReLU code altogether: as run-time options they would be predicated
+// The plain kind leaves out the affine / residual / ReLU code altogether: as run-time options they would be predicated
 // instructions that still take issue slots in the common case that uses none.
-template <bool kPlain>
-__device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* panel, int row, int half, int col0,
-                                                  const Epilogue& ep, bool has_residual) {
+enum PackKind { PACK_PLAIN, PACK_AFFINE, PACK_MASKED };      // affine map, residual, ReLU; residual, bit mask
+template <int kKind>
+__device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* panel, const uint8_t* rpanel, int row, int half,
+                                                  int col0, const Epilogue& ep, bool has_residual, uint32_t keep = 0xffffffffu) {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     float v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[g * 8 + j]);
     const int chunk = half * 4 + g;          // 16-byte chunk within the 128-byte row
-    uint4* slot = reinterpret_cast<uint4*>(panel + row * 128 + ((chunk ^ (row & 7)) << 4));
-    if (!kPlain) {
-      if (ep.bias != nullptr) {
+    const int slot = row * 128 + ((chunk ^ (row & 7)) << 4);
+    if (kKind != PACK_PLAIN) {
+      if (kKind == PACK_AFFINE && ep.bias != nullptr) {
         affine4(ep, col0 + g * 8, v);
         affine4(ep, col0 + g * 8 + 4, v + 4);
       }
-      if (has_residual) {     // the residual panel was brought into this very buffer by TMA; add in place
-        const uint4 rv = *slot;
+      if (has_residual) {     // its panel was brought by TMA, possibly into this very buffer
+        const uint4 rv = *reinterpret_cast<const uint4*>(rpanel + slot);
         const uint32_t* rw = reinterpret_cast<const uint32_t*>(&rv);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -159,16 +180,20 @@ __device__ __forceinline__ void pack_row_to_panel(const uint32_t* r, uint8_t* pa
           v[2 * j + 1] += __uint_as_float(rw[j] & 0xffff0000u);
         }
       }
-      if (ep.relu) {
+      if (kKind == PACK_AFFINE && ep.relu) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], 0.0f);
+      }
+      if (kKind == PACK_MASKED) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (keep >> (g * 8 + j)) & 1u ? v[j] : 0.0f;
       }
     }
     uint4 pk;
     __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
     for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-    *slot = pk;
+    *reinterpret_cast<uint4*>(panel + slot) = pk;
   }
 }
 
@@ -195,7 +220,8 @@ __device__ __forceinline__ uint64_t pack_f32x2(uint32_t lo, uint32_t hi) {
   return r;
 }
 __device__ __forceinline__ void add_f32x2(uint64_t& a, uint64_t b) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b)); }
-__device__ __forceinline__ void fma_f32x2(uint64_t& acc, uint64_t a) { asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc) : "l"(a)); }
+__device__ __forceinline__ void fma_f32x2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ uint64_t bf16x2_to_f32x2(uint32_t w) { return pack_f32x2(w << 16, w & 0xffff0000u); }
 __device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
   uint32_t lo, hi;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
@@ -210,13 +236,16 @@ __device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
 //   void load(const Tile&, int kb, uint8_t* a, uint8_t* b, uint64_t* bar)
 //   void load_a(...a, bar) / load_b(...b, bar)     the two halves of load(); int res_kb (0: B not resident)
 //   void store_panel(const Tile&, int panel, const void* smem)   TMA store of a 128x64 bf16 panel
-//   bool row_valid(const Tile&, int row)           row is a real output (statistics mask)
+//   static constexpr bool kTwoPanels               residual panels in buffers of their own (kBn kernels)
 //   void load_res_panel(const Tile&, int panel, void* smem, uint64_t* bar)   TMA load of the residual's panel
 //   static constexpr bool kHalo; int out_row(int row)   row of the stored tile for a GEMM row (identity unless kHalo)
 //   kHalo only: int cblks, R, S, PW; void load_halo(const Tile&, int cb, void* smem, uint64_t* bar)
-//   int valid_prefix(const Tile&)                  n if exactly rows [0, n) are real outputs, -1 if irregular
+//   int valid_prefix(const Tile&)                  rows [0, n) of the stored tile are real outputs
+//   int64_t first_row(const Tile&)                 row 0 of the tile in the dense output matrix; the others follow
 //   void store_f32(const Tile&, int col, const void* smem, bool add)   TMA store / reduction of 128 x 32 fp32 columns
-template <class P>
+// kBn: the batch-norm part of the epilogue (bn_y and so on); a kernel of its own, because its registers cost the others
+// a tenth of their speed.
+template <class P, bool kBn = false>
 __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   constexpr int BN = P::BN;
   using C = Cfg<BN>;
@@ -225,14 +254,18 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int res_kb = prob.res_kb;            // > 0: B-resident mode
   constexpr bool kHalo = P::kHalo;
+  // The residual's panels land in buffers of their own (four stages' worth of shared memory), so that the next one travels
+  // while this one is stored and its sums are taken: 340 -> 260 us for 802816 x 256 x 64.
+  const bool two_panels = kBn && P::kTwoPanels && ep.residual != nullptr;
+  const int area = two_panels ? C::STAGE_AREA2 : C::STAGE_AREA;
   const int nhalo = kHalo ? (res_kb > 0 ? 2 : MAX_HALOS) : 0;
   const int nstages = kHalo ? (res_kb > 0 ? 1 : min(C::MAX_STAGES, (C::STAGE_AREA - nhalo * HALO_BYTES) / C::B_STAGE_BYTES))
-                            : (res_kb > 0 ? min(C::MAX_STAGES, (C::STAGE_AREA - res_kb * C::B_STAGE_BYTES) / A_STAGE_BYTES)
-                                          : STAGES);
+                            : (res_kb > 0 ? min(C::MAX_STAGES, (area - res_kb * C::B_STAGE_BYTES) / A_STAGE_BYTES)
+                                          : min(STAGES, area / (A_STAGE_BYTES + C::B_STAGE_BYTES)));
   uint8_t* sA = smem;                        // halo mode: the input boxes
   uint8_t* sB = kHalo ? sA + nhalo * HALO_BYTES : sA + nstages * A_STAGE_BYTES;
-  uint8_t* sC = smem + C::STAGE_AREA;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sC + NUM_GROUPS * PANEL_BYTES);
+  uint8_t* sC = smem + area;                 // the groups' output panels, then their residual panels
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGE_AREA + NUM_GROUPS * PANEL_BYTES);
   uint64_t* empty = full + C::MAX_STAGES;
   uint64_t* tfull = empty + C::MAX_STAGES;
   uint64_t* tempty = tfull + C::ACCS;
@@ -421,6 +454,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     const int row = q * 32 + lane;          // tile row owned by this thread
     const int drow = prob.out_row(row);     // its row in the stored tile (halo mode: margin rows have none)
     uint8_t* panel = sC + grp * PANEL_BYTES;
+    uint8_t* rpanel = two_panels ? panel + NUM_GROUPS * PANEL_BYTES : panel;
     const bool leader = gt == 0;            // issues the group's copies
     const bool has_res = ep.residual != nullptr;
     const bool plain = ep.bias == nullptr && !ep.relu && !has_res;
@@ -435,22 +469,56 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
       typename P::Tile n;
       if (!leader || !prob.tile(it, n) || n.n0 + pnl * 64 >= ep.n_total) return;
       mbar_expect_tx(&rfull[grp], ep.res_bytes);
-      prob.load_res_panel(n, pnl, panel, &rfull[grp]);
+      prob.load_res_panel(n, pnl, rpanel, &rfull[grp]);
     };
+    // ... and the lines of bn_y that a unit will read go to L2 meanwhile, a row per thread.
+    auto prefetch_y = [&](int it) {
+      typename P::Tile n;
+      if (!prob.tile(it, n) || n.n0 + pnl * 64 >= ep.n_total || gt >= prob.valid_prefix(n)) return;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.bn_y + (prob.first_row(n) + gt) * ep.n_total + n.n0 + pnl * 64));
+    };
+    uint64_t neg_mean = 0;
+    if (kBn && prob.tile(0, t) && t.n0 + pnl * 64 < ep.n_total) {      // a CTA's tiles share their columns
+      const float2 m = __ldg(reinterpret_cast<const float2*>(ep.bn_aux + t.n0 + pnl * 64) + cp);
+      neg_mean = pack_f32x2(__float_as_uint(-m.x), __float_as_uint(-m.y));
+      prefetch_y(turn);
+    }
     if (has_res) fetch_residual(turn);
     for (int it = turn; prob.tile(it, t); it += TURNS) {
       const int acc = it % C::ACCS;
+      // bn: the mask of this thread's row, and of bn_y this thread's column pair of rows 32rg .. +15 (later +16 .. +31), asked
+      // for before the waits
+      uint32_t ya[kBn ? 16 : 1];
+      uint2 keep = make_uint2(0xffffffffu, 0xffffffffu);
+      const uint32_t* ysrc = nullptr;
+      auto load_y = [&](uint32_t (&v)[kBn ? 16 : 1], int r0) {
+        const int rows = prob.valid_prefix(t) - rg * 32 - r0;
+#pragma unroll
+        for (int rr = 0; rr < (kBn ? 16 : 1); ++rr) v[rr] = rr < rows ? __ldg(ysrc + (size_t)(r0 + rr) * (ep.n_total >> 1)) : 0u;
+      };
+      if (kBn && t.n0 + pnl * 64 < ep.n_total) {
+        const int64_t row0 = prob.first_row(t);
+        const int c0 = t.n0 + pnl * 64;
+        if (ep.bn_mask != nullptr && drow >= 0 && drow < prob.valid_prefix(t))
+          keep = __ldg(reinterpret_cast<const uint2*>(ep.bn_mask + ((row0 + drow) * ep.n_total + c0) / 8));
+        ysrc = reinterpret_cast<const uint32_t*>(ep.bn_y + (row0 + rg * 32) * ep.n_total + c0) + cp;
+        load_y(ya, 0);
+      }
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&tfull[acc], (uint32_t)(it / C::ACCS) & 1u, abort_flag));
       tc_fence_after();
       const int col0 = t.n0 + pnl * 64;
+      if (kBn) prefetch_y(it + TURNS);
       if (col0 < ep.n_total) {              // uniform across the group
+        const int prefix = prob.valid_prefix(t);              // rows [0, prefix) are real outputs
+        const int yrows = min(32, max(0, prefix - rg * 32));
         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + pnl * 64);
         uint32_t r[32];                       // 32 columns at a time: two halves would not fit 96 registers beside the rest
         tmem_ld_32x32b_x32(t_row, r);
         if (has_res) {
           ok = __all_sync(0xffffffffu, ok && mbar_wait(&rfull[grp], res_phase, abort_flag));
           res_phase ^= 1u;
-        } else {
+        }
+        if (!has_res || two_panels) {
           if (leader) tma_store_wait_read<0>();               // the group's previous panel has left the buffer
           named_barrier_sync(1 + grp, GROUP_THREADS);
         }
@@ -462,52 +530,61 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           __syncwarp();
           if (lane == 0) mbar_arrive(&tempty[acc]);
         };
-        if (ep.out_mode == OUT_BF16) {
-          if (plain) {
-            if (drow >= 0) pack_row_to_panel<true>(r, panel, drow, 0, col0, ep, false);
+        if (kBn || ep.out_mode == OUT_BF16) {
+          if (!kBn && plain) {
+            if (drow >= 0) pack_row_to_panel<PACK_PLAIN>(r, panel, rpanel, drow, 0, col0, ep, false);
             next_half();
-            if (drow >= 0) pack_row_to_panel<true>(r, panel, drow, 1, col0 + 32, ep, false);
+            if (drow >= 0) pack_row_to_panel<PACK_PLAIN>(r, panel, rpanel, drow, 1, col0 + 32, ep, false);
+          } else if (!kBn) {
+            if (drow >= 0) pack_row_to_panel<PACK_AFFINE>(r, panel, rpanel, drow, 0, col0, ep, has_res);
+            next_half();
+            if (drow >= 0) pack_row_to_panel<PACK_AFFINE>(r, panel, rpanel, drow, 1, col0 + 32, ep, has_res);
           } else {
-            if (drow >= 0) pack_row_to_panel<false>(r, panel, drow, 0, col0, ep, has_res);
+            if (drow >= 0) pack_row_to_panel<PACK_MASKED>(r, panel, rpanel, drow, 0, col0, ep, has_res, keep.x);
             next_half();
-            if (drow >= 0) pack_row_to_panel<false>(r, panel, drow, 1, col0 + 32, ep, has_res);
+            if (drow >= 0) pack_row_to_panel<PACK_MASKED>(r, panel, rpanel, drow, 1, col0 + 32, ep, has_res, keep.y);
           }
           fence_proxy_async();
           named_barrier_sync(1 + grp, GROUP_THREADS);         // the panel is complete and visible to the TMA engine
           if (leader) {
             prob.store_panel(t, pnl, panel);
             tma_store_commit();
+            if (two_panels) fetch_residual(it + TURNS);        // everybody has read this one
           }
-          if (ep.col_sum != nullptr) {
-            const int prefix = prob.valid_prefix(t);          // rows [0, prefix) are the real outputs, or -1
-            uint32_t mask = 0xffffffffu;                      // this thread's 32 rows
-            if (prefix >= 0) {
-              const int mine = min(32, max(0, prefix - rg * 32));
-              mask = mine >= 32 ? 0xffffffffu : (1u << mine) - 1u;
-            } else {
-              mask = 0u;
-              for (int rr = 0; rr < 32; ++rr)
-                if (prob.row_valid(t, rg * 32 + rr)) mask |= 1u << rr;
-            }
+          if (kBn || ep.col_sum != nullptr) {
             const uint8_t* colp = panel + rg * 32 * 128 + (cp & 3) * 4;
             const int chunk = cp >> 2;
             uint64_t s = 0, sq = 0;
-            if (__all_sync(0xffffffffu, mask == 0xffffffffu)) {
+            if (kBn) {
+              // dbeta and dgamma: y comes from L2 (the previous unit asked for it), coalesced over the panel's columns
+              uint32_t yb[kBn ? 16 : 1];
+              load_y(yb, 16);
+#pragma unroll
+              for (int rr = 0; rr < 32; ++rr) {
+                uint32_t w = *reinterpret_cast<const uint32_t*>(colp + rr * 128 + ((chunk ^ (rr & 7)) << 4));
+                if (rr >= yrows) w = 0u;
+                const uint64_t f = bf16x2_to_f32x2(w);
+                uint64_t d = bf16x2_to_f32x2(rr < 16 ? ya[kBn ? rr & 15 : 0] : yb[kBn ? rr & 15 : 0]);
+                add_f32x2(d, neg_mean);
+                add_f32x2(s, f);
+                fma_f32x2(sq, f, d);
+              }
+            } else if (yrows == 32) {
 #pragma unroll 16
               for (int rr = 0; rr < 32; ++rr) {
                 const uint32_t w = *reinterpret_cast<const uint32_t*>(colp + rr * 128 + ((chunk ^ (rr & 7)) << 4));
-                const uint64_t f = pack_f32x2(w << 16, w & 0xffff0000u);
+                const uint64_t f = bf16x2_to_f32x2(w);
                 add_f32x2(s, f);
-                fma_f32x2(sq, f);
+                fma_f32x2(sq, f, f);
               }
             } else {
 #pragma unroll 8
               for (int rr = 0; rr < 32; ++rr) {
                 uint32_t w = *reinterpret_cast<const uint32_t*>(colp + rr * 128 + ((chunk ^ (rr & 7)) << 4));
-                if (!((mask >> rr) & 1u)) w = 0u;             // rows outside the tensor count as zeros
-                const uint64_t f = pack_f32x2(w << 16, w & 0xffff0000u);
+                if (rr >= yrows) w = 0u;                      // rows outside the tensor count as zeros
+                const uint64_t f = bf16x2_to_f32x2(w);
                 add_f32x2(s, f);
-                fma_f32x2(sq, f);
+                fma_f32x2(sq, f, f);
               }
             }
             add_f32x2(st_sum, s);
@@ -536,7 +613,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
             }
           }
         }
-        if (has_res) {
+        if (has_res && !two_panels) {
           named_barrier_sync(1 + grp, GROUP_THREADS);         // the statistics are done with the panel, too
           if (leader) {
             tma_store_wait_read<0>();
@@ -568,7 +645,8 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
       atomicAdd(mine + BN + 1, sq.y);
       named_barrier_sync(1 + NUM_GROUPS, NUM_GROUPS * GROUP_THREADS);
       const int c = tid % BN, col = t.n0 + c;
-      if (tid < 2 * BN && col < ep.n_total) atomicAdd((tid < BN ? ep.col_sum : ep.col_sqsum) + col, sums[tid]);
+      if (tid < 2 * BN && col < ep.n_total)
+        atomicAdd((tid < BN ? ep.col_sum : ep.col_sqsum) + col, kBn && tid >= BN ? sums[tid] * __ldg(ep.bn_aux + ep.n_total + col) : sums[tid]);
     }
     if (leader) tma_store_wait_all();                // shared memory must outlive the bulk stores
   }

@@ -9,6 +9,7 @@
 // straight to fp32 accumulators of the optimizer's flat buckets and tells the bucket so, instead of handing autograd a
 // bf16 tensor that is cast, added to a zeroed .grad and cast again: three small kernels and a Python hook fewer per tensor.
 #include <torch/extension.h>
+#include "../cuda/bn_grad.h"
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <atomic>
@@ -23,8 +24,10 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
 int esgd_conv2d_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int R, int S, int stride,
                     int pad, const float* scale, const float* bias, const void* residual, int relu, float* col_sum,
                     float* col_sqsum, int* error_flag, void* stream);
+int esgd_gemm_bn_dgrad(const void* dy, const void* w, void* dx, int M, int N, int K, const void* residual, const esgd_bn_grad* bn,
+                       int* error_flag, void* stream);
 int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, int R, int S, int stride,
-                      int pad, const void* residual, int* error_flag, void* stream);
+                      int pad, const void* residual, const esgd_bn_grad* bn, int* error_flag, void* stream);
 int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
                       int stride, int pad, int* error_flag, void* stream);
 int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
@@ -32,7 +35,7 @@ int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int 
 int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, int W, int Cin, int Cout, int stride, const float* scale,
                          const float* shift, const void* residual, int relu, float* sum, float* sqsum, void* stream);
 int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, const void* residual,
-                           void* stream);
+                           const esgd_bn_grad* bn, void* stream);
 int esgd_conv_narrow_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int stride, void* stream);
 int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, int R, int S, int stride, int pad, int seg,
                         int Kpad, void* stream);
@@ -48,7 +51,7 @@ int esgd_bn_coefficients(const void* layers, int n, float eps, void* stream);
 int esgd_bn_bwd_reduce(const void* dz, const void* mask, const void* y, const float* aux, int64_t M, int C, int mode, float* dbeta,
                        float* dgamma, void* stream);
 int esgd_bn_bwd_apply(const void* dz, const void* mask, const void* y, const float* aux, const float* gamma, const float* dbeta,
-                      const float* dgamma, void* dy, void* dres, int64_t M, int C, int mode, float* acc_dgamma, float* acc_dbeta,
+                      const float* dgamma, void* dy, void* dres, int64_t M, int C, int mode, int last_first, float* acc_dgamma, float* acc_dbeta,
                       void* stream);
 int esgd_softmax_ce(const void* logits, int is_bf16, const int64_t* labels, int batch, int classes, int ld, float grad_scale,
                     float* loss_sum, float* per_sample, void* dlogits, void* stream);
@@ -294,6 +297,38 @@ struct StemGeometry {
   }
 };
 
+// A batch norm whose output a convolution reads: the convolution's data gradient then leaves the gradient with the ReLU's
+// mask applied and the two sums over it (bn_grad.h), and the batch norm's backward has one pass to do instead of two.
+//
+// Only inside a training step of this package (parameters with sinks), and only where nobody can tell a gradient whose masked
+// elements are already zero: no hooks on the tensor, no gradient captured on the way.  The sums count when the very tensor
+// that the data gradient wrote arrives, untouched; a sum with another consumer's gradient is another tensor, and goes
+// through the mask and the reduction again.
+struct BnRecord : torch::CustomClassHolder {
+  Tensor y, mask, aux;
+  std::weak_ptr<torch::autograd::Node> node;
+  Tensor dz, sums;               // left by the data gradient
+  uint32_t version = 0;
+
+  bool observed() const {
+    const auto n = node.lock();
+    if (!n || !n->tensor_pre_hooks().empty() || !n->pre_hooks().empty() || !n->retains_grad_hooks().empty()) return true;
+    const auto* captures = torch::autograd::get_current_graph_task_exec_info();
+    return captures != nullptr && !captures->empty();
+  }
+  void fill(esgd_bn_grad* g, const Tensor& dx) {
+    const int64_t c = dx.size(1);
+    sums = zeros_f32({2, c}, dx.device());
+    *g = esgd_bn_grad{y.data_ptr(), mask.defined() ? mask.data_ptr() : nullptr, fptr(aux), fptr(sums)};
+  }
+  void written(const Tensor& dx) {
+    dz = dx;
+    version = dx._version();
+  }
+};
+using BnRef = c10::intrusive_ptr<BnRecord>;
+BnRef bn_behind(const Tensor& x);     // the record of the batch norm that produced x, or null
+
 // What a convolution's epilogue does to the product: statistics of it (training), or the affine map of an inference batch
 // norm, a residual and a ReLU.
 struct ConvEpilogue {
@@ -348,7 +383,7 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
 // data-gradient GEMM, instead of autograd summing the two branches of x with a separate pass over the tensor.
 struct ConvFn : public Function<ConvFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w, int64_t kind, int64_t stride, int64_t pad,
-                               bool want_stats, bool tap, const Sink& sink, const c10::optional<Tensor>& anchor) {
+                               bool want_stats, bool tap, const Sink& sink, const c10::optional<Tensor>& anchor, const BnRef& bn) {
     c10::cuda::CUDAGuard guard(x_in.device());
     Tensor x = nhwc(x_in);
     const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3);
@@ -367,6 +402,7 @@ struct ConvFn : public Function<ConvFn> {
     ctx->save_for_backward({saved_x, wk});
     ctx->saved_data["cfg"] = std::vector<int64_t>{kind, stride, pad, n, cin, h, wd, want_stats, tap};
     save_sink(ctx, "w", sink);
+    if (bn) ctx->saved_data["bn"] = c10::IValue::make_capsule(bn);
     ctx->set_materialize_grads(false);                // an unused tap must not cost a tensor of zeros
     variable_list out{y};
     if (want_stats) {
@@ -381,7 +417,7 @@ struct ConvFn : public Function<ConvFn> {
     const auto cfg = ctx->saved_data["cfg"].toIntVector();
     const int64_t kind = cfg[0], stride = cfg[1], pad = cfg[2], n = cfg[3], cin = cfg[4], h = cfg[5], wd = cfg[6];
     const bool want_stats = cfg[7], tap = cfg[8];
-    variable_list none(9);
+    variable_list none(10);
     Tensor d_tap = tap ? grads[want_stats ? 2 : 1] : Tensor();   // gradient that reached the input through the shortcut
     Sink sink = load_sink(ctx, "w");
     if (!grads[0].defined()) {
@@ -397,50 +433,14 @@ struct ConvFn : public Function<ConvFn> {
     void* st = stream_of(x);
     Tensor dx, dw;
     const bool need_dx = ctx->needs_input_grad(0), need_dw = sink || ctx->needs_input_grad(1);
-    if (need_dx && kind == kOneByOne) {
-      Tensor res;
-      if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
-      dx = empty_nhwc(n, cin, ho, wo, x);
-      ck(gemm(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), m, cin, cout, cout, cin, cin, false, true, 0, 1, nullptr, nullptr,
-              res.defined() ? res.data_ptr() : nullptr, cin, x), "1x1 convolution data gradient");
-      if (stride == 2) {
-        Tensor full = empty_nhwc(n, cin, h, wd, x);
-        ck(esgd_subsample2_bwd(dx.data_ptr(), full.data_ptr(), n, h, wd, cin, st), "subsample backward");
-        dx = full;
-      }
-    } else if (need_dx && kind == kGeneral) {
-      const bool square = r == s && pad <= r - 1;
-      dx = empty_nhwc(n, cin, h, wd, x);
-      if (square && stride == 1) {
-        Tensor res;
-        if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
-        const void* rp = res.defined() ? res.data_ptr() : nullptr;
-        int rc = kNotTaken;
-        if (r == 3 && pad == 1)
-          rc = esgd_conv_narrow_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, rp, st);
-        if (rc == kNotTaken)
-          rc = esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, rp, flag_ptr(x), st);
-        ck(rc, "conv2d data gradient");
-        d_tap = Tensor();
-      } else if (stride == 2 && r == 3 && s == 3 && pad == 1 && h % 2 == 0 && wd % 2 == 0) {
-        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, 3, 3, 2, 1, nullptr, flag_ptr(x), st),
-           "strided conv2d data gradient");
-      } else if (square) {
-        // Any other stride / size: the gradient is spread out with (stride - 1) zeros between its pixels (plus the rows and
-        // columns at the far edge that no window reached) and then goes through the stride-1 form above.
-        const int64_t eh = (h + 2 * pad - r) % stride, ew = (wd + 2 * pad - s) % stride;
-        Tensor spread = at::zeros({n, cout, (ho - 1) * stride + 1 + eh, (wo - 1) * stride + 1 + ew}, dy.options()).contiguous(kCL);
-        spread.slice(2, 0, (ho - 1) * stride + 1, stride).slice(3, 0, (wo - 1) * stride + 1, stride).copy_(dy);
-        ck(esgd_conv2d_dgrad(spread.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, nullptr, flag_ptr(x), st),
-           "conv2d data gradient");
-      } else {
-        dx = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {stride, stride}, {pad, pad}, {1, 1}, false, {0, 0}, 1,
-                                                  {true, false, false}));
-      }
-      if (d_tap.defined()) dx = dx + d_tap;
-    } else if (need_dx) {
-      dx = d_tap;
+    BnRef bn;
+    if (const auto it = ctx->saved_data.find("bn"); sink && it != ctx->saved_data.end()) {
+      bn = c10::static_intrusive_pointer_cast<BnRecord>(it->second.toCapsule());
+      if (!bn->y.defined() || bn->observed()) bn = BnRef();
     }
+    esgd_bn_grad bg;
+    // The weight gradient goes first: what the data gradient leaves (and the batch norm's pass behind it reads) is then the
+    // newest in L2.
     if (need_dw) {
       if (kind == kOneByOne) {
         Tensor dw32;
@@ -470,8 +470,68 @@ struct ConvFn : public Function<ConvFn> {
         ck(esgd_stem_unpack(fptr(col), sink ? nullptr : dw.data_ptr(), sink ? sink->acc : nullptr, cout, r, s * cin, g.seg, g.kpad,
                             st), "stem filter gradient");
       }
-      if (sink) sink_done(sink);
     }
+    if (need_dx && kind == kOneByOne) {
+      Tensor res;
+      if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
+      dx = empty_nhwc(n, cin, ho, wo, x);
+      int rc = kNotTaken;
+      if (bn) {
+        bn->fill(&bg, dx);
+        rc = esgd_gemm_bn_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), m, cin, cout, res.defined() ? res.data_ptr() : nullptr, &bg,
+                                flag_ptr(x), st);
+        if (rc == 0) bn->written(dx);
+      }
+      if (rc == kNotTaken)
+        rc = gemm(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), m, cin, cout, cout, cin, cin, false, true, 0, 1, nullptr, nullptr,
+                  res.defined() ? res.data_ptr() : nullptr, cin, x);
+      ck(rc, "1x1 convolution data gradient");
+      if (stride == 2) {
+        Tensor full = empty_nhwc(n, cin, h, wd, x);
+        ck(esgd_subsample2_bwd(dx.data_ptr(), full.data_ptr(), n, h, wd, cin, st), "subsample backward");
+        dx = full;
+      }
+    } else if (need_dx && kind == kGeneral) {
+      const bool square = r == s && pad <= r - 1;
+      dx = empty_nhwc(n, cin, h, wd, x);
+      if (square && stride == 1) {
+        Tensor res;
+        if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
+        const void* rp = res.defined() ? res.data_ptr() : nullptr;
+        if (bn) bn->fill(&bg, dx);
+        auto launch = [&](const esgd_bn_grad* g) {
+          int rc = kNotTaken;
+          if (r == 3 && pad == 1)
+            rc = esgd_conv_narrow_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, rp, g, st);
+          if (rc == kNotTaken)
+            rc = esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, rp, g, flag_ptr(x), st);
+          return rc;
+        };
+        int rc = launch(bn ? &bg : nullptr);
+        if (bn && rc == 0) bn->written(dx);
+        if (bn && rc == kNotTaken) rc = launch(nullptr);
+        ck(rc, "conv2d data gradient");
+        d_tap = Tensor();
+      } else if (stride == 2 && r == 3 && s == 3 && pad == 1 && h % 2 == 0 && wd % 2 == 0) {
+        ck(esgd_conv2d_dgrad(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, 3, 3, 2, 1, nullptr, nullptr, flag_ptr(x), st),
+           "strided conv2d data gradient");
+      } else if (square) {
+        // Any other stride / size: the gradient is spread out with (stride - 1) zeros between its pixels (plus the rows and
+        // columns at the far edge that no window reached) and then goes through the stride-1 form above.
+        const int64_t eh = (h + 2 * pad - r) % stride, ew = (wd + 2 * pad - s) % stride;
+        Tensor spread = at::zeros({n, cout, (ho - 1) * stride + 1 + eh, (wo - 1) * stride + 1 + ew}, dy.options()).contiguous(kCL);
+        spread.slice(2, 0, (ho - 1) * stride + 1, stride).slice(3, 0, (wo - 1) * stride + 1, stride).copy_(dy);
+        ck(esgd_conv2d_dgrad(spread.data_ptr(), w.data_ptr(), dx.data_ptr(), n, h, wd, cin, cout, r, s, 1, pad, nullptr, nullptr, flag_ptr(x),
+                             st), "conv2d data gradient");
+      } else {
+        dx = std::get<0>(at::convolution_backward(dy, x, w, c10::nullopt, {stride, stride}, {pad, pad}, {1, 1}, false, {0, 0}, 1,
+                                                  {true, false, false}));
+      }
+      if (d_tap.defined()) dx = dx + d_tap;
+    } else if (need_dx) {
+      dx = d_tap;
+    }
+    if (need_dw && sink) sink_done(sink);
     none[0] = dx;
     none[1] = dw;
     return none;
@@ -495,7 +555,8 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
   const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
   Sink sink = find_sink(w);
   sink_use(sink);
-  variable_list out = ConvFn::apply(x, graph_input(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink));
+  variable_list out = ConvFn::apply(x, graph_input(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink),
+                                    sink && stride == 1 ? bn_behind(x) : BnRef());
   py::object st = want_stats ? py::cast(out[1]) : py::none();
   py::object tp = !tap ? py::none() : py::cast(fuse_tap ? out.back() : x);
   return py::make_tuple(out[0], st, tp);
@@ -648,7 +709,8 @@ struct BnActFn : public Function<BnActFn> {
     Tensor aux = at::empty({4, c}, gamma.options());       // mean, invstd, scale, shift
     Tensor z = empty_nhwc(n, c, y.size(2), y.size(3), y);
     // ReLU mask of the backward pass: a bit per element where a residual was added, else recomputed from y
-    const int64_t mode = !relu ? 0 : (res.defined() ? 1 : 2);
+    // (a bit as well where a convolution's data gradient may have to apply it)
+    const int64_t mode = !relu ? 0 : (res.defined() || (gs && bs) ? 1 : 2);
     Tensor mask;
     if (mode == 1) mask = at::empty({m, c / 8}, y.options().dtype(at::kByte));
     ck(esgd_bn_fwd(y.data_ptr(), res.defined() ? res.data_ptr() : nullptr, z.data_ptr(), mode == 1 ? mask.data_ptr() : nullptr,
@@ -659,26 +721,49 @@ struct BnActFn : public Function<BnActFn> {
     ctx->saved_data["res"] = res.defined();
     save_sink(ctx, "g", gs);
     save_sink(ctx, "b", bs);
+    if (gs && bs) {
+      auto rec = c10::make_intrusive<BnRecord>();
+      rec->y = y.detach();
+      rec->mask = mask;
+      rec->aux = aux;
+      ctx->saved_data["rec"] = c10::IValue::make_capsule(rec);
+    }
     return z;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &y = saved[0], &mask = saved[1], &gamma = saved[2], &aux = saved[3];
     c10::cuda::CUDAGuard guard(y.device());
-    const int64_t mode = ctx->saved_data["mode"].toInt(), c = y.size(1), m = y.numel() / c;
+    int64_t mode = ctx->saved_data["mode"].toInt();
+    const int64_t c = y.size(1), m = y.numel() / c;
     const bool has_res = ctx->saved_data["res"].toBool();
     Sink gs = load_sink(ctx, "g"), bs = load_sink(ctx, "b");
     Tensor dz = nhwc(grads[0]);
     void* st = stream_of(y);
-    // dbeta, dgamma; handed to autograd unless both go to sinks, so then not from the step's scratch
-    Tensor red = gs && bs ? zeros_f32({2, c}, y.device()) : at::zeros({2, c}, aux.options());
-    float* rd = fptr(red);
     const void* mp = mask.defined() ? mask.data_ptr() : nullptr;
-    ck(esgd_bn_bwd_reduce(dz.data_ptr(), mp, y.data_ptr(), fptr(aux), m, c, (int)mode, rd, rd + c, st), "bn_bwd_reduce");
-    Tensor dy = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y), dres;
-    if (has_res) dres = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y);
+    Tensor red, dres;
+    BnRef rec;
+    if (const auto it = ctx->saved_data.find("rec"); it != ctx->saved_data.end())
+      rec = c10::static_intrusive_pointer_cast<BnRecord>(it->second.toCapsule());
+    const bool fused = gs && bs && rec && rec->dz.defined() && rec->dz.is_same(dz) && rec->version == dz._version();
+    if (fused) {
+      red = rec->sums;             // dz is masked, its sums are there, and it is the shortcut's gradient as it stands
+      mode = 0;
+      if (has_res) dres = dz;
+    } else {
+      // dbeta, dgamma; handed to autograd unless both go to sinks, so then not from the step's scratch
+      red = gs && bs ? zeros_f32({2, c}, y.device()) : at::zeros({2, c}, aux.options());
+      ck(esgd_bn_bwd_reduce(dz.data_ptr(), mp, y.data_ptr(), fptr(aux), m, c, (int)mode, fptr(red), fptr(red) + c, st), "bn_bwd_reduce");
+    }
+    if (rec) {
+      rec->y = rec->mask = rec->dz = rec->sums = Tensor();
+    }
+    float* rd = fptr(red);
+    Tensor dy = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y);
+    const bool write_res = has_res && !dres.defined();
+    if (write_res) dres = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y);
     ck(esgd_bn_bwd_apply(dz.data_ptr(), mp, y.data_ptr(), fptr(aux), fptr(gamma), rd, rd + c, dy.data_ptr(),
-                         has_res ? dres.data_ptr() : nullptr, m, c, (int)mode, gs ? gs->acc : nullptr, bs ? bs->acc : nullptr, st),
+                         write_res ? dres.data_ptr() : nullptr, m, c, (int)mode, fused, gs ? gs->acc : nullptr, bs ? bs->acc : nullptr, st),
        "bn_bwd_apply");
     Tensor dgamma, dbeta;
     if (gs) sink_done(gs);
@@ -697,8 +782,21 @@ Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c1
   Sink gs = find_sink(gamma), bs = find_sink(beta);
   sink_use(gs);
   sink_use(bs);
-  return BnActFn::apply(y, graph_input(gamma, gs), graph_input(beta, bs), res, rm, rv, momentum, relu, stats, gs, bs,
-                        anchor_for(y, gs || bs));
+  Tensor z = BnActFn::apply(y, graph_input(gamma, gs), graph_input(beta, bs), res, rm, rv, momentum, relu, stats, gs, bs,
+                            anchor_for(y, gs || bs));
+  if (gs && bs) {
+    auto* node = static_cast<torch::autograd::CppNode<BnActFn>*>(z.grad_fn().get());
+    c10::static_intrusive_pointer_cast<BnRecord>(node->ctx_.saved_data.at("rec").toCapsule())->node = z.grad_fn();
+  }
+  return z;
+}
+
+BnRef bn_behind(const Tensor& x) {
+  auto* node = dynamic_cast<torch::autograd::CppNode<BnActFn>*>(x.grad_fn().get());
+  if (node == nullptr || !x.is_contiguous(kCL)) return BnRef();
+  const auto it = node->ctx_.saved_data.find("rec");
+  if (it == node->ctx_.saved_data.end()) return BnRef();
+  return c10::static_intrusive_pointer_cast<BnRecord>(it->second.toCapsule());
 }
 
 // ---------------------------------------------------------------- softmax cross-entropy
