@@ -39,6 +39,15 @@ __device__ __forceinline__ uint8_t sign_bits(const uint4& w) {
   return (uint8_t)m;
 }
 
+// Blocks of a kernel that are resident on an SM, and the size of its grid.  With more of them every block beyond these starts
+// over with its coefficients and the last wave is partly empty; with more registers a thread instead (the backward apply pass
+// of two resident blocks) too few loads are in flight.  12544 x 2048 and 802816 x 256, 8 blocks an SM -> now: forward 31 -> 28
+// and 161 -> 147 us, with a residual 41 -> 37 and 213 -> 199, apply 49 -> 34.5 and 249 -> 212.
+constexpr int kStatsBlocks = 4;
+constexpr int fwd_blocks(bool res) { return res ? 2 : 3; }
+constexpr int reduce_blocks(int mode) { return mode == 2 ? 2 : 3; }
+constexpr int apply_blocks(int mode, bool res) { return mode == 0 && !res ? 3 : 2; }
+
 struct Map {
   int groups;      // C / 8
   int cg;          // channel groups of a block (a power of two)
@@ -70,7 +79,7 @@ __device__ __forceinline__ void flush_sums(const float (&a)[8], const float (&b)
   }
 }
 
-__global__ void __launch_bounds__(256) bn_stats_kernel(const __nv_bfloat16* __restrict__ y, int64_t M, int C, Map mp,
+__global__ void __launch_bounds__(256, kStatsBlocks) bn_stats_kernel(const __nv_bfloat16* __restrict__ y, int64_t M, int C, Map mp,
                                                        float* __restrict__ sum, float* __restrict__ sqsum) {
   pdl_enter();
   const int gl = threadIdx.x % mp.cg, rl = threadIdx.x / mp.cg, g = blockIdx.y * mp.cg + gl;
@@ -106,7 +115,7 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const __nv_bfloat16* __re
 // With a residual the sign of z cannot be told from y alone, and a convolution's data gradient has no y to tell it from: the
 // backward passes then read one bit per element (mask) instead of z, a sixteenth of the bytes.
 template <bool kRes>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, fwd_blocks(kRes))
 bn_fwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ res, __nv_bfloat16* __restrict__ z,
               uint8_t* __restrict__ mask, const float* __restrict__ sum, const float* __restrict__ sqsum,
               const float* __restrict__ gamma, const float* __restrict__ beta, float* running_mean, float* running_var,
@@ -192,7 +201,7 @@ __device__ __forceinline__ void masked(const uint4& rd, const uint4& ry, uint32_
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, reduce_blocks(kMode))
 bn_bwd_reduce_kernel(const __nv_bfloat16* __restrict__ dz, const uint8_t* __restrict__ mask, const __nv_bfloat16* __restrict__ y,
                      const float* __restrict__ aux, int64_t M, int C, Map mp, float* __restrict__ dbeta, float* __restrict__ dgamma) {
   pdl_enter();
@@ -244,7 +253,7 @@ bn_bwd_reduce_kernel(const __nv_bfloat16* __restrict__ dz, const uint8_t* __rest
 // dy = a*g + b*y + c per channel, with a = gamma*invstd, b = -gamma*invstd^2*dgamma/M,
 // c = gamma*invstd*(mean*invstd*dgamma - dbeta)/M held in registers.
 template <int kMode, bool kRes>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, apply_blocks(kMode, kRes))
 bn_bwd_apply_kernel(const __nv_bfloat16* __restrict__ dz, const uint8_t* __restrict__ mask, const __nv_bfloat16* __restrict__ y,
                     const float* __restrict__ aux, const float* __restrict__ gamma, const float* __restrict__ dbeta,
                     const float* __restrict__ dgamma, __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dres, int64_t M,
@@ -324,16 +333,14 @@ Map make_map(int C) {
   m.rows_par = 256 / m.cg;
   return m;
 }
-// Four rows per thread as long as that does not fill the machine, then up to `cap` blocks in all.
-dim3 grid_for(const Map& m, int64_t M, int64_t cap) {
+// Four rows per thread as long as that does not fill the machine, then as many blocks as are resident.
+dim3 grid_for(const Map& m, int64_t M, int blocks_per_sm) {
   const int64_t chunks = (m.groups + m.cg - 1) / m.cg;
-  int64_t rows = (M + m.rows_par * 4 - 1) / (m.rows_par * 4), most = cap / chunks;
+  int64_t rows = (M + m.rows_par * 4 - 1) / (m.rows_par * 4), most = 148 * blocks_per_sm / chunks;
   if (most < 1) most = 1;
   if (rows > most) rows = most;
   return dim3((unsigned)(rows < 1 ? 1 : rows), (unsigned)chunks);
 }
-// Reductions end with a shared-memory pass and atomics per block: few, long-running blocks.
-constexpr int64_t kReduceBlocks = 148 * 2, kApplyBlocks = 148 * 8;
 
 }  // namespace
 
@@ -343,7 +350,7 @@ extern "C" {
 int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, void* stream) {
   if (C % 8) return -1;
   const Map mp = make_map(C);
-  return esgd::launch(bn_stats_kernel, grid_for(mp, M, kReduceBlocks), 256, 0, stream, (const __nv_bfloat16*)y, M, C, mp, sum, sqsum);
+  return esgd::launch(bn_stats_kernel, grid_for(mp, M, kStatsBlocks), 256, 0, stream, (const __nv_bfloat16*)y, M, C, mp, sum, sqsum);
 }
 
 // sum / sqsum: the batch sums of y.  aux [4][C] receives mean, inverse standard deviation, scale and shift; mask (optional,
@@ -355,7 +362,7 @@ int esgd_bn_fwd(const void* y, const void* residual, void* z, void* mask, const 
   const float unbias = M > 1 ? (float)M / (float)(M - 1) : 1.0f;
   const Map mp = make_map(C);
   auto kernel = residual != nullptr ? bn_fwd_kernel<true> : bn_fwd_kernel<false>;
-  return esgd::launch(kernel, grid_for(mp, M, kApplyBlocks), 256, 0, stream, (const __nv_bfloat16*)y, (const __nv_bfloat16*)residual,
+  return esgd::launch(kernel, grid_for(mp, M, fwd_blocks(residual != nullptr)), 256, 0, stream, (const __nv_bfloat16*)y, (const __nv_bfloat16*)residual,
                       (__nv_bfloat16*)z, (uint8_t*)mask, sum, sqsum, gamma, beta, running_mean, running_var, aux, M, C, mp, relu,
                       1.0f / (float)M, unbias, momentum, eps);
 }
@@ -372,7 +379,7 @@ int esgd_bn_bwd_reduce(const void* dz, const void* mask, const void* y, const fl
   if (C % 8 || mode < 0 || mode > 2 || (mode == 1 && mask == nullptr)) return -1;
   const Map mp = make_map(C);
   auto kernel = mode == 0 ? bn_bwd_reduce_kernel<0> : (mode == 1 ? bn_bwd_reduce_kernel<1> : bn_bwd_reduce_kernel<2>);
-  return esgd::launch(kernel, grid_for(mp, M, kReduceBlocks), 256, 0, stream, (const __nv_bfloat16*)dz, (const uint8_t*)mask,
+  return esgd::launch(kernel, grid_for(mp, M, reduce_blocks(mode)), 256, 0, stream, (const __nv_bfloat16*)dz, (const uint8_t*)mask,
                       (const __nv_bfloat16*)y, aux, M, C, mp, dbeta, dgamma);
 }
 
@@ -385,7 +392,7 @@ int esgd_bn_bwd_apply(const void* dz, const void* mask, const void* y, const flo
   const Map mp = make_map(C);
   auto kernel = dres != nullptr ? (mode == 0 ? bn_bwd_apply_kernel<0, true> : mode == 1 ? bn_bwd_apply_kernel<1, true> : bn_bwd_apply_kernel<2, true>)
                                 : (mode == 0 ? bn_bwd_apply_kernel<0, false> : mode == 1 ? bn_bwd_apply_kernel<1, false> : bn_bwd_apply_kernel<2, false>);
-  return esgd::launch(kernel, grid_for(mp, M, kApplyBlocks), 256, 0, stream, (const __nv_bfloat16*)dz, (const uint8_t*)mask,
+  return esgd::launch(kernel, grid_for(mp, M, apply_blocks(mode, dres != nullptr)), 256, 0, stream, (const __nv_bfloat16*)dz, (const uint8_t*)mask,
                       (const __nv_bfloat16*)y, aux, gamma, dbeta, dgamma, (__nv_bfloat16*)dy, (__nv_bfloat16*)dres, M, C, mp,
                       1.0f / (float)M, acc_dgamma, acc_dbeta, last_first);
 }
