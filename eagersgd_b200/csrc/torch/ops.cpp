@@ -180,7 +180,13 @@ class GradSinks {
  public:
   GradSinks(std::vector<int> params_per_bucket, py::function on_bucket)
       : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), on_bucket_(std::move(on_bucket)) {}
-  ~GradSinks() { close(); }
+  ~GradSinks() {
+    close();
+    if (side_) {
+      cudaEventDestroy(forked_);
+      cudaEventDestroy(joined_);
+    }
+  }
   void close() {
     std::unique_lock<std::shared_mutex> g(g_sink_mutex);
     for (auto& kv : mine_) { kv.second->owner.store(nullptr); g_sinks.erase(kv.first); }
@@ -200,7 +206,34 @@ class GradSinks {
     pending_ = total_;
     for (auto& kv : mine_) { kv.second->uses = 0; kv.second->used = false; }
   }
-  void set_active(bool on) { active_.store(on); }
+  void set_active(bool on) {
+    if (!on) join();
+    active_.store(on);
+  }
+  // Weight gradients of a step that is being captured go to a stream of their own: nothing waits for them before the bucket
+  // is complete, and in a small network neither they nor the chain of the other gradients fills the GPU.  (Outside a capture
+  // the events would cost the host what the GPU saves.)  Their operands are kept until the streams have met again.
+  c10::cuda::CUDAStream fork(const Tensor& a, const Tensor& b) {
+    const auto main = c10::cuda::getCurrentCUDAStream(a.get_device());
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(main.stream(), &status) != cudaSuccess || status != cudaStreamCaptureStatusActive) return main;
+    if (!side_) {
+      side_ = c10::cuda::getStreamFromPool(false, a.get_device());
+      C10_CUDA_CHECK(cudaEventCreateWithFlags(&forked_, cudaEventDisableTiming));
+      C10_CUDA_CHECK(cudaEventCreateWithFlags(&joined_, cudaEventDisableTiming));
+    }
+    C10_CUDA_CHECK(cudaEventRecord(forked_, main.stream()));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(side_->stream(), forked_, 0));
+    held_.push_back(a);
+    held_.push_back(b);
+    return *side_;
+  }
+  void join() {
+    if (held_.empty()) return;
+    C10_CUDA_CHECK(cudaEventRecord(joined_, side_->stream()));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(c10::cuda::getCurrentCUDAStream(side_->device_index()).stream(), joined_, 0));
+    held_.clear();
+  }
   bool active() const { return active_.load(); }
   bool used(const Tensor& param) const {
     auto it = mine_.find(param.unsafeGetTensorImpl());
@@ -211,6 +244,7 @@ class GradSinks {
   void mark_written(int bucket) { written_[bucket] = 1; }
   void param_done(int bucket) {
     if (--pending_[bucket] == 0) {
+      join();
       py::gil_scoped_acquire gil;
       on_bucket_(bucket);
     }
@@ -220,6 +254,9 @@ class GradSinks {
   std::vector<int> total_, pending_, written_;
   std::atomic<bool> active_{false};
   py::function on_bucket_;
+  c10::optional<c10::cuda::CUDAStream> side_;
+  cudaEvent_t forked_ = nullptr, joined_ = nullptr;
+  std::vector<Tensor> held_;
   std::unordered_map<at::TensorImpl*, Sink> mine_;
 };
 
@@ -442,6 +479,9 @@ struct ConvFn : public Function<ConvFn> {
     // The weight gradient goes first: what the data gradient leaves (and the batch norm's pass behind it reads) is then the
     // newest in L2.
     if (need_dw) {
+      c10::cuda::OptionalCUDAStreamGuard forked;
+      if (GradSinks* owner = sink && kind != kStem ? sink->owner.load() : nullptr) forked.reset_stream(owner->fork(dy, x));
+      void* st = stream_of(x);
       if (kind == kOneByOne) {
         Tensor dw32;
         if (!sink) dw32 = zeros_f32({cout, cin}, x.device());
