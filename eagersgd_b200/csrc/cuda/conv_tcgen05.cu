@@ -51,7 +51,7 @@ __device__ __forceinline__ void load_filter_tap(const CUtensorMap* tm, const Fil
 template <int BN_, bool kT>
 struct ConvProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kTwoPanels = false;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kTwoPanels = false, kPair = false;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, stride, pad;
@@ -122,7 +122,7 @@ struct ConvProblem {
 template <int BN_, bool kT>
 struct ConvHaloProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kTwoPanels = false;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kTwoPanels = false, kPair = false;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, pad;
@@ -181,7 +181,7 @@ struct ConvHaloProblem {
 template <int BN_>
 struct ConvWgradProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = true, B_MN = true, kZeroStages = true, kTwoPanels = false;
+  static constexpr bool A_MN = true, B_MN = true, kZeroStages = true, kTwoPanels = false, kPair = false;
   CUtensorMap tmDY, tmX, tmDW;
   int N, Ho, Wo, Cout, Cin;
   int R, S, stride, pad;

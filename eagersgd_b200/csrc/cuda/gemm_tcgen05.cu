@@ -18,10 +18,10 @@ using namespace umma;
 
 namespace {
 
-template <int BN_, bool A_MN_, bool B_MN_>
+template <int BN_, bool A_MN_, bool B_MN_, bool kPair_ = false>
 struct GemmProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false, kTwoPanels = true;
+  static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false, kTwoPanels = true, kPair = kPair_;
   CUtensorMap tmA, tmB, tmC, tmR;   // tmC: bf16 panels of 64 columns or fp32 ones of 32; tmR: optional residual
   int M, N, K;
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
@@ -32,20 +32,22 @@ struct GemmProblem {
   struct Tile { int kb0, kb1, n0, m0; };
 
   __device__ __forceinline__ bool tile(int it, Tile& t) const {
+    // a pair walks over tiles of 256 rows; m_tiles counts those
+    const int worker = kPair ? blockIdx.x / 2 : blockIdx.x, workers = kPair ? gridDim.x / 2 : gridDim.x;
     int m_idx, n_idx, split = 0;
     if (fixed_n) {
-      n_idx = blockIdx.x % n_tiles;
-      m_idx = blockIdx.x / n_tiles + it * (gridDim.x / n_tiles);
+      n_idx = worker % n_tiles;
+      m_idx = worker / n_tiles + it * (workers / n_tiles);
       if (m_idx >= m_tiles) return false;
     } else {
-      const int id = blockIdx.x + it * gridDim.x;
+      const int id = worker + it * workers;
       if (id >= m_tiles * n_tiles * splits) return false;
       split = id / (m_tiles * n_tiles);
       const int rem = id % (m_tiles * n_tiles);
       m_idx = rem / n_tiles;
       n_idx = rem % n_tiles;
     }
-    t.m0 = m_idx * BM;
+    t.m0 = kPair ? (2 * m_idx + (int)(blockIdx.x & 1)) * BM : m_idx * BM;
     t.n0 = n_idx * BN;
     t.kb0 = split * kb_per_split;
     t.kb1 = min(t.kb0 + kb_per_split, kb_total);
@@ -69,12 +71,28 @@ struct GemmProblem {
       tma_load_2d(b, &tmB, bar, k0, t.n0);
     }
   }
+  // pair: this CTA's rows of A and its half of the columns of B
+  __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint32_t leader_bar) const {
+    const int k0 = kb * BK, n0 = t.n0 + (int)(blockIdx.x & 1) * (BN / 2);
+    if (A_MN) {
+#pragma unroll
+      for (int i = 0; i < BM / 64; ++i) tma_load_2d_pair(a + i * 8192, &tmA, leader_bar, t.m0 + 64 * i, k0);
+    } else {
+      tma_load_2d_pair(a, &tmA, leader_bar, k0, t.m0);
+    }
+    if (B_MN) {
+#pragma unroll
+      for (int i = 0; i < BN / 128; ++i) tma_load_2d_pair(b + i * 8192, &tmB, leader_bar, n0 + 64 * i, k0);
+    } else {
+      tma_load_2d_pair(b, &tmB, leader_bar, k0, n0);
+    }
+  }
   __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint64_t* bar) const {
     load_a(t, kb, a, bar);
     load_b(t, kb, b, bar);
   }
   __device__ __forceinline__ void store_panel(const Tile& t, int panel, const void* smem) const {
-    tma_store_2d(&tmC, smem, t.n0 + panel * 64, t.m0);
+    if (!kPair || t.m0 < M) tma_store_2d(&tmC, smem, t.n0 + panel * 64, t.m0);
   }
   __device__ __forceinline__ int out_row(int row) const { return row; }
   __device__ __forceinline__ int valid_prefix(const Tile& t) const { return min(BM, M - t.m0); }
@@ -83,6 +101,7 @@ struct GemmProblem {
     tma_load_2d(smem, &tmR, bar, t.n0 + panel * 64, t.m0);
   }
   __device__ __forceinline__ void store_f32(const Tile& t, int col, const void* smem, bool add) const {
+    if (kPair && t.m0 >= M) return;              // the second half of the last tile
     if (add) tma_reduce_2d(&tmC, smem, col, t.m0);
     else tma_store_2d(&tmC, smem, col, t.m0);
   }
@@ -113,9 +132,9 @@ struct GemmArgs {
   int M, N, K, lda, ldb, ldc, out_mode, splits;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool kBn = false>
+template <int BN, bool A_MN, bool B_MN, bool kBn = false, bool kPair = false>
 int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
-  using P = GemmProblem<BN, A_MN, B_MN>;
+  using P = GemmProblem<BN, A_MN, B_MN, kPair>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -132,7 +151,7 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   int r = esgd::make_tensormap_bf16(&p.tmA, g.A, 2, dims, strides, box, nullptr);
   if (r != 0) return 1000 + r;
   if (B_MN) { dims[0] = (uint64_t)g.N; dims[1] = (uint64_t)g.K; box[0] = 64; box[1] = 64; }
-  else { dims[0] = (uint64_t)g.K; dims[1] = (uint64_t)g.N; box[0] = 64; box[1] = (uint32_t)BN; }
+  else { dims[0] = (uint64_t)g.K; dims[1] = (uint64_t)g.N; box[0] = 64; box[1] = (uint32_t)(kPair ? BN / 2 : BN); }
   strides[0] = (uint64_t)g.ldb * 2;
   r = esgd::make_tensormap_bf16(&p.tmB, g.B, 2, dims, strides, box, nullptr);
   if (r != 0) return 2000 + r;
@@ -155,7 +174,8 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
     if (r != 0) return 4000 + r;
   }
   p.M = g.M; p.N = g.N; p.K = g.K;
-  p.m_tiles = (g.M + BM - 1) / BM;
+  constexpr int kRows = kPair ? 2 * BM : BM;
+  p.m_tiles = (g.M + kRows - 1) / kRows;
   p.n_tiles = (g.N + BN - 1) / BN;
   p.kb_total = (g.K + BK - 1) / BK;
   int splits = g.splits < 1 ? 1 : g.splits;
@@ -165,11 +185,11 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   if (p.splits > 1 && g.out_mode != OUT_F32_ATOMIC) return -2;
   ep.res_bytes = PANEL_BYTES;
   const bool two_panels = kBn && ep.residual != nullptr;
-  const int sms = sm_count();
+  const int sms = kPair ? sm_count() / 2 : sm_count();         // workers: CTAs, or pairs of them
   int grid;
   // B stays in shared memory when its whole K extent fits beside four A stages and every CTA has several
   // tiles of one column range to amortise the load over
-  const bool resident = resident_enabled() && p.splits == 1 &&
+  const bool resident = !kPair && resident_enabled() && p.splits == 1 &&
                         p.kb_total <= (two_panels ? Cfg<BN>::MAX_RES_KB2 : Cfg<BN>::MAX_RES_KB) &&
                         p.n_tiles <= sms / 2 && p.m_tiles >= 2 * (sms / p.n_tiles);
   p.res_kb = resident ? p.kb_total : 0;
@@ -183,7 +203,13 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
     const int total = p.m_tiles * p.n_tiles * p.splits;
     grid = total < sms ? total : sms;
   }
-  return esgd::launch(gemm_kernel<P, kBn>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+  return esgd::launch<kPair ? 2 : 1>(gemm_kernel<P, kBn>, dim3(kPair ? 2 * grid : grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+}
+
+// Pairs of CTAs: 256 x 256 tiles that read each operand once for both (32 KB a k-block and CTA instead of 48, five stages
+// deep instead of three).
+bool pair_applicable(int M, int N, int K, int splits) {
+  return M > BM && N > BM && K > 4 * BK && (N + 255) / 256 <= 74;
 }
 
 template <int BN>
@@ -226,6 +252,11 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
   const int BN = tile_columns(N, (M + BM - 1) / BM * (splits > 1 ? splits : 1), sm_count());
   if (BN == 64) return launch_major<64>(a_mn, b_mn, g, ep, s);
   if (BN == 128) return launch_major<128>(a_mn, b_mn, g, ep, s);
+  if (pair_applicable(M, N, K, splits)) {
+    if (!a_mn && !b_mn) return launch<256, false, false, false, true>(g, ep, s);
+    if (!a_mn && b_mn) return launch<256, false, true, false, true>(g, ep, s);
+    if (a_mn && b_mn) return launch<256, true, true, false, true>(g, ep, s);
+  }
   return launch_major<256>(a_mn, b_mn, g, ep, s);
 }
 

@@ -15,18 +15,25 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <class... K, class... A>
+// kCluster: CTAs of a cluster (along x).
+template <int kCluster = 1, class... K, class... A>
 inline int launch(void (*kernel)(K...), dim3 grid, int threads, size_t smem, void* stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  if (kCluster > 1) {
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = kCluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   count_launch();
   return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
 }

@@ -87,6 +87,7 @@ struct Cfg {
   static constexpr int STAGES = BN == 256 ? 3 : (BN == 128 ? 5 : 6);             // with one panel per group
   static constexpr int ACCS = BN == 256 ? 2 : 4;       // accumulators in tensor memory: tiles in flight
   static constexpr int TMEM_COLS = ACCS * BN;
+  static constexpr int PAIR_STAGES = 5;                // a pair's stage: 128 rows of A and half of B's columns in each CTA
   static constexpr int MAX_STAGES = 8;                 // A-only ring of the B-resident mode
   static constexpr int STAGE_AREA = 161 * 1024;        // operand stages (ring, or A ring + resident B)
   static constexpr int STAGE_AREA2 = STAGE_AREA - NUM_GROUPS * PANEL_BYTES;      // ... beside two panels per group
@@ -236,6 +237,8 @@ __device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
 //   void load(const Tile&, int kb, uint8_t* a, uint8_t* b, uint64_t* bar)
 //   void load_a(...a, bar) / load_b(...b, bar)     the two halves of load(); int res_kb (0: B not resident)
 //   void store_panel(const Tile&, int panel, const void* smem)   TMA store of a 128x64 bf16 panel
+//   static constexpr bool kPair                    the CTA is one of a pair (below): tile() gives it its own 128 rows, load()
+//                                                  takes its half of B's columns and the address of the leader's barrier
 //   static constexpr bool kTwoPanels               residual panels in buffers of their own (kBn kernels)
 //   void load_res_panel(const Tile&, int panel, void* smem, uint64_t* bar)   TMA load of the residual's panel
 //   static constexpr bool kHalo; int out_row(int row)   row of the stored tile for a GEMM row (identity unless kHalo)
@@ -259,7 +262,10 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   const bool two_panels = kBn && P::kTwoPanels && ep.residual != nullptr;
   const int area = two_panels ? C::STAGE_AREA2 : C::STAGE_AREA;
   const int nhalo = kHalo ? (res_kb > 0 ? 2 : MAX_HALOS) : 0;
-  const int nstages = kHalo ? (res_kb > 0 ? 1 : min(C::MAX_STAGES, (C::STAGE_AREA - nhalo * HALO_BYTES) / C::B_STAGE_BYTES))
+  constexpr bool kPair = P::kPair;
+  const bool leads = !kPair || (blockIdx.x & 1) == 0;
+  constexpr int kBStage = kPair ? C::B_STAGE_BYTES / 2 : C::B_STAGE_BYTES;
+  const int nstages = kPair ? C::PAIR_STAGES : kHalo ? (res_kb > 0 ? 1 : min(C::MAX_STAGES, (C::STAGE_AREA - nhalo * HALO_BYTES) / C::B_STAGE_BYTES))
                             : (res_kb > 0 ? min(C::MAX_STAGES, (area - res_kb * C::B_STAGE_BYTES) / A_STAGE_BYTES)
                                           : min(STAGES, area / (A_STAGE_BYTES + C::B_STAGE_BYTES)));
   uint8_t* sA = smem;                        // halo mode: the input boxes
@@ -280,7 +286,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::MAX_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int a = 0; a < C::ACCS; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], BN / 64 * GROUP_THREADS / 32); }
+    for (int a = 0; a < C::ACCS; ++a) { mbar_init(&tfull[a], 1); mbar_init(&tempty[a], (kPair ? 2 : 1) * BN / 64 * GROUP_THREADS / 32); }
     mbar_init(bres, 1);
     for (int b = 0; b < NUM_GROUPS; ++b) mbar_init(&rfull[b], 1);
     for (int b = 0; b < MAX_HALOS; ++b) { mbar_init(&hfull[b], 1); mbar_init(&hempty[b], 1); }
@@ -288,8 +294,12 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, C::TMEM_COLS);
-    tmem_relinquish();
+    if (kPair) {
+      tmem_alloc_pair(tmem_slot, C::TMEM_COLS);
+    } else {
+      tmem_alloc(tmem_slot, C::TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   if (P::kZeroStages) {
     // partial boxes leave the tail rows of a stage untouched: they must read as zeros for ever
@@ -300,6 +310,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   }
   tc_fence_before();
   __syncthreads();
+  if (kPair) cluster_sync_all();             // the peer's barriers are there, too
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   esgd::pdl_enter();       // the setup above overlaps the end of the kernel before; from here on its results are there
@@ -350,7 +361,11 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
       for (int it = 0; ok && prob.tile(it, t); ++it) {
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          if (res_kb > 0) {
+          if constexpr (kPair) {
+            // both CTAs' loads arrive at the leader's barrier; it may see the peer's bytes before it expects them
+            if (leads) mbar_expect_tx(&full[stage], 2 * (A_STAGE_BYTES + kBStage));
+            prob.load(t, kb, sA + stage * A_STAGE_BYTES, sB + stage * kBStage, leader_addr(&full[stage]));
+          } else if (res_kb > 0) {
             mbar_expect_tx(&full[stage], tx_a);
             prob.load_a(t, kb, sA + stage * A_STAGE_BYTES, &full[stage]);
           } else {
@@ -363,14 +378,18 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
-      const uint32_t idesc = umma_idesc_bf16(BM, prob.n_mma, P::A_MN ? 1 : 0, P::B_MN ? 1 : 0);
+    if (leads && elect_one()) {
+      const uint32_t idesc = umma_idesc_bf16(kPair ? 2 * BM : BM, prob.n_mma, P::A_MN ? 1 : 0, P::B_MN ? 1 : 0);
       // Products of one k-block.  Below 64 reduced channels (narrow convolutions) the last steps would multiply zero fill;
       // the full block is a path of its own because a predicate per instruction slows the issue loop of narrow tiles.
       const int ksteps = prob.ksteps;
       auto issue_block = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t& accumulate) {
         constexpr uint64_t sa = P::A_MN ? (2048 >> 4) : (32 >> 4), sb = P::B_MN ? (2048 >> 4) : (32 >> 4);   // 16 K elements
-        if (ksteps == BK / 16) {
+        if constexpr (kPair) {
+          umma_bf16_pair(d, a, b, idesc, accumulate);
+#pragma unroll
+          for (int j = 1; j < BK / 16; ++j) umma_bf16_pair(d, a + j * sa, b + j * sb, idesc, 1u);
+        } else if (ksteps == BK / 16) {
           umma_bf16(d, a, b, idesc, accumulate);
 #pragma unroll
           for (int j = 1; j < BK / 16; ++j) umma_bf16(d, a + j * sa, b + j * sb, idesc, 1u);
@@ -433,13 +452,15 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint64_t a_cur = a_desc0 + (uint64_t)(stage * (A_STAGE_BYTES >> 4));
-          const uint64_t b_cur = b_desc0 + (uint64_t)((res_kb > 0 ? kb : stage) * (C::B_STAGE_BYTES >> 4));
+          const uint64_t b_cur = b_desc0 + (uint64_t)((res_kb > 0 ? kb : stage) * (kBStage >> 4));
           issue_block(d_tmem, a_cur, b_cur, accumulate);
-          umma_commit(&empty[stage]);
+          if constexpr (kPair) umma_commit_pair(&empty[stage]);
+          else umma_commit(&empty[stage]);
           if (++stage == nstages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);
+        if constexpr (kPair) umma_commit_pair(&tfull[acc]);
+        else umma_commit(&tfull[acc]);
         if (++acc == C::ACCS) { acc = 0; acc_phase ^= 1u; }
       }
     }
@@ -464,6 +485,10 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     uint32_t res_phase = 0;
     bool ok = true;
     typename P::Tile t;
+    auto release_acc = [&](int a) {
+      if (kPair) mbar_arrive_at(leader_addr(&tempty[a]));
+      else mbar_arrive(&tempty[a]);
+    };
     // The residual panel of a unit travels while the group finishes the one before it.
     auto fetch_residual = [&](int it) {
       typename P::Tile n;
@@ -528,7 +553,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           tmem_ld_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[acc]);
+          if (lane == 0) release_acc(acc);
         };
         if (kBn || ep.out_mode == OUT_BF16) {
           if (!kBn && plain) {
@@ -621,7 +646,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           }
         }
       } else {
-        if (lane == 0) mbar_arrive(&tempty[acc]);
+        if (lane == 0) release_acc(acc);
         if (has_res && leader) {
           tma_store_wait_read<0>();
           fetch_residual(it + TURNS);
@@ -658,9 +683,11 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     __nanosleep(1000000);
     if (threadIdx.x == 0 && ep.error_flag != nullptr) atomicExch(ep.error_flag, 1);
   }
+  if (kPair) cluster_sync_all();             // nobody leaves while the peer's barriers or products may still use this CTA
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, C::TMEM_COLS);
+    if (kPair) tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
+    else tmem_dealloc(tmem_base, C::TMEM_COLS);
   }
 }
 
