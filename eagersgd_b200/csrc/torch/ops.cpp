@@ -582,27 +582,38 @@ struct ConvFn : public Function<ConvFn> {
 };
 
 // Which kernel takes a convolution; -1: none, the shape is not this package's.
-int64_t conv_kind(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool narrow) {
-  const int64_t c = x.size(1), k0 = w.size(0), r = w.size(2), s = w.size(3);
+int64_t conv_kind_of(int64_t c, const Tensor& w, int64_t stride, int64_t pad, bool narrow, bool x_grad) {
+  const int64_t k0 = w.size(0), r = w.size(2), s = w.size(3);
   if (r == 1 && s == 1 && pad == 0 && stride <= 2 && c % 8 == 0 && k0 % 8 == 0) return kOneByOne;
-  if (r > 1 && c <= 4 && k0 % 8 == 0 && !x.requires_grad()) return kStem;
+  if (r > 1 && c <= 4 && k0 % 8 == 0 && !x_grad) return kStem;
   if (r > 1 && c % 8 == 0 && k0 % 8 == 0 && stride <= 2 && (narrow || c % 64 == 0)) return kGeneral;
   return -1;
 }
 
-// Returns (y, stats | None, tapped input | None), or None when the shape is not this package's.
-py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap, bool narrow) {
-  const int64_t r = w.size(2), s = w.size(3), kind = conv_kind(x, w, stride, pad, narrow);
-  if (kind < 0) return py::none();
+int64_t conv_kind(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool narrow) {
+  return conv_kind_of(x.size(1), w, stride, pad, narrow, x.requires_grad());
+}
+
+struct ConvOut {
+  Tensor y, stats, tapped;       // stats, tapped: on request
+};
+ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap) {
+  const int64_t r = w.size(2), s = w.size(3);
   // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
   const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
   Sink sink = find_sink(w);
   sink_use(sink);
   variable_list out = ConvFn::apply(x, graph_input(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink),
                                     sink && stride == 1 ? bn_behind(x) : BnRef());
-  py::object st = want_stats ? py::cast(out[1]) : py::none();
-  py::object tp = !tap ? py::none() : py::cast(fuse_tap ? out.back() : x);
-  return py::make_tuple(out[0], st, tp);
+  return {out[0], want_stats ? out[1] : Tensor(), !tap ? Tensor() : (fuse_tap ? out.back() : x)};
+}
+
+// Returns (y, stats | None, tapped input | None), or None when the shape is not this package's.
+py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap, bool narrow) {
+  const int64_t kind = conv_kind(x, w, stride, pad, narrow);
+  if (kind < 0) return py::none();
+  const ConvOut o = conv_train(kind, x, w, stride, pad, want_stats, tap);
+  return py::make_tuple(o.y, want_stats ? py::cast(o.stats) : py::none(), tap ? py::cast(o.tapped) : py::none());
 }
 
 // Inference: act(batch_norm(conv(x)) + residual) in one kernel.  coef [2][Cout] fp32: scale and shift (BnCoefficients), or
@@ -834,6 +845,52 @@ Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c1
   return z;
 }
 
+// A residual block in training (convolution, batch norm and ReLU in a row, the last batch norm adding the shortcut): what the
+// two operators above do layer by layer, in one call from Python, which spent 9 us a layer between them.  A layer is (filter,
+// stride, padding, gamma, beta, running mean, running variance, momentum); proj: the shortcut's, or None.  None when a layer
+// is not this package's.
+struct BlockLayer {
+  Tensor w, gamma, beta;
+  int64_t stride, pad, kind;
+  c10::optional<Tensor> mean, var;
+  double momentum;
+  BlockLayer(const py::tuple& t, const Tensor& x, bool narrow)
+      : w(t[0].cast<Tensor>()), gamma(t[3].cast<Tensor>()), beta(t[4].cast<Tensor>()), stride(t[1].cast<int64_t>()),
+        pad(t[2].cast<int64_t>()), mean(t[5].cast<c10::optional<Tensor>>()), var(t[6].cast<c10::optional<Tensor>>()),
+        momentum(t[7].cast<double>()) {
+    kind = w.size(2) > 1 && w.size(1) <= 4 ? -1 : conv_kind_of(w.size(1), w, stride, pad, narrow, true);
+    if (w.scalar_type() != at::kBFloat16 || gamma.scalar_type() != at::kFloat || w.size(0) % 8) kind = -1;
+  }
+  Tensor norm(const ConvOut& o, bool relu, const c10::optional<Tensor>& res) const {
+    return bn_act(o.y, gamma, beta, res, mean, var, momentum, relu, o.stats);
+  }
+};
+py::object residual_block(const Tensor& x, const std::vector<py::tuple>& layers, const c10::optional<py::tuple>& proj, bool narrow) {
+  std::vector<BlockLayer> ls;
+  ls.reserve(layers.size() + 1);
+  for (const auto& t : layers) ls.emplace_back(t, x, narrow);
+  if (proj.has_value()) ls.emplace_back(*proj, x, narrow);
+  for (const auto& l : ls)
+    if (l.kind < 0) return py::none();
+  if (x.size(1) != ls[0].w.size(1)) return py::none();
+  Tensor out;
+  {
+    py::gil_scoped_release nogil;
+    const size_t n = layers.size();
+    ConvOut c = conv_train(ls[0].kind, x, ls[0].w, ls[0].stride, ls[0].pad, true, true);
+    c10::optional<Tensor> shortcut = c.tapped;
+    if (proj.has_value()) {
+      const BlockLayer& p = ls[n];
+      shortcut = p.norm(conv_train(p.kind, c.tapped, p.w, p.stride, p.pad, true, false), false, c10::nullopt);
+    }
+    for (size_t i = 0; i < n; ++i) {
+      if (i > 0) c = conv_train(ls[i].kind, out, ls[i].w, ls[i].stride, ls[i].pad, true, false);
+      out = ls[i].norm(c, true, i + 1 == n ? shortcut : c10::nullopt);
+    }
+  }
+  return py::cast(out);
+}
+
 BnRef bn_behind(const Tensor& x) {
   auto* node = dynamic_cast<torch::autograd::CppNode<BnActFn>*>(x.grad_fn().get());
   if (node == nullptr || !x.is_contiguous(kCL)) return BnRef();
@@ -1031,6 +1088,7 @@ PYBIND11_MODULE(_esgd_torch, m) {
   py::class_<BnCoefficients, std::shared_ptr<BnCoefficients>>(m, "BnCoefficients").def(py::init<>()).def("compute", &BnCoefficients::compute);
   m.def("linear", &linear);
   m.def("bn_act", &bn_act);
+  m.def("residual_block", &residual_block);
   m.def("softmax_ce", &softmax_ce);
   m.def("lstm_layer", &lstm_layer);
   m.def("max_pool", &max_pool);

@@ -75,6 +75,21 @@ class _Conv(nn.Conv2d):
                           tap_input=tap_input)
 
 
+def _bare(m: nn.Module, cls) -> bool:
+    """Calling ``m`` does what ``cls.forward`` does in training, and nothing else."""
+    return type(m) is cls and m.training and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or
+                                                  m._backward_pre_hooks or "forward" in m.__dict__)
+
+
+def _train_layer(conv, bn):
+    """A convolution and its batch norm for ``ops.residual_block``; None when somebody could see the two being skipped."""
+    if not _bare(conv, _Conv) or not _bare(bn, BatchNormAct) or bn.virtual_batch_size or bn.momentum is None or not bn.affine:
+        return None
+    p, b = bn._parameters, bn._buffers
+    return (conv._parameters["weight"], conv.stride[0], conv.padding[0], p["weight"], p["bias"], b["running_mean"],
+            b["running_var"], bn.momentum)
+
+
 class _Block(nn.Module):
     def __init__(self, cin, filters, stride, kind, version, project, registry):
         super().__init__()
@@ -108,9 +123,23 @@ class _Block(nn.Module):
         self.bns = nn.ModuleList(bns)
         self.cout = cout
 
+    def _fused_train(self, x):
+        """The block in one call of the operators' library, or None where its layers have to be called one by one."""
+        if not self.training or not ops.native(x) or nn.modules.module._has_any_global_hook():
+            return None
+        m = self._modules
+        layers = [_train_layer(c, b) for c, b in zip(m["convs"]._modules.values(), m["bns"]._modules.values())]
+        proj = _train_layer(self.proj, self.proj_bn) if self.proj is not None else None
+        if any(e is None for e in layers) or (proj is None) != (self.proj is None):
+            return None
+        return ops.residual_block(x, layers, proj)
+
     def forward(self, x):
         n = len(self.convs)
         if self.version == 1:
+            y = self._fused_train(x)
+            if y is not None:
+                return y
             # The shortcut branches off the first convolution's tapped input: both gradients of x then meet
             # inside that convolution's data-gradient kernel instead of in a separate addition.
             yc, st, shortcut = self.convs[0](x, tap_input=True)

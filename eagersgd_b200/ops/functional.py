@@ -151,6 +151,13 @@ def bn_act(y: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, running_mea
     return F.relu(z) if relu else z
 
 
+def residual_block(x: torch.Tensor, layers, proj=None) -> Optional[torch.Tensor]:
+    """A residual block in training: ``conv2d`` and ``bn_act`` of every layer -- (filter, stride, padding, gamma, beta, running
+    mean, running variance, momentum) -- in one call, the shortcut through ``proj`` (a layer without ReLU) or straight; None for
+    shapes the kernels do not take."""
+    return _ext().residual_block(x, layers, proj, _SMALL_CHANNELS_NATIVE) if native(x) else None
+
+
 # --------------------------------------------------------------------------- inference: convolution + batch norm in one kernel
 def bn_coefficients(layers, store):
     """Scale and shift (``[2 * C]`` fp32, one after the other) of each inference batch norm in ``layers`` -- tuples of gamma,
