@@ -618,10 +618,8 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
 
 // Inference: act(batch_norm(conv(x)) + residual) in one kernel.  coef [2][Cout] fp32: scale and shift (BnCoefficients), or
 // None for a bare convolution.  No autograd; None when the shape is not this package's.
-py::object conv_bn_eval(const Tensor& x_in, const Tensor& w, int64_t stride, int64_t pad, const c10::optional<Tensor>& coef,
-                        const c10::optional<Tensor>& residual, bool relu, bool narrow) {
-  const int64_t kind = conv_kind(x_in, w, stride, pad, narrow);
-  if (kind < 0 || w.scalar_type() != at::kBFloat16) return py::none();
+Tensor conv_eval(int64_t kind, const Tensor& x_in, const Tensor& w, int64_t stride, int64_t pad, const c10::optional<Tensor>& coef,
+                 const c10::optional<Tensor>& residual, bool relu) {
   c10::cuda::CUDAGuard guard(x_in.device());
   Tensor x = nhwc(x_in), res = residual.has_value() ? nhwc(*residual) : Tensor(), kept, filters;
   const int64_t cout = w.size(0);
@@ -634,6 +632,44 @@ py::object conv_bn_eval(const Tensor& x_in, const Tensor& w, int64_t stride, int
   if (res.defined()) e.residual = res.data_ptr();
   e.relu = relu;
   launch_conv(kind, x, w, y, stride, pad, e, &kept, &filters);
+  return y;
+}
+py::object conv_bn_eval(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, const c10::optional<Tensor>& coef,
+                        const c10::optional<Tensor>& residual, bool relu, bool narrow) {
+  const int64_t kind = conv_kind(x, w, stride, pad, narrow);
+  if (kind < 0 || w.scalar_type() != at::kBFloat16) return py::none();
+  return py::cast(conv_eval(kind, x, w, stride, pad, coef, residual, relu));
+}
+
+// A residual block in inference: layers (filter, stride, padding, coefficients), each with a ReLU, the last one after the
+// shortcut (through proj, which has none, or straight).  None when a layer is not this package's.
+py::object residual_block_eval(const Tensor& x, const std::vector<py::tuple>& layers, const c10::optional<py::tuple>& proj, bool narrow) {
+  struct Layer {
+    Tensor w, coef;
+    int64_t stride, pad, kind;
+  };
+  std::vector<Layer> ls;
+  ls.reserve(layers.size() + 1);
+  auto add = [&](const py::tuple& t) {
+    Layer l{t[0].cast<Tensor>(), t[3].cast<Tensor>(), t[1].cast<int64_t>(), t[2].cast<int64_t>(), 0};
+    l.kind = l.w.scalar_type() != at::kBFloat16 ? -1 : conv_kind_of(l.w.size(1), l.w, l.stride, l.pad, narrow, true);
+    ls.push_back(l);
+    return l.kind >= 0;
+  };
+  for (const auto& t : layers)
+    if (!add(t)) return py::none();
+  if (proj.has_value() && !add(*proj)) return py::none();
+  if (x.size(1) != ls[0].w.size(1)) return py::none();
+  Tensor y = x;
+  {
+    py::gil_scoped_release nogil;
+    const size_t n = layers.size();
+    Tensor shortcut = x;
+    if (proj.has_value()) shortcut = conv_eval(ls[n].kind, x, ls[n].w, ls[n].stride, ls[n].pad, ls[n].coef, c10::nullopt, false);
+    for (size_t i = 0; i < n; ++i)
+      y = conv_eval(ls[i].kind, y, ls[i].w, ls[i].stride, ls[i].pad, ls[i].coef,
+                    i + 1 == n ? c10::optional<Tensor>(shortcut) : c10::nullopt, true);
+  }
   return py::cast(y);
 }
 
@@ -641,8 +677,12 @@ py::object conv_bn_eval(const Tensor& x_in, const Tensor& w, int64_t stride, int
 // forward pass.  The table of pointers lives on the device and is rebuilt when a tensor has moved.
 class BnCoefficients {
  public:
-  std::vector<Tensor> compute(const std::vector<std::array<Tensor, 4>>& layers) {      // gamma, beta, mean, var
+  // layers: gamma, beta, mean, var; no result unless they are fp32 and on the GPU.
+  std::vector<Tensor> compute(const std::vector<std::array<Tensor, 4>>& layers) {
     std::lock_guard<std::mutex> g(m_);
+    for (const auto& l : layers)
+      for (const auto& t : l)
+        if (!t.defined() || !t.is_cuda() || t.scalar_type() != at::kFloat) return {};
     c10::cuda::CUDAGuard guard(layers.at(0)[0].device());
     std::vector<int64_t> key;
     key.reserve(layers.size() * 6);
@@ -1089,6 +1129,7 @@ PYBIND11_MODULE(_esgd_torch, m) {
   m.def("linear", &linear);
   m.def("bn_act", &bn_act);
   m.def("residual_block", &residual_block);
+  m.def("residual_block_eval", &residual_block_eval);
   m.def("softmax_ce", &softmax_ce);
   m.def("lstm_layer", &lstm_layer);
   m.def("max_pool", &max_pool);

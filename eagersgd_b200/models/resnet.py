@@ -206,10 +206,12 @@ class ResNet(nn.Module):
         for m in st["modules"]:
             if m.training or m._forward_hooks or m._forward_pre_hooks:
                 return None
-        layers = [(m.weight, m.bias, m.running_mean, m.running_var) for m in st["norms"]]
-        if not all(t is not None and t.is_cuda and t.dtype == torch.float32 for layer in layers for t in layer):
+        layers = [(m._parameters["weight"], m._parameters["bias"], m._buffers["running_mean"], m._buffers["running_var"])
+                  for m in st["norms"]]
+        if any(t is None for layer in layers for t in layer):
             return None
-        return dict(zip(st["norms"], ops.bn_coefficients(layers, st)))
+        coef = ops.bn_coefficients(layers, st)
+        return dict(zip(st["norms"], coef)) if coef or not layers else None
 
     @staticmethod
     def _conv_eval(conv, bn, x, coef, relu, residual=None):
@@ -227,6 +229,16 @@ class ResNet(nn.Module):
         if self.first_pool:
             x = ops.max_pool_3x3_s2(x)
         for blk in self.blocks:
+            if self.version == 1:
+                m = blk._modules
+                layers = [(c._parameters["weight"], c.stride[0], c.padding[0], coef[b])
+                          for c, b in zip(m["convs"]._modules.values(), m["bns"]._modules.values())]
+                proj = blk.proj
+                y = ops.residual_block_eval(x, layers, None if proj is None else
+                                            (proj._parameters["weight"], proj.stride[0], proj.padding[0], coef[blk.proj_bn]))
+                if y is not None:
+                    x = y
+                    continue
             n, y, shortcut = len(blk.convs), x, x
             if self.version == 1:
                 if blk.proj is not None:

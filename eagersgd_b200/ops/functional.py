@@ -161,7 +161,8 @@ def residual_block(x: torch.Tensor, layers, proj=None) -> Optional[torch.Tensor]
 # --------------------------------------------------------------------------- inference: convolution + batch norm in one kernel
 def bn_coefficients(layers, store):
     """Scale and shift (``[2 * C]`` fp32, one after the other) of each inference batch norm in ``layers`` -- tuples of gamma,
-    beta, running mean, running variance -- from one launch.  ``store``: a dict of the caller's that keeps the device table."""
+    beta, running mean, running variance -- from one launch; empty unless all of them are fp32 and on the GPU.  ``store``: a
+    dict of the caller's that keeps the device table."""
     if "bn" not in store:
         store["bn"] = _ext().BnCoefficients()
     return store["bn"].compute(layers)
@@ -171,6 +172,11 @@ def conv_bn_eval(x: torch.Tensor, w: torch.Tensor, stride: int, padding: int, co
                  residual: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """act(scale * conv(x) + shift [+ residual]) rounded once, without autograd; None for shapes the kernels do not take."""
     return _ext().conv_bn_eval(x, w, stride, padding, coef, residual, relu, _SMALL_CHANNELS_NATIVE)
+
+
+def residual_block_eval(x: torch.Tensor, layers, proj=None) -> Optional[torch.Tensor]:
+    """A residual block in inference, like ``residual_block``: layers of (filter, stride, padding, coefficients)."""
+    return _ext().residual_block_eval(x, layers, proj, _SMALL_CHANNELS_NATIVE)
 
 
 # --------------------------------------------------------------------------- softmax cross-entropy
