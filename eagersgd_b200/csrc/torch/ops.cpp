@@ -121,10 +121,9 @@ class ZeroArena {
     const int64_t n = c10::multiply_integers(shape), n_al = (n + 63) / 64 * 64;    // 256-byte aligned slices
     if (off_ + n_al > cap_) return Tensor();
     if (!buf_.defined()) buf_ = at::zeros({cap_}, at::TensorOptions().dtype(at::kFloat).device(device_));
-    std::vector<int64_t> strides(shape.size());
-    int64_t s = 1;
-    for (int i = (int)shape.size() - 1; i >= 0; --i) { strides[i] = s; s *= shape[i]; }
-    Tensor out = buf_.as_strided(shape, strides, off_);
+    Tensor out = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(buf_.storage()), buf_.key_set(), buf_.dtype());
+    out.unsafeGetTensorImpl()->set_storage_offset(off_);           // a view without a trip through the dispatcher
+    out.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
     off_ += n_al;
     dirty_ = std::max(dirty_, off_);
     return out;
@@ -280,6 +279,12 @@ void sink_use(const Sink& s) {
 // The parameter as the operator's autograd input: detached when a sink takes its gradient, so that autograd neither
 // expects one nor calls the parameter's hooks.
 Tensor graph_input(const Tensor& p, const Sink& s) { return s ? p.detach() : p; }
+// The same without the detached view's microsecond: the tensor as an argument that autograd does not look at, and none where
+// it would.
+struct Held {
+  Tensor t;
+};
+c10::optional<Tensor> graph_only(const Tensor& p, const Sink& s) { return s ? c10::nullopt : c10::optional<Tensor>(p); }
 // What then keeps the operator in the graph when nothing else requires a gradient (the first layer of a network).
 c10::optional<Tensor> anchor_for(const Tensor& x, bool any_sink) {
   if (!any_sink || x.requires_grad()) return c10::nullopt;
@@ -422,17 +427,19 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
 // from x itself: backward then receives the shortcut's gradient together with dy and adds it in the epilogue of the
 // data-gradient GEMM, instead of autograd summing the two branches of x with a separate pass over the tensor.
 struct ConvFn : public Function<ConvFn> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w, int64_t kind, int64_t stride, int64_t pad,
-                               bool want_stats, bool tap, const Sink& sink, const c10::optional<Tensor>& anchor, const BnRef& bn) {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const c10::optional<Tensor>& w_in, int64_t kind,
+                               int64_t stride, int64_t pad, bool want_stats, bool tap, const Sink& sink,
+                               const c10::optional<Tensor>& anchor, const BnRef& bn, const Held& w_held, const Held& into) {
+    const Tensor& w = w_in.has_value() ? *w_in : w_held.t;
     c10::cuda::CUDAGuard guard(x_in.device());
     Tensor x = nhwc(x_in);
     const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3);
     const int64_t cout = w.size(0), r = w.size(2), s = w.size(3);
     const int64_t ho = (h + 2 * pad - r) / stride + 1, wo = (wd + 2 * pad - s) / stride + 1;
-    Tensor stats;
+    Tensor stats = into.t;                            // given: not an output of the graph's
     ConvEpilogue e;
-    if (want_stats) {
-      stats = zeros_f32({2, cout}, x.device());
+    if (want_stats) stats = zeros_f32({2, cout}, x.device());
+    if (stats.defined()) {
       e.sum = fptr(stats);
       e.sqsum = e.sum + cout;
     }
@@ -457,7 +464,7 @@ struct ConvFn : public Function<ConvFn> {
     const auto cfg = ctx->saved_data["cfg"].toIntVector();
     const int64_t kind = cfg[0], stride = cfg[1], pad = cfg[2], n = cfg[3], cin = cfg[4], h = cfg[5], wd = cfg[6];
     const bool want_stats = cfg[7], tap = cfg[8];
-    variable_list none(10);
+    variable_list none(12);
     Tensor d_tap = tap ? grads[want_stats ? 2 : 1] : Tensor();   // gradient that reached the input through the shortcut
     Sink sink = load_sink(ctx, "w");
     if (!grads[0].defined()) {
@@ -597,14 +604,15 @@ int64_t conv_kind(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
 struct ConvOut {
   Tensor y, stats, tapped;       // stats, tapped: on request
 };
-ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap) {
+ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap,
+                   const Tensor& into = Tensor()) {
   const int64_t r = w.size(2), s = w.size(3);
   // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
   const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
   Sink sink = find_sink(w);
   sink_use(sink);
-  variable_list out = ConvFn::apply(x, graph_input(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink),
-                                    sink && stride == 1 ? bn_behind(x) : BnRef());
+  variable_list out = ConvFn::apply(x, graph_only(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink),
+                                    sink && stride == 1 ? bn_behind(x) : BnRef(), Held{w}, Held{into});
   return {out[0], want_stats ? out[1] : Tensor(), !tap ? Tensor() : (fuse_tap ? out.back() : x)};
 }
 
@@ -788,12 +796,12 @@ py::object linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>&
 // ---------------------------------------------------------------- batch norm (+ residual) (+ ReLU)
 struct BnActFn : public Function<BnActFn> {
   using Opt = c10::optional<Tensor>;
-  static Tensor forward(AutogradContext* ctx, const Tensor& y_in, const Tensor& gamma, const Tensor& beta, const Opt& res_in,
-                        const Opt& rm_in, const Opt& rv_in, double momentum, bool relu, const Opt& stats_in, const Sink& gs,
-                        const Sink& bs, const Opt& anchor) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& y_in, const Opt& gamma_in, const Opt& beta_in, const Opt& res_in,
+                        const Held& rm_in, const Held& rv_in, double momentum, bool relu, const Held& stats_in, const Sink& gs,
+                        const Sink& bs, const Opt& anchor, const Held& gamma_held, const Held& beta_held) {
+    const Tensor &gamma = gamma_in.has_value() ? *gamma_in : gamma_held.t, &beta = beta_in.has_value() ? *beta_in : beta_held.t;
     c10::cuda::CUDAGuard guard(y_in.device());
-    auto get = [](const Opt& o) { return o.has_value() ? *o : Tensor(); };
-    Tensor y = nhwc(y_in), res = res_in.has_value() ? nhwc(*res_in) : Tensor(), stats = get(stats_in), rm = get(rm_in), rv = get(rv_in);
+    Tensor y = nhwc(y_in), res = res_in.has_value() ? nhwc(*res_in) : Tensor(), stats = stats_in.t, rm = rm_in.t, rv = rv_in.t;
     const int64_t n = y.size(0), c = y.size(1), m = n * y.size(2) * y.size(3);
     void* st = stream_of(y);
     if (!stats.defined()) {
@@ -817,7 +825,7 @@ struct BnActFn : public Function<BnActFn> {
     save_sink(ctx, "b", bs);
     if (gs && bs) {
       auto rec = c10::make_intrusive<BnRecord>();
-      rec->y = y.detach();
+      rec->y = y;
       rec->mask = mask;
       rec->aux = aux;
       ctx->saved_data["rec"] = c10::IValue::make_capsule(rec);
@@ -864,7 +872,7 @@ struct BnActFn : public Function<BnActFn> {
     else dgamma = red.select(0, 1);
     if (bs) sink_done(bs);
     else dbeta = red.select(0, 0);
-    variable_list out(12);
+    variable_list out(14);
     out[0] = dy; out[1] = dgamma; out[2] = dbeta; out[3] = dres;
     return out;
   }
@@ -876,8 +884,9 @@ Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c1
   Sink gs = find_sink(gamma), bs = find_sink(beta);
   sink_use(gs);
   sink_use(bs);
-  Tensor z = BnActFn::apply(y, graph_input(gamma, gs), graph_input(beta, bs), res, rm, rv, momentum, relu, stats, gs, bs,
-                            anchor_for(y, gs || bs));
+  auto held = [](const c10::optional<Tensor>& o) { return Held{o.has_value() ? *o : Tensor()}; };
+  Tensor z = BnActFn::apply(y, graph_only(gamma, gs), graph_only(beta, bs), res, held(rm), held(rv), momentum, relu, held(stats), gs,
+                            bs, anchor_for(y, gs || bs), Held{gamma}, Held{beta});
   if (gs && bs) {
     auto* node = static_cast<torch::autograd::CppNode<BnActFn>*>(z.grad_fn().get());
     c10::static_intrusive_pointer_cast<BnRecord>(node->ctx_.saved_data.at("rec").toCapsule())->node = z.grad_fn();
@@ -901,8 +910,13 @@ struct BlockLayer {
     kind = w.size(2) > 1 && w.size(1) <= 4 ? -1 : conv_kind_of(w.size(1), w, stride, pad, narrow, true);
     if (w.scalar_type() != at::kBFloat16 || gamma.scalar_type() != at::kFloat || w.size(0) % 8) kind = -1;
   }
+  Tensor stats;                  // of the convolution's output, for the batch norm behind it
+  ConvOut conv(const Tensor& x, bool tap) {
+    stats = zeros_f32({2, w.size(0)}, x.device());
+    return conv_train(kind, x, w, stride, pad, false, tap, stats);
+  }
   Tensor norm(const ConvOut& o, bool relu, const c10::optional<Tensor>& res) const {
-    return bn_act(o.y, gamma, beta, res, mean, var, momentum, relu, o.stats);
+    return bn_act(o.y, gamma, beta, res, mean, var, momentum, relu, stats);
   }
 };
 py::object residual_block(const Tensor& x, const std::vector<py::tuple>& layers, const c10::optional<py::tuple>& proj, bool narrow) {
@@ -917,14 +931,13 @@ py::object residual_block(const Tensor& x, const std::vector<py::tuple>& layers,
   {
     py::gil_scoped_release nogil;
     const size_t n = layers.size();
-    ConvOut c = conv_train(ls[0].kind, x, ls[0].w, ls[0].stride, ls[0].pad, true, true);
+    ConvOut c = ls[0].conv(x, true);
     c10::optional<Tensor> shortcut = c.tapped;
     if (proj.has_value()) {
-      const BlockLayer& p = ls[n];
-      shortcut = p.norm(conv_train(p.kind, c.tapped, p.w, p.stride, p.pad, true, false), false, c10::nullopt);
+      shortcut = ls[n].norm(ls[n].conv(c.tapped, false), false, c10::nullopt);
     }
     for (size_t i = 0; i < n; ++i) {
-      if (i > 0) c = conv_train(ls[i].kind, out, ls[i].w, ls[i].stride, ls[i].pad, true, false);
+      if (i > 0) c = ls[i].conv(out, false);
       out = ls[i].norm(c, true, i + 1 == n ? shortcut : c10::nullopt);
     }
   }
