@@ -48,10 +48,10 @@ __device__ __forceinline__ void load_filter_tap(const CUtensorMap* tm, const Fil
   }
 }
 
-template <int BN_, bool kT>
+template <int BN_, bool kT, bool kPair_>
 struct ConvProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kTwoPanels = false, kPair = false;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kTwoPanels = false, kPair = kPair_;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, stride, pad;
@@ -66,18 +66,21 @@ struct ConvProblem {
   struct Tile { int kb0, kb1, n0, w0, h0, i0; };
 
   __device__ __forceinline__ bool tile(int it, Tile& t) const {
-    const int m_tiles = w_tiles * h_tiles * i_tiles;
+    // a pair takes two boxes at a time (the last one may be past the last image: loaded as zeros, not stored)
+    const int boxes = w_tiles * h_tiles * i_tiles, m_tiles = kPair ? (boxes + 1) / 2 : boxes;
+    const int worker = kPair ? blockIdx.x / 2 : blockIdx.x, workers = kPair ? gridDim.x / 2 : gridDim.x;
     int m_idx, n_idx;
     if (fixed_n) {
-      n_idx = blockIdx.x % n_tiles;
-      m_idx = blockIdx.x / n_tiles + it * (gridDim.x / n_tiles);
+      n_idx = worker % n_tiles;
+      m_idx = worker / n_tiles + it * (workers / n_tiles);
       if (m_idx >= m_tiles) return false;
     } else {
-      const int id = blockIdx.x + it * gridDim.x;
+      const int id = worker + it * workers;
       if (id >= m_tiles * n_tiles) return false;
       m_idx = id / n_tiles;
       n_idx = id % n_tiles;
     }
+    if (kPair) m_idx = 2 * m_idx + (int)(blockIdx.x & 1);
     t.w0 = (m_idx % w_tiles) * BW;
     t.h0 = ((m_idx / w_tiles) % h_tiles) * BH;
     t.i0 = (m_idx / (w_tiles * h_tiles)) * BI;
@@ -100,11 +103,25 @@ struct ConvProblem {
     load_a(t, kb, a, bar);
     load_b(t, kb, b, bar);
   }
+  // pair: this CTA's box and its half of the output channels' filters
+  __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint32_t leader_bar) const {
+    const int tap = kb / cblks, cb = kb - tap * cblks;
+    const int r = tap / S, s = tap - r * S;
+    const int rw = taps.r0 + r * taps.dr, sw = taps.s0 + s * taps.ds, n0 = t.n0 + (int)(blockIdx.x & 1) * (BN / 2);
+    tma_load_4d_pair(a, &tmX, leader_bar, cb * 64, t.w0 * stride + s - pad, t.h0 * stride + r - pad, t.i0);
+    if (kT) {
+#pragma unroll
+      for (int i = 0; i < BN / 128; ++i) tma_load_4d_pair(b + i * 8192, &tmW, leader_bar, n0 + 64 * i, sw, rw, cb * 64);
+    } else {
+      tma_load_4d_pair(b, &tmW, leader_bar, cb * 64, sw, rw, n0);
+    }
+  }
   __device__ __forceinline__ void store_panel(const Tile& t, int panel, const void* smem) const {
-    tma_store_4d(&tmY, smem, t.n0 + panel * 64, t.w0, t.h0, t.i0);
+    if (!kPair || t.i0 < N) tma_store_4d(&tmY, smem, t.n0 + panel * 64, t.w0, t.h0, t.i0);
   }
   // A box is part of one row (BH = BI = 1), whole rows of one image (BH divides Ho) or whole images: consecutive pixels.
   __device__ __forceinline__ int valid_prefix(const Tile& t) const {
+    if (kPair && t.i0 >= N) return 0;
     return BI > 1 ? min(BI, N - t.i0) * BW * BH : min(BW, Wo - t.w0) * BH;
   }
   __device__ __forceinline__ int64_t first_row(const Tile& t) const { return ((int64_t)t.i0 * Ho + t.h0) * Wo + t.w0; }
@@ -269,21 +286,21 @@ struct ConvArgs {
 };
 
 // Tensor map over the stored filter bank [K][fR][fS][C]; forward: K = a.Cout, C = a.Cin, data gradient the other way.
-template <int BN, bool kT>
+template <int BN, bool kT, bool kPair = false>
 int filter_map(CUtensorMap* tm, const ConvArgs& a) {
   const int C = kT ? a.Cout : a.Cin, K = kT ? a.Cin : a.Cout;
   uint64_t dims[4] = {(uint64_t)C, (uint64_t)a.fS, (uint64_t)a.fR, (uint64_t)K};
   uint64_t strides[3] = {(uint64_t)C * 2, (uint64_t)a.fS * C * 2, (uint64_t)a.fR * a.fS * C * 2};
-  uint32_t box[4] = {64, 1, 1, kT ? 64u : (uint32_t)BN};
+  uint32_t box[4] = {64, 1, 1, kT ? 64u : (uint32_t)(kPair ? BN / 2 : BN)};
   return esgd::make_tensormap_bf16(tm, a.w, 4, dims, strides, box, nullptr);
 }
 inline int ksteps_of(int c) { return c >= 64 ? BK / 16 : (c + 15) / 16; }
 // narrow layers: the MMA computes no more columns than there are (the epilogue drops the rest either way)
 inline int mma_columns(int n, int bn) { return n >= bn ? bn : (n + 15) / 16 * 16; }
 
-template <int BN, bool kT, bool kBn>
+template <int BN, bool kT, bool kBn, bool kPair = false>
 int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
-  using P = ConvProblem<BN, kT>;
+  using P = ConvProblem<BN, kT, kPair>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(conv_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -324,7 +341,7 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
     if (r != 0) return 1000 + r;
   }
   {
-    int r = filter_map<BN, kT>(&p.tmW, a);
+    int r = filter_map<BN, kT, kPair>(&p.tmW, a);
     if (r != 0) return 2000 + r;
   }
   {
@@ -337,12 +354,12 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
     if (r != 0) return 3000 + r;
     ep.res_bytes = (uint32_t)(p.BW * p.BH * p.BI * 128);
   }
-  const int sms = sm_count();
-  const int total = p.w_tiles * p.h_tiles * p.i_tiles * p.n_tiles;
+  const int sms = kPair ? sm_count() / 2 : sm_count();           // workers: CTAs, or pairs of them
+  const int boxes = p.w_tiles * p.h_tiles * p.i_tiles, total = (kPair ? (boxes + 1) / 2 : boxes) * p.n_tiles;
   int grid;
   // the filter bank of the CTA's channel range stays in shared memory when it fits beside four input stages
   const int kb_total = a.R * a.S * p.cblks;
-  const bool resident = resident_enabled() && kb_total <= Cfg<BN>::MAX_RES_KB && p.n_tiles <= sms / 2 &&
+  const bool resident = !kPair && resident_enabled() && kb_total <= Cfg<BN>::MAX_RES_KB && p.n_tiles <= sms / 2 &&
                         total / p.n_tiles >= 2 * (sms / p.n_tiles);
   p.res_kb = resident ? kb_total : 0;
   p.fixed_n = (ep.col_sum != nullptr || resident) ? 1 : 0;
@@ -355,7 +372,7 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
   }
   ep.tx_bytes_a = (uint32_t)(p.BW * p.BH * p.BI * 128);
   ep.tx_bytes = ep.tx_bytes_a + (uint32_t)Cfg<BN>::B_STAGE_BYTES;
-  return esgd::launch(conv_kernel<P, kBn>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+  return esgd::launch<kPair ? 2 : 1>(conv_kernel<P, kBn>, dim3(kPair ? 2 * grid : grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 // Halo mode applies to stride-1 convolutions with full-width tiles: the box (output rows + filter margin, full
@@ -519,6 +536,10 @@ int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
     return BN == 64 ? launch_halo<64, kT, kBn>(a, ep, bh, s) : launch_halo<128, kT, kBn>(a, ep, bh, s);
   if (BN == 64) return launch<64, kT, kBn>(a, ep, s);
   if (BN == 128) return launch<128, kT, kBn>(a, ep, s);
+  // Pairs of CTAs (256-column tiles read each operand once for two boxes of pixels) where the reduction is full blocks:
+  // 256 channels at 14 x 14 and 512 at 7 x 7, batch 256: 79 -> 65 us
+  if (a.Cin % 64 == 0 && a.Cout >= 256 && a.R * a.S * (a.Cin / 64) > 4 && a.Cout <= 74 * 256)
+    return launch<256, kT, kBn, true>(a, ep, s);
   return launch<256, kT, kBn>(a, ep, s);
 }
 

@@ -363,7 +363,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
           if constexpr (kPair) {
             // both CTAs' loads arrive at the leader's barrier; it may see the peer's bytes before it expects them
-            if (leads) mbar_expect_tx(&full[stage], 2 * (A_STAGE_BYTES + kBStage));
+            if (leads) mbar_expect_tx(&full[stage], 2 * (tx_a + (uint32_t)kBStage));
             prob.load(t, kb, sA + stage * A_STAGE_BYTES, sB + stage * kBStage, leader_addr(&full[stage]));
           } else if (res_kb > 0) {
             mbar_expect_tx(&full[stage], tx_a);
