@@ -88,6 +88,26 @@ Tensor empty_nhwc(int64_t n, int64_t c, int64_t h, int64_t w, const Tensor& like
   return at::empty({n, c, h, w}, like.options(), kCL);
 }
 
+// ---------------------------------------------------------------- operands
+// The kernels take bare pointers: what an operator is handed is compared here, before anything is allocated or launched.  The
+// checks read sizes that are in the tensors anyway and cost nanoseconds.
+void check_operand(const char* op, const char* name, const Tensor& t, const Tensor& x, at::ScalarType type) {
+  TORCH_CHECK(t.scalar_type() == type, op, ": ", name, " is ", t.scalar_type(), ", not ", type);
+  TORCH_CHECK(t.device() == x.device(), op, ": ", name, " is on ", t.device(), ", the input on ", x.device());
+}
+void check_vector(const char* op, const char* name, const Tensor& t, const Tensor& x, int64_t numel) {
+  TORCH_CHECK(t.numel() == numel && t.is_contiguous(), op, ": ", name, " has to hold ", numel, " elements in a row, not ", t.sizes());
+  check_operand(op, name, t, x, at::kFloat);
+}
+void check_conv(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad) {
+  TORCH_CHECK(x.dim() == 4 && w.dim() == 4, "conv2d: takes a 4-D input and filter, not ", x.sizes(), " and ", w.sizes());
+  TORCH_CHECK(x.size(1) == w.size(1), "conv2d: the filter ", w.sizes(), " does not have the ", x.size(1), " channels of the input");
+  TORCH_CHECK(x.size(2) + 2 * pad >= w.size(2) && x.size(3) + 2 * pad >= w.size(3), "conv2d: the filter ", w.sizes(),
+              " is larger than the padded input ", x.sizes());
+  check_operand("conv2d", "the input", x, x, at::kBFloat16);
+  check_operand("conv2d", "the filter", w, x, at::kBFloat16);
+}
+
 // ---------------------------------------------------------------- per-device error word of the tensor-core kernels
 Tensor error_flag(int64_t device) {
   static std::mutex m;
@@ -591,6 +611,7 @@ struct ConvFn : public Function<ConvFn> {
 // Which kernel takes a convolution; -1: none, the shape is not this package's.
 int64_t conv_kind_of(int64_t c, const Tensor& w, int64_t stride, int64_t pad, bool narrow, bool x_grad) {
   const int64_t k0 = w.size(0), r = w.size(2), s = w.size(3);
+  if (stride < 1 || pad < 0) return -1;
   if (r == 1 && s == 1 && pad == 0 && stride <= 2 && c % 8 == 0 && k0 % 8 == 0) return kOneByOne;
   if (r > 1 && c <= 4 && k0 % 8 == 0 && !x_grad) return kStem;
   if (r > 1 && c % 8 == 0 && k0 % 8 == 0 && stride <= 2 && (narrow || c % 64 == 0)) return kGeneral;
@@ -606,6 +627,7 @@ struct ConvOut {
 };
 ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap,
                    const Tensor& into = Tensor()) {
+  check_conv(x, w, stride, pad);
   const int64_t r = w.size(2), s = w.size(3);
   // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
   const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
@@ -628,10 +650,18 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
 // None for a bare convolution.  No autograd; None when the shape is not this package's.
 Tensor conv_eval(int64_t kind, const Tensor& x_in, const Tensor& w, int64_t stride, int64_t pad, const c10::optional<Tensor>& coef,
                  const c10::optional<Tensor>& residual, bool relu) {
+  check_conv(x_in, w, stride, pad);
+  if (coef.has_value()) check_vector("conv2d", "the coefficients", *coef, x_in, 2 * w.size(0));
+  const int64_t ho = (x_in.size(2) + 2 * pad - w.size(2)) / stride + 1, wo = (x_in.size(3) + 2 * pad - w.size(3)) / stride + 1;
+  if (residual.has_value()) {
+    TORCH_CHECK(residual->sizes() == at::IntArrayRef({x_in.size(0), w.size(0), ho, wo}), "conv2d: the residual ", residual->sizes(),
+                " is not of the output's size");
+    check_operand("conv2d", "the residual", *residual, x_in, at::kBFloat16);
+  }
   c10::cuda::CUDAGuard guard(x_in.device());
   Tensor x = nhwc(x_in), res = residual.has_value() ? nhwc(*residual) : Tensor(), kept, filters;
   const int64_t cout = w.size(0);
-  Tensor y = empty_nhwc(x.size(0), cout, (x.size(2) + 2 * pad - w.size(2)) / stride + 1, (x.size(3) + 2 * pad - w.size(3)) / stride + 1, x);
+  Tensor y = empty_nhwc(x.size(0), cout, ho, wo, x);
   ConvEpilogue e;
   if (coef.has_value()) {
     e.scale = fptr(*coef);
@@ -685,12 +715,14 @@ py::object residual_block_eval(const Tensor& x, const std::vector<py::tuple>& la
 // forward pass.  The table of pointers lives on the device and is rebuilt when a tensor has moved.
 class BnCoefficients {
  public:
-  // layers: gamma, beta, mean, var; no result unless they are fp32 and on the GPU.
+  // layers: gamma, beta, mean, var; no result unless they are fp32, on the GPU and of one length a layer.
   std::vector<Tensor> compute(const std::vector<std::array<Tensor, 4>>& layers) {
     std::lock_guard<std::mutex> g(m_);
     for (const auto& l : layers)
       for (const auto& t : l)
-        if (!t.defined() || !t.is_cuda() || t.scalar_type() != at::kFloat) return {};
+        if (!t.defined() || !t.is_cuda() || t.scalar_type() != at::kFloat || !t.is_contiguous() || t.numel() != l[0].numel() ||
+            t.device() != layers[0][0].device())
+          return {};
     c10::cuda::CUDAGuard guard(layers.at(0)[0].device());
     std::vector<int64_t> key;
     key.reserve(layers.size() * 6);
@@ -784,6 +816,14 @@ struct LinearFn : public Function<LinearFn> {
 // None when the shape is not this package's.
 py::object linear(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& b) {
   if (x.size(1) % 8 || w.scalar_type() != at::kBFloat16) return py::none();
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2, "linear: takes a 2-D input and weight, not ", x.sizes(), " and ", w.sizes());
+  TORCH_CHECK(x.size(1) == w.size(1), "linear: the weight ", w.sizes(), " does not have the ", x.size(1), " columns of the input");
+  check_operand("linear", "the input", x, x, at::kBFloat16);
+  check_operand("linear", "the weight", w, x, at::kBFloat16);
+  if (b.has_value()) {
+    TORCH_CHECK(b->numel() == w.size(0), "linear: the bias ", b->sizes(), " does not have the ", w.size(0), " outputs of the weight");
+    check_operand("linear", "the bias", *b, x, b->scalar_type());
+  }
   Tensor bias = b.has_value() ? *b : Tensor();
   Sink ws = find_sink(w), bs = find_sink(bias);
   sink_use(ws);
@@ -881,6 +921,18 @@ struct BnActFn : public Function<BnActFn> {
 Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& res,
               const c10::optional<Tensor>& rm, const c10::optional<Tensor>& rv, double momentum, bool relu,
               const c10::optional<Tensor>& stats) {
+  TORCH_CHECK(y.dim() == 4, "bn_act: takes a 4-D input, not ", y.sizes());
+  const int64_t c = y.size(1);
+  check_operand("bn_act", "the input", y, y, at::kBFloat16);
+  check_vector("bn_act", "gamma", gamma, y, c);
+  check_vector("bn_act", "beta", beta, y, c);
+  if (rm.has_value()) check_vector("bn_act", "the running mean", *rm, y, c);
+  if (rv.has_value()) check_vector("bn_act", "the running variance", *rv, y, c);
+  if (stats.has_value() && stats->defined()) check_vector("bn_act", "the statistics", *stats, y, 2 * c);
+  if (res.has_value()) {
+    TORCH_CHECK(res->sizes() == y.sizes(), "bn_act: the residual ", res->sizes(), " is not of the input's size ", y.sizes());
+    check_operand("bn_act", "the residual", *res, y, at::kBFloat16);
+  }
   Sink gs = find_sink(gamma), bs = find_sink(beta);
   sink_use(gs);
   sink_use(bs);
@@ -967,7 +1019,12 @@ struct SoftmaxCEFn : public Function<SoftmaxCEFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) { return {ctx->get_saved_variables()[0] * grads[0], Tensor()}; }
 };
-Tensor softmax_ce(const Tensor& logits, const Tensor& labels) { return SoftmaxCEFn::apply(logits, labels); }
+Tensor softmax_ce(const Tensor& logits, const Tensor& labels) {
+  TORCH_CHECK(logits.dim() == 2, "softmax_ce: takes 2-D logits, not ", logits.sizes());
+  TORCH_CHECK(labels.numel() == logits.size(0), "softmax_ce: ", labels.numel(), " labels for ", logits.size(0), " rows");
+  check_operand("softmax_ce", "the labels", labels, logits, at::kLong);
+  return SoftmaxCEFn::apply(logits, labels);
+}
 
 // ---------------------------------------------------------------- pooling
 struct MaxPoolFn : public Function<MaxPoolFn> {
@@ -1119,8 +1176,16 @@ struct LstmFn : public Function<LstmFn> {
 
 // x [T, B, I] bf16, weights [4H, I] / [4H, H] bf16, bias [4H] fp32 -> h [T, B, H]; T, B, I, H multiples of 8 except T.
 Tensor lstm_layer(const Tensor& x, const Tensor& w_ih, const Tensor& w_hh, const Tensor& bias) {
-  TORCH_CHECK(w_ih.scalar_type() == at::kBFloat16 && w_hh.scalar_type() == at::kBFloat16 && bias.scalar_type() == at::kFloat &&
-              bias.is_contiguous(), "lstm_layer takes bf16 weights and an fp32 bias");
+  TORCH_CHECK(x.dim() == 3 && w_ih.dim() == 2 && w_hh.dim() == 2, "lstm_layer: takes a 3-D input and 2-D weights, not ", x.sizes(), ", ",
+              w_ih.sizes(), " and ", w_hh.sizes());
+  const int64_t h = w_hh.size(1);
+  TORCH_CHECK(w_hh.size(0) == 4 * h && w_ih.size(0) == 4 * h && w_ih.size(1) == x.size(2), "lstm_layer: weights ", w_ih.sizes(), " and ",
+              w_hh.sizes(), " for an input of ", x.sizes());
+  TORCH_CHECK(x.size(1) % 8 == 0 && x.size(2) % 8 == 0 && h % 8 == 0, "lstm_layer: takes multiples of 8");
+  check_operand("lstm_layer", "the input", x, x, at::kBFloat16);
+  check_operand("lstm_layer", "the input weight", w_ih, x, at::kBFloat16);
+  check_operand("lstm_layer", "the recurrent weight", w_hh, x, at::kBFloat16);
+  check_vector("lstm_layer", "the bias", bias, x, 4 * h);
   Sink s_ih = find_sink(w_ih), s_hh = find_sink(w_hh), s_b = find_sink(bias);
   sink_use(s_ih);
   sink_use(s_hh);

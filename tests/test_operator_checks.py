@@ -1,0 +1,123 @@
+"""The operators refuse operands that do not fit one another before a kernel is given their pointers."""
+import pytest
+import torch
+
+from eagersgd_b200 import _build
+
+BF16, F32 = torch.bfloat16, torch.float32
+
+
+def _t(*shape, dtype=BF16, device="cpu"):
+    t = torch.zeros(*shape, dtype=dtype, device=device)
+    return t.contiguous(memory_format=torch.channels_last) if t.dim() == 4 else t
+
+
+# operator -> (arguments that fit, made for a device; name of an argument -> what does not fit in its place)
+def _linear(d):
+    return dict(x=_t(16, 32, device=d), w=_t(24, 32, device=d), b=_t(24, device=d))
+
+
+def _conv1x1(d):
+    return dict(x=_t(2, 16, 8, 8, device=d), w=_t(24, 16, 1, 1, device=d))
+
+
+def _conv3x3(d):
+    return dict(x=_t(2, 16, 8, 8, device=d), w=_t(16, 16, 3, 3, device=d))
+
+
+def _stem(d):
+    return dict(x=_t(2, 3, 8, 8, device=d), w=_t(16, 3, 3, 3, device=d))
+
+
+def _eval(d):
+    return dict(x=_t(2, 16, 8, 8, device=d), w=_t(16, 16, 3, 3, device=d), coef=_t(32, dtype=F32, device=d),
+                residual=_t(2, 16, 8, 8, device=d))
+
+
+def _bn(d):
+    return dict(y=_t(2, 16, 4, 4, device=d), gamma=_t(16, dtype=F32, device=d), beta=_t(16, dtype=F32, device=d),
+                res=_t(2, 16, 4, 4, device=d), rm=_t(16, dtype=F32, device=d), rv=_t(16, dtype=F32, device=d),
+                stats=_t(2, 16, dtype=F32, device=d))
+
+
+def _ce(d):
+    return dict(logits=_t(8, 10, dtype=F32, device=d), labels=torch.zeros(8, dtype=torch.int64, device=d))
+
+
+def _lstm(d):
+    return dict(x=_t(3, 8, 16, device=d), w_ih=_t(32, 16, device=d), w_hh=_t(32, 8, device=d), bias=_t(32, dtype=F32, device=d))
+
+
+def _call(op, a):
+    e = _build.load_torch()
+    if op is _linear:
+        return e.linear(a["x"], a["w"], a["b"])
+    if op is _eval:
+        return e.conv_bn_eval(a["x"], a["w"], 1, 1, a["coef"], a["residual"], True, True)
+    if op is _bn:
+        return e.bn_act(a["y"], a["gamma"], a["beta"], a["res"], a["rm"], a["rv"], 0.1, True, a["stats"])
+    if op is _ce:
+        return e.softmax_ce(a["logits"], a["labels"])
+    if op is _lstm:
+        return e.lstm_layer(a["x"], a["w_ih"], a["w_hh"], a["bias"])
+    return e.conv2d(a["x"], a["w"], 1, a["w"].shape[2] // 2, True, False, True)
+
+
+MISFITS = [
+    (_linear, "w", lambda d: _t(24, 16, device=d)), (_linear, "w", lambda d: _t(24, 40, device=d)),
+    (_linear, "x", lambda d: _t(16, 32, 8, device=d)), (_linear, "x", lambda d: _t(16, 32, dtype=F32, device=d)),
+    (_linear, "b", lambda d: _t(16, device=d)),
+    (_conv1x1, "w", lambda d: _t(24, 8, 1, 1, device=d)), (_conv1x1, "w", lambda d: _t(24, 24, 1, 1, device=d)),
+    (_conv1x1, "w", lambda d: _t(24, 16, 1, 1, dtype=F32, device=d)),
+    (_conv3x3, "w", lambda d: _t(16, 8, 3, 3, device=d)), (_conv3x3, "w", lambda d: _t(16, 16, 3, 3, dtype=F32, device=d)),
+    (_stem, "w", lambda d: _t(16, 1, 3, 3, device=d)), (_stem, "w", lambda d: _t(16, 3, 3, 3, dtype=F32, device=d)),
+    (_eval, "w", lambda d: _t(16, 32, 3, 3, device=d)), (_eval, "coef", lambda d: _t(16, dtype=F32, device=d)),
+    (_eval, "residual", lambda d: _t(2, 16, 4, 4, device=d)), (_eval, "residual", lambda d: _t(2, 16, 8, 8, dtype=F32, device=d)),
+    (_bn, "gamma", lambda d: _t(8, dtype=F32, device=d)), (_bn, "beta", lambda d: _t(16, device=d)),
+    (_bn, "res", lambda d: _t(1, 16, 4, 4, device=d)), (_bn, "rm", lambda d: _t(8, dtype=F32, device=d)),
+    (_bn, "rv", lambda d: _t(16, device=d)), (_bn, "stats", lambda d: _t(16, dtype=F32, device=d)),
+    (_ce, "labels", lambda d: torch.zeros(7, dtype=torch.int64, device=d)), (_ce, "logits", lambda d: _t(8, 10, 2, dtype=F32, device=d)),
+    (_lstm, "w_ih", lambda d: _t(32, 8, device=d)), (_lstm, "w_hh", lambda d: _t(64, 8, device=d)),
+    (_lstm, "w_hh", lambda d: _t(32, 16, device=d)), (_lstm, "bias", lambda d: _t(8, dtype=F32, device=d)),
+    (_lstm, "x", lambda d: _t(24, 16, device=d)),
+]
+NAMES = {_linear: "linear", _ce: "softmax_ce", _lstm: "lstm_layer", _bn: "bn_act"}
+
+
+def _refuses(op, name, misfit, device):
+    a = dict(op(device))
+    a[name] = misfit(device)
+    with pytest.raises(RuntimeError, match="^%s: " % NAMES.get(op, "conv2d")):      # the operator's own words
+        _call(op, a)
+
+
+@pytest.mark.parametrize("op,name,misfit", MISFITS)
+def test_operands_that_do_not_fit_are_refused(op, name, misfit):
+    _refuses(op, name, misfit, "cpu")
+
+
+@pytest.mark.parametrize("stride,pad", [(0, 1), (-1, 1), (1, -1)])
+def test_no_kernel_for_a_stride_or_padding_that_is_none(stride, pad):
+    a = _conv3x3("cpu")
+    assert _build.load_torch().conv2d(a["x"], a["w"], stride, pad, False, False, True) is None
+
+
+def test_a_filter_larger_than_the_padded_image_is_refused():
+    with pytest.raises(RuntimeError, match="conv2d: the filter"):
+        _build.load_torch().conv2d(_t(2, 16, 2, 8), _t(16, 16, 3, 3), 1, 0, False, False, True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", sorted({m[0] for m in MISFITS}, key=lambda f: f.__name__))
+def test_the_same_on_the_gpu(op):
+    d = "cuda:0"
+    assert _call(op, op(d)) is not None
+    for o, name, misfit in MISFITS:
+        if o is op:
+            _refuses(op, name, misfit, d)
+            a = dict(op(d))
+            a[name] = op("cpu")[name]              # an operand on another device than the input
+            with pytest.raises(RuntimeError):
+                _call(op, a)
+    torch.cuda.synchronize()
+    assert _call(op, op(d)) is not None
