@@ -348,7 +348,7 @@ extern "C" {
 
 // sum / sqsum must be zeroed by the caller (they accumulate).
 int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, void* stream) {
-  if (C % 8) return -1;
+  if (C < 8 || C % 8) return -1;
   const Map mp = make_map(C);
   return esgd::launch(bn_stats_kernel, grid_for(mp, M, kStatsBlocks), 256, 0, stream, (const __nv_bfloat16*)y, M, C, mp, sum, sqsum);
 }
@@ -358,7 +358,7 @@ int esgd_bn_stats(const void* y, int64_t M, int C, float* sum, float* sqsum, voi
 int esgd_bn_fwd(const void* y, const void* residual, void* z, void* mask, const float* sum, const float* sqsum, const float* gamma,
                 const float* beta, float* running_mean, float* running_var, float* aux, int64_t M, int C, int relu,
                 float momentum, float eps, void* stream) {
-  if (C % 8) return -1;
+  if (C < 8 || C % 8) return -1;
   const float unbias = M > 1 ? (float)M / (float)(M - 1) : 1.0f;
   const Map mp = make_map(C);
   auto kernel = residual != nullptr ? bn_fwd_kernel<true> : bn_fwd_kernel<false>;
@@ -376,7 +376,7 @@ int esgd_bn_coefficients(const void* layers, int n, float eps, void* stream) {
 // scale / shift.
 int esgd_bn_bwd_reduce(const void* dz, const void* mask, const void* y, const float* aux, int64_t M, int C, int mode, float* dbeta,
                        float* dgamma, void* stream) {
-  if (C % 8 || mode < 0 || mode > 2 || (mode == 1 && mask == nullptr)) return -1;
+  if (C < 8 || C % 8 || mode < 0 || mode > 2 || (mode == 1 && mask == nullptr)) return -1;
   const Map mp = make_map(C);
   auto kernel = mode == 0 ? bn_bwd_reduce_kernel<0> : (mode == 1 ? bn_bwd_reduce_kernel<1> : bn_bwd_reduce_kernel<2>);
   return esgd::launch(kernel, grid_for(mp, M, reduce_blocks(mode)), 256, 0, stream, (const __nv_bfloat16*)dz, (const uint8_t*)mask,
@@ -388,7 +388,7 @@ int esgd_bn_bwd_reduce(const void* dz, const void* mask, const void* y, const fl
 int esgd_bn_bwd_apply(const void* dz, const void* mask, const void* y, const float* aux, const float* gamma, const float* dbeta,
                       const float* dgamma, void* dy, void* dres, int64_t M, int C, int mode, int last_first, float* acc_dgamma,
                       float* acc_dbeta, void* stream) {
-  if (C % 8 || mode < 0 || mode > 2 || (mode == 1 && mask == nullptr)) return -1;
+  if (C < 8 || C % 8 || mode < 0 || mode > 2 || (mode == 1 && mask == nullptr)) return -1;
   const Map mp = make_map(C);
   auto kernel = dres != nullptr ? (mode == 0 ? bn_bwd_apply_kernel<0, true> : mode == 1 ? bn_bwd_apply_kernel<1, true> : bn_bwd_apply_kernel<2, true>)
                                 : (mode == 0 ? bn_bwd_apply_kernel<0, false> : mode == 1 ? bn_bwd_apply_kernel<1, false> : bn_bwd_apply_kernel<2, false>);

@@ -316,8 +316,9 @@ __global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS) wgrad_narrow_kerne
   }
 }
 
-// Tiles of about `target` pixels: whole rows of an image, or whole images when they are small.
+// Tiles of about `target` pixels: whole rows of an image, or whole images when they are small.  False: there is nothing to tile.
 bool plan(Shape& s, int N, int H, int W, int stride, int target, int min_tiles) {
+  if (N < 1 || H < 1 || W < 1 || stride < 1) return false;
   s.N = N; s.H = H; s.W = W; s.stride = stride;
   s.Ho = (H + 2 - 3) / stride + 1;
   s.Wo = (W + 2 - 3) / stride + 1;
@@ -361,7 +362,7 @@ template <int CR, int CN, bool kT>
 int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t stream) {
   static Occupancy occ;
   Shape s;
-  plan(s, N, H, W, stride, 256, 148);
+  if (!plan(s, N, H, W, stride, 256, 148)) return -1;
   const int cin = kT ? CN : CR, cout = kT ? CR : CN;
   const int smem = 9 * cout * (cin * 2 + 16) + s.ti * s.rows * s.pw * (CR * 2 + 16);
   if (smem > kSmemMax) return -100;
@@ -373,7 +374,7 @@ template <int CI, int CO>
 int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int stride, cudaStream_t stream) {
   static Occupancy occ;
   Shape s;
-  plan(s, N, H, W, stride, 256, 148);
+  if (!plan(s, N, H, W, stride, 256, 148)) return -1;
   const int px = (s.ti * s.tr * s.Wo + 15) / 16 * 16;
   int smem = s.ti * s.rows * s.pw * (CI * 2 + 16) + px * (CO * 2 + 16);
   if (smem < CO * 9 * CI * 4) smem = CO * 9 * CI * 4;

@@ -1,0 +1,25 @@
+"""A launcher that is given an empty problem answers with an error code.  Each call runs in a process of its own: an integer
+division by zero ends it."""
+import subprocess
+import sys
+
+import pytest
+
+from eagersgd_b200 import _build
+
+# launcher, arguments of a small problem (pointers as text), position of the size that is set to zero
+_P = "C.c_void_p(0)"
+EMPTY = [("esgd_conv_narrow_fwd", [_P] * 3 + [2, 8, 8, 64, 64, 1] + [_P] * 3 + [0] + [_P] * 3, (3, 4, 5, 8)),
+         ("esgd_conv_narrow_fwd", [_P] * 3 + [2, 32, 32, 16, 16, 1] + [_P] * 3 + [0] + [_P] * 3, (3, 4, 5, 8)),
+         ("esgd_conv_narrow_dgrad", [_P] * 3 + [2, 8, 8, 64, 64] + [_P] * 3, (3, 4, 5)),
+         ("esgd_conv_narrow_wgrad", [_P] * 3 + [2, 8, 8, 32, 64, 1, _P], (3, 4, 5, 8)),
+         ("esgd_bn_stats", [_P, "C.c_int64(64)", 8] + [_P] * 3, (2,)),
+         ("esgd_bn_fwd", [_P] * 11 + ["C.c_int64(64)", 8, 1, "C.c_float(0.1)", "C.c_float(1e-5)", _P], (12,))]
+
+
+@pytest.mark.parametrize("fn,args,zero", [(f, a, z) for f, a, zs in EMPTY for z in zs])
+def test_an_empty_problem_is_an_error_code_and_not_the_end_of_the_process(fn, args, zero):
+    args = [str(0 if i == zero else a) for i, a in enumerate(args)]
+    code = "import ctypes as C\nprint(C.CDLL(%r).%s(%s))" % (_build.build_cuda(), fn, ", ".join(args))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and int(r.stdout) < 0, (r.returncode, r.stdout, r.stderr[-300:])
