@@ -345,6 +345,9 @@ bool plan(Shape& s, int N, int H, int W, int stride, int target, int min_tiles) 
 
 constexpr int kSmemMax = 200 * 1024;
 
+// Every load of an operand is 16 bytes wide (cp.async).
+bool aligned16(const void* a, const void* b) { return (((uintptr_t)a | (uintptr_t)b) & 15) == 0; }
+
 // Resident blocks per SM (kept per kernel for the newest shared-memory size; a layer's is always the same).
 struct Occupancy { std::atomic<uint64_t> last{0}; };
 template <class K>
@@ -363,6 +366,7 @@ int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t str
   static Occupancy occ;
   Shape s;
   if (!plan(s, N, H, W, stride, 256, 148)) return -1;
+  if (!aligned16(a.x, a.w)) return -100;
   const int cin = kT ? CN : CR, cout = kT ? CR : CN;
   const int smem = 9 * cout * (cin * 2 + 16) + s.ti * s.rows * s.pw * (CR * 2 + 16);
   if (smem > kSmemMax) return -100;
@@ -375,6 +379,7 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
   static Occupancy occ;
   Shape s;
   if (!plan(s, N, H, W, stride, 256, 148)) return -1;
+  if (!aligned16(x, dy)) return -100;
   const int px = (s.ti * s.tr * s.Wo + 15) / 16 * 16;
   int smem = s.ti * s.rows * s.pw * (CI * 2 + 16) + px * (CO * 2 + 16);
   if (smem < CO * 9 * CI * 4) smem = CO * 9 * CI * 4;

@@ -83,7 +83,11 @@ constexpr float kBnEps = 1e-5f;
 void ck(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed with code ", rc); }
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 float* fptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
-Tensor nhwc(const Tensor& t) { return t.contiguous(kCL); }
+// The kernels load 16 bytes at a time and TMA starts on 16 bytes: a tensor that begins elsewhere (a view into a larger one) is
+// copied.
+Tensor aligned(Tensor t) { return ((uintptr_t)t.data_ptr() & 15) ? t.clone() : t; }
+Tensor nhwc(const Tensor& t) { return aligned(t.contiguous(kCL)); }
+Tensor dense(const Tensor& t) { return aligned(t.contiguous()); }
 Tensor empty_nhwc(int64_t n, int64_t c, int64_t h, int64_t w, const Tensor& like) {
   return at::empty({n, c, h, w}, like.options(), kCL);
 }
@@ -410,7 +414,7 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
   const int64_t ho = y.size(2), wo = y.size(3);
   void* st = stream_of(x);
   if (kind == kOneByOne) {
-    *filters = w.contiguous();                      // [Cout, Cin]: a 1x1 filter has one memory order
+    *filters = dense(w);                            // [Cout, Cin]: a 1x1 filter has one memory order
     *kept = x;
     if (stride == 2) {
       *kept = empty_nhwc(n, cin, ho, wo, x);
@@ -764,7 +768,7 @@ struct LinearFn : public Function<LinearFn> {
                         const Sink& ws, const Sink& bs, const c10::optional<Tensor>& anchor) {
     const Tensor b = b_in.has_value() ? *b_in : Tensor();
     c10::cuda::CUDAGuard guard(x_in.device());
-    Tensor x = x_in.contiguous(), w = w_in.contiguous();
+    Tensor x = dense(x_in), w = dense(w_in);
     const int64_t m = x.size(0), k = x.size(1), n = w.size(0), np = (n + 7) / 8 * 8;
     Tensor y = at::empty({m, np}, x.options().dtype(at::kFloat));
     Tensor bias = b.defined() ? b.contiguous() : Tensor();
@@ -1064,7 +1068,7 @@ struct AvgPoolFn : public Function<AvgPoolFn> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto d = ctx->saved_data["dims"].toIntVector();
-    Tensor dy = grads[0].contiguous();
+    Tensor dy = dense(grads[0]);
     c10::cuda::CUDAGuard guard(dy.device());
     Tensor dx = empty_nhwc(d[0], d[1], d[2], d[3], dy);
     ck(esgd_avgpool_bwd(dy.data_ptr(), dx.data_ptr(), d[0], d[2] * d[3], d[1], stream_of(dy)), "avgpool backward");
@@ -1081,7 +1085,7 @@ struct LstmFn : public Function<LstmFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w_ih_in, const Tensor& w_hh_in, const Tensor& bias,
                         const Sink& s_ih, const Sink& s_hh, const Sink& s_b, const c10::optional<Tensor>& anchor) {
     c10::cuda::CUDAGuard guard(x_in.device());
-    Tensor x = x_in.contiguous(), w_ih = w_ih_in.contiguous(), w_hh = w_hh_in.contiguous();
+    Tensor x = dense(x_in), w_ih = dense(w_ih_in), w_hh = dense(w_hh_in);
     const int64_t t = x.size(0), b = x.size(1), in = x.size(2), h = w_hh.size(1);
     void* st = stream_of(x);
     const auto f32 = x.options().dtype(at::kFloat);
@@ -1130,7 +1134,7 @@ struct LstmFn : public Function<LstmFn> {
     Sink s_ih = load_sink(ctx, "ih"), s_hh = load_sink(ctx, "hh"), s_b = load_sink(ctx, "b");
     const auto f32 = x.options().dtype(at::kFloat);
     void* st = stream_of(x);
-    Tensor dy = grads[0].contiguous();
+    Tensor dy = dense(grads[0]);
     Tensor dG = at::empty({t * b, 4 * h}, x.options());
     Tensor dx, dw_ih, dw_hh, db;
     const bool need_b = s_b || ctx->needs_input_grad(3);

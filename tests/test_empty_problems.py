@@ -1,5 +1,5 @@
-"""A launcher that is given an empty problem answers with an error code.  Each call runs in a process of its own: an integer
-division by zero ends it."""
+"""A launcher that is given an empty problem, or an operand that its loads cannot start at, answers with an error code.  Each
+call runs in a process of its own: an integer division by zero ends it."""
 import subprocess
 import sys
 
@@ -23,3 +23,12 @@ def test_an_empty_problem_is_an_error_code_and_not_the_end_of_the_process(fn, ar
     code = "import ctypes as C\nprint(C.CDLL(%r).%s(%s))" % (_build.build_cuda(), fn, ", ".join(args))
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and int(r.stdout) < 0, (r.returncode, r.stdout, r.stderr[-300:])
+
+
+@pytest.mark.parametrize("fn,args", [(f, a) for f, a, _ in EMPTY if "narrow" in f])
+def test_an_operand_that_is_not_aligned_is_left_to_another_kernel(fn, args):
+    args = [str(a) for a in args]
+    args[0] = "C.c_void_p(4098)"                   # 16-byte loads would start there
+    code = "import ctypes as C\nprint(C.CDLL(%r).%s(%s))" % (_build.build_cuda(), fn, ", ".join(args))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and int(r.stdout) == -100, (r.returncode, r.stdout, r.stderr[-300:])

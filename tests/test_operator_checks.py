@@ -121,3 +121,61 @@ def test_the_same_on_the_gpu(op):
                 _call(op, a)
     torch.cuda.synchronize()
     assert _call(op, op(d)) is not None
+
+
+def _shifted(t, by=1):
+    """The same values in memory that starts ``by`` elements past an aligned address."""
+    flat = torch.empty(t.numel() + 16, dtype=t.dtype, device=t.device)[by:by + t.numel()]
+    v = flat.as_strided(t.size(), t.stride())
+    v.copy_(t)
+    assert v.data_ptr() % 16
+    return v
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["input", "weight", "gradient"])
+@pytest.mark.parametrize("cin,cout,k,stride", [(16, 16, 3, 1), (32, 32, 3, 1), (64, 64, 3, 1), (16, 32, 3, 2), (128, 64, 3, 1), (64, 128, 1, 1),
+                                               (64, 64, 1, 2), (3, 16, 3, 1)])
+def test_convolutions_take_tensors_that_start_anywhere(cin, cout, k, stride, what):
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(cin + cout + k)
+    x, w = torch.randn(3, cin, 8, 8, generator=g), torch.randn(cout, cin, k, k, generator=g)
+    cl = lambda t: t.cuda().bfloat16().contiguous(memory_format=torch.channels_last)
+    x, w = cl(x), cl(w)
+    dy = cl(torch.randn(3, cout, (8 - 1) // stride + 1, (8 - 1) // stride + 1, generator=g))
+
+    def run(x, w, dy):
+        x, w = x.detach().requires_grad_(cin > 3), w.detach().requires_grad_()
+        y, st = ops.conv2d(x, w, stride, k // 2, want_stats=True)
+        y.backward(dy)
+        return [t.float() for t in (y.detach(), st, w.grad, x.grad) if t is not None]
+
+    ref = run(x, w, dy)
+    got = run(_shifted(x) if what == "input" else x, _shifted(w) if what == "weight" else w, _shifted(dy) if what == "gradient" else dy)
+    for a, b in zip(got, ref):
+        assert (a - b).norm() <= 1e-3 * b.norm()         # sums meet in atomics; the operands are the same
+
+
+@pytest.mark.gpu
+def test_the_other_operators_take_tensors_that_start_anywhere():
+    from eagersgd_b200.ops import functional as ops
+    from eagersgd_b200.ops.lstm import lstm_layer
+    g = torch.Generator().manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    cl = lambda t: t.bfloat16().contiguous(memory_format=torch.channels_last)
+    x4, r4, gamma, beta = cl(rnd(2, 16, 6, 6)), cl(rnd(2, 16, 6, 6)), rnd(16), rnd(16)
+    x2, w2, b2 = rnd(16, 32).bfloat16(), rnd(24, 32).bfloat16(), rnd(24).bfloat16()
+    x3, w_ih, w_hh, b3 = rnd(3, 8, 16).bfloat16(), (0.1 * rnd(512, 16)).bfloat16(), (0.1 * rnd(512, 128)).bfloat16(), rnd(512)
+    calls = [(lambda x, r, a, b: ops.bn_act(x, a, b, None, None, residual=r), (x4, r4, gamma, beta)),
+             (ops.linear, (x2, w2, b2)), (ops.max_pool_3x3_s2, (x4,)), (ops.global_avg_pool, (x4,)), (lstm_layer, (x3, w_ih, w_hh, b3))]
+    for f, args in calls:
+        def run(args, shift_dy):
+            args = [a.detach().requires_grad_() for a in args]
+            y = f(*args)
+            dy = torch.ones_like(y)
+            y.backward(_shifted(dy) if shift_dy else dy)
+            return [y.detach().float()] + [a.grad.float() for a in args]
+        ref = run(args, False)
+        for got in (run([_shifted(a) for a in args], False), run(args, True)):
+            for a, b in zip(got, ref):
+                assert (a - b).norm() <= 1e-3 * b.norm() + 1e-6
