@@ -190,8 +190,21 @@ class GradSinks;
 struct SinkEntry : torch::CustomClassHolder {
   float* acc = nullptr;          // fp32 accumulator, in the parameter's own memory order (OHWI for channels_last filters)
   int bucket = 0;
-  int uses = 0;                  // forward uses of this step whose backward has not run yet
-  bool used = false;             // took part in this step
+  c10::weak_intrusive_ptr<at::TensorImpl, at::UndefinedTensorImpl> param;
+  // of the step that is under way:
+  int uses = 0;                  // forward uses whose backward has not run yet
+  bool used = false;             // an operator writes the accumulator
+  bool recomputed = false;       // used inside a backward pass (checkpointing): there may be another such use to come
+  bool hooked = false;           // autograd has written .grad
+  bool counted = false;          // taken off its bucket's count
+  explicit SinkEntry(const Tensor& p) : param(p.getIntrusivePtr()) {}
+  // Autograd may still add to .grad: the parameter is in a graph, too, and its accumulation has not run.
+  bool awaited() const {
+    if (recomputed) return true;
+    if (hooked || !used) return false;
+    const auto p = param.lock();
+    return p.defined() && torch::autograd::impl::try_get_grad_accumulator(Tensor(p)) != nullptr;
+  }
   std::atomic<GradSinks*> owner{nullptr};
 };
 using Sink = c10::intrusive_ptr<SinkEntry>;
@@ -202,7 +215,7 @@ std::unordered_map<at::TensorImpl*, Sink> g_sinks;
 class GradSinks {
  public:
   GradSinks(std::vector<int> params_per_bucket, py::function on_bucket)
-      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), on_bucket_(std::move(on_bucket)) {}
+      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), complete_(total_.size(), 0), on_bucket_(std::move(on_bucket)) {}
   ~GradSinks() {
     close();
     if (side_) {
@@ -217,7 +230,7 @@ class GradSinks {
   }
   void add(const Tensor& param, const Tensor& acc, int bucket) {
     TORCH_CHECK(acc.scalar_type() == at::kFloat && acc.numel() == param.numel());
-    auto e = c10::make_intrusive<SinkEntry>();
+    auto e = c10::make_intrusive<SinkEntry>(param);
     e->acc = acc.data_ptr<float>();
     e->bucket = bucket;
     e->owner.store(this);
@@ -227,7 +240,12 @@ class GradSinks {
   }
   void begin_step() {
     pending_ = total_;
-    for (auto& kv : mine_) { kv.second->uses = 0; kv.second->used = false; }
+    std::fill(complete_.begin(), complete_.end(), 0);
+    for (auto& kv : mine_) {
+      SinkEntry& e = *kv.second;
+      e.uses = 0;
+      e.used = e.recomputed = e.hooked = e.counted = false;
+    }
   }
   void set_active(bool on) {
     if (!on) join();
@@ -268,16 +286,34 @@ class GradSinks {
   bool written(int bucket) const { return written_[bucket] != 0; }
   void clear_written() { std::fill(written_.begin(), written_.end(), 0); }
   void mark_written(int bucket) { written_[bucket] = 1; }
-  void param_done(int bucket) {
-    if (--pending_[bucket] == 0) {
-      join();
-      py::gil_scoped_acquire gil;
-      on_bucket_(bucket);
+  // A parameter's gradient is complete once its operators' backward passes have run and, where autograd writes it as well,
+  // that has happened, too; it is counted once whichever comes last.
+  void sink_ready(SinkEntry& e) {
+    if (!e.counted) {
+      e.counted = true;
+      --pending_[e.bucket];
     }
+    settle(e.bucket);
+  }
+  void hooked(const Tensor& param) {
+    auto it = mine_.find(param.unsafeGetTensorImpl());
+    if (it == mine_.end()) return;
+    it->second->hooked = true;
+    if (it->second->uses == 0) sink_ready(*it->second);
   }
 
  private:
-  std::vector<int> total_, pending_, written_;
+  // Announces a bucket whose every gradient is there; one with a parameter that may still get more goes with the step.
+  void settle(int bucket) {
+    if (pending_[bucket] > 0 || complete_[bucket]) return;
+    for (auto& kv : mine_)
+      if (kv.second->bucket == bucket && kv.second->awaited()) return;
+    complete_[bucket] = 1;
+    join();
+    py::gil_scoped_acquire gil;
+    on_bucket_(bucket);
+  }
+  std::vector<int> total_, pending_, written_, complete_;
   std::atomic<bool> active_{false};
   py::function on_bucket_;
   c10::optional<c10::cuda::CUDAStream> side_;
@@ -298,7 +334,10 @@ Sink find_sink(const Tensor& p) {
 }
 // Called in an operator's forward for a parameter that its backward will write.
 void sink_use(const Sink& s) {
-  if (s) { ++s->uses; s->used = true; }
+  if (!s) return;
+  ++s->uses;
+  s->used = true;
+  if (torch::autograd::get_current_graph_task_id() != -1) s->recomputed = true;
 }
 // The parameter as the operator's autograd input: detached when a sink takes its gradient, so that autograd neither
 // expects one nor calls the parameter's hooks.
@@ -324,7 +363,7 @@ void sink_done(const Sink& s) {
   GradSinks* o = s->owner.load();
   if (o == nullptr || s->uses <= 0) return;
   o->mark_written(s->bucket);
-  if (--s->uses == 0) o->param_done(s->bucket);
+  if (--s->uses == 0) o->sink_ready(*s);
 }
 void save_sink(AutogradContext* ctx, const char* key, const Sink& s) {
   if (s) ctx->saved_data[key] = c10::IValue::make_capsule(s);
@@ -1229,6 +1268,6 @@ PYBIND11_MODULE(_esgd_torch, m) {
       .def("active", &GradSinks::active)
       .def("used", &GradSinks::used)
       .def("written", &GradSinks::written)
-      .def("param_done", &GradSinks::param_done)
+      .def("hooked", &GradSinks::hooked)
       .def("close", &GradSinks::close);
 }

@@ -108,7 +108,7 @@ class EagerOptimizer:
         self.slot_dtype = slot_dtype
         self._build_buckets(bucket_mb)
         self._hooks = []
-        self._sinks, self._sinks_proven, self._sinks_conflict = None, False, False
+        self._sinks, self._sinks_conflict = None, False
         if self.on_gpu:
             self._setup_gpu()
             self._install_hooks()
@@ -312,7 +312,7 @@ class EagerOptimizer:
             if self._sinks is not None and self._sinks.active():
                 if self._sinks.used(p):          # one parameter, two routes: see grad_sinks
                     self._sinks_conflict = True
-                self._sinks.param_done(b.index)
+                self._sinks.hooked(p)
                 return
             b.pending -= 1
             if b.pending == 0 and self.overlap:
@@ -343,7 +343,9 @@ class EagerOptimizer:
         """Around the forward and backward pass of a training step: operators of this package add the gradients of their
         parameters straight to fp32 accumulators of the buckets (``csrc/torch/ops.cpp``) instead of returning them to
         autograd, so those parameters' ``.grad`` stays zero and is not to be looked at before ``step()``.  Parameters that
-        carry hooks of the user's own are left to autograd."""
+        carry hooks of the user's own are left to autograd.  A parameter that autograd reaches as well (a penalty on the
+        weights beside the layer that uses them) gets both shares, and its bucket leaves only when both are there; from the
+        next step on such an optimizer leaves all of them to autograd."""
         if not self.prepare_grad_sinks():
             yield
             return
@@ -369,9 +371,7 @@ class EagerOptimizer:
 
             def on_bucket(i):
                 me = weak()
-                # A parameter that is also used outside this package's operators would get the rest of its gradient from
-                # autograd after its bucket has gone: the first step launches nothing early and finds such parameters out.
-                if me is not None and me.overlap and me._sinks_proven:
+                if me is not None and me.overlap:
                     me._launch(me.buckets[i], me.buckets[i].touched)
 
             self._sinks = _build.load_torch().GradSinks([len(b.params) for b in self.buckets], on_bucket)
@@ -422,7 +422,6 @@ class EagerOptimizer:
                 b.touched = []
             if self._sinks is not None:
                 self._sinks.clear_written()
-                self._sinks_proven = not self._sinks_conflict
             if not self.fused:
                 self._inner_step()
         else:
