@@ -225,7 +225,11 @@ class GradSinks {
   }
   void close() {
     std::unique_lock<std::shared_mutex> g(g_sink_mutex);
-    for (auto& kv : mine_) { kv.second->owner.store(nullptr); g_sinks.erase(kv.first); }
+    for (auto& kv : mine_) {
+      kv.second->owner.store(nullptr);
+      const auto it = g_sinks.find(kv.first);
+      if (it != g_sinks.end() && it->second == kv.second) g_sinks.erase(it);       // unless a later one has taken it over
+    }
     mine_.clear();
   }
   void add(const Tensor& param, const Tensor& acc, int bucket) {

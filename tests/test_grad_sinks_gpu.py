@@ -115,6 +115,22 @@ def test_a_parameter_with_a_hook_keeps_its_gradient():
     opt.close()
 
 
+def test_closing_one_of_two_owners_leaves_the_parameter_to_the_other():
+    from eagersgd_b200 import _build
+    (w,) = _layers(3, 1)
+    owners = [_build.load_torch().GradSinks([1], lambda i: None) for _ in range(2)]
+    accs = [torch.zeros(w.numel(), device="cuda") for _ in owners]
+    for o, acc in zip(owners, accs):
+        o.add(w, acc, 0)
+    owners[0].close()
+    owners[1].begin_step()
+    owners[1].set_active(True)
+    _mlp(torch.ones(32, 64, device="cuda", dtype=torch.bfloat16), [w]).backward()
+    owners[1].set_active(False)
+    assert w.grad is None and bool(accs[1].any()) and not bool(accs[0].any()) and owners[1].used(w)
+    owners[1].close()
+
+
 def test_steps_with_the_weight_gradients_on_a_stream_of_their_own():
     """The same network captured (the weight gradients of all its convolutions go to the side stream) and not (none does)."""
     import eagersgd_b200 as es
