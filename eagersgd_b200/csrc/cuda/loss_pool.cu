@@ -395,29 +395,32 @@ __global__ void __launch_bounds__(256) stem_unpack_kernel(const float* __restric
 }
 
 // Gradient of a dense layer's fp32 output: bf16 copy with the row padded to np columns (zeros), and its column sums in the
-// same pass (dy is read once).  A thread keeps four columns and walks down the rows of its block.
+// same pass (dy is read once).  A thread keeps four columns and walks down the rows of its block; a grid has 65,535 blocks
+// of rows, and beyond a million rows they go round.
 constexpr int kCastRows = 16;      // rows of a block: short enough that a small batch is not one serial chain of loads
 __global__ void __launch_bounds__(256) cast_colsum_kernel(const float* __restrict__ dy, int64_t ld, int M, int N, int np,
                                                           __nv_bfloat16* __restrict__ out, float* __restrict__ colsum, int vec) {
   pdl_enter();
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= np) return;
-  const int r0 = blockIdx.y * kCastRows, r1 = min(M, r0 + kCastRows);
   float s[4] = {0, 0, 0, 0};
+  for (int64_t r0 = (int64_t)blockIdx.y * kCastRows; r0 < M; r0 += (int64_t)gridDim.y * kCastRows) {
+    const int r1 = (int)min((int64_t)M, r0 + kCastRows);
 #pragma unroll 8
-  for (int r = r0; r < r1; ++r) {
-    float v[4];
-    if (vec && c + 4 <= N) {
-      const float4 f = __ldcs(reinterpret_cast<const float4*>(dy + r * ld + c));
-      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-    } else {
+    for (int r = (int)r0; r < r1; ++r) {
+      float v[4];
+      if (vec && c + 4 <= N) {
+        const float4 f = __ldcs(reinterpret_cast<const float4*>(dy + r * ld + c));
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = c + q < N ? dy[r * ld + c + q] : 0.0f;
+        for (int q = 0; q < 4; ++q) v[q] = c + q < N ? dy[r * ld + c + q] : 0.0f;
+      }
+      __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+      *reinterpret_cast<uint2*>(out + (int64_t)r * np + c) = *reinterpret_cast<const uint2*>(h);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] += v[q];
     }
-    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
-    *reinterpret_cast<uint2*>(out + (int64_t)r * np + c) = *reinterpret_cast<const uint2*>(h);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) s[q] += v[q];
   }
   if (colsum != nullptr) {
 #pragma unroll
@@ -509,7 +512,8 @@ int esgd_stem_unpack(const float* col, void* dw, float* acc, int Cout, int R, in
 int esgd_cast_colsum(const float* dy, int64_t ld, int M, int N, int np, void* out, float* colsum, void* stream) {
   if (np % 8 || np < N) return -1;
   const int vec = ld % 4 == 0 && ((uintptr_t)dy & 15) == 0;
-  dim3 grid((np / 4 + 255) / 256, (M + kCastRows - 1) / kCastRows);
+  const int row_blocks = M / kCastRows + (M % kCastRows != 0);
+  dim3 grid((np / 4 + 255) / 256, row_blocks < 65535 ? row_blocks : 65535);
   return esgd::launch(cast_colsum_kernel, grid, 256, 0, stream, dy, ld, M, N, np, (__nv_bfloat16*)out, colsum, vec);
 }
 

@@ -179,3 +179,19 @@ def test_the_other_operators_take_tensors_that_start_anywhere():
         for got in (run([_shifted(a) for a in args], False), run(args, True)):
             for a, b in zip(got, ref):
                 assert (a - b).norm() <= 1e-3 * b.norm() + 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [65535 * 16, 65535 * 16 + 1, 2 * 65535 * 16 + 17])
+def test_linear_over_more_rows_than_a_grid_has_blocks(rows):
+    """The gradient of a dense layer over a million rows and more; its bias gradient is the column sum."""
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, 8, device="cuda", generator=g).bfloat16().requires_grad_()
+    w, b = torch.randn(10, 8, device="cuda", generator=g).bfloat16().requires_grad_(), torch.zeros(10, device="cuda").requires_grad_()
+    dy = torch.randn(rows, 10, device="cuda", generator=g)
+    ops.linear(x, w, b).backward(dy)
+    dy16 = dy.bfloat16().double()
+    for got, ref, tol in ((x.grad, dy16 @ w.detach().double(), 4e-3), (w.grad, dy16.t() @ x.detach().double(), 4e-3),
+                          (b.grad, dy.double().sum(0), 1e-4)):
+        assert (got.double() - ref).norm() <= tol * ref.norm()      # one bf16 rounding; fp32 sums of a million terms
