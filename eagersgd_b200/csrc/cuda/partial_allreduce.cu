@@ -280,8 +280,9 @@ void esgd_collective_destroy(void* h) {
   if (c->done) cudaEventDestroy(c->done);
   delete c;
 }
-// Launch a step on the side stream behind what `stream` holds so far.
-int esgd_collective_post(void* h, void* stream) {
+// Launch a step on the side stream behind what `stream` holds so far.  hold: `stream` goes on once the step has completed, so
+// that what it does to the tensor next comes after the step's reads (for a step that waits for nobody: a world of one rank).
+int esgd_collective_post(void* h, void* stream, int hold) {
   esgd_collective* c = (esgd_collective*)h;
   cudaError_t e = cudaEventRecord(c->ready, (cudaStream_t)stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ready, 0);
@@ -289,7 +290,9 @@ int esgd_collective_post(void* h, void* stream) {
   int rc = c->local ? esgd_channel_step_local(c->dch, c->count, c->max_blocks, SRC_FLAT, c->side)
                     : esgd_channel_step(c->dch, c->count, c->max_blocks, SRC_FLAT, c->side);
   if (rc != 0) return rc;
-  return (int)cudaEventRecord(c->done, c->side);
+  e = cudaEventRecord(c->done, c->side);
+  if (e == cudaSuccess && hold) e = cudaStreamWaitEvent((cudaStream_t)stream, c->done, 0);
+  return (int)e;
 }
 // Has the posted step completed?  1 yes, 0 no, negative CUDA error code.
 int esgd_collective_test(void* h) {

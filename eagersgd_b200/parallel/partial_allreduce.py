@@ -17,6 +17,12 @@ programs that want the collective by itself.
         ...                       # overlap something
         info = ar.wait()          # info["role"], info["contributors"], ...
     ar.close()
+
+Between ``post`` and ``wait`` (or the ``test`` that succeeds) both tensors belong to the collective: on a GPU it reads the
+contribution and writes the result in place, on streams of its own.  Two cases are kinder.  A contribution on a CPU, or one on a
+GPU whose length is not a multiple of eight, is taken as it is when ``post`` is called, and work enqueued on that stream
+afterwards may overwrite it.  A result on a CPU, in bf16 or of a length that is not a multiple of eight appears only in
+``wait``, enqueued on the stream that is current there; until then ``out`` keeps what it held.
 """
 from __future__ import annotations
 
@@ -57,8 +63,8 @@ class _Collective:
         N.check_cuda(self._lib.esgd_collective_create(ch.dev_ptr, ch.count, ch.max_blocks, int(ch.local), stream.cuda_stream,
                                                       C.byref(self._h)), "collective")
 
-    def post(self, stream: int) -> None:
-        N.check_cuda(self._lib.esgd_collective_post(self._h, stream), "partial allreduce launch")
+    def post(self, stream: int, hold: bool) -> None:
+        N.check_cuda(self._lib.esgd_collective_post(self._h, stream, int(hold)), "partial allreduce launch")
         self._ch._steps += 1
 
     def test(self) -> bool:
@@ -108,12 +114,16 @@ class PartialAllreduce:
             if tensor.dtype not in (torch.float32, torch.bfloat16):
                 raise ValueError("GPU tensors must be float32 or bfloat16")
             dev = tensor.device
-            # The kernels read and write the caller's tensors directly, ragged lengths included; a tensor that does not
-            # start on 16 bytes, or a result in another type than theirs, goes through a staging buffer.
-            direct_in = tensor.data_ptr() % 16 == 0
-            direct_out = self.out.data_ptr() % 16 == 0 and self.out.dtype in (torch.float32, torch.bfloat16)
+            # The kernels read and write the caller's tensors directly where that is all a caller can expect (see the class).
+            # A ragged tensor is taken at ``post``: copied, or, where the step waits for nobody, read before the caller's
+            # stream goes on.  Ragged and 16-bit results, and tensors that do not start on 16 bytes, are staged.
+            even = n == self.count
+            direct_in = tensor.data_ptr() % 16 == 0 and (even or g.world == 1)
+            self._hold = direct_in and not even
+            direct_out = self.out.data_ptr() % 16 == 0 and even and self.out.dtype == torch.float32
+            staged = self.out.dtype if self.out.dtype in (torch.float32, torch.bfloat16) else torch.float32
             self._grad = tensor.detach().view(-1) if direct_in else torch.zeros(n, dtype=tensor.dtype, device=dev)
-            self._res = self.out.detach().view(-1) if direct_out else torch.zeros(n, dtype=torch.float32, device=dev)
+            self._res = self.out.detach().view(-1) if direct_out else torch.zeros(n, dtype=staged, device=dev)
             self._direct_out = direct_out
             self._arena, bases = create_arenas(self.count, tensor.dtype, g.rank, g.world, g.exchange)
             self._stream = torch.cuda.Stream(device=dev)
@@ -144,7 +154,8 @@ class PartialAllreduce:
         return self
 
     def post(self) -> None:
-        """Publish the tensor's current content and take part in (or miss) a round; returns at once."""
+        """Publish the tensor's current content and take part in (or miss) a round; returns at once.  The tensor is to be left
+        alone until ``wait`` (see the class for when it need not be)."""
         if not self._started:
             raise RuntimeError("start() the collective before posting")
         if self._posted:
@@ -152,7 +163,7 @@ class PartialAllreduce:
         if self.on_gpu:
             if self._grad.data_ptr() != self.tensor.data_ptr():
                 self._grad.copy_(self.tensor.view(-1))
-            self._col.post(torch.cuda.current_stream(self.tensor.device).cuda_stream)
+            self._col.post(torch.cuda.current_stream(self.tensor.device).cuda_stream, self._hold)
         else:
             src = self.tensor.detach().view(-1).numpy().copy()
 

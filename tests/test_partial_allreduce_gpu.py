@@ -537,3 +537,29 @@ def test_partial_allreduce_object_on_one_gpu(dtype, n):
         st = ar.stats()
         assert st["steps"] == 1 and st["status"] == 0 and "NVLink" in ar.describe()
     assert len(seen) == 5
+
+
+@pytest.mark.parametrize("dtype,out_dtype,n", [(torch.float32, torch.float32, 1000003), (torch.bfloat16, torch.bfloat16, 1000003),
+                                               (torch.bfloat16, torch.float32, 5), (torch.bfloat16, torch.bfloat16, 1 << 20),
+                                               (torch.float32, torch.bfloat16, 1 << 20), (torch.float32, torch.float64, 1003)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_ragged_and_16_bit_tensors_between_post_and_wait(dtype, out_dtype, n, in_place):
+    """A ragged contribution is taken at post, and a ragged or 16-bit result appears in wait."""
+    import eagersgd_b200 as es
+    if in_place and dtype != out_dtype:
+        pytest.skip("one tensor has one type")
+    src = torch.randn(n, generator=torch.Generator().manual_seed(n)).cuda().to(dtype)
+    t = torch.zeros_like(src)
+    out = t if in_place else torch.full((n,), -3.0, device="cuda", dtype=out_dtype)
+    with es.PartialAllreduce(t, es.Group(), out=out) as ar:
+        for k in range(3):
+            t.copy_(src + k)
+            want = t.to(out_dtype, copy=True)
+            held = out.clone()
+            ar.post()
+            if n % 8 and not in_place:
+                t.fill_(7.0)
+            torch.cuda.synchronize()
+            assert torch.equal(out, held)
+            assert ar.wait()["applied"]
+            assert torch.equal(out, want)
