@@ -336,7 +336,7 @@ Map make_map(int C) {
 // Four rows per thread as long as that does not fill the machine, then as many blocks as are resident.
 dim3 grid_for(const Map& m, int64_t M, int blocks_per_sm) {
   const int64_t chunks = (m.groups + m.cg - 1) / m.cg;
-  int64_t rows = (M + m.rows_par * 4 - 1) / (m.rows_par * 4), most = 148 * blocks_per_sm / chunks;
+  int64_t rows = (M + m.rows_par * 4 - 1) / (m.rows_par * 4), most = esgd::sm_count() * blocks_per_sm / chunks;
   if (most < 1) most = 1;
   if (rows > most) rows = most;
   return dim3((unsigned)(rows < 1 ? 1 : rows), (unsigned)chunks);

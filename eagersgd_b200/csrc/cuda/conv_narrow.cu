@@ -365,12 +365,12 @@ template <int CR, int CN, bool kT>
 int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t stream) {
   static Occupancy occ;
   Shape s;
-  if (!plan(s, N, H, W, stride, 256, 148)) return -1;
+  if (!plan(s, N, H, W, stride, 256, esgd::sm_count())) return -1;
   if (!aligned16(a.x, a.w)) return -100;
   const int cin = kT ? CN : CR, cout = kT ? CR : CN;
   const int smem = 9 * cout * (cin * 2 + 16) + s.ti * s.rows * s.pw * (CR * 2 + 16);
   if (smem > kSmemMax) return -100;
-  const int resident = blocks_per_sm(conv_narrow_kernel<CR, CN, kT>, kThreads, smem, occ) * 148;
+  const int resident = blocks_per_sm(conv_narrow_kernel<CR, CN, kT>, kThreads, smem, occ) * esgd::sm_count();
   return esgd::launch(conv_narrow_kernel<CR, CN, kT>, dim3(s.tiles < resident ? s.tiles : resident), kThreads, smem, stream, s, a);
 }
 
@@ -378,7 +378,7 @@ template <int CI, int CO>
 int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int stride, cudaStream_t stream) {
   static Occupancy occ;
   Shape s;
-  if (!plan(s, N, H, W, stride, 256, 148)) return -1;
+  if (!plan(s, N, H, W, stride, 256, esgd::sm_count())) return -1;
   if (!aligned16(x, dy)) return -100;
   const int px = (s.ti * s.tr * s.Wo + 15) / 16 * 16;
   int smem = s.ti * s.rows * s.pw * (CI * 2 + 16) + px * (CO * 2 + 16);
@@ -386,7 +386,7 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
   if (smem > kSmemMax) return -100;
   blocks_per_sm(wgrad_narrow_kernel<CI, CO>, WgradPlan<CI, CO>::THREADS, smem, occ);
   // one block per SM at most: every block ends with a reduction of the whole filter bank
-  const int grid = s.tiles < 148 ? s.tiles : 148;
+  const int grid = s.tiles < esgd::sm_count() ? s.tiles : esgd::sm_count();
   return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), WgradPlan<CI, CO>::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
                       (const __nv_bfloat16*)dy, dw);
 }

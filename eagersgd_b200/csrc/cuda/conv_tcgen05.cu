@@ -25,6 +25,7 @@
 #include "umma_pipeline.cuh"
 
 using namespace umma;
+using esgd::sm_count;
 
 namespace {
 
@@ -263,16 +264,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) conv_wgrad_kernel(const __grid
     tma_prefetch_desc(&prob.tmDY);
   }
   run(prob, ep);
-}
-
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n;
 }
 
 struct ConvArgs {
@@ -538,7 +529,7 @@ int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
   if (BN == 128) return launch<128, kT, kBn>(a, ep, s);
   // Pairs of CTAs (256-column tiles read each operand once for two boxes of pixels) where the reduction is full blocks:
   // 256 channels at 14 x 14 and 512 at 7 x 7, batch 256: 79 -> 65 us
-  if (a.Cin % 64 == 0 && a.Cout >= 256 && a.R * a.S * (a.Cin / 64) > 4 && a.Cout <= 74 * 256)
+  if (a.Cin % 64 == 0 && a.Cout >= 256 && a.R * a.S * (a.Cin / 64) > 4 && a.Cout <= sm_count() / 2 * 256)
     return launch<256, kT, kBn, true>(a, ep, s);
   return launch<256, kT, kBn>(a, ep, s);
 }

@@ -190,16 +190,6 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
   }
 }
 
-int wg_sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n;
-}
-
 // Geometry of a launch (host arithmetic only, shared by the launcher and by the plan query that the CPU tests
 // sweep): box sizes, stages, tap sets, pixel splits.  Returns -7 when two stages do not fit.
 int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int R, int S, int pad, int bh, int sms) {
@@ -256,7 +246,7 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
     attr_set = true;
   }
   WgHaloParams p;
-  const int pr = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, wg_sm_count());
+  const int pr = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, esgd::sm_count());
   if (pr != 0) return pr;
   p.dw = dw;
   p.error_flag = error_flag;

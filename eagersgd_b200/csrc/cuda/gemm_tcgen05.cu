@@ -15,6 +15,7 @@
 #include "umma_pipeline.cuh"
 
 using namespace umma;
+using esgd::sm_count;
 
 namespace {
 
@@ -116,16 +117,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_kernel(const __grid_const
   run<P, kBn>(prob, ep);
 }
 
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n;
-}
-
 struct GemmArgs {
   const void *A, *B;
   void* C;
@@ -209,7 +200,7 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
 // Pairs of CTAs: 256 x 256 tiles that read each operand once for both (32 KB a k-block and CTA instead of 48, five stages
 // deep instead of three).
 bool pair_applicable(int M, int N, int K, int splits) {
-  return M > BM && N > BM && K > 4 * BK && (N + 255) / 256 <= 74;
+  return M > BM && N > BM && K > 4 * BK && (N + 255) / 256 <= sm_count() / 2;
 }
 
 template <int BN>
@@ -223,6 +214,8 @@ int launch_major(int a_mn, int b_mn, const GemmArgs& g, const Epilogue& ep, cuda
 }  // namespace
 
 extern "C" {
+
+int esgd_sm_count() { return sm_count(); }
 
 // C[M,N] = A * B^T (+bias, ReLU, column statistics).  A is [M][K] (a_mn=0, row stride lda)
 // or stored [K][M] (a_mn=1); B is [N][K] (b_mn=0, row stride ldb) or stored [K][N] (b_mn=1).

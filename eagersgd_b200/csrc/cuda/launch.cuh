@@ -15,6 +15,16 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// SMs of the device; a B200's where there is none (the launchers' host arithmetic is tested without one).
+inline int sm_count() {
+  static const int count = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 0;
+    return n > 0 ? n : 148;
+  }();
+  return count;
+}
+
 // kCluster: CTAs of a cluster (along x).
 template <int kCluster = 1, class... K, class... A>
 inline int launch(void (*kernel)(K...), dim3 grid, int threads, size_t smem, void* stream, A... args) {

@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(256) cast_colsum_kernel(const float* __restric
 
 int grid_for(int64_t items) {
   int64_t b = (items + 255) / 256;
-  const int64_t cap = 148 * 16;
+  const int64_t cap = (int64_t)esgd::sm_count() * 16;
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 

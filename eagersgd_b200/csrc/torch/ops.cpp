@@ -18,6 +18,7 @@
 #include <unordered_map>
 
 extern "C" {
+int esgd_sm_count();
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn, int b_mn,
                    int out_mode, const float* scale, const void* bias, int relu, int splits, float* col_sum, float* col_sqsum,
                    const void* residual, int ldr, int* error_flag, void* stream);
@@ -389,7 +390,7 @@ int gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
 
 // Split-K factor of a weight-gradient GEMM (K = pixels): about one wave of tiles.  Each split adds a full [Cout, Cin]
 // partial result with atomics, so large filter banks take few splits.
-int wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int64_t sms = 148) {
+int wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int64_t sms) {
   const int64_t bn = cin <= 64 ? 64 : (cin <= 128 ? 128 : 256);
   const int64_t tiles = ((cout + 127) / 128) * ((cin + bn - 1) / bn);
   return (int)std::max<int64_t>(2, std::min((sms + tiles - 1) / tiles, std::max<int64_t>(1, (pixels / 64) / 8)));
@@ -563,7 +564,7 @@ struct ConvFn : public Function<ConvFn> {
         Tensor dw32;
         if (!sink) dw32 = zeros_f32({cout, cin}, x.device());
         ck(gemm(dy.data_ptr(), x.data_ptr(), sink ? sink->acc : fptr(dw32), cout, cin, m, cout, cin, cin, true, true, 2,
-                wgrad_splits(m, cout, cin), nullptr, nullptr, nullptr, 0, x), "1x1 convolution weight gradient");
+                wgrad_splits(m, cout, cin, esgd_sm_count()), nullptr, nullptr, nullptr, 0, x), "1x1 convolution weight gradient");
         if (!sink) dw = dw32.to(w.scalar_type()).view(w.sizes());
       } else if (kind == kGeneral) {
         Tensor dw32;
@@ -581,7 +582,7 @@ struct ConvFn : public Function<ConvFn> {
       } else {
         const StemGeometry g(cin, r, s);
         Tensor col = zeros_f32({cout, g.kpad}, x.device());
-        ck(gemm(dy.data_ptr(), x.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, 148, nullptr, nullptr,
+        ck(gemm(dy.data_ptr(), x.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, esgd_sm_count(), nullptr, nullptr,
                 nullptr, 0, x), "stem weight gradient");
         if (!sink) dw = at::empty(w.sizes(), w.options(), kCL);
         ck(esgd_stem_unpack(fptr(col), sink ? nullptr : dw.data_ptr(), sink ? sink->acc : nullptr, cout, r, s * cin, g.seg, g.kpad,
@@ -1156,7 +1157,7 @@ struct LstmFn : public Function<LstmFn> {
   static Tensor weight_grad(const Sink& sink, const Tensor& a, const void* ap, const Tensor& w, const void* bp, int64_t rows, int64_t m,
                             int64_t n) {
     const int64_t bn = n <= 64 ? 64 : (n <= 128 ? 128 : 256), tiles = ((m + 127) / 128) * ((n + bn - 1) / bn);
-    const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(148 / tiles, rows / 512));
+    const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(esgd_sm_count() / tiles, rows / 512));
     Tensor dw;
     if (sink || splits > 1) {
       if (!sink) dw = at::zeros({m, n}, w.options().dtype(at::kFloat));
