@@ -518,10 +518,15 @@ Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* er
   return ep;
 }
 
+// Columns of a tile (shared with the plan query below).
+int tile_width(const ConvArgs& a, int Ho, int Wo) {
+  return tile_columns(a.Cout, (int)(((int64_t)a.N * Ho * Wo + BM - 1) / BM), sm_count());
+}
+
 template <bool kT, bool kBn = false>
 int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
   const int Ho = a.out_h ? a.out_h : (a.H + 2 * a.pad - a.R) / a.stride + 1, Wo = a.out_w ? a.out_w : (a.W + 2 * a.pad - a.S) / a.stride + 1;
-  const int BN = tile_columns(a.Cout, (int)(((int64_t)a.N * Ho * Wo + BM - 1) / BM), sm_count());
+  const int BN = tile_width(a, Ho, Wo);
   int bh = 0;
   if (a.Cout <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
     return BN == 64 ? launch_halo<64, kT, kBn>(a, ep, bh, s) : launch_halo<128, kT, kBn>(a, ep, bh, s);
@@ -608,9 +613,9 @@ void esgd_conv2d_halo_plan(int N, int H, int W, int Cin, int Cout, int R, int S,
   for (int i = 0; i < 10; ++i) out[i] = 0;
   if (Cin % 8 || Cout % 8) return;
   ConvArgs a{nullptr, nullptr, nullptr, N, H, W, Cin, Cout, R, S, stride, pad};
-  const int BN = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
+  const int BN = stride == 1 ? tile_width(a, H + 2 * pad - R + 1, W + 2 * pad - S + 1) : 0;
   int bh = 0;
-  if (BN > 128 || stride != 1 || !halo_applicable(a, H + 2 * pad - R + 1, W + 2 * pad - S + 1, &bh)) return;
+  if (Cout > 128 || stride != 1 || !halo_applicable(a, H + 2 * pad - R + 1, W + 2 * pad - S + 1, &bh)) return;
   const int PW = W + 2 * pad;
   const int b_stage = BN * 128, stage_area = BN == 64 ? Cfg<64>::STAGE_AREA : Cfg<128>::STAGE_AREA;
   const int kb_total = R * S * ((Cin + 63) / 64);

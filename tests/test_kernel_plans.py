@@ -59,6 +59,25 @@ def test_forward_halo_plans_fit_their_slots():
     assert out[0] == 0
 
 
+def test_forward_halo_plans_have_the_tile_width_of_the_launch():
+    """Small problems are launched with narrower tiles while twice as many still fit one wave of the SMs."""
+    lib = _lib()
+    out = (C.c_int * 10)()
+    widths = set()
+    for n, hw, cin, cout, k in SHAPES:
+        pad = (k - 1) // 2
+        lib.esgd_conv2d_halo_plan(n, hw, hw, cin, cout, k, k, 1, pad, out)
+        if not out[0]:
+            continue
+        ho = hw + 2 * pad - k + 1
+        m_tiles, bn = -(-n * ho * ho // 128), 64 if cout <= 64 else 128
+        if bn == 128 and 2 * m_tiles * -(-cout // 128) <= lib.esgd_sm_count():
+            bn = 64
+        assert out[3] == bn, (n, hw, cin, cout, k)
+        widths.add((cout, bn))
+    assert {(72, 64), (72, 128), (128, 64), (128, 128), (64, 64)} <= widths
+
+
 @pytest.mark.parametrize("sms", [148, 132])
 def test_weight_gradient_plans_cover_the_problem(sms):
     lib = _lib()
