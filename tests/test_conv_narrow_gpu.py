@@ -14,7 +14,7 @@ def _cl(t):
 @pytest.mark.parametrize("n,ci,h,w,co,stride", [(128, 16, 32, 32, 16, 1), (1, 16, 32, 32, 16, 1), (3, 16, 5, 7, 16, 1), (37, 16, 32, 32, 32, 2),
                                                 (5, 16, 9, 11, 32, 2), (100, 32, 16, 16, 32, 1), (2, 32, 3, 3, 32, 1), (100, 32, 16, 16, 64, 2),
                                                 (7, 32, 1, 1, 32, 1), (100, 64, 8, 8, 64, 1), (1, 64, 8, 8, 64, 1), (9, 64, 13, 6, 64, 1),
-                                                (2, 16, 224, 224, 16, 1), (600, 64, 8, 8, 64, 1)])
+                                                (2, 16, 224, 224, 16, 1), (600, 64, 8, 8, 64, 1), (64, 64, 8, 8, 64, 1), (65, 64, 8, 8, 64, 1)])
 def test_conv_narrow(n, ci, h, w, co, stride):
     from eagersgd_b200.ops import functional as ops
     from eagersgd_b200.ops.gemm import check_error

@@ -11,7 +11,7 @@ from eagersgd_b200 import _build
 _P = "C.c_void_p(0)"
 EMPTY = [("esgd_conv_narrow_fwd", [_P] * 3 + [2, 8, 8, 64, 64, 1] + [_P] * 3 + [0] + [_P] * 3, (3, 4, 5, 8)),
          ("esgd_conv_narrow_fwd", [_P] * 3 + [2, 32, 32, 16, 16, 1] + [_P] * 3 + [0] + [_P] * 3, (3, 4, 5, 8)),
-         ("esgd_conv_narrow_dgrad", [_P] * 3 + [2, 8, 8, 64, 64] + [_P] * 3, (3, 4, 5)),
+         ("esgd_conv_narrow_dgrad", [_P] * 3 + [2, 8, 8, 32, 32] + [_P] * 3, (3, 4, 5)),
          ("esgd_conv_narrow_wgrad", [_P] * 3 + [2, 8, 8, 32, 64, 1, _P], (3, 4, 5, 8)),
          ("esgd_bn_stats", [_P, "C.c_int64(64)", 8] + [_P] * 3, (2,)),
          ("esgd_bn_fwd", [_P] * 11 + ["C.c_int64(64)", 8, 1, "C.c_float(0.1)", "C.c_float(1e-5)", _P], (12,))]
