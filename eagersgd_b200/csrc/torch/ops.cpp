@@ -806,6 +806,105 @@ class BnCoefficients {
   Tensor table_;
 };
 
+// The layers that a fused inference pass stands in for.  Whether calling them one by one would still do the same is asked in
+// every pass (a layer may have been exchanged, parametrized or hooked since), and of 141 modules in a ResNet-56: 22 us here
+// against 130 in Python, where a small CIFAR network's whole pass takes 270.
+class EvalLayers {
+ public:
+  // modules: (module, the type whose forward the pass stands for; None for a container, whose forward nobody calls).  children:
+  // what the lists were made from, the network's own `_modules`.
+  EvalLayers(py::dict children, const std::vector<std::pair<py::object, py::object>>& modules, py::list convs, py::list norms)
+      : norms(std::move(norms)), convs_(std::move(convs)) {
+    root_.children = snapshot(children.ptr());
+    root_.module = std::move(children);
+    for (const auto& m : modules) {
+      Entry e{m.first, m.second, {}};
+      py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(m.first.ptr(), nullptr));
+      e.children = snapshot(d ? PyDict_GetItem(d.ptr(), name().modules) : nullptr);
+      entries_.push_back(std::move(e));
+    }
+  }
+  // Every module is of its type, in evaluation mode, without hooks or a forward of its own, and where it was.
+  bool unchanged() const {
+    const Names& n = name();
+    if (!same_children(root_.module.ptr(), root_.children)) return false;
+    for (const Entry& e : entries_) {
+      const bool called = !e.type.is_none();
+      if (called && (PyObject*)Py_TYPE(e.module.ptr()) != e.type.ptr()) return false;
+      const py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(e.module.ptr(), nullptr));
+      if (!d || !same_children(PyDict_GetItem(d.ptr(), n.modules), e.children)) { PyErr_Clear(); return false; }
+      if (!called) continue;
+      if (PyDict_GetItem(d.ptr(), n.training) != Py_False || PyDict_GetItem(d.ptr(), n.forward) != nullptr) return false;
+      for (PyObject* h : n.hooks) {
+        PyObject* hooks = PyDict_GetItem(d.ptr(), h);
+        if (hooks == nullptr || !PyDict_Check(hooks) || PyDict_Size(hooks) != 0) return false;
+      }
+    }
+    for (const auto& c : convs_)
+      if (!tensor(c.ptr(), n.parameters, n.weight).defined()) return false;
+    return true;
+  }
+  // The affine maps of the norms (BnCoefficients), or none: layers have changed, or a tensor is not what the kernels take.
+  c10::optional<std::vector<Tensor>> coefficients() {
+    if (!unchanged()) return c10::nullopt;
+    const Names& n = name();
+    std::vector<std::array<Tensor, 4>> layers;
+    layers.reserve(norms.size());
+    for (const auto& m : norms) {
+      layers.push_back({tensor(m.ptr(), n.parameters, n.weight), tensor(m.ptr(), n.parameters, n.bias), tensor(m.ptr(), n.buffers, n.mean),
+                        tensor(m.ptr(), n.buffers, n.var)});
+    }
+    std::vector<Tensor> out;
+    if (!layers.empty() && (out = table_.compute(layers)).empty()) return c10::nullopt;
+    return out;
+  }
+  const py::list norms;
+
+ private:
+  struct Entry {
+    py::object module, type;
+    std::vector<py::object> children;
+  };
+  struct Names {
+    PyObject *modules, *training, *forward, *parameters, *buffers, *weight, *bias, *mean, *var;
+    std::array<PyObject*, 4> hooks;
+  };
+  static const Names& name() {
+    static const Names n = [] {
+      auto s = [](const char* t) { return PyUnicode_InternFromString(t); };
+      return Names{s("_modules"), s("training"), s("forward"), s("_parameters"), s("_buffers"), s("weight"), s("bias"), s("running_mean"),
+                   s("running_var"), {s("_forward_hooks"), s("_forward_pre_hooks"), s("_backward_hooks"), s("_backward_pre_hooks")}};
+    }();
+    return n;
+  }
+  static std::vector<py::object> snapshot(PyObject* dict) {
+    std::vector<py::object> out;
+    PyObject *k, *v;
+    for (Py_ssize_t i = 0; dict != nullptr && PyDict_Check(dict) && PyDict_Next(dict, &i, &k, &v);) out.push_back(py::reinterpret_borrow<py::object>(v));
+    return out;
+  }
+  static bool same_children(PyObject* dict, const std::vector<py::object>& want) {
+    if (dict == nullptr || !PyDict_Check(dict) || (size_t)PyDict_Size(dict) != want.size()) return false;
+    PyObject *k, *v;
+    size_t j = 0;
+    for (Py_ssize_t i = 0; PyDict_Next(dict, &i, &k, &v);)
+      if (want[j++].ptr() != v) return false;
+    return true;
+  }
+  // A parameter or buffer where a module keeps it; undefined when there is none.
+  static Tensor tensor(PyObject* module, PyObject* where, PyObject* key) {
+    const py::object d = py::reinterpret_steal<py::object>(PyObject_GenericGetDict(module, nullptr));
+    if (!d) PyErr_Clear();
+    PyObject* dict = d ? PyDict_GetItem(d.ptr(), where) : nullptr;
+    PyObject* t = dict != nullptr && PyDict_Check(dict) ? PyDict_GetItem(dict, key) : nullptr;
+    return t != nullptr && THPVariable_Check(t) ? THPVariable_Unpack(t) : Tensor();
+  }
+  Entry root_;
+  std::vector<Entry> entries_;
+  py::list convs_;
+  BnCoefficients table_;
+};
+
 // ---------------------------------------------------------------- dense layer: fp32 logits out of bf16 operands
 struct LinearFn : public Function<LinearFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& w_in, const c10::optional<Tensor>& b_in,
@@ -1252,6 +1351,11 @@ PYBIND11_MODULE(_esgd_torch, m) {
   m.def("conv2d", &conv2d);
   m.def("conv_bn_eval", &conv_bn_eval);
   py::class_<BnCoefficients, std::shared_ptr<BnCoefficients>>(m, "BnCoefficients").def(py::init<>()).def("compute", &BnCoefficients::compute);
+  py::class_<EvalLayers, std::shared_ptr<EvalLayers>>(m, "EvalLayers")
+      .def(py::init<py::dict, const std::vector<std::pair<py::object, py::object>>&, py::list, py::list>())
+      .def("unchanged", &EvalLayers::unchanged)
+      .def("coefficients", &EvalLayers::coefficients)
+      .def_readonly("norms", &EvalLayers::norms);
   m.def("linear", &linear);
   m.def("bn_act", &bn_act);
   m.def("residual_block", &residual_block);

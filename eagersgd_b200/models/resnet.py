@@ -23,8 +23,8 @@ from ..ops import functional as ops
 BN_MOMENTUM_TF = 0.997  # tf decay; torch momentum = 1 - decay
 BN_EPS = 1e-5
 
-# what the fused inference path keeps per network (the device table of its batch norms); not an attribute of the module, which
-# has to stay copyable and picklable
+# what the fused inference path keeps per network (its layers, the device table of its batch norms); not an attribute of the
+# module, which has to stay copyable and picklable
 _eval_state = weakref.WeakKeyDictionary()
 
 IMAGENET_BLOCKS = {
@@ -75,27 +75,20 @@ class _Conv(nn.Conv2d):
                           tap_input=tap_input)
 
 
-def _bare(m: nn.Module, cls, training: bool = True) -> bool:
-    """Calling ``m`` does what ``cls.forward`` does in this mode, and nothing else."""
-    return type(m) is cls and m.training == training and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or
-                                                              m._backward_pre_hooks or "forward" in m.__dict__)
-
-
-def _tensors(m: nn.Module, parameters=("weight", "bias"), buffers=()):
-    """Parameters and buffers of a module by name, without the attribute lookup; None when one has become something else."""
-    p, b = m._parameters, m._buffers
-    t = tuple([p.get(n) for n in parameters] + [b.get(n) for n in buffers])
-    return None if any(e is None for e in t) else t
+def _bare(m: nn.Module, cls) -> bool:
+    """Calling ``m`` does what ``cls.forward`` does in training, and nothing else."""
+    return type(m) is cls and m.training and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or
+                                                  m._backward_pre_hooks or "forward" in m.__dict__)
 
 
 def _train_layer(conv, bn):
     """A convolution and its batch norm for ``ops.residual_block``; None when somebody could see the two being skipped."""
     if not _bare(conv, _Conv) or not _bare(bn, BatchNormAct) or bn.virtual_batch_size or bn.momentum is None or not bn.affine:
         return None
-    w, scale, b = _tensors(conv, ("weight",)), _tensors(bn), bn._buffers
-    if w is None or scale is None or "running_mean" not in b or "running_var" not in b:
+    w, p, b = conv._parameters.get("weight"), bn._parameters, bn._buffers
+    if w is None or "running_mean" not in b or "running_var" not in b or p.get("weight") is None or p.get("bias") is None:
         return None
-    return w + (conv.stride[0], conv.padding[0]) + scale + (b["running_mean"], b["running_var"], bn.momentum)
+    return (w, conv.stride[0], conv.padding[0], p["weight"], p["bias"], b["running_mean"], b["running_var"], bn.momentum)
 
 
 class _Block(nn.Module):
@@ -204,38 +197,38 @@ class ResNet(nn.Module):
         self.feature_dim = cin
 
     # ---- inference: every convolution with its batch norm, shortcut and ReLU as one kernel
+    def _eval_layers(self):
+        """What the fused pass stands in for, or None when the network has another structure."""
+        m = self._modules
+        stem, blocks = m["stem"], m["blocks"]
+        convs, norms, modules = [stem], [b for b in (m.get("stem_bn"), m.get("final_bn")) if b is not None], [(blocks, None)]
+        for blk in blocks._modules.values():
+            if type(blk) is not _Block or blk.version != self.version:
+                return None
+            m = blk._modules
+            proj, proj_bn, pre_bn = m.get("proj"), m.get("proj_bn"), m.get("pre_bn")
+            if len(m["convs"]) != len(m["bns"]) + (blk.version == 2) or (blk.version == 1 and (proj is None) != (proj_bn is None)):
+                return None
+            modules += [(blk, _Block), (m["convs"], None), (m["bns"], None)]
+            convs += [c for c in (*m["convs"]._modules.values(), proj) if c is not None]
+            norms += [b for b in (*m["bns"]._modules.values(), proj_bn, pre_bn) if b is not None]
+        modules += [(c, _Conv) for c in convs] + [(b, BatchNormAct) for b in norms]
+        return ops.eval_layers(self._modules, modules, convs, norms)
+
     def _fused_eval(self, x):
         """The coefficients of the network's batch norms by module, when the fused inference path applies: no gradients,
         every layer in evaluation mode and what it was built as, and nobody listening to a layer's output; else None.  Asked
         in every pass: a layer may have been exchanged, parametrized or hooked since the last one."""
         if self.training or torch.is_grad_enabled() or not ops.native(x) or nn.modules.module._has_any_global_hook():
             return None
-        m = self._modules
-        convs, norms = [m["stem"]], [b for b in (m.get("stem_bn"), m.get("final_bn")) if b is not None]
-        for blk in m["blocks"]._modules.values():
-            if not _bare(blk, _Block, False) or blk.version != self.version:
-                return None
-            m = blk._modules
-            bc, bn = m["convs"]._modules.values(), m["bns"]._modules.values()
-            proj, proj_bn, pre_bn = m.get("proj"), m.get("proj_bn"), m.get("pre_bn")
-            if len(bc) != len(bn) + (blk.version == 2) or (blk.version == 1 and (proj is None) != (proj_bn is None)):
-                return None
-            convs.extend(bc)
-            norms.extend(bn)
-            if proj is not None:
-                convs.append(proj)
-            norms.extend(b for b in (proj_bn, pre_bn) if b is not None)
-        for c in convs:
-            if not _bare(c, _Conv, False) or c._parameters.get("weight") is None:
-                return None
-        layers = []
-        for b in norms:
-            t = _tensors(b, buffers=("running_mean", "running_var")) if _bare(b, BatchNormAct, False) else None
-            if t is None:
-                return None
-            layers.append(t)
-        coef = ops.bn_coefficients(layers, _eval_state.setdefault(self, {}))
-        return dict(zip(norms, coef)) if coef or not layers else None
+        for renewed in (False, True):
+            layers = _eval_state.get(self) if not renewed else self._eval_layers()
+            coef = ops.eval_coefficients(layers) if layers is not None else None
+            if coef is not None:
+                if renewed:
+                    _eval_state[self] = layers
+                return dict(zip(layers.norms, coef))
+        return None
 
     @staticmethod
     def _conv_eval(conv, bn, x, coef, relu, residual=None):

@@ -168,6 +168,18 @@ def bn_coefficients(layers, store):
     return store["bn"].compute(layers)
 
 
+def eval_layers(children, modules, convs, norms):
+    """The layers of a network for which ``conv_bn_eval`` and ``residual_block_eval`` stand in: pairs of a module and the type it
+    was built as (None: a container), its convolutions and its batch norms, and the network's ``_modules``."""
+    return _ext().EvalLayers(children, modules, convs, norms)
+
+
+def eval_coefficients(layers) -> Optional[list]:
+    """Like ``bn_coefficients`` for the batch norms of ``eval_layers``, one after the other; None when one of the layers is no
+    longer what it was, is in training mode or has a hook, or when a tensor is not fp32 on the GPU."""
+    return layers.coefficients()
+
+
 def conv_bn_eval(x: torch.Tensor, w: torch.Tensor, stride: int, padding: int, coef: Optional[torch.Tensor], relu: bool,
                  residual: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """act(scale * conv(x) + shift [+ residual]) rounded once, without autograd; None for shapes the kernels do not take."""

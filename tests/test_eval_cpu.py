@@ -86,11 +86,13 @@ def stubs(monkeypatch):
     """The library's calls in PyTorch; the list counts those of the fused path."""
     fused = []
 
-    def coefficients(layers, store):
+    def coefficients(layers):
+        if not layers.unchanged():
+            return None
         out = []
-        for g, b, m, v in layers:
-            s = g * torch.rsqrt(v + ops.BN_EPS)
-            out.append(torch.stack([s, b - m * s]))
+        for m in layers.norms:
+            s = m.weight * torch.rsqrt(m.running_var + ops.BN_EPS)
+            out.append(torch.stack([s, m.bias - m.running_mean * s]))
         return out
 
     def conv(x, w, stride, pad, coef, relu, residual=None):
@@ -120,7 +122,7 @@ def stubs(monkeypatch):
         return x
 
     monkeypatch.setattr(ops, "native", lambda x: not ops._reference_only)
-    monkeypatch.setattr(ops, "bn_coefficients", coefficients)
+    monkeypatch.setattr(ops, "eval_coefficients", coefficients)
     monkeypatch.setattr(ops, "conv_bn_eval", conv)
     monkeypatch.setattr(ops, "residual_block_eval", block)
     monkeypatch.setattr(ops, "residual_block", train_block)
