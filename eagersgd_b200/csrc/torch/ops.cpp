@@ -199,12 +199,13 @@ struct SinkEntry : torch::CustomClassHolder {
   bool hooked = false;           // autograd has written .grad
   bool counted = false;          // taken off its bucket's count
   explicit SinkEntry(const Tensor& p) : param(p.getIntrusivePtr()) {}
-  // Autograd may still add to .grad: the parameter is in a graph, too, and its accumulation has not run.
+  // Autograd may still add to .grad: the parameter is in a graph, too, and its accumulation has not run.  Looked up without a
+  // reference of our own, which costs 0.8 us a parameter (a tensor that Python knows); in a step its owner keeps it.
   bool awaited() const {
     if (recomputed) return true;
-    if (hooked || !used) return false;
-    const auto p = param.lock();
-    return p.defined() && torch::autograd::impl::try_get_grad_accumulator(Tensor(p)) != nullptr;
+    if (hooked || !used || param.expired()) return false;
+    const auto* meta = static_cast<const torch::autograd::AutogradMeta*>(param._unsafe_get_target()->autograd_meta());
+    return meta != nullptr && !meta->grad_accumulator_.expired();
   }
   std::atomic<GradSinks*> owner{nullptr};
 };
