@@ -195,7 +195,7 @@ struct ConvHaloProblem {
 // row of the NHWC storage): a k-block is a box of up to 64 output pixels, loaded once from dy (two 64-channel
 // atoms for the 128 MMA rows) and once from x at the tap's offset (zero-filled outside the image, element
 // strides for stride 2).  Boxes smaller than 64 pixels leave the tail rows of the stage at their initial
-// zeros.  Work is split over taps, channel tiles and pixel ranges (split-K) and meets in fp32 atomics.
+// zeros.  Work is split over taps, channel tiles and pixel ranges (split-K) and meets in TMA reductions.
 template <int BN_>
 struct ConvWgradProblem {
   static constexpr int BN = BN_;
@@ -470,8 +470,8 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
   p.n_tiles = (a.Cin + BN - 1) / BN;
   const int sms = sm_count();
   const int base_tiles = a.R * a.S * p.m_tiles * p.n_tiles;
-  // Every split adds its partial sums with atomics: two waves of tiles when the filter bank is small, one
-  // wave when it is large (the atomics of a 512 x 512 x 9 bank already outnumber its loads).
+  // Every split adds a whole filter bank of partial sums (TMA reductions): two waves of tiles when the bank is small, one
+  // wave when it is large (the sums of a 512 x 512 x 9 bank are already more bytes than its loads).
   const int waves = base_tiles < 32 ? 2 : 1;
   int splits = (waves * sms + base_tiles - 1) / base_tiles;
   if (splits < 1) splits = 1;
@@ -501,7 +501,7 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
     if (r != 0) return 2000 + r;
   }
   Epilogue ep;
-  ep.out_mode = OUT_F32_ATOMIC; ep.relu = 0; ep.n_total = a.Cin; ep.scale = nullptr; ep.bias = nullptr; ep.bias_kind = BIAS_F32; ep.res_bytes = 0;
+  ep.out_mode = OUT_F32_ADD; ep.relu = 0; ep.n_total = a.Cin; ep.scale = nullptr; ep.bias = nullptr; ep.bias_kind = BIAS_F32; ep.res_bytes = 0;
   ep.col_sum = nullptr; ep.col_sqsum = nullptr; ep.error_flag = error_flag;
   ep.tx_bytes = (uint32_t)(p.BW * p.BH * 128 * (BM / 64 + BN / 64));
   ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
@@ -543,7 +543,7 @@ int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
 
 extern "C" {
 
-// dw: fp32 [Cout][R][S][Cin], zeroed by the caller (split-K partial sums are added atomically).
+// dw: fp32 [Cout][R][S][Cin], zeroed by the caller (split-K partial sums are added by TMA reductions).
 // x: [N,H,W,Cin] bf16, dy: [N,Ho,Wo,Cout] bf16.  Cin % 8 == 0, Cout % 8 == 0.
 int esgd_conv2d_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
                       int stride, int pad, int* error_flag, void* stream) {

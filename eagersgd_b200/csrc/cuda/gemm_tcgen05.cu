@@ -2,7 +2,7 @@
 //
 // Operands may be K-major (rows contiguous along K) or MN-major (stored [K][MN]);
 // the latter is what weight-gradient GEMMs over NHWC activations need, where K is
-// the pixel dimension.  Split-K with fp32 atomic accumulation covers their
+// the pixel dimension.  Split-K with partial sums added by TMA reductions covers their
 // few-tiles / long-K shape.  Used for dense layers, 1x1 convolutions (NHWC makes
 // them plain GEMMs) and the LSTM projections; the reference reaches cuBLAS / cuDNN
 // through TensorFlow for the same ops (official/resnet/resnet_model.py:97-101,552)
@@ -173,7 +173,7 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   if (splits > p.kb_total) splits = p.kb_total;
   p.kb_per_split = (p.kb_total + splits - 1) / splits;
   p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
-  if (p.splits > 1 && g.out_mode != OUT_F32_ATOMIC) return -2;
+  if (p.splits > 1 && g.out_mode != OUT_F32_ADD) return -2;
   ep.res_bytes = PANEL_BYTES;
   const bool two_panels = kBn && ep.residual != nullptr;
   const int sms = kPair ? sm_count() / 2 : sm_count();         // workers: CTAs, or pairs of them
@@ -219,7 +219,7 @@ int esgd_sm_count() { return sm_count(); }
 
 // C[M,N] = A * B^T (+bias, ReLU, column statistics).  A is [M][K] (a_mn=0, row stride lda)
 // or stored [K][M] (a_mn=1); B is [N][K] (b_mn=0, row stride ldb) or stored [K][N] (b_mn=1).
-// out_mode: 0 bf16, 1 fp32, 2 fp32 atomic accumulate (split-K; C must be zeroed by the caller).
+// out_mode: 0 bf16, 1 fp32, 2 fp32, added to C by TMA reductions (split-K; C zeroed by the caller or an accumulator).
 // Requirements: 16-byte aligned bases, lda/ldb/ldc multiples of 8; N need not be.
 // relu: bit 0 ReLU, bit 1 the bias is bf16.  scale (optional, with an fp32 bias, both 16-byte aligned): the product's
 // columns are multiplied by it before the bias is added.

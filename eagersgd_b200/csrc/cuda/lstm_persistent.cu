@@ -603,7 +603,9 @@ int launch(SeqParams& p, cudaStream_t stream) {
 extern "C" {
 
 // Whether the persistent kernels take this shape on the current device: units a multiple of 128 up to 2048 (the weights
-// must fit on the chip), a batch of up to 32 that is a multiple of 8, and every CTA resident.  1 yes, 0 no.
+// must fit on the chip), a batch of up to 32 that is a multiple of 8, and every CTA resident.  1 yes, 0 no.  On a B200 that is
+// every such shape but one: backward at 2048 units with a batch of 24 or 32 needs clusters of 8 for its shared memory, and only
+// 15 of the 16 would be resident.
 int esgd_lstm_persistent_ok(int B, int H, int backward) {
   if (B <= 0 || B > 32 || B % 8 || H < 128 || H > 2048 || H % 128) return 0;
   if (backward) return (B <= 16 ? cluster_size<true, 16>(H) : cluster_size<true, 32>(H)) > 0;

@@ -2,8 +2,8 @@
 // implicit-GEMM convolution kernels.
 //
 //   warp 0     : TMA producer — the Problem policy issues the loads of one k-block
-//   warp 1     : tcgen05.mma issuer (one thread); two TMEM accumulators so the
-//                epilogue of tile i overlaps the main loop of tile i+1
+//   warp 1     : tcgen05.mma issuer (one elected thread); two TMEM accumulators of 256 columns or four narrower
+//                ones, so that the epilogues of earlier tiles overlap the main loop of the next
 //   warps 2..17: epilogue, four groups of four warps.  A unit of work is one 64-column panel of a tile: tcgen05.ld, affine
 //                map / residual / ReLU, the panel staged in shared memory in the 128-byte-swizzled layout and written
 //                with a TMA store (coalesced, clipped at the tensor edge); per-channel sum and sum of squares of the
@@ -45,7 +45,7 @@ constexpr int GROUP_THREADS = 128;
 constexpr int NUM_THREADS = 64 + NUM_GROUPS * GROUP_THREADS;
 
 enum BiasKind { BIAS_F32 = 0, BIAS_BF16 = 1, BIAS_F32_UNALIGNED = 2 };
-enum OutMode { OUT_BF16 = 0, OUT_F32 = 1, OUT_F32_ATOMIC = 2 };
+enum OutMode { OUT_BF16 = 0, OUT_F32 = 1, OUT_F32_ADD = 2 };
 
 struct Epilogue {
   int out_mode;
@@ -400,11 +400,10 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
         accumulate = 1;
       };
       // The issuing thread is one lane with nothing to hide its instruction latency behind: every instruction
-      // between two tcgen05.mma widens the gap between them.  (Timestamps taken in this loop: a 128 x 64 x 16
-      // MMA goes out every ~115 cycles, a 128 x 256 x 16 one every ~185 -- 32 and 128 cycles of tensor-pipe work
-      // plus a fixed cost per instruction; narrow tiles are bound by that cost, not by their operands' traffic.
-      // Dealing the K steps to several accumulators did not shorten it.)  Descriptors are therefore built once and advanced
-      // by adding to their address field (bits 0-13, in 16-byte units; shared memory is < 256 KB, so no carry).
+      // between two tcgen05.mma widens the gap between them.  (It has to be elected: under lane == 0, which the compiler
+      // does not know to be one lane, every MMA sat in a loop over the active lanes, and 128 x 64 x 16 ones went out ~115
+      // cycles apart, 32 of them tensor-pipe work; 3x3 on 256 x 64 x 56 x 56: 148 -> 98 us.)  Descriptors are built once and
+      // advanced by adding to their address field (bits 0-13, in 16-byte units; shared memory is < 256 KB, so no carry).
       const uint64_t a_desc0 = P::A_MN ? umma_smem_desc(smem_u32(sA), 8192, 1024) : umma_smem_desc(smem_u32(sA), 16, 1024);
       const uint64_t b_desc0 = P::B_MN ? umma_smem_desc(smem_u32(sB), 8192, 1024) : umma_smem_desc(smem_u32(sB), 16, 1024);
       int stage = 0, acc = 0, hs = 0;
@@ -617,7 +616,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           }
         } else {
           // fp32 outputs (logits, split-K weight gradients): 32 columns at a time through the same buffer
-          const bool add = ep.out_mode == OUT_F32_ATOMIC;
+          const bool add = ep.out_mode == OUT_F32_ADD;
           stage_row_f32(r, panel, row, col0, ep);
           next_half();
           fence_proxy_async();

@@ -259,8 +259,11 @@ class GradSinks {
   }
   // Weight gradients go to a stream of their own: nothing waits for them before the bucket is complete, and neither they nor
   // the chain of the other gradients fills the GPU all of the time.  Outside a capture the events cost the host 3 us, so only
-  // where the GPU has more to do than that for the layer (from a GFLOP on; ResNet-44 at batch 100, half of that a layer, lost
-  // 7%, ResNet-50 at batch 64 gained 3%).  The operands are kept until the streams have met again.
+  // where the GPU has more to do than that for the layer: from a GFLOP on.  Milliseconds of an uncaptured step without /
+  // with the side stream: ResNet-44 on 32 x 32 images, batch 100 (0.47 GFLOP a layer) 2.87 / 2.94, 128 (0.60) 2.65 / 2.74, 150
+  // (0.71) 2.85 / 2.92, 200 (0.94) 2.93 / 2.74, 256 (1.21) 3.17 / 2.94, 400 (1.89) 3.85 / 3.41; ResNet-50 on 128 x 128
+  // images, batch 16 (1.21, and 0.54 for 1x1 filters) 3.36 / 3.42, batch 64 3.64 / 3.43.  The operands are kept until the
+  // streams have met again.
   c10::cuda::CUDAStream fork(const Tensor& a, const Tensor& b, double flops) {
     const auto main = c10::cuda::getCurrentCUDAStream(a.get_device());
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
@@ -390,7 +393,7 @@ int gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
 }
 
 // Split-K factor of a weight-gradient GEMM (K = pixels): about one wave of tiles.  Each split adds a full [Cout, Cin]
-// partial result with atomics, so large filter banks take few splits.
+// partial result (reductions in L2), so large filter banks take few splits.
 int wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int64_t sms) {
   const int64_t bn = cin <= 64 ? 64 : (cin <= 128 ? 128 : 256);
   const int64_t tiles = ((cout + 127) / 128) * ((cin + bn - 1) / bn);

@@ -2,8 +2,8 @@
 
 * ``x . W_ih^T`` for every time step is ONE tcgen05 GEMM ([T*B, I] x [4H, I]^T).
 * The recurrence is one kernel per direction that keeps the recurrent weights on chip for the whole sequence
-  (csrc/cuda/lstm_persistent.cu), for H a multiple of 128 up to 2048 and batches up to 32; other shapes take a native
-  loop of split-K GEMMs and cell kernels (csrc/cuda/lstm_cell.cu).
+  (csrc/cuda/lstm_persistent.cu), for H a multiple of 128 up to 2048 and batches up to 32 (backward at H = 2048: up to 16);
+  other shapes take a native loop of split-K GEMMs and cell kernels (csrc/cuda/lstm_cell.cu).
 * The three weight / input gradients are single large GEMMs over all time steps.
 * The autograd function around them is C++ (csrc/torch/ops.cpp).
 

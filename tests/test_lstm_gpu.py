@@ -10,14 +10,15 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,B,H", [(1, 8, 128), (2, 8, 128), (3, 16, 128), (7, 16, 384), (6, 24, 640), (5, 8, 1024), (9, 24, 1152),
-                                   (4, 32, 1536), (33, 16, 2048)])
+                                   (4, 32, 1536), (33, 16, 2048), (4, 32, 1920), (5, 24, 2048), (4, 32, 2048)])
 def test_persistent_recurrence(T, B, H):
     from eagersgd_b200.ops.gemm import check_error
     from eagersgd_b200.ops.lstm import lstm_layer, lstm_layer_reference
     from eagersgd_b200.parallel import _native as N
     lib = N.cuda()
     lib.esgd_lstm_persistent_ok.argtypes = [C.c_int] * 3
-    assert lib.esgd_lstm_persistent_ok(B, H, 0) == 1 and lib.esgd_lstm_persistent_ok(B, H, 1) == 1
+    # 2048 units backward with more than 16 sequences: the clusters are not all resident, the loop of launches takes it
+    assert lib.esgd_lstm_persistent_ok(B, H, 0) == 1 and lib.esgd_lstm_persistent_ok(B, H, 1) == (H < 2048 or B <= 16)
     g = torch.Generator().manual_seed(T * 1000 + H)
     rnd = lambda *s: torch.randn(*s, generator=g).cuda()
     x = (rnd(T, B, 64) * 0.5).to(torch.bfloat16).requires_grad_()
