@@ -848,8 +848,9 @@ class EvalLayers {
       if (!tensor(c.ptr(), n.parameters, n.weight).defined()) return false;
     return true;
   }
-  // The affine maps of the norms (BnCoefficients), or none: layers have changed, or a tensor is not what the kernels take.
-  c10::optional<std::vector<Tensor>> coefficients() {
+  // The affine maps of the norms, or none: layers have changed, or a tensor is not what the kernels take.  The table is the
+  // network's and not these layers': a captured pass reads it for as long as it is replayed.
+  c10::optional<std::vector<Tensor>> coefficients(BnCoefficients& table) const {
     if (!unchanged()) return c10::nullopt;
     const Names& n = name();
     std::vector<std::array<Tensor, 4>> layers;
@@ -859,7 +860,7 @@ class EvalLayers {
                         tensor(m.ptr(), n.buffers, n.var)});
     }
     std::vector<Tensor> out;
-    if (!layers.empty() && (out = table_.compute(layers)).empty()) return c10::nullopt;
+    if (!layers.empty() && (out = table.compute(layers)).empty()) return c10::nullopt;
     return out;
   }
   const py::list norms;
@@ -906,7 +907,6 @@ class EvalLayers {
   Entry root_;
   std::vector<Entry> entries_;
   py::list convs_;
-  BnCoefficients table_;
 };
 
 // ---------------------------------------------------------------- dense layer: fp32 logits out of bf16 operands

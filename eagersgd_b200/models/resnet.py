@@ -221,12 +221,12 @@ class ResNet(nn.Module):
         in every pass: a layer may have been exchanged, parametrized or hooked since the last one."""
         if self.training or torch.is_grad_enabled() or not ops.native(x) or nn.modules.module._has_any_global_hook():
             return None
+        st = _eval_state.setdefault(self, {})
         for renewed in (False, True):
-            layers = _eval_state.get(self) if not renewed else self._eval_layers()
-            coef = ops.eval_coefficients(layers) if layers is not None else None
+            layers = self._eval_layers() if renewed else st.get("layers")
+            coef = ops.eval_coefficients(layers, st) if layers is not None else None
             if coef is not None:
-                if renewed:
-                    _eval_state[self] = layers
+                st["layers"] = layers
                 return dict(zip(layers.norms, coef))
         return None
 

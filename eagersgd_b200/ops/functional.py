@@ -174,10 +174,12 @@ def eval_layers(children, modules, convs, norms):
     return _ext().EvalLayers(children, modules, convs, norms)
 
 
-def eval_coefficients(layers) -> Optional[list]:
+def eval_coefficients(layers, store) -> Optional[list]:
     """Like ``bn_coefficients`` for the batch norms of ``eval_layers``, one after the other; None when one of the layers is no
     longer what it was, is in training mode or has a hook, or when a tensor is not fp32 on the GPU."""
-    return layers.coefficients()
+    if "bn" not in store:
+        store["bn"] = _ext().BnCoefficients()
+    return layers.coefficients(store["bn"])
 
 
 def conv_bn_eval(x: torch.Tensor, w: torch.Tensor, stride: int, padding: int, coef: Optional[torch.Tensor], relu: bool,

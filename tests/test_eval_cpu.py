@@ -86,7 +86,7 @@ def stubs(monkeypatch):
     """The library's calls in PyTorch; the list counts those of the fused path."""
     fused = []
 
-    def coefficients(layers):
+    def coefficients(layers, store):
         if not layers.unchanged():
             return None
         out = []

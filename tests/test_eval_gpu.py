@@ -70,3 +70,23 @@ def test_networks_match_the_unfused_path_and_follow_their_parameters(make):
     with torch.no_grad():
         net(x.detach())
     assert seen == [1]                           # a listener gets the layer-by-layer path
+
+
+def test_a_captured_pass_outlives_a_change_beside_it():
+    """A network that gets another child looks at its layers anew; what a captured pass reads stays where it is."""
+    from eagersgd_b200.models import resnet as R
+    from eagersgd_b200.train.step import prepare_model
+    torch.manual_seed(1)
+    net = prepare_model(R.cifar_resnet(20, 1, 10), torch.device("cuda")).eval()
+    x = _cl(torch.randn(2, 3, 32, 32, device="cuda")).bfloat16()
+    with torch.no_grad():
+        want = net(x).clone()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = net(x)
+        net.extra = torch.nn.Linear(2, 2)
+        assert torch.equal(net(x), want)
+        junk = [torch.full((n,), 7.0, device="cuda") for n in (256, 1024, 1376, 4096)]      # whatever has been freed is used again
+        graph.replay()
+        torch.cuda.synchronize()
+    assert torch.equal(y, want) and len(junk) == 4
