@@ -452,6 +452,7 @@ int esgd_softmax_ce(const void* logits, int is_bf16, const int64_t* labels, int 
 // idx (optional, one byte per output element) records the arg-max for the backward pass.
 int esgd_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, void* stream) {
   if (C % 8) return -1;
+  if (N == 0) return 0;                                // a grid of no blocks is an error
   const int OH = (H + 1) / 2, OW = (W + 1) / 2;
   return esgd::launch(maxpool_fwd_kernel, dim3(N * OH), 256, 0, stream,
                       (const __nv_bfloat16*)x, (__nv_bfloat16*)y, (uint8_t*)idx, N, H, W, C, OH, OW);
@@ -459,6 +460,7 @@ int esgd_maxpool3x3s2_fwd(const void* x, void* y, void* idx, int N, int H, int W
 
 int esgd_maxpool3x3s2_bwd(const void* idx, const void* dy, void* dx, int N, int H, int W, int C, void* stream) {
   if (C % 8) return -1;
+  if (N == 0) return 0;
   const int OH = (H + 1) / 2, OW = (W + 1) / 2;
   return esgd::launch(maxpool_bwd_kernel, dim3(N * ((H + 1) / 2)), 256, 0, stream, (const uint8_t*)idx,
                       (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, N, H, W, C, OH, OW);
@@ -519,6 +521,7 @@ int esgd_cast_colsum(const float* dy, int64_t ld, int M, int N, int np, void* ou
 
 int esgd_avgpool_fwd(const void* x, void* y, int N, int HW, int C, void* stream) {
   if (C % 8) return -1;
+  if (N == 0) return 0;
   int cg = 1;
   while (cg < 16 && cg < C / 8) cg *= 2;
   return esgd::launch(avgpool_fwd_kernel, dim3(N, (C / 8 + cg - 1) / cg), 256, 0, stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)y, N,

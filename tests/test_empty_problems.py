@@ -32,3 +32,23 @@ def test_an_operand_that_is_not_aligned_is_left_to_another_kernel(fn, args):
     code = "import ctypes as C\nprint(C.CDLL(%r).%s(%s))" % (_build.build_cuda(), fn, ", ".join(args))
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and int(r.stdout) == -100, (r.returncode, r.stdout, r.stderr[-300:])
+
+
+@pytest.mark.parametrize("fn,args", [("esgd_maxpool3x3s2_fwd", [_P] * 3 + [0, 8, 8, 64, _P]), ("esgd_maxpool3x3s2_bwd", [_P] * 3 + [0, 8, 8, 64, _P]),
+                                     ("esgd_avgpool_fwd", [_P] * 2 + [0, 49, 64, _P])])
+def test_pooling_no_images_is_nothing_to_do(fn, args):
+    code = "import ctypes as C\nprint(C.CDLL(%r).%s(%s))" % (_build.build_cuda(), fn, ", ".join(str(a) for a in args))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and int(r.stdout) == 0, (r.returncode, r.stdout, r.stderr[-300:])
+
+
+@pytest.mark.gpu
+def test_pooling_no_images():
+    import torch
+    from eagersgd_b200.ops import functional as ops
+    for f, shape in ((ops.max_pool_3x3_s2, (0, 64, 4, 4)), (ops.global_avg_pool, (0, 64))):
+        x = torch.empty(0, 64, 8, 8, device="cuda", dtype=torch.bfloat16).contiguous(memory_format=torch.channels_last).requires_grad_()
+        y = f(x)
+        assert y.shape == shape
+        y.sum().backward()
+        assert x.grad.shape == x.shape
