@@ -104,13 +104,13 @@ void check_vector(const char* op, const char* name, const Tensor& t, const Tenso
   TORCH_CHECK(t.numel() == numel && t.is_contiguous(), op, ": ", name, " has to hold ", numel, " elements in a row, not ", t.sizes());
   check_operand(op, name, t, x, at::kFloat);
 }
-void check_conv(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad) {
+void check_conv(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool stem) {
   TORCH_CHECK(x.dim() == 4 && w.dim() == 4, "conv2d: takes a 4-D input and filter, not ", x.sizes(), " and ", w.sizes());
   TORCH_CHECK(x.size(1) == w.size(1), "conv2d: the filter ", w.sizes(), " does not have the ", x.size(1), " channels of the input");
   TORCH_CHECK(x.size(2) + 2 * pad >= w.size(2) && x.size(3) + 2 * pad >= w.size(3), "conv2d: the filter ", w.sizes(),
               " is larger than the padded input ", x.sizes());
   check_operand("conv2d", "the input", x, x, at::kBFloat16);
-  check_operand("conv2d", "the filter", w, x, at::kBFloat16);
+  check_operand("conv2d", "the filter", w, x, stem && w.is_floating_point() ? w.scalar_type() : at::kBFloat16);
 }
 
 // ---------------------------------------------------------------- per-device error word of the tensor-core kernels
@@ -482,7 +482,7 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
                            e.residual, e.relu, e.sum, e.sqsum, flag_ptr(x), st);
     ck(rc, "conv2d");
   } else {
-    *filters = nhwc(w);
+    *filters = nhwc(w.to(at::kBFloat16));           // packed anyway: any floating type
     const StemGeometry g(cin, r, s);
     *kept = at::empty({n * ho * wo, g.kpad}, x.options());
     ck(esgd_im2col_small_c(x.data_ptr(), kept->data_ptr(), n, h, wd, cin, r, s, stride, pad, g.seg, g.kpad, st), "im2col");
@@ -679,7 +679,7 @@ struct ConvOut {
 };
 ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap,
                    const Tensor& into = Tensor()) {
-  check_conv(x, w, stride, pad);
+  check_conv(x, w, stride, pad, kind == kStem);
   const int64_t r = w.size(2), s = w.size(3);
   // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
   const bool fuse_tap = tap && (kind == kOneByOne || (kind == kGeneral && r == s && pad <= r - 1)) && stride == 1 && x.requires_grad() && at::GradMode::is_enabled();
@@ -702,7 +702,7 @@ py::object conv2d(const Tensor& x, const Tensor& w, int64_t stride, int64_t pad,
 // None for a bare convolution.  No autograd; None when the shape is not this package's.
 Tensor conv_eval(int64_t kind, const Tensor& x_in, const Tensor& w, int64_t stride, int64_t pad, const c10::optional<Tensor>& coef,
                  const c10::optional<Tensor>& residual, bool relu) {
-  check_conv(x_in, w, stride, pad);
+  check_conv(x_in, w, stride, pad, kind == kStem);
   if (coef.has_value()) check_vector("conv2d", "the coefficients", *coef, x_in, 2 * w.size(0));
   const int64_t ho = (x_in.size(2) + 2 * pad - w.size(2)) / stride + 1, wo = (x_in.size(3) + 2 * pad - w.size(3)) / stride + 1;
   if (residual.has_value()) {

@@ -70,7 +70,7 @@ MISFITS = [
     (_conv1x1, "w", lambda d: _t(24, 8, 1, 1, device=d)), (_conv1x1, "w", lambda d: _t(24, 24, 1, 1, device=d)),
     (_conv1x1, "w", lambda d: _t(24, 16, 1, 1, dtype=F32, device=d)),
     (_conv3x3, "w", lambda d: _t(16, 8, 3, 3, device=d)), (_conv3x3, "w", lambda d: _t(16, 16, 3, 3, dtype=F32, device=d)),
-    (_stem, "w", lambda d: _t(16, 1, 3, 3, device=d)), (_stem, "w", lambda d: _t(16, 3, 3, 3, dtype=F32, device=d)),
+    (_stem, "w", lambda d: _t(16, 1, 3, 3, device=d)), (_stem, "w", lambda d: _t(16, 3, 3, 3, dtype=torch.int32, device=d)),
     (_eval, "w", lambda d: _t(16, 32, 3, 3, device=d)), (_eval, "coef", lambda d: _t(16, dtype=F32, device=d)),
     (_eval, "residual", lambda d: _t(2, 16, 4, 4, device=d)), (_eval, "residual", lambda d: _t(2, 16, 8, 8, dtype=F32, device=d)),
     (_bn, "gamma", lambda d: _t(8, dtype=F32, device=d)), (_bn, "beta", lambda d: _t(16, device=d)),
@@ -195,3 +195,20 @@ def test_linear_over_more_rows_than_a_grid_has_blocks(rows):
     for got, ref, tol in ((x.grad, dy16 @ w.detach().double(), 4e-3), (w.grad, dy16.t() @ x.detach().double(), 4e-3),
                           (b.grad, dy.double().sum(0), 1e-4)):
         assert (got.double() - ref).norm() <= tol * ref.norm()      # one bf16 rounding; fp32 sums of a million terms
+
+
+@pytest.mark.gpu
+def test_stem_filters_in_fp32():
+    """The stem packs its filters, from any floating type; the gradient comes back in that type."""
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(2, 3, 16, 16, generator=g).cuda().bfloat16().contiguous(memory_format=torch.channels_last)
+    w = torch.randn(16, 3, 7, 7, generator=g).cuda().bfloat16().float()
+    outs = []
+    for dtype in (torch.bfloat16, torch.float32):
+        wt = w.to(dtype).requires_grad_()
+        y, _ = ops.conv2d(x, wt, 2, 3)
+        y.square().sum().backward()
+        assert wt.grad.dtype == dtype
+        outs.append((y.detach().float(), wt.grad.float()))
+    assert torch.equal(outs[0][0], outs[1][0]) and (outs[0][1] - outs[1][1]).norm() <= 1e-3 * outs[0][1].norm()
