@@ -101,6 +101,8 @@ def conv1x1(x: torch.Tensor, w: torch.Tensor, want_stats: bool = False, tap_inpu
     """1x1 convolution.  ``tap_input=True`` appends ``x`` itself to the outputs (use it for the shortcut of a
     residual block: the two gradients of ``x`` are then added inside the data-gradient GEMM)."""
     if native(x):
+        if tuple(w.shape[2:]) != (1, 1):        # [outputs, inputs] does as well; anything larger is no 1x1 filter
+            w = w.reshape(w.shape[0], x.shape[1], 1, 1)
         r = _ext().conv2d(x, w, 1, 0, want_stats, tap_input, _SMALL_CHANNELS_NATIVE)
         if r is not None:
             outs = tuple(t for t in r if t is not None)

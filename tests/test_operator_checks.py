@@ -212,3 +212,17 @@ def test_stem_filters_in_fp32():
         assert wt.grad.dtype == dtype
         outs.append((y.detach().float(), wt.grad.float()))
     assert torch.equal(outs[0][0], outs[1][0]) and (outs[0][1] - outs[1][1]).norm() <= 1e-3 * outs[0][1].norm()
+
+
+@pytest.mark.gpu
+def test_conv1x1_takes_a_matrix_and_no_larger_filter():
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(6)
+    x = torch.randn(2, 16, 8, 8, generator=g).cuda().bfloat16().contiguous(memory_format=torch.channels_last)
+    w = torch.randn(24, 16, generator=g).cuda().bfloat16().requires_grad_()
+    y = ops.conv1x1(x, w)
+    assert torch.equal(y, ops.conv1x1(x, w.view(24, 16, 1, 1)))
+    y.sum().backward()
+    assert w.grad.shape == w.shape
+    with pytest.raises(RuntimeError):
+        ops.conv1x1(x, torch.zeros(24, 16, 3, 3, device="cuda", dtype=torch.bfloat16))
