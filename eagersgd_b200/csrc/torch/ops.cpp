@@ -10,6 +10,7 @@
 // bf16 tensor that is cast, added to a zeroed .grad and cast again: three small kernels and a Python hook fewer per tensor.
 #include <torch/extension.h>
 #include "../cuda/bn_grad.h"
+#include <ATen/SavedTensorHooks.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <atomic>
@@ -1014,7 +1015,8 @@ struct BnActFn : public Function<BnActFn> {
     ctx->saved_data["res"] = res.defined();
     save_sink(ctx, "g", gs);
     save_sink(ctx, "b", bs);
-    if (gs && bs) {
+    // Saved-tensor hooks (checkpointing, offloading) are there to let go of activations: no record then, which would keep them.
+    if (gs && bs && !at::SavedTensorDefaultHooks::get_hooks().has_value()) {
       auto rec = c10::make_intrusive<BnRecord>();
       rec->y = y;
       rec->mask = mask;
@@ -1092,7 +1094,8 @@ Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c1
                             bs, anchor_for(y, gs || bs), Held{gamma}, Held{beta});
   if (gs && bs) {
     auto* node = static_cast<torch::autograd::CppNode<BnActFn>*>(z.grad_fn().get());
-    c10::static_intrusive_pointer_cast<BnRecord>(node->ctx_.saved_data.at("rec").toCapsule())->node = z.grad_fn();
+    const auto it = node->ctx_.saved_data.find("rec");
+    if (it != node->ctx_.saved_data.end()) c10::static_intrusive_pointer_cast<BnRecord>(it->second.toCapsule())->node = z.grad_fn();
   }
   return z;
 }

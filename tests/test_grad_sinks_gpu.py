@@ -131,6 +131,50 @@ def test_closing_one_of_two_owners_leaves_the_parameter_to_the_other():
     owners[1].close()
 
 
+def test_saved_tensor_hooks_can_let_go_of_activations():
+    """Offloading what backward needs to the host: the operators keep no activation on the GPU beside it, and the gradients are
+    those of a pass without hooks."""
+    from eagersgd_b200 import _build
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(6)
+    cl = lambda *s: torch.randn(*s, generator=g).cuda().bfloat16().contiguous(memory_format=torch.channels_last)
+    x, w1, w2 = cl(4, 64, 64, 64), (cl(64, 64, 3, 3) * 0.1).requires_grad_(), (cl(64, 64, 3, 3) * 0.1).requires_grad_()
+    gamma, beta = torch.rand(64, generator=g).cuda().requires_grad_(), torch.zeros(64, device="cuda").requires_grad_()
+    params = [w1, gamma, beta, w2]
+    accs = [torch.zeros_like(p, dtype=torch.float32, memory_format=torch.preserve_format) for p in params]
+    sinks = _build.load_torch().GradSinks([4], lambda i: None)
+    for p, a in zip(params, accs):
+        sinks.add(p, a, 0)
+
+    def run():
+        y, st = ops.conv2d(x, w1, 1, 1, want_stats=True)
+        z = ops.bn_act(y, gamma, beta, None, None, stats=st)
+        return ops.conv2d(z, w2, 1, 1)[0].float().square().mean()
+
+    results, held = [], []
+    for offload in (False, True, False, True):             # the second time round nothing is allocated once and for all
+        for a in accs:
+            a.zero_()
+        sinks.begin_step()
+        sinks.set_active(True)
+        torch.cuda.synchronize()
+        m0 = torch.cuda.memory_allocated()
+        if offload:
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.cuda()):
+                loss = run()
+        else:
+            loss = run()
+        held.append(torch.cuda.memory_allocated() - m0)
+        loss.backward()
+        sinks.set_active(False)
+        results.append([a.clone() for a in accs])
+        del loss
+    sinks.close()
+    assert held[3] < x.numel() * 2 <= held[2] and max(held[3], 0) < 1 << 20, held
+    for a, b in zip(results[2], results[3]):
+        assert (a - b).norm() <= 1e-2 * b.norm()            # the masked gradient's sums in one kernel, or in another
+
+
 def test_steps_with_the_weight_gradients_on_a_stream_of_their_own():
     """The same network captured (the weight gradients of all its convolutions go to the side stream) and not (none does)."""
     import eagersgd_b200 as es
