@@ -181,8 +181,8 @@ def bench_ce(shape, iters):
 
 
 def bench_lstm(shape, iters):
-    """One LSTM layer, forward + backward: T steps of batch B, input I, hidden H (recurrent GEMM with swapped
-    operands + fused gate kernel per step) against torch.nn.LSTM (cuDNN)."""
+    """One LSTM layer, forward + backward: T steps of batch B, input I, hidden H (one persistent kernel per direction where the
+    shape allows it) against torch.nn.LSTM (cuDNN)."""
     from .lstm import lstm_layer
     T, B, I, H = shape
     x = torch.randn(T, B, I, device="cuda").to(torch.bfloat16).requires_grad_()
@@ -194,13 +194,14 @@ def bench_lstm(shape, iters):
     ref = torch.nn.LSTM(I, H).cuda().to(torch.bfloat16)
     ms_lib = timeit(lambda: torch.autograd.grad(ref(x)[0], (x,) + tuple(ref.parameters()), g), iters, graph=False)
     flops = 3 * 2.0 * T * B * 4 * H * (I + H)
-    byts = 3 * 2.0 * T * 4 * H * H                      # the recurrent weights are re-read every step, fwd and bwd
+    # x, dx, y, dy, the gates written and read; the weights read twice, their gradients written
+    byts = 2.0 * T * B * (2 * I + 2 * H + 8 * H) + 3 * 2.0 * 4 * H * (I + H)
     return dict(op="lstm_layer_fwd+bwd", T=T, B=B, I=I, H=H, ms=ms, tflops=flops / ms / 1e9, gbs=byts / ms / 1e6,
                 library_ms=ms_lib)
 
 
 def bench_update(shape, iters):
-    """The fused reduce + momentum-SGD kernel path of a single-rank channel (pack, control, update)."""
+    """The fused reduce + momentum-SGD step of a single-rank channel (one launch)."""
     from ..parallel.nvlink_channel import NvlinkChannel, create_arenas
     (count,) = shape
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -212,10 +213,10 @@ def bench_update(shape, iters):
     ch = NvlinkChannel(count, 0, 1, bases, dev, grad, slot_dtype=torch.bfloat16, mode="solo", limiter=32, w32=w32,
                        mom=mom, w16=w16, hyper=hyper)
     ms = timeit(lambda: ch.step(), iters, graph=False)
-    byts = count * (2 + 2 + 2 + 4 + 4 + 4 + 4 + 2.0)   # grad read, slot write+read, w32/mom read+write, w16 write
+    byts = count * (2 + 4 + 4 + 4 + 4 + 2.0)           # grad read, w32/mom read+write, w16 write
     torch.cuda.synchronize()
     arena.free()
-    return dict(op="publish+reduce+fused_sgd(world=1)", count=count, ms=ms, gbs=byts / ms / 1e6)
+    return dict(op="fused_sgd(world=1)", count=count, ms=ms, gbs=byts / ms / 1e6)
 
 
 def bench_lars(shape, iters):
