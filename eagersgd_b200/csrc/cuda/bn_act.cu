@@ -42,7 +42,7 @@ __device__ __forceinline__ uint8_t sign_bits(const uint4& w) {
 // Blocks of a kernel that are resident on an SM, and the size of its grid.  With more of them every block beyond these starts
 // over with its coefficients and the last wave is partly empty; with more registers a thread instead (the backward apply pass
 // of two resident blocks) too few loads are in flight.  12544 x 2048 and 802816 x 256, 8 blocks an SM -> now: forward 31 -> 28
-// and 161 -> 147 us, with a residual 41 -> 37 and 213 -> 199, apply 49 -> 34.5 and 249 -> 212.
+// and 161 -> 145 us, with a residual 41 -> 37 and 213 -> 199, apply 49 -> 35 and 249 -> 208.
 constexpr int kStatsBlocks = 4;
 constexpr int fwd_blocks(bool res) { return res ? 2 : 3; }
 constexpr int reduce_blocks(int mode) { return mode == 2 ? 2 : 3; }
