@@ -115,6 +115,16 @@ def test_a_parameter_with_a_hook_keeps_its_gradient():
     opt.close()
 
 
+def test_a_second_optimizer_over_the_parameters_of_a_closed_one():
+    loss = lambda k, x, ps: _mlp(x, ps)
+    params = _layers(0)
+    _train(loss, 2, True, params=params)
+    copies = [torch.nn.Parameter(p.detach().clone()) for p in params]
+    (a, launches), (b, _) = _train(loss, 2, True, params=params), _train(loss, 2, False, params=copies)
+    _same(a, b, TOL)
+    assert launches == ["early"] * 2
+
+
 def test_closing_one_of_two_owners_leaves_the_parameter_to_the_other():
     from eagersgd_b200 import _build
     (w,) = _layers(3, 1)
