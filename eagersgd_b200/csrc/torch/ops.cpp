@@ -218,7 +218,7 @@ std::unordered_map<at::TensorImpl*, Sink> g_sinks;
 class GradSinks {
  public:
   GradSinks(std::vector<int> params_per_bucket, py::function on_bucket)
-      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), complete_(total_.size(), 0), on_bucket_(std::move(on_bucket)) {}
+      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), complete_(total_.size(), 0), in_bucket_(total_.size()), on_bucket_(std::move(on_bucket)) {}
   ~GradSinks() {
     close();
     if (side_) {
@@ -234,6 +234,7 @@ class GradSinks {
       if (it != g_sinks.end() && it->second == kv.second) g_sinks.erase(it);       // unless a later one has taken it over
     }
     mine_.clear();
+    for (auto& b : in_bucket_) b.clear();
   }
   void add(const Tensor& param, const Tensor& acc, int bucket) {
     TORCH_CHECK(acc.scalar_type() == at::kFloat && acc.numel() == param.numel());
@@ -244,6 +245,7 @@ class GradSinks {
     std::unique_lock<std::shared_mutex> g(g_sink_mutex);
     g_sinks[param.unsafeGetTensorImpl()] = e;
     mine_[param.unsafeGetTensorImpl()] = e;
+    in_bucket_.at(bucket).push_back(e.get());
   }
   void begin_step() {
     pending_ = total_;
@@ -316,14 +318,15 @@ class GradSinks {
   // Announces a bucket whose every gradient is there; one with a parameter that may still get more goes with the step.
   void settle(int bucket) {
     if (pending_[bucket] > 0 || complete_[bucket]) return;
-    for (auto& kv : mine_)
-      if (kv.second->bucket == bucket && kv.second->awaited()) return;
+    for (const SinkEntry* e : in_bucket_[bucket])
+      if (e->awaited()) return;
     complete_[bucket] = 1;
     join();
     py::gil_scoped_acquire gil;
     on_bucket_(bucket);
   }
   std::vector<int> total_, pending_, written_, complete_;
+  std::vector<std::vector<const SinkEntry*>> in_bucket_;
   std::atomic<bool> active_{false};
   py::function on_bucket_;
   c10::optional<c10::cuda::CUDAStream> side_;
