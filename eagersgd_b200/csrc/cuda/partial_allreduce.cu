@@ -264,13 +264,21 @@ struct esgd_collective {
   void* dch;
   uint64_t count;
   int max_blocks, local;
+  int hold;                       // see esgd_collective_post
+  void *out, *staged;             // where wait() puts a staged result, and what the kernels wrote; null: nothing to copy
+  uint64_t bytes;
+  const StepOutcome* outcome;
 };
 
-int esgd_collective_create(void* dch, uint64_t count, int max_blocks, int local, void* side, void** out) {
-  esgd_collective* c = new esgd_collective{nullptr, nullptr, (cudaStream_t)side, dch, count, max_blocks, local};
+// hold: a poster's stream goes on once the step has completed, so that what it does to the tensor next comes after the step's
+// reads (for a step that waits for nobody: a world of one rank).  out, staged, bytes: a result that appears in wait().
+int esgd_collective_create(void* dch, uint64_t count, int max_blocks, int local, void* side, int hold, void* out, void* staged,
+                           uint64_t bytes, const void* outcome, void** handle) {
+  esgd_collective* c = new esgd_collective{nullptr, nullptr, (cudaStream_t)side, dch, count, max_blocks, local, hold, out, staged, bytes,
+                                           (const StepOutcome*)outcome};
   cudaError_t e = cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming);
-  *out = c;
+  *handle = c;
   return (int)e;
 }
 void esgd_collective_destroy(void* h) {
@@ -280,9 +288,8 @@ void esgd_collective_destroy(void* h) {
   if (c->done) cudaEventDestroy(c->done);
   delete c;
 }
-// Launch a step on the side stream behind what `stream` holds so far.  hold: `stream` goes on once the step has completed, so
-// that what it does to the tensor next comes after the step's reads (for a step that waits for nobody: a world of one rank).
-int esgd_collective_post(void* h, void* stream, int hold) {
+// Launch a step on the side stream behind what `stream` holds so far.
+int esgd_collective_post(void* h, void* stream) {
   esgd_collective* c = (esgd_collective*)h;
   cudaError_t e = cudaEventRecord(c->ready, (cudaStream_t)stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ready, 0);
@@ -291,7 +298,7 @@ int esgd_collective_post(void* h, void* stream, int hold) {
                     : esgd_channel_step(c->dch, c->count, c->max_blocks, SRC_FLAT, c->side);
   if (rc != 0) return rc;
   e = cudaEventRecord(c->done, c->side);
-  if (e == cudaSuccess && hold) e = cudaStreamWaitEvent((cudaStream_t)stream, c->done, 0);
+  if (e == cudaSuccess && c->hold) e = cudaStreamWaitEvent((cudaStream_t)stream, c->done, 0);
   return (int)e;
 }
 // Has the posted step completed?  1 yes, 0 no, negative CUDA error code.
@@ -299,11 +306,17 @@ int esgd_collective_test(void* h) {
   cudaError_t e = cudaEventQuery(((esgd_collective*)h)->done);
   return e == cudaSuccess ? 1 : (e == cudaErrorNotReady ? 0 : -(int)e);
 }
-// Order `stream` behind the posted step and wait for it on the host.
+// Order `stream` behind the posted step and wait for it on the host.  A staged result is copied on `stream`: behind the step
+// where every step applies one (one rank), else when the outcome says that there is one.
 int esgd_collective_wait(void* h, void* stream) {
   esgd_collective* c = (esgd_collective*)h;
-  cudaError_t e = cudaStreamWaitEvent((cudaStream_t)stream, c->done, 0);
+  cudaStream_t s = (cudaStream_t)stream;
+  cudaError_t e = cudaStreamWaitEvent(s, c->done, 0);
+  const bool copy = c->staged != nullptr;
+  if (e == cudaSuccess && copy && c->local) e = cudaMemcpyAsync(c->out, c->staged, c->bytes, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaEventSynchronize(c->done);
+  if (e == cudaSuccess && copy && !c->local && c->outcome->status == 0 && c->outcome->applied)
+    e = cudaMemcpyAsync(c->out, c->staged, c->bytes, cudaMemcpyDeviceToDevice, s);
   return (int)e;
 }
 

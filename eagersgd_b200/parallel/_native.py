@@ -115,10 +115,11 @@ def cuda():
         lib.esgd_channel_step.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p]
         lib.esgd_channel_set_grad_acc.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
         lib.esgd_channel_step_local.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p]
-        lib.esgd_collective_create.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p, C.POINTER(C.c_void_p)]
+        lib.esgd_collective_create.argtypes = [C.c_void_p, C.c_uint64, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p,
+                                               C.c_uint64, C.c_void_p, C.POINTER(C.c_void_p)]
         lib.esgd_collective_destroy.argtypes = [C.c_void_p]
         lib.esgd_collective_destroy.restype = None
-        lib.esgd_collective_post.argtypes = [C.c_void_p, C.c_void_p, C.c_int]
+        lib.esgd_collective_post.argtypes = [C.c_void_p, C.c_void_p]
         lib.esgd_collective_test.argtypes = [C.c_void_p]
         lib.esgd_collective_wait.argtypes = [C.c_void_p, C.c_void_p]
         lib.esgd_outcome_alloc.argtypes = [C.POINTER(C.c_void_p)]

@@ -58,13 +58,16 @@ class _PinnedOutcome:
 class _Collective:
     """Post / test / wait of one channel on a side stream, each a single native call."""
 
-    def __init__(self, ch, stream: torch.cuda.Stream):
+    def __init__(self, ch, stream: torch.cuda.Stream, hold: bool, out: Optional[torch.Tensor], staged: Optional[torch.Tensor],
+                 outcome: int):
+        """``hold``: a poster's stream waits for the step; ``out`` / ``staged``: a result that ``wait`` copies."""
         self._lib, self._h, self._ch = N.cuda(), C.c_void_p(), ch
+        copied = (out.data_ptr(), staged.data_ptr(), out.numel() * out.element_size()) if staged is not None else (None, None, 0)
         N.check_cuda(self._lib.esgd_collective_create(ch.dev_ptr, ch.count, ch.max_blocks, int(ch.local), stream.cuda_stream,
-                                                      C.byref(self._h)), "collective")
+                                                      int(hold), *copied, outcome, C.byref(self._h)), "collective")
 
-    def post(self, stream: int, hold: bool) -> None:
-        N.check_cuda(self._lib.esgd_collective_post(self._h, stream, int(hold)), "partial allreduce launch")
+    def post(self, stream: int) -> None:
+        N.check_cuda(self._lib.esgd_collective_post(self._h, stream), "partial allreduce launch")
         self._ch._steps += 1
 
     def test(self) -> bool:
@@ -119,7 +122,6 @@ class PartialAllreduce:
             # stream goes on.  Ragged and 16-bit results, and tensors that do not start on 16 bytes, are staged.
             even = n == self.count
             direct_in = tensor.data_ptr() % 16 == 0 and (even or g.world == 1)
-            self._hold = direct_in and not even
             direct_out = self.out.data_ptr() % 16 == 0 and even and self.out.dtype == torch.float32
             staged = self.out.dtype if self.out.dtype in (torch.float32, torch.bfloat16) else torch.float32
             self._grad = tensor.detach().view(-1) if direct_in else torch.zeros(n, dtype=tensor.dtype, device=dev)
@@ -131,7 +133,10 @@ class PartialAllreduce:
             self._ch = NvlinkChannel(self.count, g.rank, g.world, bases, dev, self._grad, slot_dtype=tensor.dtype,
                                      out=self._res, grace_us=self.grace_us, mc_base=self._arena.mc_base, valid=n,
                                      keep_out=True, outcome=self._outcome.address, **self._kw)
-            self._col = _Collective(self._ch, self._stream)
+            self._converted = not direct_out and staged != self.out.dtype
+            native_copy = not direct_out and not self._converted
+            self._col = _Collective(self._ch, self._stream, direct_in and not even, self.out if native_copy else None,
+                                    self._res if native_copy else None, self._outcome.address)
         else:
             from .cpu_channel import CpuChannel, LocalSegments, SharedSegments
             npdt = {torch.float32: np.float32, torch.float64: np.float64, torch.int32: np.int32,
@@ -163,7 +168,7 @@ class PartialAllreduce:
         if self.on_gpu:
             if self._grad.data_ptr() != self.tensor.data_ptr():
                 self._grad.copy_(self.tensor.view(-1))
-            self._col.post(torch.cuda.current_stream(self.tensor.device).cuda_stream, self._hold)
+            self._col.post(torch.cuda.current_stream(self.tensor.device).cuda_stream)
         else:
             src = self.tensor.detach().view(-1).numpy().copy()
 
@@ -197,7 +202,7 @@ class PartialAllreduce:
             if o.status:
                 raise N.ChannelError(o.status, "partial allreduce")
             applied = bool(o.applied)
-            if applied and not self._direct_out:
+            if applied and self._converted:
                 self.out.view(-1).copy_(self._res)
             info = {"role": _ROLES.get(o.role, "absent"), "round": int(o.round), "contributors": int(o.contributors),
                     "sync": bool(o.is_sync), "applied": applied}
