@@ -1165,8 +1165,10 @@ BnRef bn_behind(const Tensor& x) {
 struct SoftmaxCEFn : public Function<SoftmaxCEFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& logits_in, const Tensor& labels) {
     c10::cuda::CUDAGuard guard(logits_in.device());
-    Tensor logits = logits_in.stride(1) == 1 && logits_in.stride(0) >= logits_in.size(1) ? logits_in : logits_in.contiguous();
-    const int64_t b = logits.size(0), c = logits.size(1);
+    // rows padded to a multiple of eight (the dense layer's) are read as they are, and the gradient is laid out alike; a column
+    // slice of something wider is copied, or the gradient would be as wide
+    const int64_t b = logits_in.size(0), c = logits_in.size(1), ld = logits_in.stride(0);
+    Tensor logits = logits_in.stride(1) == 1 && ld >= c && ld < c + 8 ? logits_in : logits_in.contiguous();
     Tensor loss = at::zeros({}, logits.options().dtype(at::kFloat));
     Tensor d = at::empty_strided({b, c}, {logits.stride(0), 1}, logits.options());
     ck(esgd_softmax_ce(logits.data_ptr(), logits.scalar_type() == at::kBFloat16, labels.contiguous().data_ptr<int64_t>(), b, c,

@@ -226,3 +226,22 @@ def test_conv1x1_takes_a_matrix_and_no_larger_filter():
     assert w.grad.shape == w.shape
     with pytest.raises(RuntimeError):
         ops.conv1x1(x, torch.zeros(24, 16, 3, 3, device="cuda", dtype=torch.bfloat16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [10, 16, 1 << 16])
+def test_softmax_of_a_column_slice(width):
+    """The gradient of a slice is no larger than the slice, whatever it was cut from."""
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(width)
+    labels = torch.randint(0, 10, (64,), generator=g).cuda()
+    logits = torch.randn(64, width, generator=g).cuda()[:, :10].requires_grad_()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    loss = ops.softmax_cross_entropy(logits, labels)
+    assert torch.cuda.memory_allocated() - before < 1 << 16
+    loss.backward()
+    ref = logits.detach().clone().requires_grad_()
+    want = torch.nn.functional.cross_entropy(ref, labels)
+    want.backward()
+    assert abs(float(loss) - float(want)) < 1e-5 and torch.allclose(logits.grad, ref.grad, atol=1e-6)
