@@ -118,7 +118,7 @@ def conv2d(x: torch.Tensor, w: torch.Tensor, stride: int = 1, padding: int = 0, 
     third value is returned: the tensor a residual block should feed its shortcut from (the input itself, or
     for the fused 1x1 path an alias whose gradient is added inside the data-gradient GEMM).
     """
-    if native(x):
+    if native(x) and not isinstance(stride, (tuple, list)) and not isinstance(padding, (tuple, list, str)):
         r = _ext().conv2d(x, w, stride, padding, want_stats, tap_input, _SMALL_CHANNELS_NATIVE)
         if r is None and w.shape[2] == 1 and w.shape[3] == 1 and padding == 0 and stride > 2:
             xs = x[:, :, ::stride, ::stride].contiguous(memory_format=torch.channels_last)

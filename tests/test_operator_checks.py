@@ -245,3 +245,15 @@ def test_softmax_of_a_column_slice(width):
     want = torch.nn.functional.cross_entropy(ref, labels)
     want.backward()
     assert abs(float(loss) - float(want)) < 1e-5 and torch.allclose(logits.grad, ref.grad, atol=1e-6)
+
+
+@pytest.mark.gpu
+def test_conv2d_with_a_stride_per_dimension():
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(8)
+    cl = lambda *s: torch.randn(*s, generator=g).cuda().bfloat16().contiguous(memory_format=torch.channels_last)
+    x, w = cl(2, 64, 9, 9), cl(64, 64, 3, 3)
+    for stride, padding in (((2, 1), (1, 1)), ((1, 2), 0), (1, (0, 1))):
+        y, stats, tap = ops.conv2d(x, w, stride, padding, want_stats=True, tap_input=True)
+        ref = torch.nn.functional.conv2d(x.float(), w.float(), None, stride, padding)
+        assert stats is None and tap is x and (y.float() - ref).norm() < 5e-3 * ref.norm()
