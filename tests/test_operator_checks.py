@@ -244,7 +244,7 @@ def test_softmax_of_a_column_slice(width):
     ref = logits.detach().clone().requires_grad_()
     want = torch.nn.functional.cross_entropy(ref, labels)
     want.backward()
-    assert abs(float(loss) - float(want)) < 1e-5 and torch.allclose(logits.grad, ref.grad, atol=1e-6)
+    assert abs(loss.item() - want.item()) < 1e-5 and torch.allclose(logits.grad, ref.grad, atol=1e-6)
 
 
 @pytest.mark.gpu
