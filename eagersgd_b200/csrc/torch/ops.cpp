@@ -218,7 +218,8 @@ std::unordered_map<at::TensorImpl*, Sink> g_sinks;
 class GradSinks {
  public:
   GradSinks(std::vector<int> params_per_bucket, py::function on_bucket)
-      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), complete_(total_.size(), 0), in_bucket_(total_.size()), on_bucket_(std::move(on_bucket)) {}
+      : total_(std::move(params_per_bucket)), pending_(total_), written_(total_.size(), 0), complete_(total_.size(), 0),
+        in_bucket_(total_.size()), on_bucket_(std::move(on_bucket)) {}
   ~GradSinks() {
     close();
     if (side_) {
