@@ -41,6 +41,13 @@ def test_persistent_recurrence(T, B, H):
             assert float(a.grad.float().abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("T,B,H", [(5, 32, 128), (12, 32, 256), (3, 24, 384), (40, 8, 2048), (65, 16, 1024)])
+def test_issuers_blocks_and_padding(T, B, H):
+    """Fewer blocks of the state than warps that fetch or multiply them, batches that fill half of a product, and sequences over
+    which every barrier goes round more than once."""
+    test_persistent_recurrence(T, B, H)
+
+
 def test_shapes_outside_the_persistent_range_take_the_loop():
     from eagersgd_b200.parallel import _native as N
     lib = N.cuda()
