@@ -78,17 +78,32 @@ __global__ void __launch_bounds__(256, 3) data_kernel(DevChannel* ch) {
   data_phase(ch, blockIdx.x, gridDim.x, &s_flag);
 }
 
-// One step of a one-rank channel in one launch (see local_apply).
+// One step of a one-rank channel in one launch (see local_apply).  The records are kept by a thread that has no data in small
+// steps, at the same time: behind the data they were 2 of the 5 us that a step of 4 KB took.
 __global__ void __launch_bounds__(256, 4) local_step_kernel(DevChannel* ch, int grad_src) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) ch->t_phase[0] = DevEnv::now_ns();
+  if (blockIdx.x == 0 && threadIdx.x == blockDim.x - 1) local_records(ch);
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
   if (ch->slot_bf16) local_apply<__nv_bfloat16>(ch, grad_src, tid, nth);
   else local_apply<float>(ch, grad_src, tid, nth);
-  __syncthreads();
-  if (threadIdx.x == 0 && (gridDim.x == 1 || atomicAdd(&ch->bar_end, 1u) == gridDim.x - 1)) {
-    ch->bar_end = 0;
-    local_records(ch);
+}
+
+// A staged result to where it is expected: 16 bytes a load, four in flight a thread.  It was written a moment ago and is in L2:
+// 26 MB in 9.4 us by cudaMemcpyAsync, 6.5 here.
+__global__ void __launch_bounds__(256) hand_over_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, uint64_t bytes) {
+  constexpr int kUnroll = 4;
+  const uint64_t n = bytes / 16, tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint4* s = reinterpret_cast<const uint4*>(src);
+  uint4* d = reinterpret_cast<uint4*>(dst);
+  for (uint64_t base = tid; base < n; base += stride * kUnroll) {
+    uint4 v[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (base + u * stride < n) v[u] = __ldcg(s + base + u * stride);
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u)
+      if (base + u * stride < n) d[base + u * stride] = v[u];
   }
+  if (tid < bytes % 16) dst[n * 16 + tid] = src[n * 16 + tid];
 }
 
 // All ranks of a (small) world inside ONE launch, one block per rank: used to
@@ -306,6 +321,15 @@ int esgd_collective_test(void* h) {
   cudaError_t e = cudaEventQuery(((esgd_collective*)h)->done);
   return e == cudaSuccess ? 1 : (e == cudaErrorNotReady ? 0 : -(int)e);
 }
+// Copies `bytes` from staged to out on `stream`.
+static cudaError_t hand_over(const esgd_collective* c, cudaStream_t stream) {
+  if ((((uintptr_t)c->out | (uintptr_t)c->staged) & 15) || c->bytes == 0)
+    return cudaMemcpyAsync(c->out, c->staged, c->bytes, cudaMemcpyDeviceToDevice, stream);
+  const uint64_t need = (c->bytes / 16 + 4 * 256 - 1) / (4 * 256) + 1;
+  hand_over_kernel<<<(int)(need < 148 * 8 ? need : 148 * 8), 256, 0, stream>>>((const uint8_t*)c->staged, (uint8_t*)c->out, c->bytes);
+  count_launch();
+  return cudaGetLastError();
+}
 // Order `stream` behind the posted step and wait for it on the host.  A staged result is copied on `stream`: behind the step
 // where every step applies one (one rank), else when the outcome says that there is one.
 int esgd_collective_wait(void* h, void* stream) {
@@ -313,10 +337,10 @@ int esgd_collective_wait(void* h, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaStreamWaitEvent(s, c->done, 0);
   const bool copy = c->staged != nullptr;
-  if (e == cudaSuccess && copy && c->local) e = cudaMemcpyAsync(c->out, c->staged, c->bytes, cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess && copy && c->local) e = hand_over(c, s);
   if (e == cudaSuccess) e = cudaEventSynchronize(c->done);
   if (e == cudaSuccess && copy && !c->local && c->outcome->status == 0 && c->outcome->applied)
-    e = cudaMemcpyAsync(c->out, c->staged, c->bytes, cudaMemcpyDeviceToDevice, s);
+    e = hand_over(c, s);
   return (int)e;
 }
 

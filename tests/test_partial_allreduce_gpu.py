@@ -563,3 +563,30 @@ def test_ragged_and_16_bit_tensors_between_post_and_wait(dtype, out_dtype, n, in
             assert torch.equal(out, held)
             assert ar.wait()["applied"]
             assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 2040, 2048, 2049, 32767, 592 * 256 * 8 + 8, 592 * 256 * 32 + 5])
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
+                                             (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+def test_one_rank_hands_out_every_element_once(n, dtype, out_dtype):
+    """Vectors of eight with a remainder, fewer and more of them than threads and than loads in flight; NaN, infinities and
+    zeros of both signs come out as a conversion to the two types gives them."""
+    import eagersgd_b200 as es
+    g = torch.Generator(device="cuda").manual_seed(n)
+    special = torch.tensor([float("nan"), float("inf"), -float("inf"), -0.0, 3.0e38, 1e-40], device="cuda")
+    x = torch.randn(n, device="cuda", generator=g)
+    x[:min(n, 6)] = special[:min(n, 6)]
+    x = x.to(dtype)
+    guard = torch.full((n + 64,), 7.0, device="cuda", dtype=out_dtype)
+    out = guard[:n]
+    ar = es.PartialAllreduce(x, es.init(), mode="solo", limiter=2, out=out).start()
+    for step in range(4):
+        out.fill_(5.0)
+        ar.post()
+        info = ar.wait()
+        assert info["contributors"] == 1 and info["applied"] and info["round"] == step + 1
+        assert torch.equal(torch.nan_to_num(out, nan=1.5), torch.nan_to_num(x.to(out_dtype), nan=1.5))
+    assert bool((guard[n:] == 7.0).all())
+    stats = ar.stats()
+    assert stats["steps"] == stats["participated"] == stats["activated"] == 4 and stats["forced_sync"] == 1
+    ar.close()
