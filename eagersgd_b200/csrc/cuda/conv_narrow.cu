@@ -1,13 +1,22 @@
 // 3x3 convolutions of 16 and 32 channels over small images (the CIFAR ResNets): forward, data gradient, weight gradient; 64
 // channels in small forward problems.
 //
-// A layer of 128 x 32 x 32 pixels and 16 channels is 0.6 GFLOP over 8 MB that sit in L2: it is bound by latency, and the
-// 128-row tcgen05 tiles fed 64 channels at a time spent 33 us on it, three quarters of each operand zero fill.  Here a block
-// of eight warps copies a few image rows with their margin into shared memory (cp.async, only the channels there are) and
-// every warp multiplies 16 pixels at a time with ldmatrix / mma.sync m16n8k16: the fragment rows are pixel addresses, so a
-// tap, a stride or the filter's transposition is an address offset.  The tensor pipe is not what bounds these layers.
-// Pixel and filter rows are padded by 16 bytes, which makes every ldmatrix conflict-free.
+// A layer of 128 x 32 x 32 pixels and 16 channels is 0.6 GFLOP over 8 MB that sit in L2: it is bound by latency and by the
+// instructions around the products, and the 128-row tcgen05 tiles fed 64 channels at a time spent 33 us on it, three quarters of
+// each operand zero fill.  Here a block has a run of output rows (an even share of the rows of all images: 148 blocks, one an SM,
+// so every address of the sums sees 148 atomics and not one per tile), copies the input rows it needs with their margin
+// into shared memory (cp.async, a warp per row: an address per row instead of four divisions per 16 bytes), and every
+// warp multiplies 16 pixels at a time with ldmatrix / mma.sync m16n8k16: the fragment rows are pixel addresses, so a tap, a
+// stride or the filter's transposition is an address offset.  The tensor pipe is not what bounds these layers.  Pixel and
+// filter rows are padded by 16 bytes, which makes every ldmatrix conflict-free.  Results leave by way of shared memory,
+// eight channels of a pixel a lane, so that stores, shortcut and batch-norm operands are 16 bytes wide.
 //
+// Input rows are numbered as if every image had a row of zeros above and below it ("padded rows"); output row oh of image n
+// reads padded rows n * (H + 2) + oh * stride and the two after it.
+//
+// Microseconds with sums, tiles of 256 pixels with their own index arithmetic -> now: 128 x 32 x 32, 16 channels, forward
+// 15.4 -> 6.6, data gradient with batch norm 14.6 -> 7.0, weight gradient 12.3 -> 8.0; 128 x 16 x 16, 32 channels 8.6 -> 5.4, 11.1 -> 6.5,
+// 12.9 -> 11.0.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -17,7 +26,7 @@
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kWarps = 16, kThreads = kWarps * 32;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
@@ -34,12 +43,54 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void unpack8(const uint4& w, float (&v)[8]) {
+  const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { v[2 * q] = __uint_as_float(x[q] << 16); v[2 * q + 1] = __uint_as_float(x[q] & 0xffff0000u); }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  uint4 raw;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+  return raw;
+}
+
+// Division by a number known at launch: multiply, add, shift (exact for dividends below 2^31).
+struct FastDiv {
+  uint32_t mul, shift, d;
+  FastDiv() = default;
+  explicit FastDiv(uint32_t d_) : d(d_) {
+    for (shift = 0; shift < 31 && (1u << shift) < d; ++shift) {}
+    mul = (uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << shift) - d)) / d + 1);
+  }
+  __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
 
 struct Shape {
   int N, H, W, Ho, Wo, stride;   // H x W: the image the taps read, Ho x Wo: the pixels that are computed
-  int tr, ti;                    // output rows of an image and images per tile (ti > 1 only with tr == Ho)
-  int rows, pw;                  // input rows per image in a tile, pixel pitch (W + 2)
-  int row_tiles, tiles;
+  int pw;                        // pixel pitch of an input row (W + 2)
+  int total;                     // output rows of all images
+  int per_pass, slots;           // output rows that a block takes at a time, input rows that these need at most
+  FastDiv by_wo, by_ho, by_hp;   // Wo, Ho, H + 2
+};
+
+// A pass: output rows v0 .. v1 - 1 of all images' rows.
+struct Pass {
+  int v0, v1, g0, rows;          // g0, rows: first padded row of the input that it reads, and how many
+  __device__ __forceinline__ Pass(const Shape& s, int from, int to) : v0(from), v1(to) {
+    g0 = padded(s, v0);
+    rows = padded(s, v1 - 1) + 3 - g0;
+  }
+  static __device__ __forceinline__ int padded(const Shape& s, int v) {
+    const int n = s.by_ho.div(v);
+    return n * (s.H + 2) + (v - n * s.Ho) * s.stride;
+  }
+  // Where the window of output pixel p (counted from the pass's first) starts: a pixel of the input rows in shared memory.
+  __device__ __forceinline__ int window(const Shape& s, int p) const {
+    const int row = s.by_wo.div(p);
+    return (padded(s, v0 + row) - g0) * s.pw + (p - row * s.Wo) * s.stride;
+  }
 };
 
 struct Args {
@@ -54,158 +105,256 @@ struct Args {
   const float* bn_aux;
 };
 
-// The input rows of a tile with a margin of one pixel (zeros outside the image): [ti][rows][pw] pixels of C channels.
+// The first output row of block b.
+__device__ __forceinline__ int first_row(const Shape& s, int b) { return (int)((int64_t)s.total * b / (int)gridDim.x); }
+
+// The left and right margin of every input row: zeros for as long as the block lives.
 template <int C>
-__device__ __forceinline__ void load_tile(const __nv_bfloat16* x, const Shape& s, int n0, int oh0, uint8_t* dst) {
+__device__ __forceinline__ void clear_margins(const Shape& s, uint8_t* sX) {
   constexpr int CH = C / 8, PX = C * 2 + 16;
-  const int per_img = s.rows * s.pw * CH;
-  for (int i = threadIdx.x; i < s.ti * per_img; i += kThreads) {
-    const int im = i / per_img, j = i - im * per_img;
-    const int px = j / CH, ch = j - px * CH, row = px / s.pw, col = px - row * s.pw;
-    const int n = n0 + im, h = oh0 * s.stride - 1 + row, w = col - 1;
-    const bool ok = n < s.N && h >= 0 && h < s.H && w >= 0 && w < s.W;
-    const __nv_bfloat16* src = ok ? x + (((int64_t)n * s.H + h) * s.W + w) * C + ch * 8 : x;
-    cp_async16(smem_addr(dst + (im * s.rows * s.pw + px) * PX + ch * 16), src, ok);
+  for (int i = threadIdx.x; i < s.slots * 2 * CH; i += blockDim.x) {
+    const int r = i / (2 * CH), side = i / CH % 2, ch = i % CH;
+    *reinterpret_cast<uint4*>(sX + (r * s.pw + side * (s.pw - 1)) * PX + ch * 16) = make_uint4(0, 0, 0, 0);
+  }
+}
+// The input rows of a pass, a warp a row.
+template <int C>
+__device__ __forceinline__ void load_rows(const Shape& s, const Pass& ps, const __nv_bfloat16* x, uint8_t* sX) {
+  constexpr int CH = C / 8, PX = C * 2 + 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int r = warp; r < ps.rows; r += warps) {
+    const int g = ps.g0 + r, n = s.by_hp.div(g), h = g - n * (s.H + 2) - 1;
+    const bool ok = h >= 0 && h < s.H;
+    const __nv_bfloat16* src = ok ? x + ((int64_t)n * s.H + h) * s.W * C : x;
+    const uint32_t dst = smem_addr(sX + (r * s.pw + 1) * PX);
+    for (int i = lane; i < s.W * CH; i += 32) cp_async16(dst + (i / CH) * PX + (i % CH) * 16, src + (ok ? i * 8 : 0), ok);
   }
 }
 
-// y[pixel, CN] = sum over taps and CR channels; kT: the filters [CR][3][3][CN] are used transposed and rotated (data gradient).
+// A warp's share of the output: 16 pixels a time, NT tiles of 8 columns from column wn * NT * 8 on.
+template <int CR, int CN>
+struct Tile {
+  static constexpr int WN = CN == 64 ? 2 : 1, WM = kWarps / WN;      // warps along the output channels / along the pixels
+  static constexpr int NT = CN / WN / 8;
+  static constexpr int CHW = NT;                                     // 16-byte chunks of a pixel that a warp writes
+  static constexpr int UNITS = 16 * CHW / 32;                        // ... and how many of the 16 pixels' a lane has
+  static constexpr int PITCH = NT * 8 + 4;                           // floats of a pixel's row in the staging buffer
+  static constexpr int STAGE = 16 * PITCH * 4;                       // its bytes per warp
+  static constexpr bool kRegB = CR == 16 && CN == 16;                // the filters fit the registers
+};
+
+// Products of 16 pixels whose windows start at the lanes' address x0: acc = sum over taps and CR channels.
 template <int CR, int CN, bool kT>
-__global__ void __launch_bounds__(kThreads) conv_narrow_kernel(const Shape s, const Args a) {
-  constexpr int PX = CR * 2 + 16;                              // bytes of a pixel in shared memory
-  constexpr int CIN = kT ? CN : CR, COUT = kT ? CR : CN;       // filter storage [COUT][9][CIN]
-  constexpr int WR = CIN * 2 + 16;                             // bytes of a filter row (tap, output channel)
-  constexpr int WN = CN == 64 ? 2 : 1, WM = 8 / WN;            // warps along the output channels / along the pixels
-  constexpr int NT = CN / WN / 8;                              // 8-column tiles of a warp
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float s_stat[2 * CN];
-  uint8_t* sW = smem;                                          // [9][COUT] rows
-  uint8_t* sX = smem + 9 * COUT * WR;
-  esgd::pdl_enter();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = warp / WN, wn = warp % WN;
-  for (int i = threadIdx.x; i < 9 * COUT * (CIN / 8); i += kThreads) {      // filters: [COUT][9][CIN] -> [9][COUT][CIN]
-    const int ch = i % (CIN / 8), rest = i / (CIN / 8), tap = rest % 9, co = rest / 9;
-    cp_async16(smem_addr(sW + (tap * COUT + co) * WR + ch * 16), a.w + (int64_t)i * 8, true);
+struct Products {
+  using T = Tile<CR, CN>;
+  static constexpr int PX = CR * 2 + 16;                       // bytes of a pixel in shared memory
+  static constexpr int CIN = kT ? CN : CR, COUT = kT ? CR : CN;       // filter storage [COUT][9][CIN]
+  static constexpr int WR = CIN * 2 + 16;                      // bytes of a filter row (tap, output channel)
+  static constexpr int FILTER = 9 * COUT * WR;
+  uint32_t w0;
+  uint32_t breg[T::kRegB ? 9 : 1][4];
+  // filters: [COUT][9][CIN] -> [9][COUT][CIN]
+  static __device__ __forceinline__ void load_filters(const __nv_bfloat16* w, uint8_t* sW) {
+    constexpr int CH = CIN / 8;
+    for (int i = threadIdx.x; i < 9 * COUT * CH; i += blockDim.x) {
+      const int ch = i % CH, rest = i / CH, tap = rest % 9, co = rest / 9;
+      cp_async16(smem_addr(sW + (tap * COUT + co) * WR + ch * 16), w + i * 8, true);
+    }
   }
-  if (threadIdx.x < 2 * CN) s_stat[threadIdx.x] = 0.0f;
-  float st[NT][4];                                             // sum, sum, squares, squares of this thread's two columns
+  // fragments of two column tiles: rows are output columns (forward) or reduced channels (transposed)
+  __device__ __forceinline__ void begin(const uint8_t* sW, int wn, int lane) {
+    const uint32_t b_lane = kT ? (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * WR + ((lane >> 4) & 1) * 16 + wn * T::NT * 16)
+                               : (uint32_t)((wn * T::NT * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * WR + ((lane >> 3) & 1) * 16);
+    w0 = smem_addr(sW) + b_lane;
+    if constexpr (T::kRegB) {
 #pragma unroll
-  for (int t = 0; t < NT; ++t) st[t][0] = st[t][1] = st[t][2] = st[t][3] = 0.0f;
-  const int a_pix = (lane & 7) + ((lane >> 3) & 1) * 8, a_k = ((lane >> 4) & 1) * 16;
-  // filter fragments of two column tiles: rows are output columns (forward) or reduced channels (transposed)
-  const uint32_t b_lane = kT ? (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * WR + ((lane >> 4) & 1) * 16 + wn * NT * 16)
-                             : (uint32_t)((wn * NT * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * WR + ((lane >> 3) & 1) * 16);
-  const uint32_t w0 = smem_addr(sW) + b_lane;
-  const int pixels = s.ti * s.tr * s.Wo;
-  for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x) {
-    const int n0 = tile / s.row_tiles * s.ti, oh0 = tile % s.row_tiles * s.tr;
-    __syncthreads();                                           // the previous tile has been read
-    load_tile<CR>(a.x, s, n0, oh0, sX);
-    cp_async_wait();
-    __syncthreads();
-    for (int m = wm; m * 16 < pixels; m += WM) {
-      const int p = min(m * 16 + a_pix, pixels - 1);
-      const int im = p / (s.tr * s.Wo), q = p - im * s.tr * s.Wo, oh = q / s.Wo, ow = q - oh * s.Wo;
-      const uint32_t x0 = smem_addr(sX) + (uint32_t)(((im * s.rows + oh * s.stride) * s.pw + ow * s.stride) * PX + a_k);
-      float acc[NT][4];
+      for (int tap = 0; tap < 9; ++tap) fragment(breg[tap], tap, 0, 0);
+    }
+  }
+  __device__ __forceinline__ void fragment(uint32_t (&b)[4], int tap, int k, int t) const {
+    const uint32_t wt = w0 + (uint32_t)((kT ? 8 - tap : tap) * COUT * WR);
+    if (kT) ldm4t(b, wt + k * 16 * WR + t * 16);
+    else ldm4(b, wt + t * 8 * WR + k * 32);
+  }
+  __device__ __forceinline__ void run(float (&acc)[T::NT][4], uint32_t x0, uint32_t row_bytes) const {
 #pragma unroll
-      for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f;
-      // batch-norm input and mask of this thread's outputs: on their way while the products run
-      __nv_bfloat162 by[kT ? NT : 1][2];
-      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};           // bits 8t + (c % 8) of the thread's columns
-      if (kT && a.bn_y != nullptr) {
+    for (int t = 0; t < T::NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int pp = m * 16 + (lane >> 2) + h * 8, im2 = pp / (s.tr * s.Wo);
-          if (pp >= pixels || n0 + im2 >= s.N) continue;
-          const int64_t pix = ((int64_t)(n0 + im2) * s.Ho + oh0) * s.Wo + (pp - im2 * s.tr * s.Wo);
+    for (int tap = 0; tap < 9; ++tap) {
+      const uint32_t xt = x0 + (uint32_t)(tap / 3) * row_bytes + (tap % 3) * PX;
 #pragma unroll
-          for (int t = 0; t < NT; ++t)
-            by[t][h] = *reinterpret_cast<const __nv_bfloat162*>(a.bn_y + pix * CN + wn * NT * 8 + t * 8 + (lane & 3) * 2);
-          if (a.bn_mask != nullptr) {
-            const uint8_t* mp = a.bn_mask + pix * (CN / 8) + wn * NT;
-            keep[h] = NT == 2 ? *reinterpret_cast<const uint16_t*>(mp) : *reinterpret_cast<const uint32_t*>(mp);
+      for (int k = 0; k < CR / 16; ++k) {
+        uint32_t af[4];
+        ldm4(af, xt + k * 32);
+#pragma unroll
+        for (int t = 0; t < T::NT; t += 2) {
+          uint32_t bf[4];
+          if constexpr (T::kRegB) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) bf[q] = breg[tap][q];
+          } else {
+            fragment(bf, tap, k, t);
           }
-        }
-      }
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap) {
-        const uint32_t xt = x0 + (uint32_t)((tap / 3 * s.pw + tap % 3) * PX);
-        const uint32_t wt = w0 + (uint32_t)((kT ? 8 - tap : tap) * COUT * WR);
-#pragma unroll
-        for (int k = 0; k < CR / 16; ++k) {
-          uint32_t af[4];
-          ldm4(af, xt + k * 32);
-#pragma unroll
-          for (int t = 0; t < NT; t += 2) {
-            uint32_t bf[4];
-            if (kT) ldm4t(bf, wt + k * 16 * WR + t * 16);
-            else ldm4(bf, wt + t * 8 * WR + k * 32);
-            mma16816(acc[t], af, bf[0], bf[1]);
-            mma16816(acc[t + 1], af, bf[2], bf[3]);
-          }
-        }
-      }
-      // fragment rows lane / 4 and + 8, columns 2 * (lane % 4), + 1 of every column tile
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int pp = m * 16 + (lane >> 2) + h * 8;
-        const int im2 = pp / (s.tr * s.Wo);
-        if (pp >= pixels || n0 + im2 >= s.N) continue;
-        const int64_t pix = ((int64_t)(n0 + im2) * s.Ho + oh0) * s.Wo + (pp - im2 * s.tr * s.Wo);
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const int c = wn * NT * 8 + t * 8 + (lane & 3) * 2;
-          float v0 = acc[t][2 * h], v1 = acc[t][2 * h + 1];
-          if (a.scale != nullptr) {
-            v0 = fmaf(v0, __ldg(a.scale + c), __ldg(a.shift + c));
-            v1 = fmaf(v1, __ldg(a.scale + c + 1), __ldg(a.shift + c + 1));
-          }
-          if (a.residual != nullptr) {
-            const float2 r = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a.residual + pix * CN + c));
-            v0 += r.x;
-            v1 += r.y;
-          }
-          if (a.relu) { v0 = fmaxf(v0, 0.0f); v1 = fmaxf(v1, 0.0f); }
-          if (kT) {
-            const uint32_t bits = keep[h] >> (t * 8 + (lane & 3) * 2);
-            v0 = bits & 1u ? v0 : 0.0f;
-            v1 = bits & 2u ? v1 : 0.0f;
-          }
-          const __nv_bfloat162 o = __floats2bfloat162_rn(v0, v1);
-          *reinterpret_cast<__nv_bfloat162*>(a.y + pix * CN + c) = o;
-          if (a.sum != nullptr) {
-            const float2 f = __bfloat1622float2(o);
-            float2 g = f;
-            if (kT) {
-              g = __bfloat1622float2(by[kT ? t : 0][h]);
-              g.x -= __ldg(a.bn_aux + c);
-              g.y -= __ldg(a.bn_aux + c + 1);
-            }
-            st[t][0] += f.x; st[t][1] += f.y;
-            st[t][2] = fmaf(f.x, g.x, st[t][2]); st[t][3] = fmaf(f.y, g.y, st[t][3]);
-          }
+          mma16816(acc[t], af, bf[0], bf[1]);
+          mma16816(acc[t + 1], af, bf[2], bf[3]);
         }
       }
     }
   }
-  if (a.sum != nullptr) {      // lanes with equal lane % 4, then the block's warps, then one atomic per column and block
+};
+
+// What happens to 16 pixels' products: affine map, residual, ReLU or mask, rounding, store, sums.  A lane has eight channels
+// (its chunk) of UNITS pixels.
+template <int CR, int CN, bool kBn>
+struct Output {
+  using T = Tile<CR, CN>;
+  float s1[8], s2[8], neg_mean[kBn ? 8 : 1];
+  float* stage;
+  int lane, c0;                                                // c0: the lane's first channel
+  __device__ __forceinline__ void begin(const Args& a, uint8_t* stages, int warp, int wn) {
+    lane = threadIdx.x & 31;
+    stage = reinterpret_cast<float*>(stages + warp * T::STAGE);
+    c0 = wn * T::NT * 8 + lane % T::CHW * 8;
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
+    for (int q = 0; q < 8; ++q) {
+      s1[q] = s2[q] = 0.0f;
+      if (kBn) neg_mean[kBn ? q : 0] = a.bn_y != nullptr ? -__ldg(a.bn_aux + c0 + q) : 0.0f;
+    }
+  }
+  uint4 res[T::UNITS], by[kBn ? T::UNITS : 1];
+  uint32_t keep[kBn ? T::UNITS : 1];
+  __device__ __forceinline__ int pixel(int u) const { return lane / T::CHW + u * (32 / T::CHW); }
+  // the epilogue's operands, on their way while the products run; pix: the first of the 16 pixels, n: how many there are
+  __device__ __forceinline__ void prefetch(const Args& a, int64_t pix, int n) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float v = st[t][q];
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (lane < 4) atomicAdd(&s_stat[(q >> 1) * CN + wn * NT * 8 + t * 8 + lane * 2 + (q & 1)], v);
+    for (int u = 0; u < T::UNITS; ++u) {
+      if (pixel(u) >= n) continue;
+      const int64_t at = (pix + pixel(u)) * CN + c0;
+      if (a.residual != nullptr) res[u] = *reinterpret_cast<const uint4*>(a.residual + at);
+      if (kBn && a.bn_y != nullptr) {
+        by[kBn ? u : 0] = *reinterpret_cast<const uint4*>(a.bn_y + at);
+        keep[kBn ? u : 0] = a.bn_mask != nullptr ? a.bn_mask[at / 8] : 0xffu;
       }
+    }
+  }
+  __device__ __forceinline__ void finish(const Args& a, const float (&acc)[T::NT][4], int64_t pix, int n) {
+    // fragment rows lane / 4 and + 8, columns 2 * (lane % 4), + 1 of every column tile
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < T::NT; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float2*>(stage + ((lane >> 2) + h * 8) * T::PITCH + t * 8 + (lane & 3) * 2) = make_float2(acc[t][2 * h], acc[t][2 * h + 1]);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < T::UNITS; ++u) {
+      if (pixel(u) >= n) continue;
+      const float* src = stage + pixel(u) * T::PITCH + lane % T::CHW * 8;
+      const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+      float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      if (a.scale != nullptr) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = fmaf(v[q], __ldg(a.scale + c0 + q), __ldg(a.shift + c0 + q));
+      }
+      if (a.residual != nullptr) {
+        float r[8];
+        unpack8(res[u], r);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] += r[q];
+      }
+      if (a.relu) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = fmaxf(v[q], 0.0f);
+      }
+      if (kBn && a.bn_y != nullptr) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = (keep[kBn ? u : 0] >> q) & 1u ? v[q] : 0.0f;
+      }
+      const uint4 o = pack8(v);
+      *reinterpret_cast<uint4*>(a.y + (pix + pixel(u)) * CN + c0) = o;
+      if (a.sum != nullptr) {
+        float f[8], g[8];
+        unpack8(o, f);
+        if (kBn) {
+          unpack8(by[kBn ? u : 0], g);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) g[q] += neg_mean[kBn ? q : 0];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          s1[q] += f[q];
+          s2[q] = fmaf(f[q], kBn ? g[q] : f[q], s2[q]);
+        }
+      }
+    }
+  }
+  // The warps' sums meet in shared memory, then one atomic per column and block.  part: [WM][2][CN] floats
+  __device__ __forceinline__ void flush(const Args& a, float* part, int wm) {
+    if (a.sum == nullptr) return;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+#pragma unroll
+      for (int d = T::CHW; d < 32; d *= 2) {
+        s1[q] += __shfl_xor_sync(0xffffffffu, s1[q], d);
+        s2[q] += __shfl_xor_sync(0xffffffffu, s2[q], d);
+      }
+    if (lane < T::CHW) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        part[(wm * 2) * CN + c0 + q] = s1[q];
+        part[(wm * 2 + 1) * CN + c0 + q] = s2[q];
+      }
+    }
     __syncthreads();
     if (threadIdx.x < 2 * CN) {
-      const float scale = kT && threadIdx.x >= CN ? __ldg(a.bn_aux + threadIdx.x) : 1.0f;      // 1 / std
-      atomicAdd((threadIdx.x < CN ? a.sum : a.sqsum) + threadIdx.x % CN, s_stat[threadIdx.x] * scale);
+      float v = 0.0f;
+#pragma unroll
+      for (int m = 0; m < T::WM; ++m) v += part[m * 2 * CN + threadIdx.x];
+      if (kBn && threadIdx.x >= CN) v *= __ldg(a.bn_aux + threadIdx.x);      // 1 / std
+      atomicAdd((threadIdx.x < CN ? a.sum : a.sqsum) + threadIdx.x % CN, v);
     }
   }
+};
+
+// y[pixel, CN] = sum over taps and CR channels; kT: the filters [CR][3][3][CN] are used transposed and rotated (data gradient).
+template <int CR, int CN, bool kT>
+__global__ void __launch_bounds__(kThreads, 1) conv_narrow_kernel(const Shape s, const Args a) {
+  using T = Tile<CR, CN>;
+  using P = Products<CR, CN, kT>;
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint8_t* sW = smem;
+  uint8_t* sC = sW + P::FILTER;
+  float* part = reinterpret_cast<float*>(sC + kWarps * T::STAGE);
+  uint8_t* sX = reinterpret_cast<uint8_t*>(part + T::WM * 2 * CN);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = warp / T::WN, wn = warp % T::WN;
+  clear_margins<CR>(s, sX);
+  esgd::pdl_enter();
+  P::load_filters(a.w, sW);
+  P prod;
+  Output<CR, CN, kT> out;
+  out.begin(a, sC, warp, wn);
+  const int end = first_row(s, blockIdx.x + 1);
+  const int a_pix = (lane & 7) + ((lane >> 3) & 1) * 8, a_k = ((lane >> 4) & 1) * 16;
+  bool first = true;
+  for (int v0 = first_row(s, blockIdx.x); v0 < end; v0 += s.per_pass) {
+    const Pass ps(s, v0, min(v0 + s.per_pass, end));
+    if (!first) __syncthreads();                               // the previous pass has been read
+    load_rows<CR>(s, ps, a.x, sX);
+    cp_async_wait();
+    __syncthreads();
+    if (first) prod.begin(sW, wn, lane);
+    first = false;
+    const int pixels = (ps.v1 - ps.v0) * s.Wo;
+    const int64_t pix0 = (int64_t)ps.v0 * s.Wo;
+    for (int m = wm * 16; m < pixels; m += T::WM * 16) {
+      out.prefetch(a, pix0 + m, pixels - m);
+      const uint32_t x0 = smem_addr(sX) + (uint32_t)(ps.window(s, min(m + a_pix, pixels - 1)) * P::PX + a_k);
+      float acc[T::NT][4];
+      prod.run(acc, x0, (uint32_t)(s.pw * P::PX));
+      out.finish(a, acc, pix0 + m, pixels - m);
+    }
+  }
+  out.flush(a, part, wm);
 }
 
 // dw[CO][3][3][CI] (fp32, added to) = sum over pixels of dy[pixel, CO] x[pixel + tap, CI].  Both operands are read transposed
@@ -215,180 +364,210 @@ struct WgradPlan {
   static constexpr int TILES = (CO / 16) * (CI / 8);                  // accumulator tiles per tap
   static constexpr int TAPS = TILES <= 2 ? 9 : (TILES <= 8 ? 3 : 1);  // at most 96 accumulator registers
   static constexpr int SETS = 9 / TAPS;
-  static constexpr int SLICES = TAPS == 9 ? 8 : (TAPS == 3 ? 3 : 1);
+  static constexpr int SLICES = TAPS == 9 ? 16 : (TAPS == 3 ? 5 : 1);
   static constexpr int THREADS = SETS * SLICES * 32;
+  static constexpr int BANK = CO * 9 * CI;                            // floats
 };
 
 template <int CI, int CO>
-__global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS) wgrad_narrow_kernel(const Shape s, const __nv_bfloat16* __restrict__ x,
-                                                                                 const __nv_bfloat16* __restrict__ dy,
-                                                                                 float* __restrict__ dw) {
+struct Wgrad {
   using P = WgradPlan<CI, CO>;
-  constexpr int PX = CI * 2 + 16, PD = CO * 2 + 16, MT = CO / 16, NT = CI / 8;
-  extern __shared__ __align__(16) uint8_t smem[];
-  uint8_t* sX = smem;
-  uint8_t* sD = smem + s.ti * s.rows * s.pw * PX;
-  esgd::pdl_enter();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, set = warp % P::SETS, slice = warp / P::SETS;
+  static constexpr int PX = CI * 2 + 16, PD = CO * 2 + 16, MT = CO / 16, NT = CI / 8;
   float acc[P::TAPS][MT][NT][4];
+  int lane, set, slice;
+  __device__ __forceinline__ void begin() {
+    const int warp = threadIdx.x >> 5;
+    lane = threadIdx.x & 31;
+    set = warp % P::SETS;
+    slice = warp / P::SETS;
 #pragma unroll
-  for (int t = 0; t < P::TAPS; ++t)
+    for (int t = 0; t < P::TAPS; ++t)
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+      for (int i = 0; i < MT; ++i)
 #pragma unroll
-      for (int j = 0; j < NT; ++j) acc[t][i][j][0] = acc[t][i][j][1] = acc[t][i][j][2] = acc[t][i][j][3] = 0.0f;
-  const int d_pix = (lane & 7) + ((lane >> 4) & 1) * 8, d_col = ((lane >> 3) & 1) * 16;      // dy: [k][m] -> m x k fragments
-  const int x_pix = (lane & 7) + ((lane >> 3) & 1) * 8, x_col = ((lane >> 4) & 1) * 16;      // x:  [k][n] -> k x n fragments
-  const int pixels = s.ti * s.tr * s.Wo, padded = (pixels + 15) / 16 * 16;
-  for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x) {
-    const int n0 = tile / s.row_tiles * s.ti, oh0 = tile % s.row_tiles * s.tr;
-    __syncthreads();
-    {      // input rows with margin, and the tile's pixels of dy (zeros past the end)
-      constexpr int CH = CI / 8;
-      const int per_img = s.rows * s.pw * CH;
-      for (int i = threadIdx.x; i < s.ti * per_img; i += P::THREADS) {
-        const int im = i / per_img, j = i - im * per_img;
-        const int px = j / CH, ch = j - px * CH, row = px / s.pw, col = px - row * s.pw;
-        const int n = n0 + im, h = oh0 * s.stride - 1 + row, w = col - 1;
-        const bool ok = n < s.N && h >= 0 && h < s.H && w >= 0 && w < s.W;
-        cp_async16(smem_addr(sX + (im * s.rows * s.pw + px) * PX + ch * 16), ok ? x + (((int64_t)n * s.H + h) * s.W + w) * CI + ch * 8 : x, ok);
-      }
-      constexpr int CD = CO / 8;
-      for (int i = threadIdx.x; i < padded * CD; i += P::THREADS) {
-        const int px = i / CD, ch = i - px * CD, im = px / (s.tr * s.Wo);
-        const bool ok = px < pixels && n0 + im < s.N;
-        const int64_t pix = ((int64_t)(n0 + im) * s.Ho + oh0) * s.Wo + (px - im * s.tr * s.Wo);
-        cp_async16(smem_addr(sD + px * PD + ch * 16), ok ? dy + pix * CO + ch * 8 : dy, ok);
-      }
-    }
-    cp_async_wait();
-    __syncthreads();
-    for (int k = slice; k * 16 < pixels; k += P::SLICES) {
-      uint32_t af[MT][4];
-      const uint32_t d0 = smem_addr(sD + (k * 16 + d_pix) * PD + d_col);
+        for (int j = 0; j < NT; ++j) acc[t][i][j][0] = acc[t][i][j][1] = acc[t][i][j][2] = acc[t][i][j][3] = 0.0f;
+  }
+  // 16 pixels: d0 the lanes' address of dy ([k][m] -> m x k fragments), x0 that of their windows ([k][n] -> k x n fragments)
+  __device__ __forceinline__ void step(uint32_t d0, uint32_t x0, uint32_t row_bytes) {
+    uint32_t af[MT][4];
 #pragma unroll
-      for (int i = 0; i < MT; ++i) ldm4t(af[i], d0 + i * 32);
-      const int p = min(k * 16 + x_pix, pixels - 1);               // past the end dy is zero
-      const int im = p / (s.tr * s.Wo), q = p - im * s.tr * s.Wo, oh = q / s.Wo, ow = q - oh * s.Wo;
-      const uint32_t x0 = smem_addr(sX) + (uint32_t)(((im * s.rows + oh * s.stride) * s.pw + ow * s.stride) * PX + x_col);
+    for (int i = 0; i < MT; ++i) ldm4t(af[i], d0 + i * 32);
 #pragma unroll
-      for (int t = 0; t < P::TAPS; ++t) {
-        const int tap = set * P::TAPS + t;
-        const uint32_t xt = x0 + (uint32_t)((tap / 3 * s.pw + tap % 3) * PX);
+    for (int t = 0; t < P::TAPS; ++t) {
+      const int tap = set * P::TAPS + t;
+      const uint32_t xt = x0 + (uint32_t)(tap / 3) * row_bytes + (tap % 3) * PX;
 #pragma unroll
-        for (int j = 0; j < NT; j += 2) {
-          uint32_t bf[4];
-          ldm4t(bf, xt + j * 16);
+      for (int j = 0; j < NT; j += 2) {
+        uint32_t bf[4];
+        ldm4t(bf, xt + j * 16);
 #pragma unroll
-          for (int i = 0; i < MT; ++i) {
-            mma16816(acc[t][i][j], af[i], bf[0], bf[1]);
-            mma16816(acc[t][i][j + 1], af[i], bf[2], bf[3]);
-          }
+        for (int i = 0; i < MT; ++i) {
+          mma16816(acc[t][i][j], af[i], bf[0], bf[1]);
+          mma16816(acc[t][i][j + 1], af[i], bf[2], bf[3]);
         }
       }
     }
   }
-  // The pixel slices meet in shared memory, and the block adds its filter bank to dw with one bulk reduction.
-  float* bank = reinterpret_cast<float*>(smem);                      // [CO][9][CI]
-  __syncthreads();
-  for (int sl = 0; sl < P::SLICES; ++sl) {
-    if (slice == sl) {
+  __device__ __forceinline__ int d_pix() const { return (lane & 7) + ((lane >> 4) & 1) * 8; }
+  __device__ __forceinline__ int d_col() const { return ((lane >> 3) & 1) * 16; }
+  __device__ __forceinline__ int x_pix() const { return (lane & 7) + ((lane >> 3) & 1) * 8; }
+  __device__ __forceinline__ int x_col() const { return ((lane >> 4) & 1) * 16; }
+  // Every slice writes its sums to a bank of its own ([CO][9][CI]), all threads add the banks up, and the block adds the result to
+  // dw with one bulk reduction.
+  __device__ __forceinline__ void flush(float* banks, float* dw) {
+    float* bank = banks + slice * P::BANK;
 #pragma unroll
-      for (int t = 0; t < P::TAPS; ++t)
+    for (int t = 0; t < P::TAPS; ++t)
 #pragma unroll
-        for (int i = 0; i < MT; ++i)
+      for (int i = 0; i < MT; ++i)
 #pragma unroll
-          for (int j = 0; j < NT; ++j)
+        for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float2* d = reinterpret_cast<float2*>(bank + ((i * 16 + (lane >> 2) + h * 8) * 9 + set * P::TAPS + t) * CI + j * 8 + (lane & 3) * 2);
-              float2 v = make_float2(acc[t][i][j][2 * h], acc[t][i][j][2 * h + 1]);
-              if (sl > 0) { const float2 o = *d; v.x += o.x; v.y += o.y; }
-              *d = v;
-            }
+          for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float2*>(bank + ((i * 16 + (lane >> 2) + h * 8) * 9 + set * P::TAPS + t) * CI + j * 8 + (lane & 3) * 2) =
+                make_float2(acc[t][i][j][2 * h], acc[t][i][j][2 * h + 1]);
+    __syncthreads();
+    if (P::SLICES > 1) {
+      for (int i = threadIdx.x * 4; i < P::BANK; i += P::THREADS * 4) {
+        float4 v = *reinterpret_cast<const float4*>(banks + i);
+#pragma unroll
+        for (int sl = 1; sl < P::SLICES; ++sl) {
+          const float4 o = *reinterpret_cast<const float4*>(banks + sl * P::BANK + i);
+          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+        }
+        *reinterpret_cast<float4*>(banks + i) = v;
+      }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the bulk copy below reads what was written here
     __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dw), "r"(smem_addr(banks)),
+                   "r"((uint32_t)(P::BANK * 4)) : "memory");
+      asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+    }
   }
-  if (threadIdx.x == 0) {
-    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dw), "r"(smem_addr(bank)),
-                 "r"((uint32_t)(CO * 9 * CI * 4)) : "memory");
-    asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+};
+
+template <int CI, int CO>
+__global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS, 1) wgrad_narrow_kernel(const Shape s, const __nv_bfloat16* __restrict__ x,
+                                                                                     const __nv_bfloat16* __restrict__ dy,
+                                                                                     float* __restrict__ dw) {
+  using P = WgradPlan<CI, CO>;
+  using G = Wgrad<CI, CO>;
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint8_t* sX = smem;
+  uint8_t* sD = smem + s.slots * s.pw * G::PX;
+  clear_margins<CI>(s, sX);
+  esgd::pdl_enter();
+  G g;
+  g.begin();
+  const int end = first_row(s, blockIdx.x + 1);
+  bool first = true;
+  for (int v0 = first_row(s, blockIdx.x); v0 < end; v0 += s.per_pass) {
+    const Pass ps(s, v0, min(v0 + s.per_pass, end));
+    if (!first) __syncthreads();
+    first = false;
+    load_rows<CI>(s, ps, x, sX);
+    const int pixels = (ps.v1 - ps.v0) * s.Wo, padded = (pixels + 15) / 16 * 16;
+    constexpr int CD = CO / 8;
+    const __nv_bfloat16* d = dy + (int64_t)ps.v0 * s.Wo * CO;
+    for (int i = threadIdx.x; i < padded * CD; i += P::THREADS) {      // the pass's pixels of dy, zeros past the end
+      const bool ok = i < pixels * CD;
+      cp_async16(smem_addr(sD + i / CD * G::PD + i % CD * 16), d + (ok ? i * 8 : 0), ok);
+    }
+    cp_async_wait();
+    __syncthreads();
+    for (int k = g.slice * 16; k < pixels; k += P::SLICES * 16) {
+      const uint32_t d0 = smem_addr(sD + (k + g.d_pix()) * G::PD + g.d_col());
+      const uint32_t x0 = smem_addr(sX) + (uint32_t)(ps.window(s, min(k + g.x_pix(), pixels - 1)) * G::PX + g.x_col());     // past the end dy is zero
+      g.step(d0, x0, (uint32_t)(s.pw * G::PX));
+    }
   }
+  __syncthreads();                                                    // the banks lie where the rows were
+  g.flush(reinterpret_cast<float*>(smem), dw);
 }
 
-// Tiles of about `target` pixels: whole rows of an image, or whole images when they are small.  False: there is nothing to tile.
-bool plan(Shape& s, int N, int H, int W, int stride, int target, int min_tiles) {
-  if (N < 1 || H < 1 || W < 1 || stride < 1) return false;
-  s.N = N; s.H = H; s.W = W; s.stride = stride;
-  s.Ho = (H + 2 - 3) / stride + 1;
-  s.Wo = (W + 2 - 3) / stride + 1;
-  s.pw = W + 2;
-  const auto rows_of = [&](int px) {
-    int best = 1;
-    for (int d = 1; d <= s.Ho && d * s.Wo <= px; ++d) if (s.Ho % d == 0) best = d;
-    return best;
-  };
-  // smaller tiles rather than idle SMs
-  while (target > 64 && (int64_t)N * s.Ho * s.Wo / target < min_tiles) target /= 2;
-  s.tr = rows_of(target);
-  s.ti = 1;
-  if (s.tr == s.Ho) {
-    s.ti = target / (s.Ho * s.Wo);
-    if (s.ti < 1) s.ti = 1;
-    if (s.ti > N) s.ti = N;
-  }
-  s.rows = (s.tr - 1) * stride + 3;
-  s.row_tiles = s.Ho / s.tr;
-  s.tiles = s.row_tiles * ((N + s.ti - 1) / s.ti);
-  return true;
-}
-
-constexpr int kSmemMax = 200 * 1024;
+constexpr int kSmemMax = 220 * 1024;
 
 // Every load of an operand is 16 bytes wide (cp.async).
 bool aligned16(const void* a, const void* b) { return (((uintptr_t)a | (uintptr_t)b) & 15) == 0; }
 
-// Resident blocks per SM (kept per kernel for the newest shared-memory size; a layer's is always the same).
-struct Occupancy { std::atomic<uint64_t> last{0}; };
+// Input rows that `rows` consecutive output rows need at most: a window a row, and the rows between two images.
+int slots_of(const Shape& s, int rows) {
+  const int between = s.H + 2 - s.Ho * s.stride;
+  return (rows - 1) * s.stride + 3 + (between > 0 ? (rows - 2 + s.Ho) / s.Ho * between : 0);
+}
+
+// The blocks' rows; `fixed` bytes of shared memory beside `row_bytes` of every input row and `out_bytes` of every output row.
+// -1: there is nothing to compute; -100: one row at a time is too much.
+int plan(Shape& s, int& grid, int& smem, int N, int H, int W, int stride, int fixed, int row_bytes, int out_bytes) {
+  if (N < 1 || H < 1 || W < 1 || stride < 1) return -1;
+  s.N = N; s.H = H; s.W = W; s.stride = stride;
+  s.Ho = (H + 2 - 3) / stride + 1;
+  s.Wo = (W + 2 - 3) / stride + 1;
+  s.pw = W + 2;
+  if ((int64_t)N * (H + 2) * s.pw >= (int64_t)1 << 30) return -100;
+  s.total = N * s.Ho;
+  s.by_wo = FastDiv((uint32_t)s.Wo);
+  s.by_ho = FastDiv((uint32_t)s.Ho);
+  s.by_hp = FastDiv((uint32_t)(H + 2));
+  const int sms = esgd::sm_count();
+  grid = s.total < sms ? s.total : sms;
+  const auto bytes = [&](int rows) { return (int64_t)fixed + (int64_t)slots_of(s, rows) * row_bytes + (int64_t)rows * out_bytes; };
+  int rows = (s.total + grid - 1) / grid;
+  if (bytes(1) > kSmemMax) return -100;
+  if (bytes(rows) > kSmemMax) {               // equal passes
+    int passes = 2;
+    while (bytes((rows + passes - 1) / passes) > kSmemMax) ++passes;
+    rows = (rows + passes - 1) / passes;
+  }
+  s.per_pass = rows;
+  s.slots = slots_of(s, rows);
+  smem = (int)bytes(rows);
+  return 0;
+}
+
+// More than 48 KB of shared memory has to be asked for, once per kernel and device.
+using Allowed = std::atomic<uint64_t>;
 template <class K>
-int blocks_per_sm(K kernel, int threads, int smem, Occupancy& o) {
-  const uint64_t seen = o.last.load(std::memory_order_relaxed);
-  if ((int)(seen >> 32) == smem) return (int)(seen & 0xffffffffu);
+void allow_smem(K kernel, Allowed& devices) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t bit = 1ull << (dev & 63);
+  if (devices.load(std::memory_order_relaxed) & bit) return;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess || n < 1) n = 1;
-  o.last.store(((uint64_t)smem << 32) | (uint64_t)n, std::memory_order_relaxed);
-  return n;
+  devices.fetch_or(bit, std::memory_order_relaxed);
 }
 
 template <int CR, int CN, bool kT>
 int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t stream) {
-  static Occupancy occ;
+  using T = Tile<CR, CN>;
+  using P = Products<CR, CN, kT>;
   Shape s;
-  if (!plan(s, N, H, W, stride, 256, esgd::sm_count())) return -1;
-  if (!aligned16(a.x, a.w)) return -100;
-  const int cin = kT ? CN : CR, cout = kT ? CR : CN;
-  const int smem = 9 * cout * (cin * 2 + 16) + s.ti * s.rows * s.pw * (CR * 2 + 16);
-  if (smem > kSmemMax) return -100;
-  const int resident = blocks_per_sm(conv_narrow_kernel<CR, CN, kT>, kThreads, smem, occ) * esgd::sm_count();
-  return esgd::launch(conv_narrow_kernel<CR, CN, kT>, dim3(s.tiles < resident ? s.tiles : resident), kThreads, smem, stream, s, a);
+  int grid, smem;
+  const int rc = plan(s, grid, smem, N, H, W, stride, P::FILTER + kWarps * T::STAGE + T::WM * 2 * CN * 4, (W + 2) * P::PX, 0);
+  if (rc != 0) return rc;
+  if (!aligned16(a.x, a.w) || !aligned16(a.y, a.residual) || !aligned16(a.bn_y, nullptr)) return -100;
+  static Allowed allowed{0};
+  allow_smem(conv_narrow_kernel<CR, CN, kT>, allowed);
+  return esgd::launch(conv_narrow_kernel<CR, CN, kT>, dim3(grid), kThreads, smem, stream, s, a);
 }
 
 template <int CI, int CO>
 int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int stride, cudaStream_t stream) {
-  static Occupancy occ;
+  using P = WgradPlan<CI, CO>;
+  using G = Wgrad<CI, CO>;
   Shape s;
-  if (!plan(s, N, H, W, stride, 256, esgd::sm_count())) return -1;
+  int grid, smem;
+  const int wo = stride < 1 ? 0 : (W + 2 - 3) / stride + 1;
+  const int rc = plan(s, grid, smem, N, H, W, stride, 16 * G::PD, (W + 2) * G::PX, wo * G::PD);
+  if (rc != 0) return rc;
   if (!aligned16(x, dy)) return -100;
-  const int px = (s.ti * s.tr * s.Wo + 15) / 16 * 16;
-  int smem = s.ti * s.rows * s.pw * (CI * 2 + 16) + px * (CO * 2 + 16);
-  if (smem < CO * 9 * CI * 4) smem = CO * 9 * CI * 4;
-  if (smem > kSmemMax) return -100;
-  blocks_per_sm(wgrad_narrow_kernel<CI, CO>, WgradPlan<CI, CO>::THREADS, smem, occ);
-  // one block per SM at most: every block ends with a reduction of the whole filter bank
-  const int grid = s.tiles < esgd::sm_count() ? s.tiles : esgd::sm_count();
-  return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), WgradPlan<CI, CO>::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
+  const int banks = P::SLICES * P::BANK * 4;
+  if (smem < banks) smem = banks;
+  static Allowed allowed{0};
+  allow_smem(wgrad_narrow_kernel<CI, CO>, allowed);
+  return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), P::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
                       (const __nv_bfloat16*)dy, dw);
 }
 

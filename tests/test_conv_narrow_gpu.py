@@ -35,3 +35,10 @@ def test_conv_narrow(n, ci, h, w, co, stride):
     check_error(y.device)
     assert (x.grad.float() - xr.grad).norm() < 6e-3 * xr.grad.norm()
     assert (wt.grad.float() - wr.grad).norm() < 6e-3 * wr.grad.norm()
+
+
+@pytest.mark.parametrize("n,ci,h,w,co,stride", [(700, 16, 32, 32, 16, 1), (1500, 32, 16, 16, 32, 1), (400, 16, 33, 31, 32, 2), (300, 16, 5, 3, 32, 2),
+                                                (149, 32, 1, 17, 32, 1), (147, 16, 1, 1, 16, 1), (90, 32, 3, 50, 64, 2), (37, 64, 2, 29, 64, 1)])
+def test_runs_of_rows(n, ci, h, w, co, stride):
+    """Runs of output rows that are longer than shared memory (several passes), that span many images, and that are one row."""
+    test_conv_narrow(n, ci, h, w, co, stride)
