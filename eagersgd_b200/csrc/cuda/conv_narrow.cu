@@ -15,8 +15,8 @@
 // reads padded rows n * (H + 2) + oh * stride and the two after it.
 //
 // Microseconds with sums, tiles of 256 pixels with their own index arithmetic -> now: 128 x 32 x 32, 16 channels, forward
-// 15.4 -> 6.6, data gradient with batch norm 14.6 -> 7.0, weight gradient 12.3 -> 8.0; 128 x 16 x 16, 32 channels 8.6 -> 5.4, 11.1 -> 6.5,
-// 12.9 -> 11.0.
+// 15.4 -> 6.6, data gradient with batch norm 14.6 -> 7.0, weight gradient 12.3 -> 7.4; 128 x 16 x 16, 32 channels 8.6 -> 5.4, 11.1 -> 6.5,
+// 12.9 -> 7.8.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -364,9 +364,11 @@ struct WgradPlan {
   static constexpr int TILES = (CO / 16) * (CI / 8);                  // accumulator tiles per tap
   static constexpr int TAPS = TILES <= 2 ? 9 : (TILES <= 8 ? 3 : 1);  // at most 96 accumulator registers
   static constexpr int SETS = 9 / TAPS;
-  static constexpr int SLICES = TAPS == 9 ? 16 : (TAPS == 3 ? 5 : 1);
+  static constexpr int SLICES = TAPS == 9 ? 16 : (TAPS == 3 ? 4 : 1);      // (five banks of 32 channels would not fit shared memory)
   static constexpr int THREADS = SETS * SLICES * 32;
   static constexpr int BANK = CO * 9 * CI;                            // floats
+  static constexpr int PITCH = 9 * CI + 8;                            // of an output channel in a slice's bank
+  static constexpr int BYTES = (SLICES * CO * PITCH + BANK) * 4;
 };
 
 template <int CI, int CO>
@@ -412,10 +414,10 @@ struct Wgrad {
   __device__ __forceinline__ int d_col() const { return ((lane >> 3) & 1) * 16; }
   __device__ __forceinline__ int x_pix() const { return (lane & 7) + ((lane >> 3) & 1) * 8; }
   __device__ __forceinline__ int x_col() const { return ((lane >> 4) & 1) * 16; }
-  // Every slice writes its sums to a bank of its own ([CO][9][CI]), all threads add the banks up, and the block adds the result to
-  // dw with one bulk reduction.
-  __device__ __forceinline__ void flush(float* banks, float* dw) {
-    float* bank = banks + slice * P::BANK;
+  // Every slice writes its sums to a bank of its own ([CO][9][CI], output channels a multiple of 32 words plus 8 apart: without
+  // the 8 a store went to one bank eight times, 5 of the 11 us of 32 channels) ...
+  __device__ __forceinline__ void collect(float* banks) {
+    float* bank = banks + slice * (CO * P::PITCH);
 #pragma unroll
     for (int t = 0; t < P::TAPS; ++t)
 #pragma unroll
@@ -424,25 +426,32 @@ struct Wgrad {
         for (int j = 0; j < NT; ++j)
 #pragma unroll
           for (int h = 0; h < 2; ++h)
-            *reinterpret_cast<float2*>(bank + ((i * 16 + (lane >> 2) + h * 8) * 9 + set * P::TAPS + t) * CI + j * 8 + (lane & 3) * 2) =
+            *reinterpret_cast<float2*>(bank + (i * 16 + (lane >> 2) + h * 8) * P::PITCH + (set * P::TAPS + t) * CI + j * 8 + (lane & 3) * 2) =
                 make_float2(acc[t][i][j][2 * h], acc[t][i][j][2 * h + 1]);
-    __syncthreads();
-    if (P::SLICES > 1) {
-      for (int i = threadIdx.x * 4; i < P::BANK; i += P::THREADS * 4) {
-        float4 v = *reinterpret_cast<const float4*>(banks + i);
+  }
+  // ... which all threads add up once they are there; the block adds the result to dw by bulk reductions, blocks in turn beginning
+  // at another place.
+  static __device__ __forceinline__ void commit(float* banks, float* dw) {
+    float* sum = banks + P::SLICES * (CO * P::PITCH);
+    for (int i = threadIdx.x * 4; i < P::BANK; i += blockDim.x * 4) {
+      const float* at = banks + i + i / (9 * CI) * 8;
+      float4 v = *reinterpret_cast<const float4*>(at);
 #pragma unroll
-        for (int sl = 1; sl < P::SLICES; ++sl) {
-          const float4 o = *reinterpret_cast<const float4*>(banks + sl * P::BANK + i);
-          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-        }
-        *reinterpret_cast<float4*>(banks + i) = v;
+      for (int sl = 1; sl < P::SLICES; ++sl) {
+        const float4 o = *reinterpret_cast<const float4*>(at + sl * (CO * P::PITCH));
+        v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
       }
+      *reinterpret_cast<float4*>(sum + i) = v;
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the bulk copy below reads what was written here
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the bulk copies below read what was written here
     __syncthreads();
     if (threadIdx.x == 0) {
-      asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dw), "r"(smem_addr(banks)),
-                   "r"((uint32_t)(P::BANK * 4)) : "memory");
+      constexpr int PARTS = 4, PART = P::BANK / PARTS;
+      for (int i = 0; i < PARTS; ++i) {
+        const int at = (i + (int)blockIdx.x) % PARTS * PART;
+        asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dw + at), "r"(smem_addr(sum + at)),
+                     "r"((uint32_t)(PART * 4)) : "memory");
+      }
       asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
     }
   }
@@ -484,7 +493,9 @@ __global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS, 1) wgrad_narrow_ke
     }
   }
   __syncthreads();                                                    // the banks lie where the rows were
-  g.flush(reinterpret_cast<float*>(smem), dw);
+  g.collect(reinterpret_cast<float*>(smem));
+  __syncthreads();
+  G::commit(reinterpret_cast<float*>(smem), dw);
 }
 
 constexpr int kSmemMax = 220 * 1024;
@@ -563,8 +574,7 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
   const int rc = plan(s, grid, smem, N, H, W, stride, 16 * G::PD, (W + 2) * G::PX, wo * G::PD);
   if (rc != 0) return rc;
   if (!aligned16(x, dy)) return -100;
-  const int banks = P::SLICES * P::BANK * 4;
-  if (smem < banks) smem = banks;
+  if (smem < P::BYTES) smem = P::BYTES;
   static Allowed allowed{0};
   allow_smem(wgrad_narrow_kernel<CI, CO>, allowed);
   return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), P::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
