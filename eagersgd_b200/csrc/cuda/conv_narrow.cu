@@ -1,5 +1,5 @@
 // 3x3 convolutions of 16 and 32 channels over small images (the CIFAR ResNets): forward, data gradient, weight gradient; 64
-// channels in small forward problems.
+// channels in small problems, forward and data gradient.
 //
 // A layer of 128 x 32 x 32 pixels and 16 channels is 0.6 GFLOP over 8 MB that sit in L2: it is bound by latency and by the
 // instructions around the products, and the 128-row tcgen05 tiles fed 64 channels at a time spent 33 us on it, three quarters of
@@ -585,12 +585,12 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
 
 extern "C" {
 
-// 64 input channels fill a k-block of the tile kernels, and only small forward problems are better off here.  Microseconds back
-// to back, rows in shared memory / tiles: 8 x 8 pixels, 64 images, inference epilogue 7.7 / 9.0, statistics 8.2 / 8.2; 96
-// images 9.0 / 9.5 and 9.6 / 8.2; 14 x 14, 16 images (3136 pixels) 7.8 / 9.0 and 7.5 / 8.4, 32 images 10.6 / 9.1 and
-// 11.6 / 8.5; 8 x 8, 512 images 18.6 / 12.4.  The data gradient with its batch norm lost from the first image on (8.8 / 7.7 at
-// 8 x 8, 20.2 / 13.8 at 512 images) and is the tile kernels'.
-constexpr int64_t kMaxPixels64 = 4096;
+// 64 input channels fill a k-block of the tile kernels, and only small problems are better off here.  Microseconds back to back,
+// rows in shared memory / tiles, forward with sums, inference epilogue with a shortcut, data gradient with batch norm: 8 x 8
+// pixels, one image 4.1 / 6.4, 3.6 / 8.6, 4.4 / 7.5; 64 images 5.4 / 6.5, 5.0 / 8.6, 6.2 / 7.6; 128 images (8192 pixels) 6.7 /
+// 6.7, 6.5 / 8.9, 7.6 / 8.1; 512 images 12.4 / 11.9, 12.8 / 13.4, 13.6 / 13.4; 56 x 56, one image 5.7 / 6.5, 5.5 / 8.7, 6.2 /
+// 7.6; two 6.9 / 6.6, 6.6 / 8.8, 7.4 / 7.8; four 8.5 / 6.9, 8.4 / 8.9, 9.3 / 8.1; eight 12.3 / 8.6, 12.8 / 9.5, 13.1 / 9.8.
+constexpr int64_t kMaxPixels64 = 8192;
 
 // Returns -100 for shapes this file does not take (the caller then uses the tile kernels).  3x3, padding 1, NHWC bf16.
 // y = act(scale * conv + shift + residual), each part optional; sum / sqsum (caller-zeroed) receive y's statistics.
@@ -619,6 +619,7 @@ int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H
   cudaStream_t s = (cudaStream_t)stream;
   if (Cin == 16 && Cout == 16) return launch_conv<16, 16, true>(a, N, H, W, 1, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, true>(a, N, H, W, 1, s);
+  if (Cin == 64 && Cout == 64 && (int64_t)N * H * W <= kMaxPixels64) return launch_conv<64, 64, true>(a, N, H, W, 1, s);
   return -100;
 }
 
