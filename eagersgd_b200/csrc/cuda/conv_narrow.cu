@@ -131,10 +131,91 @@ __device__ __forceinline__ void load_rows(const Shape& s, const Pass& ps, const 
   }
 }
 
+// The batch norm in front of a convolution, applied to its rows on their way into shared memory: z = act(scale * y + shift), which
+// is also stored, with its mask, for the backward pass.  As esgd_bn_fwd takes it, without a residual.
+struct BnOutput {
+  const __nv_bfloat16* y;                                      // the convolution's input is z
+  __nv_bfloat16* z;
+  uint8_t* mask;
+  const float *sum, *sqsum, *gamma, *beta;
+  float *running_mean, *running_var, *aux;
+  float inv_count, unbias, momentum, eps;
+  int relu;
+};
+// coef: [2][C] floats of shared memory
+template <int C>
+__device__ __forceinline__ void bn_coefficients(const BnOutput& b, float* coef) {
+  if (threadIdx.x >= C) return;
+  const int c = threadIdx.x;
+  const float mean = b.sum[c] * b.inv_count, var = fmaxf(b.sqsum[c] * b.inv_count - mean * mean, 0.0f), invstd = rsqrtf(var + b.eps);
+  const float sc = b.gamma[c] * invstd, sh = b.beta[c] - mean * sc;
+  coef[c] = sc;
+  coef[C + c] = sh;
+  if (blockIdx.x == 0) {
+    b.aux[c] = mean;
+    b.aux[C + c] = invstd;
+    b.aux[2 * C + c] = sc;
+    b.aux[3 * C + c] = sh;
+    if (b.running_mean != nullptr) {
+      b.running_mean[c] = (1.0f - b.momentum) * b.running_mean[c] + b.momentum * mean;
+      b.running_var[c] = (1.0f - b.momentum) * b.running_var[c] + b.momentum * var * b.unbias;
+    }
+  }
+}
+template <int C>
+__device__ __forceinline__ void load_z_rows(const Shape& s, const Pass& ps, const BnOutput& b, const float* coef, uint8_t* sX) {
+  constexpr int CH = C / 8, PX = C * 2 + 16, COLS = 4;         // loads in flight a lane
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, n = s.W * CH;
+  float sc[8], sh[8];                                          // every load of a lane is of the same channels
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    sc[q] = coef[lane % CH * 8 + q];
+    sh[q] = coef[C + lane % CH * 8 + q];
+  }
+  for (int r = warp; r < ps.rows; r += warps) {
+    const int g = ps.g0 + r, im = s.by_hp.div(g), h = g - im * (s.H + 2) - 1, row = im * s.H + h;
+    const bool ok = h >= 0 && h < s.H, mine = ok && row >= ps.v0 && row < ps.v1;       // stride 1: output rows are input rows
+    const int64_t at = ok ? (int64_t)row * s.W * C : 0;
+    for (int i0 = lane; i0 < n; i0 += 32 * COLS) {
+      uint4 ry[COLS];
+#pragma unroll
+      for (int k = 0; k < COLS; ++k)
+        if (ok && i0 + k * 32 < n) ry[k] = *reinterpret_cast<const uint4*>(b.y + at + (i0 + k * 32) * 8);
+#pragma unroll
+      for (int k = 0; k < COLS; ++k) {
+        const int i = i0 + k * 32;
+        if (i >= n) continue;
+        uint4 out = make_uint4(0, 0, 0, 0);                    // rows outside the image
+        if (ok) {
+          float v[8];
+          unpack8(ry[k], v);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            v[q] = v[q] * sc[q] + sh[q];
+            if (b.relu) v[q] = fmaxf(v[q], 0.0f);
+          }
+          out = pack8(v);
+        }
+        *reinterpret_cast<uint4*>(sX + (r * s.pw + 1 + i / CH) * PX + i % CH * 16) = out;
+        if (mine) {
+          *reinterpret_cast<uint4*>(b.z + at + i * 8) = out;
+          if (b.mask != nullptr) {
+            const uint32_t x[4] = {out.x, out.y, out.z, out.w};
+            uint32_t m = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) m |= ((x[q] & 0x7fffu) ? 1u << (2 * q) : 0u) | ((x[q] & 0x7fff0000u) ? 2u << (2 * q) : 0u);
+            b.mask[at / 8 + i] = (uint8_t)m;
+          }
+        }
+      }
+    }
+  }
+}
+
 // A warp's share of the output: 16 pixels a time, NT tiles of 8 columns from column wn * NT * 8 on.
-template <int CR, int CN>
+template <int CR, int CN, int WARPS = kWarps>
 struct Tile {
-  static constexpr int WN = CN == 64 ? 2 : 1, WM = kWarps / WN;      // warps along the output channels / along the pixels
+  static constexpr int WN = CN == 64 ? 2 : 1, WM = WARPS / WN;       // warps along the output channels / along the pixels
   static constexpr int NT = CN / WN / 8;
   static constexpr int CHW = NT;                                     // 16-byte chunks of a pixel that a warp writes
   static constexpr int UNITS = 16 * CHW / 32;                        // ... and how many of the 16 pixels' a lane has
@@ -205,9 +286,9 @@ struct Products {
 
 // What happens to 16 pixels' products: affine map, residual, ReLU or mask, rounding, store, sums.  A lane has eight channels
 // (its chunk) of UNITS pixels.
-template <int CR, int CN, bool kBn>
+template <int CR, int CN, bool kBn, int WARPS = kWarps>
 struct Output {
-  using T = Tile<CR, CN>;
+  using T = Tile<CR, CN, WARPS>;
   float s1[8], s2[8], neg_mean[kBn ? 8 : 1];
   float* stage;
   int lane, c0;                                                // c0: the lane's first channel
@@ -288,8 +369,8 @@ struct Output {
       }
     }
   }
-  // The warps' sums meet in shared memory, then one atomic per column and block.  part: [WM][2][CN] floats
-  __device__ __forceinline__ void flush(const Args& a, float* part, int wm) {
+  // The warps' sums meet in shared memory (part: [WM][2][CN] floats), then one atomic per column and block.
+  __device__ __forceinline__ void collect(const Args& a, float* part, int wm) {
     if (a.sum == nullptr) return;
 #pragma unroll
     for (int q = 0; q < 8; ++q)
@@ -305,31 +386,37 @@ struct Output {
         part[(wm * 2 + 1) * CN + c0 + q] = s2[q];
       }
     }
-    __syncthreads();
-    if (threadIdx.x < 2 * CN) {
-      float v = 0.0f;
+  }
+  static __device__ __forceinline__ void commit(const Args& a, const float* part) {
+    if (a.sum == nullptr || threadIdx.x >= 2 * CN) return;
+    float v = 0.0f;
 #pragma unroll
-      for (int m = 0; m < T::WM; ++m) v += part[m * 2 * CN + threadIdx.x];
-      if (kBn && threadIdx.x >= CN) v *= __ldg(a.bn_aux + threadIdx.x);      // 1 / std
-      atomicAdd((threadIdx.x < CN ? a.sum : a.sqsum) + threadIdx.x % CN, v);
-    }
+    for (int m = 0; m < T::WM; ++m) v += part[m * 2 * CN + threadIdx.x];
+    if (kBn && threadIdx.x >= CN) v *= __ldg(a.bn_aux + threadIdx.x);      // 1 / std
+    atomicAdd((threadIdx.x < CN ? a.sum : a.sqsum) + threadIdx.x % CN, v);
   }
 };
 
 // y[pixel, CN] = sum over taps and CR channels; kT: the filters [CR][3][3][CN] are used transposed and rotated (data gradient).
-template <int CR, int CN, bool kT>
-__global__ void __launch_bounds__(kThreads, 1) conv_narrow_kernel(const Shape s, const Args a) {
+// kBnIn: the input is a batch norm's output, made here (the 4 us of a launch of its own between two convolutions).
+template <int CR, int CN, bool kT, bool kBnIn>
+__global__ void __launch_bounds__(kThreads, 1) conv_narrow_kernel(const Shape s, const Args a, const BnOutput b) {
   using T = Tile<CR, CN>;
   using P = Products<CR, CN, kT>;
   extern __shared__ __align__(16) uint8_t smem[];
   uint8_t* sW = smem;
   uint8_t* sC = sW + P::FILTER;
   float* part = reinterpret_cast<float*>(sC + kWarps * T::STAGE);
-  uint8_t* sX = reinterpret_cast<uint8_t*>(part + T::WM * 2 * CN);
+  float* coef = part + T::WM * 2 * CN;
+  uint8_t* sX = reinterpret_cast<uint8_t*>(coef + (kBnIn ? 2 * CR : 0));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wm = warp / T::WN, wn = warp % T::WN;
   clear_margins<CR>(s, sX);
   esgd::pdl_enter();
   P::load_filters(a.w, sW);
+  if (kBnIn) {
+    bn_coefficients<CR>(b, coef);
+    __syncthreads();
+  }
   P prod;
   Output<CR, CN, kT> out;
   out.begin(a, sC, warp, wn);
@@ -339,7 +426,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_narrow_kernel(const Shape s,
   for (int v0 = first_row(s, blockIdx.x); v0 < end; v0 += s.per_pass) {
     const Pass ps(s, v0, min(v0 + s.per_pass, end));
     if (!first) __syncthreads();                               // the previous pass has been read
-    load_rows<CR>(s, ps, a.x, sX);
+    if constexpr (kBnIn) load_z_rows<CR>(s, ps, b, coef, sX);
+    else load_rows<CR>(s, ps, a.x, sX);
     cp_async_wait();
     __syncthreads();
     if (first) prod.begin(sW, wn, lane);
@@ -354,31 +442,32 @@ __global__ void __launch_bounds__(kThreads, 1) conv_narrow_kernel(const Shape s,
       out.finish(a, acc, pix0 + m, pixels - m);
     }
   }
-  out.flush(a, part, wm);
+  out.collect(a, part, wm);
+  __syncthreads();
+  out.commit(a, part);
 }
 
 // dw[CO][3][3][CI] (fp32, added to) = sum over pixels of dy[pixel, CO] x[pixel + tap, CI].  Both operands are read transposed
 // from their pixel rows.  A warp keeps the accumulators of TAPS taps; the warps of a tap group share the pixels.
-template <int CI, int CO>
+template <int CI, int CO, int WARPS = kWarps>
 struct WgradPlan {
   static constexpr int TILES = (CO / 16) * (CI / 8);                  // accumulator tiles per tap
   static constexpr int TAPS = TILES <= 2 ? 9 : (TILES <= 8 ? 3 : 1);  // at most 96 accumulator registers
   static constexpr int SETS = 9 / TAPS;
-  static constexpr int SLICES = TAPS == 9 ? 16 : (TAPS == 3 ? 4 : 1);      // (five banks of 32 channels would not fit shared memory)
+  static constexpr int SLICES = SETS == 3 && WARPS > 12 ? 4 : WARPS / SETS;      // (five banks of 32 channels would not fit shared memory)
   static constexpr int THREADS = SETS * SLICES * 32;
   static constexpr int BANK = CO * 9 * CI;                            // floats
   static constexpr int PITCH = 9 * CI + 8;                            // of an output channel in a slice's bank
   static constexpr int BYTES = (SLICES * CO * PITCH + BANK) * 4;
 };
 
-template <int CI, int CO>
+template <int CI, int CO, int WARPS = kWarps>
 struct Wgrad {
-  using P = WgradPlan<CI, CO>;
+  using P = WgradPlan<CI, CO, WARPS>;
   static constexpr int PX = CI * 2 + 16, PD = CO * 2 + 16, MT = CO / 16, NT = CI / 8;
   float acc[P::TAPS][MT][NT][4];
   int lane, set, slice;
-  __device__ __forceinline__ void begin() {
-    const int warp = threadIdx.x >> 5;
+  __device__ __forceinline__ void begin(int warp) {
     lane = threadIdx.x & 31;
     set = warp % P::SETS;
     slice = warp / P::SETS;
@@ -469,7 +558,7 @@ __global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS, 1) wgrad_narrow_ke
   clear_margins<CI>(s, sX);
   esgd::pdl_enter();
   G g;
-  g.begin();
+  g.begin(threadIdx.x >> 5);
   const int end = first_row(s, blockIdx.x + 1);
   bool first = true;
   for (int v0 = first_row(s, blockIdx.x); v0 < end; v0 += s.per_pass) {
@@ -496,6 +585,160 @@ __global__ void __launch_bounds__(WgradPlan<CI, CO>::THREADS, 1) wgrad_narrow_ke
   g.collect(reinterpret_cast<float*>(smem));
   __syncthreads();
   G::commit(reinterpret_cast<float*>(smem), dw);
+}
+
+// ---------------------------------------------------------------- a layer's whole backward pass
+// Batch norm, data gradient and weight gradient of a stride-1 layer of C channels in one launch: the rows of the batch norm's
+// gradient dy = a * dz + b * y + c are made on their way into shared memory (bf16, as a pass of its own would store them) and
+// read there by eight warps that multiply them with the filters and by six or eight that multiply them with the input's rows.
+// A block has one pass (with several the accumulators would have to outlive the loads, for which there are no registers):
+// launch_bwd() refuses problems of more rows than that.  Microseconds, three launches (4.6 + 7.0 + 7.4) -> this one: 128 x 32 x 32, 16
+// channels 19.0 -> 11.9; 128 x 16 x 16, 32 channels 17.6 -> 12.3.  The third ran on a stream of its own but did not overlap: each
+// of them fills the SMs.
+struct BnInput {
+  const __nv_bfloat16 *dz, *y;
+  const float *aux, *gamma, *dbeta, *dgamma;                   // as esgd_bn_bwd_apply takes them
+  float *acc_dgamma, *acc_dbeta;
+  float inv_count;
+};
+
+template <int C>
+__device__ __forceinline__ void load_dy_rows(const Shape& s, const Pass& ps, const BnInput& b, const float* coef, uint8_t* sD) {
+  constexpr int CH = C / 8, PX = C * 2 + 16, ROWS = 2, COLS = 2;      // eight loads in flight a lane
+  float ca[8], cb[8], cc[8];                                   // every load of a lane is of the same channels
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int c = (int)(threadIdx.x & 31) % CH * 8 + q;
+    ca[q] = coef[c];
+    cb[q] = coef[C + c];
+    cc[q] = coef[2 * C + c];
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5, n = s.W * CH;
+  for (int r0 = warp; r0 < ps.rows; r0 += ROWS * warps) {
+    const __nv_bfloat16 *dz[ROWS], *y[ROWS];
+    bool ok[ROWS];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+      const int g = ps.g0 + r0 + j * warps, im = s.by_hp.div(g), h = g - im * (s.H + 2) - 1;
+      ok[j] = r0 + j * warps < ps.rows && h >= 0 && h < s.H;
+      const int64_t at = ok[j] ? ((int64_t)im * s.H + h) * s.W * C : 0;
+      dz[j] = b.dz + at;
+      y[j] = b.y + at;
+    }
+    for (int i0 = lane; i0 < n; i0 += 32 * COLS) {
+      uint4 rd[ROWS][COLS], ry[ROWS][COLS];
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+        for (int k = 0; k < COLS; ++k)
+          if (ok[j] && i0 + k * 32 < n) {
+            rd[j][k] = *reinterpret_cast<const uint4*>(dz[j] + (i0 + k * 32) * 8);
+            ry[j][k] = *reinterpret_cast<const uint4*>(y[j] + (i0 + k * 32) * 8);
+          }
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+        for (int k = 0; k < COLS; ++k) {
+          const int i = i0 + k * 32;
+          if (r0 + j * warps >= ps.rows || i >= n) continue;
+          uint4 out = make_uint4(0, 0, 0, 0);                  // rows outside the image
+          if (ok[j]) {
+            float d[8], yy[8];
+            unpack8(rd[j][k], d);
+            unpack8(ry[j][k], yy);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) d[q] = ca[q] * d[q] + cb[q] * yy[q] + cc[q];
+            out = pack8(d);
+          }
+          *reinterpret_cast<uint4*>(sD + ((r0 + j * warps) * s.pw + 1 + i / CH) * PX + i % CH * 16) = out;
+        }
+    }
+  }
+}
+
+template <int C>
+struct BwdPlan {
+  static constexpr int DGRAD = 8, WGRAD = C == 16 ? 8 : 6;     // warps
+  static constexpr int THREADS = (DGRAD + WGRAD) * 32;
+  using T = Tile<C, C, DGRAD>;
+  using P = Products<C, C, true>;
+  using G = Wgrad<C, C, WGRAD>;
+  static constexpr int FIXED = P::FILTER + DGRAD * T::STAGE + T::WM * 2 * C * 4 + 3 * C * 4;
+};
+
+template <int C>
+__global__ void __launch_bounds__(BwdPlan<C>::THREADS, 1) bwd_narrow_kernel(const Shape s, const Args a, const BnInput b, float* dw) {
+  using B = BwdPlan<C>;
+  using T = typename B::T;
+  using P = typename B::P;
+  using G = typename B::G;
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint8_t* sW = smem;
+  uint8_t* sC = sW + P::FILTER;
+  float* part = reinterpret_cast<float*>(sC + B::DGRAD * T::STAGE);
+  float* coef = part + T::WM * 2 * C;
+  uint8_t* sX = reinterpret_cast<uint8_t*>(coef + 3 * C);
+  uint8_t* sD = sX + s.slots * s.pw * P::PX;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  esgd::pdl_enter();
+  P::load_filters(a.w, sW);
+  if (threadIdx.x < C) {
+    const int c = threadIdx.x;
+    const float is = b.aux[C + c], gm = b.gamma[c], dgamma = b.dgamma[c], dbeta = b.dbeta[c], dg = dgamma * b.inv_count, db = dbeta * b.inv_count;
+    coef[c] = gm * is;
+    coef[C + c] = -gm * is * is * dg;
+    coef[2 * C + c] = gm * is * (b.aux[c] * is * dg - db);
+    if (blockIdx.x == 0) {                                     // the parameters' own gradient accumulators
+      b.acc_dgamma[c] += dgamma;
+      b.acc_dbeta[c] += dbeta;
+    }
+  }
+  __syncthreads();
+  const int end = first_row(s, blockIdx.x + 1);
+  const uint32_t row_bytes = (uint32_t)(s.pw * P::PX);
+  {
+    const Pass ps(s, first_row(s, blockIdx.x), end);
+    const int pixels = (ps.v1 - ps.v0) * s.Wo;
+    clear_margins<C>(s, sX);
+    clear_margins<C>(s, sD);
+    load_rows<C>(s, ps, a.x, sX);
+    load_dy_rows<C>(s, ps, b, coef, sD);
+    cp_async_wait();
+    __syncthreads();
+    if (warp < B::DGRAD) {
+      Output<C, C, true, B::DGRAD> out;
+      out.begin(a, sC, warp, 0);
+      P prod;
+      prod.begin(sW, 0, lane);
+      const int a_pix = (lane & 7) + ((lane >> 3) & 1) * 8, a_k = ((lane >> 4) & 1) * 16;
+      const int64_t pix0 = (int64_t)ps.v0 * s.Wo;
+      for (int m = warp * 16; m < pixels; m += T::WM * 16) {
+        out.prefetch(a, pix0 + m, pixels - m);
+        const uint32_t x0 = smem_addr(sD) + (uint32_t)(ps.window(s, min(m + a_pix, pixels - 1)) * P::PX + a_k);
+        float acc[T::NT][4];
+        prod.run(acc, x0, row_bytes);
+        out.finish(a, acc, pix0 + m, pixels - m);
+      }
+      out.collect(a, part, warp);
+      __syncthreads();
+    } else {
+      G g;
+      g.begin(warp - B::DGRAD);
+      for (int k = g.slice * 16; k < pixels; k += G::P::SLICES * 16) {
+        // past the end dy is the margin's zeros
+        const int pd = k + g.d_pix(), px = min(k + g.x_pix(), pixels - 1);
+        const uint32_t d0 = smem_addr(sD) + (uint32_t)((pd < pixels ? ps.window(s, pd) + s.pw + 1 : 0) * P::PX + g.d_col());
+        const uint32_t x0 = smem_addr(sX) + (uint32_t)(ps.window(s, px) * P::PX + g.x_col());
+        g.step(d0, x0, row_bytes);
+      }
+      __syncthreads();                                         // the banks lie where the rows were
+      g.collect(reinterpret_cast<float*>(sX));
+    }
+    __syncthreads();
+    G::commit(reinterpret_cast<float*>(sX), dw);
+    __syncthreads();
+  }
+  Output<C, C, true, B::DGRAD>::commit(a, part);
 }
 
 constexpr int kSmemMax = 220 * 1024;
@@ -550,18 +793,19 @@ void allow_smem(K kernel, Allowed& devices) {
   devices.fetch_or(bit, std::memory_order_relaxed);
 }
 
-template <int CR, int CN, bool kT>
-int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t stream) {
+template <int CR, int CN, bool kT, bool kBnIn = false>
+int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t stream, const BnOutput& b = BnOutput()) {
   using T = Tile<CR, CN>;
   using P = Products<CR, CN, kT>;
   Shape s;
   int grid, smem;
-  const int rc = plan(s, grid, smem, N, H, W, stride, P::FILTER + kWarps * T::STAGE + T::WM * 2 * CN * 4, (W + 2) * P::PX, 0);
+  const int rc = plan(s, grid, smem, N, H, W, stride, P::FILTER + kWarps * T::STAGE + T::WM * 2 * CN * 4 + (kBnIn ? 2 * CR * 4 : 0), (W + 2) * P::PX,
+                      0);
   if (rc != 0) return rc;
-  if (!aligned16(a.x, a.w) || !aligned16(a.y, a.residual) || !aligned16(a.bn_y, nullptr)) return -100;
+  if (!aligned16(a.x, a.w) || !aligned16(a.y, a.residual) || !aligned16(a.bn_y, b.y) || !aligned16(b.z, nullptr)) return -100;
   static Allowed allowed{0};
-  allow_smem(conv_narrow_kernel<CR, CN, kT>, allowed);
-  return esgd::launch(conv_narrow_kernel<CR, CN, kT>, dim3(grid), kThreads, smem, stream, s, a);
+  allow_smem(conv_narrow_kernel<CR, CN, kT, kBnIn>, allowed);
+  return esgd::launch(conv_narrow_kernel<CR, CN, kT, kBnIn>, dim3(grid), kThreads, smem, stream, s, a, b);
 }
 
 template <int CI, int CO>
@@ -579,6 +823,21 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
   allow_smem(wgrad_narrow_kernel<CI, CO>, allowed);
   return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), P::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
                       (const __nv_bfloat16*)dy, dw);
+}
+
+template <int C>
+int launch_bwd(const Args& a, const BnInput& b, float* dw, int N, int H, int W, cudaStream_t stream) {
+  using B = BwdPlan<C>;
+  Shape s;
+  int grid, smem;
+  const int rc = plan(s, grid, smem, N, H, W, 1, B::FIXED, 2 * (W + 2) * B::P::PX, 0);
+  if (rc != 0) return rc;
+  if (s.per_pass < (s.total + grid - 1) / grid) return -100;       // more rows a block than fit beside one another
+  if (!aligned16(a.x, a.w) || !aligned16(a.y, a.residual) || !aligned16(a.bn_y, dw) || !aligned16(b.dz, b.y)) return -100;
+  if (smem < B::FIXED + B::G::P::BYTES) smem = B::FIXED + B::G::P::BYTES;
+  static Allowed allowed{0};
+  allow_smem(bwd_narrow_kernel<C>, allowed);
+  return esgd::launch(bwd_narrow_kernel<C>, dim3(grid), B::THREADS, smem, stream, s, a, b, dw);
 }
 
 }  // namespace
@@ -620,6 +879,42 @@ int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H
   if (Cin == 16 && Cout == 16) return launch_conv<16, 16, true>(a, N, H, W, 1, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, true>(a, N, H, W, 1, s);
   if (Cin == 64 && Cout == 64 && (int64_t)N * H * W <= kMaxPixels64) return launch_conv<64, 64, true>(a, N, H, W, 1, s);
+  return -100;
+}
+
+// The whole backward pass of z = act(batch_norm(conv(x, w))) for 3x3, stride 1, C channels in and out: dz [N,H,W,C] with the ReLU's
+// mask applied, y the convolution's output; aux, gamma, dbeta, dgamma, acc_dgamma, acc_dbeta as in esgd_bn_bwd_apply; residual
+// and bn as in esgd_conv_narrow_dgrad; dw as in esgd_conv_narrow_wgrad.
+int esgd_conv_narrow_bwd(const void* x, const void* w, const void* dz, const void* y, const float* aux, const float* gamma, const float* dbeta,
+                         const float* dgamma, float* acc_dgamma, float* acc_dbeta, void* dx, float* dw, int N, int H, int W, int C,
+                         const void* residual, const esgd_bn_grad* bn, void* stream) {
+  Args a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, nullptr, nullptr, (const __nv_bfloat16*)residual, 0,
+         nullptr, nullptr, nullptr, nullptr, nullptr};
+  if (bn != nullptr) {
+    a.sum = bn->sums; a.sqsum = bn->sums + C;
+    a.bn_y = (const __nv_bfloat16*)bn->y; a.bn_mask = (const uint8_t*)bn->mask; a.bn_aux = bn->aux;
+  }
+  const BnInput b{(const __nv_bfloat16*)dz, (const __nv_bfloat16*)y, aux, gamma, dbeta, dgamma, acc_dgamma, acc_dbeta,
+                  1.0f / ((float)N * (float)H * (float)W)};
+  cudaStream_t s = (cudaStream_t)stream;
+  if (C == 16) return launch_bwd<16>(a, b, dw, N, H, W, s);
+  if (C == 32) return launch_bwd<32>(a, b, dw, N, H, W, s);
+  return -100;
+}
+
+// y = conv(z, w) with y's statistics, for z = act(batch_norm(by)), C channels in and out, stride 1: z, mask, aux and the running
+// statistics are written as esgd_bn_fwd writes them.
+int esgd_conv_narrow_bn_fwd(const void* by, void* z, void* mask, const float* bsum, const float* bsqsum, const float* gamma, const float* beta,
+                            float* running_mean, float* running_var, float* aux, int relu, float momentum, float eps, const void* w,
+                            void* y, int N, int H, int W, int C, float* sum, float* sqsum, void* stream) {
+  const int64_t m = (int64_t)N * H * W;
+  Args a{(const __nv_bfloat16*)z, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, nullptr, nullptr, nullptr, 0, sum, sqsum, nullptr, nullptr, nullptr};
+  const BnOutput b{(const __nv_bfloat16*)by, (__nv_bfloat16*)z, (uint8_t*)mask, bsum, bsqsum, gamma, beta, running_mean, running_var, aux,
+                   1.0f / (float)m, m > 1 ? (float)m / (float)(m - 1) : 1.0f, momentum, eps, relu};
+  cudaStream_t s = (cudaStream_t)stream;
+  if (C == 16) return launch_conv<16, 16, false, true>(a, N, H, W, 1, s, b);
+  if (C == 32) return launch_conv<32, 32, false, true>(a, N, H, W, 1, s, b);
+  if (C == 64 && m <= kMaxPixels64) return launch_conv<64, 64, false, true>(a, N, H, W, 1, s, b);
   return -100;
 }
 

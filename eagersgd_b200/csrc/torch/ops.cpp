@@ -11,6 +11,7 @@
 #include <torch/extension.h>
 #include "../cuda/bn_grad.h"
 #include <ATen/SavedTensorHooks.h>
+#include <torch/csrc/autograd/anomaly_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <atomic>
@@ -38,6 +39,12 @@ int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, in
                          const float* shift, const void* residual, int relu, float* sum, float* sqsum, void* stream);
 int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H, int W, int Cin, int Cout, const void* residual,
                            const esgd_bn_grad* bn, void* stream);
+int esgd_conv_narrow_bn_fwd(const void* by, void* z, void* mask, const float* bsum, const float* bsqsum, const float* gamma, const float* beta,
+                            float* running_mean, float* running_var, float* aux, int relu, float momentum, float eps, const void* w,
+                            void* y, int N, int H, int W, int C, float* sum, float* sqsum, void* stream);
+int esgd_conv_narrow_bwd(const void* x, const void* w, const void* dz, const void* y, const float* aux, const float* gamma, const float* dbeta,
+                         const float* dgamma, float* acc_dgamma, float* acc_dbeta, void* dx, float* dw, int N, int H, int W, int C,
+                         const void* residual, const esgd_bn_grad* bn, void* stream);
 int esgd_conv_narrow_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int stride, void* stream);
 int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, int R, int S, int stride, int pad, int seg,
                         int Kpad, void* stream);
@@ -451,6 +458,43 @@ struct BnRecord : torch::CustomClassHolder {
 using BnRef = c10::intrusive_ptr<BnRecord>;
 BnRef bn_behind(const Tensor& x);     // the record of the batch norm that produced x, or null
 
+// A convolution and the batch norm that is its output's only reader, inside a residual block: what the one's node leaves for the
+// other's, so that a narrow layer's backward pass is one launch.  The batch norm hands on its own gradient dz in the place of
+// dy, which the convolution's backward then makes from it on the way into shared memory; between the two nodes nobody looks.
+struct LayerLink : torch::CustomClassHolder {
+  std::weak_ptr<torch::autograd::Node> conv, norm;
+  bool pending = false;                  // the rest is there: dz stands for dy
+  Tensor dz, y, aux, gamma, sums;
+  Sink gs, bs;
+  uint32_t version = 0;
+
+  bool observed() const {
+    const auto c = conv.lock(), n = norm.lock();
+    if (!c || !n || !c->tensor_pre_hooks().empty() || !c->pre_hooks().empty() || !c->retains_grad_hooks().empty() ||
+        !n->post_hooks().empty() || torch::autograd::AnomalyMode::is_enabled()) return true;
+    const auto* captures = torch::autograd::get_current_graph_task_exec_info();
+    return captures != nullptr && !captures->empty();
+  }
+  void release() {
+    pending = false;
+    dz = y = aux = gamma = sums = Tensor();
+    gs = bs = Sink();
+  }
+};
+using Link = c10::intrusive_ptr<LayerLink>;
+
+// A batch norm (without a residual) whose launch is left to the convolution that reads its output.
+struct PendingNorm {
+  Tensor y, z, mask, stats, gamma, beta, mean, var, aux;
+  bool relu = false;
+  float momentum = 0.0f;
+  void launch(void* stream) const {
+    const int64_t c = y.size(1);
+    ck(esgd_bn_fwd(y.data_ptr(), nullptr, z.data_ptr(), mask.defined() ? mask.data_ptr() : nullptr, fptr(stats), fptr(stats) + c, fptr(gamma),
+                   fptr(beta), fptr(mean), fptr(var), fptr(aux), y.numel() / c, c, relu, momentum, kBnEps, stream), "bn_fwd");
+  }
+};
+
 // What a convolution's epilogue does to the product: statistics of it (training), or the affine map of an inference batch
 // norm, a residual and a ReLU.
 struct ConvEpilogue {
@@ -461,11 +505,25 @@ struct ConvEpilogue {
 };
 
 // Launches the convolution of NHWC x with w into y; `kept` and `filters` are what a backward pass needs of the two.
+// norm: x is its output and still to be computed.
 void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y, int64_t stride, int64_t pad, const ConvEpilogue& e,
-                 Tensor* kept, Tensor* filters) {
+                 Tensor* kept, Tensor* filters, const PendingNorm* norm = nullptr) {
   const int64_t n = x.size(0), cin = x.size(1), h = x.size(2), wd = x.size(3), cout = w.size(0), r = w.size(2), s = w.size(3);
   const int64_t ho = y.size(2), wo = y.size(3);
   void* st = stream_of(x);
+  if (norm != nullptr) {
+    if (kind == kGeneral && r == 3 && s == 3 && pad == 1 && stride == 1 && cin == cout && e.scale == nullptr && e.residual == nullptr && !e.relu) {
+      *filters = nhwc(w);
+      *kept = x;
+      const int rc = esgd_conv_narrow_bn_fwd(norm->y.data_ptr(), x.data_ptr(), norm->mask.defined() ? norm->mask.data_ptr() : nullptr,
+                                             fptr(norm->stats), fptr(norm->stats) + cin, fptr(norm->gamma), fptr(norm->beta), fptr(norm->mean),
+                                             fptr(norm->var), fptr(norm->aux), norm->relu, norm->momentum, kBnEps, filters->data_ptr(),
+                                             y.data_ptr(), n, h, wd, cin, e.sum, e.sqsum, st);
+      if (rc == 0) return;
+      if (rc != kNotTaken) ck(rc, "batch norm and conv2d");
+    }
+    norm->launch(st);
+  }
   if (kind == kOneByOne) {
     *filters = dense(w);                            // [Cout, Cin]: a 1x1 filter has one memory order
     *kept = x;
@@ -506,7 +564,8 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
 struct ConvFn : public Function<ConvFn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const c10::optional<Tensor>& w_in, int64_t kind,
                                int64_t stride, int64_t pad, bool want_stats, bool tap, const Sink& sink,
-                               const c10::optional<Tensor>& anchor, const BnRef& bn, const Held& w_held, const Held& into) {
+                               const c10::optional<Tensor>& anchor, const BnRef& bn, const Held& w_held, const Held& into, const Link& link,
+                               const PendingNorm* norm) {
     const Tensor& w = w_in.has_value() ? *w_in : w_held.t;
     c10::cuda::CUDAGuard guard(x_in.device());
     Tensor x = nhwc(x_in);
@@ -522,11 +581,12 @@ struct ConvFn : public Function<ConvFn> {
     }
     Tensor y = empty_nhwc(n, cout, ho, wo, x);
     Tensor saved_x, wk;
-    launch_conv(kind, x, w, y, stride, pad, e, &saved_x, &wk);
+    launch_conv(kind, x, w, y, stride, pad, e, &saved_x, &wk, norm);
     ctx->save_for_backward({saved_x, wk});
     ctx->saved_data["cfg"] = std::vector<int64_t>{kind, stride, pad, n, cin, h, wd, want_stats, tap};
     save_sink(ctx, "w", sink);
     if (bn) ctx->saved_data["bn"] = c10::IValue::make_capsule(bn);
+    if (link) ctx->saved_data["link"] = c10::IValue::make_capsule(link);
     ctx->set_materialize_grads(false);                // an unused tap must not cost a tensor of zeros
     variable_list out{y};
     if (want_stats) {
@@ -541,7 +601,7 @@ struct ConvFn : public Function<ConvFn> {
     const auto cfg = ctx->saved_data["cfg"].toIntVector();
     const int64_t kind = cfg[0], stride = cfg[1], pad = cfg[2], n = cfg[3], cin = cfg[4], h = cfg[5], wd = cfg[6];
     const bool want_stats = cfg[7], tap = cfg[8];
-    variable_list none(12);
+    variable_list none(14);
     Tensor d_tap = tap ? grads[want_stats ? 2 : 1] : Tensor();   // gradient that reached the input through the shortcut
     Sink sink = load_sink(ctx, "w");
     if (!grads[0].defined()) {
@@ -563,6 +623,40 @@ struct ConvFn : public Function<ConvFn> {
       if (!bn->y.defined() || bn->observed()) bn = BnRef();
     }
     esgd_bn_grad bg;
+    if (const auto it = ctx->saved_data.find("link"); it != ctx->saved_data.end()) {
+      const Link link = c10::static_intrusive_pointer_cast<LayerLink>(it->second.toCapsule());
+      if (link->pending) {
+        TORCH_CHECK(link->dz.is_same(grads[0]) && link->version == grads[0]._version(), "conv2d: somebody came between a layer and its batch norm");
+        const Tensor sums = link->sums, lz = link->dz, ly = link->y, laux = link->aux, lgamma = link->gamma;
+        const Sink gs = link->gs, bs = link->bs;
+        link->release();
+        int rc = kNotTaken;
+        if (need_dx && sink) {
+          Tensor res;
+          if (d_tap.defined()) res = nhwc(d_tap.to(at::kBFloat16));
+          dx = empty_nhwc(n, cin, h, wd, x);
+          if (bn) bn->fill(&bg, dx);
+          rc = esgd_conv_narrow_bwd(x.data_ptr(), w.data_ptr(), lz.data_ptr(), ly.data_ptr(), fptr(laux), fptr(lgamma), fptr(sums),
+                                    fptr(sums) + cout, gs->acc, bs->acc, dx.data_ptr(), sink->acc, n, h, wd, cin,
+                                    res.defined() ? res.data_ptr() : nullptr, bn ? &bg : nullptr, st);
+          if (rc == 0 && bn) bn->written(dx);
+        }
+        if (rc == kNotTaken) {             // then as the batch norm would have done it
+          dy = empty_nhwc(n, cout, ho, wo, x);
+          ck(esgd_bn_bwd_apply(lz.data_ptr(), nullptr, ly.data_ptr(), fptr(laux), fptr(lgamma), fptr(sums), fptr(sums) + cout, dy.data_ptr(),
+                               nullptr, m, cout, 0, 1, gs->acc, bs->acc, st), "bn_bwd_apply");
+        } else {
+          ck(rc, "backward pass of a layer");
+        }
+        sink_done(gs);
+        sink_done(bs);
+        if (rc == 0) {
+          sink_done(sink);
+          none[0] = dx;
+          return none;
+        }
+      }
+    }
     // The weight gradient goes first: what the data gradient leaves (and the batch norm's pass behind it reads) is then the
     // newest in L2.
     if (need_dw) {
@@ -683,7 +777,7 @@ struct ConvOut {
   Tensor y, stats, tapped;       // stats, tapped: on request
 };
 ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t stride, int64_t pad, bool want_stats, bool tap,
-                   const Tensor& into = Tensor()) {
+                   const Tensor& into = Tensor(), const Link& link = Link(), const PendingNorm* norm = nullptr) {
   check_conv(x, w, stride, pad, kind == kStem);
   const int64_t r = w.size(2), s = w.size(3);
   // the stride-1 data gradients add the shortcut's gradient in their epilogue: elsewhere the tap is the input itself
@@ -691,7 +785,8 @@ ConvOut conv_train(int64_t kind, const Tensor& x, const Tensor& w, int64_t strid
   Sink sink = find_sink(w);
   sink_use(sink);
   variable_list out = ConvFn::apply(x, graph_only(w, sink), kind, stride, pad, want_stats, fuse_tap, sink, anchor_for(x, (bool)sink),
-                                    sink && stride == 1 ? bn_behind(x) : BnRef(), Held{w}, Held{into});
+                                    sink && stride == 1 ? bn_behind(x) : BnRef(), Held{w}, Held{into}, link, norm);
+  if (link) link->conv = out[0].grad_fn();
   return {out[0], want_stats ? out[1] : Tensor(), !tap ? Tensor() : (fuse_tap ? out.back() : x)};
 }
 
@@ -994,7 +1089,7 @@ struct BnActFn : public Function<BnActFn> {
   using Opt = c10::optional<Tensor>;
   static Tensor forward(AutogradContext* ctx, const Tensor& y_in, const Opt& gamma_in, const Opt& beta_in, const Opt& res_in,
                         const Held& rm_in, const Held& rv_in, double momentum, bool relu, const Held& stats_in, const Sink& gs,
-                        const Sink& bs, const Opt& anchor, const Held& gamma_held, const Held& beta_held) {
+                        const Sink& bs, const Opt& anchor, const Held& gamma_held, const Held& beta_held, const Link& link, PendingNorm* later) {
     const Tensor &gamma = gamma_in.has_value() ? *gamma_in : gamma_held.t, &beta = beta_in.has_value() ? *beta_in : beta_held.t;
     c10::cuda::CUDAGuard guard(y_in.device());
     Tensor y = nhwc(y_in), res = res_in.has_value() ? nhwc(*res_in) : Tensor(), stats = stats_in.t, rm = rm_in.t, rv = rv_in.t;
@@ -1011,9 +1106,13 @@ struct BnActFn : public Function<BnActFn> {
     const int64_t mode = !relu ? 0 : (res.defined() || (gs && bs) ? 1 : 2);
     Tensor mask;
     if (mode == 1) mask = at::empty({m, c / 8}, y.options().dtype(at::kByte));
-    ck(esgd_bn_fwd(y.data_ptr(), res.defined() ? res.data_ptr() : nullptr, z.data_ptr(), mode == 1 ? mask.data_ptr() : nullptr,
-                   fptr(stats), fptr(stats) + c, fptr(gamma), fptr(beta), fptr(rm), fptr(rv), fptr(aux), m, c, relu, (float)momentum,
-                   kBnEps, st), "bn_fwd");
+    if (later != nullptr) {
+      *later = PendingNorm{y, z, mask, stats, gamma, beta, rm, rv, aux, relu, (float)momentum};
+    } else {
+      ck(esgd_bn_fwd(y.data_ptr(), res.defined() ? res.data_ptr() : nullptr, z.data_ptr(), mode == 1 ? mask.data_ptr() : nullptr,
+                     fptr(stats), fptr(stats) + c, fptr(gamma), fptr(beta), fptr(rm), fptr(rv), fptr(aux), m, c, relu, (float)momentum,
+                     kBnEps, st), "bn_fwd");
+    }
     ctx->save_for_backward({y, mask, gamma, aux});
     ctx->saved_data["mode"] = mode;
     ctx->saved_data["res"] = res.defined();
@@ -1026,6 +1125,7 @@ struct BnActFn : public Function<BnActFn> {
       rec->mask = mask;
       rec->aux = aux;
       ctx->saved_data["rec"] = c10::IValue::make_capsule(rec);
+      if (link) ctx->saved_data["link"] = c10::IValue::make_capsule(link);
     }
     return z;
   }
@@ -1057,6 +1157,24 @@ struct BnActFn : public Function<BnActFn> {
     if (rec) {
       rec->y = rec->mask = rec->dz = rec->sums = Tensor();
     }
+    variable_list out(16);
+    if (const auto it = ctx->saved_data.find("link"); fused && it != ctx->saved_data.end()) {
+      const Link link = c10::static_intrusive_pointer_cast<LayerLink>(it->second.toCapsule());
+      if (!link->observed()) {             // the convolution's backward, which comes next, does it on the way
+        link->dz = dz;
+        link->version = dz._version();
+        link->y = y;
+        link->aux = aux;
+        link->gamma = gamma;
+        link->sums = red;
+        link->gs = gs;
+        link->bs = bs;
+        link->pending = true;
+        out[0] = dz;
+        out[3] = dres;
+        return out;
+      }
+    }
     float* rd = fptr(red);
     Tensor dy = empty_nhwc(y.size(0), c, y.size(2), y.size(3), y);
     const bool write_res = has_res && !dres.defined();
@@ -1069,15 +1187,14 @@ struct BnActFn : public Function<BnActFn> {
     else dgamma = red.select(0, 1);
     if (bs) sink_done(bs);
     else dbeta = red.select(0, 0);
-    variable_list out(14);
     out[0] = dy; out[1] = dgamma; out[2] = dbeta; out[3] = dres;
     return out;
   }
 };
 
-Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& res,
+Tensor bn_train(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& res,
               const c10::optional<Tensor>& rm, const c10::optional<Tensor>& rv, double momentum, bool relu,
-              const c10::optional<Tensor>& stats) {
+              const c10::optional<Tensor>& stats, const Link& link, PendingNorm* later) {
   TORCH_CHECK(y.dim() == 4, "bn_act: takes a 4-D input, not ", y.sizes());
   const int64_t c = y.size(1);
   check_operand("bn_act", "the input", y, y, at::kBFloat16);
@@ -1095,13 +1212,19 @@ Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c1
   sink_use(bs);
   auto held = [](const c10::optional<Tensor>& o) { return Held{o.has_value() ? *o : Tensor()}; };
   Tensor z = BnActFn::apply(y, graph_only(gamma, gs), graph_only(beta, bs), res, held(rm), held(rv), momentum, relu, held(stats), gs,
-                            bs, anchor_for(y, gs || bs), Held{gamma}, Held{beta});
+                            bs, anchor_for(y, gs || bs), Held{gamma}, Held{beta}, link, later);
   if (gs && bs) {
     auto* node = static_cast<torch::autograd::CppNode<BnActFn>*>(z.grad_fn().get());
     const auto it = node->ctx_.saved_data.find("rec");
     if (it != node->ctx_.saved_data.end()) c10::static_intrusive_pointer_cast<BnRecord>(it->second.toCapsule())->node = z.grad_fn();
+    if (link) link->norm = z.grad_fn();
   }
   return z;
+}
+Tensor bn_act(const Tensor& y, const Tensor& gamma, const Tensor& beta, const c10::optional<Tensor>& res,
+              const c10::optional<Tensor>& rm, const c10::optional<Tensor>& rv, double momentum, bool relu,
+              const c10::optional<Tensor>& stats) {
+  return bn_train(y, gamma, beta, res, rm, rv, momentum, relu, stats, Link(), nullptr);
 }
 
 // A residual block in training (convolution, batch norm and ReLU in a row, the last batch norm adding the shortcut): what the
@@ -1121,12 +1244,16 @@ struct BlockLayer {
     if (w.scalar_type() != at::kBFloat16 || gamma.scalar_type() != at::kFloat || w.size(0) % 8) kind = -1;
   }
   Tensor stats;                  // of the convolution's output, for the batch norm behind it
-  ConvOut conv(const Tensor& x, bool tap) {
+  Link link;                     // ... where one launch may do the backward pass of both
+  bool rows() const { return kind == kGeneral && w.size(2) == 3 && w.size(3) == 3 && stride == 1 && pad == 1 && w.size(0) == w.size(1); }
+  // later: the batch norm that x is still to come from
+  ConvOut conv(const Tensor& x, bool tap, const PendingNorm* later = nullptr) {
     stats = zeros_f32({2, w.size(0)}, x.device());
-    return conv_train(kind, x, w, stride, pad, false, tap, stats);
+    if (rows() && (w.size(0) == 16 || w.size(0) == 32) && at::GradMode::is_enabled()) link = c10::make_intrusive<LayerLink>();
+    return conv_train(kind, x, w, stride, pad, false, tap, stats, link, later);
   }
-  Tensor norm(const ConvOut& o, bool relu, const c10::optional<Tensor>& res) const {
-    return bn_act(o.y, gamma, beta, res, mean, var, momentum, relu, stats);
+  Tensor norm(const ConvOut& o, bool relu, const c10::optional<Tensor>& res, PendingNorm* later = nullptr) const {
+    return bn_train(o.y, gamma, beta, res, mean, var, momentum, relu, stats, link, later);
   }
 };
 py::object residual_block(const Tensor& x, const std::vector<py::tuple>& layers, const c10::optional<py::tuple>& proj, bool narrow) {
@@ -1146,9 +1273,15 @@ py::object residual_block(const Tensor& x, const std::vector<py::tuple>& layers,
     if (proj.has_value()) {
       shortcut = ls[n].norm(ls[n].conv(c.tapped, false), false, c10::nullopt);
     }
+    // A batch norm between two convolutions is left to the second where the kernels for rows in shared memory may take it (up to 64
+    // channels); not when somebody packs what is saved for the backward pass, which would then not be there yet.
+    const bool may_wait = !at::SavedTensorDefaultHooks::get_hooks().has_value();
+    PendingNorm later;
+    bool waiting = false;
     for (size_t i = 0; i < n; ++i) {
-      if (i > 0) c = ls[i].conv(out, false);
-      out = ls[i].norm(c, true, i + 1 == n ? shortcut : c10::nullopt);
+      if (i > 0) c = ls[i].conv(out, false, waiting ? &later : nullptr);
+      waiting = may_wait && i + 1 < n && ls[i + 1].rows() && ls[i + 1].w.size(0) <= 64;
+      out = ls[i].norm(c, true, i + 1 == n ? shortcut : c10::nullopt, waiting ? &later : nullptr);
     }
   }
   return py::cast(out);
