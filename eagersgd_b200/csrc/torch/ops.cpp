@@ -48,6 +48,10 @@ int esgd_conv_narrow_bwd(const void* x, const void* w, const void* dz, const voi
 int esgd_conv_narrow_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int stride, void* stream);
 int esgd_im2col_small_c(const void* x, void* col, int N, int H, int W, int C, int R, int S, int stride, int pad, int seg,
                         int Kpad, void* stream);
+int esgd_stem_fwd(const void* x, const void* w2d, void* y, void* keep, int N, int H, int W, int C, int Cout, int R, int S, int stride, int pad,
+                  int kpad, const float* scale, const float* shift, int relu, float* sum, float* sqsum, int* error_flag, void* stream);
+int esgd_stem_wgrad(const void* x, const void* dy, float* col, int N, int H, int W, int C, int Cout, int R, int S, int stride, int pad, int kpad,
+                    int* error_flag, void* stream);
 int esgd_stem_pack(const void* w, void* out, int Cout, int R, int sc, int seg, int Kpad, void* stream);
 int esgd_stem_unpack(const float* col, void* dw, float* acc, int Cout, int R, int sc, int seg, int Kpad, void* stream);
 int esgd_subsample2_fwd(const void* x, void* y, int N, int H, int W, int C, void* stream);
@@ -497,11 +501,21 @@ struct PendingNorm {
 
 // What a convolution's epilogue does to the product: statistics of it (training), or the affine map of an inference batch
 // norm, a residual and a ReLU.
+// The windows of NHWC x as a matrix, one row per output pixel.
+Tensor stem_columns(const Tensor& x, int64_t r, int64_t s, int64_t stride, int64_t pad) {
+  const int64_t n = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3);
+  const StemGeometry g(c, r, s);
+  Tensor col = at::empty({n * ((h + 2 * pad - r) / stride + 1) * ((w + 2 * pad - s) / stride + 1), g.kpad}, x.options());
+  ck(esgd_im2col_small_c(x.data_ptr(), col.data_ptr(), n, h, w, c, r, s, stride, pad, g.seg, g.kpad, stream_of(x)), "im2col");
+  return col;
+}
+
 struct ConvEpilogue {
   float *sum = nullptr, *sqsum = nullptr;
   const float *scale = nullptr, *shift = nullptr;
   const void* residual = nullptr;
   bool relu = false;
+  bool train = false;            // a backward pass may follow
 };
 
 // Launches the convolution of NHWC x with w into y; `kept` and `filters` are what a backward pass needs of the two.
@@ -547,10 +561,20 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
   } else {
     *filters = nhwc(w.to(at::kBFloat16));           // packed anyway: any floating type
     const StemGeometry g(cin, r, s);
-    *kept = at::empty({n * ho * wo, g.kpad}, x.options());
-    ck(esgd_im2col_small_c(x.data_ptr(), kept->data_ptr(), n, h, wd, cin, r, s, stride, pad, g.seg, g.kpad, st), "im2col");
     Tensor w2d = at::empty({cout, g.kpad}, x.options());
     ck(esgd_stem_pack(filters->data_ptr(), w2d.data_ptr(), cout, r, s * cin, g.seg, g.kpad, st), "stem filters");
+    if (e.residual == nullptr) {
+      // the backward pass has a copy of the images: the caller may refill their buffer before it
+      Tensor images = e.train ? empty_nhwc(n, cin, h, wd, x) : Tensor();
+      const int rc = esgd_stem_fwd(x.data_ptr(), w2d.data_ptr(), y.data_ptr(), e.train ? images.data_ptr() : nullptr, n, h, wd, cin, cout, r, s,
+                                   stride, pad, g.kpad, e.scale, e.shift, e.relu, e.sum, e.sqsum, flag_ptr(x), st);
+      if (rc != kNotTaken) {
+        ck(rc, "stem convolution");
+        *kept = images;
+        return;
+      }
+    }
+    *kept = stem_columns(x, r, s, stride, pad);
     ck(gemm(kept->data_ptr(), w2d.data_ptr(), y.data_ptr(), n * ho * wo, cout, g.kpad, g.kpad, g.kpad, cout, false, false, 0, 1, e.sum,
             e.sqsum, e.residual, cout, x, e.shift, e.relu, e.scale), "stem convolution");
   }
@@ -574,6 +598,7 @@ struct ConvFn : public Function<ConvFn> {
     const int64_t ho = (h + 2 * pad - r) / stride + 1, wo = (wd + 2 * pad - s) / stride + 1;
     Tensor stats = into.t;                            // given: not an output of the graph's
     ConvEpilogue e;
+    e.train = true;
     if (want_stats) stats = zeros_f32({2, cout}, x.device());
     if (stats.defined()) {
       e.sum = fptr(stats);
@@ -685,8 +710,15 @@ struct ConvFn : public Function<ConvFn> {
       } else {
         const StemGeometry g(cin, r, s);
         Tensor col = zeros_f32({cout, g.kpad}, x.device());
-        ck(gemm(dy.data_ptr(), x.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, esgd_sm_count(), nullptr, nullptr,
-                nullptr, 0, x), "stem weight gradient");
+        int rc = kNotTaken;
+        if (x.dim() == 4)                       // the forward pass left the images, not their columns
+          rc = esgd_stem_wgrad(x.data_ptr(), dy.data_ptr(), fptr(col), n, h, wd, cin, cout, r, s, stride, pad, g.kpad, flag_ptr(x), st);
+        if (rc == kNotTaken) {
+          const Tensor rows = x.dim() == 4 ? stem_columns(x, r, s, stride, pad) : x;
+          rc = gemm(dy.data_ptr(), rows.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, esgd_sm_count(), nullptr,
+                    nullptr, nullptr, 0, x);
+        }
+        ck(rc, "stem weight gradient");
         if (!sink) dw = at::empty(w.sizes(), w.options(), kCL);
         ck(esgd_stem_unpack(fptr(col), sink ? nullptr : dw.data_ptr(), sink ? sink->acc : nullptr, cout, r, s * cin, g.seg, g.kpad,
                             st), "stem filter gradient");
