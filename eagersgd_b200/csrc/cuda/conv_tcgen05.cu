@@ -37,6 +37,16 @@ namespace {
 // Channel counts that are no multiple of 64 are zero-filled by TMA on both operands.
 struct FilterTaps { int r0, dr, s0, ds; };
 
+// A k-block: 64 channels of one tap, taps before channels.
+struct TapStep { int r, s, cb; };
+__device__ __forceinline__ void next_tap(TapStep& k, int cblks, int S) {
+  if (++k.cb < cblks) return;
+  k.cb = 0;
+  if (++k.s < S) return;
+  k.s = 0;
+  ++k.r;
+}
+
 template <int BN, bool kTransposed>
 __device__ __forceinline__ void load_filter_tap(const CUtensorMap* tm, const FilterTaps& f, int r, int s, int cb, int n0,
                                                 uint8_t* b, uint64_t* bar) {
@@ -90,31 +100,28 @@ struct ConvProblem {
     t.kb1 = R * S * cblks;
     return true;
   }
-  __device__ __forceinline__ void load_a(const Tile& t, int kb, uint8_t* a, uint64_t* bar) const {
-    const int tap = kb / cblks, cb = kb - tap * cblks;
-    const int r = tap / S, s = tap - r * S;
-    tma_load_4d(a, &tmX, bar, cb * 64, t.w0 * stride + s - pad, t.h0 * stride + r - pad, t.i0);
+  using Step = TapStep;
+  __device__ __forceinline__ Step begin(const Tile&) const { return Step{0, 0, 0}; }
+  __device__ __forceinline__ void advance(Step& k) const { next_tap(k, cblks, S); }
+  __device__ __forceinline__ void load_a(const Tile& t, const Step& k, uint8_t* a, uint64_t* bar) const {
+    tma_load_4d(a, &tmX, bar, k.cb * 64, t.w0 * stride + k.s - pad, t.h0 * stride + k.r - pad, t.i0);
   }
-  __device__ __forceinline__ void load_b(const Tile& t, int kb, uint8_t* b, uint64_t* bar) const {
-    const int tap = kb / cblks, cb = kb - tap * cblks;
-    const int r = tap / S, s = tap - r * S;
-    load_filter_tap<BN, kT>(&tmW, taps, r, s, cb, t.n0, b, bar);
+  __device__ __forceinline__ void load_b(const Tile& t, const Step& k, uint8_t* b, uint64_t* bar) const {
+    load_filter_tap<BN, kT>(&tmW, taps, k.r, k.s, k.cb, t.n0, b, bar);
   }
-  __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint64_t* bar) const {
-    load_a(t, kb, a, bar);
-    load_b(t, kb, b, bar);
+  __device__ __forceinline__ void load(const Tile& t, const Step& k, uint8_t* a, uint8_t* b, uint64_t* bar) const {
+    load_a(t, k, a, bar);
+    load_b(t, k, b, bar);
   }
   // pair: this CTA's box and its half of the output channels' filters
-  __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint32_t leader_bar) const {
-    const int tap = kb / cblks, cb = kb - tap * cblks;
-    const int r = tap / S, s = tap - r * S;
-    const int rw = taps.r0 + r * taps.dr, sw = taps.s0 + s * taps.ds, n0 = t.n0 + (int)(blockIdx.x & 1) * (BN / 2);
-    tma_load_4d_pair(a, &tmX, leader_bar, cb * 64, t.w0 * stride + s - pad, t.h0 * stride + r - pad, t.i0);
+  __device__ __forceinline__ void load(const Tile& t, const Step& k, uint8_t* a, uint8_t* b, uint32_t leader_bar) const {
+    const int rw = taps.r0 + k.r * taps.dr, sw = taps.s0 + k.s * taps.ds, n0 = t.n0 + (int)(blockIdx.x & 1) * (BN / 2);
+    tma_load_4d_pair(a, &tmX, leader_bar, k.cb * 64, t.w0 * stride + k.s - pad, t.h0 * stride + k.r - pad, t.i0);
     if (kT) {
 #pragma unroll
-      for (int i = 0; i < BN / 128; ++i) tma_load_4d_pair(b + i * 8192, &tmW, leader_bar, n0 + 64 * i, sw, rw, cb * 64);
+      for (int i = 0; i < BN / 128; ++i) tma_load_4d_pair(b + i * 8192, &tmW, leader_bar, n0 + 64 * i, sw, rw, k.cb * 64);
     } else {
-      tma_load_4d_pair(b, &tmW, leader_bar, cb * 64, sw, rw, n0);
+      tma_load_4d_pair(b, &tmW, leader_bar, k.cb * 64, sw, rw, n0);
     }
   }
   __device__ __forceinline__ void store_panel(const Tile& t, int panel, const void* smem) const {
@@ -137,10 +144,11 @@ struct ConvProblem {
 // pipeline).  A tile is BH full output rows of one image; GEMM row m stands for the pixel (m / PW, m % PW) of
 // the box pitch PW = Wo + S - 1, so the S - 1 margin columns of every row (and the rows past BH * PW) compute
 // values that are dropped: out_row() gives a GEMM row its place in the dense [BH][Wo] tile that is stored.
-template <int BN_, bool kT>
+template <int BN_, bool kT, bool kPair_>
 struct ConvHaloProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kTwoPanels = false, kPair = false;
+  static_assert(!kPair_ || BN_ == 128, "a CTA's half of a pair's filters is one block of 64 channels");
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kTwoPanels = false, kPair = kPair_;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, pad;
@@ -154,9 +162,12 @@ struct ConvHaloProblem {
   struct Tile { int kb0, kb1, n0, h0, i0; };
 
   __device__ __forceinline__ bool tile(int it, Tile& t) const {
-    const int n_idx = blockIdx.x % n_tiles;
-    const int m_idx = blockIdx.x / n_tiles + it * (gridDim.x / n_tiles);
-    if (m_idx >= h_tiles * N) return false;
+    // a pair takes two boxes at a time (the last one may be past the last image: loaded as zeros, not stored)
+    const int boxes = h_tiles * N, worker = kPair ? blockIdx.x / 2 : blockIdx.x, workers = kPair ? gridDim.x / 2 : gridDim.x;
+    const int n_idx = worker % n_tiles;
+    int m_idx = worker / n_tiles + it * (workers / n_tiles);
+    if (m_idx >= (kPair ? (boxes + 1) / 2 : boxes)) return false;
+    if (kPair) m_idx = 2 * m_idx + (int)(blockIdx.x & 1);
     t.h0 = (m_idx % h_tiles) * BH;
     t.i0 = m_idx / h_tiles;
     t.n0 = n_idx * BN;
@@ -165,23 +176,31 @@ struct ConvHaloProblem {
     return true;
   }
   __device__ __forceinline__ void load_halo(const Tile& t, int cb, void* smem, uint64_t* bar) const {
-    tma_load_4d(smem, &tmX, bar, cb * 64, -pad, t.h0 - pad, t.i0);
+    if (kPair) tma_load_4d_pair(smem, &tmX, leader_addr(bar), cb * 64, -pad, t.h0 - pad, t.i0);
+    else tma_load_4d(smem, &tmX, bar, cb * 64, -pad, t.h0 - pad, t.i0);
   }
-  __device__ __forceinline__ void load_b(const Tile& t, int kb, uint8_t* b, uint64_t* bar) const {
-    const int tap = kb / cblks, cb = kb - tap * cblks;
-    const int r = tap / S, s = tap - r * S;
-    load_filter_tap<BN, kT>(&tmW, taps, r, s, cb, t.n0, b, bar);
+  using Step = TapStep;
+  __device__ __forceinline__ Step begin(const Tile&) const { return Step{0, 0, 0}; }
+  __device__ __forceinline__ void advance(Step& k) const { next_tap(k, cblks, S); }
+  __device__ __forceinline__ void load_b(const Tile& t, const Step& k, uint8_t* b, uint64_t* bar) const {
+    if (kPair) {               // this CTA's half of the output channels' filters
+      const int rw = taps.r0 + k.r * taps.dr, sw = taps.s0 + k.s * taps.ds, n0 = t.n0 + (int)(blockIdx.x & 1) * (BN / 2);
+      if (kT) tma_load_4d_pair(b, &tmW, leader_addr(bar), n0, sw, rw, k.cb * 64);
+      else tma_load_4d_pair(b, &tmW, leader_addr(bar), k.cb * 64, sw, rw, n0);
+    } else {
+      load_filter_tap<BN, kT>(&tmW, taps, k.r, k.s, k.cb, t.n0, b, bar);
+    }
   }
-  __device__ __forceinline__ void load_a(const Tile&, int, uint8_t*, uint64_t*) const {}
-  __device__ __forceinline__ void load(const Tile&, int, uint8_t*, uint8_t*, uint64_t*) const {}
+  __device__ __forceinline__ void load_a(const Tile&, const Step&, uint8_t*, uint64_t*) const {}
+  __device__ __forceinline__ void load(const Tile&, const Step&, uint8_t*, uint8_t*, uint64_t*) const {}
   __device__ __forceinline__ void store_panel(const Tile& t, int panel, const void* smem) const {
-    tma_store_4d(&tmY, smem, t.n0 + panel * 64, 0, t.h0, t.i0);
+    if (!kPair || t.i0 < N) tma_store_4d(&tmY, smem, t.n0 + panel * 64, 0, t.h0, t.i0);
   }
   __device__ __forceinline__ int out_row(int row) const {
     const int hl = row / PW, wl = row - hl * PW;
     return (hl < BH && wl < Wo) ? hl * Wo + wl : -1;
   }
-  __device__ __forceinline__ int valid_prefix(const Tile&) const { return BH * Wo; }
+  __device__ __forceinline__ int valid_prefix(const Tile& t) const { return kPair && t.i0 >= N ? 0 : BH * Wo; }
   __device__ __forceinline__ int64_t first_row(const Tile& t) const { return ((int64_t)t.i0 * Ho + t.h0) * Wo; }
   __device__ __forceinline__ void store_f32(const Tile&, int, const void*, bool) const {}
   __device__ __forceinline__ void load_res_panel(const Tile& t, int panel, void* smem, uint64_t* bar) const {
@@ -225,17 +244,28 @@ struct ConvWgradProblem {
     t.kb1 = min(t.kb0 + boxes_per_split, boxes_total);
     return true;
   }
-  __device__ __forceinline__ void load(const Tile& t, int kb, uint8_t* a, uint8_t* b, uint64_t* bar) const {
-    const int w0 = (kb % w_tiles) * BW, h0 = ((kb / w_tiles) % h_tiles) * BH, i0 = (kb / (w_tiles * h_tiles)) * BI;
-    const int r = t.tap / S, s = t.tap - r * S;
+  struct Step { int r, s, w0, h0, i0; };     // the tile's tap; a box of pixels
+  __device__ __forceinline__ Step begin(const Tile& t) const {
+    const int r = t.tap / S;
+    return Step{r, t.tap - r * S, (t.kb0 % w_tiles) * BW, ((t.kb0 / w_tiles) % h_tiles) * BH, (t.kb0 / (w_tiles * h_tiles)) * BI};
+  }
+  __device__ __forceinline__ void advance(Step& k) const {
+    if ((k.w0 += BW) < w_tiles * BW) return;
+    k.w0 = 0;
+    if ((k.h0 += BH) < h_tiles * BH) return;
+    k.h0 = 0;
+    k.i0 += BI;
+  }
+  __device__ __forceinline__ void load(const Tile& t, const Step& k, uint8_t* a, uint8_t* b, uint64_t* bar) const {
+    const int r = k.r, s = k.s, w0 = k.w0, h0 = k.h0, i0 = k.i0;
 #pragma unroll
     for (int i = 0; i < BM / 64; ++i) tma_load_4d(a + i * 8192, &tmDY, bar, t.m0 + 64 * i, w0, h0, i0);
 #pragma unroll
     for (int i = 0; i < BN / 64; ++i)
       tma_load_4d(b + i * 8192, &tmX, bar, t.n0 + 64 * i, w0 * stride + s - pad, h0 * stride + r - pad, i0);
   }
-  __device__ __forceinline__ void load_a(const Tile&, int, uint8_t*, uint64_t*) const {}
-  __device__ __forceinline__ void load_b(const Tile&, int, uint8_t*, uint64_t*) const {}
+  __device__ __forceinline__ void load_a(const Tile&, const Step&, uint8_t*, uint64_t*) const {}
+  __device__ __forceinline__ void load_b(const Tile&, const Step&, uint8_t*, uint64_t*) const {}
   __device__ __forceinline__ void store_panel(const Tile&, int, const void*) const {}
   __device__ __forceinline__ int valid_prefix(const Tile& t) const { return min(BM, Cout - t.m0); }
   __device__ __forceinline__ int64_t first_row(const Tile& t) const { return t.m0; }
@@ -384,9 +414,12 @@ bool halo_applicable(const ConvArgs& a, int Ho, int Wo, int* bh_out) {
   return true;
 }
 
-template <int BN, bool kT, bool kBn>
+// @PAIRS
+bool halo_pairs(const ConvArgs& a, int BN) { return BN == 128 && a.Cin % 64 == 0 && a.Cout == 128; }
+
+template <int BN, bool kT, bool kBn, bool kPair = false>
 int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
-  using P = ConvHaloProblem<BN, kT>;
+  using P = ConvHaloProblem<BN, kT, kPair>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(conv_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -414,7 +447,7 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
     if (r != 0) return 1000 + r;
   }
   {
-    int r = filter_map<BN, kT>(&p.tmW, a);
+    int r = filter_map<BN, kT, kPair>(&p.tmW, a);
     if (r != 0) return 2000 + r;
   }
   {
@@ -426,17 +459,17 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
     if (r != 0) return 3000 + r;
     ep.res_bytes = (uint32_t)(p.Wo * bh * 128);
   }
-  const int sms = sm_count();
+  const int sms = kPair ? sm_count() / 2 : sm_count();           // workers: CTAs, or pairs of them
   if (p.n_tiles > sms) return -3;
   const int kb_total = a.R * a.S * p.cblks;
   // resident filter bank: beside two input boxes
-  p.res_kb = (kb_total * Cfg<BN>::B_STAGE_BYTES + 2 * HALO_BYTES <= Cfg<BN>::STAGE_AREA) ? kb_total : 0;
-  const int total = p.h_tiles * a.N * p.n_tiles;
+  p.res_kb = (!kPair && kb_total * Cfg<BN>::B_STAGE_BYTES + 2 * HALO_BYTES <= Cfg<BN>::STAGE_AREA) ? kb_total : 0;
+  const int boxes = p.h_tiles * a.N, total = (kPair ? (boxes + 1) / 2 : boxes) * p.n_tiles;
   int grid = (sms / p.n_tiles) * p.n_tiles;
   if (grid > total) grid = total;
   ep.tx_bytes_a = (uint32_t)(p.PW * (bh + a.R - 1) * 128);
   ep.tx_bytes = 0;
-  return esgd::launch(conv_kernel<P, kBn>, dim3(grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
+  return esgd::launch<kPair ? 2 : 1>(conv_kernel<P, kBn>, dim3(kPair ? 2 * grid : grid), NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream, p, ep);
 }
 
 template <int BN>
@@ -514,7 +547,7 @@ Epilogue epilogue_for(int n, int relu, float* col_sum, float* col_sqsum, int* er
   Epilogue ep;
   ep.out_mode = OUT_BF16; ep.relu = relu; ep.n_total = n; ep.scale = nullptr; ep.bias = nullptr; ep.bias_kind = BIAS_F32; ep.res_bytes = 0;
   ep.col_sum = col_sum; ep.col_sqsum = col_sqsum; ep.error_flag = error_flag;
-  ep.tx_bytes = 0; ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = 0;
+  ep.tx_bytes = 0; ep.tx_bytes_a = 0; ep.residual = nullptr; ep.ldr = n;
   return ep;
 }
 
@@ -529,7 +562,9 @@ int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
   const int BN = tile_width(a, Ho, Wo);
   int bh = 0;
   if (a.Cout <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
-    return BN == 64 ? launch_halo<64, kT, kBn>(a, ep, bh, s) : launch_halo<128, kT, kBn>(a, ep, bh, s);
+    return BN == 64                   ? launch_halo<64, kT, kBn>(a, ep, bh, s)
+           : halo_pairs(a, BN)        ? launch_halo<128, kT, kBn, true>(a, ep, bh, s)
+                                      : launch_halo<128, kT, kBn>(a, ep, bh, s);
   if (BN == 64) return launch<64, kT, kBn>(a, ep, s);
   if (BN == 128) return launch<128, kT, kBn>(a, ep, s);
   // Pairs of CTAs (256-column tiles read each operand once for two boxes of pixels) where the reduction is full blocks:
@@ -617,9 +652,10 @@ void esgd_conv2d_halo_plan(int N, int H, int W, int Cin, int Cout, int R, int S,
   int bh = 0;
   if (Cout > 128 || stride != 1 || !halo_applicable(a, H + 2 * pad - R + 1, W + 2 * pad - S + 1, &bh)) return;
   const int PW = W + 2 * pad;
-  const int b_stage = BN * 128, stage_area = BN == 64 ? Cfg<64>::STAGE_AREA : Cfg<128>::STAGE_AREA;
+  const bool pairs = halo_pairs(a, BN);
+  const int b_stage = pairs ? BN * 64 : BN * 128, stage_area = BN == 64 ? Cfg<64>::STAGE_AREA : Cfg<128>::STAGE_AREA;
   const int kb_total = R * S * ((Cin + 63) / 64);
-  const int res_kb = (kb_total * b_stage + 2 * HALO_BYTES <= stage_area) ? kb_total : 0;
+  const int res_kb = (!pairs && kb_total * b_stage + 2 * HALO_BYTES <= stage_area) ? kb_total : 0;
   const int nhalo = res_kb > 0 ? 2 : MAX_HALOS;
   int nstages = 1;
   if (res_kb == 0) {

@@ -54,6 +54,9 @@ struct GemmProblem {
     t.kb1 = min(t.kb0 + kb_per_split, kb_total);
     return true;
   }
+  using Step = int;            // the k-block's number
+  __device__ __forceinline__ Step begin(const Tile& t) const { return t.kb0; }
+  __device__ __forceinline__ void advance(Step& kb) const { ++kb; }
   __device__ __forceinline__ void load_a(const Tile& t, int kb, uint8_t* a, uint64_t* bar) const {
     const int k0 = kb * BK;
     if (A_MN) {

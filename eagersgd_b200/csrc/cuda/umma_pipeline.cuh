@@ -225,7 +225,10 @@ __device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
 //   struct Tile { int kb0, kb1, n0; ... };
 //   int ksteps, n_mma                              16-wide K steps of a k-block that hold anything; MMA columns
 //   bool tile(int it, Tile&)                       enumerate this CTA's tiles
-//   void load(const Tile&, int kb, uint8_t* a, uint8_t* b, uint64_t* bar)
+//   struct Step; Step begin(const Tile&); void advance(Step&)    where a k-block lies, from the tile's first one on.  Counted, not
+//                                                  divided out of the block's number: divisions by run-time numbers made the one
+//                                                  thread that loads the bound of 3x3 layers (125 x 28 x 28 x 128: 37.4 -> 27.4 us)
+//   void load(const Tile&, const Step&, uint8_t* a, uint8_t* b, uint64_t* bar)
 //   void load_a(...a, bar) / load_b(...b, bar)     the two halves of load(); int res_kb (0: B not resident)
 //   void store_panel(const Tile&, int panel, const void* smem)   TMA store of a 128x64 bf16 panel
 //   static constexpr bool kPair                    the CTA is one of a pair (below): tile() gives it its own 128 rows, load()
@@ -261,7 +264,8 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   constexpr bool kPair = P::kPair;
   const bool leads = !kPair || (blockIdx.x & 1) == 0;
   constexpr int kBStage = kPair ? C::B_STAGE_BYTES / 2 : C::B_STAGE_BYTES;
-  const int nstages = kPair ? C::PAIR_STAGES : kHalo ? (res_kb > 0 ? 1 : min(C::MAX_STAGES, (C::STAGE_AREA - nhalo * HALO_BYTES) / C::B_STAGE_BYTES))
+  const int nstages = kHalo ? (res_kb > 0 ? 1 : min(C::MAX_STAGES, (C::STAGE_AREA - nhalo * HALO_BYTES) / kBStage))
+                      : kPair ? C::PAIR_STAGES
                             : (res_kb > 0 ? min(C::MAX_STAGES, (area - res_kb * C::B_STAGE_BYTES) / A_STAGE_BYTES)
                                           : min(STAGES, area / (A_STAGE_BYTES + C::B_STAGE_BYTES)));
   uint8_t* sA = smem;                        // halo mode: the input boxes
@@ -321,13 +325,14 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
       typename P::Tile t;
       if (res_kb > 0 && prob.tile(0, t)) {
         mbar_expect_tx(bres, (uint32_t)(res_kb * C::B_STAGE_BYTES));
-        for (int kb = 0; kb < res_kb; ++kb) prob.load_b(t, kb, sB + kb * C::B_STAGE_BYTES, bres);
+        typename P::Step at = prob.begin(t);
+        for (int kb = 0; kb < res_kb; ++kb, prob.advance(at)) prob.load_b(t, at, sB + kb * C::B_STAGE_BYTES, bres);
       }
       const uint32_t tx_a = ep.tx_bytes_a ? ep.tx_bytes_a : (uint32_t)A_STAGE_BYTES;
       const uint32_t tx_ab = ep.tx_bytes ? ep.tx_bytes : (uint32_t)(A_STAGE_BYTES + C::B_STAGE_BYTES);
       if constexpr (kHalo) {
         // One input box per (tile, channel block), issued one step ahead of the filter tiles it goes with.
-        const int cblks = prob.cblks, taps = prob.R * prob.S;
+        const int cblks = prob.cblks;
         typename P::Tile tn;                     // box iterator, one (tile, block) ahead
         int it_n = 0, cb_n = 0, hs_n = 0;
         uint32_t hph_n = 0;
@@ -335,7 +340,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
         auto issue_box = [&]() -> bool {
           if (!more) return true;
           if (!mbar_wait(&hempty[hs_n], hph_n ^ 1u, abort_flag)) return false;
-          mbar_expect_tx(&hfull[hs_n], ep.tx_bytes_a);
+          if (leads) mbar_expect_tx(&hfull[hs_n], (kPair ? 2 : 1) * ep.tx_bytes_a);
           prob.load_halo(tn, cb_n, sA + hs_n * HALO_BYTES, &hfull[hs_n]);
           if (++hs_n == nhalo) { hs_n = 0; hph_n ^= 1u; }
           if (++cb_n == cblks) { cb_n = 0; more = prob.tile(++it_n, tn); }
@@ -346,28 +351,30 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           for (int cb = 0; ok && cb < cblks; ++cb) {
             ok = issue_box();                    // the next box travels while this block's filter tiles are fed
             if (res_kb > 0) continue;
-            for (int tap = 0; ok && tap < taps; ++tap) {
+            for (int r = 0; ok && r < prob.R; ++r)
+            for (int s = 0; s < prob.S; ++s) {
               if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-              mbar_expect_tx(&full[stage], (uint32_t)C::B_STAGE_BYTES);
-              prob.load_b(t, tap * cblks + cb, sB + stage * C::B_STAGE_BYTES, &full[stage]);
+              if (leads) mbar_expect_tx(&full[stage], (uint32_t)C::B_STAGE_BYTES);          // a pair's halves together
+              prob.load_b(t, typename P::Step{r, s, cb}, sB + stage * kBStage, &full[stage]);
               if (++stage == nstages) { stage = 0; phase ^= 1u; }
             }
           }
         }
       } else
       for (int it = 0; ok && prob.tile(it, t); ++it) {
-        for (int kb = t.kb0; kb < t.kb1; ++kb) {
+        typename P::Step at = prob.begin(t);
+        for (int kb = t.kb0; kb < t.kb1; ++kb, prob.advance(at)) {
           if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
           if constexpr (kPair) {
             // both CTAs' loads arrive at the leader's barrier; it may see the peer's bytes before it expects them
             if (leads) mbar_expect_tx(&full[stage], 2 * (tx_a + (uint32_t)kBStage));
-            prob.load(t, kb, sA + stage * A_STAGE_BYTES, sB + stage * kBStage, leader_addr(&full[stage]));
+            prob.load(t, at, sA + stage * A_STAGE_BYTES, sB + stage * kBStage, leader_addr(&full[stage]));
           } else if (res_kb > 0) {
             mbar_expect_tx(&full[stage], tx_a);
-            prob.load_a(t, kb, sA + stage * A_STAGE_BYTES, &full[stage]);
+            prob.load_a(t, at, sA + stage * A_STAGE_BYTES, &full[stage]);
           } else {
             mbar_expect_tx(&full[stage], tx_ab);
-            prob.load(t, kb, sA + stage * A_STAGE_BYTES, sB + stage * C::B_STAGE_BYTES, &full[stage]);
+            prob.load(t, at, sA + stage * A_STAGE_BYTES, sB + stage * C::B_STAGE_BYTES, &full[stage]);
           }
           if (++stage == nstages) { stage = 0; phase ^= 1u; }
         }
@@ -380,6 +387,18 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
       // Products of one k-block.  Below 64 reduced channels (narrow convolutions) the last steps would multiply zero fill;
       // the full block is a path of its own because a predicate per instruction slows the issue loop of narrow tiles.
       const int ksteps = prob.ksteps;
+      auto commit = [](uint64_t* bar) {
+        if constexpr (kPair) umma_commit_pair(bar);
+        else umma_commit(bar);
+      };
+      auto issue_full = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t& accumulate) {
+        constexpr uint64_t sa = P::A_MN ? (2048 >> 4) : (32 >> 4), sb = P::B_MN ? (2048 >> 4) : (32 >> 4);   // 16 K elements
+#pragma unroll
+        for (int j = 0; j < BK / 16; ++j) {
+          umma_bf16(d, a + j * sa, b + j * sb, idesc, j > 0 ? 1u : accumulate);
+        }
+        accumulate = 1;
+      };
       auto issue_block = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t& accumulate) {
         constexpr uint64_t sa = P::A_MN ? (2048 >> 4) : (32 >> 4), sb = P::B_MN ? (2048 >> 4) : (32 >> 4);   // 16 K elements
         if constexpr (kPair) {
@@ -423,6 +442,12 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
             uint64_t a_row = a_desc0 + (uint64_t)(hs * (HALO_BYTES >> 4));
             uint64_t b_tap = b_desc0 + (uint64_t)(cb * (C::B_STAGE_BYTES >> 4));       // resident: k-block tap*cblks+cb
             const uint64_t b_tap_step = (uint64_t)(cblks * (C::B_STAGE_BYTES >> 4));
+            if (!kPair && res_kb > 0 && R == 3 && S == 3 && ksteps == BK / 16) {
+              // the common filter, all of it there: the 36 products in one straight line
+#pragma unroll
+              for (int tap = 0; tap < 9; ++tap)
+                issue_full(d_tmem, a_row + (uint64_t)(tap / 3) * row_step + (tap % 3) * 8, b_tap + tap * b_tap_step, accumulate);
+            } else
             for (int r = 0; ok && r < R; ++r, a_row += row_step) {
               uint64_t a_tap = a_row;
               for (int sx = 0; sx < S; ++sx, a_tap += 8, b_tap += b_tap_step) {
@@ -430,17 +455,17 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
                 if (res_kb == 0) {
                   if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
                   tc_fence_after();
-                  b_cur = b_desc0 + (uint64_t)(stage * (C::B_STAGE_BYTES >> 4));
+                  b_cur = b_desc0 + (uint64_t)(stage * (kBStage >> 4));
                 }
                 issue_block(d_tmem, a_tap, b_cur, accumulate);
                 if (res_kb == 0) {
-                  umma_commit(&empty[stage]);
+                  commit(&empty[stage]);
                   if (++stage == nstages) { stage = 0; phase ^= 1u; }
                 }
               }
             }
             if (!ok) break;
-            umma_commit(&hempty[hs]);
+            commit(&hempty[hs]);
             if (++hs == nhalo) { hs = 0; hphase ^= 1u; }
           }
         } else
@@ -450,13 +475,11 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           const uint64_t a_cur = a_desc0 + (uint64_t)(stage * (A_STAGE_BYTES >> 4));
           const uint64_t b_cur = b_desc0 + (uint64_t)((res_kb > 0 ? kb : stage) * (kBStage >> 4));
           issue_block(d_tmem, a_cur, b_cur, accumulate);
-          if constexpr (kPair) umma_commit_pair(&empty[stage]);
-          else umma_commit(&empty[stage]);
+          commit(&empty[stage]);
           if (++stage == nstages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        if constexpr (kPair) umma_commit_pair(&tfull[acc]);
-        else umma_commit(&tfull[acc]);
+        commit(&tfull[acc]);
         if (++acc == C::ACCS) { acc = 0; acc_phase ^= 1u; }
       }
     }
@@ -480,44 +503,45 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
     uint64_t st_sum = 0, st_sq = 0;
     uint32_t res_phase = 0;
     bool ok = true;
-    typename P::Tile t;
+    typename P::Tile t, next;               // this tile and the group's next one: where a tile lies takes divisions, once is enough
+    bool more = prob.tile(turn, t);
     auto release_acc = [&](int a) {
       if (kPair) mbar_arrive_at(leader_addr(&tempty[a]));
       else mbar_arrive(&tempty[a]);
     };
     // The residual panel of a unit travels while the group finishes the one before it.
-    auto fetch_residual = [&](int it) {
-      typename P::Tile n;
-      if (!leader || !prob.tile(it, n) || n.n0 + pnl * 64 >= ep.n_total) return;
+    auto fetch_residual = [&](const typename P::Tile& n) {
+      if (!leader || !more || n.n0 + pnl * 64 >= ep.n_total) return;
       mbar_expect_tx(&rfull[grp], ep.res_bytes);
       prob.load_res_panel(n, pnl, rpanel, &rfull[grp]);
     };
-    // ... and the lines of bn_y that a unit will read go to L2 meanwhile, a row per thread.
-    auto prefetch_y = [&](int it) {
-      typename P::Tile n;
-      if (!prob.tile(it, n) || n.n0 + pnl * 64 >= ep.n_total || gt >= prob.valid_prefix(n)) return;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(ep.bn_y + (prob.first_row(n) + gt) * ep.n_total + n.n0 + pnl * 64));
+    // ... and the lines that a unit will read go to L2 meanwhile, a row per thread: bn_y, or a residual panel that can only be
+    // asked for when the panel before it has left their common buffer (392000 x 256 x 64 with a residual: 93 -> 84 us, 98000 x 512 x
+    // 128: 54 -> 49; in pairs of CTAs, whose products are the longer part, 6125 x 2048 x 512, it took 22.7 for 22.1).
+    auto prefetch = [&](const void* p, int ld, const typename P::Tile& n) {
+      if (!more || n.n0 + pnl * 64 >= ep.n_total || gt >= prob.valid_prefix(n)) return;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"((const __nv_bfloat16*)p + (prob.first_row(n) + gt) * ld + n.n0 + pnl * 64));
     };
     uint64_t neg_mean = 0;
-    if (kBn && prob.tile(0, t) && t.n0 + pnl * 64 < ep.n_total) {      // a CTA's tiles share their columns
+    if (kBn && more && t.n0 + pnl * 64 < ep.n_total) {      // a CTA's tiles share their columns
       const float2 m = __ldg(reinterpret_cast<const float2*>(ep.bn_aux + t.n0 + pnl * 64) + cp);
       neg_mean = pack_f32x2(__float_as_uint(-m.x), __float_as_uint(-m.y));
-      prefetch_y(turn);
+      prefetch(ep.bn_y, ep.n_total, t);
     }
-    if (has_res) fetch_residual(turn);
+    if (has_res) fetch_residual(t);
     // The affine map of the group's columns: a thread has one factor or summand, asked for a tile ahead and put down when the
     // columns change.
     float* aff = sAff + grp * 128;
     int aff_n0 = -1;
     float aff_next = 0.0f;
-    auto ask_affine = [&](int it) {
-      typename P::Tile n;
-      if (ep.bias == nullptr || !prob.tile(it, n)) return;
+    auto ask_affine = [&](const typename P::Tile& n) {
+      if (ep.bias == nullptr || !more) return;
       const int col = n.n0 + pnl * 64 + (gt & 63);
       aff_next = gt >= 64 ? bias_at(ep, col) : ep.scale != nullptr && col < ep.n_total ? __ldg(ep.scale + col) : 1.0f;
     };
-    if (!kBn) ask_affine(turn);
-    for (int it = turn; prob.tile(it, t); it += TURNS) {
+    if (!kBn) ask_affine(t);
+    for (int it = turn; more; it += TURNS, t = next) {
+      more = prob.tile(it + TURNS, next);
       const int acc = it % C::ACCS;
       if (!kBn && ep.bias != nullptr) {
         if (t.n0 != aff_n0) {                                  // the same for all of the group
@@ -526,7 +550,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           aff_n0 = t.n0;
           named_barrier_sync(1 + grp, GROUP_THREADS);
         }
-        ask_affine(it + TURNS);
+        ask_affine(next);
       }
       // bn: the mask of this thread's row, and of bn_y this thread's column pair of rows 32rg .. +15 (later +16 .. +31), asked
       // for before the waits
@@ -549,7 +573,8 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&tfull[acc], (uint32_t)(it / C::ACCS) & 1u, abort_flag));
       tc_fence_after();
       const int col0 = t.n0 + pnl * 64;
-      if (kBn) prefetch_y(it + TURNS);
+      if (kBn) prefetch(ep.bn_y, ep.n_total, next);
+      else if (!kPair && !kHalo && has_res) prefetch(ep.residual, ep.ldr, next);
       if (col0 < ep.n_total) {              // uniform across the group
         const int prefix = prob.valid_prefix(t);              // rows [0, prefix) are real outputs
         const int yrows = min(32, max(0, prefix - rg * 32));
@@ -591,7 +616,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           if (leader) {
             prob.store_panel(t, pnl, panel);
             tma_store_commit();
-            if (two_panels) fetch_residual(it + TURNS);        // everybody has read this one
+            if (two_panels) fetch_residual(next);        // everybody has read this one
           }
           if (kBn || ep.col_sum != nullptr) {
             const uint8_t* colp = panel + rg * 32 * 128 + (cp & 3) * 4;
@@ -659,14 +684,14 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
           named_barrier_sync(1 + grp, GROUP_THREADS);         // the statistics are done with the panel, too
           if (leader) {
             tma_store_wait_read<0>();
-            fetch_residual(it + TURNS);
+            fetch_residual(next);
           }
         }
       } else {
         if (lane == 0) release_acc(acc);
         if (has_res && leader) {
           tma_store_wait_read<0>();
-          fetch_residual(it + TURNS);
+          fetch_residual(next);
         }
       }
     }
