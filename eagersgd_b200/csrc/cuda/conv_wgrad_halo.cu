@@ -207,19 +207,34 @@ int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int
   p.nstages = (WG_SMEM - 1024 - 256) / stage_bytes;
   if (p.nstages > 4) p.nstages = 4;
   if (p.nstages < 2) return -7;
-  p.taps_per_set = 512 / BN;
-  if (p.taps_per_set > R * S) p.taps_per_set = R * S;
-  p.sets = (R * S + p.taps_per_set - 1) / p.taps_per_set;
-  p.taps_per_set = (R * S + p.sets - 1) / p.sets;            // balanced sets (9 taps: 5 + 4, or 3 + 3 + 3)
   p.m_tiles = (Cout + 127) / 128;
   p.n_tiles = (Cin + BN - 1) / BN;
   p.boxes_total = p.h_tiles * N;
-  const int base = p.sets * p.m_tiles * p.n_tiles;
-  int splits = (2 * sms + base - 1) / base;                   // two waves of CTAs
-  if (splits > p.boxes_total) splits = p.boxes_total;
-  if (splits < 1) splits = 1;
-  p.boxes_per_split = (p.boxes_total + splits - 1) / splits;
-  p.splits = (p.boxes_total + p.boxes_per_split - 1) / p.boxes_per_split;
+  // One wave of CTAs; taps of a CTA by what they cost.  Many taps share the boxes they read; few leave fewer pixel ranges, whose sums
+  // meet in L2.  A box takes its loads (50 bytes a cycle and SM) or its products (49, 65, 129 cycles for 64, 128, 256 columns),
+  // sums 900 bytes a cycle of the chip.  Measured with 1, 2, 3 and 5 taps, 5 the most that fit (it was that, in two waves of CTAs:
+  // 15.1, 42, 124 us): 128 x 8 x 8 x 64 5.4, 6.3, 7.8, 9.8 us; 64 x 56 x 56 x 64 40, 33, 32, 36; 256 images of these 199, 121, 109,
+  // 116.  With 1 and 2 taps (2 in two waves: 67 and 85 us): 256 x 14 x 14 x 256 56 and 54 us, 256 x 7 x 7 x 512 55 and 72.
+  const int most = 512 / BN < R * S ? 512 / BN : R * S, per_mma = BN == 64 ? 49 : BN + 1;
+  const int box_bytes = ((Cout < 128 ? (Cout + 63) / 64 : 2) * bh + BN / 64 * (bh + R - 1)) * p.PW * 128;
+  double best = 0.0;
+  for (int n = 1; n <= most; ++n) {
+    const int sets = (R * S + n - 1) / n, taps = (R * S + sets - 1) / sets;      // balanced (9 taps: 5 + 4, or 3 + 3 + 3)
+    const int base = sets * p.m_tiles * p.n_tiles;
+    int splits = sms / base;
+    if (splits > p.boxes_total) splits = p.boxes_total;
+    if (splits < 1) splits = 1;
+    const int boxes = (p.boxes_total + splits - 1) / splits, products = taps * p.ksteps * per_mma;
+    splits = (p.boxes_total + boxes - 1) / boxes;
+    const double cost = (double)((base * splits + sms - 1) / sms) * boxes * (products > box_bytes / 50 ? products : box_bytes / 50) +
+                        (double)base * splits * taps * BN * (Cout < 128 ? Cout : 128) * 4 / 900;
+    if (n > 1 && cost >= best) continue;
+    best = cost;
+    p.sets = sets;
+    p.taps_per_set = taps;
+    p.boxes_per_split = boxes;
+    p.splits = splits;
+  }
   return 0;
 }
 
