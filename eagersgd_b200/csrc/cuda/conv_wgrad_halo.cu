@@ -190,9 +190,143 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
   }
 }
 
+// 3x3 layers of 64 input and at most 64 output channels, all nine taps in one CTA and two products a K step.  A product of 128 x 64 is
+// bound by the bytes it reads from shared memory (49 cycles where 32 would do), and of its 128 rows such a layer fills 64.  So
+// the rows are output channels of two taps, dy and dy one pixel earlier (blocks of 64 rows 128 bytes apart):
+//   sum over p of dy[p] x[p + r PW + 1]  =  sum over q of dy[q - 1] x[q + r PW],
+// and the columns are three blocks of 64, x one box row of pixels apart: taps (0..2, 0..1) in one product of 128 x 192, taps (0..2, 2)
+// in another (its lower rows are not used).  193 cycles a K step where taps one by one took 441, and dy and x are read once.
+// The sums leave by way of shared memory, a bulk reduction for each output channel.
+constexpr int kPackedLead = 1024;             // zeros in front of dy: the pixel before the first
+constexpr int kPackedPitch = 9 * 64 + 4;      // floats of an output channel's sums (an odd number of 16 bytes: no bank conflicts)
+constexpr int kPackedBank = 64 * kPackedPitch * 4;
+
+__global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_packed_kernel(const __grid_constant__ WgHaloParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int stage_bytes = p.abox + p.xbox;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + max(p.nstages * stage_bytes, kPackedBank));
+  uint64_t* empty = full + 4;
+  uint64_t* done = empty + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int box0 = blockIdx.x * p.boxes_per_split, box1 = min(box0 + p.boxes_per_split, p.boxes_total);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.nstages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&p.tmDY);
+    tma_prefetch_desc(&p.tmX);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  {
+    // what the boxes do not cover reads as zeros (dy: the pixel in front, K padding) or as finite values (x) for ever
+    uint4* p4 = reinterpret_cast<uint4*>(smem);
+    for (int i = threadIdx.x; i < p.nstages * stage_bytes / 16; i += WG_THREADS) p4[i] = make_uint4(0, 0, 0, 0);
+    fence_proxy_async();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  esgd::pdl_enter();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      int n = box0 / p.h_tiles, h = box0 - n * p.h_tiles;
+      for (int b = box0; b < box1; ++b) {
+        if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag)) break;
+        uint8_t* sa = smem + stage * stage_bytes;
+        mbar_expect_tx(&full[stage], (uint32_t)((2 * p.BH + 2) * p.PW * 128));
+        tma_load_4d(sa + kPackedLead, &p.tmDY, &full[stage], 0, 0, h * p.BH, n);
+        tma_load_4d(sa + p.abox, &p.tmX, &full[stage], 0, -p.pad, h * p.BH - p.pad, n);
+        if (++h == p.h_tiles) { h = 0; ++n; }
+        if (++stage == p.nstages) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc_bf16(128, 192, 1, 1);
+      int stage = 0;
+      uint32_t phase = 0, accumulate = 0;
+      bool ok = true;
+      constexpr uint64_t kstep = 2048 >> 4;                      // 16 pixel rows
+      const int ksteps = p.ksteps;                               // <= 8
+      for (int b = box0; ok && b < box1; ++b) {
+        if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + stage * stage_bytes);
+        const uint64_t a0 = umma_smem_desc(sa + kPackedLead - 128, 128, 1024), a1 = a0 + 8;      // one pixel further on
+        const uint64_t x0 = umma_smem_desc(sa + p.abox, (uint32_t)(p.PW * 128), 1024), x1 = x0 + 16;   // two pixels further on
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
+          if (ks < ksteps) {
+            umma_bf16(tmem_base, a0 + ks * kstep, x0 + ks * kstep, idesc, ks > 0 ? 1u : accumulate);
+            umma_bf16(tmem_base + 192, a1 + ks * kstep, x1 + ks * kstep, idesc, ks > 0 ? 1u : accumulate);
+          }
+        accumulate = 1;
+        umma_commit(&empty[stage]);
+        if (++stage == p.nstages) { stage = 0; phase ^= 1u; }
+      }
+      if (ok) umma_commit(done);
+    }
+  } else {
+    // ---- epilogue: once, after the CTA's whole pixel range
+    const int q = warp & 3;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(done, 0u, abort_flag)) && box1 > box0;
+    float* bank = reinterpret_cast<float*>(smem);
+    if (ok) {
+      tc_fence_after();
+      float* row = bank + ((q & 1) * 32 + lane) * kPackedPitch;
+      for (int part = 0; part < (q < 2 ? 2 : 1); ++part) {       // the second product has its rows in the first half alone
+        const int s = part == 1 ? 2 : q < 2 ? 1 : 0;
+#pragma unroll 1
+        for (int c = 0; c < 6; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * 192 + c * 32), v);
+          tmem_ld_wait();
+          float4* to = reinterpret_cast<float4*>(row + ((c >> 1) * 3 + s) * 64 + (c & 1) * 32);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            to[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+        }
+      }
+      tc_fence_before();
+      fence_proxy_async();
+    }
+    named_barrier_sync(1, 128);
+    const int k0 = (int)threadIdx.x - 64;
+    if (ok && k0 < p.Cout) {
+      // CTAs start with different channels: they would meet on the same lines
+      const int k = (int)((k0 + blockIdx.x * 7) % p.Cout);
+      asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(p.dw + (size_t)k * 576),
+                   "r"(smem_u32(bank + k * kPackedPitch)), "r"(576u * 4u) : "memory");
+      asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    __nanosleep(1000000);
+    if (threadIdx.x == 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 1);
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
 // Geometry of a launch (host arithmetic only, shared by the launcher and by the plan query that the CPU tests
 // sweep): box sizes, stages, tap sets, pixel splits.  Returns -7 when two stages do not fit.
-int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int R, int S, int pad, int bh, int sms) {
+int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int R, int S, int pad, int bh, int sms, double* cost_out = nullptr) {
   p.N = N; p.Cout = Cout; p.Cin = Cin; p.R = R; p.S = S; p.pad = pad;
   p.Ho = H + 2 * pad - R + 1;
   p.Wo = W + 2 * pad - S + 1;
@@ -235,7 +369,26 @@ int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int
     p.boxes_per_split = boxes;
     p.splits = splits;
   }
+  if (cost_out != nullptr) *cost_out = best;
   return 0;
+}
+
+// The packed kernel's geometry and what it costs, in the terms of wg_plan (bulk reductions: 1400 bytes a cycle); false: not its shape.
+// 64 channels, taps one by one and packed: 4 x 56 x 56 6.3 and 9.3 us, 8 images 8.3 and 10.5, 16 13.3 and 12.5, 64 32 and 21, 256 108 and
+// 62; 128 x 8 x 8 5.3 and 8.7, 2048 x 8 x 8 33 and 17, 1024 x 16 x 16 59 and 24.  The model draws the line between 8 and 16, 512 and 2048.
+bool wg_packed_plan(WgHaloParams& p, int Cin, int Cout, int R, int S, int sms, double* cost) {
+  if (R != 3 || S != 3 || Cin != 64 || Cout > 64) return false;
+  p.abox = kPackedLead + (p.ksteps * 16 + 1) * 128;
+  p.abox = (p.abox + 1023) / 1024 * 1024;
+  p.nstages = (WG_SMEM - 1024 - 256) / (p.abox + p.xbox);
+  if (p.nstages > 4) p.nstages = 4;
+  if (p.nstages < 2) return false;
+  p.splits = sms < p.boxes_total ? sms : p.boxes_total;
+  p.boxes_per_split = (p.boxes_total + p.splits - 1) / p.splits;
+  p.splits = (p.boxes_total + p.boxes_per_split - 1) / p.boxes_per_split;
+  const int box_bytes = (2 * p.BH + 2) * p.PW * 128, products = p.ksteps * 2 * 97;
+  *cost = (double)p.boxes_per_split * (products > box_bytes / 50 ? products : box_bytes / 50) + (double)p.splits * kPackedBank / 1400;
+  return true;
 }
 
 // Largest number of full output rows whose pitched pixels fit one 128-row K range; 0: outside this kernel's range.
@@ -261,8 +414,12 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
     attr_set = true;
   }
   WgHaloParams p;
-  const int pr = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, esgd::sm_count());
+  double cost = 0.0, packed_cost = 0.0;
+  const int pr = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, esgd::sm_count(), &cost);
   if (pr != 0) return pr;
+  WgHaloParams packed = p;
+  const bool use_packed = BN == 64 && ((uintptr_t)dw & 15) == 0 && wg_packed_plan(packed, Cin, Cout, R, S, esgd::sm_count(), &packed_cost) && packed_cost < cost;
+  if (use_packed) p = packed;
   p.dw = dw;
   p.error_flag = error_flag;
   {
@@ -278,6 +435,15 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
     uint32_t box[4] = {64, (uint32_t)p.PW, (uint32_t)(bh + R - 1), 1};
     int r = esgd::make_tensormap_bf16(&p.tmX, x, 4, dims, strides, box, nullptr);
     if (r != 0) return 2000 + r;
+  }
+  if (use_packed) {
+    static bool packed_set = false;
+    if (!packed_set) {
+      cudaError_t e = cudaFuncSetAttribute(conv_wgrad_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
+      if (e != cudaSuccess) return (int)e;
+      packed_set = true;
+    }
+    return esgd::launch(conv_wgrad_packed_kernel, dim3(p.splits), WG_THREADS, WG_SMEM, stream, p);
   }
   const int grid = p.sets * p.m_tiles * p.n_tiles * p.splits;
   return esgd::launch(conv_wgrad_halo_kernel<BN>, dim3(grid), WG_THREADS, WG_SMEM, stream, p);

@@ -18,10 +18,11 @@ def _close(got, ref, magnitude):
 
 
 # n, h, w, channels: pairs with 175, 91 and 76 boxes, a width that fills no tile, two blocks of input channels; tiles of one CTA with all
-# filters there; too few boxes for 128 columns; weight gradients with 1, 2 and 3 taps
+# filters there; too few boxes for 128 columns; weight gradients with 1, 2 and 3 taps,
+# and with all nine (odd rows, 40 output channels, small images)
 @pytest.mark.parametrize("n,h,w,cin,cout", [(25, 28, 28, 128, 128), (13, 28, 28, 128, 128), (19, 28, 28, 64, 128), (31, 20, 22, 192, 128),
                                             (5, 56, 56, 64, 64), (9, 28, 28, 64, 96), (1, 28, 28, 128, 128), (40, 8, 8, 64, 64),
-                                            (64, 56, 56, 64, 64), (24, 14, 14, 256, 256), (8, 7, 7, 512, 512)])
+                                            (64, 56, 56, 64, 64), (24, 56, 56, 64, 40), (1024, 8, 8, 64, 64), (40, 34, 40, 64, 64), (24, 14, 14, 256, 256), (8, 7, 7, 512, 512)])
 def test_3x3(n, h, w, cin, cout):
     from eagersgd_b200.ops import functional as ops
     from eagersgd_b200.ops.gemm import check_error
@@ -57,3 +58,18 @@ def test_residual(n, h, cin, cout, k):
     scale, shift = coef.double().view(2, 1, cout, 1, 1)
     xd, wd = x.double(), wt.double()
     _close(y, F.relu(conv(xd, wd) * scale + shift + res.double()), conv(xd.abs(), wd.abs()) * scale + shift + res.double().abs())
+
+
+# odd sizes, rows in two boxes, one image and many, channels that fill no block
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 7, 9, 64, 256), (5, 15, 31, 72, 40), (2, 5, 300, 64, 128), (130, 8, 8, 256, 512), (1, 1, 1, 8, 8)])
+def test_strided_1x1_inference(n, h, w, cin, cout):
+    from eagersgd_b200.ops import functional as ops
+    g = torch.Generator().manual_seed(n + h + w)
+    rnd = lambda *s: _cl(torch.randn(*s, generator=g)).bfloat16().cuda()
+    x, wt = rnd(n, cin, h, w), rnd(cout, cin, 1, 1) / 8
+    coef = torch.rand(2, cout, generator=g).cuda() + 0.5
+    y = ops.conv_bn_eval(x, wt, 2, 0, coef, True, None)
+    conv = lambda a, b: F.conv2d(a, b, None, 2)
+    scale, shift = coef.double().view(2, 1, cout, 1, 1)
+    xd, wd = x.double(), wt.double()
+    _close(y, F.relu(conv(xd, wd) * scale + shift), conv(xd.abs(), wd.abs()) * scale + shift)
