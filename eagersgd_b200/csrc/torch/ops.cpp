@@ -541,6 +541,14 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
   if (kind == kOneByOne) {
     *filters = dense(w);                            // [Cout, Cin]: a 1x1 filter has one memory order
     *kept = x;
+    if (stride == 2 && !e.train) {                  // nothing reads the subsampled input again: its pixels are picked by the loads
+      const int rc = esgd_conv2d_fwd(x.data_ptr(), filters->data_ptr(), y.data_ptr(), n, h, wd, cin, cout, 1, 1, 2, 0, e.scale, e.shift,
+                                     e.residual, e.relu, e.sum, e.sqsum, flag_ptr(x), st);
+      if (rc >= 0) {                                // negative: refused, nothing launched
+        ck(rc, "1x1 convolution");
+        return;
+      }
+    }
     if (stride == 2) {
       *kept = empty_nhwc(n, cin, ho, wo, x);
       ck(esgd_subsample2_fwd(x.data_ptr(), kept->data_ptr(), n, h, wd, cin, st), "subsample");
