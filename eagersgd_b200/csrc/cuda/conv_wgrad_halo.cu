@@ -42,7 +42,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int NA = 2, NB = BN / 64;                  // 64-channel atoms of the dy (128 rows) and x operands
   const int stage_bytes = NA * p.abox + NB * p.xbox;
-  uint8_t* bar_area = smem + p.nstages * stage_bytes;
+  constexpr int kPitch = BN * 4 + 16, kBank = 128 * kPitch;         // sums on their way out: an odd number of 16 bytes a row
+  uint8_t* bar_area = smem + max(p.nstages * stage_bytes, kBank);
   uint64_t* full = reinterpret_cast<uint64_t*>(bar_area);
   uint64_t* empty = full + 4;
   uint64_t* done = empty + 4;
@@ -152,31 +153,62 @@ __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __
       umma_commit(done);
     }
   } else {
-    // ---- epilogue: once, after the CTA's whole pixel range
-    const int q = warp & 3, row = q * 32 + lane;
-    const bool have = box1 > box0;
-    if (mbar_wait(done, 0u, abort_flag) && have) {
-      tc_fence_after();
+    // ---- epilogue: once, after the CTA's whole pixel range.  A tap's sums go to shared memory, then a bulk reduction for each output
+    // channel; rows of 64 channels are short for that, and a reduction of 16 bytes for each thread and four columns is quicker
+    // (16 bytes at a time and in bulk: 64 x 28 x 28 x 128 20.5 and 18.3 us, 64 x 7 x 7 x 512 20.9 and 19.0, 128 x 8 x 8 x 64 5.3 and 6.0).
+    const int q = warp & 3, row = q * 32 + lane, banks = 2 * kBank <= p.nstages * stage_bytes ? 2 : 1;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(done, 0u, abort_flag)) && box1 > box0;
+    const int out = ((int)threadIdx.x - 64 + split * 37) & 127;      // the CTAs of a range meet on different lines
+    if (ok) tc_fence_after();
+    if (BN == 64 && ok) {
       const int k = m0 + row;
       for (int tl = 0; tl < ntaps; ++tl) {
-        float* out_row = k < p.Cout ? p.dw + ((size_t)k * (p.R * p.S) + tap0 + tl) * p.Cin : nullptr;
+        float* to = k < p.Cout ? p.dw + ((size_t)k * (p.R * p.S) + tap0 + tl) * p.Cin : nullptr;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(tl * BN + c * 32), v);
           tmem_ld_wait();
           const int col0 = n0 + c * 32;
-          if (out_row != nullptr) {
+          if (to != nullptr) {
 #pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4)
-              if (col0 + j4 * 4 < p.Cin)
-                atomicAdd(reinterpret_cast<float4*>(out_row + col0 + j4 * 4),
-                          make_float4(__uint_as_float(v[j4 * 4]), __uint_as_float(v[j4 * 4 + 1]),
-                                      __uint_as_float(v[j4 * 4 + 2]), __uint_as_float(v[j4 * 4 + 3])));
+            for (int j = 0; j < 32; j += 4)
+              if (col0 + j < p.Cin)
+                atomicAdd(reinterpret_cast<float4*>(to + col0 + j),
+                          make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])));
           }
         }
       }
     }
+    for (int tl = 0; BN > 64 && tl < ntaps; ++tl) {
+      uint8_t* bank = smem + (tl & (banks - 1)) * kBank;
+      if (tl >= banks) {
+        if (banks == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        named_barrier_sync(1, 128);
+      }
+      if (ok) {
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(tl * BN + c * 32), v);
+          tmem_ld_wait();
+          float4* to = reinterpret_cast<float4*>(bank + row * kPitch + c * 128);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            to[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+        }
+        fence_proxy_async();
+      }
+      named_barrier_sync(1, 128);
+      if (ok && m0 + out < p.Cout)
+        asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(
+                         p.dw + ((size_t)(m0 + out) * (p.R * p.S) + tap0 + tl) * p.Cin + n0),
+                     "r"(smem_u32(bank + out * kPitch)), "r"((uint32_t)(min(BN, p.Cin - n0) * 4)) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    tc_fence_before();
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
@@ -346,9 +378,9 @@ int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int
   p.boxes_total = p.h_tiles * N;
   // One wave of CTAs; taps of a CTA by what they cost.  Many taps share the boxes they read; few leave fewer pixel ranges, whose sums
   // meet in L2.  A box takes its loads (50 bytes a cycle and SM) or its products (49, 65, 129 cycles for 64, 128, 256 columns),
-  // sums 900 bytes a cycle of the chip.  Measured with 1, 2, 3 and 5 taps, 5 the most that fit (it was that, in two waves of CTAs:
+  // sums 900 bytes a cycle of the chip (in bulk 1800).  Measured with 1, 2, 3 and 5 taps, 5 the most that fit (it was that, in two waves of CTAs:
   // 15.1, 42, 124 us): 128 x 8 x 8 x 64 5.4, 6.3, 7.8, 9.8 us; 64 x 56 x 56 x 64 40, 33, 32, 36; 256 images of these 199, 121, 109,
-  // 116.  With 1 and 2 taps (2 in two waves: 67 and 85 us): 256 x 14 x 14 x 256 56 and 54 us, 256 x 7 x 7 x 512 55 and 72.
+  // 116.  With 1 and 2 taps (2 in two waves: 45 and 85 us): 64 x 7 x 7 x 512 19.8 and 26.5, 256 images 53 and 69.
   const int most = 512 / BN < R * S ? 512 / BN : R * S, per_mma = BN == 64 ? 49 : BN + 1;
   const int box_bytes = ((Cout < 128 ? (Cout + 63) / 64 : 2) * bh + BN / 64 * (bh + R - 1)) * p.PW * 128;
   double best = 0.0;
@@ -361,7 +393,7 @@ int wg_plan(WgHaloParams& p, int BN, int N, int H, int W, int Cin, int Cout, int
     const int boxes = (p.boxes_total + splits - 1) / splits, products = taps * p.ksteps * per_mma;
     splits = (p.boxes_total + boxes - 1) / boxes;
     const double cost = (double)((base * splits + sms - 1) / sms) * boxes * (products > box_bytes / 50 ? products : box_bytes / 50) +
-                        (double)base * splits * taps * BN * (Cout < 128 ? Cout : 128) * 4 / 900;
+                        (double)base * splits * taps * BN * (Cout < 128 ? Cout : 128) * 4 / (BN == 64 ? 900 : 1800);
     if (n > 1 && cost >= best) continue;
     best = cost;
     p.sets = sets;
@@ -390,6 +422,10 @@ bool wg_packed_plan(WgHaloParams& p, int Cin, int Cout, int R, int S, int sms, d
   *cost = (double)p.boxes_per_split * (products > box_bytes / 50 ? products : box_bytes / 50) + (double)p.splits * kPackedBank / 1400;
   return true;
 }
+
+// Input channels of a tile.  128 leave room for the sums of four taps, 256 for two.  128 and 256: 8 x 14 x 14 x 256 6.7 and 8.7 us, 64
+// images 18.0 and 19.3, 256 images 45.5 and 53.6; but 64 x 7 x 7 x 512, whose boxes are small, 24.5 and 20.0, 256 images 68 and 53.
+int columns(int Cin) { return Cin <= 64 ? 64 : (Cin <= 256 ? 128 : 256); }
 
 // Largest number of full output rows whose pitched pixels fit one 128-row K range; 0: outside this kernel's range.
 int wg_pick_bh(int H, int W, int Cin, int Cout, int R, int S, int pad) {
@@ -465,8 +501,8 @@ int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int 
   if (bh == 0) return -100;
   cudaStream_t s = (cudaStream_t)stream;
   int rc;
-  if (Cin <= 64) rc = launch_wgrad_halo<64>(x, dy, dw, N, H, W, Cin, Cout, R, S, pad, bh, error_flag, s);
-  else if (Cin <= 128) rc = launch_wgrad_halo<128>(x, dy, dw, N, H, W, Cin, Cout, R, S, pad, bh, error_flag, s);
+  if (columns(Cin) == 64) rc = launch_wgrad_halo<64>(x, dy, dw, N, H, W, Cin, Cout, R, S, pad, bh, error_flag, s);
+  else if (columns(Cin) == 128) rc = launch_wgrad_halo<128>(x, dy, dw, N, H, W, Cin, Cout, R, S, pad, bh, error_flag, s);
   else rc = launch_wgrad_halo<256>(x, dy, dw, N, H, W, Cin, Cout, R, S, pad, bh, error_flag, s);
   return rc == -7 ? -100 : rc;          // boxes too large for two stages: the per-tap kernel takes the shape
 }
@@ -478,7 +514,7 @@ void esgd_conv2d_wgrad_halo_plan(int N, int H, int W, int Cin, int Cout, int R, 
   for (int i = 0; i < 16; ++i) out[i] = 0;
   const int bh = wg_pick_bh(H, W, Cin, Cout, R, S, pad);
   if (bh == 0) return;
-  const int BN = Cin <= 64 ? 64 : (Cin <= 128 ? 128 : 256);
+  const int BN = columns(Cin);
   WgHaloParams p;
   if (wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, sms) != 0) return;
   out[0] = 1; out[1] = p.BH; out[2] = p.PW; out[3] = p.ksteps; out[4] = p.abox; out[5] = p.xbox; out[6] = p.nstages;
