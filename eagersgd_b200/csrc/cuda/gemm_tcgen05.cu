@@ -256,6 +256,29 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
   return launch_major<256>(a_mn, b_mn, g, ep, s);
 }
 
+// Split-K factor of a weight gradient, [cout][cin] sums over `pixels`, as esgd_gemm_bf16 will launch it: the one with the least work in
+// whole rounds of the SMs (or pairs of them) and sums that meet in L2.  Cycles: 250, 300, 600 for a k-block of a tile of 64, 128, 256
+// columns, 450 for a pair's; 1000 a tile; 1600 bytes of sums.  One more split than fits a round costs a whole round: with "as many as
+// fill the SMs", rounded up, 50176 x 1024 x 256 took 19 splits and 36.3 us, 18 take 27.5; 12544 x 2048 x 512 5 and 32.8, 4 24.4;
+// 3136 x 2048 x 512 5 and 16.3, 2 10.4.  Over 45 shapes of 784 to 802816 pixels the choice is within 5 % of the best (0.5 % on average).
+int esgd_gemm_wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int sms) {
+  const int64_t blocks = (pixels + BK - 1) / BK, bank = cout * cin * 4, most = blocks < sms ? blocks : sms;
+  int64_t best = 0, chosen = 1;
+  for (int64_t s = 1; s <= most; ++s) {
+    const int64_t per = (blocks + s - 1) / s, splits = (blocks + per - 1) / per;
+    if (splits != s) continue;                                  // the same launch as a smaller number
+    const int bn = tile_columns((int)cin, (int)((cout + BM - 1) / BM * s), sms);
+    const bool pair = bn == 256 && cout > BM && cin > BM && pixels > 4 * BK && (cin + 255) / 256 <= sms / 2;
+    const int64_t rows = pair ? 2 * BM : BM, workers = pair ? sms / 2 : sms;
+    const int64_t rounds = ((cout + rows - 1) / rows * ((cin + bn - 1) / bn) * s + workers - 1) / workers;
+    const int64_t cost = rounds * (per * (pair ? 450 : bn == 64 ? 250 : bn == 128 ? 300 : 600) + 1000) + s * bank / 1600;
+    if (s > 1 && cost >= best) continue;
+    best = cost;
+    chosen = s;
+  }
+  return (int)chosen;
+}
+
 // Data gradient of a 1x1 convolution behind a batch norm: dx [M][N] = dy [M][K] * w [K][N] (+ residual), see bn_grad.h.
 // -100: not a shape for it.
 int esgd_gemm_bn_dgrad(const void* dy, const void* w, void* dx, int M, int N, int K, const void* residual, const esgd_bn_grad* bn,

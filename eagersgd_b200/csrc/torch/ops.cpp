@@ -21,6 +21,7 @@
 
 extern "C" {
 int esgd_sm_count();
+int esgd_gemm_wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int sms);
 int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int a_mn, int b_mn,
                    int out_mode, const float* scale, const void* bias, int relu, int splits, float* col_sum, float* col_sqsum,
                    const void* residual, int ldr, int* error_flag, void* stream);
@@ -408,12 +409,17 @@ int gemm(const void* a, const void* b, void* c, int64_t m, int64_t n, int64_t k,
                         cq, res, (int)ldr, flag_ptr(like), stream_of(like));
 }
 
-// Split-K factor of a weight-gradient GEMM (K = pixels): about one wave of tiles.  Each split adds a full [Cout, Cin]
-// partial result (reductions in L2), so large filter banks take few splits.
+// Split-K factor of a weight-gradient GEMM (K = pixels).  Looked for among a hundred of them: a thread remembers its sizes.
 int wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int64_t sms) {
-  const int64_t bn = cin <= 64 ? 64 : (cin <= 128 ? 128 : 256);
-  const int64_t tiles = ((cout + 127) / 128) * ((cin + bn - 1) / bn);
-  return (int)std::max<int64_t>(2, std::min((sms + tiles - 1) / tiles, std::max<int64_t>(1, (pixels / 64) / 8)));
+  struct Known {
+    int64_t pixels = 0, cout = 0, cin = 0, sms = 0;
+    int splits = 0;
+  };
+  static thread_local Known known[64];
+  Known& k = known[(pixels * 31 + cout * 7 + cin) / 8 % 64];
+  if (k.splits == 0 || k.pixels != pixels || k.cout != cout || k.cin != cin || k.sms != sms)
+    k = Known{pixels, cout, cin, sms, esgd_gemm_wgrad_splits(pixels, cout, cin, (int)sms)};
+  return k.splits;
 }
 
 // ---------------------------------------------------------------- convolutions
