@@ -505,10 +505,10 @@ int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, 
   p.n_tiles = (a.Cin + BN - 1) / BN;
   const int sms = sm_count();
   const int base_tiles = a.R * a.S * p.m_tiles * p.n_tiles;
-  // Every split adds a whole filter bank of partial sums (TMA reductions): two waves of tiles when the bank is small, one
-  // wave when it is large (the sums of a 512 x 512 x 9 bank are already more bytes than its loads).
-  const int waves = base_tiles < 32 ? 2 : 1;
-  int splits = (waves * sms + base_tiles - 1) / base_tiles;
+  // As many splits as one wave of CTAs takes: every split adds a whole filter bank of partial sums, and one more than fits costs a
+  // wave (rounded up, in one or two waves by the size of the bank, and this way, stride 2: 256 x 56 x 56 x 128 82 and 68 us, 256 x 28 x
+  // 28 x 256 125 and 96, 64 images of these 33 and 25, 256 x 14 x 14 x 512 74 and 59).
+  int splits = sms / base_tiles;
   if (splits < 1) splits = 1;
   if (splits > p.boxes_total) splits = p.boxes_total;
   p.boxes_per_split = (p.boxes_total + splits - 1) / splits;
