@@ -23,6 +23,7 @@
 #include "launch.cuh"
 #include "tensormap.cuh"
 #include "umma_pipeline.cuh"
+#include "umma_split.cuh"
 
 using namespace umma;
 using esgd::sm_count;
@@ -92,16 +93,23 @@ struct ConvProblem {
       n_idx = id % n_tiles;
     }
     if (kPair) m_idx = 2 * m_idx + (int)(blockIdx.x & 1);
+    place(m_idx, n_idx, t);
+    return true;
+  }
+  __device__ __forceinline__ void place(int m_idx, int n_idx, Tile& t) const {
     t.w0 = (m_idx % w_tiles) * BW;
     t.h0 = ((m_idx / w_tiles) % h_tiles) * BH;
     t.i0 = (m_idx / (w_tiles * h_tiles)) * BI;
     t.n0 = n_idx * BN;
     t.kb0 = 0;
     t.kb1 = R * S * cblks;
-    return true;
   }
   using Step = TapStep;
-  __device__ __forceinline__ Step begin(const Tile&) const { return Step{0, 0, 0}; }
+  __device__ __forceinline__ Step begin(const Tile& t) const {
+    if (t.kb0 == 0) return Step{0, 0, 0};
+    const int tap = t.kb0 / cblks;
+    return Step{tap / S, tap % S, t.kb0 - tap * cblks};
+  }
   __device__ __forceinline__ void advance(Step& k) const { next_tap(k, cblks, S); }
   __device__ __forceinline__ void load_a(const Tile& t, const Step& k, uint8_t* a, uint64_t* bar) const {
     tma_load_4d(a, &tmX, bar, k.cb * 64, t.w0 * stride + k.s - pad, t.h0 * stride + k.r - pad, t.i0);
@@ -287,6 +295,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) conv_kernel(const __grid_const
   run<P, kBn>(prob, ep);
 }
 
+template <class P, int S>
+__global__ void __launch_bounds__(SPLIT_THREADS, 1) conv_split_kernel(const __grid_constant__ P prob, const Epilogue ep, const SplitOut so) {
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&prob.tmX);
+    tma_prefetch_desc(&prob.tmW);
+  }
+  run_split<P, S>(prob, ep, so);
+}
+
 template <class P>
 __global__ void __launch_bounds__(NUM_THREADS, 1) conv_wgrad_kernel(const __grid_constant__ P prob, const Epilogue ep) {
   if (threadIdx.x == 0) {
@@ -319,8 +336,9 @@ inline int ksteps_of(int c) { return c >= 64 ? BK / 16 : (c + 15) / 16; }
 // narrow layers: the MMA computes no more columns than there are (the epilogue drops the rest either way)
 inline int mma_columns(int n, int bn) { return n >= bn ? bn : (n + 15) / 16 * 16; }
 
+// split: CTAs that share the reduction of a tile (64 columns), 1 for the pipeline.
 template <int BN, bool kT, bool kBn, bool kPair = false>
-int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
+int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream, int split = 1) {
   using P = ConvProblem<BN, kT, kPair>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -374,6 +392,17 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream) {
     if (r == 0 && ep.residual != nullptr) r = esgd::make_tensormap_bf16(&p.tmR, ep.residual, 4, dims, strides, box, nullptr);
     if (r != 0) return 3000 + r;
     ep.res_bytes = (uint32_t)(p.BW * p.BH * p.BI * 128);
+  }
+  if constexpr (BN == 64 && !kBn && !kPair) {
+    if (split > 1) {
+      const int tiles = p.w_tiles * p.h_tiles * p.i_tiles * p.n_tiles, blocks = a.R * a.S * p.cblks;
+      ep.tx_bytes = (uint32_t)(p.BW * p.BH * p.BI * 128 + Cfg<BN>::B_STAGE_BYTES);
+      p.res_kb = p.fixed_n = 0;
+      const SplitOut so{(__nv_bfloat16*)a.y, a.Cout, p.n_tiles, blocks, (blocks + split - 1) / split};
+      if (split == 2) return launch_split<2>(conv_split_kernel<P, 2>, tiles, stream, p, ep, so);
+      if (split == 4) return launch_split<4>(conv_split_kernel<P, 4>, tiles, stream, p, ep, so);
+      return launch_split<8>(conv_split_kernel<P, 8>, tiles, stream, p, ep, so);
+    }
   }
   const int sms = kPair ? sm_count() / 2 : sm_count();           // workers: CTAs, or pairs of them
   const int boxes = p.w_tiles * p.h_tiles * p.i_tiles, total = (kPair ? (boxes + 1) / 2 : boxes) * p.n_tiles;
@@ -558,10 +587,25 @@ int tile_width(const ConvArgs& a, int Ho, int Wo) {
   return tile_columns(a.Cout, (int)(((int64_t)a.N * Ho * Wo + BM - 1) / BM), sm_count());
 }
 
+// Tiles of 64 columns that launch() will make of the output.
+int64_t conv_tiles(const ConvArgs& a, int Ho, int Wo) {
+  const int bw = Wo < 128 ? Wo : 128;
+  int bh = 1, bi = 1;
+  if (Wo < 128) {
+    for (int d = 1; d <= 128 / bw && d <= Ho; ++d) if (Ho % d == 0) bh = d;
+    if (bh == Ho) bi = 128 / (bw * bh) < 1 ? 1 : 128 / (bw * bh) > a.N ? a.N : 128 / (bw * bh);
+  }
+  return (int64_t)((Wo + bw - 1) / bw) * ((Ho + bh - 1) / bh) * ((a.N + bi - 1) / bi) * ((a.Cout + 63) / 64);
+}
+
 template <bool kT, bool kBn = false>
 int dispatch(const ConvArgs& a, const Epilogue& ep, cudaStream_t s) {
   const int Ho = a.out_h ? a.out_h : (a.H + 2 * a.pad - a.R) / a.stride + 1, Wo = a.out_w ? a.out_w : (a.W + 2 * a.pad - a.S) / a.stride + 1;
   const int BN = tile_width(a, Ho, Wo);
+  if (!kBn && BN == 64 && ep.col_sum == nullptr && !a.ys_w && a.Cin % 64 == 0) {
+    const int split = split_ctas(conv_tiles(a, Ho, Wo), a.R * a.S * (a.Cin / 64), sm_count());
+    if (split > 1) return launch<64, kT, false>(a, ep, s, split);
+  }
   int bh = 0;
   if (a.Cout <= 128 && halo_applicable(a, (a.H + 2 * a.pad - a.R) / a.stride + 1, (a.W + 2 * a.pad - a.S) / a.stride + 1, &bh))
     return BN == 64                   ? launch_halo<64, kT, kBn>(a, ep, bh, s)

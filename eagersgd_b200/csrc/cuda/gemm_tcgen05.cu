@@ -13,6 +13,7 @@
 #include "launch.cuh"
 #include "tensormap.cuh"
 #include "umma_pipeline.cuh"
+#include "umma_split.cuh"
 
 using namespace umma;
 using esgd::sm_count;
@@ -48,11 +49,14 @@ struct GemmProblem {
       m_idx = rem / n_tiles;
       n_idx = rem % n_tiles;
     }
-    t.m0 = kPair ? (2 * m_idx + (int)(blockIdx.x & 1)) * BM : m_idx * BM;
-    t.n0 = n_idx * BN;
+    place(kPair ? 2 * m_idx + (int)(blockIdx.x & 1) : m_idx, n_idx, t);
     t.kb0 = split * kb_per_split;
     t.kb1 = min(t.kb0 + kb_per_split, kb_total);
     return true;
+  }
+  __device__ __forceinline__ void place(int m_idx, int n_idx, Tile& t) const {
+    t.m0 = m_idx * BM;
+    t.n0 = n_idx * BN;
   }
   using Step = int;            // the k-block's number
   __device__ __forceinline__ Step begin(const Tile& t) const { return t.kb0; }
@@ -120,6 +124,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_kernel(const __grid_const
   run<P, kBn>(prob, ep);
 }
 
+template <class P, int S>
+__global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __grid_constant__ P prob, const Epilogue ep, const SplitOut so) {
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&prob.tmA);
+    tma_prefetch_desc(&prob.tmB);
+  }
+  run_split<P, S>(prob, ep, so);
+}
+
 struct GemmArgs {
   const void *A, *B;
   void* C;
@@ -177,6 +190,16 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   p.kb_per_split = (p.kb_total + splits - 1) / splits;
   p.splits = (p.kb_total + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
   if (p.splits > 1 && g.out_mode != OUT_F32_ADD) return -2;
+  if constexpr (BN == 64 && !A_MN && !kBn && !kPair) {
+    const int tiles = p.m_tiles * p.n_tiles, split = split_ctas((int64_t)p.m_tiles * p.n_tiles, p.kb_total, sm_count());
+    if (split > 1 && g.out_mode == OUT_BF16 && ep.col_sum == nullptr && ep.bias_kind == BIAS_F32 && g.N % 8 == 0) {
+      p.res_kb = p.fixed_n = 0;
+      const SplitOut so{(__nv_bfloat16*)g.C, g.ldc, p.n_tiles, p.kb_total, (p.kb_total + split - 1) / split};
+      if (split == 2) return launch_split<2>(gemm_split_kernel<P, 2>, tiles, stream, p, ep, so);
+      if (split == 4) return launch_split<4>(gemm_split_kernel<P, 4>, tiles, stream, p, ep, so);
+      return launch_split<8>(gemm_split_kernel<P, 8>, tiles, stream, p, ep, so);
+    }
+  }
   ep.res_bytes = PANEL_BYTES;
   const bool two_panels = kBn && ep.residual != nullptr;
   const int sms = kPair ? sm_count() / 2 : sm_count();         // workers: CTAs, or pairs of them

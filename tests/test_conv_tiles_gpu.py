@@ -44,9 +44,11 @@ def test_3x3(n, h, w, cin, cout):
     _close(wt.grad, dw(xd, dd), dw(xd.abs(), dd.abs()))
 
 
-# one tile, several tiles of a CTA with rows left over, columns that fill no panel, pairs
+# one tile, several tiles of a CTA with rows left over, columns that fill no panel, pairs; reductions split over clusters of 8, 4 and 2
+# CTAs, with shares that are empty and columns that fill no tile
 @pytest.mark.parametrize("n,h,cin,cout,k", [(1, 7, 64, 256, 1), (33, 31, 64, 256, 1), (130, 14, 128, 200, 1), (50, 14, 512, 1024, 1), (70, 14, 64, 136, 3),
-                                            (25, 28, 128, 128, 3)])
+                                            (25, 28, 128, 128, 3), (1, 7, 512, 512, 3), (1, 9, 128, 200, 3),
+                                            (1, 14, 1024, 256, 1), (2, 14, 256, 256, 3), (8, 14, 256, 256, 3), (3, 13, 1096, 72, 1), (1, 130, 192, 64, 3)])
 def test_residual(n, h, cin, cout, k):
     from eagersgd_b200.ops import functional as ops
     g = torch.Generator().manual_seed(n + h + k)
@@ -61,7 +63,7 @@ def test_residual(n, h, cin, cout, k):
 
 
 # odd sizes, rows in two boxes, one image and many, channels that fill no block
-@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 7, 9, 64, 256), (5, 15, 31, 72, 40), (2, 5, 300, 64, 128), (130, 8, 8, 256, 512), (1, 1, 1, 8, 8)])
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 7, 9, 64, 256), (5, 15, 31, 72, 40), (2, 5, 300, 64, 128), (130, 8, 8, 256, 512), (1, 1, 1, 8, 8), (1, 13, 15, 1024, 512)])
 def test_strided_1x1_inference(n, h, w, cin, cout):
     from eagersgd_b200.ops import functional as ops
     g = torch.Generator().manual_seed(n + h + w)
