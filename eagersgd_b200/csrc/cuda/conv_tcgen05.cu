@@ -63,7 +63,8 @@ __device__ __forceinline__ void load_filter_tap(const CUtensorMap* tm, const Fil
 template <int BN_, bool kT, bool kPair_>
 struct ConvProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kTwoPanels = false, kPair = kPair_;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = false, kPair = kPair_;
+  static constexpr int kTwoPanels = 0;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, stride, pad;
@@ -156,7 +157,8 @@ template <int BN_, bool kT, bool kPair_>
 struct ConvHaloProblem {
   static constexpr int BN = BN_;
   static_assert(!kPair_ || BN_ == 128, "a CTA's half of a pair's filters is one block of 64 channels");
-  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kTwoPanels = false, kPair = kPair_;
+  static constexpr bool A_MN = false, B_MN = kT, kZeroStages = false, kHalo = true, kPair = kPair_;
+  static constexpr int kTwoPanels = 0;
   CUtensorMap tmX, tmW, tmY, tmR;   // tmR: optional residual, same geometry as the output
   int N, Ho, Wo, Cout;
   int R, S, pad;
@@ -226,7 +228,8 @@ struct ConvHaloProblem {
 template <int BN_>
 struct ConvWgradProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = true, B_MN = true, kZeroStages = true, kTwoPanels = false, kPair = false;
+  static constexpr bool A_MN = true, B_MN = true, kZeroStages = true, kPair = false;
+  static constexpr int kTwoPanels = 0;
   CUtensorMap tmDY, tmX, tmDW;
   int N, Ho, Wo, Cout, Cin;
   int R, S, stride, pad;

@@ -3,13 +3,13 @@
 //   dw[k, r, s, c] = sum over output pixels p of dy[p, k] * x[p + (r, s) - pad, c]
 //
 // The per-tap kernel (conv_tcgen05.cu) loads a dy box and an x box for every (tap, 64-pixel block): the
-// activations cross L2 -> SM once per tap.  Here a CTA owns a SET of taps (as many as fit in tensor memory as
-// separate accumulators) and, for every block of full output rows, loads ONE dy box and ONE x box (the rows plus
+// activations cross L2 -> SM once per tap.  Here a CTA owns a SET of taps (accumulators of their own in tensor memory; how many is
+// wg_plan's choice) and, for every block of full output rows, loads ONE dy box and ONE x box (the rows plus
 // the filter margin); the taps are shifted views of the x box, exactly as in the forward halo mode: both boxes
 // are indexed by the x box's pixel pitch PW = Wo + S - 1, dy's margin columns are zero-filled by TMA, and tap
 // (r, s) reads x (r * PW + s) rows further on.  Both operands are MN-major (the pixel is the K index), the
-// accumulators stay in tensor memory over the CTA's whole pixel range and are added to dw with 16-byte fp32
-// reductions at the end.
+// accumulators stay in tensor memory over the CTA's whole pixel range and are added to dw in fp32 at the end.
+// Layers of 64 channels have a kernel that takes all nine taps at once (conv_wgrad_packed_kernel).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>

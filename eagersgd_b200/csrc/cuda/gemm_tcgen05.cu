@@ -20,10 +20,11 @@ using esgd::sm_count;
 
 namespace {
 
-template <int BN_, bool A_MN_, bool B_MN_, bool kPair_ = false>
+template <int BN_, bool A_MN_, bool B_MN_, bool kPair_ = false, int kTwoPanels_ = 1>
 struct GemmProblem {
   static constexpr int BN = BN_;
-  static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false, kTwoPanels = true, kPair = kPair_;
+  static constexpr bool A_MN = A_MN_, B_MN = B_MN_, kZeroStages = false, kHalo = false, kPair = kPair_;
+  static constexpr int kTwoPanels = kTwoPanels_;
   CUtensorMap tmA, tmB, tmC, tmR;   // tmC: bf16 panels of 64 columns or fp32 ones of 32; tmR: optional residual
   int M, N, K;
   int m_tiles, n_tiles, splits, kb_total, kb_per_split;
@@ -139,9 +140,17 @@ struct GemmArgs {
   int M, N, K, lda, ldb, ldc, out_mode, splits;
 };
 
-template <int BN, bool A_MN, bool B_MN, bool kBn = false, bool kPair = false>
+// Whether B stays in shared memory: its whole K extent fits beside the A stages (max_kb k-blocks of it) and every CTA has several tiles
+// of one column range to amortise the load over.
+template <int BN>
+bool b_resident(const GemmArgs& g, int max_kb, int sms) {
+  const int m_tiles = (g.M + BM - 1) / BM, n_tiles = (g.N + BN - 1) / BN;
+  return resident_enabled() && g.splits <= 1 && (g.K + BK - 1) / BK <= max_kb && n_tiles <= sms / 2 && m_tiles >= 2 * (sms / n_tiles);
+}
+
+template <int BN, bool A_MN, bool B_MN, bool kBn = false, bool kPair = false, bool kResPanels = false>
 int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
-  using P = GemmProblem<BN, A_MN, B_MN, kPair>;
+  using P = GemmProblem<BN, A_MN, B_MN, kPair, kResPanels ? 2 : 1>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -201,14 +210,10 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
     }
   }
   ep.res_bytes = PANEL_BYTES;
-  const bool two_panels = kBn && ep.residual != nullptr;
   const int sms = kPair ? sm_count() / 2 : sm_count();         // workers: CTAs, or pairs of them
   int grid;
-  // B stays in shared memory when its whole K extent fits beside four A stages and every CTA has several
-  // tiles of one column range to amortise the load over
-  const bool resident = !kPair && resident_enabled() && p.splits == 1 &&
-                        p.kb_total <= (two_panels ? Cfg<BN>::MAX_RES_KB2 : Cfg<BN>::MAX_RES_KB) &&
-                        p.n_tiles <= sms / 2 && p.m_tiles >= 2 * (sms / p.n_tiles);
+  const int max_kb = kResPanels ? 2 : kBn && ep.residual != nullptr ? Cfg<BN>::MAX_RES_KB2 : Cfg<BN>::MAX_RES_KB;
+  const bool resident = !kPair && p.splits == 1 && b_resident<BN>(g, max_kb, sms);
   p.res_kb = resident ? p.kb_total : 0;
   p.fixed_n = (ep.col_sum != nullptr || resident) ? 1 : 0;
   if (p.fixed_n) {
@@ -276,6 +281,11 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
     if (!a_mn && b_mn) return launch<256, false, true, false, true>(g, ep, s);
     if (a_mn && b_mn) return launch<256, true, true, false, true>(g, ep, s);
   }
+  // Residual panels in buffers of their own, where resident B leaves room for the whole A of a tile beside them: K of 64 and 128
+  // (392000 x 256 x 64 83.9 -> 81.7 us, 98000 x 512 x 128 48.6 -> 46.9; 24500 x 1024 x 256 would lose A stages, 30.7 -> 32.2).  A kernel
+  // of its own: as a run-time choice it spills registers in the others.
+  if (residual != nullptr && !a_mn && !b_mn && splits <= 1 && b_resident<256>(g, 2, sm_count()))
+    return launch<256, false, false, false, false, true>(g, ep, s);
   return launch_major<256>(a_mn, b_mn, g, ep, s);
 }
 

@@ -233,7 +233,7 @@ __device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
 //   void store_panel(const Tile&, int panel, const void* smem)   TMA store of a 128x64 bf16 panel
 //   static constexpr bool kPair                    the CTA is one of a pair (below): tile() gives it its own 128 rows, load()
 //                                                  takes its half of B's columns and the address of the leader's barrier
-//   static constexpr bool kTwoPanels               residual panels in buffers of their own (kBn kernels)
+//   static constexpr int kTwoPanels                residual panels in buffers of their own: 0 no, 1 in kBn kernels, 2 in all
 //   void load_res_panel(const Tile&, int panel, void* smem, uint64_t* bar)   TMA load of the residual's panel
 //   static constexpr bool kHalo; int out_row(int row)   row of the stored tile for a GEMM row (identity unless kHalo)
 //   kHalo only: int cblks, R, S, PW; void load_halo(const Tile&, int cb, void* smem, uint64_t* bar)
@@ -258,7 +258,7 @@ __device__ __forceinline__ void run(const P& prob, const Epilogue& ep) {
   constexpr bool kHalo = P::kHalo;
   // The residual's panels land in buffers of their own (four stages' worth of shared memory), so that the next one travels
   // while this one is stored and its sums are taken: 340 -> 260 us for 802816 x 256 x 64.
-  const bool two_panels = kBn && P::kTwoPanels && ep.residual != nullptr;
+  const bool two_panels = (P::kTwoPanels == 2 || (kBn && P::kTwoPanels)) && ep.residual != nullptr;
   const int area = two_panels ? C::STAGE_AREA2 : C::STAGE_AREA;
   const int nhalo = kHalo ? (res_kb > 0 ? 2 : MAX_HALOS) : 0;
   constexpr bool kPair = P::kPair;
