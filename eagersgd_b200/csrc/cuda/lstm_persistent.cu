@@ -328,7 +328,10 @@ __global__ void __launch_bounds__(Layout<kBwd, N>::kThreads, 1) lstm_sequence_ke
     const char* const state = reinterpret_cast<const char*>((kBwd ? p.dG : p.y) + kbase) + at;
     uint8_t* const landing = sB + fw * (N * 128) + (lane >> 3) * 128;
     const int swz[2] = {((lane & 7) ^ (lane >> 3)) << 4, ((lane & 7) ^ (4 + (lane >> 3))) << 4};
-    for (int s = 1; ok && s < T; ++s) {
+    // A CTA with fewer blocks than warps: a warp without one stays out.  Nothing makes a step wait for it, so it could fall two
+    // steps behind `pub`, whose parity would then hide them from it.  (A warp with a block is waited for: its block is part of the
+    // product without which nobody publishes the next step.)
+    for (int s = 1; ok && fw < kblocks && s < T; ++s) {
       const char* const from = state + (size_t)(kBwd ? T - s : s - 1) * B * width * 2;
       uint4 v[kWindow][kQuads];
       auto load = [&](uint4 (&x)[kQuads], int kb, bool all) {

@@ -48,6 +48,28 @@ def test_issuers_blocks_and_padding(T, B, H):
     test_persistent_recurrence(T, B, H)
 
 
+@pytest.mark.parametrize("T,B,H", [(700, 8, 128), (700, 32, 128), (501, 16, 256), (400, 24, 512), (300, 8, 896)])
+def test_long_sequences_with_fewer_blocks_than_fetching_warps(T, B, H):
+    """1 to 7 blocks of the state a CTA and eight warps that fetch them, over hundreds of steps: no wait runs out (a warp that has
+    no block must not follow the steps, which do not wait for it), and every pass over the same inputs gives the same states."""
+    from eagersgd_b200.ops.gemm import check_error
+    from eagersgd_b200.ops.lstm import lstm_layer
+    g = torch.Generator().manual_seed(T + B + H)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()
+    x = (rnd(T, B, 64) * 0.5).to(torch.bfloat16).requires_grad_()
+    w_ih, w_hh = (rnd(4 * H, 64) * 0.1).to(torch.bfloat16), (rnd(4 * H, H) / H ** 0.5).to(torch.bfloat16)
+    bias, dy = rnd(4 * H) * 0.1, rnd(T, B, H).to(torch.bfloat16)
+    seen = []
+    for _ in range(5):
+        x.grad = None
+        y = lstm_layer(x, w_ih, w_hh, bias)
+        y.backward(dy)
+        check_error(y.device)
+        seen.append((y.detach().clone(), x.grad))
+    # the order of every sum is fixed, in the recurrence and in the product behind it
+    assert all(torch.equal(a, b) for other in seen[1:] for a, b in zip(seen[0], other))
+
+
 def test_shapes_outside_the_persistent_range_take_the_loop():
     from eagersgd_b200.parallel import _native as N
     lib = N.cuda()
