@@ -656,6 +656,10 @@ __device__ __forceinline__ void load_dy_rows(const Shape& s, const Pass& ps, con
   }
 }
 
+// Both groups of warps have read their rows.  They meet at a barrier with a name: __syncthreads() is for a place that the whole
+// block reaches, and these are two.
+__device__ __forceinline__ void rows_read(int threads) { asm volatile("barrier.sync 1, %0;" ::"r"(threads) : "memory"); }
+
 template <int C>
 struct BwdPlan {
   static constexpr int DGRAD = 8, WGRAD = C == 16 ? 8 : 6;     // warps
@@ -720,7 +724,7 @@ __global__ void __launch_bounds__(BwdPlan<C>::THREADS, 1) bwd_narrow_kernel(cons
         out.finish(a, acc, pix0 + m, pixels - m);
       }
       out.collect(a, part, warp);
-      __syncthreads();
+      rows_read(B::THREADS);
     } else {
       G g;
       g.begin(warp - B::DGRAD);
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(BwdPlan<C>::THREADS, 1) bwd_narrow_kernel(cons
         const uint32_t x0 = smem_addr(sX) + (uint32_t)(ps.window(s, px) * P::PX + g.x_col());
         g.step(d0, x0, row_bytes);
       }
-      __syncthreads();                                         // the banks lie where the rows were
+      rows_read(B::THREADS);                                   // the banks lie where the rows were
       g.collect(reinterpret_cast<float*>(sX));
     }
     __syncthreads();
