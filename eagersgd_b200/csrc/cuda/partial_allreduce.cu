@@ -273,6 +273,18 @@ int esgd_channel_set_grad_acc(void* dch, float* acc, void* stream) {
 }
 
 // ---- post / wait of a stand-alone collective: each one native call --------------------------------------------
+// A kernel goes to the current device's streams alone, and a thread that only waits for a result (or posts) starts on device 0.
+struct OnDevice {
+  int before = -1;
+  explicit OnDevice(int device) {
+    int now = device;
+    if (cudaGetDevice(&now) == cudaSuccess && now != device && cudaSetDevice(device) == cudaSuccess) before = now;
+  }
+  ~OnDevice() { if (before >= 0) cudaSetDevice(before); }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+};
+
 struct esgd_collective {
   cudaEvent_t ready, done;        // the caller's stream has written the tensor; the step has completed
   cudaStream_t side;
@@ -283,6 +295,7 @@ struct esgd_collective {
   void *out, *staged;             // where wait() puts a staged result, and what the kernels wrote; null: nothing to copy
   uint64_t bytes;
   const StepOutcome* outcome;
+  int device;                     // the one that was current when the collective was made
 };
 
 // hold: a poster's stream goes on once the step has completed, so that what it does to the tensor next comes after the step's
@@ -290,10 +303,11 @@ struct esgd_collective {
 int esgd_collective_create(void* dch, uint64_t count, int max_blocks, int local, void* side, int hold, void* out, void* staged,
                            uint64_t bytes, const void* outcome, void** handle) {
   esgd_collective* c = new esgd_collective{nullptr, nullptr, (cudaStream_t)side, dch, count, max_blocks, local, hold, out, staged, bytes,
-                                           (const StepOutcome*)outcome};
-  cudaError_t e = cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming);
+                                           (const StepOutcome*)outcome, 0};
   *handle = c;
+  cudaError_t e = cudaGetDevice(&c->device);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ready, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming);
   return (int)e;
 }
 void esgd_collective_destroy(void* h) {
@@ -306,6 +320,7 @@ void esgd_collective_destroy(void* h) {
 // Launch a step on the side stream behind what `stream` holds so far.
 int esgd_collective_post(void* h, void* stream) {
   esgd_collective* c = (esgd_collective*)h;
+  const OnDevice on(c->device);
   cudaError_t e = cudaEventRecord(c->ready, (cudaStream_t)stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->ready, 0);
   if (e != cudaSuccess) return (int)e;
@@ -334,6 +349,7 @@ static cudaError_t hand_over(const esgd_collective* c, cudaStream_t stream) {
 // where every step applies one (one rank), else when the outcome says that there is one.
 int esgd_collective_wait(void* h, void* stream) {
   esgd_collective* c = (esgd_collective*)h;
+  const OnDevice on(c->device);
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e = cudaStreamWaitEvent(s, c->done, 0);
   const bool copy = c->staged != nullptr;
