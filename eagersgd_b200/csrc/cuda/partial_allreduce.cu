@@ -85,6 +85,9 @@ __global__ void __launch_bounds__(256, 4) local_step_kernel(DevChannel* ch, int 
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
   if (ch->slot_bf16) local_apply<__nv_bfloat16>(ch, grad_src, tid, nth);
   else local_apply<float>(ch, grad_src, tid, nth);
+  __syncthreads();
+  // the end of the data phase is the last block's: the clock only goes forward, so the newest of all steps is this one's
+  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned long long*>(&ch->t_phase[5]), (unsigned long long)DevEnv::now_ns());
 }
 
 // A staged result to where it is expected: 16 bytes a load, four in flight a thread.  It was written a moment ago and is in L2:

@@ -501,7 +501,7 @@ __device__ inline void local_records(DevChannel* ch) {
   ch->plan.is_sync = sync_round ? 1 : 0;
   ch->plan.round = k;
   ch->applied = 1;
-  for (int q = 0; q < 6; ++q) ch->t_phase[q] = q == 4 ? 0 : t;
+  for (int q = 0; q < 5; ++q) ch->t_phase[q] = q == 4 ? 0 : t;      // the data's end is the blocks' to write
 }
 
 // The whole data phase of one rank, run by `nblk` blocks of which this is block `blk`.  `s_flag` is a

@@ -590,3 +590,24 @@ def test_one_rank_hands_out_every_element_once(n, dtype, out_dtype):
     stats = ar.stats()
     assert stats["steps"] == stats["participated"] == stats["activated"] == 4 and stats["forced_sync"] == 1
     ar.close()
+
+
+def test_phase_times_of_one_rank_cover_the_pass():
+    """The data phase lasts as long as the pass over the gradient does: 256 MB read and 256 MB written in each step."""
+    import eagersgd_b200 as es
+    x = torch.ones(64 << 20, device="cuda")
+    ar = es.PartialAllreduce(x, es.init(), mode="solo", limiter=8, out=torch.empty_like(x)).start()
+    try:
+        for _ in range(3):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            ar.post()
+            ar.wait()
+            end.record()
+            torch.cuda.synchronize()
+            t = ar._ch.phase_times_us()
+            # more than at 20 TB/s, no more than the events around the step saw (the clock ticks about once a microsecond)
+            assert 25.0 < t["data"] <= begin.elapsed_time(end) * 1e3 + 5.0, t
+            assert t["pack"] == t["control"] == t["launch_gap"] == 0.0 and t["own_share"] is None
+    finally:
+        ar.close()
