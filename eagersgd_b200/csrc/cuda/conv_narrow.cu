@@ -20,7 +20,6 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <atomic>
 #include "bn_grad.h"
 #include "launch.cuh"
 
@@ -785,18 +784,6 @@ int plan(Shape& s, int& grid, int& smem, int N, int H, int W, int stride, int fi
   return 0;
 }
 
-// More than 48 KB of shared memory has to be asked for, once per kernel and device.
-using Allowed = std::atomic<uint64_t>;
-template <class K>
-void allow_smem(K kernel, Allowed& devices) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const uint64_t bit = 1ull << (dev & 63);
-  if (devices.load(std::memory_order_relaxed) & bit) return;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-  devices.fetch_or(bit, std::memory_order_relaxed);
-}
-
 template <int CR, int CN, bool kT, bool kBnIn = false>
 int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t stream, const BnOutput& b = BnOutput()) {
   using T = Tile<CR, CN>;
@@ -807,8 +794,8 @@ int launch_conv(const Args& a, int N, int H, int W, int stride, cudaStream_t str
                       0);
   if (rc != 0) return rc;
   if (!aligned16(a.x, a.w) || !aligned16(a.y, a.residual) || !aligned16(a.bn_y, b.y) || !aligned16(b.z, nullptr)) return -100;
-  static Allowed allowed{0};
-  allow_smem(conv_narrow_kernel<CR, CN, kT, kBnIn>, allowed);
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(conv_narrow_kernel<CR, CN, kT, kBnIn>, kSmemMax, allowed)) return e;
   return esgd::launch(conv_narrow_kernel<CR, CN, kT, kBnIn>, dim3(grid), kThreads, smem, stream, s, a, b);
 }
 
@@ -823,8 +810,8 @@ int launch_wgrad(const void* x, const void* dy, float* dw, int N, int H, int W, 
   if (rc != 0) return rc;
   if (!aligned16(x, dy)) return -100;
   if (smem < P::BYTES) smem = P::BYTES;
-  static Allowed allowed{0};
-  allow_smem(wgrad_narrow_kernel<CI, CO>, allowed);
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(wgrad_narrow_kernel<CI, CO>, kSmemMax, allowed)) return e;
   return esgd::launch(wgrad_narrow_kernel<CI, CO>, dim3(grid), P::THREADS, smem, stream, s, (const __nv_bfloat16*)x,
                       (const __nv_bfloat16*)dy, dw);
 }
@@ -839,8 +826,8 @@ int launch_bwd(const Args& a, const BnInput& b, float* dw, int N, int H, int W, 
   if (s.per_pass < (s.total + grid - 1) / grid) return -100;       // more rows a block than fit beside one another
   if (!aligned16(a.x, a.w) || !aligned16(a.y, a.residual) || !aligned16(a.bn_y, dw) || !aligned16(b.dz, b.y)) return -100;
   if (smem < B::FIXED + B::G::P::BYTES) smem = B::FIXED + B::G::P::BYTES;
-  static Allowed allowed{0};
-  allow_smem(bwd_narrow_kernel<C>, allowed);
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(bwd_narrow_kernel<C>, kSmemMax, allowed)) return e;
   return esgd::launch(bwd_narrow_kernel<C>, dim3(grid), B::THREADS, smem, stream, s, a, b, dw);
 }
 

@@ -343,13 +343,8 @@ inline int mma_columns(int n, int bn) { return n >= bn ? bn : (n + 15) / 16 * 16
 template <int BN, bool kT, bool kBn, bool kPair = false>
 int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream, int split = 1) {
   using P = ConvProblem<BN, kT, kPair>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg<BN>::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(conv_kernel<P, kBn>, Cfg<BN>::SMEM_BYTES, allowed)) return e;
   P p;
   p.N = a.N; p.Cout = a.Cout; p.R = a.R; p.S = a.S; p.stride = a.stride; p.pad = a.pad;
   p.Ho = a.out_h ? a.out_h : (a.H + 2 * a.pad - a.R) / a.stride + 1;
@@ -454,13 +449,8 @@ bool halo_pairs(const ConvArgs& a, int BN) { return BN == 128 && a.Cin % 64 == 0
 template <int BN, bool kT, bool kBn, bool kPair = false>
 int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
   using P = ConvHaloProblem<BN, kT, kPair>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg<BN>::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(conv_kernel<P, kBn>, Cfg<BN>::SMEM_BYTES, allowed)) return e;
   P p;
   p.N = a.N; p.Cout = a.Cout; p.R = a.R; p.S = a.S; p.pad = a.pad;
   p.Ho = a.H + 2 * a.pad - a.R + 1;
@@ -509,13 +499,8 @@ int launch_halo(const ConvArgs& a, Epilogue ep, int bh, cudaStream_t stream) {
 template <int BN>
 int launch_wgrad(const ConvArgs& a, const void* dy, float* dw, int* error_flag, cudaStream_t stream) {
   using P = ConvWgradProblem<BN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg<BN>::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(conv_wgrad_kernel<P>, Cfg<BN>::SMEM_BYTES, allowed)) return e;
   P p;
   p.N = a.N; p.Cout = a.Cout; p.Cin = a.Cin; p.R = a.R; p.S = a.S; p.stride = a.stride; p.pad = a.pad;
   p.Ho = (a.H + 2 * a.pad - a.R) / a.stride + 1;

@@ -443,12 +443,8 @@ int wg_pick_bh(int H, int W, int Cin, int Cout, int R, int S, int pad) {
 template <int BN>
 int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, int W, int Cin, int Cout, int R, int S,
                       int pad, int bh, int* error_flag, cudaStream_t stream) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_halo_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(conv_wgrad_halo_kernel<BN>, WG_SMEM, allowed)) return e;
   WgHaloParams p;
   double cost = 0.0, packed_cost = 0.0;
   const int pr = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, esgd::sm_count(), &cost);
@@ -473,12 +469,8 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
     if (r != 0) return 2000 + r;
   }
   if (use_packed) {
-    static bool packed_set = false;
-    if (!packed_set) {
-      cudaError_t e = cudaFuncSetAttribute(conv_wgrad_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
-      if (e != cudaSuccess) return (int)e;
-      packed_set = true;
-    }
+    static esgd::SmemAllowed packed_allowed{0};
+    if (const int e = esgd::allow_smem(conv_wgrad_packed_kernel, WG_SMEM, packed_allowed)) return e;
     return esgd::launch(conv_wgrad_packed_kernel, dim3(p.splits), WG_THREADS, WG_SMEM, stream, p);
   }
   const int grid = p.sets * p.m_tiles * p.n_tiles * p.splits;

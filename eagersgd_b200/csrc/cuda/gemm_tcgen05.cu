@@ -151,13 +151,8 @@ bool b_resident(const GemmArgs& g, int max_kb, int sms) {
 template <int BN, bool A_MN, bool B_MN, bool kBn = false, bool kPair = false, bool kResPanels = false>
 int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
   using P = GemmProblem<BN, A_MN, B_MN, kPair, kResPanels ? 2 : 1>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<P, kBn>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg<BN>::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static esgd::SmemAllowed allowed{0};
+  if (const int e = esgd::allow_smem(gemm_kernel<P, kBn>, Cfg<BN>::SMEM_BYTES, allowed)) return e;
   P p;
   uint64_t dims[2], strides[1];
   uint32_t box[2];

@@ -6,6 +6,8 @@
 // this way calls pdl_enter() before it touches memory, so completion stays transitive along the stream.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
+#include <atomic>
 #include "launch_count.cuh"
 
 namespace esgd {
@@ -23,6 +25,20 @@ inline int sm_count() {
     return n > 0 ? n : 148;
   }();
   return count;
+}
+
+// More than 48 KB of dynamic shared memory have to be asked for, once for each kernel and device of the process.
+using SmemAllowed = std::atomic<uint64_t>;      // one for each kernel; bit d: asked for on device d
+template <class K>
+inline int allow_smem(K kernel, int bytes, SmemAllowed& devices) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
+  if (devices.load(std::memory_order_relaxed) & bit) return 0;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_relaxed);
+  return (int)e;
 }
 
 // kCluster: CTAs of a cluster (along x).

@@ -539,14 +539,6 @@ int map_of(CUtensorMap* tm, const void* t, const StemShape& s) {
   return esgd::make_tensormap_bf16(tm, t, 4, dims, strides, box, nullptr);
 }
 
-template <class K>
-int allow_smem(K kernel, bool& done) {
-  if (done) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
-  done = e == cudaSuccess;
-  return (int)e;
-}
-
 }  // namespace
 
 extern "C" {
@@ -566,8 +558,8 @@ int esgd_stem_fwd(const void* x, const void* w2d, void* y, void* keep, int N, in
   p.x = (const __nv_bfloat16*)x;
   p.keep = (__nv_bfloat16*)keep;
   p.scale = scale; p.shift = shift; p.relu = relu; p.sum = sum; p.sqsum = sqsum; p.error_flag = error_flag;
-  static bool allowed = false;
-  if ((rc = allow_smem(stem_fwd_kernel, allowed)) != 0) return rc;
+  static esgd::SmemAllowed allowed{0};
+  if ((rc = esgd::allow_smem(stem_fwd_kernel, kSmemLimit, allowed)) != 0) return rc;
   const int sms = esgd::sm_count();
   return esgd::launch(stem_fwd_kernel, dim3(p.s.bands < sms ? p.s.bands : sms), kFwdThreads, fwd_smem(p.s), stream, p);
 }
@@ -581,8 +573,8 @@ int esgd_stem_wgrad(const void* x, const void* dy, float* col, int N, int H, int
   if ((rc = map_of(&p.tmDY, dy, p.s)) != 0) return 1000 + rc;
   p.x = (const __nv_bfloat16*)x;
   p.col = col; p.kpad = kpad; p.error_flag = error_flag;
-  static bool allowed = false;
-  if ((rc = allow_smem(stem_wgrad_kernel, allowed)) != 0) return rc;
+  static esgd::SmemAllowed allowed{0};
+  if ((rc = esgd::allow_smem(stem_wgrad_kernel, kSmemLimit, allowed)) != 0) return rc;
   const int sms = esgd::sm_count();
   return esgd::launch(stem_wgrad_kernel, dim3(p.s.bands < sms ? p.s.bands : sms), kWgThreads, wgrad_smem(p.s), stream, p);
 }

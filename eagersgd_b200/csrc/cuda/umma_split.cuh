@@ -213,12 +213,8 @@ __device__ __forceinline__ void run_split(const P& prob, const Epilogue& ep, con
 
 template <int S, class K, class P>
 int launch_split(K kernel, int tiles, cudaStream_t stream, const P& p, const Epilogue& ep, const SplitOut& so) {
-  static bool attr_set = false;              // one for each kernel: its type is the instance's
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static esgd::SmemAllowed allowed{0};       // one for each kernel: its type is the instance's
+  if (const int e = esgd::allow_smem(kernel, SPLIT_SMEM, allowed)) return e;
   return esgd::launch<S>(kernel, dim3(tiles * S), SPLIT_THREADS, SPLIT_SMEM, stream, p, ep, so);
 }
 
