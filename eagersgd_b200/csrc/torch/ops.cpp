@@ -1204,9 +1204,10 @@ struct BnActFn : public Function<BnActFn> {
       rec->y = rec->mask = rec->dz = rec->sums = Tensor();
     }
     variable_list out(16);
-    if (const auto it = ctx->saved_data.find("link"); fused && it != ctx->saved_data.end()) {
+    if (const auto it = ctx->saved_data.find("link"); it != ctx->saved_data.end()) {
       const Link link = c10::static_intrusive_pointer_cast<LayerLink>(it->second.toCapsule());
-      if (!link->observed()) {             // the convolution's backward, which comes next, does it on the way
+      link->release();                     // of an earlier pass that broke off before the convolution's backward
+      if (fused && !link->observed()) {    // the convolution's backward, which comes next, does it on the way
         link->dz = dz;
         link->version = dz._version();
         link->y = y;

@@ -141,6 +141,34 @@ def test_somebody_is_looking(c, who):
     _compare(one, ref)
 
 
+@pytest.mark.parametrize("c", [16, 32])
+def test_backward_pass_after_one_that_broke_off(c):
+    """An error between a batch norm's backward and its convolution's (here the convolution's input has changed) leaves nothing
+    behind that a second pass over the kept graph would trip over."""
+    from eagersgd_b200 import _build
+    blocks, (x, dy) = _blocks(c, 1), _data(c, 4, 12, 10)
+    params = [p for p in blocks.parameters()]
+    sinks = _build.load_torch().GradSinks([len(params)], lambda bucket: None)
+    for p in params:
+        sinks.add(p, torch.zeros_like(p, dtype=torch.float32, memory_format=torch.preserve_format), 0)
+    sinks.begin_step()
+    sinks.set_active(True)
+    xi = x.clone().requires_grad_()
+    y = blocks[0](xi)
+    version = xi._version
+    with torch.no_grad():
+        xi.add_(0)
+    with pytest.raises(RuntimeError, match="inplace"):
+        y.backward(dy, retain_graph=True)
+    torch._C._autograd._unsafe_set_version_counter((xi,), (version,))
+    assert xi.grad is None
+    y.backward(dy)
+    sinks.set_active(False)
+    sinks.close()
+    ref, _ = _run(blocks, x, dy, True)
+    _compare([xi.grad.float()], [ref[1]])
+
+
 # ---------------------------------------------------------------------------------------------------- the kernels
 class _BnGrad(C.Structure):
     _fields_ = [("y", C.c_void_p), ("mask", C.c_void_p), ("aux", C.c_void_p), ("sums", C.c_void_p)]
