@@ -339,6 +339,25 @@ inline int ksteps_of(int c) { return c >= 64 ? BK / 16 : (c + 15) / 16; }
 // narrow layers: the MMA computes no more columns than there are (the epilogue drops the rest either way)
 inline int mma_columns(int n, int bn) { return n >= bn ? bn : (n + 15) / 16 * 16; }
 
+// Boxes of output pixels: whole rows when they fit, as many rows / images as 128 GEMM rows allow.
+struct PixelBoxes { int BW, BH, BI, w_tiles, h_tiles, i_tiles; };
+inline PixelBoxes pixel_boxes(int N, int Ho, int Wo) {
+  PixelBoxes b = {128, 1, 1, 0, 0, 0};
+  if (Wo < 128) {
+    b.BW = Wo;
+    for (int d = 1; d <= 128 / b.BW && d <= Ho; ++d) if (Ho % d == 0) b.BH = d;       // largest divisor of Ho that fits
+    if (b.BH == Ho) {
+      b.BI = 128 / (b.BW * b.BH);
+      if (b.BI > N) b.BI = N;
+      if (b.BI < 1) b.BI = 1;
+    }
+  }
+  b.w_tiles = (Wo + b.BW - 1) / b.BW;
+  b.h_tiles = (Ho + b.BH - 1) / b.BH;
+  b.i_tiles = (N + b.BI - 1) / b.BI;
+  return b;
+}
+
 // split: CTAs that share the reduction of a tile (64 columns), 1 for the pipeline.
 template <int BN, bool kT, bool kBn, bool kPair = false>
 int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream, int split = 1) {
@@ -353,19 +372,8 @@ int launch(const ConvArgs& a, Epilogue ep, cudaStream_t stream, int split = 1) {
   p.ksteps = ksteps_of(a.Cin);
   p.n_mma = mma_columns(a.Cout, BN);
   p.taps = a.taps;
-  // output-pixel box: whole rows when they fit, as many rows / images as 128 GEMM rows allow
-  if (p.Wo >= 128) { p.BW = 128; p.BH = 1; p.BI = 1; }
-  else {
-    p.BW = p.Wo;
-    int max_h = 128 / p.BW;
-    p.BH = 1;
-    for (int d = 1; d <= max_h && d <= p.Ho; ++d) if (p.Ho % d == 0) p.BH = d;   // largest divisor of Ho that fits
-    p.BI = 1;
-    if (p.BH == p.Ho) { p.BI = 128 / (p.BW * p.BH); if (p.BI > a.N) p.BI = a.N; if (p.BI < 1) p.BI = 1; }
-  }
-  p.w_tiles = (p.Wo + p.BW - 1) / p.BW;
-  p.h_tiles = (p.Ho + p.BH - 1) / p.BH;
-  p.i_tiles = (a.N + p.BI - 1) / p.BI;
+  const PixelBoxes b = pixel_boxes(a.N, p.Ho, p.Wo);
+  p.BW = b.BW; p.BH = b.BH; p.BI = b.BI; p.w_tiles = b.w_tiles; p.h_tiles = b.h_tiles; p.i_tiles = b.i_tiles;
   p.n_tiles = (a.Cout + BN - 1) / BN;
   {
     // input: dims (C, W, H, N); box in INPUT elements = output box * stride (element strides pick every stride-th)
@@ -577,13 +585,8 @@ int tile_width(const ConvArgs& a, int Ho, int Wo) {
 
 // Tiles of 64 columns that launch() will make of the output.
 int64_t conv_tiles(const ConvArgs& a, int Ho, int Wo) {
-  const int bw = Wo < 128 ? Wo : 128;
-  int bh = 1, bi = 1;
-  if (Wo < 128) {
-    for (int d = 1; d <= 128 / bw && d <= Ho; ++d) if (Ho % d == 0) bh = d;
-    if (bh == Ho) bi = 128 / (bw * bh) < 1 ? 1 : 128 / (bw * bh) > a.N ? a.N : 128 / (bw * bh);
-  }
-  return (int64_t)((Wo + bw - 1) / bw) * ((Ho + bh - 1) / bh) * ((a.N + bi - 1) / bi) * ((a.Cout + 63) / 64);
+  const PixelBoxes b = pixel_boxes(a.N, Ho, Wo);
+  return (int64_t)b.w_tiles * b.h_tiles * b.i_tiles * ((a.Cout + 63) / 64);
 }
 
 template <bool kT, bool kBn = false>
@@ -676,10 +679,10 @@ int esgd_conv2d_dgrad(const void* dy, const void* w, void* dx, int N, int H, int
 }
 
 // Host arithmetic of the halo-mode forward / data-gradient launch, without launching (no device needed).
-// out[0..9]: applicable (0/1), BH, PW, BN, resident filter k-blocks (0: streamed), input-box slots, filter stages,
-// bytes of one input box, bytes the most shifted view reaches, stage area used.
+// out[0..10]: applicable (0/1), BH, PW, BN, resident filter k-blocks (0: streamed), input-box slots, filter stages,
+// bytes of one input box, bytes the most shifted view reaches, stage area used, stage area there is.
 void esgd_conv2d_halo_plan(int N, int H, int W, int Cin, int Cout, int R, int S, int stride, int pad, int* out) {
-  for (int i = 0; i < 10; ++i) out[i] = 0;
+  for (int i = 0; i < 11; ++i) out[i] = 0;
   if (Cin % 8 || Cout % 8) return;
   ConvArgs a{nullptr, nullptr, nullptr, N, H, W, Cin, Cout, R, S, stride, pad};
   const int BN = stride == 1 ? tile_width(a, H + 2 * pad - R + 1, W + 2 * pad - S + 1) : 0;
@@ -700,6 +703,7 @@ void esgd_conv2d_halo_plan(int N, int H, int W, int Cin, int Cout, int R, int S,
   out[7] = PW * (bh + R - 1) * 128;
   out[8] = ((R - 1) * PW + (S - 1) + BM) * 128;
   out[9] = nhalo * HALO_BYTES + (res_kb > 0 ? res_kb : nstages) * b_stage;
+  out[10] = stage_area;
 }
 
 }  // extern "C"

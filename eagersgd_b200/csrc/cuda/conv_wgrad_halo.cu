@@ -36,13 +36,16 @@ struct WgHaloParams {
   int* error_flag;
 };
 
+// Sums of a tap on their way out: 128 rows of an odd number of 16 bytes (no bank conflicts).
+__host__ __device__ constexpr int wg_bank_bytes(int BN) { return 128 * (BN * 4 + 16); }
+
 template <int BN>
 __global__ void __launch_bounds__(WG_THREADS, 1) conv_wgrad_halo_kernel(const __grid_constant__ WgHaloParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int NA = 2, NB = BN / 64;                  // 64-channel atoms of the dy (128 rows) and x operands
   const int stage_bytes = NA * p.abox + NB * p.xbox;
-  constexpr int kPitch = BN * 4 + 16, kBank = 128 * kPitch;         // sums on their way out: an odd number of 16 bytes a row
+  constexpr int kBank = wg_bank_bytes(BN), kPitch = kBank / 128;     // sums on their way out
   uint8_t* bar_area = smem + max(p.nstages * stage_bytes, kBank);
   uint64_t* full = reinterpret_cast<uint64_t*>(bar_area);
   uint64_t* empty = full + 4;
@@ -423,6 +426,20 @@ bool wg_packed_plan(WgHaloParams& p, int Cin, int Cout, int R, int S, int sms, d
   return true;
 }
 
+// What a launch will be; -7 as wg_plan.  aligned16: dw is a multiple of 16 bytes (the packed kernel's bulk reductions need it).
+int wg_choose(WgHaloParams& p, bool& packed, int BN, int N, int H, int W, int Cin, int Cout, int R, int S, int pad, int bh, int sms, bool aligned16) {
+  double cost = 0.0, packed_cost = 0.0;
+  const int rc = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, sms, &cost);
+  packed = false;
+  if (rc != 0 || BN != 64 || !aligned16) return rc;
+  WgHaloParams q = p;
+  if (wg_packed_plan(q, Cin, Cout, R, S, sms, &packed_cost) && packed_cost < cost) {
+    p = q;
+    packed = true;
+  }
+  return 0;
+}
+
 // Input channels of a tile.  128 leave room for the sums of four taps, 256 for two.  128 and 256: 8 x 14 x 14 x 256 6.7 and 8.7 us, 64
 // images 18.0 and 19.3, 256 images 45.5 and 53.6; but 64 x 7 x 7 x 512, whose boxes are small, 24.5 and 20.0, 256 images 68 and 53.
 int columns(int Cin) { return Cin <= 64 ? 64 : (Cin <= 256 ? 128 : 256); }
@@ -446,12 +463,9 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
   static esgd::SmemAllowed allowed{0};
   if (const int e = esgd::allow_smem(conv_wgrad_halo_kernel<BN>, WG_SMEM, allowed)) return e;
   WgHaloParams p;
-  double cost = 0.0, packed_cost = 0.0;
-  const int pr = wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, esgd::sm_count(), &cost);
+  bool packed = false;
+  const int pr = wg_choose(p, packed, BN, N, H, W, Cin, Cout, R, S, pad, bh, esgd::sm_count(), ((uintptr_t)dw & 15) == 0);
   if (pr != 0) return pr;
-  WgHaloParams packed = p;
-  const bool use_packed = BN == 64 && ((uintptr_t)dw & 15) == 0 && wg_packed_plan(packed, Cin, Cout, R, S, esgd::sm_count(), &packed_cost) && packed_cost < cost;
-  if (use_packed) p = packed;
   p.dw = dw;
   p.error_flag = error_flag;
   {
@@ -468,7 +482,7 @@ int launch_wgrad_halo(const void* x, const void* dy, float* dw, int N, int H, in
     int r = esgd::make_tensormap_bf16(&p.tmX, x, 4, dims, strides, box, nullptr);
     if (r != 0) return 2000 + r;
   }
-  if (use_packed) {
+  if (packed) {
     static esgd::SmemAllowed packed_allowed{0};
     if (const int e = esgd::allow_smem(conv_wgrad_packed_kernel, WG_SMEM, packed_allowed)) return e;
     return esgd::launch(conv_wgrad_packed_kernel, dim3(p.splits), WG_THREADS, WG_SMEM, stream, p);
@@ -501,18 +515,24 @@ int esgd_conv2d_wgrad_halo(const void* x, const void* dy, float* dw, int N, int 
 
 // Host arithmetic of a launch without launching anything (no device needed).  out[0..11]: applicable (0/1), BH, PW,
 // ksteps, abox, xbox, nstages, sets, taps_per_set, splits, boxes_per_split, grid; out[12] = BN, out[13] = shared
-// memory requested, out[14] = m_tiles, out[15] = n_tiles.
+// memory requested, out[14] = m_tiles, out[15] = n_tiles; out[16]: 1 for the packed kernel (all nine taps, sets, m_tiles and n_tiles
+// of 1), out[17]: bytes that the sums of a CTA take on their way out, where the stages were.
 void esgd_conv2d_wgrad_halo_plan(int N, int H, int W, int Cin, int Cout, int R, int S, int pad, int sms, int* out) {
-  for (int i = 0; i < 16; ++i) out[i] = 0;
+  for (int i = 0; i < 18; ++i) out[i] = 0;
   const int bh = wg_pick_bh(H, W, Cin, Cout, R, S, pad);
   if (bh == 0) return;
   const int BN = columns(Cin);
   WgHaloParams p;
-  if (wg_plan(p, BN, N, H, W, Cin, Cout, R, S, pad, bh, sms) != 0) return;
+  bool packed = false;
+  if (wg_choose(p, packed, BN, N, H, W, Cin, Cout, R, S, pad, bh, sms, true) != 0) return;
+  if (packed) {
+    p.sets = p.m_tiles = p.n_tiles = 1;
+    p.taps_per_set = 9;
+  }
   out[0] = 1; out[1] = p.BH; out[2] = p.PW; out[3] = p.ksteps; out[4] = p.abox; out[5] = p.xbox; out[6] = p.nstages;
   out[7] = p.sets; out[8] = p.taps_per_set; out[9] = p.splits; out[10] = p.boxes_per_split;
   out[11] = p.sets * p.m_tiles * p.n_tiles * p.splits; out[12] = BN; out[13] = WG_SMEM; out[14] = p.m_tiles;
-  out[15] = p.n_tiles;
+  out[15] = p.n_tiles; out[16] = packed; out[17] = packed ? kPackedBank : wg_bank_bytes(BN);
 }
 
 }  // extern "C"

@@ -225,9 +225,7 @@ int launch(const GemmArgs& g, Epilogue ep, cudaStream_t stream) {
 
 // Pairs of CTAs: 256 x 256 tiles that read each operand once for both (32 KB a k-block and CTA instead of 48, five stages
 // deep instead of three).
-bool pair_applicable(int M, int N, int K, int splits) {
-  return M > BM && N > BM && K > 4 * BK && (N + 255) / 256 <= sm_count() / 2;
-}
+bool pair_applicable(int64_t M, int64_t N, int64_t K, int sms) { return M > BM && N > BM && K > 4 * BK && (N + 255) / 256 <= sms / 2; }
 
 template <int BN>
 int launch_major(int a_mn, int b_mn, const GemmArgs& g, const Epilogue& ep, cudaStream_t s) {
@@ -271,7 +269,7 @@ int esgd_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, i
   const int BN = tile_columns(N, (M + BM - 1) / BM * (splits > 1 ? splits : 1), sm_count());
   if (BN == 64) return launch_major<64>(a_mn, b_mn, g, ep, s);
   if (BN == 128) return launch_major<128>(a_mn, b_mn, g, ep, s);
-  if (pair_applicable(M, N, K, splits)) {
+  if (pair_applicable(M, N, K, sm_count())) {
     if (!a_mn && !b_mn) return launch<256, false, false, false, true>(g, ep, s);
     if (!a_mn && b_mn) return launch<256, false, true, false, true>(g, ep, s);
     if (a_mn && b_mn) return launch<256, true, true, false, true>(g, ep, s);
@@ -296,7 +294,7 @@ int esgd_gemm_wgrad_splits(int64_t pixels, int64_t cout, int64_t cin, int sms) {
     const int64_t per = (blocks + s - 1) / s, splits = (blocks + per - 1) / per;
     if (splits != s) continue;                                  // the same launch as a smaller number
     const int bn = tile_columns((int)cin, (int)((cout + BM - 1) / BM * s), sms);
-    const bool pair = bn == 256 && cout > BM && cin > BM && pixels > 4 * BK && (cin + 255) / 256 <= sms / 2;
+    const bool pair = bn == 256 && pair_applicable(cout, cin, pixels, sms);
     const int64_t rows = pair ? 2 * BM : BM, workers = pair ? sms / 2 : sms;
     const int64_t rounds = ((cout + rows - 1) / rows * ((cin + bn - 1) / bn) * s + workers - 1) / workers;
     const int64_t cost = rounds * (per * (pair ? 450 : bn == 64 ? 250 : bn == 128 ? 300 : 600) + 1000) + s * bank / 1600;
