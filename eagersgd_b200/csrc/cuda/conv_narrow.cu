@@ -55,7 +55,8 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   return raw;
 }
 
-// Division by a number known at launch: multiply, add, shift (exact for dividends below 2^31).
+// Division by a number known at launch, after Granlund and Montgomery (Division by Invariant Integers using Multiplication, 1994):
+// multiply, add, shift; exact for dividends below 2^31.
 struct FastDiv {
   uint32_t mul, shift, d;
   FastDiv() = default;

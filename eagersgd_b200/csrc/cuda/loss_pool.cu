@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(256) avgpool_bwd_kernel(const __nv_bfloat16* _
 }
 
 // im2col for convolutions with very few input channels (the 7x7 / 2 stem on RGB images): the sizes that stem_tcgen05.cu
-// does not take, other filters, other widths).
+// does not take (other filters, other widths).
 // Column layout per output pixel: R segments of SEG = roundup8(S*C) elements; segment r holds the
 // S*C input values of filter row r — in NHWC they are contiguous in memory — followed by zeros, and the
 // row is zero-padded to Kpad (a multiple of 64, so the product runs as a tensor-core GEMM).

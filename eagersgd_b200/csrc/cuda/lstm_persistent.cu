@@ -6,9 +6,10 @@
 // chip for the whole sequence and a step is: fetch the previous step's state as it appears (32 KB), 64 MMAs, exchange
 // partial sums inside the cluster, apply the cell to 16 units, publish.
 //
-//   weights   the A operand of tcgen05.mma, 64 columns of K at a time: the last 14 such blocks (224 KB) in tensor memory, the
-//             others in shared memory, as the room left by the state and the partial sums allows.  128 x 16 x 16 takes 12
-//             cycles with A in tensor memory and 41 with A in shared memory, so the latter go first, while the state arrives
+//   weights   the A operand of tcgen05.mma, 64 columns of K at a time: the last 14 such blocks (224 KB; 12 forward with a
+//             batch of 32, whose four accumulators are wider) in tensor memory, the others in shared memory, as the room left
+//             by the state and the partial sums allows.  128 x 16 x 16 takes 12 cycles with A in tensor memory and 41 with A in
+//             shared memory, so the latter go first, while the state arrives
 //   forward   128 rows = 4 gates x 32 units, K = half of the hidden state: clusters of 2, H/16 CTAs
 //   backward  128 rows = 128 units of dh (weights transposed), K = 4H split over clusters of up to 8 CTAs: the largest
 //             cluster size whose whole grid is resident (of 16 clusters, a B200's GPCs hold 15 of size 8 or 7 but all of size 6)
@@ -132,11 +133,6 @@ __device__ __forceinline__ uint32_t clock32() {
 __device__ __forceinline__ uint4 ld_state(const void* p) {
   uint4 v;
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint4 ld_shared(const void* p) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)) : "memory");
   return v;
 }
 __device__ __forceinline__ uint32_t newest(uint4 v) { return max(max(v.x, v.y), max(v.z, v.w)); }    // kUnset: one is not there

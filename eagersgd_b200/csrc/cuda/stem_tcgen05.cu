@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) stem_fwd_kernel(const __grid_c
   extern __shared__ __align__(1024) uint8_t smem[];
   const StemShape& s = p.s;
   uint8_t* sB = smem;                                         // three blocks of 64 filters x 64 elements
-  uint8_t* sC = sB + 3 * 8192;                                // the two epilogue groups' panels
+  uint8_t* sC = sB + 3 * 8192;                                // the epilogue groups' panels
   float* sAff = reinterpret_cast<float*>(sC + kGroups * kPanel);    // factors, summands
   float* sSum = sAff + 128;                                   // [2][64]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sSum + 128);

@@ -505,8 +505,6 @@ struct PendingNorm {
   }
 };
 
-// What a convolution's epilogue does to the product: statistics of it (training), or the affine map of an inference batch
-// norm, a residual and a ReLU.
 // The windows of NHWC x as a matrix, one row per output pixel.
 Tensor stem_columns(const Tensor& x, int64_t r, int64_t s, int64_t stride, int64_t pad) {
   const int64_t n = x.size(0), c = x.size(1), h = x.size(2), w = x.size(3);
@@ -516,6 +514,8 @@ Tensor stem_columns(const Tensor& x, int64_t r, int64_t s, int64_t stride, int64
   return col;
 }
 
+// What a convolution's epilogue does to the product: statistics of it (training), or the affine map of an inference batch
+// norm, a residual and a ReLU.
 struct ConvEpilogue {
   float *sum = nullptr, *sqsum = nullptr;
   const float *scale = nullptr, *shift = nullptr;
@@ -724,15 +724,11 @@ struct ConvFn : public Function<ConvFn> {
       } else {
         const StemGeometry g(cin, r, s);
         Tensor col = zeros_f32({cout, g.kpad}, x.device());
-        int rc = kNotTaken;
-        if (x.dim() == 4)                       // the forward pass left the images, not their columns
-          rc = esgd_stem_wgrad(x.data_ptr(), dy.data_ptr(), fptr(col), n, h, wd, cin, cout, r, s, stride, pad, g.kpad, flag_ptr(x), st);
-        if (rc == kNotTaken) {
-          const Tensor rows = x.dim() == 4 ? stem_columns(x, r, s, stride, pad) : x;
-          rc = gemm(dy.data_ptr(), rows.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, esgd_sm_count(), nullptr,
-                    nullptr, nullptr, 0, x);
-        }
-        ck(rc, "stem weight gradient");
+        // the forward pass left the images where its kernel took them, else their columns
+        ck(x.dim() == 4 ? esgd_stem_wgrad(x.data_ptr(), dy.data_ptr(), fptr(col), n, h, wd, cin, cout, r, s, stride, pad, g.kpad, flag_ptr(x), st)
+                        : gemm(dy.data_ptr(), x.data_ptr(), fptr(col), cout, g.kpad, m, cout, g.kpad, g.kpad, true, true, 2, esgd_sm_count(),
+                               nullptr, nullptr, nullptr, 0, x),
+           "stem weight gradient");
         if (!sink) dw = at::empty(w.sizes(), w.options(), kCL);
         ck(esgd_stem_unpack(fptr(col), sink ? nullptr : dw.data_ptr(), sink ? sink->acc : nullptr, cout, r, s * cin, g.seg, g.kpad,
                             st), "stem filter gradient");
