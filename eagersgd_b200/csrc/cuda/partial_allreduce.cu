@@ -22,7 +22,7 @@
 #include <utility>
 #include <vector>
 #include "partial_allreduce.cuh"
-#include "launch_count.cuh"
+#include "launch.cuh"
 
 namespace esgd { std::atomic<uint64_t> g_launches{0}; }
 
@@ -343,8 +343,8 @@ int esgd_collective_test(void* h) {
 static cudaError_t hand_over(const esgd_collective* c, cudaStream_t stream) {
   if ((((uintptr_t)c->out | (uintptr_t)c->staged) & 15) || c->bytes == 0)
     return cudaMemcpyAsync(c->out, c->staged, c->bytes, cudaMemcpyDeviceToDevice, stream);
-  const uint64_t need = (c->bytes / 16 + 4 * 256 - 1) / (4 * 256) + 1;
-  hand_over_kernel<<<(int)(need < 148 * 8 ? need : 148 * 8), 256, 0, stream>>>((const uint8_t*)c->staged, (uint8_t*)c->out, c->bytes);
+  const uint64_t need = (c->bytes / 16 + 4 * 256 - 1) / (4 * 256) + 1, most = (uint64_t)esgd::sm_count() * 8;     // 8 blocks of 256 fill an SM
+  hand_over_kernel<<<(int)(need < most ? need : most), 256, 0, stream>>>((const uint8_t*)c->staged, (uint8_t*)c->out, c->bytes);
   count_launch();
   return cudaGetLastError();
 }
