@@ -29,10 +29,11 @@ constexpr int SPLIT_SMEM = SPLIT_STAGES * SPLIT_STAGE_BYTES + 256;
 // pipeline 10.1, clusters of four 6.6).  With eight blocks sharing them costs more than it gives (7 x 7, 512 to 2048 channels: 5.2 us,
 // the pipeline 4.8), with 16 it begins to pay (1x1, 1024 to 2048 channels: 5.7 and 6.5; 1024 to 256: clusters of eight
 // 6.0, of four 5.4, the pipeline 5.9).
+constexpr int kOutside8 = 28, kOutside4 = 16;         // of a B200's 148 SMs, the ones that no cluster of eight, of four takes
 inline int split_ctas(int64_t tiles, int blocks, int sms) {
   if (blocks < 16) return 1;
-  if (tiles * 8 <= sms - 28 && blocks > 16) return 8;
-  if (tiles * 4 <= sms - 16) return 4;
+  if (tiles * 8 <= sms - kOutside8 && blocks > 16) return 8;
+  if (tiles * 4 <= sms - kOutside4) return 4;
   return tiles * 2 <= sms ? 2 : 1;
 }
 
