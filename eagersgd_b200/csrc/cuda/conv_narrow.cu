@@ -836,12 +836,19 @@ int launch_bwd(const Args& a, const BnInput& b, float* dw, int N, int H, int W, 
 
 extern "C" {
 
-// 64 input channels fill a k-block of the tile kernels, and only small problems are better off here.  Microseconds back to back,
-// rows in shared memory / tiles, forward with sums, inference epilogue with a shortcut, data gradient with batch norm: 8 x 8
-// pixels, one image 4.1 / 6.4, 3.6 / 8.6, 4.4 / 7.5; 64 images 5.4 / 6.5, 5.0 / 8.6, 6.2 / 7.6; 128 images (8192 pixels) 6.7 /
-// 6.7, 6.5 / 8.9, 7.6 / 8.1; 512 images 12.4 / 11.9, 12.8 / 13.4, 13.6 / 13.4; 56 x 56, one image 5.7 / 6.5, 5.5 / 8.7, 6.2 /
-// 7.6; two 6.9 / 6.6, 6.6 / 8.8, 7.4 / 7.8; four 8.5 / 6.9, 8.4 / 8.9, 9.3 / 8.1; eight 12.3 / 8.6, 12.8 / 9.5, 13.1 / 9.8.
-constexpr int64_t kMaxPixels64 = 8192;
+// 64 input channels fill a k-block of the tile kernels, and only the smallest problems are better off here: blocks of one output row,
+// of few pixels.  Microseconds back to back (100 launches in a graph), rows in shared memory / tiles, forward with sums, inference
+// epilogue with a shortcut, data gradient with batch norm.  One row a block: 8 x 8 pixels, one image 4.1 / 5.1, 3.6 / 5.0, 4.3 / 5.8;
+// 16 images 5.1 / 5.1, 4.6 / 5.1, 5.4 / 5.7; 14 x 14, ten 4.8 / 5.2, 4.3 / 5.2, 5.5 / 5.9; 28 x 28, five 5.1 / 5.3, 4.6 / 5.3, 5.6 /
+// 6.0; 32 x 32, two 4.7 / 5.1, 4.2 / 5.1, 5.5 / 5.9.  Two: 8 x 8, 24 images 5.3 / 5.1, 4.9 / 5.1, 6.0 / 5.8; 14 x 14, twelve 5.7 / 5.2,
+// 5.3 / 5.2, 6.2 / 5.9; 28 x 28, six 6.7 / 5.3, 6.4 / 5.2, 7.1 / 6.0.  Wider ones: 40 x 40, one image 5.2 / 5.1, 4.8 / 5.1, 5.6 /
+// 5.8; 56 x 56, one 5.7 / 5.3, 5.5 / 5.2, 6.2 / 6.0.
+bool rows_pay64(int N, int H, int W) { return (int64_t)N * H <= esgd::sm_count() && W <= 32; }
+
+// With the batch norm in front of it, which is a launch of its own ahead of the tiles: 8 x 8, 128 images (8192 pixels) 7.6 / 9.1, 256
+// images 10.1 / 11.3, 384 12.5 / 12.5; 14 x 14, 41 images (8036 pixels) 8.1 / 8.6, 48 9.1 / 8.8; 28 x 28, ten (7840 pixels) 8.0 / 8.8,
+// twelve 9.8 / 8.7; 32 x 32, eight 8.2 / 9.2.  (Rows of more than 32 pixels: the caller's choice.)
+constexpr int64_t kMaxNormPixels64 = 8192;
 
 // Returns -100 for shapes this file does not take (the caller then uses the tile kernels).  3x3, padding 1, NHWC bf16.
 // y = act(scale * conv + shift + residual), each part optional; sum / sqsum (caller-zeroed) receive y's statistics.
@@ -854,7 +861,7 @@ int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, in
   if (Cin == 16 && Cout == 32) return launch_conv<16, 32, false>(a, N, H, W, stride, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, false>(a, N, H, W, stride, s);
   if (Cin == 32 && Cout == 64) return launch_conv<32, 64, false>(a, N, H, W, stride, s);
-  if (Cin == 64 && Cout == 64 && (int64_t)N * H * W <= kMaxPixels64) return launch_conv<64, 64, false>(a, N, H, W, stride, s);
+  if (Cin == 64 && Cout == 64 && rows_pay64(N, H, W)) return launch_conv<64, 64, false>(a, N, H, W, stride, s);
   return -100;
 }
 
@@ -870,7 +877,7 @@ int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H
   cudaStream_t s = (cudaStream_t)stream;
   if (Cin == 16 && Cout == 16) return launch_conv<16, 16, true>(a, N, H, W, 1, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, true>(a, N, H, W, 1, s);
-  if (Cin == 64 && Cout == 64 && (int64_t)N * H * W <= kMaxPixels64) return launch_conv<64, 64, true>(a, N, H, W, 1, s);
+  if (Cin == 64 && Cout == 64 && rows_pay64(N, H, W)) return launch_conv<64, 64, true>(a, N, H, W, 1, s);
   return -100;
 }
 
@@ -906,7 +913,7 @@ int esgd_conv_narrow_bn_fwd(const void* by, void* z, void* mask, const float* bs
   cudaStream_t s = (cudaStream_t)stream;
   if (C == 16) return launch_conv<16, 16, false, true>(a, N, H, W, 1, s, b);
   if (C == 32) return launch_conv<32, 32, false, true>(a, N, H, W, 1, s, b);
-  if (C == 64 && m <= kMaxPixels64) return launch_conv<64, 64, false, true>(a, N, H, W, 1, s, b);
+  if (C == 64 && m <= kMaxNormPixels64) return launch_conv<64, 64, false, true>(a, N, H, W, 1, s, b);
   return -100;
 }
 

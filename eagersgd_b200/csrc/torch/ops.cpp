@@ -532,7 +532,9 @@ void launch_conv(int64_t kind, const Tensor& x, const Tensor& w, const Tensor& y
   const int64_t ho = y.size(2), wo = y.size(3);
   void* st = stream_of(x);
   if (norm != nullptr) {
-    if (kind == kGeneral && r == 3 && s == 3 && pad == 1 && stride == 1 && cin == cout && e.scale == nullptr && e.residual == nullptr && !e.relu) {
+    // 64 channels: rows of more than 32 pixels take two launches (rows in shared memory and these, us: 40 x 40, four images 9.5 and 8.5;
+    // 56 x 56, one 9.1 and 8.3, two 10.0 and 8.3; 32 x 32, eight 8.2 and 9.2)
+    if ((cin < 64 || wd <= 32) && kind == kGeneral && r == 3 && s == 3 && pad == 1 && stride == 1 && cin == cout && e.scale == nullptr && e.residual == nullptr && !e.relu) {
       *filters = nhwc(w);
       *kept = x;
       const int rc = esgd_conv_narrow_bn_fwd(norm->y.data_ptr(), x.data_ptr(), norm->mask.defined() ? norm->mask.data_ptr() : nullptr,

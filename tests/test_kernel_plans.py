@@ -170,3 +170,13 @@ def test_stems_are_launches_that_a_device_can_take(fake):
             assert h % 16 == 0 and w % 8 == 0 and len(rows) == len(more) == 1
             assert all(1 <= r[5] <= 148 and r[3] <= 227 * 1024 for r in rows + more)
     assert seen > 50
+
+
+@pytest.mark.parametrize("n,h,w,taken", [(1, 8, 8, True), (148, 1, 32, True), (149, 1, 32, False), (4, 37, 32, True), (1, 8, 33, False), (100, 8, 8, False)])
+def test_rows_in_shared_memory_for_64_channels(fake, n, h, w, taken):
+    """One output row a block, of at most 32 pixels; with the batch norm in front of it, up to 8192 pixels."""
+    rc, rows = _call(fake, "esgd_conv_narrow_fwd", P, P, P, n, h, w, 64, 64, 1, None, None, None, 0, P, P)
+    back, more = _call(fake, "esgd_conv_narrow_dgrad", P, P, P, n, h, w, 64, 64, None, None)
+    assert rc == back == (0 if taken else -100) and len(rows) == len(more) == int(taken)
+    if taken:
+        assert rows[0][5] == more[0][5] == n * h
