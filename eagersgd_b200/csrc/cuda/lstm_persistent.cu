@@ -600,9 +600,11 @@ int grid_of(bool bwd, int H, int S) { return (bwd ? H / 128 : H / 32) * S; }
 
 // How long after the cluster has published its own part a CTA asks for the others'.  Who asks too early asks twice, and one
 // CTA that is late makes all of them late; the other die sees a store after 900 cycles, and a grid of few CTAs sits on one.
-// Microseconds a step in a training step without / with it, 16 sequences: forward, 16 CTAs (256 units) 1.64 / 1.75, 32 (512)
-// 1.74 / 1.80, 64 (1024) 2.00 / 2.01, 128 (2048) 2.63 / 2.44; backward, whose CTAs read more and are later anyway, 64 (1024)
-// 2.26 / 2.29, 96 (2048) 3.20 / 3.37.
+// Forward, microseconds a step without / with it (16 CTAs are 256 units), 8, 16 and 32 sequences: 16 CTAs 1.59 / 1.66, 1.70 / 1.76,
+// 2.26 / 2.23; 48 1.93 / 1.93, 2.02 / 1.99, 2.77 / 2.67; 56 1.97 / 1.97, 2.07 / 2.05, 2.86 / 2.73; 64 1.97 / 1.97, 2.07 / 2.06, 2.87 /
+// 2.75; 72 2.16 / 2.07, 2.26 / 2.18, 3.03 / 3.05; 80 2.31 / 2.08, 2.44 / 2.17, 3.20 / 3.08; 128 2.60 / 2.38, 2.75 / 2.49, 3.55 / 3.42.
+// With 64 it has stopped costing and from 72 on it gives.  Backward, whose CTAs read more and are later anyway, in a training step
+// of 16 sequences: 64 CTAs (1024 units) 2.26 / 2.29, 96 (2048) 3.20 / 3.37.
 uint32_t hold_cycles(bool bwd, int ctas) { return !bwd && ctas >= 64 ? 350u : 0u; }
 
 // The cluster size for a layer of H units on the current device: the largest whose CTAs' share of the weights fits on the
