@@ -843,7 +843,14 @@ extern "C" {
 // 6.0; 32 x 32, two 4.7 / 5.1, 4.2 / 5.1, 5.5 / 5.9.  Two: 8 x 8, 24 images 5.3 / 5.1, 4.9 / 5.1, 6.0 / 5.8; 14 x 14, twelve 5.7 / 5.2,
 // 5.3 / 5.2, 6.2 / 5.9; 28 x 28, six 6.7 / 5.3, 6.4 / 5.2, 7.1 / 6.0.  Wider ones: 40 x 40, one image 5.2 / 5.1, 4.8 / 5.1, 5.6 /
 // 5.8; 56 x 56, one 5.7 / 5.3, 5.5 / 5.2, 6.2 / 6.0.
-bool rows_pay64(int N, int H, int W) { return (int64_t)N * H <= esgd::sm_count() && W <= 32; }
+//
+// Inference, up to 4096 pixels in rows of at most 64: the two are within 0.6 us of one another on the device (64 images of 8 x 8 5.1 to
+// 5.7 / 5.1, sixteen of 14 x 14 5.2 / 5.2, four of 28 x 28 5.2 / 5.2, one of 56 x 56 5.5 / 5.3; but one of 36 x 112 7.6 / 5.4), and a
+// few images are bound by the host, which has three or four tensor maps less to make here: 3.0 us a call and 3.4.
+bool rows_pay64(int N, int H, int W, bool inference) {
+  if ((int64_t)N * H <= esgd::sm_count() && W <= 32) return true;
+  return inference && (int64_t)N * H * W <= 4096 && W <= 64;
+}
 
 // With the batch norm in front of it, which is a launch of its own ahead of the tiles: 8 x 8, 128 images (8192 pixels) 7.6 / 9.1, 256
 // images 10.1 / 11.3, 384 12.5 / 12.5; 14 x 14, 41 images (8036 pixels) 8.1 / 8.6, 48 9.1 / 8.8; 28 x 28, ten (7840 pixels) 8.0 / 8.8,
@@ -861,7 +868,7 @@ int esgd_conv_narrow_fwd(const void* x, const void* w, void* y, int N, int H, in
   if (Cin == 16 && Cout == 32) return launch_conv<16, 32, false>(a, N, H, W, stride, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, false>(a, N, H, W, stride, s);
   if (Cin == 32 && Cout == 64) return launch_conv<32, 64, false>(a, N, H, W, stride, s);
-  if (Cin == 64 && Cout == 64 && rows_pay64(N, H, W)) return launch_conv<64, 64, false>(a, N, H, W, stride, s);
+  if (Cin == 64 && Cout == 64 && rows_pay64(N, H, W, sum == nullptr)) return launch_conv<64, 64, false>(a, N, H, W, stride, s);
   return -100;
 }
 
@@ -877,7 +884,7 @@ int esgd_conv_narrow_dgrad(const void* dy, const void* w, void* dx, int N, int H
   cudaStream_t s = (cudaStream_t)stream;
   if (Cin == 16 && Cout == 16) return launch_conv<16, 16, true>(a, N, H, W, 1, s);
   if (Cin == 32 && Cout == 32) return launch_conv<32, 32, true>(a, N, H, W, 1, s);
-  if (Cin == 64 && Cout == 64 && rows_pay64(N, H, W)) return launch_conv<64, 64, true>(a, N, H, W, 1, s);
+  if (Cin == 64 && Cout == 64 && rows_pay64(N, H, W, false)) return launch_conv<64, 64, true>(a, N, H, W, 1, s);
   return -100;
 }
 

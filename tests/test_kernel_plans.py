@@ -172,11 +172,17 @@ def test_stems_are_launches_that_a_device_can_take(fake):
     assert seen > 50
 
 
-@pytest.mark.parametrize("n,h,w,taken", [(1, 8, 8, True), (148, 1, 32, True), (149, 1, 32, False), (4, 37, 32, True), (1, 8, 33, False), (100, 8, 8, False)])
-def test_rows_in_shared_memory_for_64_channels(fake, n, h, w, taken):
-    """One output row a block, of at most 32 pixels; with the batch norm in front of it, up to 8192 pixels."""
-    rc, rows = _call(fake, "esgd_conv_narrow_fwd", P, P, P, n, h, w, 64, 64, 1, None, None, None, 0, P, P)
-    back, more = _call(fake, "esgd_conv_narrow_dgrad", P, P, P, n, h, w, 64, 64, None, None)
-    assert rc == back == (0 if taken else -100) and len(rows) == len(more) == int(taken)
-    if taken:
-        assert rows[0][5] == more[0][5] == n * h
+@pytest.mark.parametrize("n,h,w,training,inference", [(1, 8, 8, True, True), (148, 1, 32, True, True), (149, 1, 32, False, False), (149, 1, 27, False, True), (4, 37, 32, True, True),
+                                                      (1, 8, 33, False, True), (64, 8, 8, False, True), (65, 8, 8, False, False), (1, 64, 64, False, True),
+                                                      (1, 8, 65, False, False)])
+def test_rows_in_shared_memory_for_64_channels(fake, n, h, w, training, inference):
+    """One output row a block, of at most 32 pixels; in inference up to 4096 pixels in rows of at most 64 as well."""
+    sizes = (n, h, w, 64, 64)
+    inference = inference or training
+    for want, call in ((training, ("esgd_conv_narrow_fwd", P, P, P) + sizes + (1, None, None, None, 0, P, P)),
+                       (training, ("esgd_conv_narrow_dgrad", P, P, P) + sizes + (None, None)),
+                       (inference, ("esgd_conv_narrow_fwd", P, P, P) + sizes + (1, P, P, P, 1, None, None))):
+        rc, rows = _call(fake, *call)
+        assert rc == (0 if want else -100) and len(rows) == int(want), call
+        if want:
+            assert rows[0][5] == min(n * h, 148)
